@@ -1,16 +1,19 @@
-"""ctypes binding of libghost_b200.so.
+"""Loaders of libghost_b200.so (through ctypes) and of the torch binding on top of it.
 
-The shared object is the product; this module only declares prototypes and turns status codes into
+The library is the product; this module only declares prototypes and turns status codes into
 the exception types GhostSuite raises (ValueError for bad arguments, RuntimeError otherwise).
 There is no fallback: if the library is missing or the device is not sm_100 every op raises.
 """
 from __future__ import annotations
 
 import ctypes as C
+import importlib.machinery
+import importlib.util
 import os
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "libghost_b200.so")
+BINDING_PATH = os.path.join(_HERE, "_ghost_torch.so")
 
 GHOST_OK = 0
 GHOST_ERR_INVALID = -1
@@ -27,6 +30,13 @@ class SmallJob(C.Structure):
     _fields_ = [("X", _vp), ("M", _vp), ("sum_out", _vp), ("n_train", _i), ("n_val", _i), ("F", _i),
                 ("sum_is_f32", _i), ("dot_scale", _f), ("sum_scale", _f),
                 ("Xv", _vp), ("v_rank_pitch", _ll), ("v_per_rank", _i)]
+
+
+class PassJob(C.Structure):
+    """``ghost_pass_job`` of include/ghost_b200.h."""
+    _fields_ = [("X", _vp), ("Xv", _vp), ("M", _vp), ("vec", _vp), ("sum_out", _vp), ("v_rank_pitch", _ll),
+                ("n_train", _i), ("n_val", _i), ("F", _i), ("v_per_rank", _i), ("sum_is_f32", _i),
+                ("dot_scale", _f), ("sum_scale", _f)]
 
 
 # name -> (restype, argtypes); mirrors include/ghost_b200.h one to one
@@ -57,6 +67,8 @@ PROTOTYPES = {
     "ghost_small_gram_f32": (_i, [_vp, _i, _i, _i, _f, _vp, _vp]),
     "ghost_rows_sum": (_i, [_vp, _i, _i, _f, _vp, _i, _i, _vp]),
     "ghost_small_reduce_batch": (_i, [C.POINTER(SmallJob), _i, _vp]),
+    "ghost_pass_reduce": (_i, [C.POINTER(PassJob), _i, _vp]),
+    "ghost_matrix_sum": (_i, [C.POINTER(_vp), _i, _i, _i, _vp, _vp, _vp, _vp]),
     "ghost_embedding_dot_workspace_bytes": (_ll, [_i, _ll, _i]),
     "ghost_embedding_dot_workspace_bytes_for": (_ll, [_i, _ll, _i, _i]),
     "ghost_embedding_dot": (_i, [_vp, _vp, _i, _i, _i, _ll, _i, _i, _f, _vp, _vp, _ll, _vp]),
@@ -73,6 +85,7 @@ PROTOTYPES = {
 }
 
 _lib = None
+_native = None
 
 
 class GhostKernelError(RuntimeError):
@@ -95,6 +108,23 @@ def load() -> C.CDLL:
         fn.argtypes = args
     _lib = lib
     return lib
+
+
+def native():
+    """The torch binding (``_ghost_torch.so``), loaded once; raises RuntimeError when it is absent."""
+    global _native
+    if _native is None:
+        load()
+        if not os.path.exists(BINDING_PATH):
+            raise RuntimeError(f"{BINDING_PATH} is missing: build it with `python -m ghostsuite_b200.build`. "
+                               "There is no CPU or PyTorch fallback.")
+        import torch  # noqa: F401  (the binding resolves its torch symbols from the loaded libraries)
+        loader = importlib.machinery.ExtensionFileLoader("_ghost_torch", BINDING_PATH)
+        module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_ghost_torch", loader))
+        loader.exec_module(module)
+        module.set_kernel_error(GhostKernelError)
+        _native = module
+    return _native
 
 
 def last_error() -> str:

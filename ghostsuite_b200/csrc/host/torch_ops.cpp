@@ -1,0 +1,707 @@
+// Host side of the operations on torch tensors: operand preparation, workspaces, output allocation and
+// the calls into libghost_b200, in one native call per operation.  A hooked layer's work is a few
+// launches of a few microseconds; the same steps in Python and ctypes (a stream lookup, an output
+// allocation, an argument conversion each) took 20 to 60 us per operation and bound every step that
+// does not fill the GPU.  Entry points take positional arguments only (METH_FASTCALL); ghostsuite_b200/
+// ops.py holds the documented signatures.
+#include <Python.h>
+
+#include <ATen/ATen.h>
+#include <ATen/cuda/CUDAContext.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include <algorithm>
+#include <map>
+#include <mutex>
+#include <stdexcept>
+#include <string>
+#include <utility>
+#include <vector>
+
+#include "../../../include/ghost_b200.h"
+
+namespace {
+
+using at::Tensor;
+
+// ---- errors ------------------------------------------------------------------------------------
+struct GhostError : std::runtime_error {
+  int code;
+  GhostError(int c, const std::string& m) : std::runtime_error(m), code(c) {}
+};
+[[noreturn]] void invalid(const std::string& m) { throw GhostError(GHOST_ERR_INVALID, m); }
+void check(int status) {
+  if (status != GHOST_OK) throw GhostError(status, ghost_last_error());
+}
+PyObject* g_kernel_error = nullptr;     // ghostsuite_b200._lib.GhostKernelError
+
+template <typename F> PyObject* guarded(F&& f) {
+  try {
+    return f();
+  } catch (const GhostError& e) {
+    PyObject* type = e.code == GHOST_ERR_INVALID ? PyExc_ValueError
+                   : e.code == GHOST_ERR_INDEX ? PyExc_IndexError
+                   : e.code == GHOST_ERR_DEVICE || e.code > 0 || g_kernel_error == nullptr ? PyExc_RuntimeError
+                                                                                           : g_kernel_error;
+    const std::string text = e.code == GHOST_ERR_DEVICE ? std::string("ghostsuite_b200 needs a B200 (sm_100) GPU: ") + e.what()
+                                                        : std::string(e.what());
+    PyErr_SetString(type, text.c_str());
+  } catch (const c10::OutOfMemoryError& e) {
+    // torch.cuda.OutOfMemoryError where torch exposes it, as from torch.empty
+    PyObject* mod = PyImport_ImportModule("torch");
+    PyObject* type = mod ? PyObject_GetAttrString(mod, "OutOfMemoryError") : nullptr;
+    PyErr_Clear();
+    PyErr_SetString(type ? type : PyExc_RuntimeError, e.what_without_backtrace());
+    Py_XDECREF(type);
+    Py_XDECREF(mod);
+  } catch (const std::exception& e) {
+    PyErr_SetString(PyExc_RuntimeError, e.what());
+  }
+  return nullptr;
+}
+
+// ---- arguments -----------------------------------------------------------------------------------
+constexpr int kNotCuda = 1;             // positive codes: plain RuntimeError
+bool present(PyObject* o) { return o != nullptr && o != Py_None; }
+const Tensor& tensor(PyObject* o) {
+  if (!THPVariable_Check(o)) invalid("expected a tensor");
+  return THPVariable_Unpack(o);
+}
+const Tensor& cuda_tensor(PyObject* o) {
+  const Tensor& t = tensor(o);
+  if (!t.is_cuda()) throw GhostError(kNotCuda, "ghostsuite_b200 kernels need CUDA tensors (no CPU fallback exists)");
+  return t;
+}
+long long integer(PyObject* o) {
+  const long long v = PyLong_AsLongLong(o);
+  if (v == -1 && PyErr_Occurred()) { PyErr_Clear(); invalid("expected an integer"); }
+  return v;
+}
+float real(PyObject* o) {
+  const double v = PyFloat_AsDouble(o);
+  if (v == -1.0 && PyErr_Occurred()) { PyErr_Clear(); invalid("expected a number"); }
+  return static_cast<float>(v);
+}
+void need(Py_ssize_t have, Py_ssize_t want, const char* who) {
+  if (have != want) invalid(std::string(who) + ": wrong number of arguments");
+}
+PyObject* wrap(Tensor t) { return THPVariable_Wrap(std::move(t)); }
+PyObject* wrap_or_none(const Tensor& t) {
+  if (t.defined()) return THPVariable_Wrap(t);
+  Py_RETURN_NONE;
+}
+
+int is_f32(const Tensor& t) {
+  if (t.scalar_type() == at::kFloat) return 1;
+  if (t.scalar_type() == at::kBFloat16) return 0;
+  invalid(std::string("unsupported dtype ") + c10::toString(t.scalar_type()) + ": the kernels take float32 and bfloat16");
+}
+// [N, d] -> [N, 1, d]; [N, ..., d] -> [N, T, d], contiguous; float16 / float64 become float32
+Tensor as3d(const Tensor& x0) {
+  Tensor x = x0;
+  if (x.scalar_type() == at::kHalf || x.scalar_type() == at::kDouble) x = x.to(at::kFloat);
+  if (x.dim() == 3) return x.is_contiguous() ? x : x.contiguous();
+  if (x.dim() <= 2) x = x.unsqueeze(1);
+  else x = x.reshape({x.size(0), -1, x.size(-1)});
+  return x.contiguous();
+}
+Tensor ids2d(const Tensor& x0) {
+  Tensor x = x0.dim() == 2 ? x0 : x0.reshape({x0.size(0), -1});
+  if (x.scalar_type() != at::kLong) x = x.to(at::kLong);
+  return x.contiguous();
+}
+bool tma_ready(const Tensor& x) {
+  return x.scalar_type() == at::kBFloat16 && x.size(-1) % 8 == 0 && (reinterpret_cast<uintptr_t>(x.data_ptr()) & 15u) == 0;
+}
+long long pad8(long long n) { return (n + 7) / 8 * 8; }
+Tensor empty(at::IntArrayRef size, const Tensor& like, at::ScalarType dt) { return at::empty(size, like.options().dtype(dt)); }
+
+// Device and stream of one operation.
+struct Launch {
+  c10::cuda::CUDAGuard guard;
+  c10::cuda::CUDAStream stream;
+  explicit Launch(const Tensor& t) : guard(t.device()), stream(c10::cuda::getCurrentCUDAStream(t.get_device())) {}
+  void* st() const { return static_cast<void*>(stream.stream()); }
+};
+
+// ---- workspace -------------------------------------------------------------------------------------
+// One growing buffer per (device, stream).  A buffer that is replaced goes back to torch's caching
+// allocator, which hands it out again in stream order, so kernels queued on it are safe; callers hold
+// the GIL for a whole operation, so two threads on one stream cannot mix their parts.
+std::mutex g_arena_mu;
+std::map<std::pair<int, void*>, Tensor> g_arenas;
+
+class Workspace {
+ public:
+  long long plan(long long nbytes) {
+    const long long at = total_;
+    total_ += (nbytes + 255) / 256 * 256;
+    return at;
+  }
+  char* commit(const Launch& L, const Tensor& like) {
+    const long long want = total_ + 256;
+    std::lock_guard<std::mutex> lock(g_arena_mu);
+    Tensor& buf = g_arenas[{like.get_device(), L.st()}];
+    if (!buf.defined() || buf.numel() < want) {
+      buf = Tensor();
+      buf = at::empty({want > (1 << 20) ? want : (1 << 20)}, like.options().dtype(at::kByte));
+    }
+    const uintptr_t base = reinterpret_cast<uintptr_t>(buf.data_ptr());
+    return reinterpret_cast<char*>((base + 255) / 256 * 256);
+  }
+
+ private:
+  long long total_ = 0;
+};
+
+PyObject* py_arena_clear(PyObject*, PyObject* const*, Py_ssize_t) {
+  std::lock_guard<std::mutex> lock(g_arena_mu);
+  g_arenas.clear();
+  Py_RETURN_NONE;
+}
+
+// hi/lo layouts of an fp32 operand pair so that sum_k L[k] R[k] = hi*hi + lo*hi + hi*lo
+constexpr int kSplitLeft[3] = {0, 1, 0};
+constexpr int kSplitRight[3] = {0, 0, 1};
+constexpr int kPlain[3] = {0, 0, 0};
+
+void cast(const Tensor& src, long long row0, long long samples, long long T, void* dst, long long ld_dst, long long cpad,
+          int parts, const int (&kinds)[3], bool row_stack, void* st) {
+  const long long cols = src.size(-1);
+  const char* p = static_cast<const char*>(src.data_ptr()) + row0 * cols * src.element_size();
+  check(ghost_cast_split_bf16(p, is_f32(src), samples, T, static_cast<int>(cols), cols, dst, ld_dst, static_cast<int>(cpad),
+                              parts, kinds[0], kinds[1], kinds[2], row_stack ? 1 : 0, st));
+}
+
+void check_split(long long n_train, long long n_val, const char* who) {
+  if (n_train <= 0) invalid("No training samples to compute dot product, check batch sizes.");
+  if (n_val <= 0) invalid(std::string(who) + " needs at least one validation sample");
+}
+
+// ---- Gram path -----------------------------------------------------------------------------------------
+Tensor gram_dot(const Launch& L, const Tensor& A, const Tensor& G, long long n_val, int round_mode, float scale) {
+  const long long N = A.size(0), T = A.size(1), n_train = N - n_val;
+  check_split(n_train, n_val, "gram_dot");
+  if (G.size(0) != N || G.size(1) != T) invalid("gram_dot: activation and out-grad disagree on [batch, tokens]");
+  Tensor M = empty({n_val, n_train}, A, at::kFloat);
+  Workspace ws;
+  struct Op { int kind; long long cp, off_t, off_v; } op[2];      // kind 0 as it is, 1 padded copy, 2 split
+  const Tensor* xs[2] = {&A, &G};
+  for (int i = 0; i < 2; ++i) {
+    const Tensor& x = *xs[i];
+    const long long cp = pad8(x.size(-1));
+    if (is_f32(x)) {
+      op[i] = {2, cp, ws.plan(n_train * T * 3 * cp * 2), 0};
+      op[i].off_v = ws.plan(n_val * T * 3 * cp * 2);
+    } else if (tma_ready(x)) {
+      op[i] = {0, cp, 0, 0};
+    } else {
+      op[i] = {1, cp, ws.plan(N * T * cp * 2), 0};
+    }
+  }
+  char* base = ws.commit(L, A);
+  const char *pt[2], *pv[2];
+  long long k[2];
+  for (int i = 0; i < 2; ++i) {
+    const Tensor& x = *xs[i];
+    const long long cp = op[i].cp;
+    if (op[i].kind == 2) {
+      cast(x, 0, n_train, T, base + op[i].off_t, 3 * cp, cp, 3, kSplitLeft, false, L.st());
+      cast(x, n_train * T, n_val, T, base + op[i].off_v, 3 * cp, cp, 3, kSplitRight, false, L.st());
+      pt[i] = base + op[i].off_t;
+      pv[i] = base + op[i].off_v;
+      k[i] = 3 * cp;
+    } else {
+      if (op[i].kind == 1) cast(x, 0, N, T, base + op[i].off_t, cp, cp, 1, kPlain, false, L.st());
+      pt[i] = op[i].kind == 1 ? base + op[i].off_t : static_cast<const char*>(x.data_ptr());
+      pv[i] = pt[i] + n_train * T * cp * 2;
+      k[i] = cp;
+    }
+  }
+  check(ghost_gram_dot_bf16(pt[0], pv[0], pt[1], pv[1], static_cast<int>(n_train), static_cast<int>(n_val), T,
+                            static_cast<int>(k[0]), static_cast<int>(k[1]), k[0], k[0], k[1], k[1], round_mode, scale,
+                            M.data_ptr<float>(), L.st()));
+  return M;
+}
+
+PyObject* py_gram_dot(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    need(n, 5, "gram_dot");
+    const Tensor &A0 = cuda_tensor(a[0]), &G0 = cuda_tensor(a[1]);
+    Launch L(A0);
+    return wrap(gram_dot(L, as3d(A0), as3d(G0), integer(a[2]), static_cast<int>(integer(a[3])), real(a[4])));
+  });
+}
+
+// ---- token-contracted GEMMs --------------------------------------------------------------------------
+struct XtyOperands {
+  const Tensor* x[2];
+  long long samples, T, cp[2], off[2] = {0, 0};
+  int kind[2];                      // 0 as it is, 1 padded copy, 2 split
+  bool split;
+  XtyOperands(Workspace& ws, const Tensor& X, const Tensor& Y, long long samples_, long long T_) : samples(samples_), T(T_) {
+    x[0] = &X;
+    x[1] = &Y;
+    split = is_f32(X) || is_f32(Y);
+    for (int i = 0; i < 2; ++i) {
+      cp[i] = pad8(x[i]->size(-1));
+      kind[i] = split ? 2 : tma_ready(*x[i]) ? 0 : 1;
+      if (kind[i]) off[i] = ws.plan(samples * (split ? 3 : 1) * T * cp[i] * 2);
+    }
+  }
+  const void* get(int i, char* base, void* st) const {
+    if (kind[i] == 0) return x[i]->data_ptr();
+    if (kind[i] == 1) cast(*x[i], 0, samples, T, base + off[i], cp[i], cp[i], 1, kPlain, true, st);
+    else cast(*x[i], 0, samples, T, base + off[i], cp[i], cp[i], 3, i == 0 ? kSplitLeft : kSplitRight, true, st);
+    return base + off[i];
+  }
+  long long tokens() const { return split ? 3 * T : T; }
+};
+
+// scale * sum over the first `samples` samples of X^T Y, into out
+void wgrad(const Launch& L, const Tensor& X, const Tensor& Y, long long samples, float scale, Tensor& out, bool accumulate) {
+  const long long T = X.size(1);
+  const int m = static_cast<int>(X.size(2)), n = static_cast<int>(Y.size(2));
+  Workspace ws;
+  const long long ws_bytes = ghost_wgrad_workspace_bytes(m, n);
+  const long long off_ws = ws.plan(ws_bytes);
+  XtyOperands ops(ws, X, Y, samples, T);
+  char* base = ws.commit(L, X);
+  const void* xp = ops.get(0, base, L.st());
+  const void* yp = ops.get(1, base, L.st());
+  check(ghost_wgrad_bf16(xp, yp, samples * ops.tokens(), m, n, ops.cp[0], ops.cp[1], scale, accumulate ? 1 : 0,
+                         out.data_ptr(), is_f32(out), base + off_ws, ws_bytes, L.st()));
+}
+
+// (X, Y, scale, f32_out, out or None, accumulate)
+PyObject* py_wgrad(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    need(n, 6, "wgrad");
+    const Tensor &X0 = cuda_tensor(a[0]), &Y0 = cuda_tensor(a[1]);
+    Launch L(X0);
+    const Tensor X = as3d(X0), Y = as3d(Y0);
+    if (Y.size(0) != X.size(0) || Y.size(1) != X.size(1)) invalid("wgrad operands disagree on the token layout");
+    const bool have = present(a[4]);
+    Tensor out = have ? cuda_tensor(a[4]) : empty({X.size(2), Y.size(2)}, X, integer(a[3]) ? at::kFloat : at::kBFloat16);
+    wgrad(L, X, Y, X.size(0), real(a[2]), out, have && integer(a[5]));
+    return wrap(out);
+  });
+}
+
+// ---- per-sample path -----------------------------------------------------------------------------------
+struct PerSample { Tensor M, grad, colsums; };
+
+PerSample persample_dot(const Launch& L, const Tensor& X, const Tensor& Y, long long n_val, float dot_scale, bool want_grad,
+                        float grad_scale, at::ScalarType grad_dt, int colsum_of) {
+  const long long N = X.size(0), T = X.size(1), n_train = N - n_val;
+  const int m = static_cast<int>(X.size(2)), n = static_cast<int>(Y.size(2));
+  check_split(n_train, n_val, "persample_dot");
+  if (Y.size(0) != N || Y.size(1) != T) invalid("persample_dot operands disagree on the token layout");
+  PerSample r;
+  r.M = empty({n_val, n_train}, X, at::kFloat);
+  if (want_grad) r.grad = empty({m, n}, X, grad_dt);
+  Workspace ws;
+  XtyOperands ops(ws, X, Y, N, T);
+  const int f32 = ops.split ? 1 : 0;
+  const long long ws_bytes = ghost_persample_workspace_bytes(static_cast<int>(n_train), static_cast<int>(n_val), m, n, f32);
+  const long long off_ws = ws.plan(ws_bytes);
+  char* base = ws.commit(L, X);
+  if (colsum_of && !ops.split) r.colsums = empty({N, colsum_of == 1 ? m : n}, X, at::kFloat);
+  const void* xp = ops.get(0, base, L.st());
+  const void* yp = ops.get(1, base, L.st());
+  check(ghost_persample_dot_bf16(xp, yp, static_cast<int>(n_train), static_cast<int>(n_val), ops.tokens(), m, n, ops.cp[0],
+                                 ops.cp[1], dot_scale, r.M.data_ptr<float>(), f32, want_grad ? r.grad.data_ptr() : nullptr,
+                                 want_grad ? is_f32(r.grad) : 0, grad_scale, 0, r.colsums.defined() ? colsum_of : 0,
+                                 r.colsums.defined() ? r.colsums.data_ptr<float>() : nullptr, base + off_ws, ws_bytes, L.st()));
+  return r;
+}
+
+// (X, Y, n_val, dot_scale, want_grad, grad_scale, grad_is_f32, colsum_of: 0 / 1 = X / 2 = Y)
+PyObject* py_persample_dot(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    need(n, 8, "persample_dot");
+    const Tensor &X0 = cuda_tensor(a[0]), &Y0 = cuda_tensor(a[1]);
+    Launch L(X0);
+    PerSample r = persample_dot(L, as3d(X0), as3d(Y0), integer(a[2]), real(a[3]), integer(a[4]) != 0, real(a[5]),
+                                integer(a[6]) ? at::kFloat : at::kBFloat16, static_cast<int>(integer(a[7])));
+    return Py_BuildValue("(NNN)", wrap(r.M), wrap_or_none(r.grad), wrap_or_none(r.colsums));
+  });
+}
+
+// ---- column sums, norms --------------------------------------------------------------------------------
+Tensor colsum(const Launch& L, const Tensor& G) {
+  const long long N = G.size(0), T = G.size(1), p = G.size(2);
+  Tensor out = empty({N, p}, G, at::kFloat);
+  check(ghost_colsum(G.data_ptr(), is_f32(G), static_cast<int>(N), T, static_cast<int>(p), p, out.data_ptr<float>(), L.st()));
+  return out;
+}
+
+PyObject* py_colsum(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    need(n, 1, "colsum");
+    const Tensor& G0 = cuda_tensor(a[0]);
+    Launch L(G0);
+    return wrap(colsum(L, as3d(G0)));
+  });
+}
+
+// (A, G, eps, rms) -> (gw, gb)
+PyObject* py_norm_persample(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    need(n, 4, "norm_persample");
+    Tensor A = cuda_tensor(a[0]), G = cuda_tensor(a[1]);
+    Launch L(A);
+    if (A.scalar_type() != G.scalar_type()) {
+      const at::ScalarType common = c10::promoteTypes(A.scalar_type(), G.scalar_type());
+      A = A.to(common);
+      G = G.to(common);
+    }
+    A = as3d(A);
+    G = as3d(G);
+    const long long N = A.size(0), T = A.size(1), F = A.size(2);
+    if (G.sizes() != A.sizes()) invalid("LayerNorm input and out-grad shapes differ");
+    Tensor both = empty({2, N, F}, A, at::kFloat);
+    Tensor gw = both.select(0, 0), gb = both.select(0, 1);
+    Workspace ws;
+    const long long ws_bytes = ghost_layernorm_workspace_bytes(static_cast<int>(N), T, static_cast<int>(F));
+    const long long off = ws.plan(ws_bytes);
+    char* base = ws.commit(L, A);
+    auto fn = integer(a[3]) ? ghost_rmsnorm_persample : ghost_layernorm_persample;
+    check(fn(A.data_ptr(), G.data_ptr(), is_f32(A), static_cast<int>(N), T, static_cast<int>(F), real(a[2]),
+             gw.data_ptr<float>(), gb.data_ptr<float>(), base + off, ws_bytes, L.st()));
+    return Py_BuildValue("(NN)", wrap(gw), wrap(gb));
+  });
+}
+
+// ---- embedding ------------------------------------------------------------------------------------------
+// (ids, G, n_val, vocab, scale)
+PyObject* py_embedding_dot(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    need(n, 5, "embedding_dot");
+    const Tensor &ids0 = cuda_tensor(a[0]), &G0 = cuda_tensor(a[1]);
+    Launch L(G0);
+    const Tensor ids = ids2d(ids0), G = as3d(G0);
+    const long long N = G.size(0), T = G.size(1), d = G.size(2), n_val = integer(a[2]), vocab = integer(a[3]);
+    if (ids.size(0) != N || ids.size(1) != T) invalid("embedding ids and out-grad disagree on [batch, tokens]");
+    const long long n_train = N - n_val;
+    if (n_train <= 0) invalid("No training samples to compute dot product, check batch sizes.");
+    Tensor M = empty({n_val, n_train}, G, at::kFloat);
+    Workspace ws;
+    const long long ws_bytes = ghost_embedding_dot_workspace_bytes_for(static_cast<int>(n_val), T, static_cast<int>(vocab),
+                                                                       static_cast<int>(d));
+    const long long off = ws.plan(ws_bytes);
+    char* base = ws.commit(L, G);
+    check(ghost_embedding_dot(reinterpret_cast<const long long*>(ids.data_ptr()), G.data_ptr(), is_f32(G),
+                              static_cast<int>(n_train), static_cast<int>(n_val), T, static_cast<int>(d),
+                              static_cast<int>(vocab), real(a[4]), M.data_ptr<float>(), base + off, ws_bytes, L.st()));
+    return wrap(M);
+  });
+}
+
+// (ids, G, n_train, vocab, pre_scale, divisor, out or None, accumulate)
+PyObject* py_embedding_wgrad(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    need(n, 8, "embedding_wgrad");
+    const Tensor &ids0 = cuda_tensor(a[0]), &G0 = cuda_tensor(a[1]);
+    Launch L(G0);
+    const Tensor ids = ids2d(ids0), G = as3d(G0);
+    const long long T = G.size(1), d = G.size(2), n_train = integer(a[2]), vocab = integer(a[3]);
+    const bool have = present(a[6]);
+    Tensor out = have ? cuda_tensor(a[6]) : empty({vocab, d}, G, G.scalar_type());
+    if (out.scalar_type() != G.scalar_type()) invalid("embedding_wgrad output must have the dtype of the out-grad");
+    Workspace ws;
+    const long long ws_bytes = ghost_embedding_wgrad_workspace_bytes(static_cast<int>(n_train), T, static_cast<int>(vocab));
+    const long long off = ws.plan(ws_bytes);
+    char* base = ws.commit(L, G);
+    check(ghost_embedding_wgrad(reinterpret_cast<const long long*>(ids.data_ptr()), G.data_ptr(), is_f32(G),
+                                static_cast<int>(n_train), T, static_cast<int>(d), static_cast<int>(vocab), real(a[4]),
+                                real(a[5]), have && integer(a[7]) ? 1 : 0, out.data_ptr(), base + off, ws_bytes, L.st()));
+    return wrap(out);
+  });
+}
+
+// ---- GradProj ---------------------------------------------------------------------------------------------
+void check_projection_out(const Tensor& out, long long B, long long k, const char* who) {
+  if (out.scalar_type() != at::kFloat || out.dim() != 2 || out.size(0) != B || out.stride(1) != 1 || out.size(1) < k)
+    invalid(std::string(who) + " output must be a float32 [B, >= k_r*k_c] row-major view");
+}
+
+// (G, A, P_r, P_c, k_r, k_c, scale, out)
+PyObject* py_gradproj_dense(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    need(n, 8, "gradproj_dense");
+    const Tensor &G0 = cuda_tensor(a[0]), &A0 = cuda_tensor(a[1]), &P_r = cuda_tensor(a[2]), &P_c = cuda_tensor(a[3]);
+    const Tensor& out = cuda_tensor(a[7]);
+    Launch L(G0);
+    const Tensor G = as3d(G0), A = as3d(A0);
+    const long long B = G.size(0), T = G.size(1), k_r = integer(a[4]), k_c = integer(a[5]);
+    if (A.size(0) != B || A.size(1) != T)
+      throw GhostError(kNotCuda, "Batch size mismatch between activations and output gradients");
+    check_projection_out(out, B, k_r * k_c, "gradproj");
+    const bool split = is_f32(G) || is_f32(A);
+    Workspace ws;
+    const Tensor* x[2] = {&G, &A};
+    long long cp[2], off[2] = {0, 0};
+    int kind[2];
+    for (int i = 0; i < 2; ++i) {
+      cp[i] = pad8(x[i]->size(-1));
+      kind[i] = split ? 2 : tma_ready(*x[i]) ? 0 : 1;
+      if (kind[i]) off[i] = ws.plan(B * T * (split ? 3 : 1) * cp[i] * 2);
+    }
+    char* base = ws.commit(L, G);
+    const void* p[2];
+    long long len[2];
+    for (int i = 0; i < 2; ++i) {
+      len[i] = split ? 3 * cp[i] : cp[i];
+      p[i] = kind[i] ? static_cast<const void*>(base + off[i]) : x[i]->data_ptr();
+      if (kind[i] == 1) cast(*x[i], 0, B, T, base + off[i], cp[i], cp[i], 1, kPlain, false, L.st());
+      else if (kind[i] == 2) cast(*x[i], 0, B, T, base + off[i], 3 * cp[i], cp[i], 3, kSplitLeft, false, L.st());
+    }
+    if (P_r.size(1) != len[0] || P_c.size(1) != len[1])
+      invalid("projection matrices were prepared for a different dtype/feature size");
+    check(ghost_gradproj_dense_bf16(p[0], p[1], static_cast<int>(B), T, static_cast<int>(len[0]), static_cast<int>(len[1]),
+                                    len[0], len[1], P_r.data_ptr(), P_c.data_ptr(), static_cast<int>(k_r),
+                                    static_cast<int>(k_c), P_r.size(1), P_c.size(1), real(a[6]), out.data_ptr<float>(),
+                                    out.stride(0), L.st()));
+    Py_INCREF(a[7]);
+    return a[7];
+  });
+}
+
+// (ids, G, P_o, P_i_t, k_o, k_i, scale, out or None)
+PyObject* py_gradproj_embedding(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    need(n, 8, "gradproj_embedding");
+    const Tensor &ids0 = cuda_tensor(a[0]), &G0 = cuda_tensor(a[1]), &P_o = cuda_tensor(a[2]), &P_i_t = cuda_tensor(a[3]);
+    Launch L(G0);
+    const Tensor ids = ids2d(ids0), G = as3d(G0);
+    const long long B = G.size(0), T = G.size(1), d = G.size(2), k_o = integer(a[4]), k_i = integer(a[5]);
+    if (ids.size(0) != B || ids.size(1) != T)
+      throw GhostError(kNotCuda, "Batch size mismatch between token ids and output gradients");
+    const bool split = is_f32(G) != 0;
+    const long long cp = pad8(d);
+    if (P_o.scalar_type() != at::kBFloat16 || P_o.dim() != 2 || P_o.size(0) != k_o || P_o.size(1) != (split ? 3 : 1) * cp)
+      invalid("P_o was prepared for a different dtype/feature size");
+    if (P_i_t.scalar_type() != at::kFloat || P_i_t.dim() != 2 || P_i_t.size(1) != k_i || !P_i_t.is_contiguous())
+      invalid("P_i must be passed as the contiguous float32 [vocab, k_i] transpose");
+    Tensor out = present(a[7]) ? cuda_tensor(a[7]) : empty({B, k_o * k_i}, G, at::kFloat);
+    check_projection_out(out, B, k_o * k_i, "embedding projection");
+    // The prepared split lays a float32 matrix out as (hi, hi, lo): the residual part starts at 2 * cp.
+    // The kernel covers up to 64 x 64 of a sample's block per launch; larger projections go block by
+    // block into the zeroed output.
+    const bool chunked = k_o > 64 || k_i > 64;
+    if (chunked) out.narrow(1, 0, k_o * k_i).zero_();
+    const long long ld_po = P_o.size(1);
+    for (long long o0 = 0; o0 < k_o; o0 += 64)
+      for (long long i0 = 0; i0 < k_i; i0 += 64)
+        check(ghost_gradproj_embedding(reinterpret_cast<const long long*>(ids.data_ptr()), G.data_ptr(), is_f32(G),
+                                       static_cast<int>(B), T, static_cast<int>(d), d,
+                                       static_cast<const char*>(P_o.data_ptr()) + o0 * ld_po * 2, ld_po, static_cast<int>(cp),
+                                       split ? static_cast<int>(2 * cp) : 0, P_i_t.data_ptr<float>() + i0, k_i,
+                                       static_cast<int>(P_i_t.size(0)), static_cast<int>(std::min(64ll, k_o - o0)),
+                                       static_cast<int>(std::min(64ll, k_i - i0)), real(a[6]), chunked ? 1 : 0,
+                                       out.data_ptr<float>() + o0 * k_i + i0, out.stride(0), static_cast<int>(k_i), L.st()));
+    return wrap(out);
+  });
+}
+
+// (P1, P2, scale)
+PyObject* py_projection_similarity(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    need(n, 3, "projection_similarity");
+    Tensor P1 = cuda_tensor(a[0]), P2 = cuda_tensor(a[1]);
+    Launch L(P1);
+    if (P1.dim() != 2 || P2.dim() != 2 || P1.size(1) != P2.size(1)) invalid("projection sets have different dimensions");
+    if (P1.scalar_type() != P2.scalar_type()) {
+      const at::ScalarType common = c10::promoteTypes(P1.scalar_type(), P2.scalar_type());
+      P1 = P1.to(common);
+      P2 = P2.to(common);
+    }
+    if (P1.scalar_type() != at::kFloat && P1.scalar_type() != at::kBFloat16) {
+      P1 = P1.to(at::kFloat);
+      P2 = P2.to(at::kFloat);
+    }
+    if (P1.stride(1) != 1) P1 = P1.contiguous();
+    if (P2.stride(1) != 1) P2 = P2.contiguous();
+    Tensor S = empty({P1.size(0), P2.size(0)}, P1, at::kFloat);
+    check(ghost_projection_similarity(P1.data_ptr(), P2.data_ptr(), is_f32(P1), static_cast<int>(P1.size(0)),
+                                      static_cast<int>(P2.size(0)), P1.size(1), P1.stride(0), P2.stride(0), real(a[2]),
+                                      S.data_ptr<float>(), S.stride(0), L.st()));
+    return wrap(S);
+  });
+}
+
+// ---- end of a backward pass ---------------------------------------------------------------------------------
+PyObject *k_X, *k_M, *k_sum_out, *k_n_train, *k_n_val, *k_dot_scale, *k_sum_scale, *k_Xv;
+
+PyObject* item(PyObject* dict, PyObject* key) { return PyDict_GetItemWithError(dict, key); }   // borrowed
+
+ghost_pass_job read_job(PyObject* d, int* device) {
+  if (!PyDict_Check(d)) invalid("small_reduce_batch takes a list of dicts");
+  ghost_pass_job j = {};
+  PyObject *x = item(d, k_X), *m = item(d, k_M), *s = item(d, k_sum_out);
+  if (!present(x)) invalid("small_reduce_batch: a job has no input");
+  const Tensor& X = cuda_tensor(x);
+  if (X.scalar_type() != at::kFloat || X.dim() != 2 || !X.is_contiguous())
+    invalid("small_reduce_batch takes contiguous float32 [N, F] tensors");
+  PyObject *nt = item(d, k_n_train), *nv = item(d, k_n_val);
+  if (!present(nt) || !present(nv)) invalid("small_reduce_batch: a job has no n_train / n_val");
+  *device = X.get_device();
+  j.X = X.data_ptr<float>();
+  j.F = static_cast<int>(X.size(1));
+  j.n_train = static_cast<int>(integer(nt));
+  j.n_val = static_cast<int>(integer(nv));
+  j.dot_scale = present(item(d, k_dot_scale)) ? real(item(d, k_dot_scale)) : 1.f;
+  j.sum_scale = present(item(d, k_sum_scale)) ? real(item(d, k_sum_scale)) : 1.f;
+  j.sum_is_f32 = 1;
+  if (present(m)) {
+    const Tensor& M = cuda_tensor(m);
+    if (M.scalar_type() != at::kFloat || !M.is_contiguous() || M.numel() != static_cast<long long>(j.n_val) * j.n_train)
+      invalid("small_reduce_batch: M must be a contiguous float32 [n_val, n_train] tensor");
+    j.M = M.data_ptr<float>();
+  }
+  if (present(s)) {
+    const Tensor& out = cuda_tensor(s);
+    if (!out.is_contiguous() || out.numel() != X.size(1)) invalid("small_reduce_batch: sum_out must be a contiguous [F] tensor");
+    j.sum_out = out.data_ptr();
+    j.sum_is_f32 = is_f32(out);
+  }
+  PyObject* xv = item(d, k_Xv);
+  if (present(xv)) {
+    if (!PyTuple_Check(xv) || PyTuple_GET_SIZE(xv) != 3) invalid("small_reduce_batch: bad layout of the separate validation rows");
+    const Tensor& g = cuda_tensor(PyTuple_GET_ITEM(xv, 0));
+    const long long offset = integer(PyTuple_GET_ITEM(xv, 1)), per_rank = integer(PyTuple_GET_ITEM(xv, 2));
+    if (g.scalar_type() != at::kFloat || g.dim() != 2 || !g.is_contiguous() || offset + per_rank * X.size(1) > g.size(1) ||
+        g.size(0) * per_rank != j.n_val || X.size(0) < j.n_train)
+      invalid("small_reduce_batch: bad layout of the separate validation rows");
+    j.Xv = g.data_ptr<float>() + offset;
+    j.v_rank_pitch = g.size(1);
+    j.v_per_rank = static_cast<int>(per_rank);
+  }
+  return j;
+}
+
+// (jobs: list of dicts, matrices: list of [n_val, n_train] tensors) -> list of [n_train] tensors, one per
+// matrix: the jobs' reductions and every listed matrix's sum over the validation samples, one launch
+// per device.  A matrix that a job fills gets its sum from that job.
+PyObject* py_pass_reduce(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    need(n, 2, "pass_reduce");
+    if (!PyList_Check(a[0]) || !PyList_Check(a[1])) invalid("pass_reduce takes two lists");
+    std::map<int, std::vector<ghost_pass_job>> per_device;
+    std::map<int, Tensor> any;               // a tensor of each device, for its stream
+    std::map<const float*, std::pair<int, size_t>> filled;
+    for (Py_ssize_t i = 0; i < PyList_GET_SIZE(a[0]); ++i) {
+      PyObject* d = PyList_GET_ITEM(a[0], i);
+      int dev = 0;
+      ghost_pass_job j = read_job(d, &dev);
+      if (j.M == nullptr && j.sum_out == nullptr) invalid("small_reduce_batch: a job has no output");
+      if (j.M) filled[j.M] = {dev, per_device[dev].size()};
+      per_device[dev].push_back(j);
+      any.emplace(dev, cuda_tensor(item(d, k_X)));
+    }
+    const Py_ssize_t n_mats = PyList_GET_SIZE(a[1]);
+    PyObject* out = PyList_New(n_mats);
+    if (!out) throw std::bad_alloc();
+    try {
+      // one buffer per run of equal column counts keeps the vectors' allocations to one or two
+      for (Py_ssize_t i = 0; i < n_mats;) {
+        const Tensor first = cuda_tensor(PyList_GET_ITEM(a[1], i));
+        Py_ssize_t e = i;
+        while (e < n_mats) {
+          const Tensor& t = cuda_tensor(PyList_GET_ITEM(a[1], e));
+          if (t.scalar_type() != at::kFloat || t.dim() != 2 || !t.is_contiguous())
+            invalid("pass_reduce: matrices are contiguous float32 [n_val, n_train]");
+          if (t.size(1) != first.size(1) || t.get_device() != first.get_device()) break;
+          ++e;
+        }
+        Tensor vecs = empty({e - i, first.size(1)}, first, at::kFloat);
+        for (Py_ssize_t k = i; k < e; ++k) {
+          const Tensor& t = cuda_tensor(PyList_GET_ITEM(a[1], k));
+          Tensor v = vecs.select(0, k - i);
+          float* vp = v.data_ptr<float>();
+          auto it = filled.find(t.data_ptr<float>());
+          if (it != filled.end() && per_device[it->second.first][it->second.second].vec == nullptr) {
+            per_device[it->second.first][it->second.second].vec = vp;
+          } else {
+            ghost_pass_job j = {};
+            j.M = t.data_ptr<float>();
+            j.vec = vp;
+            j.n_val = static_cast<int>(t.size(0));
+            j.n_train = static_cast<int>(t.size(1));
+            per_device[t.get_device()].push_back(j);
+            any.emplace(t.get_device(), t);
+          }
+          PyList_SET_ITEM(out, k, wrap(v));
+        }
+        i = e;
+      }
+      for (auto& [dev, jobs] : per_device) {
+        Launch L(any.at(dev));
+        check(ghost_pass_reduce(jobs.data(), static_cast<int>(jobs.size()), L.st()));
+      }
+    } catch (...) {
+      Py_DECREF(out);
+      throw;
+    }
+    return out;
+  });
+}
+
+// (matrices: list of equal [n_val, n_train]) -> float32 buffer of n_val * n_train + n_train + 1 elements: the
+// summed matrix, its column sums, and the device error word (bits of an int32)
+PyObject* py_matrix_sum(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    need(n, 1, "matrix_sum");
+    if (!PyList_Check(a[0]) || PyList_GET_SIZE(a[0]) == 0) invalid("matrix_sum takes a list of matrices");
+    const Tensor& first = cuda_tensor(PyList_GET_ITEM(a[0], 0));
+    if (first.dim() != 2) invalid("matrix_sum: matrices are [n_val, n_train]");
+    Launch L(first);
+    const long long nv = first.size(0), nt = first.size(1);
+    std::vector<const float*> p;
+    for (Py_ssize_t i = 0; i < PyList_GET_SIZE(a[0]); ++i) {
+      const Tensor& t = cuda_tensor(PyList_GET_ITEM(a[0], i));
+      if (t.scalar_type() != at::kFloat || !t.is_contiguous() || t.sizes() != first.sizes() || t.get_device() != first.get_device())
+        invalid("matrix_sum: matrices must be contiguous float32 of one shape on one device");
+      p.push_back(t.data_ptr<float>());
+    }
+    Tensor out = empty({nv * nt + nt + 1}, first, at::kFloat);
+    float* o = out.data_ptr<float>();
+    check(ghost_matrix_sum(p.data(), static_cast<int>(p.size()), static_cast<int>(nv), static_cast<int>(nt), o, o + nv * nt,
+                           reinterpret_cast<int*>(o + nv * nt + nt), L.st()));
+    return wrap(out);
+  });
+}
+
+PyObject* py_set_kernel_error(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  if (n == 1) {
+    Py_XDECREF(g_kernel_error);
+    Py_INCREF(a[0]);
+    g_kernel_error = a[0];
+  }
+  Py_RETURN_NONE;
+}
+
+#define GB_METHOD(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(py_##name)), METH_FASTCALL, nullptr}
+PyMethodDef kMethods[] = {
+    GB_METHOD(gram_dot),          GB_METHOD(wgrad),
+    GB_METHOD(persample_dot),     GB_METHOD(colsum),
+    GB_METHOD(norm_persample),    GB_METHOD(embedding_dot),
+    GB_METHOD(embedding_wgrad),   GB_METHOD(gradproj_dense),
+    GB_METHOD(gradproj_embedding), GB_METHOD(projection_similarity),
+    GB_METHOD(pass_reduce),       GB_METHOD(matrix_sum),
+    GB_METHOD(arena_clear),       GB_METHOD(set_kernel_error),
+    {nullptr, nullptr, 0, nullptr}};
+PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_ghost_torch", nullptr, -1, kMethods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__ghost_torch() {
+  struct { PyObject** at; const char* name; } keys[] = {{&k_X, "X"}, {&k_M, "M"}, {&k_sum_out, "sum_out"}, {&k_n_train, "n_train"},
+                                                        {&k_n_val, "n_val"}, {&k_dot_scale, "dot_scale"},
+                                                        {&k_sum_scale, "sum_scale"}, {&k_Xv, "Xv"}};
+  for (auto& k : keys) *k.at = PyUnicode_InternFromString(k.name);
+  return PyModule_Create(&kModule);
+}

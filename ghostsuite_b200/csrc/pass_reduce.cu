@@ -1,0 +1,346 @@
+// End-of-pass reductions.  A backward pass leaves one small job per parameter: the [n_val, n_train]
+// Gram of per-sample vectors (bias, LayerNorm, RMS norm), the sum of their train rows, and the column
+// sum over the validation samples of every parameter's matrix.  All of them run in one launch whose
+// jobs travel as kernel parameters; a second kernel adds the finished matrices of a step up.
+#include <string.h>
+
+#include <cooperative_groups.h>
+
+#include "common.cuh"
+
+namespace cg = cooperative_groups;
+
+namespace gb {
+
+// One cluster of eight CTAs per (job, block of 32 train samples).  The vectors are a few hundred
+// kilobytes in L2, so what bounds a job is how few SMs fetch them and the latency of each round of
+// loads: the eight CTAs split the vector length F; a CTA brings its columns of 32 train and eight
+// validation rows into shared memory with full-line copies, all in flight at once, and a lane then
+// holds one train sample against eight validation samples.  Partial sums meet in distributed shared
+// memory in a fixed order, so results do not depend on timing.  A warp per (validation, train) pair,
+// the form before it, fetched every row once per partner; lanes that loaded one row each from global
+// memory touched 32 lines per instruction.
+static constexpr int kPassCluster = 8;
+static constexpr int kPassThreads = 256;
+static constexpr int kPassSub = 256;                   // columns staged at a time
+static constexpr int kPassPitch = kPassSub + 4;        // rows 16 bytes apart modulo 128: no bank conflicts
+static constexpr int kPassSmem = 40 * kPassPitch * 4;  // 32 train rows, then eight validation rows
+
+template <int CAP> struct PassJobs { ghost_pass_job job[CAP]; };
+
+__device__ __forceinline__ const float* pass_val_row(const ghost_pass_job& j, int v) {
+  return j.Xv == nullptr ? j.X + static_cast<long long>(j.n_train + v) * j.F
+                         : j.Xv + static_cast<long long>(v / j.v_per_rank) * j.v_rank_pitch +
+                               static_cast<long long>(v % j.v_per_rank) * j.F;
+}
+
+// Columns [f, f + width) of the block's rows into shared memory, zero up to the next multiple of four
+__device__ __forceinline__ void pass_stage(const ghost_pass_job& j, bool vec, int b0, int v0, int f, int width, float* st) {
+  const int quads = (width + 3) / 4;
+  for (int i = threadIdx.x; i < 40 * quads; i += kPassThreads) {
+    const int r = i / quads, q = (i - r * quads) * 4;
+    const float* src;
+    if (r < 32) src = b0 + r < j.n_train ? j.X + static_cast<long long>(b0 + r) * j.F : nullptr;
+    else src = v0 + r - 32 < j.n_val ? pass_val_row(j, v0 + r - 32) : nullptr;
+    float* dst = st + r * kPassPitch + q;
+    if (src == nullptr) {
+      *reinterpret_cast<float4*>(dst) = make_float4(0.f, 0.f, 0.f, 0.f);
+    } else if (vec) {                    // F is a multiple of four then, and so is every width
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))),
+                   "l"(src + f + q) : "memory");
+    } else {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) dst[e] = q + e < width ? __ldg(src + f + q + e) : 0.f;
+    }
+  }
+  asm volatile("cp.async.wait_all;" ::: "memory");
+}
+
+// sum_out over columns [f0, f1): the clusters of a job take groups of 128 columns in turn, four groups at
+// a time; a warp adds every eighth train row, and the eight partial rows meet in shared memory.
+template <bool VEC>
+__device__ __forceinline__ void pass_row_sums(const ghost_pass_job& j, int f0, int f1, int blk, int n_blk, float* red) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int c0 = f0 + blk * 128; c0 < f1; c0 += 4 * 128 * n_blk) {
+    float4 acc[4];
+#pragma unroll
+    for (int g = 0; g < 4; ++g) acc[g] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+    for (int n = warp; n < j.n_train; n += 8) {
+      const float* row = j.X + static_cast<long long>(n) * j.F;
+#pragma unroll
+      for (int g = 0; g < 4; ++g) {
+        const int c = c0 + g * 128 * n_blk + lane * 4;
+        if constexpr (VEC) {
+          if (c < f1) {
+            const float4 x = __ldg(reinterpret_cast<const float4*>(row + c));
+            acc[g].x += x.x; acc[g].y += x.y; acc[g].z += x.z; acc[g].w += x.w;
+          }
+        } else {
+          if (c < f1) acc[g].x += __ldg(row + c);
+          if (c + 1 < f1) acc[g].y += __ldg(row + c + 1);
+          if (c + 2 < f1) acc[g].z += __ldg(row + c + 2);
+          if (c + 3 < f1) acc[g].w += __ldg(row + c + 3);
+        }
+      }
+    }
+    __syncthreads();                     // whatever used `red` before is done with it
+#pragma unroll
+    for (int g = 0; g < 4; ++g) *reinterpret_cast<float4*>(red + (warp * 4 + g) * 128 + lane * 4) = acc[g];
+    __syncthreads();
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int i = h * kPassThreads + threadIdx.x, c = c0 + (i >> 7) * 128 * n_blk + (i & 127);
+      if (c >= f1) continue;
+      float s = 0.f;
+#pragma unroll
+      for (int w = 0; w < 8; ++w) s += red[w * 512 + i];
+      s *= j.sum_scale;
+      if (j.sum_is_f32) static_cast<float*>(j.sum_out)[c] = s;
+      else static_cast<__nv_bfloat16*>(j.sum_out)[c] = __float2bfloat16_rn(s);
+    }
+  }
+}
+
+template <int CAP>
+__global__ void __cluster_dims__(kPassCluster, 1, 1) __launch_bounds__(kPassThreads)
+pass_reduce_kernel(const __grid_constant__ PassJobs<CAP> jobs) {
+  extern __shared__ __align__(16) float stage[];       // kPassSmem bytes
+  __shared__ float part[2][8][32];       // this CTA's share of F, read by rank 0 of the cluster
+  __shared__ float cols[8][32];
+  const ghost_pass_job& j = jobs.job[blockIdx.z];
+  const int blk = blockIdx.y;
+  const int n_blk = (j.n_train + 31) / 32;
+  if (blk >= n_blk) return;              // the whole cluster leaves
+  const int rank = blockIdx.x;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int b = blk * 32 + lane;
+  const bool live = b < j.n_train;
+
+  if (j.X == nullptr) {                  // the matrix exists already: column sums only
+    if (rank != 0) return;
+    float s = 0.f;
+    if (live)
+      for (int v = warp; v < j.n_val; v += 8) s += j.M[static_cast<long long>(v) * j.n_train + b];
+    cols[warp][lane] = s;
+    __syncthreads();
+    if (warp == 0 && live) {
+#pragma unroll
+      for (int w = 1; w < 8; ++w) s += cols[w][lane];
+      j.vec[b] = s;
+    }
+    return;
+  }
+
+  const int F = j.F;
+  const int chunk = ((F + kPassCluster - 1) / kPassCluster + 7) / 8 * 8;
+  const int f0 = rank * chunk;
+  const int f1 = f0 + chunk < F ? f0 + chunk : F;
+  const bool vec_x = (F & 3) == 0 && (reinterpret_cast<uintptr_t>(j.X) & 15) == 0;
+
+  if (j.M != nullptr) {
+    cg::cluster_group cluster = cg::this_cluster();
+    const bool vec = vec_x && (j.Xv == nullptr || ((reinterpret_cast<uintptr_t>(j.Xv) & 15) == 0 && (j.v_rank_pitch & 3) == 0));
+    float col = 0.f;                     // rank 0: this thread's share of vec
+    int buf = 0;
+    for (int v0 = 0; v0 < j.n_val; v0 += 8, buf ^= 1) {
+      float acc[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) acc[i] = 0.f;
+      for (int f = f0; f < f1; f += kPassSub) {
+        const int width = f1 - f < kPassSub ? f1 - f : kPassSub;
+        __syncthreads();
+        pass_stage(j, vec, blk * 32, v0, f, width, stage);
+        __syncthreads();
+        for (int q = warp * 4; q < width; q += 32) {
+          const float4 x = *reinterpret_cast<const float4*>(stage + lane * kPassPitch + q);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const float4 y = *reinterpret_cast<const float4*>(stage + (32 + i) * kPassPitch + q);
+            acc[i] = fmaf(x.x, y.x, acc[i]); acc[i] = fmaf(x.y, y.y, acc[i]);
+            acc[i] = fmaf(x.z, y.z, acc[i]); acc[i] = fmaf(x.w, y.w, acc[i]);
+          }
+        }
+      }
+      __syncthreads();
+      float* red = stage;                // [warp][validation row][train lane]
+#pragma unroll
+      for (int i = 0; i < 8; ++i) red[(warp * 8 + i) * 32 + lane] = acc[i];
+      __syncthreads();
+      float s = 0.f;                     // thread (warp, lane) now owns pair (v0 + warp, b)
+#pragma unroll
+      for (int w = 0; w < 8; ++w) s += red[(w * 8 + warp) * 32 + lane];
+      part[buf][warp][lane] = s;
+      // one cluster barrier per block: `part` alternates, and rank 0 reads block k's before it
+      // arrives at block k + 1's barrier, which every CTA passes before writing that buffer again
+      cluster.sync();
+      if (rank == 0) {
+        float m = 0.f;
+#pragma unroll
+        for (int r = 0; r < kPassCluster; ++r) m += *cluster.map_shared_rank(&part[buf][warp][lane], r);
+        m *= j.dot_scale;
+        if (v0 + warp < j.n_val && live) {
+          j.M[static_cast<long long>(v0 + warp) * j.n_train + b] = m;
+          col += m;
+        }
+      }
+    }
+    if (rank == 0 && j.vec != nullptr) {
+      cols[warp][lane] = col;
+      __syncthreads();
+      if (warp == 0 && live) {
+        float s = 0.f;
+#pragma unroll
+        for (int w = 0; w < 8; ++w) s += cols[w][lane];
+        j.vec[b] = s;
+      }
+    }
+    if (j.sum_out == nullptr) cluster.sync();   // no CTA leaves while rank 0 still reads its shared memory
+  }
+  if (j.sum_out != nullptr) {
+    if (vec_x) pass_row_sums<true>(j, f0, f1, blk, n_blk, stage);
+    else pass_row_sums<false>(j, f0, f1, blk, n_blk, stage);
+    if (j.M != nullptr) cg::this_cluster().sync();
+  }
+}
+
+template <int CAP>
+static int launch_pass(const ghost_pass_job* jobs, int n, int blocks, cudaStream_t st) {
+  PassJobs<CAP> batch;
+  memcpy(batch.job, jobs, sizeof(ghost_pass_job) * n);
+  pass_reduce_kernel<CAP><<<dim3(kPassCluster, blocks, n), kPassThreads, kPassSmem, st>>>(batch);
+  count_launch();
+  return post_launch("pass_reduce_kernel");
+}
+
+// total[v, b] = sum_p mats[p][v, b];  vec[b] = sum_v total[v, b].  One CTA per 32 train samples, its
+// 32 warps split over eight validation rows and four groups of matrices: a step has one matrix per
+// parameter, a few kilobytes each, and the time is the chain of loads per thread.
+static constexpr int kSumPointers = 440;   // 3520 bytes of pointers: below the 4 KB every driver takes
+struct MatrixList { const float* m[kSumPointers]; };
+
+__global__ void __launch_bounds__(1024)
+matrix_sum_kernel(const __grid_constant__ MatrixList list, int n, int n_val, int n_train, int accumulate,
+                  float* total, float* vec, const int* err_word, int* err_out) {
+  __shared__ float red[4][8][32];
+  __shared__ float cols[8][32];
+  const int lane = threadIdx.x & 31, row = (threadIdx.x >> 5) & 7, grp = threadIdx.x >> 8;
+  const int b = blockIdx.x * 32 + lane;
+  float col = 0.f;
+  for (int v0 = 0; v0 < n_val; v0 += 8) {
+    const int v = v0 + row;
+    const long long at = static_cast<long long>(v) * n_train + b;
+    const bool live = v < n_val && b < n_train;
+    float s = 0.f;
+    if (live) {
+#pragma unroll 8
+      for (int p = grp; p < n; p += 4) s += __ldg(list.m[p] + at);
+    }
+    red[grp][row][lane] = s;
+    __syncthreads();
+    if (grp == 0 && live) {
+      s = (red[0][row][lane] + red[1][row][lane]) + (red[2][row][lane] + red[3][row][lane]);
+      if (accumulate) s += total[at];
+      total[at] = s;
+      col += s;
+    }
+    __syncthreads();
+  }
+  if (grp == 0) cols[row][lane] = col;
+  __syncthreads();
+  if (threadIdx.x < 32 && b < n_train) {
+    float s = 0.f;
+#pragma unroll
+    for (int r = 0; r < 8; ++r) s += cols[r][lane];
+    vec[b] = s;
+  }
+  if (err_out != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *err_out = *err_word;
+}
+
+}  // namespace gb
+
+using namespace gb;
+
+extern "C" int ghost_pass_reduce(const ghost_pass_job* jobs, int n_jobs, void* stream) {
+  const DeviceState* ds = device_state();
+  if (!ds) return GHOST_ERR_DEVICE;
+  GB_REQUIRE(jobs != nullptr && n_jobs > 0, "ghost_pass_reduce: no jobs");
+  for (int i = 0; i < n_jobs; ++i) {
+    const ghost_pass_job& j = jobs[i];
+    GB_REQUIRE(j.n_train > 0 && j.n_val >= 0 && (j.M == nullptr || j.n_val > 0), "ghost_pass_reduce: job %d has an empty dimension", i);
+    GB_REQUIRE(j.n_train <= 32 * 65535, "ghost_pass_reduce: job %d has too many train samples", i);
+    if (j.X == nullptr) {
+      GB_REQUIRE(j.M != nullptr && j.vec != nullptr, "ghost_pass_reduce: job %d has no input or no output", i);
+      continue;
+    }
+    GB_REQUIRE(j.M != nullptr || j.sum_out != nullptr, "ghost_pass_reduce: job %d has no input or no output", i);
+    GB_REQUIRE(j.F > 0, "ghost_pass_reduce: job %d has an empty dimension", i);
+    GB_REQUIRE(j.M != nullptr || j.vec == nullptr, "ghost_pass_reduce: job %d wants column sums without a matrix", i);
+    GB_REQUIRE(j.Xv == nullptr || (j.v_per_rank > 0 && j.v_rank_pitch >= static_cast<long long>(j.v_per_rank) * j.F),
+               "ghost_pass_reduce: job %d has separate validation rows without a valid layout", i);
+  }
+  // Kernel parameters are copied whole whatever the job count, so short lists take a small block.
+  // A few jobs are one layer called on its own; the largest block (28 KB of the 32 KB a launch
+  // takes) holds all parameters of a GPT-2-sized model.
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  constexpr int kLarge = 300;
+  for (int first = 0; first < n_jobs; first += kLarge) {
+    const int n = n_jobs - first < kLarge ? n_jobs - first : kLarge;
+    int most = 1;
+    for (int i = 0; i < n; ++i) most = jobs[first + i].n_train > most ? jobs[first + i].n_train : most;
+    const int blocks = ceil_div(most, 32);
+    const int rc = n <= 4 ? launch_pass<4>(jobs + first, n, blocks, st)
+                 : n <= 40 ? launch_pass<40>(jobs + first, n, blocks, st)
+                           : launch_pass<kLarge>(jobs + first, n, blocks, st);
+    if (rc != GHOST_OK) return rc;
+  }
+  return GHOST_OK;
+}
+
+extern "C" int ghost_small_reduce_batch(const ghost_small_job* jobs, int n_jobs, void* stream) {
+  GB_REQUIRE(jobs != nullptr && n_jobs > 0, "ghost_small_reduce_batch: no jobs");
+  constexpr int kAtATime = 48;
+  ghost_pass_job batch[kAtATime];
+  for (int first = 0; first < n_jobs; first += kAtATime) {
+    const int n = n_jobs - first < kAtATime ? n_jobs - first : kAtATime;
+    for (int i = 0; i < n; ++i) {
+      const ghost_small_job& s = jobs[first + i];
+      GB_REQUIRE(s.X != nullptr, "ghost_small_reduce_batch: job %d has no input or no output", first + i);
+      batch[i] = ghost_pass_job{s.X, s.Xv, s.M, nullptr, s.sum_out, s.v_rank_pitch, s.n_train, s.n_val, s.F,
+                                s.v_per_rank, s.sum_is_f32, s.dot_scale, s.sum_scale};
+    }
+    const int rc = ghost_pass_reduce(batch, n, stream);
+    if (rc != GHOST_OK) return rc;
+  }
+  return GHOST_OK;
+}
+
+extern "C" int ghost_small_gram_f32(const float* X, int n_train, int n_val, int F, float scale,
+                                    float* M_out, void* stream) {
+  GB_REQUIRE(X && M_out, "ghost_small_gram_f32: null pointer");
+  GB_REQUIRE(n_train > 0, "No training samples to compute dot product, check batch sizes.");
+  GB_REQUIRE(n_val > 0 && F > 0, "ghost_small_gram_f32: bad dimensions");
+  const ghost_pass_job j = {X, nullptr, M_out, nullptr, nullptr, 0, n_train, n_val, F, 0, 1, scale, 1.f};
+  return ghost_pass_reduce(&j, 1, stream);
+}
+
+extern "C" int ghost_matrix_sum(const float* const* mats, int n_mats, int n_val, int n_train, float* total,
+                                float* vec, int* err_out, void* stream) {
+  const DeviceState* ds = device_state();
+  if (!ds) return GHOST_ERR_DEVICE;
+  GB_REQUIRE(mats && total && vec, "ghost_matrix_sum: null pointer");
+  GB_REQUIRE(n_mats > 0 && n_val > 0 && n_train > 0, "ghost_matrix_sum: empty dimension");
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  for (int first = 0; first < n_mats; first += kSumPointers) {
+    const int n = n_mats - first < kSumPointers ? n_mats - first : kSumPointers;
+    MatrixList list;
+    memcpy(list.m, mats + first, sizeof(float*) * n);
+    const bool last = first + n == n_mats;
+    matrix_sum_kernel<<<ceil_div(n_train, 32), 1024, 0, st>>>(list, n, n_val, n_train, first > 0 ? 1 : 0, total, vec,
+                                                              ds->err_word, last ? err_out : nullptr);
+    count_launch();
+    const int rc = post_launch("matrix_sum_kernel");
+    if (rc != GHOST_OK) return rc;
+  }
+  return GHOST_OK;
+}

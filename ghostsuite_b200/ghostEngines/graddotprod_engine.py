@@ -15,7 +15,7 @@ from typing import Optional
 import torch
 from torch import nn
 
-from .. import _lib
+from .. import _lib, ops
 from . import autograd_grad_sample_dotprod
 from . import supported_layers_grad_samplers_dotprod as _layers
 from . import transformers_support
@@ -81,7 +81,7 @@ class GradDotProdEngine:
     def _prepare_and_apply_train_grad(self):
         if self._grad_creation_locked:
             return
-        for name, param in self.module.named_parameters():
+        for name, param in _named_parameters(self.module):
             if not param.initially_requires_grad or "dummy_bias" in name:
                 continue
             if not hasattr(param, "train_grad"):
@@ -92,9 +92,8 @@ class GradDotProdEngine:
         self._lock_grad_creation()
 
     def _clear_train_grad(self):
-        for param in self.module.parameters():
-            if hasattr(param, "train_grad"):
-                del param.train_grad
+        for _, param in _named_parameters(self.module):
+            param.__dict__.pop("train_grad", None)
         self._unlock_grad_creation()
 
     def prepare_gradients(self):
@@ -114,45 +113,51 @@ class GradDotProdEngine:
         reduction instead of one in-place add per parameter."""
         _layers.finalize_pending_dots()
         vectors, matrices = [], []
-        for _, param in self.module.named_parameters():
-            if hasattr(param, "grad_dot_prod") and param.initially_requires_grad:
-                if param.grad_dot_prod.numel() > 0:
-                    m = getattr(param, "grad_dot_prod_matrix", None)
+        for _, param in _named_parameters(self.module):
+            own = param.__dict__
+            if "grad_dot_prod" in own and param.initially_requires_grad:
+                vector = own.pop("grad_dot_prod")
+                m = own.pop("grad_dot_prod_matrix", None)
+                if vector.numel() > 0:
                     if m is not None:
                         matrices.append(m)
                     else:
-                        vectors.append(param.grad_dot_prod)
-                delattr(param, "grad_dot_prod")
-                if hasattr(param, "grad_dot_prod_matrix"):
-                    delattr(param, "grad_dot_prod_matrix")
-        total = None
-        total_matrix = None
-        if matrices:
+                        vectors.append(vector)
+        total = total_matrix = packed = None
+        if matrices and not vectors and _summable(matrices):
+            packed = ops.matrix_sum(matrices)         # matrix, vector and error word in one buffer
+        elif matrices:
             total_matrix = torch.stack(matrices).sum(dim=0)
             total = total_matrix.sum(dim=0)
         if vectors:
             extra = torch.stack(vectors).sum(dim=0)
             total = extra if total is None else total + extra
             total_matrix = None          # a parameter without a matrix makes the summed matrix partial
-        if total is None:
+        if total is None and packed is None:
             warnings.warn("No gradient dot products computed for this iteration.")
             return
         # device -> host: all copies are queued first and waited for once (this is also the step's
         # sync point); the train batch is copied once when inputs and labels are one tensor
         x_cpu = _to_host_async(self.X_train)
         y_cpu = x_cpu if self.Y_train is self.X_train else _to_host_async(self.Y_train)
-        entry = {
-            "dot_product": _to_host_async(total),
-            "X_train": x_cpu,
-            "Y_train": y_cpu,
-            "iter_num": self.iter_num,
-            "batch_idx": self.batch_idx,
-        }
+        if packed is not None:
+            host = _to_host_async(packed)
+            torch.cuda.current_stream(packed.device).synchronize()
+            n_val, n_train = matrices[0].shape
+            if int(host[-1:].view(torch.int32)) != 0:
+                _lib.poll_kernel_error()
+            total_matrix, total = host[:n_val * n_train].view(n_val, n_train), host[n_val * n_train:-1]
+        else:
+            on_device = total
+            total = _to_host_async(total)
+            total_matrix = _to_host_async(total_matrix)
+            if on_device.is_cuda:
+                torch.cuda.current_stream(on_device.device).synchronize()
+                _lib.poll_kernel_error()
+        entry = {"dot_product": total, "X_train": x_cpu, "Y_train": y_cpu, "iter_num": self.iter_num,
+                 "batch_idx": self.batch_idx}
         if total_matrix is not None:
-            entry["dot_product_matrix"] = _to_host_async(total_matrix)
-        if total.is_cuda:
-            torch.cuda.current_stream(total.device).synchronize()
-            _lib.poll_kernel_error()
+            entry["dot_product_matrix"] = total_matrix
         self.dot_product_log.append(entry)
 
     def save_dot_product_log(self, iter_num: int):
@@ -173,6 +178,32 @@ class GradDotProdEngine:
         self.Y_train = Y_train
         self.iter_num = iter_num
         self.batch_idx = batch_idx
+
+
+def _named_parameters(module: nn.Module):
+    """``list(module.named_parameters())`` without its nested generators, which cost more than what a
+    step does with each parameter.  Walks the live tree, so later changes of the model count."""
+    out, seen = [], set()
+    stack = [("", module)]
+    while stack:
+        prefix, m = stack.pop()
+        if id(m) in seen:
+            continue
+        seen.add(id(m))
+        for name, p in m._parameters.items():
+            if p is not None and id(p) not in seen:
+                seen.add(id(p))
+                out.append((prefix + name, p))
+        if m._modules:
+            stack.extend([(f"{prefix}{name}.", c) for name, c in reversed(m._modules.items()) if c is not None])
+    return out
+
+
+def _summable(matrices) -> bool:
+    """Whether one launch can add these matrices up."""
+    first = matrices[0]
+    return first.is_cuda and all(m.shape == first.shape and m.dtype is torch.float32 and m.device == first.device
+                                 and m.is_contiguous() for m in matrices)
 
 
 def _to_host_async(data):

@@ -111,7 +111,8 @@ def _create_or_accumulate_train_grad(param: torch.Tensor, grad: torch.Tensor) ->
     """``param.train_grad`` is created on first use and added to afterwards (reference :44-69)."""
     assert grad.shape == param.shape, \
         f"Gradient shape ({grad.shape}) does not match parameter shape ({param.shape})"
-    grad = grad.detach()
+    if grad.requires_grad:
+        grad = grad.detach()
     if hasattr(param, "train_grad"):
         param.train_grad.add_(grad)
     else:
@@ -122,8 +123,7 @@ def _create_or_accumulate_train_grad(param: torch.Tensor, grad: torch.Tensor) ->
 
 # While a backward pass runs, two kinds of small work are not launched layer by layer but collected
 # and run when the pass ends (``finalize_pending_dots``, queued as an autograd callback by the hook
-# plumbing): the per-parameter [n_train] vectors (one stacked reduction per matrix shape), and the
-# bias / LayerNorm / RMS-norm terms' small reductions -- the [n_val, n_train] Gram of a layer's
+# plumbing): the per-parameter [n_train] vectors, and the bias / LayerNorm / RMS-norm terms' small reductions -- the [n_val, n_train] Gram of a layer's
 # per-sample vectors and the sum of its train rows -- which go out as ONE batched launch instead of
 # two launches per parameter.  Their output tensors exist from the moment the hook ran (the
 # parameter's ``grad_dot_prod_matrix`` is set at once) and are filled when the pass ends; train
@@ -184,9 +184,9 @@ def _train_grad_from_vectors(param: torch.Tensor, X: torch.Tensor, n_train: int,
 
 
 def finalize_pending_dots() -> None:
-    """Run the collected small reductions in one batched launch, hand their train gradients over,
-    then set ``param.grad_dot_prod = param.grad_dot_prod_matrix.sum(0)`` for every collected
-    parameter with one stack + one reduction per matrix shape.  A tied parameter keeps its last
+    """Run the collected small reductions and the sums over the validation samples
+    (``param.grad_dot_prod = param.grad_dot_prod_matrix.sum(0)`` for every collected parameter) in one
+    launch, and hand the train gradients among them over.  A tied parameter keeps its last
     matrix, as it does when every hook overwrites the attribute.  Safe to call when nothing is
     pending."""
     global _PENDING_DOTS, _PENDING_SMALL
@@ -196,24 +196,21 @@ def finalize_pending_dots() -> None:
         small, _PENDING_SMALL = _PENDING_SMALL, None
     if small:
         _exchange_pending_val_rows(small)        # validation rows of a batch split over ranks
-        ops.small_reduce_batch(small)
-        for job in small:
-            if job.get("param") is not None:
-                _create_or_accumulate_train_grad(job["param"], job["sum_out"].view_as(job["param"]))
-    if not pending:
-        return
-    last = {}
-    for param, M in pending:
-        last[id(param)] = (param, M)
-    groups = {}
-    for param, M in last.values():
-        groups.setdefault((tuple(M.shape), M.dtype, M.device), []).append((param, M))
-    for items in groups.values():
-        stacked = torch.stack([M for _, M in items])          # [P, n_val, n_train]
-        vectors = stacked.sum(dim=1)
-        for i, (param, M) in enumerate(items):
+    last = {id(param): (param, M) for param, M in pending or ()}
+    on_device = [item for item in last.values() if item[1].is_cuda]
+    if small or on_device:
+        vectors = ops.pass_reduce(small or [], [M for _, M in on_device])
+        for (param, M), vector in zip(on_device, vectors):
             if getattr(param, "grad_dot_prod_matrix", None) is M:
-                param.grad_dot_prod = vectors[i]
+                param.grad_dot_prod = vector
+        for job in small or ():
+            param = job.get("param")
+            if param is not None:
+                grad = job["sum_out"]
+                _create_or_accumulate_train_grad(param, grad if grad.shape == param.shape else grad.view_as(param))
+    for param, M in last.values():
+        if not M.is_cuda and getattr(param, "grad_dot_prod_matrix", None) is M:
+            param.grad_dot_prod = M.sum(dim=0)
 
 
 def _set_dot(param: torch.Tensor, M: torch.Tensor) -> None:

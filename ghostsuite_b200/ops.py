@@ -1,10 +1,10 @@
 """Kernel entry points on torch CUDA tensors.
 
-Each function validates shapes, hands raw device pointers to ``libghost_b200.so`` on torch's current
-stream, and returns torch tensors.  torch is used for memory and stream lookup only; the
-arithmetic runs in the library's kernels.  Scratch memory comes from a grow-only arena per
-(device, stream), so no allocation happens in steady state and nothing is freed while kernels that
-use it may still be queued.
+Each function hands its tensors to the native binding (``csrc/host/torch_ops.cpp``), which validates
+shapes, prepares operands, allocates outputs and calls ``libghost_b200.so`` on torch's current
+stream; a few rarely called ones do so here through ctypes.  The arithmetic runs in the library's
+kernels.  Scratch memory comes from a grow-only arena per (device, stream), so no allocation happens
+in steady state and nothing is freed while kernels that use it may still be queued.
 """
 from __future__ import annotations
 
@@ -17,8 +17,19 @@ from . import _lib
 _BF16 = torch.bfloat16
 _F32 = torch.float32
 
-_arenas: Dict[Tuple[int, int], torch.Tensor] = {}
+_native = _lib.native
 
+
+class _Arenas:
+    """The native binding's workspaces."""
+
+    @staticmethod
+    def clear() -> None:
+        """Give every workspace back to torch's allocator."""
+        _native().arena_clear()
+
+
+_arenas = _Arenas()
 
 _timing: Optional[list] = None
 
@@ -68,40 +79,13 @@ class _Timed:
 
 
 def _stream_ptr() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 def _require_cuda(*tensors: torch.Tensor) -> None:
     for t in tensors:
         if not t.is_cuda:
             raise RuntimeError("ghostsuite_b200 kernels need CUDA tensors (no CPU fallback exists)")
-
-
-class _Arena:
-    """Bump allocator over one cached uint8 tensor; reset at the start of every public op."""
-
-    def __init__(self, device: torch.device):
-        self.device = device
-        self.key = (device.index if device.index is not None else torch.cuda.current_device(),
-                    _stream_ptr())
-        self.requests = []
-
-    def plan(self, nbytes: int) -> int:
-        """Reserve nbytes (256-byte aligned); returns the offset."""
-        off = sum(self.requests)
-        self.requests.append((int(nbytes) + 255) // 256 * 256)
-        return off
-
-    def commit(self) -> int:
-        total = sum(self.requests) + 256
-        buf = _arenas.get(self.key)
-        if buf is None or buf.numel() < total:
-            # grow-only; the old buffer stays referenced by torch's caching allocator semantics
-            # (stream-ordered reuse), so queued kernels that still read it are safe
-            buf = torch.empty(max(total, 1 << 20), dtype=torch.uint8, device=self.device)
-            _arenas[self.key] = buf
-        base = buf.data_ptr()
-        return (base + 255) // 256 * 256
 
 
 def _dt_flag(t: torch.Tensor) -> int:
@@ -140,9 +124,17 @@ def _cast(lib, src: torch.Tensor, samples: int, T: int, dst_ptr: int, ld_dst: in
                                          k[0], k[1], k[2], 1 if row_stack else 0, _stream_ptr()))
 
 
-# hi/lo layouts of an fp32 operand pair so that  sum_k L[k] R[k] = hi*hi + lo*hi + hi*lo
-_SPLIT_LEFT = (0, 1, 0)
+#: hi/lo layout of the projection matrices of an fp32 model, the right operand of
+#: ``sum_k L[k] R[k] = hi*hi + lo*hi + hi*lo``
 _SPLIT_RIGHT = (0, 0, 1)
+
+
+def _cols(x: torch.Tensor) -> int:
+    return int(x.shape[-1])
+
+
+def _rows(x: torch.Tensor) -> int:
+    return x.numel() // max(1, int(x.shape[-1]))
 
 
 # --------------------------------------------------------------------------------------------
@@ -155,125 +147,38 @@ def gram_dot(A: torch.Tensor, G: torch.Tensor, n_val: int, round_mode: int = 0,
     bf16 inputs are used as they are (copied only if their feature size is not a multiple of 8);
     fp32 inputs are split into bf16 hi/lo parts so the result keeps fp32-class accuracy.
     """
-    lib = _lib.load()
-    _require_cuda(A, G)
-    A, G = _as3d(A), _as3d(G)
-    N, T, d = A.shape
-    p = G.shape[-1]
-    n_train = N - n_val
-    if n_train <= 0:
-        raise ValueError("No training samples to compute dot product, check batch sizes.")
-    if n_val <= 0:
-        raise ValueError("gram_dot needs at least one validation sample")
-    if G.shape[0] != N or G.shape[1] != T:
-        raise ValueError(f"activation {tuple(A.shape)} and out-grad {tuple(G.shape)} disagree")
-    M = torch.empty((n_val, n_train), dtype=_F32, device=A.device)
-    arena = _Arena(A.device)
-    ops = []
-    for x in (A, G):
-        f = x.shape[-1]
-        if x.dtype == _F32:
-            cp = _pad8(f)
-            off_t = arena.plan(n_train * T * 3 * cp * 2)
-            off_v = arena.plan(n_val * T * 3 * cp * 2)
-            ops.append(("split", x, cp, off_t, off_v))
-        elif _tma_ready(x):
-            ops.append(("asis", x, f, 0, 0))
-        else:
-            cp = _pad8(f)
-            off_t = arena.plan(N * T * cp * 2)
-            ops.append(("copy", x, cp, off_t, 0))
-    base = arena.commit()
+    if _timing is None:
+        return _native().gram_dot(A, G, n_val, round_mode, scale)
     # algorithmic work (the fp32 hi/lo split executes three times this on the tensor pipe)
-    timer = _Timed("ghost_gram_kernel", "tensor", 2.0 * n_train * T * n_val * T * (d + p),
-                   float(A.element_size()) * N * T * (d + p))
-    timer.__enter__()
-    ptrs = []
-    for kind, x, cp, off_t, off_v in ops:
-        if kind == "asis":
-            pt = x.data_ptr()
-            pv = pt + n_train * T * x.shape[-1] * 2
-            ptrs.append((pt, pv, x.shape[-1], x.shape[-1], x.shape[-1]))
-        elif kind == "copy":
-            _cast(lib, x, N, T, base + off_t, cp, cp, (0,), False)
-            pt = base + off_t
-            ptrs.append((pt, pt + n_train * T * cp * 2, cp, cp, cp))
-        else:
-            _cast(lib, x[:n_train], n_train, T, base + off_t, 3 * cp, cp, _SPLIT_LEFT, False)
-            _cast(lib, x[n_train:], n_val, T, base + off_v, 3 * cp, cp, _SPLIT_RIGHT, False)
-            ptrs.append((base + off_t, base + off_v, 3 * cp, 3 * cp, 3 * cp))
-    (at, av, ka, ld_at, ld_av), (gt, gv, kg, ld_gt, ld_gv) = ptrs
-    _lib.check(lib.ghost_gram_dot_bf16(at, av, gt, gv, n_train, n_val, T, ka, kg, ld_at, ld_av,
-                                       ld_gt, ld_gv, int(round_mode), float(scale), M.data_ptr(),
-                                       _stream_ptr()))
-    timer.__exit__(None, None, None)
-    return M
+    N, T = A.shape[0], max(1, _rows(A) // A.shape[0])
+    width = _cols(A) + _cols(G)
+    with _Timed("ghost_gram_kernel", "tensor", 2.0 * (N - n_val) * T * n_val * T * width,
+                float(A.element_size()) * N * T * width):
+        return _native().gram_dot(A, G, n_val, round_mode, scale)
 
 
 # --------------------------------------------------------------------------------------------
 # train-gradient recovery and the per-sample-gradient path
 # --------------------------------------------------------------------------------------------
-def _xty_operands(lib, arena: _Arena, X: torch.Tensor, Y: torch.Tensor, samples: int, T: int):
-    """Plan bf16 operands for the token-contracted GEMMs.  Returns a closure that materialises them
-    after ``arena.commit()`` and yields (x_ptr, y_ptr, ldx, ldy, T_eff)."""
-    split = X.dtype == _F32 or Y.dtype == _F32
-    plans = []
-    for x, kinds in ((X, _SPLIT_LEFT), (Y, _SPLIT_RIGHT)):
-        f = x.shape[-1]
-        cp = _pad8(f)
-        if split:
-            plans.append(("split", x, cp, arena.plan(samples * 3 * T * cp * 2), kinds))
-        elif _tma_ready(x):
-            plans.append(("asis", x, f, 0, kinds))
-        else:
-            plans.append(("copy", x, cp, arena.plan(samples * T * cp * 2), kinds))
-
-    def materialise(base: int):
-        out = []
-        for kind, x, cp, off, kinds in plans:
-            if kind == "asis":
-                out.append((x.data_ptr(), x.shape[-1]))
-            elif kind == "copy":
-                _cast(lib, x, samples, T, base + off, cp, cp, (0,), True)
-                out.append((base + off, cp))
-            else:
-                _cast(lib, x, samples, T, base + off, cp, cp, kinds, True)
-                out.append((base + off, cp))
-        return out[0][0], out[1][0], out[0][1], out[1][1], (3 * T if split else T)
-
-    return materialise, split
-
-
 def wgrad(X: torch.Tensor, Y: torch.Tensor, scale: float, out_dtype: torch.dtype,
           out: Optional[torch.Tensor] = None, accumulate: bool = False) -> torch.Tensor:
     """``scale * sum over all rows of X^T Y`` -> ``[X.shape[-1], Y.shape[-1]]`` in ``out_dtype``.
 
     ``X``/``Y`` are ``[samples, T, cols]`` (train samples only).
     """
-    lib = _lib.load()
-    _require_cuda(X, Y)
-    X, Y = _as3d(X), _as3d(Y)
-    S, T, m = X.shape
-    n = Y.shape[-1]
-    if Y.shape[0] != S or Y.shape[1] != T:
-        raise ValueError("wgrad operands disagree on the token layout")
-    if out is None:
-        out = torch.empty((m, n), dtype=out_dtype, device=X.device)
-        accumulate = False
-    arena = _Arena(X.device)
-    ws_bytes = int(lib.ghost_wgrad_workspace_bytes(m, n))
-    off_ws = arena.plan(ws_bytes)
-    mat, _ = _xty_operands(lib, arena, X, Y, S, T)
-    base = arena.commit()
-    with _Timed("xty_gemm_pair_kernel[wgrad]", "tensor", 2.0 * S * T * m * n, 2.0 * S * T * (m + n)):
-        xp, yp, ldx, ldy, T_eff = mat(base)
-        _lib.check(lib.ghost_wgrad_bf16(xp, yp, S * T_eff, m, n, ldx, ldy, float(scale),
-                                        1 if accumulate else 0, out.data_ptr(), _dt_flag(out),
-                                        base + off_ws, ws_bytes, _stream_ptr()))
-    return out
+    if out is None and out_dtype not in (_F32, _BF16):
+        raise ValueError(f"unsupported dtype {out_dtype}: the kernels take float32 and bfloat16")
+    if _timing is None:
+        return _native().wgrad(X, Y, scale, out_dtype is _F32, out, accumulate)
+    with _Timed("xty_gemm_pair_kernel[wgrad]", "tensor", 2.0 * _rows(X) * _cols(X) * _cols(Y),
+                2.0 * _rows(X) * (_cols(X) + _cols(Y))):
+        return _native().wgrad(X, Y, scale, out_dtype is _F32, out, accumulate)
 
 
 _PERSAMPLE_NAME = "xty_gemm_pair_kernel+tile_dot_mma_kernel[persample]"
+
+
+_COLSUM_FLAG = {None: 0, "X": 1, "Y": 2}
 
 
 def persample_dot(X: torch.Tensor, Y: torch.Tensor, n_val: int, dot_scale: float = 1.0,
@@ -287,46 +192,20 @@ def persample_dot(X: torch.Tensor, Y: torch.Tensor, n_val: int, dot_scale: float
     (float32) of that operand, taken inside the GEMM pass, or None when the operands are fp32 (their
     bf16 hi/lo split is what the kernel sees).
     """
-    lib = _lib.load()
-    _require_cuda(X, Y)
-    X, Y = _as3d(X), _as3d(Y)
-    N, T, m = X.shape
-    n = Y.shape[-1]
-    n_train = N - n_val
-    if n_train <= 0:
-        raise ValueError("No training samples to compute dot product, check batch sizes.")
-    if n_val <= 0:
-        raise ValueError("persample_dot needs at least one validation sample")
-    if Y.shape[0] != N or Y.shape[1] != T:
-        raise ValueError("persample_dot operands disagree on the token layout")
-    M = torch.empty((n_val, n_train), dtype=_F32, device=X.device)
-    grad = None
-    if want_grad:
-        grad = torch.empty((m, n), dtype=grad_dtype or X.dtype, device=X.device)
-    arena = _Arena(X.device)
-    mat, split = _xty_operands(lib, arena, X, Y, N, T)
-    v_f32 = 1 if split else 0
-    ws_bytes = int(lib.ghost_persample_workspace_bytes(n_train, n_val, m, n, v_f32))
-    off_ws = arena.plan(ws_bytes)
-    base = arena.commit()
-    if colsum_of not in (None, "X", "Y"):
+    if colsum_of not in _COLSUM_FLAG:
         raise ValueError("colsum_of must be None, 'X' or 'Y'")
-    colsums = None
-    cs_flag = 0
-    if colsum_of is not None and not split:
-        colsums = torch.empty((N, m if colsum_of == "X" else n), dtype=_F32, device=X.device)
-        cs_flag = 1 if colsum_of == "X" else 2
-    with _Timed(_PERSAMPLE_NAME, "tensor",
-                2.0 * N * T * m * n + 2.0 * n_val * n_train * m * n, 2.0 * N * T * (m + n)):
-        xp, yp, ldx, ldy, T_eff = mat(base)
-        _lib.check(lib.ghost_persample_dot_bf16(
-            xp, yp, n_train, n_val, T_eff, m, n, ldx, ldy, float(dot_scale), M.data_ptr(), v_f32,
-            grad.data_ptr() if want_grad else None, _dt_flag(grad) if want_grad else 0,
-            float(grad_scale), 0, cs_flag, colsums.data_ptr() if colsums is not None else None,
-            base + off_ws, ws_bytes, _stream_ptr()))
-    if colsum_of is None:
-        return M, grad
-    return M, grad, colsums
+    gdt = grad_dtype if grad_dtype is not None else (_BF16 if X.dtype is _BF16 else _F32)
+    if gdt is not _F32 and gdt is not _BF16:
+        raise ValueError(f"unsupported dtype {gdt}: the kernels take float32 and bfloat16")
+    args = (X, Y, n_val, dot_scale, want_grad, grad_scale, gdt is _F32, _COLSUM_FLAG[colsum_of])
+    if _timing is None:
+        res = _native().persample_dot(*args)
+    else:
+        m, n, rows, N = _cols(X), _cols(Y), _rows(X), X.shape[0]
+        with _Timed(_PERSAMPLE_NAME, "tensor", 2.0 * rows * m * n + 2.0 * n_val * (N - n_val) * m * n,
+                    2.0 * rows * (m + n)):
+            res = _native().persample_dot(*args)
+    return res if colsum_of is not None else res[:2]
 
 
 def persample_tiles(X: torch.Tensor, Y: torch.Tensor, sample0: int, samples: int,
@@ -467,14 +346,10 @@ def persample_dot_exchanged(X: torch.Tensor, Y: torch.Tensor, n_val_local: int, 
 # --------------------------------------------------------------------------------------------
 def colsum(G: torch.Tensor) -> torch.Tensor:
     """Per-sample column sums over tokens: ``[N, T, p] -> [N, p]`` float32."""
-    lib = _lib.load()
-    _require_cuda(G)
-    G = _as3d(G)
-    N, T, p = G.shape
-    out = torch.empty((N, p), dtype=_F32, device=G.device)
-    with _Timed("colsum_kernel", "hbm", 0.0, float(N) * T * p * G.element_size()):
-        _lib.check(lib.ghost_colsum(G.data_ptr(), _dt_flag(G), N, T, p, p, out.data_ptr(), _stream_ptr()))
-    return out
+    if _timing is None:
+        return _native().colsum(G)
+    with _Timed("colsum_kernel", "hbm", 0.0, float(G.numel()) * G.element_size()):
+        return _native().colsum(G)
 
 
 def small_gram(X: torch.Tensor, n_val: int, scale: float = 1.0) -> torch.Tensor:
@@ -510,7 +385,7 @@ def rows_sum(X: torch.Tensor, n_rows: int, scale: float, out_dtype: torch.dtype,
 
 
 def small_reduce_batch(jobs) -> None:
-    """Run many :func:`small_gram` / :func:`rows_sum` reductions in one launch (48 jobs per launch).
+    """Run many :func:`small_gram` / :func:`rows_sum` reductions in one launch per 48 of them.
     ``jobs``: dicts with ``X`` (contiguous float32 ``[n_train + n_val, F]``), ``n_train``, ``n_val`` and
     optionally ``M`` (float32 ``[n_val, n_train]`` output, with ``dot_scale``) and ``sum_out``
     (float32 / bfloat16 ``[F]`` output, with ``sum_scale``); the outputs are written in place.  A job
@@ -518,44 +393,29 @@ def small_reduce_batch(jobs) -> None:
     * F : ...]`` (row ``r * per_rank + i``; ``gathered`` is a contiguous float32 ``[ranks, pitch]`` tensor, the
     result of one all-gather that carried many jobs' validation rows) and only its train rows from
     ``X``."""
-    if not jobs:
-        return
-    lib = _lib.load()
-    arr = (_lib.SmallJob * len(jobs))()
-    nbytes = 0.0
-    for rec, job in zip(arr, jobs):
-        X = job["X"]
-        M, out = job.get("M"), job.get("sum_out")
-        _require_cuda(X)
-        if X.dtype != _F32 or X.dim() != 2 or not X.is_contiguous():
-            raise ValueError("small_reduce_batch takes contiguous float32 [N, F] tensors")
-        if M is not None and (M.dtype != _F32 or not M.is_contiguous()
-                              or M.numel() != job["n_val"] * job["n_train"]):
-            raise ValueError("small_reduce_batch: M must be a contiguous float32 [n_val, n_train] tensor")
-        if out is not None and (not out.is_contiguous() or out.numel() != X.shape[1]):
-            raise ValueError("small_reduce_batch: sum_out must be a contiguous [F] tensor")
-        rec.X = X.data_ptr()
-        rec.M = M.data_ptr() if M is not None else None
-        rec.sum_out = out.data_ptr() if out is not None else None
-        rec.n_train, rec.n_val, rec.F = int(job["n_train"]), int(job["n_val"]), int(X.shape[1])
-        rec.sum_is_f32 = _dt_flag(out) if out is not None else 1
-        rec.dot_scale = float(job.get("dot_scale", 1.0))
-        rec.sum_scale = float(job.get("sum_scale", 1.0))
-        xv = job.get("Xv")
-        if xv is not None:
-            gathered, offset, per_rank = xv
-            if gathered.dtype != _F32 or gathered.dim() != 2 or not gathered.is_contiguous() \
-                    or offset + per_rank * X.shape[1] > gathered.shape[1] \
-                    or gathered.shape[0] * per_rank != job["n_val"] or X.shape[0] < job["n_train"]:
-                raise ValueError("small_reduce_batch: bad layout of the separate validation rows")
-            rec.Xv = gathered.data_ptr() + 4 * int(offset)
-            rec.v_rank_pitch = int(gathered.shape[1])
-            rec.v_per_rank = int(per_rank)
-        else:
-            rec.Xv = None
-        nbytes += 4.0 * X.numel()
-    with _Timed("small_reduce_batch_kernel", "hbm", 0.0, nbytes):
-        _lib.check(lib.ghost_small_reduce_batch(arr, len(jobs), _stream_ptr()))
+    jobs = list(jobs)
+    for first in range(0, len(jobs), 48):
+        pass_reduce(jobs[first:first + 48], [])
+
+
+def pass_reduce(jobs: list, matrices: list) -> list:
+    """What is left to reduce when a backward pass ends, in one launch: the jobs of
+    :func:`small_reduce_batch`, and for every ``[n_val, n_train]`` float32 matrix its sum over the
+    validation samples (returned as a list of ``[n_train]`` tensors; a matrix may be one that a job
+    of the same call fills)."""
+    if _timing is None:
+        return _native().pass_reduce(jobs, matrices)
+    with _Timed("pass_reduce_kernel", "hbm", 0.0, 4.0 * sum(j["X"].numel() for j in jobs)):
+        return _native().pass_reduce(jobs, matrices)
+
+
+def matrix_sum(matrices: list) -> torch.Tensor:
+    """Sum of equal ``[n_val, n_train]`` float32 matrices as one flat float32 buffer: the matrix, its
+    column sums (``n_train`` values), and the device error word (the bits of an int32)."""
+    if _timing is None:
+        return _native().matrix_sum(matrices)
+    with _Timed("matrix_sum_kernel", "hbm", 0.0, 4.0 * len(matrices) * matrices[0].numel()):
+        return _native().matrix_sum(matrices)
 
 
 def layernorm_persample(A: torch.Tensor, G: torch.Tensor, eps: float, rms: bool = False
@@ -563,87 +423,34 @@ def layernorm_persample(A: torch.Tensor, G: torch.Tensor, eps: float, rms: bool 
     """Per-sample LayerNorm gamma/beta gradients ``([N, F], [N, F])`` float32 in one pass.  With
     ``rms=True`` the normalisation is RMS norm's (no centring); the second result is then just the
     token sum of the out-grad."""
-    lib = _lib.load()
-    _require_cuda(A, G)
-    if A.dtype != G.dtype:
-        common = torch.promote_types(A.dtype, G.dtype)
-        A, G = A.to(common), G.to(common)
-    A, G = _as3d(A), _as3d(G)
-    N, T, F = A.shape
-    if G.shape != A.shape:
-        raise ValueError("LayerNorm input and out-grad shapes differ")
-    gw = torch.empty((N, F), dtype=_F32, device=A.device)
-    gb = torch.empty((N, F), dtype=_F32, device=A.device)
-    arena = _Arena(A.device)
-    ws_bytes = int(lib.ghost_layernorm_workspace_bytes(N, T, F))
-    off = arena.plan(ws_bytes)
-    base = arena.commit()
-    with _Timed("layernorm_persample_kernel", "hbm", 0.0, 2.0 * N * T * F * A.element_size() + 8.0 * N * F):
-        fn = lib.ghost_rmsnorm_persample if rms else lib.ghost_layernorm_persample
-        _lib.check(fn(A.data_ptr(), G.data_ptr(), _dt_flag(A), N, T, F, float(eps), gw.data_ptr(),
-                      gb.data_ptr(), base + off, ws_bytes, _stream_ptr()))
-    return gw, gb
+    if _timing is None:
+        return _native().norm_persample(A, G, eps, rms)
+    with _Timed("layernorm_persample_kernel", "hbm", 0.0, 2.0 * A.numel() * A.element_size() + 8.0 * A.shape[0] * _cols(A)):
+        return _native().norm_persample(A, G, eps, rms)
 
 
 # --------------------------------------------------------------------------------------------
 # Embedding
 # --------------------------------------------------------------------------------------------
-def _ids2d(ids: torch.Tensor) -> torch.Tensor:
-    ids = ids.reshape(ids.shape[0], -1)
-    if ids.dtype != torch.int64:
-        ids = ids.long()
-    return ids.contiguous()
-
-
 def embedding_dot(ids: torch.Tensor, G: torch.Tensor, n_val: int, vocab: int,
                   scale: float = 1.0) -> torch.Tensor:
-    lib = _lib.load()
-    _require_cuda(ids, G)
-    ids = _ids2d(ids)
-    G = _as3d(G)
-    N, T, d = G.shape
-    if ids.shape[0] != N or ids.shape[1] != T:
-        raise ValueError("embedding ids and out-grad disagree on [batch, tokens]")
-    n_train = N - n_val
-    if n_train <= 0:
-        raise ValueError("No training samples to compute dot product, check batch sizes.")
-    M = torch.empty((n_val, n_train), dtype=_F32, device=G.device)
-    arena = _Arena(G.device)
-    ws_bytes = int(lib.ghost_embedding_dot_workspace_bytes_for(n_val, T, vocab, d))
-    off = arena.plan(ws_bytes)
-    base = arena.commit()
-    with _Timed("emb_dot_kernel", "hbm", 0.0, float(N) * T * d * G.element_size() + 8.0 * N * T):
-        _lib.check(lib.ghost_embedding_dot(ids.data_ptr(), G.data_ptr(), _dt_flag(G), n_train, n_val, T,
-                                           d, int(vocab), float(scale), M.data_ptr(), base + off,
-                                           ws_bytes, _stream_ptr()))
-    return M
+    if _timing is None:
+        return _native().embedding_dot(ids, G, n_val, vocab, scale)
+    with _Timed("emb_dot_kernel", "hbm", 0.0, float(G.numel()) * G.element_size() + 8.0 * ids.numel()):
+        return _native().embedding_dot(ids, G, n_val, vocab, scale)
 
 
 def embedding_wgrad(ids: torch.Tensor, G: torch.Tensor, n_train: int, vocab: int, pre_scale: float,
                     divisor: float, out: Optional[torch.Tensor] = None,
                     accumulate: bool = False) -> torch.Tensor:
     """Averaged train gradient of an embedding table ``[vocab, d]`` in the dtype of ``G``."""
-    lib = _lib.load()
-    _require_cuda(ids, G)
-    ids = _ids2d(ids)
-    G = _as3d(G)
-    N, T, d = G.shape
-    if out is None:
-        out = torch.empty((vocab, d), dtype=G.dtype, device=G.device)
-        accumulate = False
-    elif out.dtype != G.dtype:
-        raise ValueError("embedding_wgrad output must have the dtype of the out-grad")
-    arena = _Arena(G.device)
-    ws_bytes = int(lib.ghost_embedding_wgrad_workspace_bytes(n_train, T, vocab))
-    off = arena.plan(ws_bytes)
-    base = arena.commit()
+    args = (ids, G, n_train, vocab, pre_scale, divisor, out, accumulate)
+    if _timing is None:
+        return _native().embedding_wgrad(*args)
+    share = n_train / max(1, G.shape[0])
     with _Timed("emb_segsum_kernel", "hbm", 0.0,
-                (float(n_train) * T * d + float(vocab) * d) * G.element_size() + 8.0 * n_train * T):
-        _lib.check(lib.ghost_embedding_wgrad(ids.data_ptr(), G.data_ptr(), _dt_flag(G), n_train, T, d,
-                                             int(vocab), float(pre_scale), float(divisor),
-                                             1 if accumulate else 0, out.data_ptr(), base + off,
-                                             ws_bytes, _stream_ptr()))
-    return out
+                (share * G.numel() + float(vocab) * _cols(G)) * G.element_size() + 8.0 * share * ids.numel()):
+        return _native().embedding_wgrad(*args)
 
 
 # --------------------------------------------------------------------------------------------
@@ -668,51 +475,13 @@ def gradproj_dense(G: torch.Tensor, A: torch.Tensor, P_r: torch.Tensor, P_c: tor
     """``out[b] = scale * (G_b P_r^T)^T (A_b P_c^T)`` written into ``out`` (``[B, >= k_r*k_c]`` fp32,
     possibly a column slice of a wider row-major buffer).  ``P_r``/``P_c`` come from
     :func:`prepare_projection` (split layout iff the activations are fp32)."""
-    lib = _lib.load()
-    _require_cuda(G, A, P_r, P_c, out)
-    G, A = _as3d(G), _as3d(A)
-    B, T, n_r = G.shape
-    n_c = A.shape[-1]
-    if A.shape[0] != B or A.shape[1] != T:
-        raise RuntimeError("Batch size mismatch between activations and output gradients")
-    if out.dtype != _F32 or out.dim() != 2 or out.shape[0] != B or out.stride(1) != 1 \
-            or out.shape[1] < k_r * k_c:
-        raise ValueError("gradproj output must be a float32 [B, >= k_r*k_c] row-major view")
-    split = G.dtype == _F32 or A.dtype == _F32
-    arena = _Arena(G.device)
-    plans = []
-    for x in (G, A):
-        cp = _pad8(x.shape[-1])
-        if split:
-            plans.append(("split", x, cp, arena.plan(B * T * 3 * cp * 2)))
-        elif _tma_ready(x):
-            plans.append(("asis", x, x.shape[-1], 0))
-        else:
-            plans.append(("copy", x, cp, arena.plan(B * T * cp * 2)))
-    base = arena.commit()
-    timer = _Timed("gradproj_kernel", "hbm", 2.0 * B * T * (n_r * k_r + n_c * k_c + k_r * k_c),
-                   float(B) * T * (n_r + n_c) * G.element_size() + 2.0 * (k_r * n_r + k_c * n_c)
-                   + 4.0 * B * k_r * k_c)
-    timer.__enter__()
-    ptrs = []
-    for kind, x, cp, off in plans:
-        if kind == "asis":
-            ptrs.append((x.data_ptr(), cp, cp))
-        elif kind == "copy":
-            _cast(lib, x, B, T, base + off, cp, cp, (0,), False)
-            ptrs.append((base + off, cp, cp))
-        else:
-            _cast(lib, x, B, T, base + off, 3 * cp, cp, _SPLIT_LEFT, False)
-            ptrs.append((base + off, 3 * cp, 3 * cp))
-    (gp, kr_len, ldg), (ap, kc_len, lda) = ptrs
-    if P_r.shape[1] != kr_len or P_c.shape[1] != kc_len:
-        raise ValueError("projection matrices were prepared for a different dtype/feature size")
-    _lib.check(lib.ghost_gradproj_dense_bf16(gp, ap, B, T, kr_len, kc_len, ldg, lda, P_r.data_ptr(),
-                                             P_c.data_ptr(), int(k_r), int(k_c), P_r.shape[1],
-                                             P_c.shape[1], float(scale), out.data_ptr(),
-                                             out.stride(0), _stream_ptr()))
-    timer.__exit__(None, None, None)
-    return out
+    if _timing is None:
+        return _native().gradproj_dense(G, A, P_r, P_c, k_r, k_c, scale, out)
+    n_r, n_c = _cols(G), _cols(A)
+    with _Timed("gradproj_kernel", "hbm", 2.0 * _rows(G) * (n_r * k_r + n_c * k_c + k_r * k_c),
+                float(_rows(G)) * (n_r + n_c) * G.element_size() + 2.0 * (k_r * n_r + k_c * n_c)
+                + 4.0 * G.shape[0] * k_r * k_c):
+        return _native().gradproj_dense(G, A, P_r, P_c, k_r, k_c, scale, out)
 
 
 def prepare_embedding_projection(P_i: torch.Tensor) -> torch.Tensor:
@@ -729,41 +498,12 @@ def gradproj_embedding(ids: torch.Tensor, G: torch.Tensor, P_o_prepared: torch.T
     ``out`` when given: a ``[B, >= k_o*k_i]`` row-major view, e.g. a column slice of the engine's
     buffer).  ``P_o_prepared`` comes from :func:`prepare_projection` (split layout iff ``G`` is
     float32), ``P_i_t`` from :func:`prepare_embedding_projection`."""
-    lib = _lib.load()
-    _require_cuda(ids, G, P_o_prepared, P_i_t)
-    ids = _ids2d(ids)
-    G = _as3d(G)
-    B, T, d = G.shape
-    if ids.shape[0] != B or ids.shape[1] != T:
-        raise RuntimeError("Batch size mismatch between token ids and output gradients")
-    split = G.dtype == _F32
-    cp = _pad8(d)
-    if P_o_prepared.dtype != _BF16 or P_o_prepared.shape[0] != k_o or P_o_prepared.shape[1] != (3 if split else 1) * cp:
-        raise ValueError("P_o was prepared for a different dtype/feature size")
-    if P_i_t.dtype != _F32 or P_i_t.dim() != 2 or P_i_t.shape[1] != k_i or not P_i_t.is_contiguous():
-        raise ValueError("P_i must be passed as the contiguous float32 [vocab, k_i] transpose")
-    if out is None:
-        out = torch.empty((B, k_o * k_i), dtype=_F32, device=G.device)
-    elif out.dtype != _F32 or out.dim() != 2 or out.shape[0] != B or out.stride(1) != 1 or out.shape[1] < k_o * k_i:
-        raise ValueError("embedding projection output must be a float32 [B, >= k_o*k_i] row-major view")
-    with _Timed("gradproj_embedding_kernel", "hbm", 2.0 * B * T * (d * k_o + k_o * k_i),
-                float(B) * T * (d * G.element_size() + 8 + 4 * k_i) + 4.0 * B * k_o * k_i):
-        # _SPLIT_RIGHT lays a float32 matrix out as (hi, hi, lo): the residual part starts at 2 * cp.
-        # The kernel covers up to 64 x 64 of a sample's block per launch; larger projections go
-        # block by block into the zeroed output.
-        chunked = k_o > 64 or k_i > 64
-        if chunked:
-            out[:, :k_o * k_i].zero_()
-        ld_po = P_o_prepared.shape[1]
-        for o0 in range(0, k_o, 64):
-            for i0 in range(0, k_i, 64):
-                _lib.check(lib.ghost_gradproj_embedding(
-                    ids.data_ptr(), G.data_ptr(), _dt_flag(G), B, T, d, d,
-                    P_o_prepared.data_ptr() + o0 * ld_po * 2, ld_po, cp, 2 * cp if split else 0,
-                    P_i_t.data_ptr() + i0 * 4, k_i, P_i_t.shape[0], min(64, k_o - o0), min(64, k_i - i0),
-                    float(scale), 1 if chunked else 0, out.data_ptr() + (o0 * k_i + i0) * 4,
-                    out.stride(0), k_i, _stream_ptr()))
-    return out
+    if _timing is None:
+        return _native().gradproj_embedding(ids, G, P_o_prepared, P_i_t, k_o, k_i, scale, out)
+    rows, d = ids.numel(), _cols(G)
+    with _Timed("gradproj_embedding_kernel", "hbm", 2.0 * rows * (d * k_o + k_o * k_i),
+                float(rows) * (d * G.element_size() + 8 + 4 * k_i) + 4.0 * ids.shape[0] * k_o * k_i):
+        return _native().gradproj_embedding(ids, G, P_o_prepared, P_i_t, k_o, k_i, scale, out)
 
 
 #: largest block (rows of either operand) the similarity kernel is used for; beyond it the operands
@@ -774,27 +514,11 @@ SIMILARITY_KERNEL_MAX_ROWS = 128
 def projection_similarity(P1: torch.Tensor, P2: torch.Tensor, scale: float = 1.0) -> torch.Tensor:
     """``scale * P1 @ P2.T`` -> ``[n1, n2]`` float32 for two blocks of projection rows (float32 or
     bfloat16, same dtype, unit stride along the projection dimension)."""
-    lib = _lib.load()
-    _require_cuda(P1, P2)
-    if P1.dim() != 2 or P2.dim() != 2 or P1.shape[1] != P2.shape[1]:
-        raise ValueError("projection sets have different dimensions")
-    if P1.dtype != P2.dtype:
-        common = torch.promote_types(P1.dtype, P2.dtype)
-        P1, P2 = P1.to(common), P2.to(common)
-    if P1.dtype not in (_F32, _BF16):
-        P1, P2 = P1.float(), P2.float()
-    if P1.stride(1) != 1:
-        P1 = P1.contiguous()
-    if P2.stride(1) != 1:
-        P2 = P2.contiguous()
-    n1, D = P1.shape
-    n2 = P2.shape[0]
-    S = torch.empty((n1, n2), dtype=_F32, device=P1.device)
-    with _Timed("proj_similarity_kernel", "hbm", 2.0 * n1 * n2 * D, float(n1 + n2) * D * P1.element_size()):
-        _lib.check(lib.ghost_projection_similarity(P1.data_ptr(), P2.data_ptr(), _dt_flag(P1), n1, n2, D,
-                                                   P1.stride(0), P2.stride(0), float(scale), S.data_ptr(),
-                                                   S.stride(0), _stream_ptr()))
-    return S
+    if _timing is None:
+        return _native().projection_similarity(P1, P2, scale)
+    with _Timed("proj_similarity_kernel", "hbm", 2.0 * P1.shape[0] * P2.numel(),
+                float(P1.numel() + P2.numel()) * P1.element_size()):
+        return _native().projection_similarity(P1, P2, scale)
 
 
 def launch_count() -> int:

@@ -206,6 +206,31 @@ typedef struct ghost_small_job {
 } ghost_small_job;
 int ghost_small_reduce_batch(const ghost_small_job* jobs, int n_jobs, void* stream);
 
+/* All reductions that are left when a backward pass ends, in one launch (300 jobs per launch).  As
+ * ghost_small_job, and vec[b] = sum_v M[v, b] when vec is not NULL.  A job without X takes M as it is
+ * (a matrix some other call has filled on this stream) and only writes vec.  Adds to the lines above
+ * the per-parameter [n_train] vectors, which the reference forms by summing the validation batch
+ * first (ghostEngines/supported_layers_grad_samplers_dotprod.py:134, :143-146, :416-417). */
+typedef struct ghost_pass_job {
+  const float* X;
+  const float* Xv;
+  float* M;
+  float* vec;
+  void* sum_out;
+  long long v_rank_pitch;
+  int n_train, n_val, F;
+  int v_per_rank;
+  int sum_is_f32;
+  float dot_scale, sum_scale;
+} ghost_pass_job;
+int ghost_pass_reduce(const ghost_pass_job* jobs, int n_jobs, void* stream);
+/* total[v, b] = sum_i mats[i][v, b] over n_mats device matrices [n_val, n_train] (mats is a HOST array
+ * of device pointers) and vec[b] = sum_v total[v, b]; err_out, if not NULL, receives the device error
+ * word as ghost_poll_kernel_error would read it at this point of the stream.  Replaces the in-place
+ * add per parameter of ghostEngines/graddotprod_engine.py:195-262. */
+int ghost_matrix_sum(const float* const* mats, int n_mats, int n_val, int n_train, float* total, float* vec,
+                     int* err_out, void* stream);
+
 /* ---- Embedding -------------------------------------------------------------------------------- */
 /* M[v,b] = scale * sum_{t,s : ids_b[t] == ids_v[s]} <G_b[t], G_v[s]>.  ids: int64 [N, T]; G: [N, T, d].
  * Validation tokens are chained per id; a train token walks the chain of its id.  The workspace
