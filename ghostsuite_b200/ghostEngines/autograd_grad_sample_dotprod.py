@@ -54,18 +54,47 @@ def add_hooks(model: nn.Module, val_batch_size: int, loss_reduction: str = "mean
             _layers.maybe_register_rmsnorm(type(layer))
         if type(layer) in _supported_layers_dotprod and requires_grad(layer):
             layer.name = name
-            handles.append(layer.register_forward_hook(_capture_activations))
 
             def backward_hook(this_layer, grad_input, grad_output):
                 _prepare_sample_grad_or_dotprod(this_layer, grad_output, val_batch_size, loss_reduction)
                 _apply_train_grad(this_layer, val_batch_size)
                 return None
 
-            handles.append(layer.register_full_backward_hook(backward_hook))
+            handles.extend(register_hook_pair(layer, _capture_activations, backward_hook))
         elif not list(layer.children()) and requires_grad(layer):
             print(f"WARNING: Skipping atomic layer '{name}' of type {type(layer)} because it is not supported.")
 
     model.__dict__.setdefault("autograd_grad_sample_hooks", []).extend(handles)
+
+
+def register_hook_pair(layer: nn.Module, capture, backward_hook):
+    """Register ``capture(layer, inputs, outputs)`` on the forward pass and ``backward_hook(layer,
+    grad_input, (grad,))`` on the output's gradient; returns the removable handles.
+
+    The backward hooks read the output gradient only, so a hook on the output tensor serves them; a
+    module's full backward hook wraps input and output in two more autograd nodes per call (about
+    60 us of host time per layer and step) and hands over the same tensor later.  Embeddings keep the
+    module hook: their input has no gradient, in which case a module hook that a user registers
+    after this one fires at the output too, and would come before a hook on the tensor inside."""
+    if isinstance(layer, nn.Embedding):
+        return [layer.register_forward_hook(capture), layer.register_full_backward_hook(backward_hook)]
+
+    def forward_hook(layer, inputs, outputs):
+        out = outputs if torch.is_tensor(outputs) else next((o for o in outputs if torch.is_tensor(o)), None)
+        task = torch._C._current_graph_task_id()
+        if task != -1 and layer.__dict__.get("_ghost_done_in") == task:
+            # non-re-entrant activation checkpointing runs this layer again inside the backward pass that
+            # has already called its hook: nothing would consume the input kept here
+            return
+        capture(layer, inputs, outputs)
+        if out is not None and out.requires_grad and torch.is_grad_enabled():
+            def on_gradient(grad):
+                layer.__dict__["_ghost_done_in"] = torch._C._current_graph_task_id()
+                backward_hook(layer, None, (grad,))
+
+            out.register_hook(on_gradient)
+
+    return [layer.register_forward_hook(forward_hook)]
 
 
 def remove_hooks(model: nn.Module):
@@ -83,28 +112,31 @@ def _capture_activations(layer: nn.Module, inputs: Tuple, outputs: Tuple):
     backward hook and keeps nothing alive."""
     if not torch.is_grad_enabled():
         return
-    layer.activations = inputs[0].detach()
+    layer.__dict__["activations"] = inputs[0].detach()
 
 
 def _prepare_sample_grad_or_dotprod(layer: nn.Module, grad_output: Tuple[torch.Tensor],
                                     val_batch_size: int, loss_reduction: str = "mean"):
     """Backward hook, part 1: dot products of this layer's parameters (reference :97-137)."""
-    backprops = grad_output[0].detach()
-    if not hasattr(layer, "activations"):
-        layer.activations = None
-    A = layer.activations
+    backprops = grad_output[0]
+    if backprops.requires_grad:
+        backprops = backprops.detach()
+    # instance attributes are written to the dictionary: nn.Module.__setattr__ searches the parameter,
+    # buffer and module tables for each of these names first
+    own = layer.__dict__
+    A = own.setdefault("activations", None)
     dot_fn, _ = _supported_layers_dotprod[type(layer)]
 
     # mixed precision: bring both operands to the common floating type (ids stay integer)
-    if A is not None and A.is_floating_point() and A.dtype != backprops.dtype:
+    if A is not None and A.dtype is not backprops.dtype and A.is_floating_point():
         common = torch.promote_types(A.dtype, backprops.dtype)
         A = A.to(common)
         backprops = backprops.to(common)
-        layer.activations = A
+        own["activations"] = A
 
     # 'mean' losses carry a 1/batch factor (the batch this process ran); the train-gradient kernels
     # undo it in their epilogue
-    layer._ghost_backprop_scale = float(backprops.shape[0]) if loss_reduction == "mean" else 1.0
+    own["_ghost_backprop_scale"] = float(backprops.shape[0]) if loss_reduction == "mean" else 1.0
     # the per-parameter [n_train] vectors are reduced in one batched op when the backward pass ends
     if _layers.begin_deferred_dots():
         try:
@@ -115,26 +147,30 @@ def _prepare_sample_grad_or_dotprod(layer: nn.Module, grad_output: Tuple[torch.T
     if exchange is not None and VALIDATION_GATHER is not None and A is not None and A.is_floating_point():
         # validation batch split over ranks: the ranks exchange validation gradients where the layer
         # type allows it ...
-        layer._ghost_val_batch = val_batch_size
+        own["_ghost_val_batch"] = val_batch_size
         try:
             handled = _layers.dot_product_with_exchange(layer, A, backprops, val_batch_size, exchange)
         except BaseException:
             _layers.finalize_pending_dots()
             raise
         if handled:
-            layer.backprops = backprops
+            own["backprops"] = backprops
             return
     if VALIDATION_GATHER is not None and A is not None:
         # ... and validation operands everywhere else
         A, backprops, val_batch_size = VALIDATION_GATHER(layer, A, backprops, val_batch_size)
-        layer.activations = A
-    layer._ghost_val_batch = val_batch_size
+        own["activations"] = A
+    own["_ghost_val_batch"] = val_batch_size
     try:
         dot_fn(layer, A, backprops, val_batch_size=val_batch_size)
     except BaseException:
         _layers.finalize_pending_dots()          # a failed pass may never reach its callback
         raise
-    layer.backprops = backprops
+    own["backprops"] = backprops
+
+
+_PASS_ATTRIBUTES = ("activations", "backprops", "_ghost_backprop_scale", "_ghost_val_batch", "_ghost_colsums",
+                    "_ghost_cached_train_grad", "_ghost_ln_cache", "_ghost_conv_tokens")
 
 
 def _apply_train_grad(layer: nn.Module, val_batch_size: int, loss_reduction: str = "mean"):
@@ -162,9 +198,9 @@ def _apply_train_grad(layer: nn.Module, val_batch_size: int, loss_reduction: str
             if bias is not None and getattr(bias, "initially_requires_grad", bias.requires_grad):
                 _train_grad_bias_from_layer(layer, val_batch_size, loss_reduction)
     finally:
-        for attr in ("activations", "backprops", "_ghost_backprop_scale", "_ghost_val_batch", "_ghost_colsums",
-                     "_ghost_cached_train_grad", "_ghost_ln_cache", "_ghost_conv_tokens"):
-            layer.__dict__.pop(attr, None)
+        own = layer.__dict__
+        for attr in _PASS_ATTRIBUTES:
+            own.pop(attr, None)
 
 
 def _train_grad_bias_from_layer(layer: nn.Module, val_batch_size: int, loss_reduction: str) -> None:

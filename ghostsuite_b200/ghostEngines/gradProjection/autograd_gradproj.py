@@ -16,6 +16,7 @@ import torch
 import torch.nn as nn
 
 from ... import ops
+from ..autograd_grad_sample_dotprod import register_hook_pair
 
 
 def _flatten_tokens(x: torch.Tensor) -> torch.Tensor:
@@ -37,8 +38,7 @@ class GradProjHooks:
         self.P_o = P_o            # [k_o, n_o] float32
         self.layer_name = layer_name
         self.layer_type = layer_type
-        self._handle_forward = None
-        self._handle_backward = None
+        self._handles = []
         self._kernel_P = {}       # split flag -> (P_i, P_o) in the kernel's bf16 layout
         self._P_i_t = None        # embedding layers: float32 [vocab, k_i] transpose of P_i
         self._out_fn: Optional[Callable[[int], torch.Tensor]] = None
@@ -63,7 +63,7 @@ class GradProjHooks:
         # the backward hook, so only it keeps the input alive.
         if not torch.is_grad_enabled():
             return
-        module._ghost_A_raw = inputs[0].detach()
+        module.__dict__["_ghost_A_raw"] = inputs[0].detach()
 
     def backward_hook_compute_proj(self, module: nn.Module, grad_input, grad_output) -> None:
         A_raw = getattr(module, "_ghost_A_raw", None)
@@ -127,15 +127,12 @@ class GradProjHooks:
         module._ghost_grad_proj = out.view(batch, k_o, k_i)
 
     def attach(self, module: nn.Module) -> None:
-        self._handle_forward = module.register_forward_hook(self.forward_hook_store_inputs)
-        self._handle_backward = module.register_full_backward_hook(self.backward_hook_compute_proj)
+        self._handles = register_hook_pair(module, self.forward_hook_store_inputs, self.backward_hook_compute_proj)
 
     def detach(self) -> None:
-        for attr in ("_handle_forward", "_handle_backward"):
-            handle = getattr(self, attr)
-            if handle is not None:
-                handle.remove()
-                setattr(self, attr, None)
+        for handle in self._handles:
+            handle.remove()
+        self._handles = []
 
 
 def create_projection_hooks(module: nn.Module, layer_name: str, P_i: torch.Tensor,
