@@ -127,6 +127,15 @@ def native():
     return _native
 
 
+def named_parameters(module) -> list:
+    """``list(module.named_parameters())`` for a module on a GPU without its nested generators, which
+    cost more than what a step does with each parameter.  Walks the live tree, so later changes of
+    the model count; without the binding (CPU-only use of the engines' bookkeeping) torch's own."""
+    if not os.path.exists(BINDING_PATH):
+        return list(module.named_parameters())
+    return native().named_parameters(module)
+
+
 def last_error() -> str:
     return load().ghost_last_error().decode("utf-8", "replace")
 

@@ -15,6 +15,7 @@
 #include <algorithm>
 #include <map>
 #include <mutex>
+#include <set>
 #include <stdexcept>
 #include <string>
 #include <utility>
@@ -347,31 +348,93 @@ PyObject* py_colsum(PyObject*, PyObject* const* a, Py_ssize_t n) {
   });
 }
 
+struct Norm { Tensor gw, gb; };
+
+Norm norm_persample(const Launch& L, Tensor A, Tensor G, float eps, bool rms) {
+  if (A.scalar_type() != G.scalar_type()) {
+    const at::ScalarType common = c10::promoteTypes(A.scalar_type(), G.scalar_type());
+    A = A.to(common);
+    G = G.to(common);
+  }
+  A = as3d(A);
+  G = as3d(G);
+  const long long N = A.size(0), T = A.size(1), F = A.size(2);
+  if (G.sizes() != A.sizes()) invalid("LayerNorm input and out-grad shapes differ");
+  Tensor both = empty({2, N, F}, A, at::kFloat);
+  Norm r{both.select(0, 0), both.select(0, 1)};
+  Workspace ws;
+  const long long ws_bytes = ghost_layernorm_workspace_bytes(static_cast<int>(N), T, static_cast<int>(F));
+  const long long off = ws.plan(ws_bytes);
+  char* base = ws.commit(L, A);
+  auto fn = rms ? ghost_rmsnorm_persample : ghost_layernorm_persample;
+  check(fn(A.data_ptr(), G.data_ptr(), is_f32(A), static_cast<int>(N), T, static_cast<int>(F), eps, r.gw.data_ptr<float>(),
+           r.gb.data_ptr<float>(), base + off, ws_bytes, L.st()));
+  return r;
+}
+
 // (A, G, eps, rms) -> (gw, gb)
 PyObject* py_norm_persample(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return guarded([&]() -> PyObject* {
     need(n, 4, "norm_persample");
-    Tensor A = cuda_tensor(a[0]), G = cuda_tensor(a[1]);
+    const Tensor &A = cuda_tensor(a[0]), &G = cuda_tensor(a[1]);
     Launch L(A);
-    if (A.scalar_type() != G.scalar_type()) {
-      const at::ScalarType common = c10::promoteTypes(A.scalar_type(), G.scalar_type());
-      A = A.to(common);
-      G = G.to(common);
+    Norm r = norm_persample(L, A, G, real(a[2]), integer(a[3]) != 0);
+    return Py_BuildValue("(NN)", wrap(r.gw), wrap(r.gb));
+  });
+}
+
+// ---- whole hooks ----------------------------------------------------------------------------------------
+// dtype argument of an optional output: -1 = not wanted, 0 = bfloat16, 1 = float32
+Tensor optional_empty(at::IntArrayRef size, const Tensor& like, long long dt) {
+  return dt < 0 ? Tensor() : empty(size, like, dt ? at::kFloat : at::kBFloat16);
+}
+
+// Everything the backward hook of a Linear / Conv1D layer computes or allocates:
+// (A, B, n_val, weight_is_in_by_out, use_gram, weight grad dtype, grad scale, has_bias, bias grad dtype)
+// -> (M, weight grad, column sums of B, unfilled bias matrix, unfilled bias grad), None where not wanted.
+PyObject* py_dense_hook(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    need(n, 9, "dense_hook");
+    const Tensor &A0 = cuda_tensor(a[0]), &B0 = cuda_tensor(a[1]);
+    Launch L(A0);
+    const Tensor A = as3d(A0), B = as3d(B0);
+    const long long n_val = integer(a[2]), N = A.size(0), n_train = N - n_val, p = B.size(2);
+    const bool in_by_out = integer(a[3]) != 0, gram = integer(a[4]) != 0, bias = integer(a[7]) != 0;
+    const long long gdt = integer(a[5]), bdt = integer(a[8]);
+    const float scale = real(a[6]);
+    const Tensor &X = in_by_out ? A : B, &Y = in_by_out ? B : A;
+    Tensor M, grad, sums;
+    if (gram) {
+      M = gram_dot(L, A, B, n_val, 0, 1.f);
+      grad = optional_empty({X.size(2), Y.size(2)}, X, gdt);
+      if (grad.defined()) wgrad(L, X, Y, n_train, scale, grad, false);
+    } else {
+      PerSample r = persample_dot(L, X, Y, n_val, 1.f, gdt >= 0, scale, gdt == 0 ? at::kBFloat16 : at::kFloat,
+                                  !bias ? 0 : in_by_out ? 2 : 1);
+      M = r.M;
+      grad = r.grad;
+      sums = r.colsums;
     }
-    A = as3d(A);
-    G = as3d(G);
-    const long long N = A.size(0), T = A.size(1), F = A.size(2);
-    if (G.sizes() != A.sizes()) invalid("LayerNorm input and out-grad shapes differ");
-    Tensor both = empty({2, N, F}, A, at::kFloat);
-    Tensor gw = both.select(0, 0), gb = both.select(0, 1);
-    Workspace ws;
-    const long long ws_bytes = ghost_layernorm_workspace_bytes(static_cast<int>(N), T, static_cast<int>(F));
-    const long long off = ws.plan(ws_bytes);
-    char* base = ws.commit(L, A);
-    auto fn = integer(a[3]) ? ghost_rmsnorm_persample : ghost_layernorm_persample;
-    check(fn(A.data_ptr(), G.data_ptr(), is_f32(A), static_cast<int>(N), T, static_cast<int>(F), real(a[2]),
-             gw.data_ptr<float>(), gb.data_ptr<float>(), base + off, ws_bytes, L.st()));
-    return Py_BuildValue("(NN)", wrap(gw), wrap(gb));
+    if (bias && !sums.defined()) sums = colsum(L, B);
+    Tensor Mb = bias ? empty({n_val, n_train}, A, at::kFloat) : Tensor();
+    Tensor sb = optional_empty({p}, A, bias ? bdt : -1);
+    return Py_BuildValue("(NNNNN)", wrap(M), wrap_or_none(grad), wrap_or_none(sums), wrap_or_none(Mb), wrap_or_none(sb));
+  });
+}
+
+// The same for a LayerNorm / RMS norm layer: (A, G, eps, rms, n_val, weight grad dtype, bias grad dtype) ->
+// (gw, gb, unfilled weight matrix, bias matrix, weight grad, bias grad); no bias: dtype -1, two Nones
+PyObject* py_norm_hook(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    need(n, 7, "norm_hook");
+    const Tensor &A = cuda_tensor(a[0]), &G = cuda_tensor(a[1]);
+    Launch L(A);
+    Norm r = norm_persample(L, A, G, real(a[2]), integer(a[3]) != 0);
+    const long long n_val = integer(a[4]), n_train = r.gw.size(0) - n_val, F = r.gw.size(1), bdt = integer(a[6]);
+    check_split(n_train, n_val, "norm_hook");
+    Tensor M = empty({bdt >= 0 ? 2 : 1, n_val, n_train}, A, at::kFloat);
+    return Py_BuildValue("(NNNNNN)", wrap(r.gw), wrap(r.gb), wrap(M.select(0, 0)), wrap_or_none(bdt >= 0 ? M.select(0, 1) : Tensor()),
+                         wrap_or_none(optional_empty({F}, A, integer(a[5]))), wrap_or_none(optional_empty({F}, A, bdt)));
   });
 }
 
@@ -675,6 +738,52 @@ PyObject* py_matrix_sum(PyObject*, PyObject* const* a, Py_ssize_t n) {
   });
 }
 
+// (module) -> [(qualified name, parameter)] as module.named_parameters() gives them: every parameter once,
+// modules in depth-first order.  The engines walk the model three times a step.
+void walk_parameters(PyObject* module, const std::string& prefix, std::set<PyObject*>& seen, PyObject* out) {
+  if (!seen.insert(module).second) return;
+  PyObject* dict = PyObject_GetAttrString(module, "__dict__");
+  if (!dict) { PyErr_Clear(); return; }
+  PyObject *key, *value;
+  Py_ssize_t pos = 0;
+  PyObject* params = PyDict_Check(dict) ? PyDict_GetItemString(dict, "_parameters") : nullptr;
+  if (params && PyDict_Check(params)) {
+    while (PyDict_Next(params, &pos, &key, &value)) {
+      if (value == Py_None || !seen.insert(value).second) continue;
+      const char* name = PyUnicode_AsUTF8(key);
+      PyObject* entry = Py_BuildValue("(sO)", (prefix + (name ? name : "")).c_str(), value);
+      if (!entry || PyList_Append(out, entry) != 0) { Py_XDECREF(entry); Py_DECREF(dict); throw std::bad_alloc(); }
+      Py_DECREF(entry);
+    }
+  }
+  PyObject* modules = PyDict_Check(dict) ? PyDict_GetItemString(dict, "_modules") : nullptr;
+  if (modules && PyDict_Check(modules)) {
+    pos = 0;
+    while (PyDict_Next(modules, &pos, &key, &value)) {
+      if (value == Py_None) continue;
+      const char* name = PyUnicode_AsUTF8(key);
+      walk_parameters(value, prefix + (name ? name : "") + ".", seen, out);
+    }
+  }
+  Py_DECREF(dict);
+}
+
+PyObject* py_named_parameters(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    need(n, 1, "named_parameters");
+    PyObject* out = PyList_New(0);
+    if (!out) throw std::bad_alloc();
+    std::set<PyObject*> seen;
+    try {
+      walk_parameters(a[0], "", seen, out);
+    } catch (...) {
+      Py_DECREF(out);
+      throw;
+    }
+    return out;
+  });
+}
+
 PyObject* py_set_kernel_error(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (n == 1) {
     Py_XDECREF(g_kernel_error);
@@ -692,6 +801,8 @@ PyMethodDef kMethods[] = {
     GB_METHOD(embedding_wgrad),   GB_METHOD(gradproj_dense),
     GB_METHOD(gradproj_embedding), GB_METHOD(projection_similarity),
     GB_METHOD(pass_reduce),       GB_METHOD(matrix_sum),
+    GB_METHOD(dense_hook),        GB_METHOD(norm_hook),
+    GB_METHOD(named_parameters),
     GB_METHOD(arena_clear),       GB_METHOD(set_kernel_error),
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_ghost_torch", nullptr, -1, kMethods, nullptr, nullptr, nullptr, nullptr};

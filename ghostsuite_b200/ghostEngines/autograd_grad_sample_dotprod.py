@@ -170,7 +170,7 @@ def _prepare_sample_grad_or_dotprod(layer: nn.Module, grad_output: Tuple[torch.T
 
 
 _PASS_ATTRIBUTES = ("activations", "backprops", "_ghost_backprop_scale", "_ghost_val_batch", "_ghost_colsums",
-                    "_ghost_cached_train_grad", "_ghost_ln_cache", "_ghost_conv_tokens")
+                    "_ghost_bias_grad", "_ghost_norm_grads", "_ghost_cached_train_grad", "_ghost_ln_cache", "_ghost_conv_tokens")
 
 
 def _apply_train_grad(layer: nn.Module, val_batch_size: int, loss_reduction: str = "mean"):
@@ -219,7 +219,7 @@ def _train_grad_bias_from_layer(layer: nn.Module, val_batch_size: int, loss_redu
     if loss_reduction == "mean":
         scale /= n_train
     out_dtype = layer.bias.dtype if layer.bias.dtype in (torch.float32, torch.bfloat16) else torch.float32
-    _layers._train_grad_from_vectors(layer.bias, colsums, n_train, scale, out_dtype)
+    _layers._train_grad_from_vectors(layer.bias, colsums, n_train, scale, out_dtype, layer.__dict__.get("_ghost_bias_grad"))
 
 
 def _compute_train_grad_bias(B: torch.Tensor, val_batch_size: int, loss_reduction: str = "mean") -> torch.Tensor:

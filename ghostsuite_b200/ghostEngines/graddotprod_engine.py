@@ -81,7 +81,7 @@ class GradDotProdEngine:
     def _prepare_and_apply_train_grad(self):
         if self._grad_creation_locked:
             return
-        for name, param in _named_parameters(self.module):
+        for name, param in _lib.named_parameters(self.module):
             if not param.initially_requires_grad or "dummy_bias" in name:
                 continue
             if not hasattr(param, "train_grad"):
@@ -92,7 +92,7 @@ class GradDotProdEngine:
         self._lock_grad_creation()
 
     def _clear_train_grad(self):
-        for _, param in _named_parameters(self.module):
+        for _, param in _lib.named_parameters(self.module):
             param.__dict__.pop("train_grad", None)
         self._unlock_grad_creation()
 
@@ -113,7 +113,7 @@ class GradDotProdEngine:
         reduction instead of one in-place add per parameter."""
         _layers.finalize_pending_dots()
         vectors, matrices = [], []
-        for _, param in _named_parameters(self.module):
+        for _, param in _lib.named_parameters(self.module):
             own = param.__dict__
             if "grad_dot_prod" in own and param.initially_requires_grad:
                 vector = own.pop("grad_dot_prod")
@@ -178,25 +178,6 @@ class GradDotProdEngine:
         self.Y_train = Y_train
         self.iter_num = iter_num
         self.batch_idx = batch_idx
-
-
-def _named_parameters(module: nn.Module):
-    """``list(module.named_parameters())`` without its nested generators, which cost more than what a
-    step does with each parameter.  Walks the live tree, so later changes of the model count."""
-    out, seen = [], set()
-    stack = [("", module)]
-    while stack:
-        prefix, m = stack.pop()
-        if id(m) in seen:
-            continue
-        seen.add(id(m))
-        for name, p in m._parameters.items():
-            if p is not None and id(p) not in seen:
-                seen.add(id(p))
-                out.append((prefix + name, p))
-        if m._modules:
-            stack.extend([(f"{prefix}{name}.", c) for name, c in reversed(m._modules.items()) if c is not None])
-    return out
 
 
 def _summable(matrices) -> bool:

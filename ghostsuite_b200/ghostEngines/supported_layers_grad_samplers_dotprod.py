@@ -54,6 +54,9 @@ _DOT_PRODUCTS_PER_S = 6.0e12
 _TILE_BYTES_PER_S = 5.0e12
 
 
+_GRAD_TYPES = (torch.float32, torch.bfloat16)
+
+
 def _token_count(A: torch.Tensor) -> int:
     if A.dim() <= 2:
         return 1
@@ -160,26 +163,29 @@ def _small_job_for(X: torch.Tensor, n_train: int, n_val: int, want: str):
         return job
 
 
-def _gram_of_vectors(X: torch.Tensor, val_batch_size: int) -> torch.Tensor:
+def _gram_of_vectors(X: torch.Tensor, val_batch_size: int, M: torch.Tensor = None) -> torch.Tensor:
     """``[n_val, n_train]`` Gram of per-sample vectors: at once, or as part of the batched launch at
-    the end of the backward pass in flight."""
+    the end of the backward pass in flight (into ``M`` when given)."""
     n_train = X.shape[0] - val_batch_size
     job = _small_job_for(X, n_train, val_batch_size, "M")
     if job is None:
         return ops.small_gram(X, val_batch_size)
-    M = torch.empty((val_batch_size, n_train), dtype=torch.float32, device=X.device)
+    if M is None:
+        M = torch.empty((val_batch_size, n_train), dtype=torch.float32, device=X.device)
     job["M"], job["n_val"], job["dot_scale"] = M, val_batch_size, 1.0
     return M
 
 
 def _train_grad_from_vectors(param: torch.Tensor, X: torch.Tensor, n_train: int, scale: float,
-                             out_dtype: torch.dtype) -> None:
-    """``param.train_grad (+)= scale * X[:n_train].sum(0)``: at once, or from the batched launch."""
+                             out_dtype: torch.dtype, out: torch.Tensor = None) -> None:
+    """``param.train_grad (+)= scale * X[:n_train].sum(0)``: at once, or from the batched launch (into
+    ``out`` when given)."""
     job = _small_job_for(X, n_train, X.shape[0] - n_train, "sum_out")
     if job is None:
         _create_or_accumulate_train_grad(param, ops.rows_sum(X, n_train, scale, out_dtype))
         return
-    out = torch.empty((X.shape[1],), dtype=out_dtype, device=X.device)
+    if out is None:
+        out = torch.empty((X.shape[1],), dtype=out_dtype, device=X.device)
     job["sum_out"], job["sum_scale"], job["param"] = out, scale, param
 
 
@@ -400,6 +406,9 @@ def _dense_dot_product(layer: nn.Module, A: torch.Tensor, B: torch.Tensor, val_b
     A = A.detach()
     B = B.detach()
     _should_use_ghost_computation(layer, A, B, val_batch_size=val_batch_size)
+    if val_batch_size > 0 and "_ghost_backprop_scale" in layer.__dict__:
+        _dense_hook(layer, A, B, val_batch_size, n_train, weight_is_in_by_out)
+        return
     colsums = None
     if val_batch_size > 0:
         if layer.use_ghost_computation:
@@ -423,6 +432,30 @@ def _dense_dot_product(layer: nn.Module, A: torch.Tensor, B: torch.Tensor, val_b
         _set_dot(layer.weight, M)
     if getattr(layer, "bias", None) is not None and val_batch_size > 0:
         _bias_terms(layer, B, val_batch_size, colsums)
+
+
+def _dense_hook(layer: nn.Module, A: torch.Tensor, B: torch.Tensor, n_val: int, n_train: int,
+                weight_is_in_by_out: bool) -> None:
+    """``_dense_dot_product`` inside a backward hook: the train gradients are asked for right after the
+    dot products, so one native call computes both and allocates what the end of the pass fills."""
+    own = layer.__dict__
+    weight = layer.weight
+    bias = getattr(layer, "bias", None)
+    scale = own["_ghost_backprop_scale"] / n_train
+    bias_dtype = None
+    if bias is not None and getattr(bias, "initially_requires_grad", bias.requires_grad):
+        bias_dtype = torch.bfloat16 if bias.dtype is torch.bfloat16 else torch.float32
+    M, grad, colsums, bias_M, bias_grad = ops.dense_hook(
+        A, B, n_val, weight_is_in_by_out, layer.use_ghost_computation,
+        _grad_dtype(weight, A) if getattr(weight, "initially_requires_grad", True) else None, scale,
+        bias is not None, bias_dtype)
+    if grad is not None:
+        own["_ghost_cached_train_grad"] = (A.data_ptr(), B.data_ptr(), A.size(0), grad)
+    _set_dot(weight, M)
+    if bias is not None:
+        _set_dot(bias, _gram_of_vectors(colsums, n_val, bias_M))
+        own["_ghost_colsums"] = colsums
+        own["_ghost_bias_grad"] = bias_grad
 
 
 def _dense_train_grad(layer: nn.Module, A: torch.Tensor, B: torch.Tensor, val_batch_size: int,
@@ -506,10 +539,34 @@ def _layernorm_vectors(layer: nn.LayerNorm, A: torch.Tensor, B: torch.Tensor):
     return gw, gb
 
 
+def _norm_hook(layer: nn.Module, A: torch.Tensor, B: torch.Tensor, n_val: int, eps: float, rms: bool) -> bool:
+    """The dot products of a norm layer inside a backward hook, whose train gradients are asked for
+    right after: one native call for the vectors and every output.  False when the layer is called
+    on its own, or has parameters of a type the batched launch does not write."""
+    own = layer.__dict__
+    weight, bias = layer.weight, getattr(layer, "bias", None)
+    if "_ghost_backprop_scale" not in own or "_ghost_ln_cache" in own or n_val <= 0 or not A.is_cuda \
+            or weight.dtype not in _GRAD_TYPES or not (bias is None or bias.dtype in _GRAD_TYPES):
+        return False
+    if not rms and len(layer.normalized_shape) != 1:
+        return False
+    gw, gb, Mw, Mb, sw, sb = ops.norm_hook(A, B, eps, rms, n_val, weight.dtype,
+                                           bias.dtype if bias is not None else None)
+    key = (A.data_ptr(), B.data_ptr(), A.size(0))
+    own["_ghost_ln_cache"] = (key, gw) if rms else (key, gw, gb)
+    own["_ghost_norm_grads"] = (sw, sb)
+    _set_dot(weight, _gram_of_vectors(gw, n_val, Mw))
+    if bias is not None:
+        _set_dot(bias, _gram_of_vectors(gb, n_val, Mb))
+    return True
+
+
 def _compute_layernorm_dot_product(layer: nn.LayerNorm, A: torch.Tensor, B: torch.Tensor,
                                    val_batch_size: int):
     """nn.LayerNorm: gamma and beta dot products from one pass over A and B (reference :242-300)."""
     if A.size(0) - val_batch_size <= 0:
+        return
+    if _norm_hook(layer, A, B, val_batch_size, layer.eps, False):
         return
     gw, gb = _layernorm_vectors(layer, A, B)
     _set_dot(layer.weight, _gram_of_vectors(gw, val_batch_size))
@@ -526,9 +583,10 @@ def _compute_layernorm_train_grad(layer: nn.LayerNorm, A: torch.Tensor, B: torch
     gw, gb = _layernorm_vectors(layer, A, B)
     layer.__dict__.pop("_ghost_ln_cache", None)
     scale = _backprop_scale(layer) / n_train
-    _train_grad_from_vectors(layer.weight, gw, n_train, scale, layer.weight.dtype)
+    sw, sb = layer.__dict__.pop("_ghost_norm_grads", (None, None))
+    _train_grad_from_vectors(layer.weight, gw, n_train, scale, layer.weight.dtype, sw)
     if layer.bias is not None:
-        _train_grad_from_vectors(layer.bias, gb, n_train, scale, layer.bias.dtype)
+        _train_grad_from_vectors(layer.bias, gb, n_train, scale, layer.bias.dtype, sb)
     return None
 
 
@@ -560,6 +618,8 @@ def _compute_rmsnorm_dot_product(layer: nn.Module, A: torch.Tensor, B: torch.Ten
     """RMS norm: weight dot products from one pass over A and B."""
     if A.size(0) - val_batch_size <= 0:
         return
+    if getattr(layer, "bias", None) is None and _norm_hook(layer, A, B, val_batch_size, _rmsnorm_eps(layer, A), True):
+        return
     _set_dot(layer.weight, _gram_of_vectors(_rmsnorm_vectors(layer, A, B), val_batch_size))
 
 
@@ -572,7 +632,8 @@ def _compute_rmsnorm_train_grad(layer: nn.Module, A: torch.Tensor, B: torch.Tens
     gw = _rmsnorm_vectors(layer, A, B)
     layer.__dict__.pop("_ghost_ln_cache", None)
     scale = _backprop_scale(layer) / n_train
-    _train_grad_from_vectors(layer.weight, gw, n_train, scale, layer.weight.dtype)
+    sw, _ = layer.__dict__.pop("_ghost_norm_grads", (None, None))
+    _train_grad_from_vectors(layer.weight, gw, n_train, scale, layer.weight.dtype, sw)
     return None
 
 

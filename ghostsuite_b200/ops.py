@@ -208,6 +208,31 @@ def persample_dot(X: torch.Tensor, Y: torch.Tensor, n_val: int, dot_scale: float
     return res if colsum_of is not None else res[:2]
 
 
+def _dtype_code(dt: Optional[torch.dtype]) -> int:
+    return -1 if dt is None else (1 if dt is _F32 else 0)
+
+
+def dense_hook(A: torch.Tensor, B: torch.Tensor, n_val: int, weight_is_in_by_out: bool, use_gram: bool,
+               grad_dtype: Optional[torch.dtype], grad_scale: float, has_bias: bool,
+               bias_grad_dtype: Optional[torch.dtype]):
+    """All that the backward hook of a Linear / Conv1D layer needs, in one native call: ``(M, weight
+    gradient, column sums of B, bias matrix, bias gradient)``, None where not wanted (a dtype of None,
+    no bias).  The last two are allocated only: they are filled by the launch that ends the backward
+    pass (:func:`pass_reduce`)."""
+    args = (A, B, n_val, weight_is_in_by_out, use_gram, _dtype_code(grad_dtype), grad_scale, has_bias,
+            _dtype_code(bias_grad_dtype))
+    if _timing is None:
+        return _native().dense_hook(*args)
+    d, p, rows, N = _cols(A), _cols(B), _rows(A), A.shape[0]
+    if use_gram:
+        T = rows // N
+        name, flops = "ghost_gram_kernel+xty_gemm_pair_kernel", 2.0 * (N - n_val) * T * (n_val * T * (d + p) + d * p)
+    else:
+        name, flops = _PERSAMPLE_NAME, 2.0 * rows * d * p + 2.0 * n_val * (N - n_val) * d * p
+    with _Timed(name, "tensor", flops, 2.0 * rows * (d + p)):
+        return _native().dense_hook(*args)
+
+
 def persample_tiles(X: torch.Tensor, Y: torch.Tensor, sample0: int, samples: int,
                     colsum_of: Optional[str] = None, colsums: Optional[torch.Tensor] = None) -> torch.Tensor:
     """First pass of the per-sample path alone: the bf16 tiles ``X_s^T Y_s`` of samples
@@ -427,6 +452,17 @@ def layernorm_persample(A: torch.Tensor, G: torch.Tensor, eps: float, rms: bool 
         return _native().norm_persample(A, G, eps, rms)
     with _Timed("layernorm_persample_kernel", "hbm", 0.0, 2.0 * A.numel() * A.element_size() + 8.0 * A.shape[0] * _cols(A)):
         return _native().norm_persample(A, G, eps, rms)
+
+
+def norm_hook(A: torch.Tensor, G: torch.Tensor, eps: float, rms: bool, n_val: int, weight_dtype: torch.dtype,
+              bias_dtype: Optional[torch.dtype]):
+    """:func:`layernorm_persample` plus what the launch that ends the backward pass fills:
+    ``(gw, gb, weight matrix, bias matrix, weight gradient, bias gradient)``; no bias: a dtype of None."""
+    args = (A, G, eps, rms, n_val, _dtype_code(weight_dtype), _dtype_code(bias_dtype))
+    if _timing is None:
+        return _native().norm_hook(*args)
+    with _Timed("layernorm_persample_kernel", "hbm", 0.0, 2.0 * A.numel() * A.element_size() + 8.0 * A.shape[0] * _cols(A)):
+        return _native().norm_hook(*args)
 
 
 # --------------------------------------------------------------------------------------------
