@@ -1,0 +1,280 @@
+// Linear / Conv1D layers with few token rows: dot-product matrix, train gradient and per-sample column
+// sums in ONE launch, float32 arithmetic on the CUDA cores straight from the operands.
+//
+// The tensor-core paths need bf16 operands (two to six conversion launches for float32 layers), zeroed
+// outputs, a GEMM whose grid is a handful of tiles, and a scaling pass: eight to twelve launches whose
+// fixed costs are ten times the arithmetic when a layer has tens of rows.  Here the blocks of one grid
+// share out the three results; nothing is converted, zeroed or written twice.  Layer 1024 -> 1024,
+// 64 + 16 samples of one token, float32: 11 launches, 93 us of GPU time before, one of 7 us now.
+#include "common.cuh"
+
+namespace gb {
+
+struct SmallDense {
+  const void *A, *B;                    // [N, T, d], [N, T, p]
+  int n_train, n_val, T, d, p;
+  int in_by_out;                        // weight [d, p] instead of [p, d]
+  float* M;                             // [n_val, n_train]
+  void* grad;                           // null: not wanted
+  int grad_f32;
+  float grad_scale;
+  float* colsums;                       // [N, p]; null: not wanted
+  // blocks [0, gram_blocks): pairs of sample groups; then wgrad_blocks tiles of 64 x 64; then column sums
+  int sv, sb, groups_b, gram_blocks;    // samples of a group (validation, train)
+  int tiles_n, wgrad_blocks, col_blocks;
+};
+
+__device__ __forceinline__ float sd_f32(float v) { return v; }
+__device__ __forceinline__ float sd_f32(__nv_bfloat16 v) { return __bfloat162float(v); }
+
+// four consecutive elements, zero beyond `left`; VEC: row starts are aligned and `left` is a multiple of four
+template <typename E, bool VEC>
+__device__ __forceinline__ float4 sd_load4(const E* p, int left) {
+  if constexpr (VEC) {
+    if (left <= 0) return make_float4(0.f, 0.f, 0.f, 0.f);
+    if constexpr (sizeof(E) == 4) {
+      return __ldg(reinterpret_cast<const float4*>(p));
+    } else {
+      const uint2 w = __ldg(reinterpret_cast<const uint2*>(p));
+      return make_float4(__uint_as_float(w.x << 16), __uint_as_float(w.x & 0xffff0000u), __uint_as_float(w.y << 16),
+                         __uint_as_float(w.y & 0xffff0000u));
+    }
+  } else {
+    return make_float4(left > 0 ? sd_f32(p[0]) : 0.f, left > 1 ? sd_f32(p[1]) : 0.f, left > 2 ? sd_f32(p[2]) : 0.f,
+                       left > 3 ? sd_f32(p[3]) : 0.f);
+  }
+}
+
+static constexpr int kSdV = 8, kSdB = 4;   // validation x train rows of a Gram tile
+
+// The 8 x 4 products of one tile over columns of X [.., K]: eight warps take 128-column units in turn, a
+// lane four columns of all twelve rows, so every row is read with full lines and once.  A butterfly
+// that halves the number of values with the distance leaves entry `lane` of the tile in every lane.
+template <typename E, bool VEC>
+__device__ __forceinline__ float sd_gram(const E* X, int K, long long row_v, int rows_v, long long row_b, int rows_b, int warp, int lane) {
+  float acc[kSdV * kSdB];
+#pragma unroll
+  for (int e = 0; e < kSdV * kSdB; ++e) acc[e] = 0.f;
+  for (int k0 = warp * 128; k0 < K; k0 += 1024) {
+    const int k = k0 + lane * 4;
+    float4 v[kSdV], b[kSdB];
+#pragma unroll
+    for (int i = 0; i < kSdV; ++i) v[i] = sd_load4<E, VEC>(X + (row_v + (i < rows_v ? i : 0)) * K + k, K - k);
+#pragma unroll
+    for (int j = 0; j < kSdB; ++j) b[j] = sd_load4<E, VEC>(X + (row_b + (j < rows_b ? j : 0)) * K + k, K - k);
+#pragma unroll
+    for (int i = 0; i < kSdV; ++i)
+#pragma unroll
+      for (int j = 0; j < kSdB; ++j) {
+        float& s = acc[i * kSdB + j];
+        s = fmaf(v[i].x, b[j].x, s); s = fmaf(v[i].y, b[j].y, s); s = fmaf(v[i].z, b[j].z, s); s = fmaf(v[i].w, b[j].w, s);
+      }
+  }
+#pragma unroll
+  for (int o = 16; o >= 1; o >>= 1) {
+    const bool up = (lane & o) != 0;
+#pragma unroll
+    for (int e = 0; e < o; ++e) {
+      const float send = up ? acc[e] : acc[e + o], keep = up ? acc[e + o] : acc[e];
+      acc[e] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+    }
+  }
+  return acc[0];
+}
+
+template <typename E, bool VEC>
+__global__ void __launch_bounds__(256, 2) dense_small_kernel(const SmallDense q) {
+  __shared__ __align__(16) float sm[2 * 2 * 16 * 64];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const E* A = static_cast<const E*>(q.A);
+  const E* B = static_cast<const E*>(q.B);
+  int blk = blockIdx.x;
+
+  if (blk < q.gram_blocks) {
+    float* red = sm;                     // [operand][warp][32 entries]
+    const int v0 = blk / q.groups_b * q.sv, b0 = blk % q.groups_b * q.sb;
+    const int nv = min(q.sv, q.n_val - v0), nb = min(q.sb, q.n_train - b0);
+    const long long first_v = static_cast<long long>(q.n_train + v0) * q.T, first_b = static_cast<long long>(b0) * q.T;
+    const int rows_v = nv * q.T, rows_b = nb * q.T;      // T == 1, or one sample per side, or a few short ones
+    float total = 0.f;                   // warp 0: T == 1: entry `lane`; else thread's pair (see below)
+    for (int i0 = 0; i0 < rows_v; i0 += kSdV)
+      for (int j0 = 0; j0 < rows_b; j0 += kSdB) {
+        const int rv = min(kSdV, rows_v - i0), rb = min(kSdB, rows_b - j0);
+        red[warp * 32 + lane] = sd_gram<E, VEC>(A, q.d, first_v + i0, rv, first_b + j0, rb, warp, lane);
+        red[256 + warp * 32 + lane] = sd_gram<E, VEC>(B, q.p, first_v + i0, rv, first_b + j0, rb, warp, lane);
+        __syncthreads();
+        if (warp == 0) {
+          float sa = 0.f, sg = 0.f;
+#pragma unroll
+          for (int w = 0; w < 8; ++w) { sa += red[w * 32 + lane]; sg += red[256 + w * 32 + lane]; }
+          const int i = lane / kSdB, j = lane % kSdB;
+          const float prod = i < rv && j < rb ? sa * sg : 0.f;
+          if (q.T == 1) {
+            total = prod;                // groups are tile-sized: one tile
+          } else {                       // pairs (v, b) of the group sum their entries of this tile
+            const int mine_v = i0 + i < rows_v ? (i0 + i) / q.T : -1, mine_b = j0 + j < rows_b ? (j0 + j) / q.T : -1;
+            for (int pr = 0; pr < nv * nb; ++pr) {
+              float s = mine_v == pr / nb && mine_b == pr % nb ? prod : 0.f;
+#pragma unroll
+              for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+              if (lane == pr) total += s;
+            }
+          }
+        }
+        __syncthreads();
+      }
+    if (warp == 0) {
+      const int i = q.T == 1 ? lane / kSdB : lane / nb, j = q.T == 1 ? lane % kSdB : lane % nb;
+      if (i < nv && j < nb) q.M[static_cast<long long>(v0 + i) * q.n_train + b0 + j] = total;
+    }
+    return;
+  }
+  blk -= q.gram_blocks;
+
+  if (blk < q.wgrad_blocks) {            // 64 x 64 outputs, 16 rows per stage, the next stage's loads in flight
+    const E* X = q.in_by_out ? A : B;
+    const E* Y = q.in_by_out ? B : A;
+    const int m = q.in_by_out ? q.d : q.p, n = q.in_by_out ? q.p : q.d;
+    const int m0 = blk / q.tiles_n * 64, n0 = blk % q.tiles_n * 64;
+    const int rows = q.n_train * q.T;
+    float (*xs)[16][64] = reinterpret_cast<float (*)[16][64]>(sm);
+    float (*ys)[16][64] = reinterpret_cast<float (*)[16][64]>(sm + 2 * 16 * 64);
+    const int lr = threadIdx.x >> 4, lc = (threadIdx.x & 15) * 4;
+    const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
+    float acc[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+    auto fetch = [&](int r0, float4& x, float4& y) {
+      const int r = r0 + lr;
+      const bool in = r < rows;
+      x = sd_load4<E, VEC>(X + static_cast<long long>(in ? r : 0) * m + m0 + lc, in ? m - m0 - lc : 0);
+      y = sd_load4<E, VEC>(Y + static_cast<long long>(in ? r : 0) * n + n0 + lc, in ? n - n0 - lc : 0);
+    };
+    float4 x, y;
+    fetch(0, x, y);
+    *reinterpret_cast<float4*>(&xs[0][lr][lc]) = x;
+    *reinterpret_cast<float4*>(&ys[0][lr][lc]) = y;
+    __syncthreads();
+    int buf = 0;
+    for (int r0 = 0; r0 < rows; r0 += 16, buf ^= 1) {
+      const bool more = r0 + 16 < rows;
+      if (more) fetch(r0 + 16, x, y);
+#pragma unroll
+      for (int k = 0; k < 16; ++k) {
+        const float4 a = *reinterpret_cast<const float4*>(&xs[buf][k][ty * 4]);
+        const float4 b = *reinterpret_cast<const float4*>(&ys[buf][k][tx * 4]);
+        const float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
+      }
+      if (more) {
+        *reinterpret_cast<float4*>(&xs[buf ^ 1][lr][lc]) = x;
+        *reinterpret_cast<float4*>(&ys[buf ^ 1][lr][lc]) = y;
+      }
+      __syncthreads();
+    }
+    const bool quad = (n & 3) == 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int r = m0 + ty * 4 + i, c = n0 + tx * 4;
+      if (r >= m || c >= n) continue;
+      const long long at = static_cast<long long>(r) * n + c;
+      float o[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) o[j] = acc[i][j] * q.grad_scale;
+      if (q.grad_f32) {
+        float* g = static_cast<float*>(q.grad) + at;
+        if (quad) *reinterpret_cast<float4*>(g) = make_float4(o[0], o[1], o[2], o[3]);
+        else
+#pragma unroll
+          for (int j = 0; j < 4; ++j) if (c + j < n) g[j] = o[j];
+      } else {
+        __nv_bfloat16* g = static_cast<__nv_bfloat16*>(q.grad) + at;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) if (c + j < n) g[j] = __float2bfloat16_rn(o[j]);
+      }
+    }
+    return;
+  }
+  blk -= q.wgrad_blocks;
+
+  const int blocks_c = (q.p + 1023) / 1024;
+  const int s = blk / blocks_c, c = blk % blocks_c * 1024 + threadIdx.x * 4;
+  if (c >= q.p) return;
+  float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+  const E* row = B + static_cast<long long>(s) * q.T * q.p + c;
+#pragma unroll 4
+  for (int t = 0; t < q.T; ++t) {
+    const float4 x = sd_load4<E, VEC>(row + static_cast<long long>(t) * q.p, q.p - c);
+    sum.x += x.x; sum.y += x.y; sum.z += x.z; sum.w += x.w;
+  }
+  float* o = q.colsums + static_cast<long long>(s) * q.p + c;
+  o[0] = sum.x;
+  if (c + 1 < q.p) o[1] = sum.y;
+  if (c + 2 < q.p) o[2] = sum.z;
+  if (c + 3 < q.p) o[3] = sum.w;
+}
+
+}  // namespace gb
+
+using namespace gb;
+
+// The line between this kernel and the tensor-core paths.  Pairs x features is the traffic of the Gram part
+// (about one byte of L2 reads each; 2e7 take 5 us), rows x d x p the multiply-adds of the train
+// gradient (about 12e12 a second here).  Beyond these the fixed costs it avoids -- some 40 us of
+// launches for float32 operands, 20 us for bf16 -- no longer pay for slower arithmetic.  A pair of
+// samples is one block, which walks its token tiles in turn (1.5 us each): at most eight of them.
+extern "C" int ghost_dense_small_fits(int is_f32, int n_train, int n_val, long long T, int d, int p) {
+  const double pairs = static_cast<double>(n_train) * T * n_val * T;
+  const double macs = static_cast<double>(n_train) * T * d * p;
+  const double rows = static_cast<double>(n_train + n_val) * T;
+  return T <= 16 && pairs * (d + p) <= 2e7 && macs <= (is_f32 ? 3e8 : 6e7) && rows * p <= 1e8 ? 1 : 0;
+}
+
+extern "C" int ghost_dense_small(const void* A, const void* B, int is_f32, int n_train, int n_val, long long T, int d,
+                                 int p, int in_by_out, float* M_out, void* grad_out, int grad_is_f32, float grad_scale,
+                                 float* colsum_out, void* stream) {
+  const DeviceState* ds = device_state();
+  if (!ds) return GHOST_ERR_DEVICE;
+  GB_REQUIRE(A && B && M_out, "ghost_dense_small: null pointer");
+  GB_REQUIRE(n_train > 0, "No training samples to compute dot product, check batch sizes.");
+  GB_REQUIRE(n_val > 0 && T > 0 && d > 0 && p > 0, "ghost_dense_small: empty dimension");
+  GB_REQUIRE(ghost_dense_small_fits(is_f32, n_train, n_val, T, d, p), "ghost_dense_small: beyond the sizes this kernel is for");
+  SmallDense q = {};
+  q.A = A; q.B = B;
+  q.n_train = n_train; q.n_val = n_val; q.T = static_cast<int>(T); q.d = d; q.p = p;
+  q.in_by_out = in_by_out;
+  q.M = M_out;
+  q.grad = grad_out; q.grad_f32 = grad_is_f32; q.grad_scale = grad_scale;
+  q.colsums = colsum_out;
+  // groups of whole samples: a tile's worth of one-token samples, fewer longer ones, at least one
+  q.sv = T >= kSdV ? 1 : static_cast<int>(kSdV / T);
+  q.sb = T >= kSdB ? 1 : static_cast<int>(kSdB / T);
+  q.groups_b = ceil_div(n_train, q.sb);
+  const long long gram = static_cast<long long>(ceil_div(n_val, q.sv)) * q.groups_b;
+  const int m = in_by_out ? d : p, n = in_by_out ? p : d;
+  q.tiles_n = ceil_div(n, 64);
+  const long long wgrad = grad_out ? static_cast<long long>(ceil_div(m, 64)) * q.tiles_n : 0;
+  const long long col = colsum_out ? static_cast<long long>(n_train + n_val) * ceil_div(p, 1024) : 0;
+  GB_REQUIRE(gram + wgrad + col < (1ll << 31), "ghost_dense_small: too many blocks");
+  q.gram_blocks = static_cast<int>(gram);
+  q.wgrad_blocks = static_cast<int>(wgrad);
+  q.col_blocks = static_cast<int>(col);
+  const uintptr_t align = is_f32 ? 15 : 7;
+  const bool vec = d % 4 == 0 && p % 4 == 0 && (reinterpret_cast<uintptr_t>(A) & align) == 0 && (reinterpret_cast<uintptr_t>(B) & align) == 0;
+  const unsigned grid = static_cast<unsigned>(gram + wgrad + col);
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (is_f32) {
+    if (vec) dense_small_kernel<float, true><<<grid, 256, 0, st>>>(q);
+    else dense_small_kernel<float, false><<<grid, 256, 0, st>>>(q);
+  } else {
+    if (vec) dense_small_kernel<__nv_bfloat16, true><<<grid, 256, 0, st>>>(q);
+    else dense_small_kernel<__nv_bfloat16, false><<<grid, 256, 0, st>>>(q);
+  }
+  count_launch();
+  return post_launch("dense_small_kernel");
+}

@@ -390,11 +390,11 @@ Tensor optional_empty(at::IntArrayRef size, const Tensor& like, long long dt) {
 }
 
 // Everything the backward hook of a Linear / Conv1D layer computes or allocates:
-// (A, B, n_val, weight_is_in_by_out, use_gram, weight grad dtype, grad scale, has_bias, bias grad dtype)
+// (A, B, n_val, weight_is_in_by_out, use_gram, weight grad dtype, grad scale, has_bias, bias grad dtype, any_path)
 // -> (M, weight grad, column sums of B, unfilled bias matrix, unfilled bias grad), None where not wanted.
 PyObject* py_dense_hook(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return guarded([&]() -> PyObject* {
-    need(n, 9, "dense_hook");
+    need(n, 10, "dense_hook");
     const Tensor &A0 = cuda_tensor(a[0]), &B0 = cuda_tensor(a[1]);
     Launch L(A0);
     const Tensor A = as3d(A0), B = as3d(B0);
@@ -404,7 +404,19 @@ PyObject* py_dense_hook(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const float scale = real(a[6]);
     const Tensor &X = in_by_out ? A : B, &Y = in_by_out ? B : A;
     Tensor M, grad, sums;
-    if (gram) {
+    const int dI = static_cast<int>(A.size(2)), pI = static_cast<int>(p);
+    check_split(n_train, n_val, "dense_hook");
+    if (B.size(0) != N || B.size(1) != A.size(1)) invalid("activation and out-grad disagree on [batch, tokens]");
+    if (integer(a[9]) && A.scalar_type() == B.scalar_type() &&
+        ghost_dense_small_fits(is_f32(A), static_cast<int>(n_train), static_cast<int>(n_val), A.size(1), dI, pI)) {
+      M = empty({n_val, n_train}, A, at::kFloat);
+      grad = optional_empty({X.size(2), Y.size(2)}, X, gdt);
+      const bool copy = bias && !(A.size(1) == 1 && is_f32(B));    // one float32 token: its rows are the sums
+      if (bias) sums = copy ? empty({N, p}, A, at::kFloat) : B.view({N, p});
+      check(ghost_dense_small(A.data_ptr(), B.data_ptr(), is_f32(A), static_cast<int>(n_train), static_cast<int>(n_val),
+                              A.size(1), dI, pI, in_by_out ? 1 : 0, M.data_ptr<float>(), grad.defined() ? grad.data_ptr() : nullptr,
+                              grad.defined() ? is_f32(grad) : 0, scale, copy ? sums.data_ptr<float>() : nullptr, L.st()));
+    } else if (gram) {
       M = gram_dot(L, A, B, n_val, 0, 1.f);
       grad = optional_empty({X.size(2), Y.size(2)}, X, gdt);
       if (grad.defined()) wgrad(L, X, Y, n_train, scale, grad, false);

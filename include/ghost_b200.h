@@ -149,6 +149,17 @@ int ghost_tile_dot_bf16(const void* V, int v_ranks, int v_per_rank, const void* 
                         int n_cols, float dot_scale, float* M_out, void* grad_out, int grad_is_f32,
                         float grad_scale, int grad_accumulate, void* stream);
 
+/* ---- Linear / Conv1D layers with few token rows -------------------------------------------------- */
+/* M_out[v, b] = <grad_v, grad_b> as the two paths above, the train gradient grad_out = grad_scale *
+ * sum_b X_b^T Y_b (if not NULL; [p, d], or [d, p] with in_by_out) and the per-sample column sums of B
+ * (if not NULL; fp32 [N, p]) in one launch, from A [N, T, d] and B [N, T, p] as they are (both fp32 or
+ * both bf16, dense rows), products and sums in fp32.  For the sizes ghost_dense_small_fits accepts
+ * (returns 1); others are GHOST_ERR_INVALID.  Replaces, for such layers, the lines of both paths. */
+int ghost_dense_small_fits(int is_f32, int n_train, int n_val, long long T, int d, int p);
+int ghost_dense_small(const void* A, const void* B, int is_f32, int n_train, int n_val, long long T, int d,
+                      int p, int in_by_out, float* M_out, void* grad_out, int grad_is_f32,
+                      float grad_scale, float* colsum_out, void* stream);
+
 /* ---- bias / LayerNorm / small reductions ------------------------------------------------------- */
 /* out[n, c] = sum_t G[n, t, c]  (fp32).  Replaces the token sums of
  * ghostEngines/supported_layers_grad_samplers_dotprod.py:138-146, 454-471 and

@@ -294,6 +294,33 @@ def test_tile_pass_and_gathered_tile_dot(case):
         assert torch.equal(res[1], one[1]) and O.rel_fro(res[2], one[2].double().cpu()) < 1e-6
 
 
+# edges of the one-launch kernel: T on both sides of its 8 x 4 token tile and of whole-sample groups,
+# one sample, widths off and on its 64 / 128 / 1024 column units, odd widths (no 16-byte loads)
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("case", [(1, 1, 1, 1, 1), (64, 16, 1, 512, 1024), (9, 9, 1, 130, 67), (5, 3, 2, 64, 1028),
+                                  (3, 5, 3, 33, 65), (4, 3, 4, 128, 64), (2, 2, 7, 40, 200), (3, 2, 8, 260, 12),
+                                  (2, 3, 9, 68, 1025), (5, 2, 16, 100, 36)])
+@pytest.mark.parametrize("in_by_out", [False, True])
+def test_dense_small(case, dtype, in_by_out):
+    o = ops()
+    n_t, n_v, T, d, p = case
+    g = torch.Generator().manual_seed(31)
+    A = (torch.randn(n_t + n_v, T, d, generator=g) / d ** 0.5).to(dtype)
+    B = (torch.randn(n_t + n_v, T, p, generator=g) / p ** 0.5).to(dtype)
+    from ghostsuite_b200 import _lib
+    assert _lib.load().ghost_dense_small_fits(int(dtype == torch.float32), n_t, n_v, T, d, p) == 1
+    l0 = _lib.launch_count()
+    M, grad, sums, Mb, sb = o.dense_hook(A.cuda(), B.cuda(), n_v, in_by_out, True, torch.float32, 0.5, True, torch.float32)
+    assert _lib.launch_count() - l0 == 1
+    after()
+    # float32 sums of exact products of the given values
+    assert O.rel_fro(M, O.linear_dot_exact(A, B, n_v)) < 1e-5
+    ref = 0.5 * torch.einsum("btp,btd->pd", B[:n_t].double(), A[:n_t].double())
+    assert O.rel_fro(grad, ref.t() if in_by_out else ref) < 1e-5
+    assert O.rel_fro(sums, B.double().sum(1)) < 1e-5
+    assert Mb.shape == (n_v, n_t) and sb.shape == (p,)
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("shape", [(8, 6, 24), (12, 1, 10), (5, 300, 520), (3, 1024, 768)])
 def test_colsum_and_bias(shape, dtype):
