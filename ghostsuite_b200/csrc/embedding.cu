@@ -2,15 +2,15 @@
 //
 // embedding_dot:  M[v, b] = sum_{t, s : id_b[t] == id_v[s]} <G_b[t], G_v[s]>
 //   The reference scatters the validation rows into a [vocab, d] table and gathers it at the train
-//   ids (ghostEngines/supported_layers_grad_samplers_dotprod.py:203-210); here the validation
-//   tokens are chained per token id in a vocab-sized head table (4 bytes per id) and every train
-//   token walks the chain of its id, so no [vocab, d] scratch exists and the result is split per
-//   validation sample.
+//   ids (ghostEngines/supported_layers_grad_samplers_dotprod.py:203-210); here train and validation
+//   tokens are bucketed by id and joined id by id, so no [vocab, d] scratch exists, every row is
+//   fetched about once, and the result is split per validation sample.
 //
-// embedding_wgrad: averaged train gradient of the table (:214-235).  Train tokens are bucketed by
-//   id (count, scan, fill), each bucket is put in ascending token order and summed in float32 in
-//   that order, rounded to the table dtype once, then divided by n_train -- the arithmetic and
-//   the order of the CPU index_add_, so the result is bit-identical to it.
+// embedding_wgrad: averaged train gradient of the table (:214-235).  Each train bucket is summed in
+//   ascending token order in float32, rounded to the table dtype once, then divided by n_train --
+//   the arithmetic and the order of the CPU index_add_, so the result is bit-identical to it.
+//
+// Both results share the buckets (count, allocate, fill): ghost_embedding_pass makes them once.
 #include <limits.h>
 
 #include <mutex>
@@ -61,16 +61,16 @@ template <typename T> __device__ __forceinline__ T from_f32(float x);
 template <> __device__ __forceinline__ float from_f32<float>(float x) { return x; }
 template <> __device__ __forceinline__ __nv_bfloat16 from_f32<__nv_bfloat16>(float x) { return __float2bfloat16_rn(x); }
 
-// ---------------------------------------------------------------- dot product
+// ---------------------------------------------------------------- dot product, least workspace
+// Validation tokens chained per id in a vocab-sized head table; every train token walks the chain of its
+// id.  For callers that have no room for the buckets (ghost_embedding_dot_noalloc).
 __global__ void emb_chain_val_kernel(const long long* __restrict__ ids_val, long long n_tok, int vocab,
-                                     int* __restrict__ head, int* __restrict__ next, int* __restrict__ cnt,
-                                     int* __restrict__ err) {
+                                     int* __restrict__ head, int* __restrict__ next, int* __restrict__ err) {
   for (long long j = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; j < n_tok;
        j += static_cast<long long>(gridDim.x) * blockDim.x) {
     const long long id = ids_val[j];
     if (id >= 0 && id < vocab) {
       next[j] = atomicExch(&head[id], static_cast<int>(j));
-      if (cnt != nullptr) atomicAdd(&cnt[id], 1);
     } else {            // the reference's index_add_ raises here; skipped and reported through the error word
       next[j] = -1;
       atomicExch(err, kErrBadIndex);
@@ -78,47 +78,12 @@ __global__ void emb_chain_val_kernel(const long long* __restrict__ ids_val, long
   }
 }
 
-// Ids that many validation tokens share (padding, separators, position ids with a large validation
-// batch) would make every train token with that id walk a long chain.  For the `cap` most ... first
-// ids whose chain is longer than `threshold`, the validation rows are summed once per (id,
-// validation sample) into R[slot][v][d] (float32); a train token then takes n_val dot products
-// against R instead of walking the chain.  cnt[id] is overwritten with -(slot + 1) for such ids.
-__global__ void emb_hot_assign_kernel(int* __restrict__ cnt, int vocab, int threshold, int cap,
-                                      int* __restrict__ n_hot) {
-  for (int id = blockIdx.x * blockDim.x + threadIdx.x; id < vocab; id += gridDim.x * blockDim.x) {
-    if (cnt[id] > threshold) {
-      const int h = atomicAdd(n_hot, 1);
-      if (h < cap) cnt[id] = -(h + 1);
-    }
-  }
-}
-
-// one warp per validation token: rows of hot ids are added into R[slot][v]
-template <typename T>
-__global__ void __launch_bounds__(256)
-emb_hot_reduce_kernel(const long long* __restrict__ ids_val, const T* __restrict__ Gval, long long n_tok,
-                      long long Tn, int d, int n_val, int vocab, const int* __restrict__ cnt,
-                      float* __restrict__ R) {
-  const int lane = threadIdx.x & 31;
-  const long long warps = static_cast<long long>(gridDim.x) * 8;
-  for (long long j = static_cast<long long>(blockIdx.x) * 8 + (threadIdx.x >> 5); j < n_tok; j += warps) {
-    const long long id = ids_val[j];
-    if (id < 0 || id >= vocab) continue;
-    const int c = cnt[id];
-    if (c >= 0) continue;
-    float* dst = R + (static_cast<long long>(-c - 1) * n_val + j / Tn) * d;
-    const T* row = Gval + j * d;
-    for (int f = lane; f < d; f += 32) atomicAdd(dst + f, ld_f32<T>(row + f));
-  }
-}
-
 // grid (token blocks of one sample, n_train); 8 warps, each walks kTokPerWarp tokens
 template <typename T>
 __global__ void __launch_bounds__(256)
-emb_dot_kernel(const long long* __restrict__ ids, const T* __restrict__ G, int n_train, int n_val,
+emb_chain_dot_kernel(const long long* __restrict__ ids, const T* __restrict__ G, int n_train, int n_val,
                long long Tn, int d, int vocab, const int* __restrict__ head,
-               const int* __restrict__ next, const int* __restrict__ cnt, const float* __restrict__ R,
-               float scale, float* __restrict__ M, int tok_per_block, int* __restrict__ err) {
+               const int* __restrict__ next, float scale, float* __restrict__ M, int tok_per_block, int* __restrict__ err) {
   extern __shared__ float s_acc[];   // [n_val]
   const int b = blockIdx.y;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -137,20 +102,6 @@ emb_dot_kernel(const long long* __restrict__ ids, const T* __restrict__ G, int n
     }
     int j = head[id];
     const T* row = G + (static_cast<long long>(b) * Tn + t) * d;
-    const int c = (cnt != nullptr) ? cnt[id] : 0;
-    if (c < 0) {
-      // an id shared by many validation tokens: one dot product per validation sample against the
-      // pre-summed rows
-      const float* Rh = R + static_cast<long long>(-c - 1) * n_val * d;
-      for (int v = 0; v < n_val; ++v) {
-        const float* rv = Rh + static_cast<long long>(v) * d;
-        float s = 0.f;
-        for (int f = lane; f < d; f += 32) s = fmaf(ld_f32<T>(row + f), rv[f], s);
-        s = ewarp_sum(s);
-        if (lane == 0 && s != 0.f) atomicAdd(&s_acc[v], s);
-      }
-      continue;
-    }
     while (j >= 0) {
       const T* vrow = Gval + static_cast<long long>(j) * d;
       float s = 0.f;
@@ -177,83 +128,6 @@ emb_dot_kernel(const long long* __restrict__ ids, const T* __restrict__ G, int n
   for (int v = threadIdx.x; v < n_val; v += blockDim.x) {
     const float s = s_acc[v];
     if (s != 0.f) atomicAdd(&M[static_cast<long long>(v) * n_train + b], s * scale);
-  }
-}
-
-// ---------------------------------------------------------------- train gradient
-__global__ void emb_count_kernel(const long long* __restrict__ ids, long long n_tok, int vocab,
-                                 int* __restrict__ counts, int* __restrict__ err) {
-  for (long long j = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; j < n_tok;
-       j += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const long long id = ids[j];
-    if (id >= 0 && id < vocab) atomicAdd(&counts[id], 1);
-    else atomicExch(err, kErrBadIndex);
-  }
-}
-
-constexpr int kEmbSmallBucket = 32;      // buckets up to this size are sorted and summed by one warp
-
-// Exclusive scan of counts[0..vocab) into offsets (single block of 1024 threads; tiles of 4096 ids,
-// four consecutive ids per thread, the next tile's loads issued before this tile is scanned), and
-// the list of rows with more than kEmbSmallBucket tokens for emb_big_bucket_kernel.
-__global__ void __launch_bounds__(1024)
-emb_scan_kernel(const int* __restrict__ counts, int vocab, int* __restrict__ offsets, int* __restrict__ big,
-                int* __restrict__ n_big) {
-  __shared__ int s_warp[2][32];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  auto load4 = [&](int base, int (&c)[4]) {
-#pragma unroll
-    for (int e = 0; e < 4; ++e) c[e] = (base + e < vocab) ? counts[base + e] : 0;
-  };
-  int carry = 0, cur[4], nxt[4];
-  load4(threadIdx.x * 4, cur);
-  int buf = 0;
-  for (int tile = 0; tile < vocab; tile += 4096, buf ^= 1) {
-    const int base = tile + threadIdx.x * 4;
-    load4(base + 4096, nxt);
-    const int total = cur[0] + cur[1] + cur[2] + cur[3];
-    int x = total;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int y = __shfl_up_sync(0xffffffffu, x, o);
-      if (lane >= o) x += y;
-    }
-    if (lane == 31) s_warp[buf][warp] = x;
-    __syncthreads();
-    // every warp scans the 32 warp totals itself (one barrier per tile; the two buffers alternate)
-    int w = s_warp[buf][lane];
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int y = __shfl_up_sync(0xffffffffu, w, o);
-      if (lane >= o) w += y;
-    }
-    const int tile_total = __shfl_sync(0xffffffffu, w, 31);
-    const int warp_off = __shfl_sync(0xffffffffu, w, (warp + 31) & 31);
-    int run = carry + (warp == 0 ? 0 : warp_off) + x - total;
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      if (base + e < vocab) {
-        offsets[base + e] = run;
-        if (cur[e] > kEmbSmallBucket) big[atomicAdd(n_big, 1)] = base + e;
-      }
-      run += cur[e];
-      cur[e] = nxt[e];
-    }
-    carry += tile_total;
-  }
-  if (threadIdx.x == 0) offsets[vocab] = carry;
-}
-
-__global__ void emb_fill_kernel(const long long* __restrict__ ids, long long n_tok, int vocab,
-                                const int* __restrict__ offsets, int* __restrict__ cursor,
-                                int* __restrict__ perm) {
-  for (long long j = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; j < n_tok;
-       j += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const long long id = ids[j];
-    if (id >= 0 && id < vocab) {
-      const int pos = atomicAdd(&cursor[id], 1);
-      perm[offsets[id] + pos] = static_cast<int>(j);
-    }
   }
 }
 
@@ -333,167 +207,536 @@ template <> struct EmbRaw<float> {
   }
 };
 
-// one warp per table row: ascending-order float32 segment sum, dtype rounding as the reference.
-// Rows with more than kEmbSmallBucket tokens are left to emb_big_bucket_kernel.  The work of a
-// row is the list of (256-feature step, token) units, step-major; the loads of eight units are
-// issued before their rows are added in order, so a row with one or two tokens has all its loads
-// in flight at once.
+// ---------------------------------------------------------------- buckets of tokens by id
+// Train and validation tokens have indices of their own, both from zero; a scan runs over the train tokens
+// and then, from `first_val` on, over the validation tokens.
+struct EmbBuckets {
+  const long long *ids_b, *ids_v;
+  long long n_tok, first_val;           // tokens that take part, train tokens among them
+  int vocab;
+  int *cnt_b, *cnt_v;                   // [vocab] tokens per id, train / validation (cnt_v null: no dot products)
+  int *off_b, *off_v;                   // [vocab] first position of the id's bucket in perm_b / perm_v
+  int *rank;                            // [n_tok] position inside the bucket, -1 for an id outside the table
+  int *perm_b, *perm_v;
+  int *totals;                          // [0] train tokens placed, [1] validation, [2] big rows, [3] items, [4] hot ids
+  int *big;                             // ids with more than kEmbSmallBucket train tokens
+  int2 *items;                          // (id, train chunk) pairs of the join
+  int *slot;                            // [vocab] summed-row slot of a hot id, -1 otherwise
+  int *hot;                             // ids by slot
+  int hot_threshold, want_big;
+  int* err;
+};
+
+constexpr int kEmbSmallBucket = 32;      // buckets up to this size are sorted and summed by one warp
+constexpr int kEmbHotCap = 256;
+constexpr int kEmbChunk = 32;            // train tokens of a join item
+
+// Counting hands every token its place in the bucket, so filling needs no second round of atomics.
+// It also clears M, which the join adds to two launches later.
+__global__ void __launch_bounds__(256) emb_count_kernel(const EmbBuckets q, float* __restrict__ M, long long m_size) {
+  if (M != nullptr)
+    for (long long i = blockIdx.x * 256ll + threadIdx.x; i < m_size; i += gridDim.x * 256ll) M[i] = 0.f;
+  for (long long j = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; j < q.n_tok;
+       j += static_cast<long long>(gridDim.x) * blockDim.x) {
+    const long long id = j < q.first_val ? q.ids_b[j] : q.ids_v[j - q.first_val];
+    if (id >= 0 && id < q.vocab) {
+      q.rank[j] = atomicAdd((j < q.first_val ? q.cnt_b : q.cnt_v) + id, 1);
+    } else {            // the reference's index_add_ raises here; skipped and reported through the error word
+      q.rank[j] = -1;
+      atomicExch(q.err, kErrBadIndex);
+    }
+  }
+}
+
+// Buckets may lie in any order, so a block of ids takes its space with one atomic instead of waiting for
+// a scan over the whole table (22 us in one block for 50 k ids, 3 us now); the ids of a block stay in
+// ascending order, which the segment sum relies on.  Also listed here: rows for the big-bucket
+// kernel, join items, and ids that many validation tokens share (padding, separators).
+__global__ void __launch_bounds__(256) emb_alloc_kernel(const EmbBuckets q) {
+  __shared__ int s_warp[2][8], s_base[2];
+  const int id = blockIdx.x * 256 + threadIdx.x;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const bool in = id < q.vocab;
+  const int n[2] = {in ? q.cnt_b[id] : 0, in && q.cnt_v ? q.cnt_v[id] : 0};
+  int before[2];
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    int x = n[h];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
+    }
+    before[h] = x - n[h];
+    if (lane == 31) s_warp[h][warp] = x;
+  }
+  __syncthreads();
+  if (threadIdx.x < 2) {
+    int sum = 0;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) { const int c = s_warp[threadIdx.x][w]; s_warp[threadIdx.x][w] = sum; sum += c; }
+    s_base[threadIdx.x] = sum ? atomicAdd(q.totals + threadIdx.x, sum) : 0;
+  }
+  __syncthreads();
+  if (!in) return;
+  q.off_b[id] = s_base[0] + s_warp[0][warp] + before[0];
+  if (q.want_big && n[0] > kEmbSmallBucket) q.big[atomicAdd(q.totals + 2, 1)] = id;
+  if (q.cnt_v == nullptr) return;
+  q.off_v[id] = s_base[1] + s_warp[1][warp] + before[1];
+  int slot = -1;
+  if (n[1] > 0 && n[0] > 0) {
+    const int chunks = (n[0] + kEmbChunk - 1) / kEmbChunk;
+    const int at = atomicAdd(q.totals + 3, chunks);
+    for (int c = 0; c < chunks; ++c) q.items[at + c] = make_int2(id, c);
+    if (n[1] > q.hot_threshold) {
+      slot = atomicAdd(q.totals + 4, 1);
+      if (slot < kEmbHotCap) q.hot[slot] = id; else slot = -1;
+    }
+  }
+  q.slot[id] = slot;
+}
+
+__global__ void __launch_bounds__(256) emb_fill_kernel(const EmbBuckets q) {
+  for (long long j = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; j < q.n_tok;
+       j += static_cast<long long>(gridDim.x) * blockDim.x) {
+    const int r = q.rank[j];
+    if (r < 0) continue;
+    if (j < q.first_val) q.perm_b[q.off_b[q.ids_b[j]] + r] = static_cast<int>(j);
+    else q.perm_v[q.off_v[q.ids_v[j - q.first_val]] + r] = static_cast<int>(j - q.first_val);
+  }
+}
+
+// ---------------------------------------------------------------- dot product: join by id
+// R[slot][v] = sum of validation sample v's rows with the hot id of `slot` (float32).  One CTA per (slot,
+// sample): the sample's tokens are picked out of the bucket 1024 at a time; a thread adds eight
+// features of every groups-th token, four rows in flight, and the groups meet in shared memory.
+template <typename T>
+__global__ void __launch_bounds__(256)
+emb_hot_reduce_kernel(const EmbBuckets q, const T* __restrict__ Gv, long long Tn, int d, int n_val, float* __restrict__ R) {
+  __shared__ int s_tok[1024];
+  __shared__ __align__(16) float s_sum[256 * 8];
+  __shared__ int s_n;
+  const int hot = min(q.totals[4], kEmbHotCap);
+  const bool vec = (d % 8 == 0) && ((reinterpret_cast<uintptr_t>(Gv) & 15u) == 0);
+  const int per_row = min(256, (d + 7) / 8), groups = 256 / per_row;
+  const int grp = threadIdx.x / per_row, fi = threadIdx.x % per_row;
+  for (int w = blockIdx.x; w < hot * n_val; w += gridDim.x) {
+    const int slot = w / n_val, v = w % n_val;
+    const int id = q.hot[slot], cnt = q.cnt_v[id], off = q.off_v[id];
+    const long long lo = v * Tn, hi = lo + Tn;
+    float* dst = R + static_cast<long long>(w) * d;
+    for (int c0 = 0; c0 < cnt; c0 += 1024) {
+      __syncthreads();
+      if (threadIdx.x == 0) s_n = 0;
+      __syncthreads();
+      for (int i = c0 + threadIdx.x; i < min(cnt, c0 + 1024); i += 256) {
+        const int j = q.perm_v[off + i];
+        if (j >= lo && j < hi) s_tok[atomicAdd(&s_n, 1)] = j;
+      }
+      __syncthreads();
+      const int n = s_n;
+      for (int f0 = 0; f0 < d; f0 += per_row * 8) {
+        const int f = f0 + fi * 8;
+        float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        if (grp < groups && f < d) {
+#pragma unroll 4
+          for (int i = grp; i < n; i += groups) {
+            float x[8];
+            emb_load_row<T>(Gv, s_tok[i], d, f, vec, x);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) s[e] += x[e];
+          }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int e = 0; e < 8; ++e) s_sum[threadIdx.x * 8 + e] = s[e];
+        __syncthreads();
+        for (int i = threadIdx.x; i < per_row * 8 && f0 + i < d; i += 256) {
+          float t = c0 == 0 ? 0.f : dst[f0 + i];
+          for (int g = 0; g < groups; ++g) t += s_sum[g * per_row * 8 + i];
+          dst[f0 + i] = t;
+        }
+      }
+    }
+  }
+}
+
+// a lane's NCH groups of eight features (f0 + 256 * h) of one row, as loaded and as float32
+template <typename E, int NCH, bool VEC> struct EmbLaneRow {
+  typename EmbRaw<E>::type raw[NCH];
+  __device__ __forceinline__ void load(const E* row, int f0, int d) {
+#pragma unroll
+    for (int h = 0; h < NCH; ++h) raw[h] = f0 + h * 256 < d ? EmbRaw<E>::load(row + f0 + h * 256) : EmbRaw<E>::zero();
+  }
+  __device__ __forceinline__ void get(float (&x)[NCH * 8]) const {
+#pragma unroll
+    for (int h = 0; h < NCH; ++h) {
+      float t[8];
+      EmbRaw<E>::unpack(raw[h], t);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) x[h * 8 + e] = t[e];
+    }
+  }
+};
+template <typename E, int NCH> struct EmbLaneRow<E, NCH, false> {      // rows without 16-byte alignment
+  float v[NCH * 8];
+  __device__ __forceinline__ void load(const E* row, int f0, int d) {
+#pragma unroll
+    for (int h = 0; h < NCH; ++h)
+#pragma unroll
+      for (int e = 0; e < 8; ++e) v[h * 8 + e] = f0 + h * 256 + e < d ? ld_f32<E>(row + f0 + h * 256 + e) : 0.f;
+  }
+  __device__ __forceinline__ void get(float (&x)[NCH * 8]) const {
+#pragma unroll
+    for (int e = 0; e < NCH * 8; ++e) x[e] = v[e];
+  }
+};
+
+// One join item per warp: up to 32 train rows of one id against the id's validation rows (or, for a hot
+// id, one summed row per validation sample), VB validation rows held in registers at a time while the
+// train rows pass by with the next one's loads in flight.  Every row comes from HBM once; repeats hit
+// L1 / L2.  What bounds it is the products themselves (a fused multiply-add and its share of unpacking
+// per feature and pair).  Walking a chain per train token, the form before it, re-read the
+// validation rows for every train token behind two dependent loads: 150 us against 26 for text ids
+// (40 x 1024 tokens of 768 bf16 features), 125 against 40 for position ids.
+template <typename T, int NCH, int VB, bool VEC>
+__global__ void __launch_bounds__(128)
+emb_join_kernel(const EmbBuckets q, const T* __restrict__ Gb, const T* __restrict__ Gv, int n_train, int n_val, int Tn, int d,
+                const float* __restrict__ R, float scale, float* __restrict__ M, long long pitch, int local) {
+  extern __shared__ float s_M[];         // [n_val, n_train] when `local`
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (local) {
+    for (int i = threadIdx.x; i < n_val * n_train; i += 128) s_M[i] = 0.f;
+    __syncthreads();
+  }
+  float* acc_M = local ? s_M : M;
+  const long long acc_pitch = local ? n_train : pitch;
+  const float out_scale = local ? 1.f : scale;
+  const int n_items = q.totals[3];
+  for (int it = blockIdx.x * 4 + warp; it < n_items; it += gridDim.x * 4) {
+    const int2 item = q.items[it];
+    const int id = item.x, slot = q.slot[id];
+    const int nb = min(kEmbChunk, q.cnt_b[id] - item.y * kEmbChunk);
+    const int cv = slot >= 0 ? n_val : q.cnt_v[id];
+    const int my_b = lane < nb ? q.perm_b[q.off_b[id] + item.y * kEmbChunk + lane] : 0;
+    for (int w0 = 0; w0 < cv; w0 += 32) {
+      const int nw = min(32, cv - w0);
+      const int my_v = slot >= 0 || lane >= nw ? 0 : q.perm_v[q.off_v[id] + w0 + lane];
+      for (int v0 = 0; v0 < nw; v0 += VB) {
+        int sample[VB];
+        for (int fc = 0; fc < d; fc += NCH * 256) {
+          float y[VB][NCH * 8];
+#pragma unroll
+          for (int u = 0; u < VB; ++u) {
+            const int vi = min(v0 + u, nw - 1);
+            const int jv = __shfl_sync(0xffffffffu, my_v, vi);
+            if (slot >= 0) {
+              sample[u] = w0 + vi;
+              EmbLaneRow<float, NCH, VEC> r;
+              r.load(R + (static_cast<long long>(slot) * n_val + w0 + vi) * d, fc + lane * 8, d);
+              r.get(y[u]);
+            } else {
+              sample[u] = jv / Tn;
+              EmbLaneRow<T, NCH, VEC> r;
+              r.load(Gv + static_cast<long long>(jv) * d, fc + lane * 8, d);
+              r.get(y[u]);
+            }
+          }
+          EmbLaneRow<T, NCH, VEC> next;
+          int jb = __shfl_sync(0xffffffffu, my_b, 0);
+          next.load(Gb + static_cast<long long>(jb) * d, fc + lane * 8, d);
+          for (int i = 0; i < nb; ++i) {
+            const int b = jb / Tn;
+            float x[NCH * 8];
+            next.get(x);
+            if (i + 1 < nb) {
+              jb = __shfl_sync(0xffffffffu, my_b, i + 1);
+              next.load(Gb + static_cast<long long>(jb) * d, fc + lane * 8, d);
+            }
+            float s[VB];
+#pragma unroll
+            for (int u = 0; u < VB; ++u) s[u] = 0.f;
+#pragma unroll
+            for (int e = 0; e < NCH * 8; ++e)
+#pragma unroll
+              for (int u = 0; u < VB; ++u) s[u] = fmaf(x[e], y[u][e], s[u]);
+            // halve the set of values with the distance: lane (u << (5 - log2 VB)) ends with row u's sum
+            int width = VB;
+#pragma unroll
+            for (int o = 16; o >= 1; o >>= 1) {
+              if (width > 1) {
+                width >>= 1;
+                const bool up = (lane & o) != 0;
+#pragma unroll
+                for (int u = 0; u < VB / 2; ++u)
+                  if (u < width) {
+                    const float send = up ? s[u] : s[u + width], keep = up ? s[u + width] : s[u];
+                    s[u] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+                  }
+              } else {
+                s[0] += __shfl_xor_sync(0xffffffffu, s[0], o);
+              }
+            }
+            constexpr int kEvery = 32 / VB;
+            const int u = lane / kEvery;
+            if (lane % kEvery == 0 && v0 + u < nw) {
+              int sv = sample[0];
+#pragma unroll
+              for (int w = 1; w < VB; ++w) sv = u == w ? sample[w] : sv;
+              atomicAdd(acc_M + sv * acc_pitch + b, s[0] * out_scale);
+            }
+          }
+        }
+      }
+    }
+  }
+  if (local) {
+    __syncthreads();
+    for (int i = threadIdx.x; i < n_val * n_train; i += 128) {
+      const float s = s_M[i];
+      if (s != 0.f) atomicAdd(M + i / n_train * pitch + i % n_train, s * scale);
+    }
+  }
+}
+
+// ---------------------------------------------------------------- train gradient
+// Ascending-order float32 segment sum of the buckets of up to 32 tokens, dtype rounding as the reference.
+// A warp takes eight consecutive table rows, whose buckets lie one after the other: their sizes, their
+// token lists and the loads of their first eight (256-feature step, token) units are each one round of
+// memory latency for all eight rows, where a warp per row went through offsets, tokens, loads and
+// store with one or two rows' bytes in flight.  The (row, token) pairs of a group of rows with up to 32
+// tokens are put in order by one bitonic network.  Rows without tokens are zero-filled on the way.
+// Larger buckets are left to emb_big_bucket_kernel.
+constexpr int kEmbRowsPerWarp = 8;
+constexpr int kEmbTokenBits = 28;        // a sort key is (row of the group, token); more tokens: one row at a time
+
 template <typename T>
 __global__ void __launch_bounds__(256, 3)
-emb_segsum_kernel(const T* __restrict__ G, int d, int vocab, const int* __restrict__ offsets,
-                  const int* __restrict__ perm, float pre_scale, float divisor, int accumulate,
+emb_segsum_kernel(const EmbBuckets q, const T* __restrict__ G, int d, float pre_scale, float divisor, int accumulate,
                   T* __restrict__ out) {
-  const int k = blockIdx.x * 8 + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
-  if (k >= vocab) return;
-  const int off = offsets[k];
-  const int cnt = offsets[k + 1] - off;
-  if (cnt > kEmbSmallBucket) return;
+  const int k0 = (blockIdx.x * 8 + (threadIdx.x >> 5)) * kEmbRowsPerWarp;
+  if (k0 >= q.vocab) return;
+  const int rows = min(kEmbRowsPerWarp, q.vocab - k0);
   const bool vec = (d % 8 == 0) && ((reinterpret_cast<uintptr_t>(G) & 15u) == 0) &&
                    ((reinterpret_cast<uintptr_t>(out) & 15u) == 0);
   const int steps = (d + 255) / 256;
-  if (cnt == 0) {
-    const float zero[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    for (int c = 0; c < steps; ++c) emb_store_row<T>(out, k, d, c * 256 + lane * 8, vec, zero, divisor, accumulate);
-    return;
-  }
-  int mine = INT_MAX;
-  if (lane < cnt) mine = perm[off + lane];
-  if (cnt > 1) {
-    // bitonic sort of 32 keys across the warp, ascending
-#pragma unroll
-    for (int size = 2; size <= 32; size <<= 1) {
-#pragma unroll
-      for (int stride = size >> 1; stride > 0; stride >>= 1) {
-        const int other = __shfl_xor_sync(0xffffffffu, mine, stride);
-        const bool up = ((lane & size) == 0);
-        const bool lower = ((lane & stride) == 0);
-        const int lo = min(mine, other), hi = max(mine, other);
-        mine = (lower == up) ? lo : hi;
-      }
-    }
-  }
-  // each lane owns 8 consecutive features of a step (16-byte loads and stores when d % 8 == 0);
-  // loaded rows stay packed until they are added (32 registers per batch for either dtype)
-  constexpr int kBatch = sizeof(T) == 2 ? 8 : 4;
-  const int units = steps * cnt;
-  float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-  int step = 0, i = 0;                     // unit -> (step, token index), advanced without divisions
-  auto finish_unit = [&]() {
-    if (++i == cnt) {                      // last token of this step: write the row's 256 features
-      emb_store_row<T>(out, k, d, step * 256 + lane * 8, vec, acc, divisor, accumulate);
-#pragma unroll
-      for (int e = 0; e < 8; ++e) acc[e] = 0.f;
-      i = 0;
-      ++step;
-    }
-  };
-  if (!vec) {                              // odd feature counts: one unit at a time
-    for (int u = 0; u < units; ++u) {
-      float x[8];
-      emb_load_row<T>(G, __shfl_sync(0xffffffffu, mine, i), d, step * 256 + lane * 8, false, x);
-      emb_accumulate<T>(x, pre_scale, acc);
-      finish_unit();
-    }
-    return;
-  }
+  const int my_cnt = lane < rows ? q.cnt_b[k0 + lane] : 0, my_off = lane < rows ? q.off_b[k0 + lane] : 0;
+  const bool wide_ids = q.first_val >= (1ll << kEmbTokenBits);
   using Raw = typename EmbRaw<T>::type;
-  for (int u0 = 0; u0 < units; u0 += kBatch) {
-    Raw x[kBatch];
-    {
-      int c = step, ii = i;
-#pragma unroll
-      for (int r = 0; r < kBatch; ++r) {
-        const int j = __shfl_sync(0xffffffffu, mine, ii & 31);
-        const int f = c * 256 + lane * 8;
-        if (u0 + r < units && f < d) x[r] = EmbRaw<T>::load(G + static_cast<long long>(j) * d + f);
-        else x[r] = EmbRaw<T>::zero();
-        if (++ii == cnt) { ii = 0; ++c; }
-      }
-    }
-#pragma unroll
-    for (int r = 0; r < kBatch; ++r) {
-      if (u0 + r < units) {
-        float xf[8];
-        EmbRaw<T>::unpack(x[r], xf);
-        emb_accumulate<T>(xf, pre_scale, acc);
-        finish_unit();
-      }
-    }
-  }
-}
+  constexpr int kBatch = sizeof(T) == 2 ? 8 : 4;      // 32 registers of loaded rows for either dtype
 
-// Rows that many tokens share (padding, separators, position ids of a large batch).  The list of
-// such rows is made by emb_scan_kernel; one CTA per listed row first sorts the row's token
-// list into ascending order -- a bitonic network whose comparators all point the same way, so
-// entries past the end of the list act as +infinity without being stored; in shared memory up to
-// `smem_cap` entries, in place in global memory beyond -- and then sums the rows in that order.
-// The sum itself is sequential per feature (float addition in the CPU's order), so the loads of
-// the next eight rows are issued before the current eight are added.
-__device__ __forceinline__ void emb_bitonic_ascending(int* keys, int cnt, int n2, int tid, int nthreads) {
-  for (int k = 2; k <= n2; k <<= 1) {
-    for (int j = k >> 1; j > 0; j >>= 1) {
-      // the first stage of every merge pairs i with its mirror image inside the block of k
-      for (int i = tid; i < n2; i += nthreads) {
-        const int l = (j == (k >> 1)) ? (i ^ (k - 1)) : (i ^ j);
-        if (l > i && l < cnt) {
-          const int a = keys[i], b = keys[l];
-          if (a > b) { keys[i] = b; keys[l] = a; }
+  int r0 = 0;
+  while (r0 < rows) {
+    // rows [r0, r1): as many as fit 32 tokens together; zero rows are stored, big ones skipped
+    int n = 0, r1 = r0, row_of = 0, pos_in = 0, off_in = 0;
+    while (r1 < rows) {
+      int c = __shfl_sync(0xffffffffu, my_cnt, r1);
+      const int off = __shfl_sync(0xffffffffu, my_off, r1);
+      if (c > kEmbSmallBucket) c = 0;
+      else if (c == 0) {
+        const float zero[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        for (int s = 0; s < steps; ++s) emb_store_row<T>(out, k0 + r1, d, s * 256 + lane * 8, vec, zero, divisor, accumulate);
+      } else {
+        if (n > 0 && (n + c > 32 || wide_ids)) break;
+        if (lane >= n && lane < n + c) { row_of = r1; pos_in = lane - n; off_in = off; }
+        n += c;
+      }
+      ++r1;
+    }
+    r0 = r1;
+    if (n == 0) continue;
+    int key = INT_MAX;
+    if (lane < n) key = q.perm_b[off_in + pos_in];
+    if (!wide_ids && lane < n) key |= row_of << kEmbTokenBits;
+    if (n > 1) {
+#pragma unroll
+      for (int size = 2; size <= 32; size <<= 1) {
+#pragma unroll
+        for (int stride = size >> 1; stride > 0; stride >>= 1) {
+          const int other = __shfl_xor_sync(0xffffffffu, key, stride);
+          const bool up = ((lane & size) == 0);
+          const bool lower = ((lane & stride) == 0);
+          const int lo = min(key, other), hi = max(key, other);
+          key = (lower == up) ? lo : hi;
         }
       }
-      __syncthreads();
+    }
+    // the sort keeps rows together and in order, so lane i's row is still row_of
+    const int tok = wide_ids ? key : key & ((1 << kEmbTokenBits) - 1);
+    const int next_row = __shfl_down_sync(0xffffffffu, row_of, 1);
+    const unsigned ends = __ballot_sync(0xffffffffu, lane < n && (lane == n - 1 || next_row != row_of));
+    const int units = steps * n;
+    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    int step = 0, i = 0;                   // unit -> (step, token), advanced without divisions
+    auto finish_unit = [&]() {
+      const int row = __shfl_sync(0xffffffffu, row_of, i);
+      if ((ends >> i) & 1u) {              // last token of the row: write its 256 features
+        emb_store_row<T>(out, k0 + row, d, step * 256 + lane * 8, vec, acc, divisor, accumulate);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) acc[e] = 0.f;
+      }
+      if (++i == n) { i = 0; ++step; }
+    };
+    if (!vec) {                            // odd feature counts: one unit at a time
+      for (int u = 0; u < units; ++u) {
+        float x[8];
+        emb_load_row<T>(G, __shfl_sync(0xffffffffu, tok, i), d, step * 256 + lane * 8, false, x);
+        emb_accumulate<T>(x, pre_scale, acc);
+        finish_unit();
+      }
+      continue;
+    }
+    for (int u0 = 0; u0 < units; u0 += kBatch) {
+      Raw x[kBatch];
+      {
+        int c = step, ii = i;
+#pragma unroll
+        for (int r = 0; r < kBatch; ++r) {
+          const int j = __shfl_sync(0xffffffffu, tok, ii);
+          const int f = c * 256 + lane * 8;
+          if (u0 + r < units && f < d) x[r] = EmbRaw<T>::load(G + static_cast<long long>(j) * d + f);
+          else x[r] = EmbRaw<T>::zero();
+          if (++ii == n) { ii = 0; ++c; }
+        }
+      }
+#pragma unroll
+      for (int r = 0; r < kBatch; ++r) {
+        if (u0 + r < units) {
+          float xf[8];
+          EmbRaw<T>::unpack(x[r], xf);
+          emb_accumulate<T>(xf, pre_scale, acc);
+          finish_unit();
+        }
+      }
     }
   }
 }
 
+// Rows that many tokens share (padding, separators, frequent words).  A CTA takes 256 bytes of one row's
+// features (128 bf16, 64 float32).  Ascending order comes from a bit map instead of a sort: the row's
+// tokens set bits of a window of 32768 tokens in shared memory, and prefix sums of the words' bit counts
+// turn the map into an ordered list.  The sum is sequential per feature (float addition in the CPU's
+// order), so its bound is the issue rate of one warp, eight instructions a token; a four-slot ring of
+// 32-row stages filled with cp.async keeps the rows arriving at that pace.  One CTA per row with a
+// sorted list and eight rows in flight: 492 us for text ids (the longest row 1250 tokens), 18 us now.
+constexpr int kBigThreads = 128;
+constexpr int kBigWindow = 32768;        // tokens of a bit map: 1024 words, eight per thread
+constexpr int kBigList = 2048;           // list entries held at a time
+constexpr int kBigStage = 32, kBigSlots = 4;
+
 template <typename T>
-__global__ void __launch_bounds__(256)
-emb_big_bucket_kernel(const T* __restrict__ G, int d, const int* __restrict__ offsets, int* __restrict__ perm,
-                      const int* __restrict__ big, const int* __restrict__ n_big, int smem_cap,
-                      float pre_scale, float divisor, int accumulate, T* __restrict__ out) {
-  extern __shared__ int s_keys[];
-  const int tid = threadIdx.x;
-  const int total = *n_big;
-  const bool vec = (d % 8 == 0) && ((reinterpret_cast<uintptr_t>(G) & 15u) == 0) &&
-                   ((reinterpret_cast<uintptr_t>(out) & 15u) == 0);
-  for (int bi = blockIdx.x; bi < total; bi += gridDim.x) {
-    const int k = big[bi];
-    const int off = offsets[k];
-    const int cnt = offsets[k + 1] - off;
-    int n2 = 64;
-    while (n2 < cnt) n2 <<= 1;
-    const int* keys;
-    __syncthreads();                      // the previous row's readers are done with s_keys
-    if (cnt <= smem_cap) {
-      for (int i = tid; i < cnt; i += blockDim.x) s_keys[i] = perm[off + i];
+__global__ void __launch_bounds__(kBigThreads)
+emb_big_bucket_kernel(const EmbBuckets q, const T* __restrict__ G, int d, int slices, float pre_scale, float divisor,
+                      int accumulate, T* __restrict__ out) {
+  constexpr int kFeat = 256 / static_cast<int>(sizeof(T));
+  constexpr int kPer = 16 / static_cast<int>(sizeof(T));       // features of a 16-byte piece
+  __shared__ unsigned s_map[kBigWindow / 32];
+  __shared__ unsigned short s_list[kBigList];
+  __shared__ int s_warp[kBigThreads / 32];
+  __shared__ __align__(16) T s_ring[kBigSlots][kBigStage][kFeat];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int total = q.totals[2];
+  const bool vec = (d % 8 == 0) && ((reinterpret_cast<uintptr_t>(G) & 15u) == 0);
+  const long long n_train_tok = q.first_val;
+  for (long long w = blockIdx.x; w < static_cast<long long>(total) * slices; w += gridDim.x) {
+    const int k = q.big[w / slices];
+    const int f0 = static_cast<int>(w % slices) * kFeat;
+    const int cnt = q.cnt_b[k], off = q.off_b[k];
+    const int f = f0 + tid;
+    const bool mine = tid < kFeat && f < d;
+    float acc = 0.f;
+    for (long long win = 0; win < n_train_tok; win += kBigWindow) {
       __syncthreads();
-      emb_bitonic_ascending(s_keys, cnt, n2, tid, blockDim.x);
-      keys = s_keys;
-    } else {
-      __threadfence_block();
-      emb_bitonic_ascending(perm + off, cnt, n2, tid, blockDim.x);   // in place; the CTA owns this range
-      keys = perm + off;
-    }
-    for (int f = tid * 8; f < d; f += blockDim.x * 8) {
-      float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-      float cur[8][8], nxt[8][8];
-      auto fetch = [&](int i0, float (&buf)[8][8]) {
-#pragma unroll
-        for (int r = 0; r < 8; ++r)
-          if (i0 + r < cnt) emb_load_row<T>(G, keys[i0 + r], d, f, vec, buf[r]);
-      };
-      fetch(0, cur);
-      for (int i0 = 0; i0 < cnt; i0 += 8) {
-        fetch(i0 + 8, nxt);
-#pragma unroll
-        for (int r = 0; r < 8; ++r)
-          if (i0 + r < cnt) emb_accumulate<T>(cur[r], pre_scale, acc);
-#pragma unroll
-        for (int r = 0; r < 8; ++r)
-#pragma unroll
-          for (int e = 0; e < 8; ++e) cur[r][e] = nxt[r][e];
+      for (int i = tid; i < kBigWindow / 32; i += kBigThreads) s_map[i] = 0u;
+      __syncthreads();
+      for (int i = tid; i < cnt; i += kBigThreads) {
+        const long long j = q.perm_b[off + i] - win;
+        if (j >= 0 && j < kBigWindow) atomicOr(&s_map[j >> 5], 1u << (j & 31));
       }
-      emb_store_row<T>(out, k, d, f, vec, acc, divisor, accumulate);
+      __syncthreads();
+      unsigned m[8];
+      int own = 0;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) { m[e] = s_map[tid * 8 + e]; own += __popc(m[e]); }
+      int x = own;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+      }
+      if (lane == 31) s_warp[warp] = x;
+      __syncthreads();
+      int first = x - own, in_window = 0;
+#pragma unroll
+      for (int v = 0; v < kBigThreads / 32; ++v) {
+        if (v < warp) first += s_warp[v];
+        in_window += s_warp[v];
+      }
+      for (int lo = 0; lo < in_window; lo += kBigList) {       // entries [lo, lo + kBigList) of the ordered list
+        const int n = min(kBigList, in_window - lo);
+        __syncthreads();
+        if (first < lo + n && first + own > lo) {
+          int at = first - lo;
+#pragma unroll
+          for (int e = 0; e < 8; ++e) {
+            unsigned bits = m[e];
+            while (bits) {
+              const int bit = __ffs(bits) - 1;
+              bits &= bits - 1;
+              if (at >= 0 && at < n) s_list[at] = static_cast<unsigned short>((tid * 8 + e) * 32 + bit);
+              ++at;
+            }
+          }
+        }
+        __syncthreads();
+        if (vec) {
+          const int n_stages = (n + kBigStage - 1) / kBigStage;
+          auto issue = [&](int st) {
+            if (st < n_stages) {
+#pragma unroll
+              for (int e = 0; e < kBigStage * 16 / kBigThreads; ++e) {
+                const int c = e * kBigThreads + tid, r = c >> 4, piece = (c & 15) * kPer;
+                const int i = st * kBigStage + r;
+                if (i < n && f0 + piece < d) {
+                  const T* src = G + (win + s_list[i]) * d + f0 + piece;
+                  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(static_cast<uint32_t>(
+                                   __cvta_generic_to_shared(&s_ring[st % kBigSlots][r][piece]))), "l"(src) : "memory");
+                }
+              }
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+          };
+          for (int st = 0; st < kBigSlots - 1; ++st) issue(st);
+          for (int st = 0; st < n_stages; ++st) {
+            asm volatile("cp.async.wait_group %0;" ::"n"(kBigSlots - 2) : "memory");
+            __syncthreads();              // stage `st` has arrived; slot of stage st - 1 is free
+            issue(st + kBigSlots - 1);
+            if (mine) {
+              const int rows = min(kBigStage, n - st * kBigStage);
+              if (rows == kBigStage) {
+#pragma unroll 8
+                for (int r = 0; r < kBigStage; ++r)
+                  acc = __fadd_rn(acc, round_to<T>(__fmul_rn(ld_f32<T>(&s_ring[st % kBigSlots][r][tid]), pre_scale)));
+              } else {
+                for (int r = 0; r < rows; ++r)
+                  acc = __fadd_rn(acc, round_to<T>(__fmul_rn(ld_f32<T>(&s_ring[st % kBigSlots][r][tid]), pre_scale)));
+              }
+            }
+          }
+          asm volatile("cp.async.wait_all;" ::: "memory");
+        } else if (mine) {
+#pragma unroll 4
+          for (int i = 0; i < n; ++i)
+            acc = __fadd_rn(acc, round_to<T>(__fmul_rn(ld_f32<T>(G + (win + s_list[i]) * d + f), pre_scale)));
+        }
+      }
+    }
+    if (mine) {
+      T* dst = out + static_cast<long long>(k) * d + f;
+      float o = round_to<T>(__fdiv_rn(round_to<T>(acc), divisor));
+      if (accumulate) o = round_to<T>(__fadd_rn(ld_f32<T>(dst), o));
+      *dst = from_f32<T>(o);
     }
   }
 }
@@ -504,18 +747,148 @@ static inline long long up256(long long x) { return (x + 255) / 256 * 256; }
 
 using namespace gb;
 
-// head [vocab] + next [n_val * T]: the least a caller must provide.  With the full size below the
-// repeated-id path is enabled as well: cnt [vocab], a counter, and R [kEmbHotCap, n_val, d] float32.
-constexpr int kEmbHotCap = 256;
-static long long emb_dot_min_bytes(int n_val, long long T, int vocab) {
+// head [vocab] + next [n_val * T]: the least a caller of ghost_embedding_dot must provide (chain kernels).
+extern "C" long long ghost_embedding_dot_workspace_bytes(int n_val, long long T, int vocab) {
   return up256(4ll * vocab) + up256(4ll * n_val * T);
 }
-extern "C" long long ghost_embedding_dot_workspace_bytes_for(int n_val, long long T, int vocab, int d) {
-  return emb_dot_min_bytes(n_val, T, vocab) + up256(4ll * vocab) + 256 +
-         up256(4ll * kEmbHotCap * static_cast<long long>(n_val) * d);
+
+extern "C" long long ghost_embedding_pass_workspace_bytes(int n_train, int n_val, long long T, int vocab, int d) {
+  const long long tb = static_cast<long long>(n_train) * T, tv = static_cast<long long>(n_val) * T;
+  return up256(4ll * (2 * static_cast<long long>(vocab) + 8)) + 3 * up256(4ll * vocab)     // counts and totals; offsets, slots
+         + up256(4ll * (tb + tv)) + up256(4ll * tb) + up256(4ll * tv)                      // rank, perm_b, perm_v
+         + up256(4ll * (tb / (kEmbSmallBucket + 1) + 2)) + up256(8ll * (tb / kEmbChunk + vocab + 1)) +   // big rows, items
+         + up256(4ll * kEmbHotCap) + up256(4ll * kEmbHotCap * static_cast<long long>(n_val) * d);
 }
-extern "C" long long ghost_embedding_dot_workspace_bytes(int n_val, long long T, int vocab) {
-  return emb_dot_min_bytes(n_val, T, vocab);
+extern "C" long long ghost_embedding_wgrad_workspace_bytes(int n_train, long long T, int vocab) {
+  return ghost_embedding_pass_workspace_bytes(n_train, 0, T, vocab, 0);
+}
+
+namespace gb {
+
+template <typename T>
+static int emb_pass(const EmbBuckets& q, const T* Gb, const T* Gv, int n_train, int n_val, long long Tn, int d, float scale,
+                    float* M, long long pitch, bool clear_M, float* R, float pre_scale, float divisor, int accumulate, T* out, const DeviceState* ds, cudaStream_t st) {
+  int blocks = static_cast<int>((q.n_tok + 255) / 256);
+  if (blocks > ds->sm_count * 8) blocks = ds->sm_count * 8;
+  emb_count_kernel<<<blocks, 256, 0, st>>>(q, clear_M ? M : nullptr, n_val * pitch);
+  emb_alloc_kernel<<<ceil_div(q.vocab, 256), 256, 0, st>>>(q);
+  emb_fill_kernel<<<blocks, 256, 0, st>>>(q);
+  count_launch(3);
+  const bool vec = d % 8 == 0 && ((reinterpret_cast<uintptr_t>(Gb) | reinterpret_cast<uintptr_t>(Gv)) & 15u) == 0;
+  if (M != nullptr) {
+    if (static_cast<long long>(n_val) * Tn > q.hot_threshold) {
+      int hb = kEmbHotCap * n_val;
+      if (hb > ds->sm_count * 8) hb = ds->sm_count * 8;
+      emb_hot_reduce_kernel<T><<<hb, 256, 0, st>>>(q, Gv, Tn, d, n_val, R);
+      count_launch();
+    }
+    // a matrix of up to 16 KB is summed up in shared memory first: few, hot addresses otherwise
+    const int local = static_cast<long long>(n_val) * n_train <= 4096 ? 1 : 0;
+    const size_t smem = local ? sizeof(float) * n_val * n_train : 0;
+    long long most = (static_cast<long long>(n_train) * Tn / kEmbChunk + q.vocab + 1 + 3) / 4;
+    const int jb = static_cast<int>(most < ds->sm_count * 4 ? most : ds->sm_count * 4);
+    const int Ti = static_cast<int>(Tn);
+    // register rows: the smallest number of 256-feature groups that covers d, at most four; four
+    // validation rows at a time where they fit the registers next to it
+#define GB_JOIN(NCH, VB, V) emb_join_kernel<T, NCH, VB, V><<<jb, 128, smem, st>>>(q, Gb, Gv, n_train, n_val, Ti, d, R, scale, M, pitch, local)
+    if (!vec) GB_JOIN(1, 4, false);
+    else if (d <= 256) GB_JOIN(1, 4, true);
+    else if (d <= 512) GB_JOIN(2, 4, true);
+    else if (d <= 768) GB_JOIN(3, 4, true);
+    else GB_JOIN(4, 2, true);
+#undef GB_JOIN
+    count_launch();
+  }
+  if (out != nullptr) {
+    emb_segsum_kernel<T><<<ceil_div(q.vocab, 8 * kEmbRowsPerWarp), 256, 0, st>>>(q, Gb, d, pre_scale, divisor, accumulate, out);
+    const int slices = ceil_div(d, 256 / static_cast<int>(sizeof(T)));
+    const long long most = (static_cast<long long>(n_train) * Tn / (kEmbSmallBucket + 1) + 1) * slices;
+    const int bb = static_cast<int>(most < ds->sm_count * 4 ? most : ds->sm_count * 4);
+    emb_big_bucket_kernel<T><<<bb, kBigThreads, 0, st>>>(q, Gb, d, slices, pre_scale, divisor, accumulate, out);
+    count_launch(2);
+  }
+  return post_launch("ghost_embedding_pass");
+}
+
+}  // namespace gb
+
+namespace gb {
+
+// Train samples [b0, b0 + n_b) against all validation samples (M non-null), and their gradient (out non-null)
+static int emb_pass_group(const long long* ids, const void* G, int is_f32, int n_train, int b0, int n_b, int n_val,
+                          long long T, int d, int vocab, float scale, float* M, float pre_scale, float divisor,
+                          int accumulate, void* out, void* ws, const DeviceState* ds, cudaStream_t st) {
+  const long long tb = static_cast<long long>(n_b) * T, tv = static_cast<long long>(n_val) * T;
+  uint8_t* at = static_cast<uint8_t*>(ws);
+  auto take = [&](long long bytes) { void* p = at; at += up256(bytes); return p; };
+  EmbBuckets q = {};
+  q.ids_b = ids + b0 * T;
+  q.ids_v = ids + n_train * T;
+  q.first_val = tb;
+  q.n_tok = tb + tv;
+  q.vocab = vocab;
+  const long long zero_bytes = 4ll * (2 * static_cast<long long>(vocab) + 8);
+  q.totals = static_cast<int*>(take(zero_bytes));
+  q.cnt_b = q.totals + 8;
+  q.cnt_v = M ? q.cnt_b + vocab : nullptr;
+  q.off_b = static_cast<int*>(take(4ll * vocab));
+  q.off_v = static_cast<int*>(take(4ll * vocab));
+  q.slot = static_cast<int*>(take(4ll * vocab));
+  q.rank = static_cast<int*>(take(4ll * (tb + tv)));
+  q.perm_b = static_cast<int*>(take(4ll * tb));
+  q.perm_v = static_cast<int*>(take(4ll * tv));
+  q.big = static_cast<int*>(take(4ll * (tb / (kEmbSmallBucket + 1) + 2)));
+  q.items = static_cast<int2*>(take(8ll * (tb / kEmbChunk + vocab + 1)));
+  q.hot = static_cast<int*>(take(4ll * kEmbHotCap));
+  float* R = static_cast<float*>(take(4ll * kEmbHotCap * static_cast<long long>(n_val) * (M ? d : 0)));
+  // a hot id costs n_val dot products per train token; worth it from twice as many validation tokens on
+  q.hot_threshold = 2 * n_val > 8 ? 2 * n_val : 8;
+  q.want_big = out != nullptr;
+  q.err = ds->err_word;
+  GB_CUDA_OK(cudaMemsetAsync(q.totals, 0, M ? zero_bytes : 4ll * (vocab + 8), st));
+  float* Mg = M ? M + b0 : nullptr;
+  if (is_f32) {
+    const float* g = static_cast<const float*>(G);
+    return emb_pass<float>(q, g + b0 * T * d, g + n_train * T * d, n_b, n_val, T, d, scale, Mg, n_train, b0 == 0, R,
+                           pre_scale, divisor, accumulate, static_cast<float*>(out), ds, st);
+  }
+  const __nv_bfloat16* g = static_cast<const __nv_bfloat16*>(G);
+  return emb_pass<__nv_bfloat16>(q, g + b0 * T * d, g + n_train * T * d, n_b, n_val, T, d, scale, Mg, n_train, b0 == 0, R,
+                                 pre_scale, divisor, accumulate, static_cast<__nv_bfloat16*>(out), ds, st);
+}
+
+}  // namespace gb
+
+extern "C" int ghost_embedding_pass(const long long* ids, const void* G, int is_f32, int n_train, int n_val, long long T,
+                                    int d, int vocab, float scale, float* M_out, float pre_scale, float divisor,
+                                    int accumulate, void* grad_out, void* ws, long long ws_bytes, void* stream) {
+  const DeviceState* ds = device_state();
+  if (!ds) return GHOST_ERR_DEVICE;
+  GB_REQUIRE(ids && G && ws && (M_out || grad_out), "ghost_embedding_pass: null pointer");
+  GB_REQUIRE(n_train > 0, "No training samples to compute dot product, check batch sizes.");
+  GB_REQUIRE(T > 0 && d > 0 && vocab > 0 && (n_val > 0 || M_out == nullptr), "ghost_embedding_pass: bad dimensions");
+  if (M_out == nullptr) n_val = 0;
+  GB_REQUIRE((static_cast<long long>(n_train) + n_val) * T < INT_MAX, "ghost_embedding_pass: too many tokens");
+  GB_REQUIRE(n_val <= 8192, "ghost_embedding_pass: at most 8192 validation samples");
+  GB_REQUIRE(grad_out == nullptr || divisor != 0.f, "ghost_embedding_pass: divisor must be non-zero");
+  GB_REQUIRE(ws_bytes >= ghost_embedding_pass_workspace_bytes(n_train, n_val, T, vocab, M_out ? d : 0),
+             "ghost_embedding_pass: workspace too small");
+  return emb_pass_group(ids, G, is_f32, n_train, 0, n_train, n_val, T, d, vocab, scale, M_out, pre_scale, divisor, accumulate,
+                        grad_out, ws, ds, static_cast<cudaStream_t>(stream));
+}
+
+// Room for the join with the train samples in groups of at least 32 (all of them at once in most batches)
+static int emb_dot_group(int n_val) { return n_val > 32 ? n_val : 32; }
+extern "C" long long ghost_embedding_dot_workspace_bytes_for(int n_val, long long T, int vocab, int d) {
+  return ghost_embedding_pass_workspace_bytes(emb_dot_group(n_val), n_val, T, vocab, d);
+}
+
+extern "C" int ghost_embedding_wgrad(const long long* ids, const void* G, int is_f32, int n_train, long long T,
+                                     int d, int vocab, float pre_scale, float divisor, int accumulate,
+                                     void* out, void* ws, long long ws_bytes, void* stream) {
+  GB_REQUIRE(ids && G && out && ws, "ghost_embedding_wgrad: null pointer");
+  return ghost_embedding_pass(ids, G, is_f32, n_train, 0, T, d, vocab, 1.f, nullptr, pre_scale, divisor, accumulate, out, ws,
+                              ws_bytes, stream);
 }
 
 extern "C" int ghost_embedding_dot(const long long* ids, const void* G, int is_f32, int n_train, int n_val,
@@ -530,107 +903,37 @@ extern "C" int ghost_embedding_dot(const long long* ids, const void* G, int is_f
   GB_REQUIRE(n_val <= 8192, "ghost_embedding_dot: at most 8192 validation samples");
   GB_REQUIRE(ws_bytes >= ghost_embedding_dot_workspace_bytes(n_val, T, vocab), "ghost_embedding_dot: workspace too small");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  // as many train samples at a time as the workspace has room for, in groups of 32 and more
+  int group = n_train;
+  auto fits = [&](int g) {
+    return (static_cast<long long>(g) + n_val) * T < INT_MAX && ws_bytes >= ghost_embedding_pass_workspace_bytes(g, n_val, T, vocab, d);
+  };
+  while (group > emb_dot_group(n_val) && !fits(group)) group = (group + 1) / 2 > emb_dot_group(n_val) ? (group + 1) / 2 : emb_dot_group(n_val);
+  if (fits(group)) {
+    for (int b0 = 0; b0 < n_train; b0 += group) {
+      const int rc = emb_pass_group(ids, G, is_f32, n_train, b0, n_train - b0 < group ? n_train - b0 : group, n_val, T, d, vocab,
+                                    scale, M_out, 1.f, 1.f, 0, nullptr, ws, ds, st);
+      if (rc != GHOST_OK) return rc;
+    }
+    return GHOST_OK;
+  }
   int* head = static_cast<int*>(ws);
   int* next = reinterpret_cast<int*>(static_cast<uint8_t*>(ws) + up256(4ll * vocab));
   const long long n_vtok = static_cast<long long>(n_val) * T;
-  // the repeated-id path needs the larger workspace (ghost_embedding_dot_workspace_bytes_for)
-  const bool hot = ws_bytes >= ghost_embedding_dot_workspace_bytes_for(n_val, T, vocab, d);
-  uint8_t* extra = static_cast<uint8_t*>(ws) + emb_dot_min_bytes(n_val, T, vocab);
-  int* cnt = hot ? reinterpret_cast<int*>(extra) : nullptr;
-  int* n_hot = hot ? reinterpret_cast<int*>(extra + up256(4ll * vocab)) : nullptr;
-  float* R = hot ? reinterpret_cast<float*>(extra + up256(4ll * vocab) + 256) : nullptr;
-  if (hot) GB_CUDA_OK(cudaMemsetAsync(cnt, 0, up256(4ll * vocab) + 256, st));
   GB_CUDA_OK(cudaMemsetAsync(head, 0xFF, 4ull * vocab, st));
   GB_CUDA_OK(cudaMemsetAsync(M_out, 0, sizeof(float) * static_cast<size_t>(n_val) * n_train, st));
   int blocks = static_cast<int>((n_vtok + 255) / 256);
   if (blocks > ds->sm_count * 8) blocks = ds->sm_count * 8;
-  emb_chain_val_kernel<<<blocks, 256, 0, st>>>(ids + static_cast<long long>(n_train) * T, n_vtok, vocab, head, next, cnt, ds->err_word);
-  count_launch();
-  int rc = post_launch("emb_chain_val_kernel");
-  if (rc != GHOST_OK) return rc;
-  if (hot) {
-    // chains longer than four dot products per validation sample are worth summing up front
-    const int threshold = 4 * n_val > 16 ? 4 * n_val : 16;
-    if (n_vtok > threshold) {
-      GB_CUDA_OK(cudaMemsetAsync(R, 0, 4ull * kEmbHotCap * static_cast<size_t>(n_val) * d, st));
-      int vb = ceil_div(vocab, 256);
-      if (vb > ds->sm_count * 4) vb = ds->sm_count * 4;
-      emb_hot_assign_kernel<<<vb, 256, 0, st>>>(cnt, vocab, threshold, kEmbHotCap, n_hot);
-      int rb = static_cast<int>((n_vtok + 7) / 8);
-      if (rb > ds->sm_count * 8) rb = ds->sm_count * 8;
-      const long long* ids_val = ids + static_cast<long long>(n_train) * T;
-      if (is_f32)
-        emb_hot_reduce_kernel<float><<<rb, 256, 0, st>>>(ids_val, static_cast<const float*>(G) + static_cast<long long>(n_train) * T * d, n_vtok, T, d, n_val, vocab, cnt, R);
-      else
-        emb_hot_reduce_kernel<__nv_bfloat16><<<rb, 256, 0, st>>>(ids_val, static_cast<const __nv_bfloat16*>(G) + static_cast<long long>(n_train) * T * d, n_vtok, T, d, n_val, vocab, cnt, R);
-      count_launch(2);
-      if ((rc = post_launch("emb_hot_reduce_kernel")) != GHOST_OK) return rc;
-    }
-  }
+  emb_chain_val_kernel<<<blocks, 256, 0, st>>>(ids + static_cast<long long>(n_train) * T, n_vtok, vocab, head, next, ds->err_word);
   const int tok_per_block = 64;
   dim3 grid(ceil_div(T, tok_per_block), n_train);
   const size_t smem = sizeof(float) * n_val;
   if (is_f32)
-    emb_dot_kernel<float><<<grid, 256, smem, st>>>(ids, static_cast<const float*>(G), n_train, n_val, T, d, vocab, head, next, cnt, R, scale, M_out, tok_per_block, ds->err_word);
+    emb_chain_dot_kernel<float><<<grid, 256, smem, st>>>(ids, static_cast<const float*>(G), n_train, n_val, T, d, vocab, head, next, scale, M_out, tok_per_block, ds->err_word);
   else
-    emb_dot_kernel<__nv_bfloat16><<<grid, 256, smem, st>>>(ids, static_cast<const __nv_bfloat16*>(G), n_train, n_val, T, d, vocab, head, next, cnt, R, scale, M_out, tok_per_block, ds->err_word);
-  count_launch();
-  return post_launch("emb_dot_kernel");
-}
-
-// counts, offsets, cursor ([vocab + 1] each), the token permutation, and the list of rows with more
-// than kEmbSmallBucket tokens (its counter in front)
-static long long emb_big_list_bytes(long long n_tok) { return up256(4ll * (n_tok / (kEmbSmallBucket + 1) + 2)); }
-extern "C" long long ghost_embedding_wgrad_workspace_bytes(int n_train, long long T, int vocab) {
-  return 3 * up256(4ll * (vocab + 1)) + up256(4ll * n_train * T) + emb_big_list_bytes(static_cast<long long>(n_train) * T);
-}
-
-extern "C" int ghost_embedding_wgrad(const long long* ids, const void* G, int is_f32, int n_train, long long T,
-                                     int d, int vocab, float pre_scale, float divisor, int accumulate,
-                                     void* out, void* ws, long long ws_bytes, void* stream) {
-  const DeviceState* ds = device_state();
-  if (!ds) return GHOST_ERR_DEVICE;
-  GB_REQUIRE(ids && G && out && ws, "ghost_embedding_wgrad: null pointer");
-  GB_REQUIRE(n_train > 0 && T > 0 && d > 0 && vocab > 0, "ghost_embedding_wgrad: bad dimensions");
-  GB_REQUIRE(static_cast<long long>(n_train) * T < INT_MAX, "ghost_embedding_wgrad: too many tokens");
-  GB_REQUIRE(divisor != 0.f, "ghost_embedding_wgrad: divisor must be non-zero");
-  GB_REQUIRE(ws_bytes >= ghost_embedding_wgrad_workspace_bytes(n_train, T, vocab), "ghost_embedding_wgrad: workspace too small");
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  uint8_t* w = static_cast<uint8_t*>(ws);
-  const long long seg = up256(4ll * (vocab + 1));
-  const long long n_tok = static_cast<long long>(n_train) * T;
-  // counts, cursor and the big-row counter sit next to each other: one memset clears them
-  int* counts = reinterpret_cast<int*>(w);
-  int* cursor = reinterpret_cast<int*>(w + seg);
-  int* n_big = reinterpret_cast<int*>(w + 2 * seg);
-  int* big = n_big + 1;
-  int* offsets = reinterpret_cast<int*>(w + 2 * seg + emb_big_list_bytes(n_tok));
-  int* perm = reinterpret_cast<int*>(w + 3 * seg + emb_big_list_bytes(n_tok));
-  GB_CUDA_OK(cudaMemsetAsync(counts, 0, 2 * seg + 4, st));
-  int blocks = static_cast<int>((n_tok + 255) / 256);
-  if (blocks > ds->sm_count * 8) blocks = ds->sm_count * 8;
-  emb_count_kernel<<<blocks, 256, 0, st>>>(ids, n_tok, vocab, counts, ds->err_word);
-  emb_scan_kernel<<<1, 1024, 0, st>>>(counts, vocab, offsets, big, n_big);
-  emb_fill_kernel<<<blocks, 256, 0, st>>>(ids, n_tok, vocab, offsets, cursor, perm);
-  // rows shared by many tokens: sorted in up to 128 KB of shared memory (32768 tokens), else in place
-  constexpr int kSmemCap = 32768;
-  static bool attr_set[64] = {};
-  if (!attr_set[ds->device]) {
-    GB_CUDA_OK(cudaFuncSetAttribute(emb_big_bucket_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemCap * 4));
-    GB_CUDA_OK(cudaFuncSetAttribute(emb_big_bucket_kernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemCap * 4));
-    attr_set[ds->device] = true;
-  }
-  long long big_max = n_tok / (kEmbSmallBucket + 1) + 1;
-  const int big_blocks = static_cast<int>(big_max < ds->sm_count ? big_max : ds->sm_count);
-  if (is_f32) {
-    emb_segsum_kernel<float><<<ceil_div(vocab, 8), 256, 0, st>>>(static_cast<const float*>(G), d, vocab, offsets, perm, pre_scale, divisor, accumulate, static_cast<float*>(out));
-    emb_big_bucket_kernel<float><<<big_blocks, 256, kSmemCap * 4, st>>>(static_cast<const float*>(G), d, offsets, perm, big, n_big, kSmemCap, pre_scale, divisor, accumulate, static_cast<float*>(out));
-  } else {
-    emb_segsum_kernel<__nv_bfloat16><<<ceil_div(vocab, 8), 256, 0, st>>>(static_cast<const __nv_bfloat16*>(G), d, vocab, offsets, perm, pre_scale, divisor, accumulate, static_cast<__nv_bfloat16*>(out));
-    emb_big_bucket_kernel<__nv_bfloat16><<<big_blocks, 256, kSmemCap * 4, st>>>(static_cast<const __nv_bfloat16*>(G), d, offsets, perm, big, n_big, kSmemCap, pre_scale, divisor, accumulate, static_cast<__nv_bfloat16*>(out));
-  }
-  count_launch(5);
-  return post_launch("ghost_embedding_wgrad");
+    emb_chain_dot_kernel<__nv_bfloat16><<<grid, 256, smem, st>>>(ids, static_cast<const __nv_bfloat16*>(G), n_train, n_val, T, d, vocab, head, next, scale, M_out, tok_per_block, ds->err_word);
+  count_launch(2);
+  return post_launch("emb_chain_dot_kernel");
 }
 
 // ------------------------------------------------------------------------------------------------

@@ -464,14 +464,38 @@ PyObject* py_embedding_dot(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (n_train <= 0) invalid("No training samples to compute dot product, check batch sizes.");
     Tensor M = empty({n_val, n_train}, G, at::kFloat);
     Workspace ws;
-    const long long ws_bytes = ghost_embedding_dot_workspace_bytes_for(static_cast<int>(n_val), T, static_cast<int>(vocab),
-                                                                       static_cast<int>(d));
+    const long long ws_bytes = ghost_embedding_pass_workspace_bytes(static_cast<int>(n_train), static_cast<int>(n_val), T,
+                                                                    static_cast<int>(vocab), static_cast<int>(d));
     const long long off = ws.plan(ws_bytes);
     char* base = ws.commit(L, G);
     check(ghost_embedding_dot(reinterpret_cast<const long long*>(ids.data_ptr()), G.data_ptr(), is_f32(G),
                               static_cast<int>(n_train), static_cast<int>(n_val), T, static_cast<int>(d),
                               static_cast<int>(vocab), real(a[4]), M.data_ptr<float>(), base + off, ws_bytes, L.st()));
     return wrap(M);
+  });
+}
+
+// dot products and train gradient in one pass: (ids, G, n_val, vocab, pre_scale) -> (M, grad in the dtype of G)
+PyObject* py_embedding_hook(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    need(n, 5, "embedding_hook");
+    const Tensor &ids0 = cuda_tensor(a[0]), &G0 = cuda_tensor(a[1]);
+    Launch L(G0);
+    const Tensor ids = ids2d(ids0), G = as3d(G0);
+    const long long N = G.size(0), T = G.size(1), d = G.size(2), n_val = integer(a[2]), vocab = integer(a[3]), n_train = N - n_val;
+    if (ids.size(0) != N || ids.size(1) != T) invalid("embedding ids and out-grad disagree on [batch, tokens]");
+    check_split(n_train, n_val, "embedding_hook");
+    Tensor M = empty({n_val, n_train}, G, at::kFloat), grad = empty({vocab, d}, G, G.scalar_type());
+    Workspace ws;
+    const long long ws_bytes = ghost_embedding_pass_workspace_bytes(static_cast<int>(n_train), static_cast<int>(n_val), T,
+                                                                    static_cast<int>(vocab), static_cast<int>(d));
+    const long long off = ws.plan(ws_bytes);
+    char* base = ws.commit(L, G);
+    check(ghost_embedding_pass(reinterpret_cast<const long long*>(ids.data_ptr()), G.data_ptr(), is_f32(G),
+                               static_cast<int>(n_train), static_cast<int>(n_val), T, static_cast<int>(d),
+                               static_cast<int>(vocab), 1.f, M.data_ptr<float>(), real(a[4]), static_cast<float>(n_train), 0,
+                               grad.data_ptr(), base + off, ws_bytes, L.st()));
+    return Py_BuildValue("(NN)", wrap(M), wrap(grad));
   });
 }
 
@@ -814,7 +838,7 @@ PyMethodDef kMethods[] = {
     GB_METHOD(gradproj_embedding), GB_METHOD(projection_similarity),
     GB_METHOD(pass_reduce),       GB_METHOD(matrix_sum),
     GB_METHOD(dense_hook),        GB_METHOD(norm_hook),
-    GB_METHOD(named_parameters),
+    GB_METHOD(embedding_hook),    GB_METHOD(named_parameters),
     GB_METHOD(arena_clear),       GB_METHOD(set_kernel_error),
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_ghost_torch", nullptr, -1, kMethods, nullptr, nullptr, nullptr, nullptr};

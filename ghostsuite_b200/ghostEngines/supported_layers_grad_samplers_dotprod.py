@@ -507,6 +507,14 @@ def _compute_embedding_dot_product(layer: nn.Embedding, A: torch.Tensor, B: torc
                                    val_batch_size: int):
     """nn.Embedding: id-equality-masked Gram of the out-grad rows (reference :181-211)."""
     _check_batch(A, B, val_batch_size)
+    own = layer.__dict__
+    if "_ghost_backprop_scale" in own and val_batch_size > 0 \
+            and getattr(layer.weight, "initially_requires_grad", layer.weight.requires_grad):
+        # inside a backward hook: the train gradient is asked for next and needs the same buckets
+        M, grad = ops.embedding_hook(A, B, val_batch_size, layer.weight.shape[0], own["_ghost_backprop_scale"])
+        own["_ghost_cached_train_grad"] = (A.data_ptr(), B.data_ptr(), A.size(0), grad)
+        _set_dot(layer.weight, M)
+        return
     M = ops.embedding_dot(A.detach(), B.detach(), val_batch_size, layer.weight.shape[0])
     _set_dot(layer.weight, M)
 
@@ -517,8 +525,11 @@ def _compute_embedding_train_grad(layer: nn.Embedding, A: torch.Tensor, B: torch
     n_train = A.size(0) - val_batch_size
     if n_train <= 0:
         return None
-    grad = ops.embedding_wgrad(A, B, n_train, layer.weight.shape[0], _backprop_scale(layer),
-                               float(n_train))
+    cached = layer.__dict__.pop("_ghost_cached_train_grad", None)
+    if cached is not None and cached[:3] == (A.data_ptr(), B.data_ptr(), A.size(0)):
+        grad = cached[3]
+    else:
+        grad = ops.embedding_wgrad(A, B, n_train, layer.weight.shape[0], _backprop_scale(layer), float(n_train))
     if grad.dtype != layer.weight.dtype:
         grad = grad.to(layer.weight.dtype)
     return grad

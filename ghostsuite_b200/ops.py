@@ -490,6 +490,17 @@ def embedding_wgrad(ids: torch.Tensor, G: torch.Tensor, n_train: int, vocab: int
         return _native().embedding_wgrad(*args)
 
 
+def embedding_hook(ids: torch.Tensor, G: torch.Tensor, n_val: int, vocab: int, pre_scale: float):
+    """:func:`embedding_dot` and :func:`embedding_wgrad` (divided by the train samples) from one set of
+    buckets: ``(M[n_val, n_train], train gradient [vocab, d] in the dtype of G)``."""
+    args = (ids, G, n_val, vocab, pre_scale)
+    if _timing is None:
+        return _native().embedding_hook(*args)
+    with _Timed("emb_join_kernel+emb_segsum_kernel", "hbm", 0.0,
+                (float(G.numel()) + float(vocab) * _cols(G)) * G.element_size() + 8.0 * ids.numel()):
+        return _native().embedding_hook(*args)
+
+
 # --------------------------------------------------------------------------------------------
 # GradProj
 # --------------------------------------------------------------------------------------------

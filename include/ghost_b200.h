@@ -244,12 +244,13 @@ int ghost_matrix_sum(const float* const* mats, int n_mats, int n_val, int n_trai
 
 /* ---- Embedding -------------------------------------------------------------------------------- */
 /* M[v,b] = scale * sum_{t,s : ids_b[t] == ids_v[s]} <G_b[t], G_v[s]>.  ids: int64 [N, T]; G: [N, T, d].
- * Validation tokens are chained per id; a train token walks the chain of its id.  The workspace
- * must hold at least ghost_embedding_dot_workspace_bytes (the chain tables).  With
- * ghost_embedding_dot_workspace_bytes_for or more, ids that more than max(16, 4 * n_val) validation
- * tokens share (padding, separators; up to 256 such ids) are first summed per (id, validation
- * sample), so a train token costs at most n_val dot products however often its id repeats; with the
- * smaller workspace the work is sum over ids of count_train(id) * count_val(id) * d.  An id
+ * Train and validation tokens are bucketed by id and joined id by id.  The workspace must hold at least
+ * ghost_embedding_dot_workspace_bytes: chain tables only, every train token then walks the
+ * validation tokens of its id, sum over ids of count_train(id) * count_val(id) * d work.  With
+ * ghost_embedding_dot_workspace_bytes_for or more the buckets fit (train samples in groups of 32 and
+ * more), and ids that more than max(8, 2 * n_val) validation tokens share (padding, separators; up to
+ * 256 such ids) are first summed per (id, validation sample), so a train token costs at most n_val
+ * dot products however often its id repeats.  An id
  * outside [0, vocab) contributes nothing and makes the next ghost_poll_kernel_error return
  * GHOST_ERR_INDEX.  Replaces ghostEngines/supported_layers_grad_samplers_dotprod.py:181-211. */
 long long ghost_embedding_dot_workspace_bytes(int n_val, long long T, int vocab);
@@ -276,6 +277,13 @@ long long ghost_embedding_wgrad_workspace_bytes(int n_train, long long T, int vo
 int ghost_embedding_wgrad(const long long* ids, const void* G, int is_f32, int n_train, long long T,
                           int d, int vocab, float pre_scale, float divisor, int accumulate, void* out,
                           void* ws, long long ws_bytes, void* stream);
+
+/* Both of the above from one set of buckets: the dot products if M_out != NULL (n_val may be 0 otherwise) and
+ * the averaged train gradient if grad_out != NULL, with the arguments they have there. */
+long long ghost_embedding_pass_workspace_bytes(int n_train, int n_val, long long T, int vocab, int d);
+int ghost_embedding_pass(const long long* ids, const void* G, int is_f32, int n_train, int n_val, long long T,
+                         int d, int vocab, float scale, float* M_out, float pre_scale, float divisor,
+                         int accumulate, void* grad_out, void* ws, long long ws_bytes, void* stream);
 
 /* ---- GradProj ------------------------------------------------------------------------------------ */
 /* out + b * out_stride <- scale * (G_b P_r^T)^T (A_b P_c^T), [k_r, k_c] fp32 row-major, for every

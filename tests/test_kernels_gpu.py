@@ -444,6 +444,24 @@ def test_embedding_with_heavily_repeated_ids(case, dtype):
     assert torch.equal(grad.cpu().float(), ref.float())
 
 
+# one call for both results, at the feature counts where a lane's share of a row changes (256, 512, 768,
+# 1024 and beyond, ragged), rows of one, 32, 33 and many tokens side by side, more hot ids than slots
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("case", [(3, 2, 40, 256, 9), (3, 2, 64, 264, 200), (2, 1, 70, 520, 33), (4, 3, 33, 768, 5),
+                                  (2, 2, 50, 776, 64), (3, 1, 37, 1032, 12), (2, 3, 45, 37, 20), (1, 1, 1, 8, 1),
+                                  (4, 2, 8000, 8, 300)])
+def test_embedding_hook(case, dtype):
+    n_t, n_v, T, d, vocab = case
+    N = n_t + n_v
+    g = torch.Generator().manual_seed(41)
+    ids = (torch.rand(N, T, generator=g).pow(2) * vocab).long().clamp_(max=vocab - 1)
+    G = (torch.randn(N, T, d, generator=g) / d ** 0.5).to(dtype)
+    M, grad = ops().embedding_hook(ids.cuda(), G.cuda(), n_v, vocab, float(N))
+    after()
+    assert O.rel_fro(M, O.embedding_dot_exact(ids, G, n_v)) < (1e-5 if dtype == torch.float32 else 1e-4)
+    assert torch.equal(grad.cpu().float(), O.embedding_train_grad(ids, G * N, n_v, vocab, sequential=True).float())
+
+
 def test_embedding_out_of_range_ids_are_reported():
     """An id outside the table makes the reference's index_add_ raise.  The kernels skip such a token
     and record it; the next poll of the error word raises IndexError."""
