@@ -218,22 +218,25 @@ struct EmbBuckets {
   int *off_b, *off_v;                   // [vocab] first position of the id's bucket in perm_b / perm_v
   int *rank;                            // [n_tok] position inside the bucket, -1 for an id outside the table
   int *perm_b, *perm_v;
-  int *totals;                          // [0] train tokens placed, [1] validation, [2] big rows, [3] items, [4] hot ids
+  int *totals;                          // [0] train tokens placed, [1] validation, [2] big rows, [3] items, [4] hot ids, [5] small rows
+  int4 *small;                          // (id, offset, tokens) of the rows with 1 to kEmbSmallBucket train tokens
   int *big;                             // ids with more than kEmbSmallBucket train tokens
   int2 *items;                          // (id, train chunk) pairs of the join
   int *slot;                            // [vocab] summed-row slot of a hot id, -1 otherwise
   int *hot;                             // ids by slot
-  int hot_threshold, want_big;
+  int hot_threshold, want_rows;         // want_rows: the train gradient is wanted, list its rows
   int* err;
 };
 
 constexpr int kEmbSmallBucket = 32;      // buckets up to this size are sorted and summed by one warp
 constexpr int kEmbHotCap = 256;
-constexpr int kEmbChunk = 32;            // train tokens of a join item
+constexpr int kEmbChunk = 8;             // train tokens of a join item
 
 // Counting hands every token its place in the bucket, so filling needs no second round of atomics.
-// It also clears M, which the join adds to two launches later.
-__global__ void __launch_bounds__(256) emb_count_kernel(const EmbBuckets q, float* __restrict__ M, long long m_size) {
+// It also clears M, which the join adds to two launches later, and zero-fills the gradient, most of
+// whose rows stay empty: the stores go out under the latency of the atomics.
+__global__ void __launch_bounds__(256) emb_count_kernel(const EmbBuckets q, float* __restrict__ M, long long m_size,
+                                                        uint4* __restrict__ zero, long long zero_size) {
   if (M != nullptr)
     for (long long i = blockIdx.x * 256ll + threadIdx.x; i < m_size; i += gridDim.x * 256ll) M[i] = 0.f;
   for (long long j = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; j < q.n_tok;
@@ -246,21 +249,23 @@ __global__ void __launch_bounds__(256) emb_count_kernel(const EmbBuckets q, floa
       atomicExch(q.err, kErrBadIndex);
     }
   }
+  const uint4 z = make_uint4(0u, 0u, 0u, 0u);
+  for (long long i = blockIdx.x * 256ll + threadIdx.x; i < zero_size; i += gridDim.x * 256ll) zero[i] = z;
 }
 
 // Buckets may lie in any order, so a block of ids takes its space with one atomic instead of waiting for
-// a scan over the whole table (22 us in one block for 50 k ids, 3 us now); the ids of a block stay in
-// ascending order, which the segment sum relies on.  Also listed here: rows for the big-bucket
-// kernel, join items, and ids that many validation tokens share (padding, separators).
+// a scan over the whole table (22 us in one block for 50 k ids, 4 us now).  Also listed here: the
+// gradient's rows by size, join items, and ids that many validation tokens share (padding, separators).
 __global__ void __launch_bounds__(256) emb_alloc_kernel(const EmbBuckets q) {
-  __shared__ int s_warp[2][8], s_base[2];
+  __shared__ int s_warp[3][8], s_base[3];
   const int id = blockIdx.x * 256 + threadIdx.x;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const bool in = id < q.vocab;
-  const int n[2] = {in ? q.cnt_b[id] : 0, in && q.cnt_v ? q.cnt_v[id] : 0};
-  int before[2];
+  const int tokens = in ? q.cnt_b[id] : 0;
+  const int n[3] = {tokens, in && q.cnt_v ? q.cnt_v[id] : 0, q.want_rows && tokens > 0 && tokens <= kEmbSmallBucket ? 1 : 0};
+  int before[3];
 #pragma unroll
-  for (int h = 0; h < 2; ++h) {
+  for (int h = 0; h < 3; ++h) {
     int x = n[h];
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -271,16 +276,18 @@ __global__ void __launch_bounds__(256) emb_alloc_kernel(const EmbBuckets q) {
     if (lane == 31) s_warp[h][warp] = x;
   }
   __syncthreads();
-  if (threadIdx.x < 2) {
+  if (threadIdx.x < 3) {
     int sum = 0;
 #pragma unroll
     for (int w = 0; w < 8; ++w) { const int c = s_warp[threadIdx.x][w]; s_warp[threadIdx.x][w] = sum; sum += c; }
-    s_base[threadIdx.x] = sum ? atomicAdd(q.totals + threadIdx.x, sum) : 0;
+    s_base[threadIdx.x] = sum ? atomicAdd(q.totals + (threadIdx.x == 2 ? 5 : threadIdx.x), sum) : 0;
   }
   __syncthreads();
   if (!in) return;
-  q.off_b[id] = s_base[0] + s_warp[0][warp] + before[0];
-  if (q.want_big && n[0] > kEmbSmallBucket) q.big[atomicAdd(q.totals + 2, 1)] = id;
+  const int off = s_base[0] + s_warp[0][warp] + before[0];
+  q.off_b[id] = off;
+  if (n[2]) q.small[s_base[2] + s_warp[2][warp] + before[2]] = make_int4(id, off, tokens, 0);
+  if (q.want_rows && n[0] > kEmbSmallBucket) q.big[atomicAdd(q.totals + 2, 1)] = id;
   if (q.cnt_v == nullptr) return;
   q.off_v[id] = s_base[1] + s_warp[1][warp] + before[1];
   int slot = -1;
@@ -392,11 +399,11 @@ template <typename E, int NCH> struct EmbLaneRow<E, NCH, false> {      // rows w
   }
 };
 
-// One join item per warp: up to 32 train rows of one id against the id's validation rows (or, for a hot
+// One join item per warp: up to eight train rows of one id against the id's validation rows (or, for a hot
 // id, one summed row per validation sample), VB validation rows held in registers at a time while the
-// train rows pass by with the next one's loads in flight.  Every row comes from HBM once; repeats hit
-// L1 / L2.  What bounds it is the products themselves (a fused multiply-add and its share of unpacking
-// per feature and pair).  Walking a chain per train token, the form before it, re-read the
+// train rows pass by with the next two's loads in flight.  Every row comes from HBM once; repeats hit
+// L1 / L2.  Items are small because ids are not: with 32 train rows an item, the few warps that drew the
+// frequent ids ran four times as long as the rest.  Walking a chain per train token, the form before it, re-read the
 // validation rows for every train token behind two dependent loads: 150 us against 26 for text ids
 // (40 x 1024 tokens of 768 bf16 features), 125 against 40 for position ids.
 template <typename T, int NCH, int VB, bool VEC>
@@ -442,17 +449,15 @@ emb_join_kernel(const EmbBuckets q, const T* __restrict__ Gb, const T* __restric
               r.get(y[u]);
             }
           }
-          EmbLaneRow<T, NCH, VEC> next;
-          int jb = __shfl_sync(0xffffffffu, my_b, 0);
-          next.load(Gb + static_cast<long long>(jb) * d, fc + lane * 8, d);
+          EmbLaneRow<T, NCH, VEC> next[2];             // train rows i + 1 and i + 2
+          next[0].load(Gb + static_cast<long long>(__shfl_sync(0xffffffffu, my_b, 0)) * d, fc + lane * 8, d);
+          next[1].load(Gb + static_cast<long long>(__shfl_sync(0xffffffffu, my_b, nb > 1 ? 1 : 0)) * d, fc + lane * 8, d);
           for (int i = 0; i < nb; ++i) {
-            const int b = jb / Tn;
+            const int b = __shfl_sync(0xffffffffu, my_b, i) / Tn;
             float x[NCH * 8];
-            next.get(x);
-            if (i + 1 < nb) {
-              jb = __shfl_sync(0xffffffffu, my_b, i + 1);
-              next.load(Gb + static_cast<long long>(jb) * d, fc + lane * 8, d);
-            }
+            next[0].get(x);
+            next[0] = next[1];
+            if (i + 2 < nb) next[1].load(Gb + static_cast<long long>(__shfl_sync(0xffffffffu, my_b, i + 2)) * d, fc + lane * 8, d);
             float s[VB];
 #pragma unroll
             for (int u = 0; u < VB; ++u) s[u] = 0.f;
@@ -500,83 +505,53 @@ emb_join_kernel(const EmbBuckets q, const T* __restrict__ Gb, const T* __restric
 }
 
 // ---------------------------------------------------------------- train gradient
-// Ascending-order float32 segment sum of the buckets of up to 32 tokens, dtype rounding as the reference.
-// A warp takes eight consecutive table rows, whose buckets lie one after the other: their sizes, their
-// token lists and the loads of their first eight (256-feature step, token) units are each one round of
-// memory latency for all eight rows, where a warp per row went through offsets, tokens, loads and
-// store with one or two rows' bytes in flight.  The (row, token) pairs of a group of rows with up to 32
-// tokens are put in order by one bitonic network.  Rows without tokens are zero-filled on the way.
-// Larger buckets are left to emb_big_bucket_kernel.
-constexpr int kEmbRowsPerWarp = 8;
-constexpr int kEmbTokenBits = 28;        // a sort key is (row of the group, token); more tokens: one row at a time
-
+// One warp per listed table row (1 to 32 tokens): ascending-order float32 segment sum, dtype rounding as the
+// reference.  Empty rows were zero-filled by the counting kernel, so the chain per row is list entry,
+// token list, rows, store; the next entry is fetched a row ahead.  The work of a row is the list of
+// (256-feature step, token) units, step-major; the loads of eight units are issued before their rows are
+// added in order, so a row with one or two tokens has all its loads in flight at once.
 template <typename T>
 __global__ void __launch_bounds__(256, 3)
 emb_segsum_kernel(const EmbBuckets q, const T* __restrict__ G, int d, float pre_scale, float divisor, int accumulate,
                   T* __restrict__ out) {
   const int lane = threadIdx.x & 31;
-  const int k0 = (blockIdx.x * 8 + (threadIdx.x >> 5)) * kEmbRowsPerWarp;
-  if (k0 >= q.vocab) return;
-  const int rows = min(kEmbRowsPerWarp, q.vocab - k0);
   const bool vec = (d % 8 == 0) && ((reinterpret_cast<uintptr_t>(G) & 15u) == 0) &&
                    ((reinterpret_cast<uintptr_t>(out) & 15u) == 0);
   const int steps = (d + 255) / 256;
-  const int my_cnt = lane < rows ? q.cnt_b[k0 + lane] : 0, my_off = lane < rows ? q.off_b[k0 + lane] : 0;
-  const bool wide_ids = q.first_val >= (1ll << kEmbTokenBits);
+  const int total = q.totals[5], stride = gridDim.x * 8;
   using Raw = typename EmbRaw<T>::type;
   constexpr int kBatch = sizeof(T) == 2 ? 8 : 4;      // 32 registers of loaded rows for either dtype
-
-  int r0 = 0;
-  while (r0 < rows) {
-    // rows [r0, r1): as many as fit 32 tokens together; zero rows are stored, big ones skipped
-    int n = 0, r1 = r0, row_of = 0, pos_in = 0, off_in = 0;
-    while (r1 < rows) {
-      int c = __shfl_sync(0xffffffffu, my_cnt, r1);
-      const int off = __shfl_sync(0xffffffffu, my_off, r1);
-      if (c > kEmbSmallBucket) c = 0;
-      else if (c == 0) {
-        const float zero[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-        for (int s = 0; s < steps; ++s) emb_store_row<T>(out, k0 + r1, d, s * 256 + lane * 8, vec, zero, divisor, accumulate);
-      } else {
-        if (n > 0 && (n + c > 32 || wide_ids)) break;
-        if (lane >= n && lane < n + c) { row_of = r1; pos_in = lane - n; off_in = off; }
-        n += c;
-      }
-      ++r1;
-    }
-    r0 = r1;
-    if (n == 0) continue;
-    int key = INT_MAX;
-    if (lane < n) key = q.perm_b[off_in + pos_in];
-    if (!wide_ids && lane < n) key |= row_of << kEmbTokenBits;
+  int w = blockIdx.x * 8 + (threadIdx.x >> 5);
+  int4 entry = w < total ? q.small[w] : make_int4(0, 0, 0, 0);
+  for (; w < total; w += stride) {
+    const int k = entry.x, off = entry.y, n = entry.z;
+    int tok = lane < n ? q.perm_b[off + lane] : INT_MAX;
+    if (w + stride < total) entry = q.small[w + stride];
     if (n > 1) {
+      // bitonic sort of 32 keys across the warp, ascending
 #pragma unroll
       for (int size = 2; size <= 32; size <<= 1) {
 #pragma unroll
-        for (int stride = size >> 1; stride > 0; stride >>= 1) {
-          const int other = __shfl_xor_sync(0xffffffffu, key, stride);
+        for (int stride2 = size >> 1; stride2 > 0; stride2 >>= 1) {
+          const int other = __shfl_xor_sync(0xffffffffu, tok, stride2);
           const bool up = ((lane & size) == 0);
-          const bool lower = ((lane & stride) == 0);
-          const int lo = min(key, other), hi = max(key, other);
-          key = (lower == up) ? lo : hi;
+          const bool lower = ((lane & stride2) == 0);
+          const int lo = min(tok, other), hi = max(tok, other);
+          tok = (lower == up) ? lo : hi;
         }
       }
     }
-    // the sort keeps rows together and in order, so lane i's row is still row_of
-    const int tok = wide_ids ? key : key & ((1 << kEmbTokenBits) - 1);
-    const int next_row = __shfl_down_sync(0xffffffffu, row_of, 1);
-    const unsigned ends = __ballot_sync(0xffffffffu, lane < n && (lane == n - 1 || next_row != row_of));
     const int units = steps * n;
     float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     int step = 0, i = 0;                   // unit -> (step, token), advanced without divisions
     auto finish_unit = [&]() {
-      const int row = __shfl_sync(0xffffffffu, row_of, i);
-      if ((ends >> i) & 1u) {              // last token of the row: write its 256 features
-        emb_store_row<T>(out, k0 + row, d, step * 256 + lane * 8, vec, acc, divisor, accumulate);
+      if (++i == n) {                      // last token of this step: write the row's 256 features
+        emb_store_row<T>(out, k, d, step * 256 + lane * 8, vec, acc, divisor, accumulate);
 #pragma unroll
         for (int e = 0; e < 8; ++e) acc[e] = 0.f;
+        i = 0;
+        ++step;
       }
-      if (++i == n) { i = 0; ++step; }
     };
     if (!vec) {                            // odd feature counts: one unit at a time
       for (int u = 0; u < units; ++u) {
@@ -617,13 +592,13 @@ emb_segsum_kernel(const EmbBuckets q, const T* __restrict__ G, int d, float pre_
 // features (128 bf16, 64 float32).  Ascending order comes from a bit map instead of a sort: the row's
 // tokens set bits of a window of 32768 tokens in shared memory, and prefix sums of the words' bit counts
 // turn the map into an ordered list.  The sum is sequential per feature (float addition in the CPU's
-// order), so its bound is the issue rate of one warp, eight instructions a token; a four-slot ring of
-// 32-row stages filled with cp.async keeps the rows arriving at that pace.  One CTA per row with a
+// order), so its bound is the issue rate of one warp, eight instructions a token; a three-slot ring of
+// 64-row stages filled with cp.async keeps the rows arriving at that pace.  One CTA per row with a
 // sorted list and eight rows in flight: 492 us for text ids (the longest row 1250 tokens), 18 us now.
 constexpr int kBigThreads = 128;
 constexpr int kBigWindow = 32768;        // tokens of a bit map: 1024 words, eight per thread
 constexpr int kBigList = 2048;           // list entries held at a time
-constexpr int kBigStage = 32, kBigSlots = 4;
+constexpr int kBigStage = 64, kBigSlots = 3;
 
 template <typename T>
 __global__ void __launch_bounds__(kBigThreads)
@@ -634,7 +609,8 @@ emb_big_bucket_kernel(const EmbBuckets q, const T* __restrict__ G, int d, int sl
   __shared__ unsigned s_map[kBigWindow / 32];
   __shared__ unsigned short s_list[kBigList];
   __shared__ int s_warp[kBigThreads / 32];
-  __shared__ __align__(16) T s_ring[kBigSlots][kBigStage][kFeat];
+  extern __shared__ __align__(16) unsigned char s_dyn[];
+  T (*s_ring)[kBigStage][kFeat] = reinterpret_cast<T (*)[kBigStage][kFeat]>(s_dyn);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int total = q.totals[2];
   const bool vec = (d % 8 == 0) && ((reinterpret_cast<uintptr_t>(G) & 15u) == 0);
@@ -650,6 +626,7 @@ emb_big_bucket_kernel(const EmbBuckets q, const T* __restrict__ G, int d, int sl
       __syncthreads();
       for (int i = tid; i < kBigWindow / 32; i += kBigThreads) s_map[i] = 0u;
       __syncthreads();
+#pragma unroll 4
       for (int i = tid; i < cnt; i += kBigThreads) {
         const long long j = q.perm_b[off + i] - win;
         if (j >= 0 && j < kBigWindow) atomicOr(&s_map[j >> 5], 1u << (j & 31));
@@ -757,7 +734,7 @@ extern "C" long long ghost_embedding_pass_workspace_bytes(int n_train, int n_val
   return up256(4ll * (2 * static_cast<long long>(vocab) + 8)) + 3 * up256(4ll * vocab)     // counts and totals; offsets, slots
          + up256(4ll * (tb + tv)) + up256(4ll * tb) + up256(4ll * tv)                      // rank, perm_b, perm_v
          + up256(4ll * (tb / (kEmbSmallBucket + 1) + 2)) + up256(8ll * (tb / kEmbChunk + vocab + 1)) +   // big rows, items
-         + up256(4ll * kEmbHotCap) + up256(4ll * kEmbHotCap * static_cast<long long>(n_val) * d);
+         + up256(4ll * kEmbHotCap) + up256(16ll * (vocab < tb ? vocab : tb)) + up256(4ll * kEmbHotCap * static_cast<long long>(n_val) * d);
 }
 extern "C" long long ghost_embedding_wgrad_workspace_bytes(int n_train, long long T, int vocab) {
   return ghost_embedding_pass_workspace_bytes(n_train, 0, T, vocab, 0);
@@ -770,7 +747,13 @@ static int emb_pass(const EmbBuckets& q, const T* Gb, const T* Gv, int n_train, 
                     float* M, long long pitch, bool clear_M, float* R, float pre_scale, float divisor, int accumulate, T* out, const DeviceState* ds, cudaStream_t st) {
   int blocks = static_cast<int>((q.n_tok + 255) / 256);
   if (blocks > ds->sm_count * 8) blocks = ds->sm_count * 8;
-  emb_count_kernel<<<blocks, 256, 0, st>>>(q, clear_M ? M : nullptr, n_val * pitch);
+  // the gradient is zero-filled by the counting kernel where 16-byte stores can (torch buffers always)
+  const long long out_bytes = static_cast<long long>(q.vocab) * d * static_cast<long long>(sizeof(T));
+  const bool fill = out != nullptr && !accumulate, quick = fill && out_bytes % 16 == 0 && (reinterpret_cast<uintptr_t>(out) & 15u) == 0;
+  if (fill && !quick) GB_CUDA_OK(cudaMemsetAsync(out, 0, out_bytes, st));
+  if (quick) blocks = ds->sm_count * 8;
+  emb_count_kernel<<<blocks, 256, 0, st>>>(q, clear_M ? M : nullptr, n_val * pitch, reinterpret_cast<uint4*>(out),
+                                           quick ? out_bytes / 16 : 0);
   emb_alloc_kernel<<<ceil_div(q.vocab, 256), 256, 0, st>>>(q);
   emb_fill_kernel<<<blocks, 256, 0, st>>>(q);
   count_launch(3);
@@ -800,11 +783,19 @@ static int emb_pass(const EmbBuckets& q, const T* Gb, const T* Gv, int n_train, 
     count_launch();
   }
   if (out != nullptr) {
-    emb_segsum_kernel<T><<<ceil_div(q.vocab, 8 * kEmbRowsPerWarp), 256, 0, st>>>(q, Gb, d, pre_scale, divisor, accumulate, out);
+    const long long rows = q.vocab < q.first_val ? q.vocab : q.first_val;      // at most one row per token
+    const int sb = static_cast<int>((rows + 7) / 8 < ds->sm_count * 3 ? (rows + 7) / 8 : ds->sm_count * 3);
+    emb_segsum_kernel<T><<<sb, 256, 0, st>>>(q, Gb, d, pre_scale, divisor, accumulate, out);
     const int slices = ceil_div(d, 256 / static_cast<int>(sizeof(T)));
     const long long most = (static_cast<long long>(n_train) * Tn / (kEmbSmallBucket + 1) + 1) * slices;
-    const int bb = static_cast<int>(most < ds->sm_count * 4 ? most : ds->sm_count * 4);
-    emb_big_bucket_kernel<T><<<bb, kBigThreads, 0, st>>>(q, Gb, d, slices, pre_scale, divisor, accumulate, out);
+    const int bb = static_cast<int>(most < ds->sm_count * 3 ? most : ds->sm_count * 3);
+    constexpr int kBigRing = kBigSlots * kBigStage * 256;
+    static bool attr_set[64] = {};
+    if (!attr_set[ds->device]) {
+      GB_CUDA_OK(cudaFuncSetAttribute(emb_big_bucket_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBigRing));
+      attr_set[ds->device] = true;
+    }
+    emb_big_bucket_kernel<T><<<bb, kBigThreads, kBigRing, st>>>(q, Gb, d, slices, pre_scale, divisor, accumulate, out);
     count_launch(2);
   }
   return post_launch("ghost_embedding_pass");
@@ -840,10 +831,11 @@ static int emb_pass_group(const long long* ids, const void* G, int is_f32, int n
   q.big = static_cast<int*>(take(4ll * (tb / (kEmbSmallBucket + 1) + 2)));
   q.items = static_cast<int2*>(take(8ll * (tb / kEmbChunk + vocab + 1)));
   q.hot = static_cast<int*>(take(4ll * kEmbHotCap));
+  q.small = static_cast<int4*>(take(16ll * (vocab < tb ? vocab : tb)));
   float* R = static_cast<float*>(take(4ll * kEmbHotCap * static_cast<long long>(n_val) * (M ? d : 0)));
   // a hot id costs n_val dot products per train token; worth it from twice as many validation tokens on
   q.hot_threshold = 2 * n_val > 8 ? 2 * n_val : 8;
-  q.want_big = out != nullptr;
+  q.want_rows = out != nullptr;
   q.err = ds->err_word;
   GB_CUDA_OK(cudaMemsetAsync(q.totals, 0, M ? zero_bytes : 4ll * (vocab + 8), st));
   float* Mg = M ? M + b0 : nullptr;
