@@ -8,8 +8,7 @@
 //   kEpiAccumulate  train-gradient recovery (ghostEngines/supported_layers_grad_samplers_dotprod.py
 //                   :168 and :502): contraction over all train tokens, optionally split across
 //                   CTAs; partial tiles are added into an fp32 workspace with red.global.add.
-//   kEpiStore       per-validation-sample weight gradients V[v] written to a workspace
-//                   (per-sample form of :133-134).
+//   kEpiDirect      the same with one CTA per tile: scaled, cast and stored to the result.
 //   kEpiStoreTiles  per-sample weight-gradient tiles (train and validation samples alike) written
 //                   tile-major as bf16 (fp32 for split fp32 inputs); tile_dot.cu then contracts
 //                   them into the [n_val, n_train] matrix and the train-gradient sum in one
@@ -23,10 +22,11 @@
 #include "common.cuh"
 #include "sm100_ptx.cuh"
 #include "xty_colsum.cuh"
+#include "xty_store.cuh"
 
 namespace gb {
 
-enum { kEpiAccumulate = 0, kEpiStore = 1, kEpiStoreTiles = 2 };
+enum { kEpiAccumulate = 0, kEpiDirect = 1, kEpiStoreTiles = 2 };
 
 struct XtyParams {
   int mode;
@@ -41,10 +41,11 @@ struct XtyParams {
   // kEpiAccumulate: fp32 [m_cols, ld_acc] accumulation workspace
   float* acc_ws;
   long long ld_acc;
-  // kEpiStore: row-major [sample][m_cols][ld_v]; kEpiStoreTiles: tile-major [tile][sample][128][256]
+  // kEpiDirect: the result [m_cols, n_cols]; kEpiStoreTiles: tile-major [tile][sample][128][256]
   void* vgrad;
-  long long ld_v;
   int v_is_f32;
+  float out_scale;           // kEpiDirect
+  int out_accumulate, out_vec;
   int sample_major;          // unit order (sample, tile), dealt round-robin to the CTAs; needs k_splits == 1
   // per-sample column sums of one operand (bias terms), taken by four extra warps that read the
   // operand rows through L2: 0 = none, 1 = X, 2 = Y; out [all samples, cols of that operand] fp32
@@ -290,30 +291,16 @@ xty_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant_
           if (m_ok && !empty_k)
             red_add_row32(p.acc_ws + static_cast<long long>(m) * p.ld_acc + n0 + c0, r, p.n_cols - (n0 + c0));
         }
-      } else if (p.mode == kEpiStore) {
-        const long long vbase = (static_cast<long long>(sample) * p.m_cols + m) * p.ld_v;
+      } else if (p.mode == kEpiDirect) {
 #pragma unroll 1
         for (int c0 = 0; c0 < BN; c0 += 32) {
-          if (n0 + c0 >= p.ld_v) break;
+          if (n0 + c0 >= p.n_cols) break;
           uint32_t r[32];
           tmem_ld32(t_acc + c0, r);
           tmem_ld_wait();
-          if (m_ok) {
-            // columns in [n_cols, ld_v) are written too (their accumulators are exact zeros from
-            // the TMA zero fill) so that the vector loads of the dot epilogue never see garbage
-            if (p.v_is_f32) {
-              float* dst = static_cast<float*>(p.vgrad) + vbase + n0 + c0;
-#pragma unroll
-              for (int j = 0; j < 32; ++j)
-                if (n0 + c0 + j < p.ld_v) dst[j] = empty_k ? 0.f : __uint_as_float(r[j]);
-            } else {
-              __nv_bfloat16* dst = static_cast<__nv_bfloat16*>(p.vgrad) + vbase + n0 + c0;
-#pragma unroll
-              for (int j = 0; j < 32; ++j)
-                if (n0 + c0 + j < p.ld_v)
-                  dst[j] = __float2bfloat16_rn(empty_k ? 0.f : __uint_as_float(r[j]));
-            }
-          }
+          if (m_ok)
+            store_grad_row32(p.vgrad, p.v_is_f32, p.out_accumulate, p.out_scale,
+                             static_cast<long long>(m) * p.n_cols + n0 + c0, r, p.n_cols - (n0 + c0), p.out_vec != 0);
         }
       } else {
         // kEpiStoreTiles: the whole 128 x 256 tile (zero padded), tile-major:
@@ -386,7 +373,8 @@ int launch_xty_pair_tiles(const void* X, const void* Y, long long n_samples_tota
                           int n_cols, long long ldx, long long ldy, int samples, int sample0, void* vgrad,
                           int v_is_f32, int colsum_of, float* colsum_out, const DeviceState* ds, cudaStream_t st);
 int launch_xty_pair_wgrad(const void* X, const void* Y, long long n_rows, int m_cols, int n_cols, long long ldx,
-                          long long ldy, float* acc_ws, long long ld_acc, const DeviceState* ds, cudaStream_t st);
+                          long long ldy, int splits, float* acc_ws, long long ld_acc, void* out, int out_is_f32,
+                          float scale, int accumulate, const DeviceState* ds, cudaStream_t st);
 bool xty_pair_usable(const DeviceState* ds);
 static int g_wgrad_pair_mode = 1;      // same meaning as below
 static int g_persample_pair_mode = 1;  // 0 off, 1 where no half of a pair would idle, 2 wherever applicable
@@ -490,31 +478,33 @@ extern "C" int ghost_wgrad_bf16(const void* X, const void* Y, long long n_rows, 
   p.T = n_rows;
   const int kb = ceil_div(n_rows, XtyCfg::BK);
   const int tiles = p.m_tiles * p.n_tiles;
-  // Split-K factor: the CTAs run ceil(units / SMs) rounds of (k-blocks per split + a fixed cost per
-  // unit for the accumulator hand-over and the red.add epilogue, measured at about 64 k-blocks' worth); take
-  // the factor with the shortest critical path.
-  int splits = 1;
-  long long best = -1;
-  for (int s = 1; s <= 64 && s <= kb; ++s) {
-    const long long units = static_cast<long long>(tiles) * s;
-    const long long rounds = (units + ds->sm_count - 1) / ds->sm_count;
-    const long long cost = rounds * (ceil_div(kb, s) + 64);
-    if (best < 0 || cost < best) { best = cost; splits = s; }
-  }
-  p.kb_per_split = ceil_div(kb, splits);
-  p.k_splits = ceil_div(kb, p.kb_per_split);
+  const double elems = static_cast<double>(m_cols) * n_cols;
   p.acc_ws = static_cast<float*>(ws);
   p.ld_acc = round_up(n_cols, 4);
+  p.vgrad = out;
+  p.v_is_f32 = out_is_f32;
+  p.out_scale = scale;
+  p.out_accumulate = accumulate;
+  p.out_vec = n_cols % 8 == 0 && (reinterpret_cast<uintptr_t>(out) & 15u) == 0;
   p.err = ds->err_word;
   CUtensorMap tx, ty;
   int rc;
   if ((rc = make_xty_maps(&tx, &ty, p, X, Y, 1, n_rows, ldx, ldy)) != GHOST_OK) return rc;
-  GB_CUDA_OK(cudaMemsetAsync(ws, 0, static_cast<size_t>(m_cols) * p.ld_acc * 4, st));
-  if (pair_kernel_fits(g_wgrad_pair_mode, m_cols, n_cols) && p.blocked_x && p.blocked_y && xty_pair_usable(ds))
-    rc = launch_xty_pair_wgrad(X, Y, n_rows, m_cols, n_cols, ldx, ldy, p.acc_ws, p.ld_acc, ds, st);
-  else
+  const bool pair = pair_kernel_fits(g_wgrad_pair_mode, m_cols, n_cols) && p.blocked_x && p.blocked_y && xty_pair_usable(ds);
+  const int splits = pair ? pick_k_splits(static_cast<long long>(ceil_div(m_cols, 256)) * p.n_tiles, ds->sm_count / 2,
+                                          ceil_div(n_rows, 128), 32, elems)
+                          : pick_k_splits(tiles, ds->sm_count, kb, 64, elems);
+  if (splits > 1) GB_CUDA_OK(cudaMemsetAsync(ws, 0, static_cast<size_t>(m_cols) * p.ld_acc * 4, st));
+  else p.mode = kEpiDirect;
+  if (pair) {
+    rc = launch_xty_pair_wgrad(X, Y, n_rows, m_cols, n_cols, ldx, ldy, splits, p.acc_ws, p.ld_acc, out, out_is_f32, scale,
+                               accumulate, ds, st);
+  } else {
+    p.kb_per_split = ceil_div(kb, splits);
+    p.k_splits = ceil_div(kb, p.kb_per_split);
     rc = launch_xty(tx, ty, p, ds, st);
-  if (rc != GHOST_OK) return rc;
+  }
+  if (rc != GHOST_OK || splits == 1) return rc;
   return finalize_xty(p.acc_ws, p.ld_acc, out, out_is_f32, m_cols, n_cols, scale, accumulate, st);
 }
 

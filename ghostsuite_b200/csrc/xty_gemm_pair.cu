@@ -16,7 +16,9 @@
 // Train-gradient pass (one "sample" holding all token rows): a unit is a 256 x 256 block and one of
 // k_splits ranges of 128-row blocks; units are walked split-major, so the pairs running at the same
 // time read the same token rows; every CTA adds its 128 x 256 half into the fp32 workspace with
-// red.global.add.v4.f32, exactly as the single-CTA kernel does.
+// red.global.add.v4.f32, exactly as the single-CTA kernel does.  With one split the CTA stores its half
+// to the result itself, scaled and cast: 11008 x 4096 over 32768 rows then spends no 250 us on zeroing
+// and rescaling a 180 MB workspace next to 2640 us of GEMM.
 //
 // Barriers: full[s] lives in the leader and collects the bytes of both CTAs' loads; empty[s] and
 // acc_full[a] exist in both CTAs and are signalled by the leader's tcgen05.commit to the pair;
@@ -26,6 +28,7 @@
 #include "common.cuh"
 #include "sm100_ptx.cuh"
 #include "xty_colsum.cuh"
+#include "xty_store.cuh"
 
 namespace gb {
 
@@ -38,7 +41,11 @@ struct XtyPairParams {
   void* vgrad;
   int v_is_f32;
   int tma_store;             // bf16 tiles: staged in shared memory and stored by the copy engine
-  int accumulate;            // 0: store tiles; 1: add into acc_ws ("samples" = k_splits, one real sample)
+  int accumulate;            // 0: store tiles; 1: add into acc_ws ("samples" = k_splits, one real sample);
+                             // 2: one split, stored to `out`
+  void* out;                 // [m_cols, n_cols]
+  int out_is_f32, out_accumulate, out_vec;
+  float out_scale;
   int kb_per_split;          // row blocks (BK tokens) per split (accumulate)
   float* acc_ws;             // [m_cols, ld_acc] fp32, zeroed by the host
   long long ld_acc;
@@ -266,7 +273,10 @@ xty_gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
           uint32_t r[32];
           tmem_ld32(t_acc + c0, r);
           tmem_ld_wait();
-          if (live)
+          if (live && p.accumulate == 2)
+            store_grad_row32(p.out, p.out_is_f32, p.out_accumulate, p.out_scale, static_cast<long long>(m) * p.n_cols + n0 + c0,
+                             r, p.n_cols - (n0 + c0), p.out_vec != 0);
+          else if (live)
             red_add_row32_pair(p.acc_ws + static_cast<long long>(m) * p.ld_acc + n0 + c0, r, p.n_cols - (n0 + c0));
         }
       } else if (tile128 < p.m_tiles128 && p.tma_store) {
@@ -418,6 +428,9 @@ int launch_xty_pair_tiles(const void* X, const void* Y, long long n_samples_tota
   const unsigned long long out_rows = static_cast<unsigned long long>(p.m_tiles128) * p.n_tiles * samples * Cfg::BM;
   p.tma_store = (!v_is_f32 && out_rows < (1ull << 31)) ? 1 : 0;
   p.accumulate = 0;
+  p.out = nullptr;
+  p.out_is_f32 = p.out_accumulate = p.out_vec = 0;
+  p.out_scale = 1.f;
   p.kb_per_split = 0;
   p.acc_ws = nullptr;
   p.ld_acc = 0;
@@ -445,11 +458,11 @@ int launch_xty_pair_tiles(const void* X, const void* Y, long long n_samples_tota
   return post_launch("xty_gemm_pair_kernel");
 }
 
-// Train-gradient pass: acc_ws[m_cols, ld_acc] (fp32, zeroed by the caller) += X^T Y over n_rows token
-// rows.  Both column counts are multiples of 64.
+// Train-gradient pass over n_rows token rows, both column counts multiples of 64: one split stores
+// scale * X^T Y to `out`, more of them add into acc_ws[m_cols, ld_acc] (fp32, zeroed by the caller).
 int launch_xty_pair_wgrad(const void* X, const void* Y, long long n_rows, int m_cols, int n_cols, long long ldx,
-                          long long ldy, float* acc_ws, long long ld_acc, const DeviceState* ds,
-                          cudaStream_t st) {
+                          long long ldy, int splits, float* acc_ws, long long ld_acc, void* out, int out_is_f32,
+                          float scale, int accumulate, const DeviceState* ds, cudaStream_t st) {
   using Cfg = XtyPairCfg;
   XtyPairParams p;
   p.m_cols = m_cols;
@@ -462,7 +475,12 @@ int launch_xty_pair_wgrad(const void* X, const void* Y, long long n_rows, int m_
   p.vgrad = nullptr;
   p.v_is_f32 = 0;
   p.tma_store = 0;
-  p.accumulate = 1;
+  p.accumulate = splits == 1 ? 2 : 1;
+  p.out = out;
+  p.out_is_f32 = out_is_f32;
+  p.out_accumulate = accumulate;
+  p.out_vec = (reinterpret_cast<uintptr_t>(out) & 15u) == 0;
+  p.out_scale = scale;
   p.acc_ws = acc_ws;
   p.ld_acc = ld_acc;
   p.cs_of = 0;
@@ -474,15 +492,6 @@ int launch_xty_pair_wgrad(const void* X, const void* Y, long long n_rows, int m_
   const long long pairs_max = ds->sm_count / 2;
   const int kb = static_cast<int>(ceil_div(n_rows, static_cast<long long>(Cfg::BK)));
   const long long blocks = static_cast<long long>(p.m_tiles) * p.n_tiles;
-  // Split-K factor with the shortest critical path: ceil(units / pairs) rounds of (row blocks per
-  // split + a fixed cost per unit for the accumulator hand-over and the red.add epilogue).
-  int splits = 1;
-  long long best = -1;
-  for (int s = 1; s <= 64 && s <= kb; ++s) {
-    const long long rounds = (blocks * s + pairs_max - 1) / pairs_max;
-    const long long cost = rounds * (ceil_div(kb, s) + 32);
-    if (best < 0 || cost < best) { best = cost; splits = s; }
-  }
   p.kb_per_split = ceil_div(kb, splits);
   p.samples = ceil_div(kb, p.kb_per_split);
   CUtensorMap tx, ty;

@@ -1,0 +1,63 @@
+// Direct store of a train gradient: 32 consecutive accumulator columns of one output row, scaled, cast to
+// the parameter dtype and written (or added) to the row-major result.  Used where no other CTA adds to
+// the same tile, so that neither the fp32 workspace nor the scaling pass over it is needed.
+#pragma once
+#include <cuda_bf16.h>
+#include <stdint.h>
+
+namespace gb {
+
+// `vec`: rows start on 16-byte boundaries, so whole groups of 32 columns go out as 16-byte stores
+__device__ __forceinline__ void store_grad_row32(void* out, int is_f32, int accumulate, float scale, long long at,
+                                                 const uint32_t (&r)[32], int ncol, bool vec) {
+  if (is_f32) {
+    float* o = static_cast<float*>(out) + at;
+    if (vec && ncol >= 32 && !accumulate) {
+#pragma unroll
+      for (int j = 0; j < 32; j += 4)
+        *reinterpret_cast<float4*>(o + j) = make_float4(__uint_as_float(r[j]) * scale, __uint_as_float(r[j + 1]) * scale,
+                                                        __uint_as_float(r[j + 2]) * scale, __uint_as_float(r[j + 3]) * scale);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 32; ++j)
+        if (j < ncol) o[j] = __uint_as_float(r[j]) * scale + (accumulate ? o[j] : 0.f);
+    }
+  } else {
+    __nv_bfloat16* o = static_cast<__nv_bfloat16*>(out) + at;
+    if (vec && ncol >= 32 && !accumulate) {
+#pragma unroll
+      for (int j = 0; j < 32; j += 8) {
+        uint32_t w[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const __nv_bfloat162 h = __floats2bfloat162_rn(__uint_as_float(r[j + 2 * e]) * scale, __uint_as_float(r[j + 2 * e + 1]) * scale);
+          w[e] = *reinterpret_cast<const uint32_t*>(&h);
+        }
+        *reinterpret_cast<uint4*>(o + j) = make_uint4(w[0], w[1], w[2], w[3]);
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < 32; ++j)
+        if (j < ncol) o[j] = __float2bfloat16_rn(__uint_as_float(r[j]) * scale + (accumulate ? __bfloat162float(o[j]) : 0.f));
+    }
+  }
+}
+
+// Split-K factor of a train-gradient pass with the shortest critical path, in units of one row block
+// of one tile (about 0.28 us on both kernels): ceil(units / workers) rounds of (row blocks per split + a
+// fixed cost per unit for the accumulator hand-over and the epilogue).  Splitting also pays for zeroing
+// the fp32 workspace and for the scaling pass: two launches (5 us) and ten bytes per weight element
+// at 5 TB/s; one split stores the result itself.  Fixed costs, measured: `add_cost` with red.add
+// into the workspace, a quarter of it with plain stores.
+inline int pick_k_splits(long long tiles, int workers, int kb, int add_cost, double weight_elems) {
+  int splits = 1;
+  double best = static_cast<double>((tiles + workers - 1) / workers) * (kb + add_cost / 4);
+  const double merge = (5.0 + weight_elems * 10.0 / 5e6) / 0.28;
+  for (int s = 2; s <= 64 && s <= kb; ++s) {
+    const double cost = static_cast<double>((tiles * s + workers - 1) / workers) * ((kb + s - 1) / s + add_cost) + merge;
+    if (cost < best) { best = cost; splits = s; }
+  }
+  return splits;
+}
+
+}  // namespace gb
