@@ -16,6 +16,7 @@
 #include <mutex>
 
 #include "common.cuh"
+#include "mma_sync.cuh"
 
 namespace gb {
 
@@ -221,16 +222,18 @@ struct EmbBuckets {
   int *totals;                          // [0] train tokens placed, [1] validation, [2] big rows, [3] items, [4] hot ids, [5] small rows
   int4 *small;                          // (id, offset, tokens) of the rows with 1 to kEmbSmallBucket train tokens
   int *big;                             // ids with more than kEmbSmallBucket train tokens
-  int2 *items;                          // (id, train chunk) pairs of the join
-  int *slot;                            // [vocab] summed-row slot of a hot id, -1 otherwise
+  int4 *items;                          // join items: (first train position, train rows, first validation position
+                                        // or slot, validation rows or -1 for the slot's summed rows)
   int *hot;                             // ids by slot
-  int hot_threshold, want_rows;         // want_rows: the train gradient is wanted, list its rows
+  long long max_items;
+  int hot_threshold, max_parts, want_rows;         // want_rows: the train gradient is wanted, list its rows
   int* err;
 };
 
 constexpr int kEmbSmallBucket = 32;      // buckets up to this size are sorted and summed by one warp
 constexpr int kEmbHotCap = 256;
-constexpr int kEmbChunk = 8;             // train tokens of a join item
+constexpr int kEmbChunk = 8;             // train rows of a join item
+constexpr int kEmbValChunk = 32;         // validation rows of a join item
 
 // Counting hands every token its place in the bucket, so filling needs no second round of atomics.
 // It also clears M, which the join adds to two launches later, and zero-fills the gradient, most of
@@ -289,18 +292,26 @@ __global__ void __launch_bounds__(256) emb_alloc_kernel(const EmbBuckets q) {
   if (n[2]) q.small[s_base[2] + s_warp[2][warp] + before[2]] = make_int4(id, off, tokens, 0);
   if (q.want_rows && n[0] > kEmbSmallBucket) q.big[atomicAdd(q.totals + 2, 1)] = id;
   if (q.cnt_v == nullptr) return;
-  q.off_v[id] = s_base[1] + s_warp[1][warp] + before[1];
+  const int off_v = s_base[1] + s_warp[1][warp] + before[1];
+  q.off_v[id] = off_v;
+  if (n[1] == 0 || n[0] == 0) return;
   int slot = -1;
-  if (n[1] > 0 && n[0] > 0) {
-    const int chunks = (n[0] + kEmbChunk - 1) / kEmbChunk;
-    const int at = atomicAdd(q.totals + 3, chunks);
-    for (int c = 0; c < chunks; ++c) q.items[at + c] = make_int2(id, c);
-    if (n[1] > q.hot_threshold) {
-      slot = atomicAdd(q.totals + 4, 1);
-      if (slot < kEmbHotCap) q.hot[slot] = id; else slot = -1;
-    }
+  if (n[1] > q.hot_threshold) {
+    slot = atomicAdd(q.totals + 4, 1);
+    if (slot < kEmbHotCap) q.hot[slot] = id; else slot = -1;
   }
-  q.slot[id] = slot;
+  const int chunks = (n[0] + kEmbChunk - 1) / kEmbChunk, parts = slot >= 0 ? 1 : (n[1] + kEmbValChunk - 1) / kEmbValChunk;
+  // more hot ids than slots: their long validation lists stay in one item per train chunk
+  const bool long_list = parts > q.max_parts;
+  int at = atomicAdd(q.totals + 3, chunks * (long_list ? 1 : parts));
+  for (int c = 0; c < chunks; ++c) {
+    const int b0 = off + c * kEmbChunk, nb = min(kEmbChunk, n[0] - c * kEmbChunk);
+    if (slot >= 0) q.items[at++] = make_int4(b0, nb, slot, -1);
+    else if (long_list) q.items[at++] = make_int4(b0, nb, off_v, n[1]);
+    else
+      for (int v = 0; v < parts; ++v)
+        q.items[at++] = make_int4(b0, nb, off_v + v * kEmbValChunk, min(kEmbValChunk, n[1] - v * kEmbValChunk));
+  }
 }
 
 __global__ void __launch_bounds__(256) emb_fill_kernel(const EmbBuckets q) {
@@ -368,136 +379,161 @@ emb_hot_reduce_kernel(const EmbBuckets q, const T* __restrict__ Gv, long long Tn
   }
 }
 
-// a lane's NCH groups of eight features (f0 + 256 * h) of one row, as loaded and as float32
-template <typename E, int NCH, bool VEC> struct EmbLaneRow {
-  typename EmbRaw<E>::type raw[NCH];
-  __device__ __forceinline__ void load(const E* row, int f0, int d) {
+// Eight consecutive contraction elements of one row as bf16x2 words: the values themselves for a bf16 row,
+// three parts (8 + 8 + 8 bits of the mantissa) for a float32 row, whose leading six products rebuild the
+// float32 product.
+template <typename E> struct EmbOct;
+template <> struct EmbOct<__nv_bfloat16> {
+  static constexpr int kParts = 1;
+  uint4 raw;
+  uint32_t w[1][4];
+  template <bool VEC> __device__ __forceinline__ void load(const __nv_bfloat16* row, int k, int d, bool ok) {
+    raw = make_uint4(0u, 0u, 0u, 0u);
+    if (!ok) return;
+    if (VEC) {
+      if (k < d) raw = __ldg(reinterpret_cast<const uint4*>(row + k));
+    } else {
+      __nv_bfloat16 v[8];
 #pragma unroll
-    for (int h = 0; h < NCH; ++h) raw[h] = f0 + h * 256 < d ? EmbRaw<E>::load(row + f0 + h * 256) : EmbRaw<E>::zero();
+      for (int e = 0; e < 8; ++e) v[e] = k + e < d ? row[k + e] : __float2bfloat16_rn(0.f);
+      raw = make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]), pack_bf16x2(v[6], v[7]));
+    }
   }
-  __device__ __forceinline__ void get(float (&x)[NCH * 8]) const {
+  __device__ __forceinline__ void split() { w[0][0] = raw.x; w[0][1] = raw.y; w[0][2] = raw.z; w[0][3] = raw.w; }
+};
+template <> struct EmbOct<float> {
+  static constexpr int kParts = 3;
+  float v[8];
+  uint32_t w[3][4];
+  template <bool VEC> __device__ __forceinline__ void load(const float* row, int k, int d, bool ok) {
 #pragma unroll
-    for (int h = 0; h < NCH; ++h) {
-      float t[8];
-      EmbRaw<E>::unpack(raw[h], t);
+    for (int e = 0; e < 8; ++e) v[e] = 0.f;
+    if (!ok) return;
+    if (VEC) {
+      if (k < d) {
+        *reinterpret_cast<float4*>(&v[0]) = __ldg(reinterpret_cast<const float4*>(row + k));
+        *reinterpret_cast<float4*>(&v[4]) = __ldg(reinterpret_cast<const float4*>(row + k + 4));
+      }
+    } else {
 #pragma unroll
-      for (int e = 0; e < 8; ++e) x[h * 8 + e] = t[e];
+      for (int e = 0; e < 8; ++e) if (k + e < d) v[e] = __ldg(row + k + e);
+    }
+  }
+  __device__ __forceinline__ void split() {
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+      float a = v[2 * h], b = v[2 * h + 1];
+#pragma unroll
+      for (int p = 0; p < 3; ++p) {
+        const __nv_bfloat16 x = __float2bfloat16_rn(a), y = __float2bfloat16_rn(b);
+        w[p][h] = pack_bf16x2(x, y);
+        a -= __bfloat162float(x);
+        b -= __bfloat162float(y);
+      }
     }
   }
 };
-template <typename E, int NCH> struct EmbLaneRow<E, NCH, false> {      // rows without 16-byte alignment
-  float v[NCH * 8];
-  __device__ __forceinline__ void load(const E* row, int f0, int d) {
-#pragma unroll
-    for (int h = 0; h < NCH; ++h)
-#pragma unroll
-      for (int e = 0; e < 8; ++e) v[h * 8 + e] = f0 + h * 256 + e < d ? ld_f32<E>(row + f0 + h * 256 + e) : 0.f;
-  }
-  __device__ __forceinline__ void get(float (&x)[NCH * 8]) const {
-#pragma unroll
-    for (int e = 0; e < NCH * 8; ++e) x[e] = v[e];
-  }
-};
 
-// One join item per warp: up to eight train rows of one id against the id's validation rows (or, for a hot
-// id, one summed row per validation sample), VB validation rows held in registers at a time while the
-// train rows pass by with the next two's loads in flight.  Every row comes from HBM once; repeats hit
-// L1 / L2.  Items are small because ids are not: with 32 train rows an item, the few warps that drew the
-// frequent ids ran four times as long as the rest.  Walking a chain per train token, the form before it, re-read the
-// validation rows for every train token behind two dependent loads: 150 us against 26 for text ids
-// (40 x 1024 tokens of 768 bf16 features), 125 against 40 for position ids.
-template <typename T, int NCH, int VB, bool VEC>
-__global__ void __launch_bounds__(128)
+// acc += 16 validation rows x 8 train rows over the whole row length; a lane supplies rows g and g + 8 of
+// the first operand, row g of the second, 8 of every 32 columns (the contraction order inside a
+// step is permuted alike for both).  The loads of kDepth steps are issued together.
+template <typename VT, typename BT, bool VEC>
+__device__ __forceinline__ void emb_mma_rows(const VT* va, const VT* vb, const BT* tr, bool va_ok, bool vb_ok, bool tr_ok,
+                                             int d, int c, float (&acc)[4]) {
+  constexpr int kDepth = (sizeof(VT) + 2 * sizeof(BT)) <= 6 ? 4 : 2;
+  for (int k0 = c * 8; k0 < (d + 31) / 32 * 32; k0 += 32 * kDepth) {
+    EmbOct<VT> a[kDepth], b[kDepth];
+    EmbOct<BT> t[kDepth];
+#pragma unroll
+    for (int s = 0; s < kDepth; ++s) {
+      a[s].template load<VEC>(va, k0 + 32 * s, d, va_ok);
+      b[s].template load<VEC>(vb, k0 + 32 * s, d, vb_ok);
+      t[s].template load<VEC>(tr, k0 + 32 * s, d, tr_ok);
+    }
+#pragma unroll
+    for (int s = 0; s < kDepth; ++s) {
+      a[s].split();
+      b[s].split();
+      t[s].split();
+#pragma unroll
+      for (int p = 0; p < EmbOct<VT>::kParts; ++p)
+#pragma unroll
+        for (int r = 0; r < EmbOct<BT>::kParts; ++r)
+          if (p + r <= 2) {
+            mma_16816(acc, a[s].w[p][0], b[s].w[p][0], a[s].w[p][1], b[s].w[p][1], t[s].w[r][0], t[s].w[r][1]);
+            mma_16816(acc, a[s].w[p][2], b[s].w[p][2], a[s].w[p][3], b[s].w[p][3], t[s].w[r][2], t[s].w[r][3]);
+          }
+    }
+  }
+}
+
+// One join item per warp: up to eight train rows of one id against up to 32 validation rows of it (or, for a
+// hot id, one summed row per validation sample), 16 at a time on mma.sync with fragments loaded
+// straight from global memory.  Rows come from HBM once; repeats hit L1 / L2.  What bounds it is the
+// latency of item -> token lists -> rows, so the kernel keeps registers low, items small (frequent ids
+// fall apart into many) and the next item's entry in flight.  Forms before it, for text ids (40 x 1024 tokens
+// of 768 bf16 features): a chain walk per train token, 150 us; validation rows in registers and
+// products on the CUDA cores, 80 us at eight warps per SM.
+template <typename T, bool VEC>
+__global__ void __launch_bounds__(256, 2)
 emb_join_kernel(const EmbBuckets q, const T* __restrict__ Gb, const T* __restrict__ Gv, int n_train, int n_val, int Tn, int d,
                 const float* __restrict__ R, float scale, float* __restrict__ M, long long pitch, int local) {
   extern __shared__ float s_M[];         // [n_val, n_train] when `local`
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int lane = threadIdx.x & 31, g = lane >> 2, c = lane & 3;
   if (local) {
-    for (int i = threadIdx.x; i < n_val * n_train; i += 128) s_M[i] = 0.f;
+    for (int i = threadIdx.x; i < n_val * n_train; i += 256) s_M[i] = 0.f;
     __syncthreads();
   }
   float* acc_M = local ? s_M : M;
   const long long acc_pitch = local ? n_train : pitch;
   const float out_scale = local ? 1.f : scale;
-  const int n_items = q.totals[3];
-  for (int it = blockIdx.x * 4 + warp; it < n_items; it += gridDim.x * 4) {
-    const int2 item = q.items[it];
-    const int id = item.x, slot = q.slot[id];
-    const int nb = min(kEmbChunk, q.cnt_b[id] - item.y * kEmbChunk);
-    const int cv = slot >= 0 ? n_val : q.cnt_v[id];
-    const int my_b = lane < nb ? q.perm_b[q.off_b[id] + item.y * kEmbChunk + lane] : 0;
-    for (int w0 = 0; w0 < cv; w0 += 32) {
-      const int nw = min(32, cv - w0);
-      const int my_v = slot >= 0 || lane >= nw ? 0 : q.perm_v[q.off_v[id] + w0 + lane];
-      for (int v0 = 0; v0 < nw; v0 += VB) {
-        int sample[VB];
-        for (int fc = 0; fc < d; fc += NCH * 256) {
-          float y[VB][NCH * 8];
+  const bool single = n_val == 1 && n_train == 1;
+  const int n_items = q.totals[3], stride = gridDim.x * 8;
+  int it = blockIdx.x * 8 + (threadIdx.x >> 5);
+  int4 item = it < n_items ? q.items[it] : make_int4(0, 0, 0, 0);
+  for (; it < n_items; it += stride) {
+    const int nb = item.y, at_v = item.z;
+    const bool hot = item.w < 0;
+    const int cv = hot ? n_val : item.w;
+    const int my_b = lane < nb ? q.perm_b[item.x + lane] : 0;
+    if (it + stride < n_items) item = q.items[it + stride];
+    const int jb = __shfl_sync(0xffffffffu, my_b, g);
+    const bool b_ok = g < nb;
+    const int col = my_b / Tn;             // lanes 0..7: train sample of row `lane`
+    const int b0 = __shfl_sync(0xffffffffu, col, 2 * c), b1 = __shfl_sync(0xffffffffu, col, 2 * c + 1);
+    for (int v0 = 0; v0 < cv; v0 += 16) {
+      const int r0 = v0 + g, r1 = v0 + g + 8;
+      const bool ok0 = r0 < cv, ok1 = r1 < cv;
+      float acc[4] = {0.f, 0.f, 0.f, 0.f};
+      int s0 = r0, s1 = r1;
+      if (hot) {
+        const float* base = R + static_cast<long long>(at_v) * n_val * d;
+        emb_mma_rows<float, T, VEC>(base + static_cast<long long>(ok0 ? r0 : 0) * d, base + static_cast<long long>(ok1 ? r1 : 0) * d,
+                                    Gb + static_cast<long long>(jb) * d, ok0, ok1, b_ok, d, c, acc);
+      } else {
+        const int j0 = ok0 ? q.perm_v[at_v + r0] : 0, j1 = ok1 ? q.perm_v[at_v + r1] : 0;
+        s0 = j0 / Tn;
+        s1 = j1 / Tn;
+        emb_mma_rows<T, T, VEC>(Gv + static_cast<long long>(j0) * d, Gv + static_cast<long long>(j1) * d,
+                                Gb + static_cast<long long>(jb) * d, ok0, ok1, b_ok, d, c, acc);
+      }
+      if (single) {                        // every entry belongs to the one pair
+        float s = (acc[0] + acc[1]) + (acc[2] + acc[3]);      // absent rows and columns are zero
 #pragma unroll
-          for (int u = 0; u < VB; ++u) {
-            const int vi = min(v0 + u, nw - 1);
-            const int jv = __shfl_sync(0xffffffffu, my_v, vi);
-            if (slot >= 0) {
-              sample[u] = w0 + vi;
-              EmbLaneRow<float, NCH, VEC> r;
-              r.load(R + (static_cast<long long>(slot) * n_val + w0 + vi) * d, fc + lane * 8, d);
-              r.get(y[u]);
-            } else {
-              sample[u] = jv / Tn;
-              EmbLaneRow<T, NCH, VEC> r;
-              r.load(Gv + static_cast<long long>(jv) * d, fc + lane * 8, d);
-              r.get(y[u]);
-            }
-          }
-          EmbLaneRow<T, NCH, VEC> next[2];             // train rows i + 1 and i + 2
-          next[0].load(Gb + static_cast<long long>(__shfl_sync(0xffffffffu, my_b, 0)) * d, fc + lane * 8, d);
-          next[1].load(Gb + static_cast<long long>(__shfl_sync(0xffffffffu, my_b, nb > 1 ? 1 : 0)) * d, fc + lane * 8, d);
-          for (int i = 0; i < nb; ++i) {
-            const int b = __shfl_sync(0xffffffffu, my_b, i) / Tn;
-            float x[NCH * 8];
-            next[0].get(x);
-            next[0] = next[1];
-            if (i + 2 < nb) next[1].load(Gb + static_cast<long long>(__shfl_sync(0xffffffffu, my_b, i + 2)) * d, fc + lane * 8, d);
-            float s[VB];
-#pragma unroll
-            for (int u = 0; u < VB; ++u) s[u] = 0.f;
-#pragma unroll
-            for (int e = 0; e < NCH * 8; ++e)
-#pragma unroll
-              for (int u = 0; u < VB; ++u) s[u] = fmaf(x[e], y[u][e], s[u]);
-            // halve the set of values with the distance: lane (u << (5 - log2 VB)) ends with row u's sum
-            int width = VB;
-#pragma unroll
-            for (int o = 16; o >= 1; o >>= 1) {
-              if (width > 1) {
-                width >>= 1;
-                const bool up = (lane & o) != 0;
-#pragma unroll
-                for (int u = 0; u < VB / 2; ++u)
-                  if (u < width) {
-                    const float send = up ? s[u] : s[u + width], keep = up ? s[u + width] : s[u];
-                    s[u] = keep + __shfl_xor_sync(0xffffffffu, send, o);
-                  }
-              } else {
-                s[0] += __shfl_xor_sync(0xffffffffu, s[0], o);
-              }
-            }
-            constexpr int kEvery = 32 / VB;
-            const int u = lane / kEvery;
-            if (lane % kEvery == 0 && v0 + u < nw) {
-              int sv = sample[0];
-#pragma unroll
-              for (int w = 1; w < VB; ++w) sv = u == w ? sample[w] : sv;
-              atomicAdd(acc_M + sv * acc_pitch + b, s[0] * out_scale);
-            }
-          }
-        }
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (lane == 0) atomicAdd(acc_M, s * out_scale);
+      } else {
+        const bool c0 = 2 * c < nb, c1 = 2 * c + 1 < nb;
+        if (ok0 && c0) atomicAdd(acc_M + s0 * acc_pitch + b0, acc[0] * out_scale);
+        if (ok0 && c1) atomicAdd(acc_M + s0 * acc_pitch + b1, acc[1] * out_scale);
+        if (ok1 && c0) atomicAdd(acc_M + s1 * acc_pitch + b0, acc[2] * out_scale);
+        if (ok1 && c1) atomicAdd(acc_M + s1 * acc_pitch + b1, acc[3] * out_scale);
       }
     }
   }
   if (local) {
     __syncthreads();
-    for (int i = threadIdx.x; i < n_val * n_train; i += 128) {
+    for (int i = threadIdx.x; i < n_val * n_train; i += 256) {
       const float s = s_M[i];
       if (s != 0.f) atomicAdd(M + i / n_train * pitch + i % n_train, s * scale);
     }
@@ -729,11 +765,17 @@ extern "C" long long ghost_embedding_dot_workspace_bytes(int n_val, long long T,
   return up256(4ll * vocab) + up256(4ll * n_val * T);
 }
 
+// Every id with tokens on both sides splits into train chunks times at most kEmbMaxParts validation parts.
+constexpr int kEmbMaxParts = 2;
+static long long emb_max_items(long long tb, int vocab) {
+  return kEmbMaxParts * (tb / kEmbChunk + (tb < vocab ? tb : vocab) + 1);
+}
+
 extern "C" long long ghost_embedding_pass_workspace_bytes(int n_train, int n_val, long long T, int vocab, int d) {
   const long long tb = static_cast<long long>(n_train) * T, tv = static_cast<long long>(n_val) * T;
-  return up256(4ll * (2 * static_cast<long long>(vocab) + 8)) + 3 * up256(4ll * vocab)     // counts and totals; offsets, slots
+  return up256(4ll * (2 * static_cast<long long>(vocab) + 8)) + 2 * up256(4ll * vocab)     // counts and totals; offsets
          + up256(4ll * (tb + tv)) + up256(4ll * tb) + up256(4ll * tv)                      // rank, perm_b, perm_v
-         + up256(4ll * (tb / (kEmbSmallBucket + 1) + 2)) + up256(8ll * (tb / kEmbChunk + vocab + 1)) +   // big rows, items
+         + up256(4ll * (tb / (kEmbSmallBucket + 1) + 2)) + up256(16ll * emb_max_items(tb, vocab))   // big rows, items
          + up256(4ll * kEmbHotCap) + up256(16ll * (vocab < tb ? vocab : tb)) + up256(4ll * kEmbHotCap * static_cast<long long>(n_val) * d);
 }
 extern "C" long long ghost_embedding_wgrad_workspace_bytes(int n_train, long long T, int vocab) {
@@ -768,18 +810,11 @@ static int emb_pass(const EmbBuckets& q, const T* Gb, const T* Gv, int n_train, 
     // a matrix of up to 16 KB is summed up in shared memory first: few, hot addresses otherwise
     const int local = static_cast<long long>(n_val) * n_train <= 4096 ? 1 : 0;
     const size_t smem = local ? sizeof(float) * n_val * n_train : 0;
-    long long most = (static_cast<long long>(n_train) * Tn / kEmbChunk + q.vocab + 1 + 3) / 4;
-    const int jb = static_cast<int>(most < ds->sm_count * 4 ? most : ds->sm_count * 4);
     const int Ti = static_cast<int>(Tn);
-    // register rows: the smallest number of 256-feature groups that covers d, at most four; four
-    // validation rows at a time where they fit the registers next to it
-#define GB_JOIN(NCH, VB, V) emb_join_kernel<T, NCH, VB, V><<<jb, 128, smem, st>>>(q, Gb, Gv, n_train, n_val, Ti, d, R, scale, M, pitch, local)
-    if (!vec) GB_JOIN(1, 4, false);
-    else if (d <= 256) GB_JOIN(1, 4, true);
-    else if (d <= 512) GB_JOIN(2, 4, true);
-    else if (d <= 768) GB_JOIN(3, 4, true);
-    else GB_JOIN(4, 2, true);
-#undef GB_JOIN
+    const long long most = (q.max_items + 7) / 8;
+    const int jb = static_cast<int>(most < ds->sm_count * 2 ? most : ds->sm_count * 2);
+    if (vec) emb_join_kernel<T, true><<<jb, 256, smem, st>>>(q, Gb, Gv, n_train, n_val, Ti, d, R, scale, M, pitch, local);
+    else emb_join_kernel<T, false><<<jb, 256, smem, st>>>(q, Gb, Gv, n_train, n_val, Ti, d, R, scale, M, pitch, local);
     count_launch();
   }
   if (out != nullptr) {
@@ -824,17 +859,19 @@ static int emb_pass_group(const long long* ids, const void* G, int is_f32, int n
   q.cnt_v = M ? q.cnt_b + vocab : nullptr;
   q.off_b = static_cast<int*>(take(4ll * vocab));
   q.off_v = static_cast<int*>(take(4ll * vocab));
-  q.slot = static_cast<int*>(take(4ll * vocab));
   q.rank = static_cast<int*>(take(4ll * (tb + tv)));
   q.perm_b = static_cast<int*>(take(4ll * tb));
   q.perm_v = static_cast<int*>(take(4ll * tv));
   q.big = static_cast<int*>(take(4ll * (tb / (kEmbSmallBucket + 1) + 2)));
-  q.items = static_cast<int2*>(take(8ll * (tb / kEmbChunk + vocab + 1)));
+  q.max_items = emb_max_items(tb, vocab);
+  q.items = static_cast<int4*>(take(16ll * q.max_items));
   q.hot = static_cast<int*>(take(4ll * kEmbHotCap));
   q.small = static_cast<int4*>(take(16ll * (vocab < tb ? vocab : tb)));
   float* R = static_cast<float*>(take(4ll * kEmbHotCap * static_cast<long long>(n_val) * (M ? d : 0)));
-  // a hot id costs n_val dot products per train token; worth it from twice as many validation tokens on
-  q.hot_threshold = 2 * n_val > 8 ? 2 * n_val : 8;
+  // A hot id costs n_val dot products per train token instead of one per validation token, after a pass over
+  // its validation rows; the products are cheap, so that pass pays from a few join items' worth on.
+  q.hot_threshold = 2 * n_val > kEmbMaxParts * kEmbValChunk ? 2 * n_val : kEmbMaxParts * kEmbValChunk;
+  q.max_parts = kEmbMaxParts;
   q.want_rows = out != nullptr;
   q.err = ds->err_word;
   GB_CUDA_OK(cudaMemsetAsync(q.totals, 0, M ? zero_bytes : 4ll * (vocab + 8), st));

@@ -63,6 +63,18 @@ int ghost_cast_split_bf16(const void* src, int src_is_f32, long long samples, lo
                           long long ld_src, void* dst, long long ld_dst, int cpad, int parts,
                           int kind0, int kind1, int kind2, int row_stack, void* stream);
 
+/* The same from a convolution operand: token (oy, ox) of sample n holds the C * kh * kw inputs of
+ * src [samples, C, H, W] (dense) under the kernel window, in the order of torch's unfold; tokens per
+ * sample are Ho * Wo of a convolution with strides (sy, sx), zero paddings (py, px) and dilations
+ * (dy, dx).  A 1 x 1 window turns an [N, p, Ho, Wo] out-grad into tokens.  Replaces the F.unfold of
+ * ghostEngines/supported_layers_grad_samplers_dotprod.py:513-592 and the casts after it. */
+int ghost_conv_tokens_bf16(const void* src, int src_is_f32, long long samples, int C, int H, int W, int kh,
+                           int kw, int sy, int sx, int py, int px, int dy, int dx, void* dst,
+                           long long ld_dst, int cpad, int parts, int kind0, int kind1, int kind2,
+                           int row_stack, void* stream);
+/* out[r] = sum_i x[r, i] of a dense [rows, len] matrix (fp32 sums): bias terms of a convolution. */
+int ghost_row_sums(const void* x, int is_f32, long long rows, long long len, float* out, void* stream);
+
 /* ---- Linear / Conv1D weight dot product, Gram ("ghost") path --------------------------------- */
 /* M[v,b] = scale * sum_{t in b, s in v} (a_train[t] . a_val[s]) * (g_train[t] . g_val[s]).
  * a_*: [n_* * T, ka] bf16, g_*: [n_* * T, kg] bf16.  round_mode 0: fp32 Gram entries multiplied in
@@ -248,7 +260,7 @@ int ghost_matrix_sum(const float* const* mats, int n_mats, int n_val, int n_trai
  * ghost_embedding_dot_workspace_bytes: chain tables only, every train token then walks the
  * validation tokens of its id, sum over ids of count_train(id) * count_val(id) * d work.  With
  * ghost_embedding_dot_workspace_bytes_for or more the buckets fit (train samples in groups of 32 and
- * more), and ids that more than max(8, 2 * n_val) validation tokens share (padding, separators; up to
+ * more), and ids that more than max(64, 2 * n_val) validation tokens share (padding, separators; up to
  * 256 such ids) are first summed per (id, validation sample), so a train token costs at most n_val
  * dot products however often its id repeats.  An id
  * outside [0, vocab) contributes nothing and makes the next ghost_poll_kernel_error return
