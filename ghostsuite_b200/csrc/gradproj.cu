@@ -14,6 +14,9 @@
 // single threads that drive the pipeline (a barrier wait, an expect-tx, the TMA and MMA issues --
 // each on the order of 100 cycles), hence wide stages and one multi-lane TMA instruction per stage.
 //
+// The embedding form (kEmb) has token ids in place of A: the rows of P_c^T are gathered by id straight into
+// the staged block, out[b] = scale * sum_t (P_r g_t)(P_c[:, id_t])^T, and only G is streamed.
+//
 // CTA layout (192 threads): warps 0-3 epilogue, warp 4 TMA producer, warp 5 MMA issuer.
 #include "common.cuh"
 #include "sm100_ptx.cuh"
@@ -33,6 +36,12 @@ struct GpParams {
   float scale;
   float* out;              // sample b at out + b * out_stride, [k_r, k_c] row-major
   long long out_stride;
+  int out_ld;              // pitch of an output row (k_c, or more inside a wider block)
+  // embedding form: token ids [B, T] and the rows that stand for A P_c^T, [vocab, >= k_c] fp32
+  const long long* ids;
+  const float* rows;
+  long long ld_rows;
+  int vocab, rows_vec;
   int* err;
 };
 
@@ -64,7 +73,7 @@ __device__ __forceinline__ int gp_staged_index(int row, int elem) {
   return row * KMAX + ((((elem >> 2) ^ row) & (KMAX / 4 - 1)) << 2) + (elem & 3);
 }
 
-template <int KMAX>
+template <int KMAX, bool kEmb>
 __global__ void __launch_bounds__(192, 1)
 gradproj_kernel(const __grid_constant__ CUtensorMap tm_g, const __grid_constant__ CUtensorMap tm_pr,
                 const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_pc,
@@ -91,7 +100,7 @@ gradproj_kernel(const __grid_constant__ CUtensorMap tm_g, const __grid_constant_
   long long u1 = u0 + p.units_per_cta + (bx < p.units_extra ? 1 : 0);
   if (u1 > p.units) u1 = p.units;
   const int kb_r = (p.n_r + ATOMS * BK - 1) / (ATOMS * BK);            // pipeline stages over G's columns
-  const int kb_total = kb_r + (p.n_c + ATOMS * BK - 1) / (ATOMS * BK);
+  const int kb_total = kEmb ? kb_r : kb_r + (p.n_c + ATOMS * BK - 1) / (ATOMS * BK);
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
@@ -101,7 +110,8 @@ gradproj_kernel(const __grid_constant__ CUtensorMap tm_g, const __grid_constant_
   }
   if (warp == 5) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
   if (warp == 4 && lane == 0) {
-    tma_prefetch_desc(&tm_g); tma_prefetch_desc(&tm_pr); tma_prefetch_desc(&tm_a); tma_prefetch_desc(&tm_pc);
+    tma_prefetch_desc(&tm_g); tma_prefetch_desc(&tm_pr);
+    if (!kEmb) { tma_prefetch_desc(&tm_a); tma_prefetch_desc(&tm_pc); }
   }
   tc_fence_before_sync();
   __syncthreads();
@@ -193,7 +203,7 @@ gradproj_kernel(const __grid_constant__ CUtensorMap tm_g, const __grid_constant_
         for (int j = 0; j < CT; ++j) {
           const int c = tx * CT + j;
           if (r < p.k_r && c < p.k_c && o[i][j] != 0.f)
-            atomicAdd(dst + static_cast<long long>(r) * p.k_c + c, o[i][j] * p.scale);
+            atomicAdd(dst + static_cast<long long>(r) * p.out_ld + c, o[i][j] * p.scale);
           o[i][j] = 0.f;
         }
       }
@@ -213,10 +223,37 @@ gradproj_kernel(const __grid_constant__ CUtensorMap tm_g, const __grid_constant_
       }
     };
 
+    // embedding form: row `tid` of the gathered block, fetched while the tensor core still works on the
+    // unit; a token past the end or with an id outside the table contributes zeros
+    constexpr int kRowQuads = kEmb ? KMAX / 4 : 1;
+    float4 mine[kRowQuads];
+    auto gather = [&](int b, long long t) {
+      long long id = -1;
+      if (t < p.T) {
+        id = p.ids[static_cast<long long>(b) * p.T + t];
+        if (id < 0 || id >= p.vocab) { id = -1; atomicExch(p.err, kErrBadIndex); }
+      }
+      const float* src = p.rows + (id < 0 ? 0 : id) * p.ld_rows;
+#pragma unroll
+      for (int q = 0; q < kRowQuads; ++q) {
+        mine[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (id < 0 || 4 * q >= p.k_c) continue;
+        if (p.rows_vec) {
+          mine[q] = __ldg(reinterpret_cast<const float4*>(src + 4 * q));
+        } else {
+          mine[q].x = __ldg(src + 4 * q);
+          if (4 * q + 1 < p.k_c) mine[q].y = __ldg(src + 4 * q + 1);
+          if (4 * q + 2 < p.k_c) mine[q].z = __ldg(src + 4 * q + 2);
+          if (4 * q + 3 < p.k_c) mine[q].w = __ldg(src + 4 * q + 3);
+        }
+      }
+    };
+
     bool alive = true;
     for (long long u = u0; u < u1; ++u) {
       const int b = static_cast<int>(u / p.chunks_per_sample);
       if (b != cur_b) { if (cur_b >= 0) flush(cur_b); cur_b = b; }
+      if constexpr (kEmb) gather(b, u % p.chunks_per_sample * BM + tid);
       if (!named_bar_and(2, 128, mbar_wait(&acc_full[acc], acc_phase, abort_flag, p.err, 124))) { alive = false; break; }
       tc_fence_after_sync();
       const uint32_t t_r = tmem_base + lane_base + acc * 256;
@@ -225,7 +262,13 @@ gradproj_kernel(const __grid_constant__ CUtensorMap tm_g, const __grid_constant_
       for (int half = 0; half < 2; ++half) {
         if ((warp >> 1) == half) {
           stage_block(t_r, p.kr_pad, s_r);
-          stage_block(t_r + 128, p.kc_pad, s_c);
+          if constexpr (kEmb) {
+#pragma unroll
+            for (int q = 0; q < kRowQuads; ++q)
+              *reinterpret_cast<float4*>(&s_c[gp_staged_index<KMAX>(tid & 63, 4 * q)]) = mine[q];
+          } else {
+            stage_block(t_r + 128, p.kc_pad, s_c);
+          }
           tc_fence_before_sync();
           __syncwarp();
           if (lane == 0) mbar_arrive(&acc_empty[acc]);     // four arrivals per tile, one per warp
@@ -262,21 +305,46 @@ gradproj_kernel(const __grid_constant__ CUtensorMap tm_g, const __grid_constant_
   if (warp == 5) { tc_fence_after_sync(); tmem_dealloc(tmem_base, 512); }
 }
 
-template <int KMAX>
+template <int KMAX, bool kEmb>
 static int launch_gradproj(const CUtensorMap& tg, const CUtensorMap& tpr, const CUtensorMap& ta,
                            const CUtensorMap& tpc, GpParams& p, const DeviceState* ds, cudaStream_t st) {
   using Cfg = GpCfg<KMAX>;
   static bool attr_set[64] = {};
   if (!attr_set[ds->device]) {
-    GB_CUDA_OK(cudaFuncSetAttribute(gradproj_kernel<KMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes));
+    GB_CUDA_OK(cudaFuncSetAttribute(gradproj_kernel<KMAX, kEmb>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes));
     attr_set[ds->device] = true;
   }
   const int grid = static_cast<int>(p.units < ds->sm_count ? p.units : ds->sm_count);
   p.units_per_cta = static_cast<int>(p.units / grid);
   p.units_extra = static_cast<int>(p.units % grid);
-  gradproj_kernel<KMAX><<<grid, 192, Cfg::kSmemBytes, st>>>(tg, tpr, ta, tpc, p);
+  gradproj_kernel<KMAX, kEmb><<<grid, 192, Cfg::kSmemBytes, st>>>(tg, tpr, ta, tpc, p);
   count_launch();
   return post_launch("gradproj_kernel");
+}
+
+// The embedding form for bf16 rows that TMA can read (proj_extras.cu holds the entry point and the
+// kernel for the rest).  16 x 2048 tokens of 1024 features, k = 32: bound by streaming G once.
+int launch_gradproj_embedding(const long long* ids, const void* G, int B, long long T, int d, long long ldg, const void* P_o,
+                              long long ldp_o, const float* P_i_t, long long ld_pit, int vocab, int k_o, int k_i, float scale,
+                              float* out, long long out_stride, int out_ld, const DeviceState* ds, cudaStream_t st) {
+  GpParams p = {};
+  p.B = B; p.T = T; p.n_r = d; p.n_c = 0; p.k_r = k_o; p.k_c = k_i;
+  p.kr_pad = (k_o + 15) / 16 * 16;
+  p.kc_pad = (k_i + 15) / 16 * 16;
+  p.chunks_per_sample = ceil_div(T, 128);
+  p.units = static_cast<long long>(B) * p.chunks_per_sample;
+  p.scale = scale;
+  p.out = out; p.out_stride = out_stride; p.out_ld = out_ld;
+  p.ids = ids; p.rows = P_i_t; p.ld_rows = ld_pit; p.vocab = vocab;
+  p.rows_vec = k_i % 4 == 0 && ld_pit % 4 == 0 && (reinterpret_cast<uintptr_t>(P_i_t) & 15u) == 0;
+  p.err = ds->err_word;
+  CUtensorMap tg, tp;
+  int rc;
+  if ((rc = make_tmap_bf16_3d(&tg, G, B, T, d, ldg, 128)) != GHOST_OK) return rc;
+  if ((rc = make_tmap_bf16_3d(&tp, P_o, 1, k_o, d, ldp_o, p.kr_pad)) != GHOST_OK) return rc;
+  const int kmax = p.kr_pad > p.kc_pad ? p.kr_pad : p.kc_pad;
+  if (kmax <= 32) return launch_gradproj<32, true>(tg, tp, tg, tp, p, ds, st);
+  return launch_gradproj<64, true>(tg, tp, tg, tp, p, ds, st);
 }
 
 }  // namespace gb
@@ -306,6 +374,7 @@ extern "C" int ghost_gradproj_dense_bf16(const void* G, const void* A, int B, lo
   p.scale = scale;
   p.out = out;
   p.out_stride = out_stride;
+  p.out_ld = k_c;
   p.err = ds->err_word;
   CUtensorMap tg, tpr, ta, tpc;
   int rc;
@@ -316,7 +385,7 @@ extern "C" int ghost_gradproj_dense_bf16(const void* G, const void* A, int B, lo
   if ((rc = make_tmap_bf16_3d(&tpc, P_c, 1, k_c, n_c, ldpc, p.kc_pad)) != GHOST_OK) return rc;
   GB_CUDA_OK(cudaMemset2DAsync(out, out_stride * sizeof(float), 0, static_cast<size_t>(k_r) * k_c * sizeof(float), B, st));
   const int kmax = p.kr_pad > p.kc_pad ? p.kr_pad : p.kc_pad;
-  if (kmax <= 32) return launch_gradproj<32>(tg, tpr, ta, tpc, p, ds, st);
-  if (kmax <= 64) return launch_gradproj<64>(tg, tpr, ta, tpc, p, ds, st);
-  return launch_gradproj<128>(tg, tpr, ta, tpc, p, ds, st);
+  if (kmax <= 32) return launch_gradproj<32, false>(tg, tpr, ta, tpc, p, ds, st);
+  if (kmax <= 64) return launch_gradproj<64, false>(tg, tpr, ta, tpc, p, ds, st);
+  return launch_gradproj<128, false>(tg, tpr, ta, tpc, p, ds, st);
 }

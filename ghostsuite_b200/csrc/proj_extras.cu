@@ -3,8 +3,9 @@
 //  * gradproj_embedding_kernel: per-sample projected gradient of an embedding table,
 //      out[b][o][i] = scale * sum_t (P_o g_bt)[o] * P_i[i, id_bt]
 //    (GhostSuite computes it with a Python loop over every token and one .item() host sync per
-//    token: ghostEngines/gradProjection/autograd_gradproj.py:167-222).  The out-grad rows are
-//    streamed once; P_o g_t for 16 tokens per warp runs on mma.sync with fragments loaded straight
+//    token: ghostEngines/gradProjection/autograd_gradproj.py:167-222).  bf16 rows that TMA can read
+//    go through gradproj.cu's tcgen05 pipeline; for float32 and unaligned rows this kernel streams
+//    the out-grad rows once; P_o g_t for 16 tokens per warp runs on mma.sync with fragments loaded straight
 //    from global memory, the k_o x k_i outer-product accumulation over a block of 64 tokens on the
 //    CUDA cores out of shared memory, where the gathered rows of P_i^T sit.
 //
@@ -175,67 +176,178 @@ struct SimParams {
   const void* P2;   // [n2, D], row pitch ld2
   int n1, n2;
   long long D, ld1, ld2;
+  long long per_cta;       // 32-element steps of the contraction a CTA covers
   float scale;
   float* S;         // [n1, ld_s]
   long long ld_s;
 };
 
-template <typename PT, bool VEC>
-__global__ void __launch_bounds__(256) proj_similarity_kernel(SimParams p) {
-  __shared__ float part[8][16 * 16];
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int g = lane >> 2, c = lane & 3;
-  const int i0 = blockIdx.y * 16, j0 = blockIdx.z * 16;
-  constexpr bool kSplit = sizeof(PT) == 4;
-  const PT* A = static_cast<const PT*>(p.P1);
-  const PT* Bm = static_cast<const PT*>(p.P2);
-  const bool a0_ok = i0 + g < p.n1, a1_ok = i0 + g + 8 < p.n1;
-  const bool b0_ok = j0 + g < p.n2, b1_ok = j0 + g + 8 < p.n2;
-  const PT* ar0 = A + static_cast<long long>(i0 + g) * p.ld1;
-  const PT* ar1 = A + static_cast<long long>(i0 + g + 8) * p.ld1;
-  const PT* br0 = Bm + static_cast<long long>(j0 + g) * p.ld2;
-  const PT* br1 = Bm + static_cast<long long>(j0 + g + 8) * p.ld2;
-
-  // every warp of the grid takes one contiguous range of 16-element blocks of the contraction
-  const long long nkb = (p.D + 15) / 16;
-  const long long warps = static_cast<long long>(gridDim.x) * 8;
-  const long long per = (nkb + warps - 1) / warps;
-  const long long w = static_cast<long long>(blockIdx.x) * 8 + warp;
-  const long long kb_lo = w * per;
-  const long long kb_hi = (kb_lo + per < nkb) ? kb_lo + per : nkb;
-
-  float acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-#pragma unroll 4
-  for (long long kb = kb_lo; kb < kb_hi; ++kb) {
-    const long long k = kb * 16 + 4 * c;
-    const Quad a0 = load_quad<VEC>(ar0, k, p.D, a0_ok);
-    const Quad a1 = load_quad<VEC>(ar1, k, p.D, a1_ok);
-    const Quad b0 = load_quad<VEC>(br0, k, p.D, b0_ok);
-    const Quad b1 = load_quad<VEC>(br1, k, p.D, b1_ok);
-    mma_16816(acc[0], a0.hi[0], a1.hi[0], a0.hi[1], a1.hi[1], b0.hi[0], b0.hi[1]);
-    mma_16816(acc[1], a0.hi[0], a1.hi[0], a0.hi[1], a1.hi[1], b1.hi[0], b1.hi[1]);
-    if (kSplit) {
-      mma_16816(acc[0], a0.lo[0], a1.lo[0], a0.lo[1], a1.lo[1], b0.hi[0], b0.hi[1]);
-      mma_16816(acc[1], a0.lo[0], a1.lo[0], a0.lo[1], a1.lo[1], b1.hi[0], b1.hi[1]);
-      mma_16816(acc[0], a0.hi[0], a1.hi[0], a0.hi[1], a1.hi[1], b0.lo[0], b0.lo[1]);
-      mma_16816(acc[1], a0.hi[0], a1.hi[0], a0.hi[1], a1.hi[1], b1.lo[0], b1.lo[1]);
+// Eight consecutive contraction elements of one row: hi parts, and lo parts for float rows
+template <typename PT, bool VEC> struct SimOct {
+  float v[sizeof(PT) == 4 ? 8 : 1];
+  uint4 raw;
+  __device__ __forceinline__ void load(const PT* row, long long k, long long d, bool ok) {
+    if constexpr (sizeof(PT) == 4) {
+      if (VEC) {
+        const bool in = ok && k < d;       // D % 8 == 0
+        const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+        *reinterpret_cast<float4*>(&v[0]) = in ? __ldg(reinterpret_cast<const float4*>(row + k)) : z;
+        *reinterpret_cast<float4*>(&v[4]) = in ? __ldg(reinterpret_cast<const float4*>(row + k + 4)) : z;
+      } else {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[e] = ok && k + e < d ? __ldg(row + k + e) : 0.f;
+      }
+    } else {
+      if (VEC) {
+        raw = ok && k < d ? __ldg(reinterpret_cast<const uint4*>(row + k)) : make_uint4(0u, 0u, 0u, 0u);
+      } else {
+        __nv_bfloat16 x[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) x[e] = ok && k + e < d ? row[k + e] : __float2bfloat16_rn(0.f);
+        raw = make_uint4(pack_bf16x2(x[0], x[1]), pack_bf16x2(x[2], x[3]), pack_bf16x2(x[4], x[5]), pack_bf16x2(x[6], x[7]));
+      }
     }
   }
-  // fragment -> [16][16]: n-tile j covers columns 8j .. 8j+7
+  __device__ __forceinline__ void parts(uint32_t (&hi)[4], uint32_t (&lo)[4]) const {
+    if constexpr (sizeof(PT) == 4) {
 #pragma unroll
-  for (int j = 0; j < 2; ++j) {
-    part[warp][g * 16 + 8 * j + 2 * c] = acc[j][0];
-    part[warp][g * 16 + 8 * j + 2 * c + 1] = acc[j][1];
-    part[warp][(g + 8) * 16 + 8 * j + 2 * c] = acc[j][2];
-    part[warp][(g + 8) * 16 + 8 * j + 2 * c + 1] = acc[j][3];
+      for (int h = 0; h < 4; ++h) {
+        const __nv_bfloat16 x = __float2bfloat16_rn(v[2 * h]), y = __float2bfloat16_rn(v[2 * h + 1]);
+        hi[h] = pack_bf16x2(x, y);
+        lo[h] = pack_bf16x2(__float2bfloat16_rn(v[2 * h] - __bfloat162float(x)), __float2bfloat16_rn(v[2 * h + 1] - __bfloat162float(y)));
+      }
+    } else {
+      hi[0] = raw.x; hi[1] = raw.y; hi[2] = raw.z; hi[3] = raw.w;
+    }
   }
-  __syncthreads();
-  float s = 0.f;
+};
+
+// A warp holds a (16 MT) x (8 NT) block of scores for every WK-th step of its CTA's range; WM x WN warps
+// tile the CTA's block and WK of them split its range, so operand rows are fetched once per block of up
+// to 64 x 64 scores (again from L2 / L1 for the next block and the neighbouring warps) instead of once
+// per 16 x 16.  All loads of a 32-element step go out together.
+template <typename PT, int MT, int NT, int WM, int WN, bool VEC>
+__global__ void __launch_bounds__(256) proj_similarity_kernel(const SimParams p) {
+  constexpr int WK = 8 / (WM * WN);
+  constexpr int BM = 16 * MT * WM, BN = 8 * NT * WN;
+  constexpr bool kSplit = sizeof(PT) == 4;
+  __shared__ float part[WK > 1 ? WK : 1][BM * BN / (WK > 1 ? 1 : BM * BN)];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int g = lane >> 2, c = lane & 3;
+  const int wk = warp / (WM * WN), wm = warp % (WM * WN) / WN, wn = warp % WN;
+  const int i0 = blockIdx.y * BM + wm * 16 * MT, j0 = blockIdx.z * BN + wn * 8 * NT;
+  const PT* A = static_cast<const PT*>(p.P1);
+  const PT* B = static_cast<const PT*>(p.P2);
+  const PT* ar[2 * MT];
+  const PT* br[NT];
 #pragma unroll
-  for (int ww = 0; ww < 8; ++ww) s += part[ww][tid];
-  const int i = i0 + (tid >> 4), j = j0 + (tid & 15);
-  if (i < p.n1 && j < p.n2 && s != 0.f) atomicAdd(p.S + static_cast<long long>(i) * p.ld_s + j, p.scale * s);
+  for (int m = 0; m < 2 * MT; ++m) ar[m] = A + static_cast<long long>(min(i0 + 8 * m + g, p.n1 - 1)) * p.ld1;
+#pragma unroll
+  for (int n = 0; n < NT; ++n) br[n] = B + static_cast<long long>(min(j0 + 8 * n + g, p.n2 - 1)) * p.ld2;
+
+  float acc[MT][NT][4];
+#pragma unroll
+  for (int m = 0; m < MT; ++m)
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[m][n][e] = 0.f;
+  const long long s0 = blockIdx.x * p.per_cta, steps = (p.D + 31) / 32;
+  const long long s1 = s0 + p.per_cta < steps ? s0 + p.per_cta : steps;
+  const bool some = i0 < p.n1 && j0 < p.n2;            // a warp whose whole block lies outside idles
+  // few rows per warp: several steps' loads in flight instead of one's
+  constexpr int kUnroll = 2 * MT + NT <= 4 ? 4 : 2 * MT + NT <= 6 ? 2 : 1;
+#pragma unroll kUnroll
+  for (long long s = s0 + wk; some && s < s1; s += WK) {
+    const long long k = s * 32 + 8 * c;
+    SimOct<PT, VEC> a[2 * MT], b[NT];
+#pragma unroll
+    for (int m = 0; m < 2 * MT; ++m) a[m].load(ar[m], k, p.D, true);
+#pragma unroll
+    for (int n = 0; n < NT; ++n) b[n].load(br[n], k, p.D, true);
+    uint32_t ah[2 * MT][4], al[2 * MT][4];
+#pragma unroll
+    for (int m = 0; m < 2 * MT; ++m) a[m].parts(ah[m], al[m]);
+#pragma unroll
+    for (int n = 0; n < NT; ++n) {
+      uint32_t bh[4], bl[4];
+      b[n].parts(bh, bl);
+#pragma unroll
+      for (int m = 0; m < MT; ++m)
+#pragma unroll
+        for (int h = 0; h < 4; h += 2) {
+          mma_16816(acc[m][n], ah[2 * m][h], ah[2 * m + 1][h], ah[2 * m][h + 1], ah[2 * m + 1][h + 1], bh[h], bh[h + 1]);
+          if (kSplit) {
+            mma_16816(acc[m][n], al[2 * m][h], al[2 * m + 1][h], al[2 * m][h + 1], al[2 * m + 1][h + 1], bh[h], bh[h + 1]);
+            mma_16816(acc[m][n], ah[2 * m][h], ah[2 * m + 1][h], ah[2 * m][h + 1], ah[2 * m + 1][h + 1], bl[h], bl[h + 1]);
+          }
+        }
+    }
+  }
+  auto add = [&](int i, int j, float v) {
+    if (i < p.n1 && j < p.n2) atomicAdd(p.S + static_cast<long long>(i) * p.ld_s + j, p.scale * v);
+  };
+  if constexpr (WK == 1) {
+    if (some) {
+#pragma unroll
+      for (int m = 0; m < MT; ++m)
+#pragma unroll
+        for (int n = 0; n < NT; ++n)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) add(i0 + 16 * m + g + 8 * (e >> 1), j0 + 8 * n + 2 * c + (e & 1), acc[m][n][e]);
+    }
+  } else {
+#pragma unroll
+    for (int m = 0; m < MT; ++m)
+#pragma unroll
+      for (int n = 0; n < NT; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          part[wk][(wm * 16 * MT + 16 * m + g + 8 * (e >> 1)) * BN + wn * 8 * NT + 8 * n + 2 * c + (e & 1)] = acc[m][n][e];
+    __syncthreads();
+    for (int e = threadIdx.x; e < BM * BN; e += 256) {
+      float v = 0.f;
+#pragma unroll
+      for (int w = 0; w < WK; ++w) v += part[w][e];
+      add(blockIdx.y * BM + e / BN, blockIdx.z * BN + e % BN, v);
+    }
+  }
 }
+
+template <typename PT, int MT, int NT, int WM, int WN>
+static int launch_similarity(SimParams p, bool vec, const DeviceState* ds, cudaStream_t st) {
+  const int bi = ceil_div(p.n1, 16 * MT * WM), bj = ceil_div(p.n2, 8 * NT * WN);
+  GB_REQUIRE(bi <= 65535 && bj <= 65535, "ghost_projection_similarity: too many rows");
+  // one wave of two CTAs per SM, but at least eight steps for each of a CTA's WK warps of a block
+  const long long steps = (p.D + 31) / 32;
+  long long splits = (2ll * ds->sm_count + bi * bj - 1) / (static_cast<long long>(bi) * bj);
+  const long long least = 8 * (8 / (WM * WN));
+  const long long most = (steps + least - 1) / least;
+  if (splits > most) splits = most;
+  if (splits < 1) splits = 1;
+  p.per_cta = (steps + splits - 1) / splits;
+  const dim3 grid(static_cast<unsigned>((steps + p.per_cta - 1) / p.per_cta), static_cast<unsigned>(bi), static_cast<unsigned>(bj));
+  if (vec) proj_similarity_kernel<PT, MT, NT, WM, WN, true><<<grid, 256, 0, st>>>(p);
+  else proj_similarity_kernel<PT, MT, NT, WM, WN, false><<<grid, 256, 0, st>>>(p);
+  count_launch();
+  return post_launch("proj_similarity_kernel");
+}
+
+// Block shape by row counts: the smallest that holds both sets, up to 64 x 64 scores
+template <typename PT>
+static int dispatch_similarity(const SimParams& p, bool vec, const DeviceState* ds, cudaStream_t st) {
+  if (p.n1 <= 16 && p.n2 <= 8) return launch_similarity<PT, 1, 1, 1, 1>(p, vec, ds, st);
+  if (p.n1 <= 16 && p.n2 <= 16) return launch_similarity<PT, 1, 2, 1, 1>(p, vec, ds, st);
+  if (p.n1 <= 16) return launch_similarity<PT, 1, 4, 1, 2>(p, vec, ds, st);
+  if (p.n1 <= 32 && p.n2 <= 32) return launch_similarity<PT, 2, 4, 1, 1>(p, vec, ds, st);
+  if (p.n2 <= 16) return launch_similarity<PT, 2, 2, 2, 1>(p, vec, ds, st);
+  return launch_similarity<PT, 2, 4, 2, 2>(p, vec, ds, st);
+}
+
+// gradproj.cu
+int launch_gradproj_embedding(const long long* ids, const void* G, int B, long long T, int d, long long ldg, const void* P_o,
+                              long long ldp_o, const float* P_i_t, long long ld_pit, int vocab, int k_o, int k_i, float scale,
+                              float* out, long long out_stride, int out_ld, const DeviceState* ds, cudaStream_t st);
 
 }  // namespace gb
 
@@ -272,6 +384,9 @@ extern "C" int ghost_gradproj_embedding(const long long* ids, const void* G, int
   p.P_o = static_cast<const __nv_bfloat16*>(P_o); p.ldp = ldp_o; p.cp = p_cols; p.lo_off = p_lo_offset;
   p.PiT = P_i_t; p.ld_pit = ld_pit; p.scale = scale; p.out = out; p.out_stride = out_stride; p.out_ld = out_ld;
   p.err = ds->err_word;
+  if (!g_is_f32 && d % 8 == 0 && ldg % 8 == 0 && (reinterpret_cast<uintptr_t>(G) & 15u) == 0 && T < (1ll << 31) - 128)
+    return launch_gradproj_embedding(ids, G, B, T, d, ldg, P_o, ldp_o, P_i_t, ld_pit, vocab, k_o, k_i, scale, out, out_stride,
+                                     out_ld, ds, st);
   const long long n_blocks = (T + kTokBlock - 1) / kTokBlock;
   long long splits = (2ll * ds->sm_count + B - 1) / B;
   if (splits > n_blocks) splits = n_blocks;
@@ -291,32 +406,14 @@ extern "C" int ghost_projection_similarity(const void* P1, const void* P2, int i
   GB_REQUIRE(P1 && P2 && S, "ghost_projection_similarity: null pointer");
   GB_REQUIRE(n1 > 0 && n2 > 0 && D > 0, "ghost_projection_similarity: empty dimension");
   GB_REQUIRE(ld1 >= D && ld2 >= D && ld_s >= n2, "ghost_projection_similarity: pitch smaller than the row it holds");
-  const int bi = (n1 + 15) / 16, bj = (n2 + 15) / 16;
-  GB_REQUIRE(bi <= 65535 && bj <= 65535, "ghost_projection_similarity: too many rows");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   GB_CUDA_OK(cudaMemset2DAsync(S, static_cast<size_t>(ld_s) * 4, 0, static_cast<size_t>(n2) * 4,
                                static_cast<size_t>(n1), st));
   SimParams p = {};
   p.P1 = P1; p.P2 = P2; p.n1 = n1; p.n2 = n2; p.D = D; p.ld1 = ld1; p.ld2 = ld2; p.scale = scale; p.S = S;
   p.ld_s = ld_s;
-  // enough CTAs to fill the GPU a few times over, but no warp with fewer than 8 blocks of 16 elements
-  const long long nkb = (D + 15) / 16;
-  long long splits = (4ll * ds->sm_count + bi * bj - 1) / (static_cast<long long>(bi) * bj);
-  const long long max_splits = (nkb + 63) / 64;
-  if (splits > max_splits) splits = max_splits;
-  if (splits < 1) splits = 1;
-  const dim3 grid(static_cast<unsigned>(splits), static_cast<unsigned>(bi), static_cast<unsigned>(bj));
   const int esize = is_f32 ? 4 : 2;
-  const bool vec = D % 4 == 0 && ld1 % 4 == 0 && ld2 % 4 == 0 &&
-                   (reinterpret_cast<uintptr_t>(P1) % (4 * esize)) == 0 &&
-                   (reinterpret_cast<uintptr_t>(P2) % (4 * esize)) == 0;
-  if (is_f32) {
-    if (vec) proj_similarity_kernel<float, true><<<grid, 256, 0, st>>>(p);
-    else proj_similarity_kernel<float, false><<<grid, 256, 0, st>>>(p);
-  } else {
-    if (vec) proj_similarity_kernel<__nv_bfloat16, true><<<grid, 256, 0, st>>>(p);
-    else proj_similarity_kernel<__nv_bfloat16, false><<<grid, 256, 0, st>>>(p);
-  }
-  count_launch();
-  return post_launch("proj_similarity_kernel");
+  const bool vec = D % 8 == 0 && (ld1 * esize) % 16 == 0 && (ld2 * esize) % 16 == 0 &&
+                   ((reinterpret_cast<uintptr_t>(P1) | reinterpret_cast<uintptr_t>(P2)) & 15u) == 0;
+  return is_f32 ? dispatch_similarity<float>(p, vec, ds, st) : dispatch_similarity<__nv_bfloat16>(p, vec, ds, st);
 }
