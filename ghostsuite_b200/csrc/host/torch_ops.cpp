@@ -168,13 +168,34 @@ constexpr int kSplitLeft[3] = {0, 1, 0};
 constexpr int kSplitRight[3] = {0, 0, 1};
 constexpr int kPlain[3] = {0, 0, 0};
 
-void cast(const Tensor& src, long long row0, long long samples, long long T, void* dst, long long ld_dst, long long cpad,
-          int parts, const int (&kinds)[3], bool row_stack, void* st) {
-  const long long cols = src.size(-1);
-  const char* p = static_cast<const char*>(src.data_ptr()) + row0 * cols * src.element_size();
-  check(ghost_cast_split_bf16(p, is_f32(src), samples, T, static_cast<int>(cols), cols, dst, ld_dst, static_cast<int>(cpad),
-                              parts, kinds[0], kinds[1], kinds[2], row_stack ? 1 : 0, st));
-}
+// An operand [N, T, cols] of the layer math: a tensor with exactly these dimensions, or a convolution
+// operand [N, C, H, W] whose tokens are the output positions.
+struct Conv { int C, H, W, kh, kw, sy, sx, py, px, dy, dx; };
+struct Operand {
+  const Tensor& t;
+  long long N, T, cols;
+  const Conv* conv;
+  explicit Operand(const Tensor& x) : t(x), N(x.size(0)), T(x.size(1)), cols(x.size(2)), conv(nullptr) {}
+  Operand(const Tensor& x, const Conv& c, long long tokens)
+      : t(x), N(x.size(0)), T(tokens), cols(static_cast<long long>(c.C) * c.kh * c.kw), conv(&c) {}
+  int f32() const { return is_f32(t); }
+  // readable as it is by the tensor-core entry points
+  bool ready() const { return conv == nullptr && tma_ready(t); }
+  // bf16 copy of samples [first, first + samples)
+  void cast(long long first, long long samples, void* dst, long long ld_dst, long long cpad, int parts, const int (&kinds)[3],
+            bool row_stack, void* st) const {
+    const long long per = conv ? static_cast<long long>(conv->C) * conv->H * conv->W : T * cols;
+    const char* p = static_cast<const char*>(t.data_ptr()) + first * per * t.element_size();
+    const int cp = static_cast<int>(cpad), stack = row_stack ? 1 : 0;
+    if (conv)
+      check(ghost_conv_tokens_bf16(p, f32(), samples, conv->C, conv->H, conv->W, conv->kh, conv->kw, conv->sy, conv->sx,
+                                   conv->py, conv->px, conv->dy, conv->dx, dst, ld_dst, cp, parts, kinds[0], kinds[1],
+                                   kinds[2], stack, st));
+    else
+      check(ghost_cast_split_bf16(p, f32(), samples, T, static_cast<int>(cols), cols, dst, ld_dst, cp, parts, kinds[0],
+                                  kinds[1], kinds[2], stack, st));
+  }
+};
 
 void check_split(long long n_train, long long n_val, const char* who) {
   if (n_train <= 0) invalid("No training samples to compute dot product, check batch sizes.");
@@ -182,41 +203,41 @@ void check_split(long long n_train, long long n_val, const char* who) {
 }
 
 // ---- Gram path -----------------------------------------------------------------------------------------
-Tensor gram_dot(const Launch& L, const Tensor& A, const Tensor& G, long long n_val, int round_mode, float scale) {
-  const long long N = A.size(0), T = A.size(1), n_train = N - n_val;
+Tensor gram_dot(const Launch& L, const Operand& A, const Operand& G, long long n_val, int round_mode, float scale) {
+  const long long N = A.N, T = A.T, n_train = N - n_val;
   check_split(n_train, n_val, "gram_dot");
-  if (G.size(0) != N || G.size(1) != T) invalid("gram_dot: activation and out-grad disagree on [batch, tokens]");
-  Tensor M = empty({n_val, n_train}, A, at::kFloat);
+  if (G.N != N || G.T != T) invalid("gram_dot: activation and out-grad disagree on [batch, tokens]");
+  Tensor M = empty({n_val, n_train}, A.t, at::kFloat);
   Workspace ws;
-  struct Op { int kind; long long cp, off_t, off_v; } op[2];      // kind 0 as it is, 1 padded copy, 2 split
-  const Tensor* xs[2] = {&A, &G};
+  struct Plan { int kind; long long cp, off_t, off_v; } op[2];      // kind 0 as it is, 1 padded copy, 2 split
+  const Operand* xs[2] = {&A, &G};
   for (int i = 0; i < 2; ++i) {
-    const Tensor& x = *xs[i];
-    const long long cp = pad8(x.size(-1));
-    if (is_f32(x)) {
+    const Operand& x = *xs[i];
+    const long long cp = pad8(x.cols);
+    if (x.f32()) {
       op[i] = {2, cp, ws.plan(n_train * T * 3 * cp * 2), 0};
       op[i].off_v = ws.plan(n_val * T * 3 * cp * 2);
-    } else if (tma_ready(x)) {
+    } else if (x.ready()) {
       op[i] = {0, cp, 0, 0};
     } else {
       op[i] = {1, cp, ws.plan(N * T * cp * 2), 0};
     }
   }
-  char* base = ws.commit(L, A);
+  char* base = ws.commit(L, A.t);
   const char *pt[2], *pv[2];
   long long k[2];
   for (int i = 0; i < 2; ++i) {
-    const Tensor& x = *xs[i];
+    const Operand& x = *xs[i];
     const long long cp = op[i].cp;
     if (op[i].kind == 2) {
-      cast(x, 0, n_train, T, base + op[i].off_t, 3 * cp, cp, 3, kSplitLeft, false, L.st());
-      cast(x, n_train * T, n_val, T, base + op[i].off_v, 3 * cp, cp, 3, kSplitRight, false, L.st());
+      x.cast(0, n_train, base + op[i].off_t, 3 * cp, cp, 3, kSplitLeft, false, L.st());
+      x.cast(n_train, n_val, base + op[i].off_v, 3 * cp, cp, 3, kSplitRight, false, L.st());
       pt[i] = base + op[i].off_t;
       pv[i] = base + op[i].off_v;
       k[i] = 3 * cp;
     } else {
-      if (op[i].kind == 1) cast(x, 0, N, T, base + op[i].off_t, cp, cp, 1, kPlain, false, L.st());
-      pt[i] = op[i].kind == 1 ? base + op[i].off_t : static_cast<const char*>(x.data_ptr());
+      if (op[i].kind == 1) x.cast(0, N, base + op[i].off_t, cp, cp, 1, kPlain, false, L.st());
+      pt[i] = op[i].kind == 1 ? base + op[i].off_t : static_cast<const char*>(x.t.data_ptr());
       pv[i] = pt[i] + n_train * T * cp * 2;
       k[i] = cp;
     }
@@ -232,44 +253,44 @@ PyObject* py_gram_dot(PyObject*, PyObject* const* a, Py_ssize_t n) {
     need(n, 5, "gram_dot");
     const Tensor &A0 = cuda_tensor(a[0]), &G0 = cuda_tensor(a[1]);
     Launch L(A0);
-    return wrap(gram_dot(L, as3d(A0), as3d(G0), integer(a[2]), static_cast<int>(integer(a[3])), real(a[4])));
+    const Tensor A = as3d(A0), G = as3d(G0);
+    return wrap(gram_dot(L, Operand(A), Operand(G), integer(a[2]), static_cast<int>(integer(a[3])), real(a[4])));
   });
 }
 
 // ---- token-contracted GEMMs --------------------------------------------------------------------------
 struct XtyOperands {
-  const Tensor* x[2];
+  const Operand* x[2];
   long long samples, T, cp[2], off[2] = {0, 0};
   int kind[2];                      // 0 as it is, 1 padded copy, 2 split
   bool split;
-  XtyOperands(Workspace& ws, const Tensor& X, const Tensor& Y, long long samples_, long long T_) : samples(samples_), T(T_) {
+  XtyOperands(Workspace& ws, const Operand& X, const Operand& Y, long long samples_) : samples(samples_), T(X.T) {
     x[0] = &X;
     x[1] = &Y;
-    split = is_f32(X) || is_f32(Y);
+    split = X.f32() || Y.f32();
     for (int i = 0; i < 2; ++i) {
-      cp[i] = pad8(x[i]->size(-1));
-      kind[i] = split ? 2 : tma_ready(*x[i]) ? 0 : 1;
+      cp[i] = pad8(x[i]->cols);
+      kind[i] = split ? 2 : x[i]->ready() ? 0 : 1;
       if (kind[i]) off[i] = ws.plan(samples * (split ? 3 : 1) * T * cp[i] * 2);
     }
   }
   const void* get(int i, char* base, void* st) const {
-    if (kind[i] == 0) return x[i]->data_ptr();
-    if (kind[i] == 1) cast(*x[i], 0, samples, T, base + off[i], cp[i], cp[i], 1, kPlain, true, st);
-    else cast(*x[i], 0, samples, T, base + off[i], cp[i], cp[i], 3, i == 0 ? kSplitLeft : kSplitRight, true, st);
+    if (kind[i] == 0) return x[i]->t.data_ptr();
+    if (kind[i] == 1) x[i]->cast(0, samples, base + off[i], cp[i], cp[i], 1, kPlain, true, st);
+    else x[i]->cast(0, samples, base + off[i], cp[i], cp[i], 3, i == 0 ? kSplitLeft : kSplitRight, true, st);
     return base + off[i];
   }
   long long tokens() const { return split ? 3 * T : T; }
 };
 
 // scale * sum over the first `samples` samples of X^T Y, into out
-void wgrad(const Launch& L, const Tensor& X, const Tensor& Y, long long samples, float scale, Tensor& out, bool accumulate) {
-  const long long T = X.size(1);
-  const int m = static_cast<int>(X.size(2)), n = static_cast<int>(Y.size(2));
+void wgrad(const Launch& L, const Operand& X, const Operand& Y, long long samples, float scale, Tensor& out, bool accumulate) {
+  const int m = static_cast<int>(X.cols), n = static_cast<int>(Y.cols);
   Workspace ws;
   const long long ws_bytes = ghost_wgrad_workspace_bytes(m, n);
   const long long off_ws = ws.plan(ws_bytes);
-  XtyOperands ops(ws, X, Y, samples, T);
-  char* base = ws.commit(L, X);
+  XtyOperands ops(ws, X, Y, samples);
+  char* base = ws.commit(L, X.t);
   const void* xp = ops.get(0, base, L.st());
   const void* yp = ops.get(1, base, L.st());
   check(ghost_wgrad_bf16(xp, yp, samples * ops.tokens(), m, n, ops.cp[0], ops.cp[1], scale, accumulate ? 1 : 0,
@@ -286,7 +307,7 @@ PyObject* py_wgrad(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (Y.size(0) != X.size(0) || Y.size(1) != X.size(1)) invalid("wgrad operands disagree on the token layout");
     const bool have = present(a[4]);
     Tensor out = have ? cuda_tensor(a[4]) : empty({X.size(2), Y.size(2)}, X, integer(a[3]) ? at::kFloat : at::kBFloat16);
-    wgrad(L, X, Y, X.size(0), real(a[2]), out, have && integer(a[5]));
+    wgrad(L, Operand(X), Operand(Y), X.size(0), real(a[2]), out, have && integer(a[5]));
     return wrap(out);
   });
 }
@@ -294,22 +315,22 @@ PyObject* py_wgrad(PyObject*, PyObject* const* a, Py_ssize_t n) {
 // ---- per-sample path -----------------------------------------------------------------------------------
 struct PerSample { Tensor M, grad, colsums; };
 
-PerSample persample_dot(const Launch& L, const Tensor& X, const Tensor& Y, long long n_val, float dot_scale, bool want_grad,
+PerSample persample_dot(const Launch& L, const Operand& X, const Operand& Y, long long n_val, float dot_scale, bool want_grad,
                         float grad_scale, at::ScalarType grad_dt, int colsum_of) {
-  const long long N = X.size(0), T = X.size(1), n_train = N - n_val;
-  const int m = static_cast<int>(X.size(2)), n = static_cast<int>(Y.size(2));
+  const long long N = X.N, T = X.T, n_train = N - n_val;
+  const int m = static_cast<int>(X.cols), n = static_cast<int>(Y.cols);
   check_split(n_train, n_val, "persample_dot");
-  if (Y.size(0) != N || Y.size(1) != T) invalid("persample_dot operands disagree on the token layout");
+  if (Y.N != N || Y.T != T) invalid("persample_dot operands disagree on the token layout");
   PerSample r;
-  r.M = empty({n_val, n_train}, X, at::kFloat);
-  if (want_grad) r.grad = empty({m, n}, X, grad_dt);
+  r.M = empty({n_val, n_train}, X.t, at::kFloat);
+  if (want_grad) r.grad = empty({m, n}, X.t, grad_dt);
   Workspace ws;
-  XtyOperands ops(ws, X, Y, N, T);
+  XtyOperands ops(ws, X, Y, N);
   const int f32 = ops.split ? 1 : 0;
   const long long ws_bytes = ghost_persample_workspace_bytes(static_cast<int>(n_train), static_cast<int>(n_val), m, n, f32);
   const long long off_ws = ws.plan(ws_bytes);
-  char* base = ws.commit(L, X);
-  if (colsum_of && !ops.split) r.colsums = empty({N, colsum_of == 1 ? m : n}, X, at::kFloat);
+  char* base = ws.commit(L, X.t);
+  if (colsum_of && !ops.split) r.colsums = empty({N, colsum_of == 1 ? m : n}, X.t, at::kFloat);
   const void* xp = ops.get(0, base, L.st());
   const void* yp = ops.get(1, base, L.st());
   check(ghost_persample_dot_bf16(xp, yp, static_cast<int>(n_train), static_cast<int>(n_val), ops.tokens(), m, n, ops.cp[0],
@@ -325,7 +346,8 @@ PyObject* py_persample_dot(PyObject*, PyObject* const* a, Py_ssize_t n) {
     need(n, 8, "persample_dot");
     const Tensor &X0 = cuda_tensor(a[0]), &Y0 = cuda_tensor(a[1]);
     Launch L(X0);
-    PerSample r = persample_dot(L, as3d(X0), as3d(Y0), integer(a[2]), real(a[3]), integer(a[4]) != 0, real(a[5]),
+    const Tensor X = as3d(X0), Y = as3d(Y0);
+    PerSample r = persample_dot(L, Operand(X), Operand(Y), integer(a[2]), real(a[3]), integer(a[4]) != 0, real(a[5]),
                                 integer(a[6]) ? at::kFloat : at::kBFloat16, static_cast<int>(integer(a[7])));
     return Py_BuildValue("(NNN)", wrap(r.M), wrap_or_none(r.grad), wrap_or_none(r.colsums));
   });
@@ -389,6 +411,24 @@ Tensor optional_empty(at::IntArrayRef size, const Tensor& like, long long dt) {
   return dt < 0 ? Tensor() : empty(size, like, dt ? at::kFloat : at::kBFloat16);
 }
 
+// One of the two tensor-core paths, with the train gradient (dtype code gdt) and, where it costs nothing
+// extra, the column sums of B.
+void dense_paths(const Launch& L, const Operand& A, const Operand& B, long long n_val, bool in_by_out, bool gram, long long gdt,
+                 float scale, bool want_sums, Tensor& M, Tensor& grad, Tensor& sums) {
+  const Operand &X = in_by_out ? A : B, &Y = in_by_out ? B : A;
+  if (gram) {
+    M = gram_dot(L, A, B, n_val, 0, 1.f);
+    grad = optional_empty({X.cols, Y.cols}, X.t, gdt);
+    if (grad.defined()) wgrad(L, X, Y, A.N - n_val, scale, grad, false);
+  } else {
+    PerSample r = persample_dot(L, X, Y, n_val, 1.f, gdt >= 0, scale, gdt == 0 ? at::kBFloat16 : at::kFloat,
+                                !want_sums ? 0 : in_by_out ? 2 : 1);
+    M = r.M;
+    grad = r.grad;
+    sums = r.colsums;
+  }
+}
+
 // Everything the backward hook of a Linear / Conv1D layer computes or allocates:
 // (A, B, n_val, weight_is_in_by_out, use_gram, weight grad dtype, grad scale, has_bias, bias grad dtype, any_path)
 // -> (M, weight grad, column sums of B, unfilled bias matrix, unfilled bias grad), None where not wanted.
@@ -416,20 +456,46 @@ PyObject* py_dense_hook(PyObject*, PyObject* const* a, Py_ssize_t n) {
       check(ghost_dense_small(A.data_ptr(), B.data_ptr(), is_f32(A), static_cast<int>(n_train), static_cast<int>(n_val),
                               A.size(1), dI, pI, in_by_out ? 1 : 0, M.data_ptr<float>(), grad.defined() ? grad.data_ptr() : nullptr,
                               grad.defined() ? is_f32(grad) : 0, scale, copy ? sums.data_ptr<float>() : nullptr, L.st()));
-    } else if (gram) {
-      M = gram_dot(L, A, B, n_val, 0, 1.f);
-      grad = optional_empty({X.size(2), Y.size(2)}, X, gdt);
-      if (grad.defined()) wgrad(L, X, Y, n_train, scale, grad, false);
     } else {
-      PerSample r = persample_dot(L, X, Y, n_val, 1.f, gdt >= 0, scale, gdt == 0 ? at::kBFloat16 : at::kFloat,
-                                  !bias ? 0 : in_by_out ? 2 : 1);
-      M = r.M;
-      grad = r.grad;
-      sums = r.colsums;
+      dense_paths(L, Operand(A), Operand(B), n_val, in_by_out, gram, gdt, scale, bias, M, grad, sums);
     }
     if (bias && !sums.defined()) sums = colsum(L, B);
     Tensor Mb = bias ? empty({n_val, n_train}, A, at::kFloat) : Tensor();
     Tensor sb = optional_empty({p}, A, bias ? bdt : -1);
+    return Py_BuildValue("(NNNNN)", wrap(M), wrap_or_none(grad), wrap_or_none(sums), wrap_or_none(Mb), wrap_or_none(sb));
+  });
+}
+
+// The same for a Conv2d layer with groups == 1: (A [N, C, H, W], B [N, p, Ho, Wo], n_val, (kh, kw, sy, sx, py, px, dy,
+// dx), use_gram, weight grad dtype, grad scale, has_bias, bias grad dtype); the weight gradient is [p, C * kh * kw]
+PyObject* py_conv_hook(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    need(n, 9, "conv_hook");
+    const Tensor &A0 = cuda_tensor(a[0]), &B0 = cuda_tensor(a[1]);
+    Launch L(A0);
+    const Tensor A = A0.contiguous(), B = B0.contiguous();
+    if (A.dim() != 4 || B.dim() != 4 || A.size(0) != B.size(0)) invalid("conv_hook takes [N, C, H, W] and [N, p, Ho, Wo]");
+    if (!PyTuple_Check(a[3]) || PyTuple_GET_SIZE(a[3]) != 8) invalid("conv_hook: bad window");
+    int w[8];
+    for (int i = 0; i < 8; ++i) w[i] = static_cast<int>(integer(PyTuple_GET_ITEM(a[3], i)));
+    const Conv ca = {static_cast<int>(A.size(1)), static_cast<int>(A.size(2)), static_cast<int>(A.size(3)), w[0], w[1], w[2],
+                     w[3], w[4], w[5], w[6], w[7]};
+    const Conv cb = {static_cast<int>(B.size(1)), static_cast<int>(B.size(2)), static_cast<int>(B.size(3)), 1, 1, 1, 1, 0, 0, 1, 1};
+    if (w[2] <= 0 || w[3] <= 0 || (ca.H + 2 * w[4] - w[6] * (w[0] - 1) - 1) / w[2] + 1 != B.size(2) ||
+        (ca.W + 2 * w[5] - w[7] * (w[1] - 1) - 1) / w[3] + 1 != B.size(3))
+      invalid("conv_hook: the out-grad is not this convolution's output size");
+    const long long T = B.size(2) * B.size(3), N = A.size(0), p = B.size(1), n_val = integer(a[2]), n_train = N - n_val;
+    check_split(n_train, n_val, "conv_hook");
+    const bool bias = integer(a[7]) != 0;
+    Tensor M, grad, sums;
+    dense_paths(L, Operand(A, ca, T), Operand(B, cb, T), n_val, false, integer(a[4]) != 0, integer(a[5]), real(a[6]), false, M,
+                grad, sums);
+    if (bias) {
+      sums = empty({N, p}, A, at::kFloat);
+      check(ghost_row_sums(B.data_ptr(), is_f32(B), N * p, T, sums.data_ptr<float>(), L.st()));
+    }
+    Tensor Mb = bias ? empty({n_val, n_train}, A, at::kFloat) : Tensor();
+    Tensor sb = optional_empty({p}, A, bias ? integer(a[8]) : -1);
     return Py_BuildValue("(NNNNN)", wrap(M), wrap_or_none(grad), wrap_or_none(sums), wrap_or_none(Mb), wrap_or_none(sb));
   });
 }
@@ -555,8 +621,8 @@ PyObject* py_gradproj_dense(PyObject*, PyObject* const* a, Py_ssize_t n) {
     for (int i = 0; i < 2; ++i) {
       len[i] = split ? 3 * cp[i] : cp[i];
       p[i] = kind[i] ? static_cast<const void*>(base + off[i]) : x[i]->data_ptr();
-      if (kind[i] == 1) cast(*x[i], 0, B, T, base + off[i], cp[i], cp[i], 1, kPlain, false, L.st());
-      else if (kind[i] == 2) cast(*x[i], 0, B, T, base + off[i], 3 * cp[i], cp[i], 3, kSplitLeft, false, L.st());
+      if (kind[i] == 1) Operand(*x[i]).cast(0, B, base + off[i], cp[i], cp[i], 1, kPlain, false, L.st());
+      else if (kind[i] == 2) Operand(*x[i]).cast(0, B, base + off[i], 3 * cp[i], cp[i], 3, kSplitLeft, false, L.st());
     }
     if (P_r.size(1) != len[0] || P_c.size(1) != len[1])
       invalid("projection matrices were prepared for a different dtype/feature size");
@@ -837,7 +903,8 @@ PyMethodDef kMethods[] = {
     GB_METHOD(embedding_wgrad),   GB_METHOD(gradproj_dense),
     GB_METHOD(gradproj_embedding), GB_METHOD(projection_similarity),
     GB_METHOD(pass_reduce),       GB_METHOD(matrix_sum),
-    GB_METHOD(dense_hook),        GB_METHOD(norm_hook),
+    GB_METHOD(dense_hook),        GB_METHOD(conv_hook),
+    GB_METHOD(norm_hook),
     GB_METHOD(embedding_hook),    GB_METHOD(named_parameters),
     GB_METHOD(arena_clear),       GB_METHOD(set_kernel_error),
     {nullptr, nullptr, 0, nullptr}};

@@ -681,6 +681,38 @@ def _conv2d_tokens(layer: nn.Conv2d, A: torch.Tensor, B: torch.Tensor):
     return A_tok, B_tok
 
 
+def _conv_hook(layer: nn.Conv2d, A: torch.Tensor, B: torch.Tensor, n_val: int) -> bool:
+    """A Conv2d layer inside a backward hook: everything in one native call that lays the operands out
+    itself, no unfolded copy.  False for what that call does not take (called on its own, a padding
+    mode other than zeros or padding given by name, other data types)."""
+    own = layer.__dict__
+    if "_ghost_backprop_scale" not in own or n_val <= 0 or layer.groups != 1 or layer.padding_mode != "zeros" \
+            or isinstance(layer.padding, str) or A.dtype not in _GRAD_TYPES or B.dtype is not A.dtype or A.dim() != 4:
+        return False
+    weight, bias = layer.weight, layer.bias
+    n_train = A.size(0) - n_val
+    if not hasattr(layer, "use_ghost_computation"):
+        N, p = B.shape[0], B.shape[1]
+        T, d = B.shape[2] * B.shape[3], A.shape[1] * layer.kernel_size[0] * layer.kernel_size[1]
+        _should_use_ghost_computation(layer, A.new_empty(()).expand(N, d, T), B.new_empty(()).expand(N, p, T), conv=True,
+                                      val_batch_size=n_val)
+    bias_dtype = None
+    if bias is not None and getattr(bias, "initially_requires_grad", bias.requires_grad):
+        bias_dtype = torch.bfloat16 if bias.dtype is torch.bfloat16 else torch.float32
+    M, grad, sums, bias_M, bias_grad = ops.conv_hook(
+        A, B, n_val, (*layer.kernel_size, *layer.stride, *layer.padding, *layer.dilation), layer.use_ghost_computation,
+        _grad_dtype(weight, A) if getattr(weight, "initially_requires_grad", True) else None,
+        own["_ghost_backprop_scale"] / n_train, bias is not None, bias_dtype)
+    if grad is not None:
+        own["_ghost_cached_train_grad"] = (A.data_ptr(), B.data_ptr(), A.size(0), grad)
+    _set_dot(weight, M)
+    if bias is not None:
+        _set_dot(bias, _gram_of_vectors(sums, n_val, bias_M))
+        own["_ghost_colsums"] = sums
+        own["_ghost_bias_grad"] = bias_grad
+    return True
+
+
 def _compute_conv2d_dot_product(layer: nn.Conv2d, A: torch.Tensor, B: torch.Tensor,
                                 val_batch_size: int) -> None:
     """nn.Conv2d weight and bias dot products (reference :513-563).  The reference's ghost branch
@@ -688,6 +720,8 @@ def _compute_conv2d_dot_product(layer: nn.Conv2d, A: torch.Tensor, B: torch.Tens
     C*kh*kw == out_channels; both kernels here compute the per-sample-gradient products."""
     if A.size(0) - val_batch_size <= 0:
         raise ValueError("No training samples to compute dot product")
+    if _conv_hook(layer, A, B, val_batch_size):
+        return
     A_tok, B_tok = _conv2d_tokens(layer, A, B)
     if not hasattr(layer, "use_ghost_computation"):
         _should_use_ghost_computation(layer, A_tok.transpose(1, 2), B_tok.transpose(1, 2), conv=True,

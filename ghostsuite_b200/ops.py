@@ -234,6 +234,20 @@ def dense_hook(A: torch.Tensor, B: torch.Tensor, n_val: int, weight_is_in_by_out
         return _native().dense_hook(*args)
 
 
+def conv_hook(A: torch.Tensor, B: torch.Tensor, n_val: int, window: Tuple[int, ...], use_gram: bool,
+              grad_dtype: Optional[torch.dtype], grad_scale: float, has_bias: bool,
+              bias_grad_dtype: Optional[torch.dtype]):
+    """:func:`dense_hook` for a Conv2d (groups == 1): ``A [N, C, H, W]``, ``B [N, p, Ho, Wo]``, ``window =
+    (kh, kw, stride y, x, padding y, x, dilation y, x)``.  Output positions are the tokens; the operands are
+    laid out for the tensor-core paths straight from these tensors.  The weight gradient is ``[p, C*kh*kw]``."""
+    args = (A, B, n_val, window, use_gram, _dtype_code(grad_dtype), grad_scale, has_bias, _dtype_code(bias_grad_dtype))
+    if _timing is None:
+        return _native().conv_hook(*args)
+    N, p, T, d = A.shape[0], B.shape[1], B.shape[2] * B.shape[3], A.shape[1] * window[0] * window[1]
+    with _Timed(_PERSAMPLE_NAME, "tensor", 2.0 * N * T * d * p + 2.0 * n_val * (N - n_val) * d * p, 2.0 * N * T * (d + p)):
+        return _native().conv_hook(*args)
+
+
 def persample_tiles(X: torch.Tensor, Y: torch.Tensor, sample0: int, samples: int,
                     colsum_of: Optional[str] = None, colsums: Optional[torch.Tensor] = None) -> torch.Tensor:
     """First pass of the per-sample path alone: the bf16 tiles ``X_s^T Y_s`` of samples

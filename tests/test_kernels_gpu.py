@@ -294,6 +294,48 @@ def test_tile_pass_and_gathered_tile_dot(case):
         assert torch.equal(res[1], one[1]) and O.rel_fro(res[2], one[2].double().cpu()) < 1e-6
 
 
+# both sides of the split-K rule: one CTA per tile stores the result, many add into the workspace
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("rows,m,n", [(20000, 64, 128), (20000, 72, 40), (300, 256, 520), (130, 37, 264)])
+@pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float32])
+def test_wgrad_direct_and_split(rows, m, n, dtype, out_dtype):
+    g = torch.Generator().manual_seed(17)
+    X, Y = (torch.randn(1, rows, c, generator=g).to(dtype).cuda() for c in (m, n))
+    out = ops().wgrad(X, Y, 0.25, out_dtype)
+    ref = 0.25 * X[0].double().t() @ Y[0].double()
+    after()
+    tol = 1e-4 if dtype == torch.float32 else 1e-5          # hi/lo parts; exact products
+    assert O.rel_fro(out, ref) < (3e-3 if out_dtype == torch.bfloat16 else tol)       # 2^-9 of rounding
+    more = ops().wgrad(X, Y, 0.25, out_dtype, out=out.clone(), accumulate=True)
+    after()
+    assert O.rel_fro(more, out.double() + ref) < (6e-3 if out_dtype == torch.bfloat16 else tol)
+
+
+# tokens and features on both sides of the 64 x 64 tile, windows that overhang the input, every option
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("use_gram", [False, True])
+@pytest.mark.parametrize("case", [(3, 2, 4, 9, 7, 5, (3, 3), (1, 1), (1, 1), (1, 1)),
+                                  (4, 1, 3, 12, 11, 8, (5, 3), (2, 1), (2, 0), (1, 1)),
+                                  (2, 2, 7, 10, 13, 70, (3, 2), (1, 2), (2, 1), (2, 3)),
+                                  (5, 3, 65, 8, 8, 24, (1, 1), (1, 1), (0, 0), (1, 1))])
+def test_conv_hook(case, use_gram, dtype):
+    n_t, n_v, C, H, W, p, k, stride, pad, dil = case
+    N = n_t + n_v
+    g = torch.Generator().manual_seed(19)
+    A = torch.randn(N, C, H, W, generator=g).to(dtype)
+    tok = torch.nn.functional.unfold(A.double(), k, dilation=dil, padding=pad, stride=stride).transpose(1, 2)
+    Ho = (H + 2 * pad[0] - dil[0] * (k[0] - 1) - 1) // stride[0] + 1
+    B = torch.randn(N, p, Ho, tok.shape[1] // Ho, generator=g).to(dtype)
+    Bt = B.double().reshape(N, p, -1).transpose(1, 2)
+    M, grad, sums, _, _ = ops().conv_hook(A.cuda(), B.cuda(), n_v, (*k, *stride, *pad, *dil), use_gram, torch.float32, 0.5,
+                                          True, torch.float32)
+    after()
+    per = torch.einsum("ntp,ntd->npd", Bt, tok).reshape(N, -1)
+    assert O.rel_fro(M, per[n_t:] @ per[:n_t].t()) < TOL[dtype]
+    assert O.rel_fro(grad.reshape(-1), 0.5 * per[:n_t].sum(0)) < (1e-4 if dtype == torch.float32 else 1e-2)
+    assert O.rel_fro(sums, Bt.sum(1)) < 1e-5
+
+
 # edges of the one-launch kernel: T on both sides of its 8 x 4 token tile and of whole-sample groups,
 # one sample, widths off and on its 64 / 128 / 1024 column units, odd widths (no 16-byte loads)
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
@@ -619,6 +661,20 @@ def test_projection_similarity(case, dtype):
         S2 = ops().projection_similarity(wide[:, 8:8 + D], P2.cuda(), 0.5)
         after()
         assert O.rel_fro(S2, ref) < 1e-4
+
+
+# every block shape of the kernel with ragged edges, odd and tiny contraction lengths
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("case", [(16, 8, 40), (15, 16, 1000), (3, 70, 264), (31, 25, 2048), (70, 9, 33), (65, 130, 8200), (1, 1, 1)])
+def test_projection_similarity_block_shapes(case, dtype):
+    n1, n2, D = case
+    g = torch.Generator().manual_seed(23)
+    a, b = (torch.randn(n, D, generator=g).to(dtype) for n in (n1, n2))
+    S = ops().projection_similarity(a.cuda(), b.cuda(), 0.5)
+    after()
+    # float32 rows carry two bf16 parts each: 2^-16 per product, relative to the row norms
+    err = (S.cpu().double() - 0.5 * a.double() @ b.double().t()).abs()
+    assert (err <= 2.0 ** -15 * a.double().norm(dim=1)[:, None] * b.double().norm(dim=1)[None]).all()
 
 
 def test_small_reduce_batch_matches_single_launches():
