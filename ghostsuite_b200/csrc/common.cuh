@@ -80,9 +80,10 @@ int make_tmap_plain_2d(CUtensorMap* out, const void* base, int elem_bytes, uint6
 // rows) from shared memory written with the 64-byte swizzle: 16-byte chunk c of row r sits at
 // r * 64 + ((c ^ ((r >> 1) & 3)) * 16).
 int make_tmap_bf16_store_2d(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows);
-// Plain 3-D map of a dense [planes, rows, cols] array; box = [1, box_rows, box_cols].
-int make_tmap_plain_3d(CUtensorMap* out, const void* base, int elem_bytes, uint64_t planes, uint64_t rows,
-                       uint64_t cols, uint32_t box_rows, uint32_t box_cols);
+// Per-sample fp32 tiles [tiles][samples][32768], seen as [tiles, 1024 panels, samples, 32]: a box holds
+// eight panels (256 elements) of `box_rows` samples, each panel a swizzled [box_rows][32] block.
+// Coordinates: (0, sample, panel, tile).
+int make_tmap_f32_tiles(CUtensorMap* out, const void* base, uint64_t tiles, uint64_t samples, uint32_t box_rows);
 
 inline int ceil_div(long long a, long long b) { return static_cast<int>((a + b - 1) / b); }
 

@@ -21,9 +21,8 @@
 // arithmetic off the CUDA cores the kernel is bound by the stream, and up to 32 validation rows
 // share one pass over the train rows.
 //
-// fp32 tiles (tile_dot_kernel<float>): warp w owns train samples 4w..4w+3 of the block, lane l
-// elements 8l..8l+7 of the stage, every shared-memory read is a conflict-free 16-byte access and
-// a thread accumulates an 8 x 4 block of dot products on the CUDA cores (exact fp32 products).
+// fp32 tiles (tile_dot_f32_kernel): the same split of a stage over the warps, with the products on the
+// CUDA cores (exact fp32 products).
 #include "common.cuh"
 #include "sm100_ptx.cuh"
 
@@ -31,11 +30,10 @@ namespace gb {
 
 constexpr int kTileElems = 128 * 256;
 constexpr int kTdCols = 256;            // elements per stage row
-constexpr int kTdValRows = 8;
 constexpr int kTdTrainRows = 32;
 
 struct TileDotParams {
-  long long stages;           // tiles * (32768 / 256)
+  long long stages;           // bf16: tiles * (32768 / 512); fp32: m_cols * n_tiles_n rows of 256 elements
   long long stages_per_cta;
   int n_val, n_grp;           // validation samples, train samples in this group
   int v_off;                  // index of the first validation sample inside V's sample dimension
@@ -53,40 +51,44 @@ struct TileDotParams {
   int* err;
 };
 
-template <typename T>
-struct TdCfg {
-  static constexpr int kRowBytes = kTdCols * sizeof(T);
-  static constexpr int kStageBytes = (kTdValRows + kTdTrainRows) * kRowBytes;    // 20 KB / 40 KB
-  static constexpr int kStages = sizeof(T) == 2 ? 8 : 4;
-  static constexpr int kSmemBytes = kStages * kStageBytes + 8 * kTdCols * 4 + 1024 + 256;
-};
-
-__device__ __forceinline__ void td_load8(const __nv_bfloat16* p, float (&x)[8]) {
-  const uint4 w = *reinterpret_cast<const uint4*>(p);
-  const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
-#pragma unroll
-  for (int e = 0; e < 4; ++e) {
-    x[2 * e] = __uint_as_float(ww[e] << 16);
-    x[2 * e + 1] = __uint_as_float(ww[e] & 0xffff0000u);
-  }
-}
-__device__ __forceinline__ void td_load8(const float* p, float (&x)[8]) {
-  const float4 a = *reinterpret_cast<const float4*>(p);
-  const float4 b = *reinterpret_cast<const float4*>(p + 4);
+// eight floats of a swizzled 128-byte panel row: 16-byte chunks c and c + 1, row index r (mod 8)
+__device__ __forceinline__ void td_load8(const uint8_t* row, int c, int r, float (&x)[8]) {
+  const float4 a = *reinterpret_cast<const float4*>(row + ((c ^ r) << 4));
+  const float4 b = *reinterpret_cast<const float4*>(row + (((c + 1) ^ r) << 4));
   x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w;
   x[4] = b.x; x[5] = b.y; x[6] = b.z; x[7] = b.w;
 }
 
-template <typename T>
+// Stage of the fp32 kernel: 256 elements of every row, as eight 128-byte-swizzled panels of 32.
+template <int VR>
+struct TdF32Cfg {
+  static constexpr int kPanels = kTdCols / 32;
+  static constexpr int kValBytes = kPanels * VR * 128;
+  static constexpr int kStageBytes = kValBytes + kPanels * kTdTrainRows * 128;   // 40 / 48 KB
+  static constexpr int kStages = 4;
+  static constexpr int kRedBytes = 8 * kTdTrainRows * VR * 4;                    // per-warp partial dot blocks
+  static constexpr int kSmemBytes = kStages * kStageBytes + kRedBytes + 1024 + 256;
+};
+
+// VR validation rows x 32 train rows per pass.  Warp w owns panel w of a stage; lane (g, q) holds train
+// rows g, g + 8, g + 16, g + 24 and elements 8q .. 8q + 7 of it, so the swizzle puts the eight 16-byte reads of
+// a quarter-warp into different banks, the column sums are seven shuffles, and the warps run through
+// the ring on their own: no barrier among them until the block is done.  Stages follow the rows of
+// the weight, so rows that only pad the last tile are not read.
+//
+// What bounds it: the stream and, on small layers, the latency of a handful of stages.  With a warp
+// per four train rows, which read all validation rows and met at two barriers per stage, the pass over 64 + 16
+// samples of 128 x 576 float32 took 39 us; it takes 14.7 us now (24 MB, L2-resident).
+template <int VR>
 __global__ void __launch_bounds__(288, 1)
-tile_dot_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_w,
-                const TileDotParams p) {
-  using Cfg = TdCfg<T>;
-  constexpr int kStages = Cfg::kStages;
+tile_dot_f32_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_w,
+                    const TileDotParams p) {
+  using Cfg = TdF32Cfg<VR>;
+  constexpr int kStages = Cfg::kStages, TR = kTdTrainRows;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  float* s_part = reinterpret_cast<float*>(smem + kStages * Cfg::kStageBytes);     // [8 warps][256]
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kStages * Cfg::kStageBytes + 8 * kTdCols * 4);
+  float* s_red = reinterpret_cast<float*>(smem + kStages * Cfg::kStageBytes);            // [8 warps][32][VR]
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kStages * Cfg::kStageBytes + Cfg::kRedBytes);
   uint64_t* full_bar = bars;
   uint64_t* empty_bar = bars + kStages;
   volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + 2 * kStages);
@@ -94,7 +96,6 @@ tile_dot_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_constant_
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const long long s_begin = static_cast<long long>(blockIdx.x) * p.stages_per_cta;
   const long long s_end = (s_begin + p.stages_per_cta < p.stages) ? s_begin + p.stages_per_cta : p.stages;
-  constexpr int kStagesPerTile = kTileElems / kTdCols;   // 128
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 8); }
@@ -108,16 +109,17 @@ tile_dot_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_constant_
     // ---------------------------------------------------------------- TMA producer
     if (lane == 0) {
       int stage = 0; uint32_t phase = 0; bool ok = true;
-      for (int j0 = 0; j0 < p.n_grp && ok; j0 += kTdTrainRows)
-        for (int v0 = 0; v0 < p.n_val && ok; v0 += kTdValRows)
+      for (int j0 = 0; j0 < p.n_grp && ok; j0 += TR)
+        for (int v0 = 0; v0 < p.n_val && ok; v0 += VR)
           for (long long s = s_begin; s < s_end; ++s) {
             if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag, p.err, 431)) { ok = false; break; }
             uint8_t* st = smem + stage * Cfg::kStageBytes;
-            const int tile = static_cast<int>(s / kStagesPerTile);
-            const int col = static_cast<int>(s % kStagesPerTile) * kTdCols;
+            const int r = static_cast<int>(s / p.n_tiles_n);
+            const int tile = (r >> 7) * p.n_tiles_n + static_cast<int>(s % p.n_tiles_n);
+            const int panel = (r & 127) * Cfg::kPanels;
             mbar_arrive_expect_tx(&full_bar[stage], Cfg::kStageBytes);
-            tma_load_3d(st, &tm_v, &full_bar[stage], col, p.v_off + v0, tile);
-            tma_load_3d(st + kTdValRows * Cfg::kRowBytes, &tm_w, &full_bar[stage], col, j0, tile);
+            tma_load_4d(st, &tm_v, &full_bar[stage], 0, p.v_off + v0, panel, tile);
+            tma_load_4d(st + Cfg::kValBytes, &tm_w, &full_bar[stage], 0, j0, panel, tile);
             if (++stage == kStages) { stage = 0; phase ^= 1; }
           }
     }
@@ -125,93 +127,114 @@ tile_dot_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_constant_
   }
 
   // ------------------------------------------------------------------ compute warps 0-7
+  const int g = lane >> 2, q = lane & 3;
+  // element of the stage whose column sum ends up in this lane (see the butterfly below)
+  const int mine = warp * 32 + q * 8 + ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1);
   int stage = 0; uint32_t phase = 0;
   bool alive = true;
-  for (int j0 = 0; j0 < p.n_grp && alive; j0 += kTdTrainRows) {
-    for (int v0 = 0; v0 < p.n_val && alive; v0 += kTdValRows) {
-      float acc[8][4];
+  for (int j0 = 0; j0 < p.n_grp && alive; j0 += TR) {
+    for (int v0 = 0; v0 < p.n_val && alive; v0 += VR) {
+      float acc[VR][4];
 #pragma unroll
-      for (int i = 0; i < 8; ++i)
+      for (int i = 0; i < VR; ++i)
 #pragma unroll
-        for (int q = 0; q < 4; ++q) acc[i][q] = 0.f;
+        for (int k = 0; k < 4; ++k) acc[i][k] = 0.f;
       const bool do_sum = (v0 == 0) && (p.sum != nullptr || p.out != nullptr);
-      bool bvalid[4];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) bvalid[q] = (j0 + warp * 4 + q) < p.n_grp;
 #pragma unroll 1
       for (long long s = s_begin; s < s_end; ++s) {
-        const bool ok = mbar_wait(&full_bar[stage], phase, abort_flag, p.err, 132);
-        if (!named_bar_and(1, 256, ok)) { alive = false; break; }
-        const T* vbuf = reinterpret_cast<const T*>(smem + stage * Cfg::kStageBytes);
-        const T* wbuf = vbuf + kTdValRows * kTdCols;
-        float w[4][8];
-        float ssum[8];
+        int ok = 1;
+        if (lane == 0) ok = mbar_wait(&full_bar[stage], phase, abort_flag, p.err, 132) ? 1 : 0;
+        ok = __shfl_sync(0xffffffffu, ok, 0);
+        if (!ok) { alive = false; break; }
+        const uint8_t* vbuf = smem + stage * Cfg::kStageBytes + warp * (VR * 128);
+        const uint8_t* wbuf = smem + stage * Cfg::kStageBytes + Cfg::kValBytes + warp * (TR * 128);
+        float w[4][8], sum[8];
 #pragma unroll
-        for (int x = 0; x < 8; ++x) ssum[x] = 0.f;
+        for (int k = 0; k < 4; ++k) td_load8(wbuf + (k * 8 + g) * 128, 2 * q, g, w[k]);
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          td_load8(wbuf + (warp * 4 + q) * kTdCols + lane * 8, w[q]);
+        for (int i = 0; i < VR; ++i) {
+          float v[8];
+          td_load8(vbuf + i * 128, 2 * q, i & 7, v);
 #pragma unroll
-          for (int x = 0; x < 8; ++x) ssum[x] += bvalid[q] ? w[q][x] : 0.f;
-        }
+          for (int k = 0; k < 4; ++k)
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          float vv[8];
-          td_load8(vbuf + i * kTdCols + lane * 8, vv);
-#pragma unroll
-          for (int q = 0; q < 4; ++q)
-#pragma unroll
-            for (int x = 0; x < 8; ++x) acc[i][q] = fmaf(vv[x], w[q][x], acc[i][q]);
+            for (int x = 0; x < 8; ++x) acc[i][k] = fmaf(v[x], w[k][x], acc[i][k]);
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(&empty_bar[stage]);     // this warp is done with the stage
         if (++stage == kStages) { stage = 0; phase ^= 1; }
         if (do_sum) {
-          float4* mine = reinterpret_cast<float4*>(s_part + warp * kTdCols + lane * 8);
-          mine[0] = make_float4(ssum[0], ssum[1], ssum[2], ssum[3]);
-          mine[1] = make_float4(ssum[4], ssum[5], ssum[6], ssum[7]);
-          asm volatile("bar.sync 2, 256;" ::: "memory");
-          float t = 0.f;
+          // train rows of the group summed over this lane's four, then over the eight lanes g: a
+          // butterfly that halves the elements with every step leaves one in each lane
 #pragma unroll
-          for (int ww = 0; ww < 8; ++ww) t += s_part[ww * kTdCols + threadIdx.x];
+          for (int x = 0; x < 8; ++x) {
+            sum[x] = 0.f;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) sum[x] += j0 + k * 8 + g < p.n_grp ? w[k][x] : 0.f;
+          }
+#pragma unroll
+          for (int h = 4; h >= 1; h >>= 1) {
+            const bool up = (lane & (h * 4)) != 0;
+#pragma unroll
+            for (int x = 0; x < h; ++x) {
+              const float send = up ? sum[x] : sum[x + h], keep = up ? sum[x + h] : sum[x];
+              sum[x] = keep + __shfl_xor_sync(0xffffffffu, send, h * 4);
+            }
+          }
+          const int r = static_cast<int>(s / p.n_tiles_n), tn = static_cast<int>(s % p.n_tiles_n);
+          float t = sum[0];
           if (p.out != nullptr) {
-            // one stage is one 256-column row segment of one 128 x 256 tile
-            const long long tile = s / kStagesPerTile;
-            const int r = static_cast<int>(tile / p.n_tiles_n) * 128 + static_cast<int>(s % kStagesPerTile);
-            const int c = static_cast<int>(tile % p.n_tiles_n) * 256 + static_cast<int>(threadIdx.x);
-            if (r < p.m_cols && c < p.n_cols) {
+            const int c = tn * 256 + mine;
+            if (c < p.n_cols) {
               const long long o = static_cast<long long>(r) * p.n_cols + c;
-              float val = t * p.out_scale;
+              t *= p.out_scale;
               if (p.out_is_f32) {
                 float* dst = static_cast<float*>(p.out) + o;
-                if (p.out_accumulate || j0 > 0) val += *dst;
-                *dst = val;
+                if (p.out_accumulate || j0 > 0) t += *dst;
+                *dst = t;
               } else {
                 __nv_bfloat16* dst = static_cast<__nv_bfloat16*>(p.out) + o;
-                if (p.out_accumulate || j0 > 0) val += __bfloat162float(*dst);
-                *dst = __float2bfloat16_rn(val);
+                if (p.out_accumulate || j0 > 0) t += __bfloat162float(*dst);
+                *dst = __float2bfloat16_rn(t);
               }
             }
           } else {
-            float* dst = p.sum + s * kTdCols + threadIdx.x;
+            float* dst = p.sum + (static_cast<long long>(r >> 7) * p.n_tiles_n + tn) * kTileElems + (r & 127) * kTdCols + mine;
             if (!(p.sum_init && j0 == 0)) t += *dst;
             *dst = t;
           }
         }
       }
-      if (!alive) break;
-      // reduce the 8 x 4 block over the 32 lanes, one atomic per (v, b) and CTA
+      // the only CTA-wide agreement: every compute warp gets here once per block, aborted or not
+      if (!named_bar_and(1, 256, alive)) { alive = false; break; }
+      // reduce the 32 x VR block over the four lanes q, then over the warps; one atomic per (v, b) and CTA
+      float* part = s_red + warp * (TR * VR);
 #pragma unroll
-      for (int i = 0; i < 8; ++i)
+      for (int i = 0; i < VR; ++i) {
+        float a[4];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          float a = acc[i][q];
+        for (int k = 0; k < 4; ++k) a[k] = acc[i][k];
 #pragma unroll
-          for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-          const int v = v0 + i, b = j0 + warp * 4 + q;
-          if (lane == 0 && v < p.n_val && b < p.n_grp && a != 0.f)
-            atomicAdd(&p.M[static_cast<long long>(v) * p.n_train + p.b0 + b], a * p.scale);
+        for (int h = 2; h >= 1; h >>= 1) {
+          const bool up = (lane & h) != 0;
+#pragma unroll
+          for (int k = 0; k < h; ++k) {
+            const float send = up ? a[k] : a[k + h], keep = up ? a[k + h] : a[k];
+            a[k] = keep + __shfl_xor_sync(0xffffffffu, send, h);
+          }
         }
+        part[i * TR + q * 8 + g] = a[0];       // lane q is left with k = q
+      }
+      asm volatile("bar.sync 2, 256;" ::: "memory");
+      for (int idx = threadIdx.x; idx < TR * VR; idx += 256) {
+        float t = 0.f;
+#pragma unroll
+        for (int w = 0; w < 8; ++w) t += s_red[w * (TR * VR) + idx];
+        const int b = j0 + idx % TR, v = v0 + idx / TR;
+        if (v < p.n_val && b < p.n_grp && t != 0.f)
+          atomicAdd(&p.M[static_cast<long long>(v) * p.n_train + p.b0 + b], t * p.scale);
+      }
+      asm volatile("bar.sync 2, 256;" ::: "memory");
     }
   }
 }
@@ -485,28 +508,26 @@ __global__ void tile_sum_finalize_kernel(const float* __restrict__ sum, int n_ti
   }
 }
 
-template <typename T>
-static int launch_tile_dot_t(const void* V, int v_samples, const void* W, int w_samples, long long tiles,
-                             TileDotParams& p, const DeviceState* ds, cudaStream_t st) {
-  using Cfg = TdCfg<T>;
+template <int VR>
+static int launch_tile_dot_f32(const void* V, int v_samples, const void* W, int w_samples, long long tiles,
+                               TileDotParams& p, const DeviceState* ds, cudaStream_t st) {
+  using Cfg = TdF32Cfg<VR>;
   CUtensorMap tv, tw;
   int rc;
-  if ((rc = make_tmap_plain_3d(&tv, V, sizeof(T), tiles, v_samples, kTileElems, kTdValRows, kTdCols)) != GHOST_OK)
-    return rc;
-  if ((rc = make_tmap_plain_3d(&tw, W, sizeof(T), tiles, w_samples, kTileElems, kTdTrainRows, kTdCols)) != GHOST_OK)
-    return rc;
+  if ((rc = make_tmap_f32_tiles(&tv, V, tiles, v_samples, VR)) != GHOST_OK) return rc;
+  if ((rc = make_tmap_f32_tiles(&tw, W, tiles, w_samples, kTdTrainRows)) != GHOST_OK) return rc;
   static bool attr_set[64] = {};
   if (!attr_set[ds->device]) {
-    GB_CUDA_OK(cudaFuncSetAttribute(tile_dot_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes));
+    GB_CUDA_OK(cudaFuncSetAttribute(tile_dot_f32_kernel<VR>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes));
     attr_set[ds->device] = true;
   }
   long long ctas = ds->sm_count;
   if (ctas > p.stages) ctas = p.stages;
   p.stages_per_cta = (p.stages + ctas - 1) / ctas;
   ctas = (p.stages + p.stages_per_cta - 1) / p.stages_per_cta;
-  tile_dot_kernel<T><<<static_cast<int>(ctas), 288, Cfg::kSmemBytes, st>>>(tv, tw, p);
+  tile_dot_f32_kernel<VR><<<static_cast<int>(ctas), 288, Cfg::kSmemBytes, st>>>(tv, tw, p);
   count_launch();
-  return post_launch("tile_dot_kernel");
+  return post_launch("tile_dot_f32_kernel");
 }
 
 template <int NVT, int MT>
@@ -558,12 +579,13 @@ int launch_tile_dot(const void* V, int v_samples, int v_off, const void* W, int 
   p.v_per_rank = v_per_rank;
   p.out = out; p.out_is_f32 = out_is_f32; p.out_accumulate = out_accumulate;
   p.m_cols = m_cols; p.n_cols = n_cols; p.n_tiles_n = n_tiles_n; p.out_scale = out_scale;
-  p.stages = tiles * (kTileElems / (is_f32 ? kTdCols : kMmaCols));
+  p.stages = is_f32 ? static_cast<long long>(m_cols) * n_tiles_n : tiles * (kTileElems / kMmaCols);
   p.stages_per_cta = 0;
   p.n_val = n_val; p.n_grp = n_grp; p.b0 = b0; p.n_train = n_train;
   p.scale = scale; p.M = M; p.sum = sum; p.sum_init = sum_init;
   p.err = ds->err_word;
-  if (is_f32) return launch_tile_dot_t<float>(V, v_samples, W, w_samples, tiles, p, ds, st);
+  if (is_f32 && n_val <= 8) return launch_tile_dot_f32<8>(V, v_samples, W, w_samples, tiles, p, ds, st);
+  if (is_f32) return launch_tile_dot_f32<16>(V, v_samples, W, w_samples, tiles, p, ds, st);
   if (n_val <= 8) return launch_tile_dot_mma<1>(V, v_samples, W, w_samples, tiles, p, ds, st);
   if (n_val <= 16) return launch_tile_dot_mma<2>(V, v_samples, W, w_samples, tiles, p, ds, st);
   return launch_tile_dot_mma<4>(V, v_samples, W, w_samples, tiles, p, ds, st);

@@ -244,6 +244,32 @@ def test_persample_dot_cta_pair_kernel(case, dtype):
     assert lib.ghost_set_persample_pair_mode(3) < 0
 
 
+# edges of the float32 streaming kernel: 8- and 16-row validation blocks, 32-row train blocks, weights that
+# end inside a tile, train groups that add up over several launches
+@pytest.mark.parametrize("case", [(1, 1, 3, 1), (32, 8, 129, 255), (33, 9, 127, 257), (5, 17, 1, 300), (70, 16, 130, 40)])
+@pytest.mark.parametrize("grad_dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("budget", [12 << 30, 3 << 20])
+def test_persample_float32_tiles_exact(case, grad_dtype, budget):
+    """Small whole numbers: every product and partial sum is a whole number below 2^24, so the float32
+    results are exact whatever the order of the additions; the bf16 gradient is one rounding of it."""
+    from ghostsuite_b200 import _lib
+    n_t, n_v, p, d = case
+    gen = torch.Generator().manual_seed(sum(case))
+    A = torch.randint(-3, 4, (n_t + n_v, 5, d), generator=gen).float()
+    G = torch.randint(-3, 4, (n_t + n_v, 5, p), generator=gen).float()
+    per = torch.einsum("ntp,ntd->npd", G.double(), A.double())
+    want = per[n_t:].flatten(1) @ per[:n_t].flatten(1).T
+    lib = _lib.load()
+    try:
+        _lib.check(lib.ghost_set_persample_budget_bytes(budget))
+        M, grad = ops().persample_dot(G.cuda(), A.cuda(), n_v, want_grad=True, grad_scale=1.0, grad_dtype=grad_dtype)
+        after()
+    finally:
+        _lib.check(lib.ghost_set_persample_budget_bytes(12 << 30))
+    assert torch.equal(M.cpu().double(), want)
+    assert torch.equal(grad.cpu(), per[:n_t].sum(0).to(grad_dtype))
+
+
 @pytest.mark.parametrize("case", [(5, 8, 70, 64, 128), (12, 8, 64, 256, 512), (7, 16, 33, 192, 320),
                                   (33, 4, 40, 72, 264), (3, 32, 20, 128, 256)])
 def test_tile_pass_and_gathered_tile_dot(case):
