@@ -159,9 +159,12 @@ __device__ __forceinline__ void emb_store_row(T* __restrict__ out, int k, int d,
                                               float divisor, int accumulate) {
   T* dst = out + static_cast<long long>(k) * d + f;
   float o[8];
+  // dividing by a power of two and multiplying by its reciprocal are the same rounding of the same number
+  const bool pow2 = (__float_as_uint(divisor) & 0x7fffffu) == 0;
+  const float inv = 1.f / divisor;
 #pragma unroll
   for (int e = 0; e < 8; ++e) {
-    o[e] = round_to<T>(__fdiv_rn(round_to<T>(acc[e]), divisor));
+    o[e] = round_to<T>(pow2 ? __fmul_rn(round_to<T>(acc[e]), inv) : __fdiv_rn(round_to<T>(acc[e]), divisor));
     if (accumulate && f + e < d) o[e] = round_to<T>(__fadd_rn(ld_f32<T>(dst + e), o[e]));
   }
   if (vec) {
@@ -219,7 +222,8 @@ struct EmbBuckets {
   int *off_b, *off_v;                   // [vocab] first position of the id's bucket in perm_b / perm_v
   int *rank;                            // [n_tok] position inside the bucket, -1 for an id outside the table
   int *perm_b, *perm_v;
-  int *totals;                          // [0] train tokens placed, [1] validation, [2] big rows, [3] items, [4] hot ids, [5] small rows
+  int *totals;                          // [0] train tokens placed, [1] validation, [2] big rows, [3] items, [4] hot ids, [5] small rows,
+                                        // [6, 7] 64-bit count of gradient items handed out
   int4 *small;                          // (id, offset, tokens) of the rows with 1 to kEmbSmallBucket train tokens
   int *big;                             // ids with more than kEmbSmallBucket train tokens
   int4 *items;                          // join items: (first train position, train rows, first validation position
@@ -518,7 +522,8 @@ emb_join_kernel(const EmbBuckets q, const T* __restrict__ Gb, const T* __restric
                                 Gb + static_cast<long long>(jb) * d, ok0, ok1, b_ok, d, c, acc);
       }
       if (single) {                        // every entry belongs to the one pair
-        float s = (acc[0] + acc[1]) + (acc[2] + acc[3]);      // absent rows and columns are zero
+        const bool c0 = 2 * c < nb, c1 = 2 * c + 1 < nb;      // an absent row times an infinite one is no zero
+        float s = ((ok0 && c0 ? acc[0] : 0.f) + (ok0 && c1 ? acc[1] : 0.f)) + ((ok1 && c0 ? acc[2] : 0.f) + (ok1 && c1 ? acc[3] : 0.f));
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
         if (lane == 0) atomicAdd(acc_M, s * out_scale);
@@ -541,85 +546,75 @@ emb_join_kernel(const EmbBuckets q, const T* __restrict__ Gb, const T* __restric
 }
 
 // ---------------------------------------------------------------- train gradient
-// One warp per listed table row (1 to 32 tokens): ascending-order float32 segment sum, dtype rounding as the
-// reference.  Empty rows were zero-filled by the counting kernel, so the chain per row is list entry,
-// token list, rows, store; the next entry is fetched a row ahead.  The work of a row is the list of
-// (256-feature step, token) units, step-major; the loads of eight units are issued before their rows are
-// added in order, so a row with one or two tokens has all its loads in flight at once.
+// Both parts below add a row's tokens in ascending order in float32 and round as the reference does.
+// Rows that share few tokens (one to kEmbSmallBucket): a warp per listed row and 256 features.  The row's
+// tokens are sorted across the warp, loads of kBatch of them are issued before they are added in order.
+// Items are handed out kEmbGrab at a time by a counter, the next hand-out fetched while one is worked on:
+// static shares left the warps with the rows of 20 to 32 tokens running alone.
+constexpr int kEmbGrab = 4;
+
 template <typename T>
-__global__ void __launch_bounds__(256, 3)
-emb_segsum_kernel(const EmbBuckets q, const T* __restrict__ G, int d, float pre_scale, float divisor, int accumulate,
-                  T* __restrict__ out) {
+__device__ __forceinline__ void emb_small_rows(const EmbBuckets& q, const T* __restrict__ G, int d, float pre_scale,
+                                               float divisor, int accumulate, T* __restrict__ out) {
   const int lane = threadIdx.x & 31;
   const bool vec = (d % 8 == 0) && ((reinterpret_cast<uintptr_t>(G) & 15u) == 0) &&
                    ((reinterpret_cast<uintptr_t>(out) & 15u) == 0);
   const int steps = (d + 255) / 256;
-  const int total = q.totals[5], stride = gridDim.x * 8;
+  const long long total = static_cast<long long>(q.totals[5]) * steps;
   using Raw = typename EmbRaw<T>::type;
   constexpr int kBatch = sizeof(T) == 2 ? 8 : 4;      // 32 registers of loaded rows for either dtype
-  int w = blockIdx.x * 8 + (threadIdx.x >> 5);
-  int4 entry = w < total ? q.small[w] : make_int4(0, 0, 0, 0);
-  for (; w < total; w += stride) {
-    const int k = entry.x, off = entry.y, n = entry.z;
-    int tok = lane < n ? q.perm_b[off + lane] : INT_MAX;
-    if (w + stride < total) entry = q.small[w + stride];
-    if (n > 1) {
-      // bitonic sort of 32 keys across the warp, ascending
+  unsigned long long* counter = reinterpret_cast<unsigned long long*>(q.totals + 6);
+  auto grab = [&]() -> long long {
+    return lane == 0 ? static_cast<long long>(atomicAdd(counter, static_cast<unsigned long long>(kEmbGrab))) : 0;
+  };
+  long long mine = grab();
+  while (true) {
+    const long long first = __shfl_sync(0xffffffffu, mine, 0);
+    if (first >= total) return;
+    mine = grab();
+    const long long last = first + kEmbGrab < total ? first + kEmbGrab : total;
+    int4 entry = q.small[first / steps];
+    for (long long w = first; w < last; ++w) {
+      const int k = entry.x, off = entry.y, n = entry.z;
+      const int f = static_cast<int>(w % steps) * 256 + lane * 8;
+      int tok = lane < n ? q.perm_b[off + lane] : INT_MAX;
+      if (w + 1 < last) entry = q.small[(w + 1) / steps];
+      // bitonic sort of the first n keys, ascending
 #pragma unroll
       for (int size = 2; size <= 32; size <<= 1) {
+        if (size >= 2 * n) break;
 #pragma unroll
-        for (int stride2 = size >> 1; stride2 > 0; stride2 >>= 1) {
-          const int other = __shfl_xor_sync(0xffffffffu, tok, stride2);
-          const bool up = ((lane & size) == 0);
-          const bool lower = ((lane & stride2) == 0);
-          const int lo = min(tok, other), hi = max(tok, other);
-          tok = (lower == up) ? lo : hi;
+        for (int stride = size >> 1; stride > 0; stride >>= 1) {
+          const int other = __shfl_xor_sync(0xffffffffu, tok, stride);
+          const bool up = ((lane & size) == 0), lower = ((lane & stride) == 0);
+          tok = (lower == up) ? min(tok, other) : max(tok, other);
         }
       }
-    }
-    const int units = steps * n;
-    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    int step = 0, i = 0;                   // unit -> (step, token), advanced without divisions
-    auto finish_unit = [&]() {
-      if (++i == n) {                      // last token of this step: write the row's 256 features
-        emb_store_row<T>(out, k, d, step * 256 + lane * 8, vec, acc, divisor, accumulate);
+      float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+      if (vec) {
+        for (int i0 = 0; i0 < n; i0 += kBatch) {
+          Raw x[kBatch];
 #pragma unroll
-        for (int e = 0; e < 8; ++e) acc[e] = 0.f;
-        i = 0;
-        ++step;
-      }
-    };
-    if (!vec) {                            // odd feature counts: one unit at a time
-      for (int u = 0; u < units; ++u) {
-        float x[8];
-        emb_load_row<T>(G, __shfl_sync(0xffffffffu, tok, i), d, step * 256 + lane * 8, false, x);
-        emb_accumulate<T>(x, pre_scale, acc);
-        finish_unit();
-      }
-      continue;
-    }
-    for (int u0 = 0; u0 < units; u0 += kBatch) {
-      Raw x[kBatch];
-      {
-        int c = step, ii = i;
+          for (int r = 0; r < kBatch; ++r) {
+            const int j = __shfl_sync(0xffffffffu, tok, i0 + r);
+            x[r] = i0 + r < n && f < d ? EmbRaw<T>::load(G + static_cast<long long>(j) * d + f) : EmbRaw<T>::zero();
+          }
 #pragma unroll
-        for (int r = 0; r < kBatch; ++r) {
-          const int j = __shfl_sync(0xffffffffu, tok, ii);
-          const int f = c * 256 + lane * 8;
-          if (u0 + r < units && f < d) x[r] = EmbRaw<T>::load(G + static_cast<long long>(j) * d + f);
-          else x[r] = EmbRaw<T>::zero();
-          if (++ii == n) { ii = 0; ++c; }
+          for (int r = 0; r < kBatch; ++r) {
+            if (i0 + r >= n) break;
+            float xf[8];
+            EmbRaw<T>::unpack(x[r], xf);
+            emb_accumulate<T>(xf, pre_scale, acc);
+          }
+        }
+      } else {
+        for (int i = 0; i < n; ++i) {
+          float x[8];
+          emb_load_row<T>(G, __shfl_sync(0xffffffffu, tok, i), d, f, false, x);
+          emb_accumulate<T>(x, pre_scale, acc);
         }
       }
-#pragma unroll
-      for (int r = 0; r < kBatch; ++r) {
-        if (u0 + r < units) {
-          float xf[8];
-          EmbRaw<T>::unpack(x[r], xf);
-          emb_accumulate<T>(xf, pre_scale, acc);
-          finish_unit();
-        }
-      }
+      emb_store_row<T>(out, k, d, f, vec, acc, divisor, accumulate);
     }
   }
 }
@@ -629,22 +624,20 @@ emb_segsum_kernel(const EmbBuckets q, const T* __restrict__ G, int d, float pre_
 // tokens set bits of a window of 32768 tokens in shared memory, and prefix sums of the words' bit counts
 // turn the map into an ordered list.  The sum is sequential per feature (float addition in the CPU's
 // order), so its bound is the issue rate of one warp, eight instructions a token; a three-slot ring of
-// 64-row stages filled with cp.async keeps the rows arriving at that pace.  One CTA per row with a
-// sorted list and eight rows in flight: 492 us for text ids (the longest row 1250 tokens), 18 us now.
-constexpr int kBigThreads = 128;
+// 32-row stages filled with cp.async keeps the rows arriving at that pace.
+constexpr int kEmbGradThreads = 128;
 constexpr int kBigWindow = 32768;        // tokens of a bit map: 1024 words, eight per thread
 constexpr int kBigList = 2048;           // list entries held at a time
-constexpr int kBigStage = 64, kBigSlots = 3;
+constexpr int kBigStage = 32, kBigSlots = 3;
 
 template <typename T>
-__global__ void __launch_bounds__(kBigThreads)
-emb_big_bucket_kernel(const EmbBuckets q, const T* __restrict__ G, int d, int slices, float pre_scale, float divisor,
-                      int accumulate, T* __restrict__ out) {
+__device__ __forceinline__ void emb_big_rows(const EmbBuckets& q, const T* __restrict__ G, int d, int slices, float pre_scale,
+                                             float divisor, int accumulate, T* __restrict__ out) {
   constexpr int kFeat = 256 / static_cast<int>(sizeof(T));
   constexpr int kPer = 16 / static_cast<int>(sizeof(T));       // features of a 16-byte piece
   __shared__ unsigned s_map[kBigWindow / 32];
   __shared__ unsigned short s_list[kBigList];
-  __shared__ int s_warp[kBigThreads / 32];
+  __shared__ int s_warp[kEmbGradThreads / 32];
   extern __shared__ __align__(16) unsigned char s_dyn[];
   T (*s_ring)[kBigStage][kFeat] = reinterpret_cast<T (*)[kBigStage][kFeat]>(s_dyn);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -660,10 +653,10 @@ emb_big_bucket_kernel(const EmbBuckets q, const T* __restrict__ G, int d, int sl
     float acc = 0.f;
     for (long long win = 0; win < n_train_tok; win += kBigWindow) {
       __syncthreads();
-      for (int i = tid; i < kBigWindow / 32; i += kBigThreads) s_map[i] = 0u;
+      for (int i = tid; i < kBigWindow / 32; i += kEmbGradThreads) s_map[i] = 0u;
       __syncthreads();
 #pragma unroll 4
-      for (int i = tid; i < cnt; i += kBigThreads) {
+      for (int i = tid; i < cnt; i += kEmbGradThreads) {
         const long long j = q.perm_b[off + i] - win;
         if (j >= 0 && j < kBigWindow) atomicOr(&s_map[j >> 5], 1u << (j & 31));
       }
@@ -682,7 +675,7 @@ emb_big_bucket_kernel(const EmbBuckets q, const T* __restrict__ G, int d, int sl
       __syncthreads();
       int first = x - own, in_window = 0;
 #pragma unroll
-      for (int v = 0; v < kBigThreads / 32; ++v) {
+      for (int v = 0; v < kEmbGradThreads / 32; ++v) {
         if (v < warp) first += s_warp[v];
         in_window += s_warp[v];
       }
@@ -708,8 +701,8 @@ emb_big_bucket_kernel(const EmbBuckets q, const T* __restrict__ G, int d, int sl
           auto issue = [&](int st) {
             if (st < n_stages) {
 #pragma unroll
-              for (int e = 0; e < kBigStage * 16 / kBigThreads; ++e) {
-                const int c = e * kBigThreads + tid, r = c >> 4, piece = (c & 15) * kPer;
+              for (int e = 0; e < kBigStage * 16 / kEmbGradThreads; ++e) {
+                const int c = e * kEmbGradThreads + tid, r = c >> 4, piece = (c & 15) * kPer;
                 const int i = st * kBigStage + r;
                 if (i < n && f0 + piece < d) {
                   const T* src = G + (win + s_list[i]) * d + f0 + piece;
@@ -752,6 +745,17 @@ emb_big_bucket_kernel(const EmbBuckets q, const T* __restrict__ G, int d, int sl
       *dst = from_f32<T>(o);
     }
   }
+}
+
+// One launch for both: every CTA takes its share of the long rows, whose chains are the longest, and goes on
+// with the short ones.  Apart, a launch of each (text ids, 40 x 1024 tokens of 768 bf16 features) took 46 and
+// 35 us, mostly with a few warps left per SM; MEASURED_NEW.
+template <typename T>
+__global__ void __launch_bounds__(kEmbGradThreads, 6)
+emb_grad_kernel(const EmbBuckets q, const T* __restrict__ G, int d, int slices, float pre_scale, float divisor,
+                int accumulate, T* __restrict__ out) {
+  emb_big_rows<T>(q, G, d, slices, pre_scale, divisor, accumulate, out);
+  emb_small_rows<T>(q, G, d, pre_scale, divisor, accumulate, out);
 }
 
 static inline long long up256(long long x) { return (x + 255) / 256 * 256; }
@@ -818,20 +822,14 @@ static int emb_pass(const EmbBuckets& q, const T* Gb, const T* Gv, int n_train, 
     count_launch();
   }
   if (out != nullptr) {
+    // every row with tokens is a long row's slices or a short row's steps: at least one item per warp
     const long long rows = q.vocab < q.first_val ? q.vocab : q.first_val;      // at most one row per token
-    const int sb = static_cast<int>((rows + 7) / 8 < ds->sm_count * 3 ? (rows + 7) / 8 : ds->sm_count * 3);
-    emb_segsum_kernel<T><<<sb, 256, 0, st>>>(q, Gb, d, pre_scale, divisor, accumulate, out);
     const int slices = ceil_div(d, 256 / static_cast<int>(sizeof(T)));
-    const long long most = (static_cast<long long>(n_train) * Tn / (kEmbSmallBucket + 1) + 1) * slices;
-    const int bb = static_cast<int>(most < ds->sm_count * 3 ? most : ds->sm_count * 3);
+    const long long most = rows * slices;
+    const int gb = static_cast<int>(most < ds->sm_count * 6 ? most : ds->sm_count * 6);
     constexpr int kBigRing = kBigSlots * kBigStage * 256;
-    static bool attr_set[64] = {};
-    if (!attr_set[ds->device]) {
-      GB_CUDA_OK(cudaFuncSetAttribute(emb_big_bucket_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBigRing));
-      attr_set[ds->device] = true;
-    }
-    emb_big_bucket_kernel<T><<<bb, kBigThreads, kBigRing, st>>>(q, Gb, d, slices, pre_scale, divisor, accumulate, out);
-    count_launch(2);
+    emb_grad_kernel<T><<<gb, kEmbGradThreads, kBigRing, st>>>(q, Gb, d, slices, pre_scale, divisor, accumulate, out);
+    count_launch();
   }
   return post_launch("ghost_embedding_pass");
 }
