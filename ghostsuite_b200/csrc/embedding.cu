@@ -261,7 +261,7 @@ __global__ void __launch_bounds__(256) emb_count_kernel(const EmbBuckets q, floa
 }
 
 // Buckets may lie in any order, so a block of ids takes its space with one atomic instead of waiting for
-// a scan over the whole table (22 us in one block for 50 k ids, 4 us now).  Also listed here: the
+// a scan over the whole table (22 us in one block for 50 k ids, 4.6 us now).  Also listed here: the
 // gradient's rows by size, join items, and ids that many validation tokens share (padding, separators).
 __global__ void __launch_bounds__(256) emb_alloc_kernel(const EmbBuckets q) {
   __shared__ int s_warp[3][8], s_base[3];
@@ -290,31 +290,48 @@ __global__ void __launch_bounds__(256) emb_alloc_kernel(const EmbBuckets q) {
     s_base[threadIdx.x] = sum ? atomicAdd(q.totals + (threadIdx.x == 2 ? 5 : threadIdx.x), sum) : 0;
   }
   __syncthreads();
-  if (!in) return;
   const int off = s_base[0] + s_warp[0][warp] + before[0];
-  q.off_b[id] = off;
+  if (in) q.off_b[id] = off;
   if (n[2]) q.small[s_base[2] + s_warp[2][warp] + before[2]] = make_int4(id, off, tokens, 0);
   if (q.want_rows && n[0] > kEmbSmallBucket) q.big[atomicAdd(q.totals + 2, 1)] = id;
   if (q.cnt_v == nullptr) return;
   const int off_v = s_base[1] + s_warp[1][warp] + before[1];
-  q.off_v[id] = off_v;
-  if (n[1] == 0 || n[0] == 0) return;
-  int slot = -1;
-  if (n[1] > q.hot_threshold) {
-    slot = atomicAdd(q.totals + 4, 1);
-    if (slot < kEmbHotCap) q.hot[slot] = id; else slot = -1;
+  if (in) q.off_v[id] = off_v;
+  int slot = -1, parts = 0;
+  if (n[1] > 0 && n[0] > 0) {
+    if (n[1] > q.hot_threshold) {
+      slot = atomicAdd(q.totals + 4, 1);
+      if (slot < kEmbHotCap) q.hot[slot] = id; else slot = -1;
+    }
+    parts = slot >= 0 ? 1 : (n[1] + kEmbValChunk - 1) / kEmbValChunk;
+    // more hot ids than slots: their long validation lists stay in one item per train chunk
+    if (parts > q.max_parts) parts = -1;
   }
-  const int chunks = (n[0] + kEmbChunk - 1) / kEmbChunk, parts = slot >= 0 ? 1 : (n[1] + kEmbValChunk - 1) / kEmbValChunk;
-  // more hot ids than slots: their long validation lists stay in one item per train chunk
-  const bool long_list = parts > q.max_parts;
-  int at = atomicAdd(q.totals + 3, chunks * (long_list ? 1 : parts));
-  for (int c = 0; c < chunks; ++c) {
-    const int b0 = off + c * kEmbChunk, nb = min(kEmbChunk, n[0] - c * kEmbChunk);
-    if (slot >= 0) q.items[at++] = make_int4(b0, nb, slot, -1);
-    else if (long_list) q.items[at++] = make_int4(b0, nb, off_v, n[1]);
-    else
-      for (int v = 0; v < parts; ++v)
-        q.items[at++] = make_int4(b0, nb, off_v + v * kEmbValChunk, min(kEmbValChunk, n[1] - v * kEmbValChunk));
+  // the items of an id are written by the whole warp: a frequent word has hundreds
+  const int count = (n[0] + kEmbChunk - 1) / kEmbChunk * (parts < 0 ? 1 : parts);
+  int at = count;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, at, o);
+    if (lane >= o) at += y;
+  }
+  const int warp_items = __shfl_sync(0xffffffffu, at, 31);
+  int base = 0;
+  if (lane == 0 && warp_items > 0) base = atomicAdd(q.totals + 3, warp_items);
+  at += __shfl_sync(0xffffffffu, base, 0) - count;
+  for (unsigned todo = __ballot_sync(0xffffffffu, count > 0); todo != 0; todo &= todo - 1) {
+    const int who = __ffs(todo) - 1;
+    const int w_count = __shfl_sync(0xffffffffu, count, who), w_at = __shfl_sync(0xffffffffu, at, who);
+    const int w_parts = __shfl_sync(0xffffffffu, parts, who), w_slot = __shfl_sync(0xffffffffu, slot, who);
+    const int w_b = __shfl_sync(0xffffffffu, off, who), w_nb = __shfl_sync(0xffffffffu, n[0], who);
+    const int w_v = __shfl_sync(0xffffffffu, off_v, who), w_nv = __shfl_sync(0xffffffffu, n[1], who);
+    for (int i = lane; i < w_count; i += 32) {
+      const int c = w_parts > 1 ? i / w_parts : i, v = w_parts > 1 ? i % w_parts : 0;
+      const int4 rows = w_slot >= 0   ? make_int4(0, 0, w_slot, -1)
+                        : w_parts < 0 ? make_int4(0, 0, w_v, w_nv)
+                                      : make_int4(0, 0, w_v + v * kEmbValChunk, min(kEmbValChunk, w_nv - v * kEmbValChunk));
+      q.items[w_at + i] = make_int4(w_b + c * kEmbChunk, min(kEmbChunk, w_nb - c * kEmbChunk), rows.z, rows.w);
+    }
   }
 }
 
@@ -572,13 +589,20 @@ __device__ __forceinline__ void emb_small_rows(const EmbBuckets& q, const T* __r
     const long long first = __shfl_sync(0xffffffffu, mine, 0);
     if (first >= total) return;
     mine = grab();
-    const long long last = first + kEmbGrab < total ? first + kEmbGrab : total;
-    int4 entry = q.small[first / steps];
-    for (long long w = first; w < last; ++w) {
+    // (row, step) of the first item by one division, of the others by counting on
+    int row = total <= INT_MAX ? static_cast<int>(static_cast<unsigned>(first) / static_cast<unsigned>(steps))
+                               : static_cast<int>(first / steps);
+    int step = static_cast<int>(first - static_cast<long long>(row) * steps);
+    int items = static_cast<int>(first + kEmbGrab < total ? kEmbGrab : total - first);
+    int4 entry = q.small[row];
+    for (; items > 0; --items) {
       const int k = entry.x, off = entry.y, n = entry.z;
-      const int f = static_cast<int>(w % steps) * 256 + lane * 8;
+      const int f = step * 256 + lane * 8;
       int tok = lane < n ? q.perm_b[off + lane] : INT_MAX;
-      if (w + 1 < last) entry = q.small[(w + 1) / steps];
+      if (++step == steps) {
+        step = 0;
+        if (++row < q.totals[5]) entry = q.small[row];
+      }
       // bitonic sort of the first n keys, ascending
 #pragma unroll
       for (int size = 2; size <= 32; size <<= 1) {
@@ -596,8 +620,9 @@ __device__ __forceinline__ void emb_small_rows(const EmbBuckets& q, const T* __r
           Raw x[kBatch];
 #pragma unroll
           for (int r = 0; r < kBatch; ++r) {
+            if (i0 + r >= n) break;
             const int j = __shfl_sync(0xffffffffu, tok, i0 + r);
-            x[r] = i0 + r < n && f < d ? EmbRaw<T>::load(G + static_cast<long long>(j) * d + f) : EmbRaw<T>::zero();
+            x[r] = f < d ? EmbRaw<T>::load(G + static_cast<long long>(j) * d + f) : EmbRaw<T>::zero();
           }
 #pragma unroll
           for (int r = 0; r < kBatch; ++r) {
@@ -749,7 +774,7 @@ __device__ __forceinline__ void emb_big_rows(const EmbBuckets& q, const T* __res
 
 // One launch for both: every CTA takes its share of the long rows, whose chains are the longest, and goes on
 // with the short ones.  Apart, a launch of each (text ids, 40 x 1024 tokens of 768 bf16 features) took 46 and
-// 35 us, mostly with a few warps left per SM; MEASURED_NEW.
+// 35 us, mostly with a few warps left per SM; 39 us together, 30 of them the longest rows' chains.
 template <typename T>
 __global__ void __launch_bounds__(kEmbGradThreads, 6)
 emb_grad_kernel(const EmbBuckets q, const T* __restrict__ G, int d, int slices, float pre_scale, float divisor,

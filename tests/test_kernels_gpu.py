@@ -821,3 +821,26 @@ def test_rmsnorm_persample(shape, dtype):
     tol = 1e-4 if dtype == torch.float32 else 2e-2
     assert O.rel_fro(gw, want) < tol
     assert O.rel_fro(gsum, G.double().sum(1)) < tol
+
+
+# ids with 1 to 40 train and up to 4 validation tokens: load batches, sort sizes, the line between short and long
+# rows, several join items an id; divisors on and off a power of two
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("n_t,n_v,d", [(8, 3, 8), (8, 2, 264), (6, 3, 768), (1, 1, 520), (16, 4, 1024), (5, 2, 37)])
+def test_embedding_hook_small_rows_exact(dtype, n_t, n_v, d):
+    """Whole numbers up to 3: the matrix and the sums are exact in any order, the gradient is two roundings."""
+    gen = torch.Generator().manual_seed(d + n_t)
+    train = [k for k in range(60) for _ in range(k % 41)]
+    val = [k for k in range(60) for _ in range((k * 7) % 5)]
+    T = max(-(-len(train) // n_t), -(-len(val) // n_v))
+    train += [63] * (n_t * T - len(train))             # an id of the train tokens only
+    val += [62] * (n_v * T - len(val))                 # and one of the validation tokens only
+    ids = torch.cat([torch.tensor(train)[torch.randperm(n_t * T, generator=gen)].view(n_t, T),
+                     torch.tensor(val)[torch.randperm(n_v * T, generator=gen)].view(n_v, T)])
+    G = torch.randint(-3, 4, (n_t + n_v, T, d), generator=gen).to(dtype)
+    M, grad = ops().embedding_hook(ids.cuda(), G.cuda(), n_v, 64, 1.0)
+    after()
+    per = torch.zeros(n_t + n_v, 64, d, dtype=torch.float64)
+    per.scatter_add_(1, ids.unsqueeze(-1).expand(-1, -1, d), G.double())
+    assert torch.equal(M.cpu().double(), per[n_t:].flatten(1) @ per[:n_t].flatten(1).T)
+    assert torch.equal(grad.cpu(), (per[:n_t].sum(0).to(dtype) / n_t).to(dtype))
