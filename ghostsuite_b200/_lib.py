@@ -137,9 +137,13 @@ def named_parameters(module) -> list:
     """``list(module.named_parameters())`` for a module on a GPU without its nested generators, which
     cost more than what a step does with each parameter.  Walks the live tree, so later changes of
     the model count; without the binding (CPU-only use of the engines' bookkeeping) torch's own."""
-    if not os.path.exists(BINDING_PATH):
+    from torch.nn import Module
+    own = type(module)
+    if own.named_parameters is not Module.named_parameters or own.named_modules is not Module.named_modules \
+            or not os.path.exists(BINDING_PATH):
         return list(module.named_parameters())
-    return native().named_parameters(module)
+    found = native().named_parameters(module)
+    return list(module.named_parameters()) if found is None else found
 
 
 def last_error() -> str:

@@ -90,3 +90,24 @@ def test_choose_ki_ko_reproduces_the_reference_table(golden):
     assert table.shape[0] >= 7
     for n_i, n_o, k_total, k_min, k_i, k_o in table.tolist():
         assert choose_ki_ko(n_i, n_o, k_total, k_min) == (k_i, k_o), (n_i, n_o, k_total, k_min)
+
+
+def test_parameter_walk_of_modules_with_tables_of_their_own():
+    """Wrappers that rename their parameters, scripted modules and shared parameters: as torch lists them."""
+    from ghostsuite_b200 import _lib
+
+    class Renaming(nn.Module):
+        def __init__(self):
+            super().__init__()
+            self.inner = nn.Linear(2, 2)
+
+        def named_parameters(self, *args, **kwargs):
+            for name, p in super().named_parameters(*args, **kwargs):
+                yield name.replace("inner.", ""), p
+
+    tied = nn.Sequential(nn.Linear(2, 2), nn.Linear(2, 2))
+    tied[1].weight = tied[0].weight
+    for m in (Renaming(), torch.jit.script(nn.Linear(2, 2)), nn.Sequential(torch.jit.script(nn.Linear(2, 2))), tied):
+        want, got = list(m.named_parameters()), _lib.named_parameters(m)
+        assert [n for n, _ in got] == [n for n, _ in want]
+        assert all(a.data_ptr() == b.data_ptr() for (_, a), (_, b) in zip(got, want))
