@@ -177,7 +177,7 @@ __global__ void __launch_bounds__(256, 2) dense_small_kernel(const SmallDense q)
       }
       __syncthreads();
     }
-    const bool quad = (n & 3) == 0;
+    const bool quad = (n & 3) == 0 && (reinterpret_cast<uintptr_t>(q.grad) & 15u) == 0;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const int r = m0 + ty * 4 + i, c = n0 + tx * 4;

@@ -706,7 +706,8 @@ def _conv_hook(layer: nn.Conv2d, A: torch.Tensor, B: torch.Tensor, n_val: int) -
     mode other than zeros or padding given by name, other data types)."""
     own = layer.__dict__
     if "_ghost_backprop_scale" not in own or n_val <= 0 or layer.groups != 1 or layer.padding_mode != "zeros" \
-            or isinstance(layer.padding, str) or A.dtype not in _GRAD_TYPES or B.dtype is not A.dtype or A.dim() != 4:
+            or isinstance(layer.padding, str) or A.dtype not in _GRAD_TYPES or B.dtype is not A.dtype or A.dim() != 4 \
+            or A.size(0) > 65535 or layer.weight[0].numel() > 1 << 21:      # limits of the kernel's grid
         return False
     weight, bias = layer.weight, layer.bias
     n_train = A.size(0) - n_val
