@@ -451,11 +451,11 @@ PyObject* py_dense_hook(PyObject*, PyObject* const* a, Py_ssize_t n) {
         ghost_dense_small_fits(is_f32(A), static_cast<int>(n_train), static_cast<int>(n_val), A.size(1), dI, pI)) {
       M = empty({n_val, n_train}, A, at::kFloat);
       grad = optional_empty({X.size(2), Y.size(2)}, X, gdt);
-      const bool copy = bias && !(A.size(1) == 1 && is_f32(B));    // one float32 token: its rows are the sums
-      if (bias) sums = copy ? empty({N, p}, A, at::kFloat) : B.view({N, p});
+      // written out even for one float32 token, whose row is the sum: they are read when the pass ends
+      if (bias) sums = empty({N, p}, A, at::kFloat);
       check(ghost_dense_small(A.data_ptr(), B.data_ptr(), is_f32(A), static_cast<int>(n_train), static_cast<int>(n_val),
                               A.size(1), dI, pI, in_by_out ? 1 : 0, M.data_ptr<float>(), grad.defined() ? grad.data_ptr() : nullptr,
-                              grad.defined() ? is_f32(grad) : 0, scale, copy ? sums.data_ptr<float>() : nullptr, L.st()));
+                              grad.defined() ? is_f32(grad) : 0, scale, bias ? sums.data_ptr<float>() : nullptr, L.st()));
     } else {
       dense_paths(L, Operand(A), Operand(B), n_val, in_by_out, gram, gdt, scale, bias, M, grad, sums);
     }
@@ -841,15 +841,18 @@ PyObject* py_matrix_sum(PyObject*, PyObject* const* a, Py_ssize_t n) {
 }
 
 // (module) -> [(qualified name, parameter)] as module.named_parameters() gives them: every parameter once,
-// modules in depth-first order.  The engines walk the model three times a step.
-void walk_parameters(PyObject* module, const std::string& prefix, std::set<PyObject*>& seen, PyObject* out) {
-  if (!seen.insert(module).second) return;
+// modules in depth-first order.  The engines walk the model three times a step.  False: a module keeps its
+// tables elsewhere than in its dictionary (scripted modules), and the caller asks torch.
+bool walk_parameters(PyObject* module, const std::string& prefix, std::set<PyObject*>& seen, PyObject* out) {
+  if (!seen.insert(module).second) return true;
   PyObject* dict = PyObject_GetAttrString(module, "__dict__");
-  if (!dict) { PyErr_Clear(); return; }
+  if (!dict) { PyErr_Clear(); return false; }
   PyObject *key, *value;
   Py_ssize_t pos = 0;
   PyObject* params = PyDict_Check(dict) ? PyDict_GetItemString(dict, "_parameters") : nullptr;
-  if (params && PyDict_Check(params)) {
+  PyObject* modules = PyDict_Check(dict) ? PyDict_GetItemString(dict, "_modules") : nullptr;
+  bool ok = params && PyDict_Check(params) && modules && PyDict_Check(modules);
+  if (ok) {
     while (PyDict_Next(params, &pos, &key, &value)) {
       if (value == Py_None || !seen.insert(value).second) continue;
       const char* name = PyUnicode_AsUTF8(key);
@@ -858,16 +861,16 @@ void walk_parameters(PyObject* module, const std::string& prefix, std::set<PyObj
       Py_DECREF(entry);
     }
   }
-  PyObject* modules = PyDict_Check(dict) ? PyDict_GetItemString(dict, "_modules") : nullptr;
-  if (modules && PyDict_Check(modules)) {
+  if (ok) {
     pos = 0;
-    while (PyDict_Next(modules, &pos, &key, &value)) {
+    while (ok && PyDict_Next(modules, &pos, &key, &value)) {
       if (value == Py_None) continue;
       const char* name = PyUnicode_AsUTF8(key);
-      walk_parameters(value, prefix + (name ? name : "") + ".", seen, out);
+      ok = walk_parameters(value, prefix + (name ? name : "") + ".", seen, out);
     }
   }
   Py_DECREF(dict);
+  return ok;
 }
 
 PyObject* py_named_parameters(PyObject*, PyObject* const* a, Py_ssize_t n) {
@@ -877,7 +880,10 @@ PyObject* py_named_parameters(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (!out) throw std::bad_alloc();
     std::set<PyObject*> seen;
     try {
-      walk_parameters(a[0], "", seen, out);
+      if (!walk_parameters(a[0], "", seen, out)) {
+        Py_DECREF(out);
+        Py_RETURN_NONE;
+      }
     } catch (...) {
       Py_DECREF(out);
       throw;
