@@ -300,7 +300,123 @@ __global__ void layernorm_reduce_kernel(const float* __restrict__ part, int N, i
   }
 }
 
-// generic F: one block per (sample, split); rows handled one at a time by the whole block
+// F beyond the warp-per-row kernel (above 1024, or no multiple of eight) up to 8192: a block owns the whole
+// width, a thread PT features of it (pieces of eight, or every THREADS-th feature when rows are not
+// 16-byte aligned), and R = 32 / PT rows go through the two reductions together, so their loads are in
+// flight at once and one barrier serves R rows.  The gradients of a thread's features stay in registers.
+// Bound by the latency of a group of rows (loads, two reductions) more than by HBM: 3 to 4 TB/s.  The
+// block-per-row kernel below reads every row three times in single elements and meets at four
+// barriers per row; whole LayerNorm hook, 24 samples of 1024 rows of bf16: F = 4096 803 -> 138 us, F = 2048
+// 380 -> 97, F = 731 173 -> 60; RMS norm, 12 x 1024 rows of F = 8192: 1179 -> 138.
+template <typename T, bool VEC, int PT, int THREADS>
+__global__ void __launch_bounds__(THREADS, THREADS == 256 ? 2 : 1)
+norm_wide_kernel(const T* __restrict__ A, const T* __restrict__ G, long long Tn, int F, float eps, float* __restrict__ gw,
+                 float* __restrict__ gb, float* __restrict__ part, int t_splits, int rms) {
+  constexpr int R = 32 / PT, W = THREADS / 32;
+  __shared__ float red[2][R][W];
+  const int n = blockIdx.y, split = blockIdx.x;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const long long per = (Tn + t_splits - 1) / t_splits;
+  const long long t0 = split * per;
+  const long long t1 = (t0 + per < Tn) ? t0 + per : Tn;
+  const float invF = 1.f / static_cast<float>(F);
+  auto feature = [&](int e) -> int {
+    return VEC ? (e / 8) * THREADS * 8 + static_cast<int>(threadIdx.x) * 8 + e % 8 : e * THREADS + static_cast<int>(threadIdx.x);
+  };
+  auto load = [&](const T* row, float (&x)[PT]) {
+    if constexpr (VEC) {
+#pragma unroll
+      for (int c = 0; c < PT / 8; ++c) {
+        float v[8];
+        if (feature(c * 8) < F) {
+          Vec8<T>::load(row + feature(c * 8), v);
+        } else {
+#pragma unroll
+          for (int j = 0; j < 8; ++j) v[j] = 0.f;
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) x[c * 8 + j] = v[j];
+      }
+    } else {
+#pragma unroll
+      for (int e = 0; e < PT; ++e) x[e] = feature(e) < F ? to_f32<T>(row[feature(e)]) : 0.f;
+    }
+  };
+  int buf = 0;
+  // sums of one value per row over the block; the buffers alternate, so one barrier is enough
+  auto block_sum = [&](float (&s)[R]) {
+#pragma unroll
+    for (int r = 0; r < R; ++r) s[r] = warp_sum(s[r]);
+    if (lane == 0)
+#pragma unroll
+      for (int r = 0; r < R; ++r) red[buf][r][warp] = s[r];
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      s[r] = 0.f;
+#pragma unroll
+      for (int w = 0; w < W; ++w) s[r] += red[buf][r][w];
+    }
+    buf ^= 1;
+  };
+  float aw[PT], ab[PT];
+#pragma unroll
+  for (int e = 0; e < PT; ++e) { aw[e] = 0.f; ab[e] = 0.f; }
+  for (long long t = t0; t < t1; t += R) {
+    float x[R][PT], g[R][PT], s[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const long long row = (static_cast<long long>(n) * Tn + (t + r < t1 ? t + r : t)) * F;
+      load(A + row, x[r]);
+      load(G + row, g[r]);
+    }
+    if (!rms) {                          // RMS norm: no centring
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        s[r] = 0.f;
+#pragma unroll
+        for (int e = 0; e < PT; ++e) s[r] += x[r][e];
+      }
+      block_sum(s);
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+#pragma unroll
+        for (int e = 0; e < PT; ++e) x[r][e] = feature(e) < F ? x[r][e] - s[r] * invF : 0.f;
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      s[r] = 0.f;
+#pragma unroll
+      for (int e = 0; e < PT; ++e) s[r] += x[r][e] * x[r][e];
+    }
+    block_sum(s);
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      if (t + r >= t1) break;
+      const float rstd = rsqrtf(s[r] * invF + eps);
+#pragma unroll
+      for (int e = 0; e < PT; ++e) {
+        aw[e] = fmaf(g[r][e], x[r][e] * rstd, aw[e]);
+        ab[e] += g[r][e];
+      }
+    }
+  }
+#pragma unroll
+  for (int e = 0; e < PT; ++e) {
+    const int f = feature(e);
+    if (f >= F) continue;
+    if (t_splits > 1) {
+      float* dst = part + (static_cast<long long>(split) * gridDim.y + n) * 2 * F;
+      dst[f] = aw[e];
+      dst[F + f] = ab[e];
+    } else {
+      gw[static_cast<long long>(n) * F + f] = aw[e];
+      gb[static_cast<long long>(n) * F + f] = ab[e];
+    }
+  }
+}
+
+// F above 8192: one block per (sample, split); rows handled one at a time by the whole block
 template <typename T>
 __global__ void __launch_bounds__(256)
 layernorm_persample_generic_kernel(const T* __restrict__ A, const T* __restrict__ G, long long Tn, int F,
@@ -429,40 +545,51 @@ extern "C" int ghost_colsum(const void* G, int is_f32, int N, long long T, int c
   return post_launch("colsum_kernel");
 }
 
-static int ln_splits(long long Tn, int N, int sm_count) {
-  long long want = (2ll * sm_count) / N;   // at most two resident CTAs per SM: one wave
-  const long long maxs = (Tn + 63) / 64;
+static int ln_splits(long long Tn, int N, int resident, int min_rows) {
+  long long want = resident / N;           // one wave
+  const long long maxs = (Tn + min_rows - 1) / min_rows;
   if (want > maxs) want = maxs;
   if (want < 1) want = 1;
-  if (want > 65535) want = 65535;
   return static_cast<int>(want);
 }
 
+// Rows below which another split costs more than it gives: a warp of the warp-per-row kernel should see eight,
+// a block of the wide kernel goes through its rows two to eight at a time.
+static constexpr int kLnMinRows = 64, kLnWideMinRows = 8;
+
 extern "C" long long ghost_layernorm_workspace_bytes(int N, long long T, int F) {
-  // upper bound over devices: at most 1024 splits are ever used
-  long long splits = (T + 63) / 64;
-  if (splits > 1024) splits = 1024;
+  // one wave of at most two CTAs per SM over the N samples: 512 is above any device this runs on
+  long long splits = (T + kLnWideMinRows - 1) / kLnWideMinRows;
+  const long long wave = N > 0 ? 512 / N : 1;
+  if (splits > wave) splits = wave;
+  if (splits < 1) splits = 1;
   return splits * N * 2 * F * 4 + 256;
+}
+
+template <typename T, bool VEC>
+static void launch_norm_wide(dim3 grid, const T* A, const T* G, long long Tn, int F, float eps, float* gw, float* gb, float* ws,
+                             int splits, cudaStream_t st, int rms) {
+  if (!VEC && F <= 1024) norm_wide_kernel<T, false, 4, 256><<<grid, 256, 0, st>>>(A, G, Tn, F, eps, gw, gb, ws, splits, rms);
+  else if (F <= 2048) norm_wide_kernel<T, VEC, 8, 256><<<grid, 256, 0, st>>>(A, G, Tn, F, eps, gw, gb, ws, splits, rms);
+  else if (F <= 4096) norm_wide_kernel<T, VEC, 16, 256><<<grid, 256, 0, st>>>(A, G, Tn, F, eps, gw, gb, ws, splits, rms);
+  else norm_wide_kernel<T, VEC, 16, 512><<<grid, 512, 0, st>>>(A, G, Tn, F, eps, gw, gb, ws, splits, rms);
 }
 
 template <typename T>
 static int launch_ln(const T* A, const T* G, int N, long long Tn, int F, float eps, float* gw, float* gb,
                      float* ws, long long ws_bytes, const DeviceState* ds, cudaStream_t st, int rms) {
-  const bool fast = (F % 8 == 0) && (F <= 1024) &&
-                    ((reinterpret_cast<uintptr_t>(A) & 15u) == 0) && ((reinterpret_cast<uintptr_t>(G) & 15u) == 0);
-  if (fast) {
-    int splits = ln_splits(Tn, N, ds->sm_count);
-    if (splits > 1024) splits = 1024;
-    if (splits > 1) {
-      GB_REQUIRE(ws && ws_bytes >= static_cast<long long>(splits) * N * 2 * F * 4,
-                 "ghost_layernorm_persample: workspace too small");
-    }
+  const bool aligned = (F % 8 == 0) && ((reinterpret_cast<uintptr_t>(A) & 15u) == 0) && ((reinterpret_cast<uintptr_t>(G) & 15u) == 0);
+  const int resident = (F <= 4096 ? 2 : 1) * (ds->sm_count < 256 ? ds->sm_count : 256);
+  int splits = ln_splits(Tn, N, resident, aligned && F <= 1024 ? kLnMinRows : kLnWideMinRows);
+  const bool room = splits == 1 || (ws && ws_bytes >= static_cast<long long>(splits) * N * 2 * F * 4);
+  if (aligned && F <= 1024) GB_REQUIRE(room, "ghost_layernorm_persample: workspace too small");
+  if (F <= 8192 && room) {               // the kernel after it needs no workspace
     dim3 grid(splits, N);
     // per-warp cp.async rings (3 slots x (A row + G row)), reused for the cross-warp reduction
     const size_t ring = sizeof(T) * 8 * kLnSlots * 2 * static_cast<size_t>(F);
     const size_t red = sizeof(float) * 8 * 2 * static_cast<size_t>(F);
     const size_t smem = ring > red ? ring : red;
-    const int nchunk = (F + 255) / 256;
+    const int nchunk = aligned ? (F + 255) / 256 : 0;
 #define GB_LN_LAUNCH(NC)                                                                              \
     do {                                                                                              \
       if (smem > 48 * 1024)                                                                           \
@@ -471,10 +598,12 @@ static int launch_ln(const T* A, const T* G, int N, long long Tn, int F, float e
       layernorm_persample_kernel<T, NC><<<grid, 256, smem, st>>>(A, G, Tn, F, eps, gw, gb, ws, splits, rms); \
     } while (0)
     switch (nchunk) {
+      case 0: launch_norm_wide<T, false>(grid, A, G, Tn, F, eps, gw, gb, ws, splits, st, rms); break;
       case 1: GB_LN_LAUNCH(1); break;
       case 2: GB_LN_LAUNCH(2); break;
       case 3: GB_LN_LAUNCH(3); break;
-      default: GB_LN_LAUNCH(4); break;
+      case 4: GB_LN_LAUNCH(4); break;
+      default: launch_norm_wide<T, true>(grid, A, G, Tn, F, eps, gw, gb, ws, splits, st, rms); break;
     }
 #undef GB_LN_LAUNCH
     count_launch();
@@ -487,7 +616,7 @@ static int launch_ln(const T* A, const T* G, int N, long long Tn, int F, float e
     count_launch();
     return post_launch("layernorm_reduce_kernel");
   }
-  const int splits = pick_splits(Tn, N, ds->sm_count, 32);
+  splits = pick_splits(Tn, N, ds->sm_count, 32);
   if (splits > 1) {
     GB_CUDA_OK(cudaMemsetAsync(gw, 0, sizeof(float) * static_cast<size_t>(N) * F, st));
     GB_CUDA_OK(cudaMemsetAsync(gb, 0, sizeof(float) * static_cast<size_t>(N) * F, st));

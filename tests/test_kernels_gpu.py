@@ -844,3 +844,23 @@ def test_embedding_hook_small_rows_exact(dtype, n_t, n_v, d):
     per.scatter_add_(1, ids.unsqueeze(-1).expand(-1, -1, d), G.double())
     assert torch.equal(M.cpu().double(), per[n_t:].flatten(1) @ per[:n_t].flatten(1).T)
     assert torch.equal(grad.cpu(), (per[:n_t].sum(0).to(dtype) / n_t).to(dtype))
+
+
+# widths around the lines of the block-per-rows kernel (1024, 2048, 4096, 8192, multiples of eight or not), row
+# counts that leave a group of rows unfinished, one row, several splits
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("rms", [False, True])
+@pytest.mark.parametrize("N,T,F", [(2, 1, 1032), (3, 5, 2048), (1, 387, 731), (2, 130, 4104), (2, 33, 8192), (1, 9, 8189),
+                                   (2, 67, 1025), (3, 200, 2056), (1, 3, 8200), (5, 7, 3)])
+def test_norm_wide_rows(dtype, rms, N, T, F):
+    gen = torch.Generator().manual_seed(F)
+    A = (torch.randn(N, T, F, generator=gen) * 1.5 + 0.3).to(dtype)
+    G = (torch.randn(N, T, F, generator=gen) / F ** 0.5).to(dtype)
+    gw, gb = ops().layernorm_persample(A.cuda(), G.cuda(), 1e-5, rms=rms)
+    after()
+    x, g = A.double(), G.double()
+    x = x if rms else x - x.mean(-1, keepdim=True)
+    x = x / (x.pow(2).mean(-1, keepdim=True) + 1e-5).sqrt()
+    # float32 sums of F values and of T rows around values of order one: a few ulp of sqrt(F + T)
+    assert O.rel_fro(gw, (g * x).sum(1)) < 2e-6
+    assert O.rel_fro(gb, g.sum(1)) < 2e-6
