@@ -22,38 +22,49 @@ template <> __device__ __forceinline__ float ct_f32<__nv_bfloat16>(__nv_bfloat16
 
 // A 64-token x 64-feature tile per block, turned in shared memory: lanes run over tokens for the loads
 // (adjacent positions of one input row) and over features for the stores (128 bytes of an output
-// row).  Bound by the stores, which are kh * kw * parts times the input.  The library unfold before it
-// ran one launch per sample and produced [features, tokens], transposed and split by two more passes:
-// 575 us for 80 samples of 64 x 16 x 16 with a 3 x 3 window, against 19 us.
+// row).  Bound by issue slots: the divisions that find a feature's channel and window position are made once
+// a block (once a lane and feature they were half of all instructions: 52 us for the operands of 80
+// samples of 64 x 16 x 16 with a 3 x 3 window and 128 outputs, float32; 24.6 now), and hi and lo parts
+// once an element.  The library unfold before it ran one launch per sample and two more passes: 575 us.
 template <typename E>
 __global__ void __launch_bounds__(256) conv_tokens_kernel(const ConvTokens q) {
   __shared__ float tile[64][65];
-  const long long t0 = blockIdx.x * 64ll;
+  __shared__ long long s_off[64];        // of a feature: channel and window position as an offset into the sample
+  __shared__ int2 s_ij[64];              // and the position alone; far outside for the padding features
+  constexpr int kFar = -(1 << 30);
+  const unsigned t0 = blockIdx.x * 64u;  // tokens of a sample fit an int
   const int f0 = blockIdx.y * 64;
   const long long n = blockIdx.z;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const unsigned tokens = static_cast<unsigned>(q.T);
   const E* src = static_cast<const E*>(q.src) + n * q.C * q.H * q.W;
-  int y0[2], x0[2];
-  bool ok[2];
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    const long long t = t0 + h * 32 + lane;
-    ok[h] = t < q.T;
-    const int oy = static_cast<int>(ok[h] ? t / q.Wo : 0), ox = static_cast<int>(ok[h] ? t % q.Wo : 0);
-    y0[h] = oy * q.sy - q.py;
-    x0[h] = ox * q.sx - q.px;
-  }
-  const int window = q.kh * q.kw;
-#pragma unroll
-  for (int r = 0; r < 8; ++r) {
-    const int f = f0 + warp * 8 + r;
+  if (threadIdx.x < 64) {
+    const int f = f0 + threadIdx.x, window = q.kh * q.kw;
     const int c = f / window, w = f % window;
     const int i = w / q.kw * q.dy, j = w % q.kw * q.dx;
+    s_off[threadIdx.x] = (static_cast<long long>(c) * q.H + i) * q.W + j;
+    s_ij[threadIdx.x] = make_int2(f < q.cols ? i : kFar, j);
+  }
+  int y0[2], x0[2];
+  long long base[2];
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const unsigned t = t0 + h * 32 + lane;
+    const int oy = static_cast<int>(t / static_cast<unsigned>(q.Wo)), ox = static_cast<int>(t % static_cast<unsigned>(q.Wo));
+    y0[h] = t < tokens ? oy * q.sy - q.py : kFar;
+    x0[h] = ox * q.sx - q.px;
+    base[h] = static_cast<long long>(y0[h]) * q.W + x0[h];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int r = 0; r < 8; ++r) {
+    const int2 ij = s_ij[warp * 8 + r];
+    const long long off = s_off[warp * 8 + r];
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-      const int y = y0[h] + i, x = x0[h] + j;
-      const bool in = f < q.cols && ok[h] && y >= 0 && y < q.H && x >= 0 && x < q.W;
-      tile[warp * 8 + r][h * 32 + lane] = in ? ct_f32<E>(src[(static_cast<long long>(c) * q.H + y) * q.W + x]) : 0.f;
+      const bool in = static_cast<unsigned>(y0[h] + ij.x) < static_cast<unsigned>(q.H) &&
+                      static_cast<unsigned>(x0[h] + ij.y) < static_cast<unsigned>(q.W);
+      tile[warp * 8 + r][h * 32 + lane] = in ? ct_f32<E>(src[base[h] + off]) : 0.f;
     }
   }
   __syncthreads();
@@ -61,25 +72,25 @@ __global__ void __launch_bounds__(256) conv_tokens_kernel(const ConvTokens q) {
   for (int h = 0; h < 2; ++h) {
     const int u = h * 256 + threadIdx.x;
     const int tl = u >> 3, fl = (u & 7) * 8;
-    const long long t = t0 + tl;
-    if (t >= q.T || f0 + fl >= q.cpad) continue;
-    float v[8];
+    const unsigned t = t0 + tl;
+    if (t >= tokens || f0 + fl >= q.cpad) continue;
+    uint32_t hw[4], lw[4];               // the values as bf16, and what that leaves of them
 #pragma unroll
-    for (int e = 0; e < 8; ++e) v[e] = tile[fl + e][tl];
-    for (int part = 0; part < q.parts; ++part) {
-      uint32_t w[4];
+    for (int e = 0; e < 4; ++e) {
+      const float va = tile[fl + 2 * e][tl], vb = tile[fl + 2 * e + 1][tl];
+      const __nv_bfloat162 hi = __floats2bfloat162_rn(va, vb);
+      const __nv_bfloat162 lo = __floats2bfloat162_rn(va - __bfloat162float(hi.x), vb - __bfloat162float(hi.y));
+      hw[e] = *reinterpret_cast<const uint32_t*>(&hi);
+      lw[e] = *reinterpret_cast<const uint32_t*>(&lo);
+    }
+    const long long stride = q.row_stack ? q.T * q.ld_dst : q.cpad;
+    __nv_bfloat16* dst = q.dst + (q.row_stack ? n * q.parts * q.T + t : n * q.T + t) * q.ld_dst + f0 + fl;
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        __nv_bfloat16 a = __float2bfloat16_rn(v[2 * e]), b = __float2bfloat16_rn(v[2 * e + 1]);
-        if (q.kind[part] == 1) {
-          a = __float2bfloat16_rn(v[2 * e] - __bfloat162float(a));
-          b = __float2bfloat16_rn(v[2 * e + 1] - __bfloat162float(b));
-        }
-        w[e] = static_cast<uint32_t>(__bfloat16_as_ushort(a)) | (static_cast<uint32_t>(__bfloat16_as_ushort(b)) << 16);
-      }
-      const long long at = q.row_stack ? ((n * q.parts + part) * q.T + t) * q.ld_dst + f0 + fl
-                                       : (n * q.T + t) * q.ld_dst + static_cast<long long>(part) * q.cpad + f0 + fl;
-      *reinterpret_cast<uint4*>(q.dst + at) = make_uint4(w[0], w[1], w[2], w[3]);
+    for (int part = 0; part < 3; ++part) {
+      if (part >= q.parts) break;
+      const bool low = q.kind[part] == 1;
+      *reinterpret_cast<uint4*>(dst + part * stride) =
+          make_uint4(low ? lw[0] : hw[0], low ? lw[1] : hw[1], low ? lw[2] : hw[2], low ? lw[3] : hw[3]);
     }
   }
 }
@@ -114,6 +125,7 @@ extern "C" int ghost_conv_tokens_bf16(const void* src, int src_is_f32, long long
   GB_REQUIRE(H + 2 * py > dy * (kh - 1) && W + 2 * px > dx * (kw - 1), "ghost_conv_tokens_bf16: the window is larger than the padded input");
   const long long cols = static_cast<long long>(C) * kh * kw;
   GB_REQUIRE(cols <= (1 << 22), "ghost_conv_tokens_bf16: too many features per token");
+  GB_REQUIRE(static_cast<long long>(Ho) * Wo < (1ll << 31) - 64, "ghost_conv_tokens_bf16: too many output positions");
   GB_REQUIRE(parts >= 1 && parts <= 3, "ghost_conv_tokens_bf16: parts must be 1..3");
   GB_REQUIRE(cpad % 8 == 0 && cpad >= cols && ld_dst % 8 == 0 && ld_dst >= (row_stack ? cpad : parts * cpad) &&
                  (reinterpret_cast<uintptr_t>(dst) & 15u) == 0, "ghost_conv_tokens_bf16: bad destination layout");
