@@ -844,10 +844,10 @@ def reference_gpu_leg(dev, reps: int = 5):
                 r_dot(layer, a, b, nv)
                 r_grad(layer, a, b, nv)           # the reference passes B * N here; the product is not timed
             elif kind == "conv1d":
-                O.conv1d_dot_reference(a, b, nv)
+                O.conv1d_dot_reference(a, b, nv, O.use_gram_rule(T, d * p))
                 O.conv1d_train_grad(a, b, nv)
             else:
-                O.linear_dot_reference(a, b, nv)
+                O.linear_dot_reference(a, b, nv, O.use_gram_rule(T, d * p))
                 O.linear_train_grad(a, b, nv)
 
         rec = {"layer": name, "n_train": n_t, "n_val": n_v, "T": T, "d_in": d, "d_out": p}
