@@ -499,7 +499,7 @@ def embedding_wgrad(ids: torch.Tensor, G: torch.Tensor, n_train: int, vocab: int
     if _timing is None:
         return _native().embedding_wgrad(*args)
     share = n_train / max(1, G.shape[0])
-    with _Timed("emb_segsum_kernel", "hbm", 0.0,
+    with _Timed("emb_grad_kernel", "hbm", 0.0,
                 (share * G.numel() + float(vocab) * _cols(G)) * G.element_size() + 8.0 * share * ids.numel()):
         return _native().embedding_wgrad(*args)
 
@@ -510,7 +510,7 @@ def embedding_hook(ids: torch.Tensor, G: torch.Tensor, n_val: int, vocab: int, p
     args = (ids, G, n_val, vocab, pre_scale)
     if _timing is None:
         return _native().embedding_hook(*args)
-    with _Timed("emb_join_kernel+emb_segsum_kernel", "hbm", 0.0,
+    with _Timed("emb_join_kernel+emb_grad_kernel", "hbm", 0.0,
                 (float(G.numel()) + float(vocab) * _cols(G)) * G.element_size() + 8.0 * ids.numel()):
         return _native().embedding_hook(*args)
 
