@@ -71,11 +71,13 @@ def register_hook_pair(layer: nn.Module, capture, backward_hook):
     """Register ``capture(layer, inputs, outputs)`` on the forward pass and ``backward_hook(layer,
     grad_input, (grad,))`` on the output's gradient; returns the removable handles.
 
-    The backward hooks read the output gradient only, so a hook on the output tensor serves them; a
-    module's full backward hook wraps input and output in two more autograd nodes per call (about
-    60 us of host time per layer and step) and hands over the same tensor later.  Embeddings keep the
-    module hook: their input has no gradient, in which case a module hook that a user registers
-    after this one fires at the output too, and would come before a hook on the tensor inside."""
+    The backward hooks read the output gradient only, so a hook on the autograd node that produced the
+    output serves them; a module's full backward hook wraps input and output in two more nodes per call
+    (about 60 us of host time per layer and step).  On the node, like there, the gradient is what the
+    hooks that a user has put on the output tensor leave of it, and ``autograd.grad`` up to the output
+    calls nothing.  Embeddings keep the module hook: their input has no gradient, in which case a module
+    hook that a user registers after this one fires at the output too, and would come before a hook on
+    the node inside."""
     if isinstance(layer, nn.Embedding):
         return [layer.register_forward_hook(capture), layer.register_full_backward_hook(backward_hook)]
 
@@ -88,11 +90,13 @@ def register_hook_pair(layer: nn.Module, capture, backward_hook):
             return
         capture(layer, inputs, outputs)
         if out is not None and out.requires_grad and torch.is_grad_enabled():
-            def on_gradient(grad):
-                layer.__dict__["_ghost_done_in"] = torch._C._current_graph_task_id()
-                backward_hook(layer, None, (grad,))
+            node, index = out.grad_fn, out.output_nr
 
-            out.register_hook(on_gradient)
+            def on_gradients(grads):
+                layer.__dict__["_ghost_done_in"] = torch._C._current_graph_task_id()
+                backward_hook(layer, None, (grads[index],))
+
+            node.register_prehook(on_gradients)
 
     return [layer.register_forward_hook(forward_hook)]
 

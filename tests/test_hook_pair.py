@@ -1,0 +1,79 @@
+"""The pair of hooks that both engines put on a layer: which gradient and which input the backward hook
+gets.  Its product must be the weight gradient that autograd itself computes."""
+import pytest
+import torch
+import torch.nn.functional as F
+from torch import nn
+from transformers.pytorch_utils import Conv1D
+
+from ghostsuite_b200.ghostEngines.autograd_grad_sample_dotprod import register_hook_pair
+
+LAYERS = {"linear": lambda: nn.Linear(4, 4), "linear_no_bias": lambda: nn.Linear(4, 4, bias=False),
+          "conv1d": lambda: Conv1D(4, 4)}
+SHAPES = {"2d": (3, 4), "3d": (3, 2, 4)}
+
+
+class Hooked:
+    """A layer with the pair on it; ``seen`` collects the (input, gradient) that the hook was given."""
+
+    def __init__(self, kind, shape):
+        torch.manual_seed(0)
+        self.layer, self.seen = LAYERS[kind](), []
+        self.x = torch.randn(SHAPES[shape], requires_grad=True) * 1
+        self.handles = register_hook_pair(self.layer, self.capture, self.hook)
+
+    @staticmethod
+    def capture(layer, inputs, outputs):
+        if torch.is_grad_enabled():
+            layer.__dict__["kept"] = inputs[0].detach()
+
+    def hook(self, layer, grad_input, grad_output):
+        A = layer.__dict__.pop("kept", None)
+        if A is None:
+            raise RuntimeError("no input kept")
+        self.seen.append((A, grad_output[0].clone()))
+
+    def check(self, calls=1):
+        """The hook's products add up to autograd's weight gradient."""
+        assert len(self.seen) == calls
+        total = sum(A.reshape(-1, 4).t() @ g.reshape(-1, 4) for A, g in self.seen)
+        want = self.layer.weight.grad
+        torch.testing.assert_close(total, want if isinstance(self.layer, Conv1D) else want.t(), rtol=1e-5, atol=1e-5)
+
+
+every_layer = pytest.mark.parametrize("kind", LAYERS)
+every_shape = pytest.mark.parametrize("shape", SHAPES)
+
+
+@every_layer
+@every_shape
+def test_a_users_tensor_hook_comes_first(kind, shape):
+    h = Hooked(kind, shape)
+    y = h.layer(h.x)
+    y.register_hook(lambda g: g * 10)
+    (y ** 2).sum().backward()
+    h.check()
+
+
+@every_layer
+@every_shape
+def test_a_users_module_hooks(kind, shape):
+    h = Hooked(kind, shape)
+    order = []
+    h.layer.register_full_backward_pre_hook(lambda m, g: (g[0] * 3,))
+    h.layer.register_full_backward_hook(lambda m, gi, go: order.append(len(h.seen)))
+    (h.layer(h.x) ** 2).sum().backward()
+    h.check()
+    assert order == [1]                  # after this pair's hook, whose results it may read
+
+
+@every_layer
+@every_shape
+def test_gradients_up_to_the_output_call_nothing(kind, shape):
+    h = Hooked(kind, shape)
+    y = h.layer(h.x)
+    loss = (y ** 2).sum()
+    torch.autograd.grad(loss, y, retain_graph=True)
+    assert not h.seen
+    loss.backward()
+    h.check()
