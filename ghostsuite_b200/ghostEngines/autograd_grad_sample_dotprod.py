@@ -90,15 +90,31 @@ def register_hook_pair(layer: nn.Module, capture, backward_hook):
             return
         capture(layer, inputs, outputs)
         if out is not None and out.requires_grad and torch.is_grad_enabled():
-            node, index = out.grad_fn, out.output_nr
+            node, index = _producing_node(out)
+            shape = out.shape
 
             def on_gradients(grads):
                 layer.__dict__["_ghost_done_in"] = torch._C._current_graph_task_id()
-                backward_hook(layer, None, (grads[index],))
+                grad = grads[index]
+                if grad is not None and grad.shape != shape:
+                    grad = grad.reshape(shape)
+                backward_hook(layer, None, (grad,))
 
             node.register_prehook(on_gradients)
 
     return [layer.register_forward_hook(forward_hook)]
+
+
+def _producing_node(out: torch.Tensor):
+    """``(node, output index)`` that hands on the gradient of ``out``.  Linear layers return a reshaped view
+    of their product; an in-place operation on a view gives it a new node and drops the old one with
+    its hooks, so there the base's node is taken."""
+    if out._is_view():
+        base = out._base
+        if base.requires_grad and base.grad_fn is not None and base.numel() == out.numel() \
+                and base.is_contiguous() and out.is_contiguous():
+            return base.grad_fn, base.output_nr
+    return out.grad_fn, out.output_nr
 
 
 def remove_hooks(model: nn.Module):

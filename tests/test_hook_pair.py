@@ -77,3 +77,35 @@ def test_gradients_up_to_the_output_call_nothing(kind, shape):
     assert not h.seen
     loss.backward()
     h.check()
+
+
+@every_layer
+@every_shape
+@pytest.mark.parametrize("when", ["none", "before", "after"])
+def test_in_place_operation_on_the_output(kind, shape, when):
+    h = Hooked(kind, shape)
+    y = h.layer(h.x)
+    if when == "before":
+        y.register_hook(lambda g: g * 10)
+    z = F.relu(y, inplace=True)
+    if when == "after":
+        z.register_hook(lambda g: g * 10)
+    (z ** 2).sum().backward()
+    h.check()
+
+
+def test_output_that_is_part_of_its_base():
+    """A view whose elements are not its base's in order: the hook stays at the view's own node."""
+    class Turned(nn.Linear):
+        def forward(self, x):
+            return super().forward(x).transpose(0, 1)
+
+    LAYERS["turned"] = lambda: Turned(4, 4)
+    try:
+        h = Hooked("turned", "3d")
+    finally:
+        del LAYERS["turned"]
+    (h.layer(h.x) ** 2).sum().backward()
+    (A, g), = h.seen
+    assert g.shape == (2, 3, 4)
+    torch.testing.assert_close(A.reshape(-1, 4).t() @ g.transpose(0, 1).reshape(-1, 4), h.layer.weight.grad.t())
