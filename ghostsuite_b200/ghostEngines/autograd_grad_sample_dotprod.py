@@ -60,16 +60,17 @@ def add_hooks(model: nn.Module, val_batch_size: int, loss_reduction: str = "mean
                 _apply_train_grad(this_layer, val_batch_size)
                 return None
 
-            handles.extend(register_hook_pair(layer, _capture_activations, backward_hook))
+            handles.extend(register_hook_pair(layer, _capture_activations, backward_hook, "activations"))
         elif not list(layer.children()) and requires_grad(layer):
             print(f"WARNING: Skipping atomic layer '{name}' of type {type(layer)} because it is not supported.")
 
     model.__dict__.setdefault("autograd_grad_sample_hooks", []).extend(handles)
 
 
-def register_hook_pair(layer: nn.Module, capture, backward_hook):
-    """Register ``capture(layer, inputs, outputs)`` on the forward pass and ``backward_hook(layer,
-    grad_input, (grad,))`` on the output's gradient; returns the removable handles.
+def register_hook_pair(layer: nn.Module, capture, backward_hook, slot: str):
+    """Register ``capture(layer, inputs, outputs)``, which keeps the input as attribute ``slot``, on the
+    forward pass and ``backward_hook(layer, grad_input, (grad,))`` on the output's gradient; returns the
+    removable handles.
 
     The backward hooks read the output gradient only, so a hook on the autograd node that produced the
     output serves them; a module's full backward hook wraps input and output in two more nodes per call
@@ -77,30 +78,39 @@ def register_hook_pair(layer: nn.Module, capture, backward_hook):
     hooks that a user has put on the output tensor leave of it, and ``autograd.grad`` up to the output
     calls nothing.  Embeddings keep the module hook: their input has no gradient, in which case a module
     hook that a user registers after this one fires at the output too, and would come before a hook on
-    the node inside."""
+    the node inside.
+
+    Every call's backward hook gets the input of that call.  Of calls that follow each other without
+    a backward pass in between only the last may be differentiated, as with one slot per layer; a
+    recomputation inside the backward pass (activation checkpointing) makes room for one more."""
     if isinstance(layer, nn.Embedding):
         return [layer.register_forward_hook(capture), layer.register_full_backward_hook(backward_hook)]
 
+    due = slot + "_due"
+
     def forward_hook(layer, inputs, outputs):
-        out = outputs if torch.is_tensor(outputs) else next((o for o in outputs if torch.is_tensor(o)), None)
-        task = torch._C._current_graph_task_id()
-        if task != -1 and layer.__dict__.get("_ghost_done_in") == task:
-            # non-re-entrant activation checkpointing runs this layer again inside the backward pass that
-            # has already called its hook: nothing would consume the input kept here
-            return
         capture(layer, inputs, outputs)
-        if out is not None and out.requires_grad and torch.is_grad_enabled():
-            node, index = _producing_node(out)
-            shape = out.shape
+        out = outputs if torch.is_tensor(outputs) else next((o for o in outputs if torch.is_tensor(o)), None)
+        if out is None or not out.requires_grad or not torch.is_grad_enabled():
+            return
+        own = layer.__dict__
+        own[due] = True
+        # a list, emptied by the hook: a graph that outlives its backward pass keeps no input alive
+        kept = [own.get(slot)]
+        if torch._C._current_graph_task_id() != -1:
+            own.pop(slot, None)          # recomputed: no hook may follow that would clear it
+        node, index = _producing_node(out)
+        shape = out.shape
 
-            def on_gradients(grads):
-                layer.__dict__["_ghost_done_in"] = torch._C._current_graph_task_id()
-                grad = grads[index]
-                if grad is not None and grad.shape != shape:
-                    grad = grad.reshape(shape)
-                backward_hook(layer, None, (grad,))
+        def on_gradients(grads):
+            grad = grads[index]
+            if grad is not None and grad.shape != shape:
+                grad = grad.reshape(shape)
+            value = kept.pop() if kept else None
+            own[slot] = value if own.pop(due, False) else None
+            backward_hook(layer, None, (grad,))
 
-            node.register_prehook(on_gradients)
+        node.register_prehook(on_gradients)
 
     return [layer.register_forward_hook(forward_hook)]
 

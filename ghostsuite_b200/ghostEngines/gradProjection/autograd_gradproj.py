@@ -127,7 +127,8 @@ class GradProjHooks:
         module._ghost_grad_proj = out.view(batch, k_o, k_i)
 
     def attach(self, module: nn.Module) -> None:
-        self._handles = register_hook_pair(module, self.forward_hook_store_inputs, self.backward_hook_compute_proj)
+        self._handles = register_hook_pair(module, self.forward_hook_store_inputs, self.backward_hook_compute_proj,
+                                           "_ghost_A_raw")
 
     def detach(self) -> None:
         for handle in self._handles:

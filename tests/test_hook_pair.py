@@ -4,6 +4,7 @@ import pytest
 import torch
 import torch.nn.functional as F
 from torch import nn
+from torch.utils.checkpoint import checkpoint
 from transformers.pytorch_utils import Conv1D
 
 from ghostsuite_b200.ghostEngines.autograd_grad_sample_dotprod import register_hook_pair
@@ -20,7 +21,7 @@ class Hooked:
         torch.manual_seed(0)
         self.layer, self.seen = LAYERS[kind](), []
         self.x = torch.randn(SHAPES[shape], requires_grad=True) * 1
-        self.handles = register_hook_pair(self.layer, self.capture, self.hook)
+        self.handles = register_hook_pair(self.layer, self.capture, self.hook, "kept")
 
     @staticmethod
     def capture(layer, inputs, outputs):
@@ -109,3 +110,67 @@ def test_output_that_is_part_of_its_base():
     (A, g), = h.seen
     assert g.shape == (2, 3, 4)
     torch.testing.assert_close(A.reshape(-1, 4).t() @ g.transpose(0, 1).reshape(-1, 4), h.layer.weight.grad.t())
+
+
+@every_layer
+@every_shape
+@pytest.mark.parametrize("reentrant", [False, True])
+def test_shared_layer_under_checkpointing(kind, shape, reentrant):
+    """Both calls are consumed, each with its own input, and nothing stays behind."""
+    h = Hooked(kind, shape)
+    x = h.x
+    for _ in range(2):
+        x = checkpoint(lambda t: h.layer(t).relu(), x, use_reentrant=reentrant)
+    (x ** 2).sum().backward()
+    h.check(calls=2)
+    assert not any(a.startswith("kept") for a in h.layer.__dict__)
+
+
+@every_layer
+@every_shape
+def test_shared_layer_with_one_call_checkpointed(kind, shape):
+    h = Hooked(kind, shape)
+    x = checkpoint(lambda t: h.layer(t).relu(), h.x, use_reentrant=False)
+    (h.layer(x) ** 2).sum().backward()
+    h.check(calls=2)
+
+
+@every_layer
+@every_shape
+@pytest.mark.parametrize("block", ["ends in the layer", "goes on"])
+def test_checkpointed_block(kind, shape, block):
+    h = Hooked(kind, shape)
+    tail = (lambda t: t) if block == "ends in the layer" else (lambda t: (t ** 2).sin())
+    x = checkpoint(lambda t: tail(h.layer(t.relu() * 2)), h.x, use_reentrant=False)
+    (x ** 2).sum().backward()
+    h.check()
+    assert not any(a.startswith("kept") for a in h.layer.__dict__)
+
+
+@every_layer
+@every_shape
+def test_shared_layer_without_recomputation_is_refused(kind, shape):
+    h = Hooked(kind, shape)
+    with pytest.raises(RuntimeError, match="no input kept"):
+        h.layer(h.layer(h.x).relu()).sum().backward()
+
+
+@every_layer
+@every_shape
+def test_another_forward_before_the_backward_pass(kind, shape):
+    """The hook gets the input of the call that is differentiated, not the last one's."""
+    h = Hooked(kind, shape)
+    loss = (h.layer(h.x) ** 2).sum()
+    h.layer(h.x * 5 + 1)
+    loss.backward()
+    h.check()
+
+
+def test_two_pairs_on_one_layer():
+    h = Hooked("linear", "3d")
+    other = []
+    register_hook_pair(h.layer, lambda m, i, o: m.__dict__.__setitem__("second", i[0].detach()),
+                       lambda m, gi, go: other.append(m.__dict__.pop("second")), "second")
+    (h.layer(h.x) ** 2).sum().backward()
+    h.check()
+    assert torch.equal(other[0], h.x)
