@@ -223,7 +223,7 @@ struct EmbBuckets {
   int *rank;                            // [n_tok] position inside the bucket, -1 for an id outside the table
   int *perm_b, *perm_v;
   int *totals;                          // [0] train tokens placed, [1] validation, [2] big rows, [3] items, [4] hot ids, [5] small rows,
-                                        // [6, 7] 64-bit count of gradient items handed out
+                                        // [6, 7] 64-bit count of gradient items handed out, [8] CTAs done with the join
   int4 *small;                          // (id, offset, tokens) of the rows with 1 to kEmbSmallBucket train tokens
   int *big;                             // ids with more than kEmbSmallBucket train tokens
   int4 *items;                          // join items: (first train position, train rows, first validation position
@@ -236,16 +236,17 @@ struct EmbBuckets {
 
 constexpr int kEmbSmallBucket = 32;      // buckets up to this size are sorted and summed by one warp
 constexpr int kEmbHotCap = 256;
+constexpr int kEmbTotals = 12;
 constexpr int kEmbChunk = 8;             // train rows of a join item
 constexpr int kEmbValChunk = 32;         // validation rows of a join item
 
 // Counting hands every token its place in the bucket, so filling needs no second round of atomics.
-// It also clears M, which the join adds to two launches later, and zero-fills the gradient, most of
+// It also clears the sums that the join adds to two launches later, and zero-fills the gradient, most of
 // whose rows stay empty: the stores go out under the latency of the atomics.
-__global__ void __launch_bounds__(256) emb_count_kernel(const EmbBuckets q, float* __restrict__ M, long long m_size,
+__global__ void __launch_bounds__(256) emb_count_kernel(const EmbBuckets q, double* __restrict__ M64, long long m_size,
                                                         uint4* __restrict__ zero, long long zero_size) {
-  if (M != nullptr)
-    for (long long i = blockIdx.x * 256ll + threadIdx.x; i < m_size; i += gridDim.x * 256ll) M[i] = 0.f;
+  if (M64 != nullptr)
+    for (long long i = blockIdx.x * 256ll + threadIdx.x; i < m_size; i += gridDim.x * 256ll) M64[i] = 0.;
   for (long long j = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; j < q.n_tok;
        j += static_cast<long long>(gridDim.x) * blockDim.x) {
     const long long id = j < q.first_val ? q.ids_b[j] : q.ids_v[j - q.first_val];
@@ -458,6 +459,10 @@ template <> struct EmbOct<float> {
 // acc += 16 validation rows x 8 train rows over the whole row length; a lane supplies rows g and g + 8 of
 // the first operand, row g of the second, 8 of every 32 columns (the contraction order inside a
 // step is permuted alike for both).  The loads of kDepth steps are issued together.
+// The tensor core's accumulator truncates, an error that grows with every product added to it, so each
+// product starts from zero and the sums are made in float32 registers, in short chains: 1.2e-5 off the
+// 64-bit result over 2048 float32 features without that, 3e-8 with it, 6e-8 with multiply-adds on the CUDA
+// cores (16 + 8 samples of 512 text tokens; 236 us a hook either way).
 template <typename VT, typename BT, bool VEC>
 __device__ __forceinline__ void emb_mma_rows(const VT* va, const VT* vb, const BT* tr, bool va_ok, bool vb_ok, bool tr_ok,
                                              int d, int c, float (&acc)[4]) {
@@ -471,20 +476,33 @@ __device__ __forceinline__ void emb_mma_rows(const VT* va, const VT* vb, const B
       b[s].template load<VEC>(vb, k0 + 32 * s, d, vb_ok);
       t[s].template load<VEC>(tr, k0 + 32 * s, d, tr_ok);
     }
+    float group[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
     for (int s = 0; s < kDepth; ++s) {
       a[s].split();
       b[s].split();
       t[s].split();
+      float first[4], second[4];
+      mma_16816_new(first, a[s].w[0][0], b[s].w[0][0], a[s].w[0][1], b[s].w[0][1], t[s].w[0][0], t[s].w[0][1]);
+      mma_16816_new(second, a[s].w[0][2], b[s].w[0][2], a[s].w[0][3], b[s].w[0][3], t[s].w[0][2], t[s].w[0][3]);
 #pragma unroll
-      for (int p = 0; p < EmbOct<VT>::kParts; ++p)
+      for (int e = 0; e < 4; ++e) group[e] += first[e] + second[e];
+      if constexpr (EmbOct<VT>::kParts > 1 || EmbOct<BT>::kParts > 1) {
+        float low[4] = {0.f, 0.f, 0.f, 0.f};         // everything but the leading parts: 2^-8 of them and less
 #pragma unroll
-        for (int r = 0; r < EmbOct<BT>::kParts; ++r)
-          if (p + r <= 2) {
-            mma_16816(acc, a[s].w[p][0], b[s].w[p][0], a[s].w[p][1], b[s].w[p][1], t[s].w[r][0], t[s].w[r][1]);
-            mma_16816(acc, a[s].w[p][2], b[s].w[p][2], a[s].w[p][3], b[s].w[p][3], t[s].w[r][2], t[s].w[r][3]);
-          }
+        for (int h = 0; h < 4; h += 2)
+#pragma unroll
+          for (int p = 0; p < EmbOct<VT>::kParts; ++p)
+#pragma unroll
+            for (int r = 0; r < EmbOct<BT>::kParts; ++r)
+              if (p + r >= 1 && p + r <= 2)
+                mma_16816(low, a[s].w[p][h], b[s].w[p][h], a[s].w[p][h + 1], b[s].w[p][h + 1], t[s].w[r][h], t[s].w[r][h + 1]);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) group[e] += low[e];
+      }
     }
+#pragma unroll
+    for (int e = 0; e < 4; ++e) acc[e] += group[e];
   }
 }
 
@@ -498,16 +516,21 @@ __device__ __forceinline__ void emb_mma_rows(const VT* va, const VT* vb, const B
 template <typename T, bool VEC>
 __global__ void __launch_bounds__(256, 2)
 emb_join_kernel(const EmbBuckets q, const T* __restrict__ Gb, const T* __restrict__ Gv, int n_train, int n_val, int Tn, int d,
-                const float* __restrict__ R, float scale, float* __restrict__ M, long long pitch, int local) {
+                const float* __restrict__ R, float scale, double* __restrict__ M64, float* __restrict__ M, long long pitch,
+                int local) {
   extern __shared__ float s_M[];         // [n_val, n_train] when `local`
   const int lane = threadIdx.x & 31, g = lane >> 2, c = lane & 3;
   if (local) {
     for (int i = threadIdx.x; i < n_val * n_train; i += 256) s_M[i] = 0.f;
     __syncthreads();
   }
-  float* acc_M = local ? s_M : M;
-  const long long acc_pitch = local ? n_train : pitch;
-  const float out_scale = local ? 1.f : scale;
+  // Sums over the items of many CTAs: hundreds of float32 additions to one entry cost more accuracy than
+  // the products, so they are made in float64 and rounded once.
+  auto add = [&](int v, int b, float x) {
+    const long long at = static_cast<long long>(v) * n_train + b;
+    if (local) atomicAdd(s_M + at, x);
+    else atomicAdd(M64 + at, static_cast<double>(x));
+  };
   const bool single = n_val == 1 && n_train == 1;
   const int n_items = q.totals[3], stride = gridDim.x * 8;
   int it = blockIdx.x * 8 + (threadIdx.x >> 5);
@@ -538,18 +561,17 @@ emb_join_kernel(const EmbBuckets q, const T* __restrict__ Gb, const T* __restric
         emb_mma_rows<T, T, VEC>(Gv + static_cast<long long>(j0) * d, Gv + static_cast<long long>(j1) * d,
                                 Gb + static_cast<long long>(jb) * d, ok0, ok1, b_ok, d, c, acc);
       }
+      const bool c0 = 2 * c < nb, c1 = 2 * c + 1 < nb;      // an absent row times an infinite one is no zero
       if (single) {                        // every entry belongs to the one pair
-        const bool c0 = 2 * c < nb, c1 = 2 * c + 1 < nb;      // an absent row times an infinite one is no zero
         float s = ((ok0 && c0 ? acc[0] : 0.f) + (ok0 && c1 ? acc[1] : 0.f)) + ((ok1 && c0 ? acc[2] : 0.f) + (ok1 && c1 ? acc[3] : 0.f));
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (lane == 0) atomicAdd(acc_M, s * out_scale);
+        if (lane == 0) add(0, 0, s);
       } else {
-        const bool c0 = 2 * c < nb, c1 = 2 * c + 1 < nb;
-        if (ok0 && c0) atomicAdd(acc_M + s0 * acc_pitch + b0, acc[0] * out_scale);
-        if (ok0 && c1) atomicAdd(acc_M + s0 * acc_pitch + b1, acc[1] * out_scale);
-        if (ok1 && c0) atomicAdd(acc_M + s1 * acc_pitch + b0, acc[2] * out_scale);
-        if (ok1 && c1) atomicAdd(acc_M + s1 * acc_pitch + b1, acc[3] * out_scale);
+        if (ok0 && c0) add(s0, b0, acc[0]);
+        if (ok0 && c1) add(s0, b1, acc[1]);
+        if (ok1 && c0) add(s1, b0, acc[2]);
+        if (ok1 && c1) add(s1, b1, acc[3]);
       }
     }
   }
@@ -557,12 +579,31 @@ emb_join_kernel(const EmbBuckets q, const T* __restrict__ Gb, const T* __restric
     __syncthreads();
     for (int i = threadIdx.x; i < n_val * n_train; i += 256) {
       const float s = s_M[i];
-      if (s != 0.f) atomicAdd(M + i / n_train * pitch + i % n_train, s * scale);
+      if (s != 0.f) atomicAdd(M64 + i, static_cast<double>(s));
+    }
+    // the last CTA rounds the finished sums
+    __shared__ int s_last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) s_last = atomicAdd(q.totals + 8, 1) == static_cast<int>(gridDim.x) - 1;
+    __syncthreads();
+    if (s_last) {
+      __threadfence();
+      for (int i = threadIdx.x; i < n_val * n_train; i += 256)
+        M[i / n_train * pitch + i % n_train] = static_cast<float>(__ldcg(M64 + i) * scale);
     }
   }
   // Launched beside the gradient kernel, whose results it does not read; but what follows in the stream
   // waits for this grid only, so it ends no earlier.
   asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+// The same rounding for a matrix that is too large for one CTA.
+__global__ void __launch_bounds__(256) emb_round_kernel(const double* __restrict__ M64, int n_val, int n_train, float scale,
+                                                        float* __restrict__ M, long long pitch) {
+  const long long size = static_cast<long long>(n_val) * n_train;
+  for (long long i = blockIdx.x * 256ll + threadIdx.x; i < size; i += gridDim.x * 256ll)
+    M[i / n_train * pitch + i % n_train] = static_cast<float>(M64[i] * scale);
 }
 
 // ---------------------------------------------------------------- train gradient
@@ -809,7 +850,8 @@ static long long emb_max_items(long long tb, int vocab) {
 
 extern "C" long long ghost_embedding_pass_workspace_bytes(int n_train, int n_val, long long T, int vocab, int d) {
   const long long tb = static_cast<long long>(n_train) * T, tv = static_cast<long long>(n_val) * T;
-  return up256(4ll * (2 * static_cast<long long>(vocab) + 8)) + 2 * up256(4ll * vocab)     // counts and totals; offsets
+  return up256(4ll * (2 * static_cast<long long>(vocab) + kEmbTotals)) + 2 * up256(4ll * vocab)     // counts and totals; offsets
+         + up256(8ll * n_train * n_val)                                                    // sums of the matrix
          + up256(4ll * (tb + tv)) + up256(4ll * tb) + up256(4ll * tv)                      // rank, perm_b, perm_v
          + up256(4ll * (tb / (kEmbSmallBucket + 1) + 2)) + up256(16ll * emb_max_items(tb, vocab))   // big rows, items
          + up256(4ll * kEmbHotCap) + up256(16ll * (vocab < tb ? vocab : tb)) + up256(4ll * kEmbHotCap * static_cast<long long>(n_val) * d);
@@ -822,7 +864,7 @@ namespace gb {
 
 template <typename T>
 static int emb_pass(const EmbBuckets& q, const T* Gb, const T* Gv, int n_train, int n_val, long long Tn, int d, float scale,
-                    float* M, long long pitch, bool clear_M, float* R, float pre_scale, float divisor, int accumulate, T* out, const DeviceState* ds, cudaStream_t st) {
+                    float* M, long long pitch, double* M64, float* R, float pre_scale, float divisor, int accumulate, T* out, const DeviceState* ds, cudaStream_t st) {
   int blocks = static_cast<int>((q.n_tok + 255) / 256);
   if (blocks > ds->sm_count * 8) blocks = ds->sm_count * 8;
   // the gradient is zero-filled by the counting kernel where 16-byte stores can (torch buffers always)
@@ -830,7 +872,7 @@ static int emb_pass(const EmbBuckets& q, const T* Gb, const T* Gv, int n_train, 
   const bool fill = out != nullptr && !accumulate, quick = fill && out_bytes % 16 == 0 && (reinterpret_cast<uintptr_t>(out) & 15u) == 0;
   if (fill && !quick) GB_CUDA_OK(cudaMemsetAsync(out, 0, out_bytes, st));
   if (quick) blocks = ds->sm_count * 8;
-  emb_count_kernel<<<blocks, 256, 0, st>>>(q, clear_M ? M : nullptr, n_val * pitch, reinterpret_cast<uint4*>(out),
+  emb_count_kernel<<<blocks, 256, 0, st>>>(q, M64, static_cast<long long>(n_val) * n_train, reinterpret_cast<uint4*>(out),
                                            quick ? out_bytes / 16 : 0);
   emb_alloc_kernel<<<ceil_div(q.vocab, 256), 256, 0, st>>>(q);
   emb_fill_kernel<<<blocks, 256, 0, st>>>(q);
@@ -872,8 +914,13 @@ static int emb_pass(const EmbBuckets& q, const T* Gb, const T* Gv, int n_train, 
     cfg.attrs = &beside;
     cfg.numAttrs = out != nullptr ? 1 : 0;
     GB_CUDA_OK(cudaLaunchKernelEx(&cfg, vec ? emb_join_kernel<T, true> : emb_join_kernel<T, false>, q, Gb, Gv, n_train, n_val, Ti,
-                                  d, static_cast<const float*>(R), scale, M, pitch, local));
+                                  d, static_cast<const float*>(R), scale, M64, M, pitch, local));
     count_launch();
+    if (!local) {
+      const int rb = ceil_div(static_cast<long long>(n_val) * n_train, 256);
+      emb_round_kernel<<<rb < ds->sm_count * 8 ? rb : ds->sm_count * 8, 256, 0, st>>>(M64, n_val, n_train, scale, M, pitch);
+      count_launch();
+    }
   }
   return post_launch("ghost_embedding_pass");
 }
@@ -895,9 +942,9 @@ static int emb_pass_group(const long long* ids, const void* G, int is_f32, int n
   q.first_val = tb;
   q.n_tok = tb + tv;
   q.vocab = vocab;
-  const long long zero_bytes = 4ll * (2 * static_cast<long long>(vocab) + 8);
+  const long long zero_bytes = 4ll * (2 * static_cast<long long>(vocab) + kEmbTotals);
   q.totals = static_cast<int*>(take(zero_bytes));
-  q.cnt_b = q.totals + 8;
+  q.cnt_b = q.totals + kEmbTotals;
   q.cnt_v = M ? q.cnt_b + vocab : nullptr;
   q.off_b = static_cast<int*>(take(4ll * vocab));
   q.off_v = static_cast<int*>(take(4ll * vocab));
@@ -909,6 +956,7 @@ static int emb_pass_group(const long long* ids, const void* G, int is_f32, int n
   q.items = static_cast<int4*>(take(16ll * q.max_items));
   q.hot = static_cast<int*>(take(4ll * kEmbHotCap));
   q.small = static_cast<int4*>(take(16ll * (vocab < tb ? vocab : tb)));
+  double* M64 = static_cast<double*>(take(M ? 8ll * n_b * n_val : 0));
   float* R = static_cast<float*>(take(4ll * kEmbHotCap * static_cast<long long>(n_val) * (M ? d : 0)));
   // A hot id costs n_val dot products per train token instead of one per validation token, after a pass over
   // its validation rows; the products are cheap, so that pass pays from a few join items' worth on.
@@ -916,15 +964,15 @@ static int emb_pass_group(const long long* ids, const void* G, int is_f32, int n
   q.max_parts = kEmbMaxParts;
   q.want_rows = out != nullptr;
   q.err = ds->err_word;
-  GB_CUDA_OK(cudaMemsetAsync(q.totals, 0, M ? zero_bytes : 4ll * (vocab + 8), st));
+  GB_CUDA_OK(cudaMemsetAsync(q.totals, 0, M ? zero_bytes : 4ll * (vocab + kEmbTotals), st));
   float* Mg = M ? M + b0 : nullptr;
   if (is_f32) {
     const float* g = static_cast<const float*>(G);
-    return emb_pass<float>(q, g + b0 * T * d, g + n_train * T * d, n_b, n_val, T, d, scale, Mg, n_train, b0 == 0, R,
+    return emb_pass<float>(q, g + b0 * T * d, g + n_train * T * d, n_b, n_val, T, d, scale, Mg, n_train, M ? M64 : nullptr, R,
                            pre_scale, divisor, accumulate, static_cast<float*>(out), ds, st);
   }
   const __nv_bfloat16* g = static_cast<const __nv_bfloat16*>(G);
-  return emb_pass<__nv_bfloat16>(q, g + b0 * T * d, g + n_train * T * d, n_b, n_val, T, d, scale, Mg, n_train, b0 == 0, R,
+  return emb_pass<__nv_bfloat16>(q, g + b0 * T * d, g + n_train * T * d, n_b, n_val, T, d, scale, Mg, n_train, M ? M64 : nullptr, R,
                                  pre_scale, divisor, accumulate, static_cast<__nv_bfloat16*>(out), ds, st);
 }
 

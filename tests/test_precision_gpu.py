@@ -1,0 +1,71 @@
+"""Accuracy of the sums against 64 bits, at lengths where the order of a sum shows.
+
+The tensor core adds into an accumulator that it truncates, so a long chain of products of one sign
+comes out too small by up to 2^-23 per product added (2^-24 on average); float32 additions round to
+nearest and leave no such bias.  The data are therefore positive and the tests look at the mean signed
+error over many entries: chains of a few products stay below 2^-23, rounding averages out."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+BIAS = 2.0 ** -23
+
+
+def ops():
+    from ghostsuite_b200 import ops as _ops
+    return _ops
+
+
+def positive(shape, dtype, seed):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    return (0.5 + torch.rand(shape, generator=g, device="cuda")).to(dtype)
+
+
+def bias(got, want):
+    want = want.double()
+    return ((got.double() - want) / want).mean().abs().item()
+
+
+# text-like ids (every validation token of an id in one list) and one id above the summed-rows line; feature
+# counts on both sides of one load step
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("d", [256, 731, 2048])
+@pytest.mark.parametrize("vocab", [1, 40])
+def test_embedding_matrix(vocab, d, dtype):
+    n_t, n_v, T = 16, 8, 48
+    g = torch.Generator(device="cuda").manual_seed(3)
+    ids = torch.randint(0, vocab, (n_t + n_v, T), generator=g, device="cuda")
+    G = positive((n_t + n_v, T, d), dtype, 4)
+    M = ops().embedding_dot(ids, G, n_v, vocab)
+    R = torch.zeros(n_t + n_v, vocab, d, dtype=torch.float64, device="cuda")
+    for i in range(n_t + n_v):
+        R[i].index_add_(0, ids[i], G[i].double())
+    R = R.reshape(n_t + n_v, -1)
+    assert bias(M, R[n_t:] @ R[:n_t].t()) < BIAS
+
+
+def test_embedding_matrix_beyond_one_block():
+    """More entries than a block sums in shared memory; groups of train samples through the C entry."""
+    n_t, n_v, T, d, vocab = 300, 20, 6, 64, 9
+    g = torch.Generator(device="cuda").manual_seed(5)
+    ids = torch.randint(0, vocab, (n_t + n_v, T), generator=g, device="cuda")
+    ids[:, 0] = 4                        # every pair shares an id: the errors below are relative to the entry
+    G = positive((n_t + n_v, T, d), torch.float32, 6)
+    R = torch.zeros(n_t + n_v, vocab, d, dtype=torch.float64, device="cuda")
+    for i in range(n_t + n_v):
+        R[i].index_add_(0, ids[i], G[i].double())
+    R = R.reshape(n_t + n_v, -1)
+    want = 0.5 * R[n_t:] @ R[:n_t].t()
+    M = ops().embedding_dot(ids, G, n_v, vocab, 0.5)
+    # a dot product of 64 terms in float32, then 64-bit sums: 2^-24 per addition of the longest chain
+    assert ((M.double() - want) / want).abs().max() < 8 * BIAS and bias(M, want) < BIAS
+    from ghostsuite_b200 import _lib
+    lib = _lib.load()
+    room = int(lib.ghost_embedding_dot_workspace_bytes_for(n_v, T, vocab, d))       # groups of 32
+    ws = torch.empty(room, dtype=torch.uint8, device="cuda")
+    M2 = torch.full_like(M, 7.0)
+    _lib.check(lib.ghost_embedding_dot(ids.data_ptr(), G.data_ptr(), 1, n_t, n_v, T, d, vocab, 0.5, M2.data_ptr(),
+                                       ws.data_ptr(), room, torch.cuda.current_stream().cuda_stream))
+    torch.cuda.synchronize()
+    assert ((M2.double() - want) / want).abs().max() < 8 * BIAS
