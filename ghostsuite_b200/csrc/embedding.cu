@@ -506,6 +506,36 @@ __device__ __forceinline__ void emb_mma_rows(const VT* va, const VT* vb, const B
   }
 }
 
+// <v, b> of two rows in float32 by one warp
+template <typename VT, typename BT>
+__device__ __forceinline__ float emb_plain_dot(const VT* v, const BT* b, int d, int lane) {
+  float s = 0.f;
+  for (int f = lane; f < d; f += 32) s = fmaf(ld_f32<VT>(v + f), ld_f32<BT>(b + f), s);
+  return ewarp_sum(s);
+}
+
+// The parts of an infinite float32 value are an infinity and NaN, so an entry that is not finite (and ought
+// to be infinite, or lies beyond the parts' range) is made again from the rows as they are.  Lane
+// (g, c) holds entries (g, 2c), (g, 2c + 1), (g + 8, 2c), (g + 8, 2c + 1); `lv` is its two validation rows.
+template <typename VT, typename BT>
+__device__ __noinline__ float4 emb_redo(const VT* V, const BT* B, int2 lv, int my_b, unsigned todo, int d, float4 sums) {
+  float acc[4] = {sums.x, sums.y, sums.z, sums.w};
+  const int lane = threadIdx.x & 31;
+  for (unsigned who_mask = __ballot_sync(0xffffffffu, todo != 0); who_mask != 0; who_mask &= who_mask - 1) {
+    const int who = __ffs(who_mask) - 1;
+    const unsigned what = __shfl_sync(0xffffffffu, todo, who);
+    const int r0 = __shfl_sync(0xffffffffu, lv.x, who), r1 = __shfl_sync(0xffffffffu, lv.y, who);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int b = __shfl_sync(0xffffffffu, my_b, 2 * (who & 3) + (e & 1));
+      if (!(what >> e & 1)) continue;
+      const float s = emb_plain_dot<VT, BT>(V + static_cast<long long>(e < 2 ? r0 : r1) * d, B + static_cast<long long>(b) * d, d, lane);
+      if (lane == who) acc[e] = s;
+    }
+  }
+  return make_float4(acc[0], acc[1], acc[2], acc[3]);
+}
+
 // One join item per warp: up to eight train rows of one id against up to 32 validation rows of it (or, for a
 // hot id, one summed row per validation sample), 16 at a time on mma.sync with fragments loaded
 // straight from global memory.  Rows come from HBM once; repeats hit L1 / L2.  What bounds it is the
@@ -549,19 +579,28 @@ emb_join_kernel(const EmbBuckets q, const T* __restrict__ Gb, const T* __restric
       const int r0 = v0 + g, r1 = v0 + g + 8;
       const bool ok0 = r0 < cv, ok1 = r1 < cv;
       float acc[4] = {0.f, 0.f, 0.f, 0.f};
-      int s0 = r0, s1 = r1;
+      int s0 = r0, s1 = r1, j0 = 0, j1 = 0;
       if (hot) {
         const float* base = R + static_cast<long long>(at_v) * n_val * d;
         emb_mma_rows<float, T, VEC>(base + static_cast<long long>(ok0 ? r0 : 0) * d, base + static_cast<long long>(ok1 ? r1 : 0) * d,
                                     Gb + static_cast<long long>(jb) * d, ok0, ok1, b_ok, d, c, acc);
       } else {
-        const int j0 = ok0 ? q.perm_v[at_v + r0] : 0, j1 = ok1 ? q.perm_v[at_v + r1] : 0;
+        j0 = ok0 ? q.perm_v[at_v + r0] : 0;
+        j1 = ok1 ? q.perm_v[at_v + r1] : 0;
         s0 = j0 / Tn;
         s1 = j1 / Tn;
         emb_mma_rows<T, T, VEC>(Gv + static_cast<long long>(j0) * d, Gv + static_cast<long long>(j1) * d,
                                 Gb + static_cast<long long>(jb) * d, ok0, ok1, b_ok, d, c, acc);
       }
       const bool c0 = 2 * c < nb, c1 = 2 * c + 1 < nb;      // an absent row times an infinite one is no zero
+      const unsigned redo = (ok0 && c0 && !isfinite(acc[0]) ? 1u : 0u) | (ok0 && c1 && !isfinite(acc[1]) ? 2u : 0u) |
+                            (ok1 && c0 && !isfinite(acc[2]) ? 4u : 0u) | (ok1 && c1 && !isfinite(acc[3]) ? 8u : 0u);
+      if (__any_sync(0xffffffffu, redo != 0)) {
+        const float4 was = make_float4(acc[0], acc[1], acc[2], acc[3]);
+        const float4 is = hot ? emb_redo<float, T>(R + static_cast<long long>(at_v) * n_val * d, Gb, make_int2(s0, s1), my_b, redo, d, was)
+                              : emb_redo<T, T>(Gv, Gb, make_int2(j0, j1), my_b, redo, d, was);
+        acc[0] = is.x; acc[1] = is.y; acc[2] = is.z; acc[3] = is.w;
+      }
       if (single) {                        // every entry belongs to the one pair
         float s = ((ok0 && c0 ? acc[0] : 0.f) + (ok0 && c1 ? acc[1] : 0.f)) + ((ok1 && c0 ? acc[2] : 0.f) + (ok1 && c1 ? acc[3] : 0.f));
 #pragma unroll

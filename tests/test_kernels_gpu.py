@@ -530,6 +530,41 @@ def test_embedding_hook(case, dtype):
     assert torch.equal(grad.cpu().float(), O.embedding_train_grad(ids, G * N, n_v, vocab, sequential=True).float())
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("vocab,n_v", [(9, 2), (1, 3), (9, 80)])       # joined rows, summed rows, many validation rows
+def test_embedding_matrix_with_infinities(vocab, n_v, dtype):
+    """Entries are infinite or NaN exactly where the plain sums are, and no other entry is touched."""
+    n_t, T, d = 5, 40, 72
+    N = n_t + n_v
+    g = torch.Generator().manual_seed(12)
+    ids = torch.randint(0, vocab, (N, T), generator=g)
+    if n_v > 2:                  # an id of many validation tokens has a summed row, zero, for a sample without it
+        ids[:, 10:10 + vocab] = torch.arange(vocab)
+    G = (0.5 + torch.rand(N, T, d, generator=g)).to(dtype)
+    G[1, 3, 5] = float("inf")
+    G[2, 0, 0], G[2, 1, 1] = float("inf"), -float("inf")
+    G[n_t + 1, 7, 9] = -float("inf")
+    if dtype == torch.float32:
+        G[3, 2, 2] = 3.4e38                      # finite, but beyond what a bf16 part can hold
+        G[n_t:, :, 2] = 1e-3
+    M = ops().embedding_dot(ids.cuda(), G.cuda(), n_v, vocab).cpu()
+    after()
+    R = torch.zeros(N, vocab, d, dtype=torch.float64)
+    for i in range(N):
+        R[i].index_add_(0, ids[i], G[i].double())
+    # rows without the id are absent, not zero: they meet no infinity
+    has = torch.zeros(N, vocab, dtype=torch.bool).scatter_(1, ids, True)
+    want = torch.zeros(n_v, n_t, dtype=torch.float64)
+    for v in range(n_v):
+        for b in range(n_t):
+            both = has[n_t + v] & has[b]
+            want[v, b] = (R[n_t + v][both] * R[b][both]).sum()
+    assert torch.equal(M.isnan(), want.isnan())
+    assert torch.equal(M.isposinf(), want.isposinf()) and torch.equal(M.isneginf(), want.isneginf())
+    fin = want.isfinite()
+    assert ((M.double() - want)[fin].abs() <= 1e-5 * want[fin].abs()).all()
+
+
 def test_embedding_out_of_range_ids_are_reported():
     """An id outside the table makes the reference's index_add_ raise.  The kernels skip such a token
     and record it; the next poll of the error word raises IndexError."""
