@@ -492,8 +492,8 @@ extern "C" int ghost_wgrad_bf16(const void* X, const void* Y, long long n_rows, 
   if ((rc = make_xty_maps(&tx, &ty, p, X, Y, 1, n_rows, ldx, ldy)) != GHOST_OK) return rc;
   const bool pair = pair_kernel_fits(g_wgrad_pair_mode, m_cols, n_cols) && p.blocked_x && p.blocked_y && xty_pair_usable(ds);
   const int splits = pair ? pick_k_splits(static_cast<long long>(ceil_div(m_cols, 256)) * p.n_tiles, ds->sm_count / 2,
-                                          ceil_div(n_rows, 128), 32, elems)
-                          : pick_k_splits(tiles, ds->sm_count, kb, 64, elems);
+                                          ceil_div(n_rows, 128), 32, elems, out_is_f32 != 0)
+                          : pick_k_splits(tiles, ds->sm_count, kb, 64, elems, out_is_f32 != 0);
   if (splits > 1) GB_CUDA_OK(cudaMemsetAsync(ws, 0, static_cast<size_t>(m_cols) * p.ld_acc * 4, st));
   else p.mode = kEpiDirect;
   if (pair) {

@@ -49,10 +49,13 @@ __device__ __forceinline__ void store_grad_row32(void* out, int is_f32, int accu
 // the fp32 workspace and for the scaling pass: two launches (5 us) and ten bytes per weight element
 // at 5 TB/s; one split stores the result itself.  Fixed costs, measured: `add_cost` with red.add
 // into the workspace, a quarter of it with plain stores.
-inline int pick_k_splits(long long tiles, int workers, int kb, int add_cost, double weight_elems) {
+// The tensor core's accumulator truncates, so the error grows with the rows one split covers.  A bf16
+// result does not show it; a float32 result does (4096 rows of 768 x 768, bf16 operands: 4.2e-6 off the
+// 64-bit result in one split, 4.5e-7 in ten), so there the merge is not counted against splitting.
+inline int pick_k_splits(long long tiles, int workers, int kb, int add_cost, double weight_elems, bool f32_result) {
   int splits = 1;
-  double best = static_cast<double>((tiles + workers - 1) / workers) * (kb + add_cost / 4);
-  const double merge = (5.0 + weight_elems * 10.0 / 5e6) / 0.28;
+  double best = static_cast<double>((tiles + workers - 1) / workers) * (kb + (f32_result ? add_cost : add_cost / 4));
+  const double merge = f32_result ? 0. : (5.0 + weight_elems * 10.0 / 5e6) / 0.28;
   for (int s = 2; s <= 64 && s <= kb; ++s) {
     const double cost = static_cast<double>((tiles * s + workers - 1) / workers) * ((kb + s - 1) / s + add_cost) + merge;
     if (cost < best) { best = cost; splits = s; }

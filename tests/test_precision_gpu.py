@@ -69,3 +69,14 @@ def test_embedding_matrix_beyond_one_block():
                                        ws.data_ptr(), room, torch.cuda.current_stream().cuda_stream))
     torch.cuda.synchronize()
     assert ((M2.double() - want) / want).abs().max() < 8 * BIAS
+
+
+# float32 results: no chain longer than what the split of the rows allows (products of 16 rows each)
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("m,n,chain", [(64, 64, 4), (256, 256, 8), (768, 768, 32), (1000, 768, 64)])
+def test_wgrad_float32_result(m, n, chain, dtype):
+    rows = 4096
+    X, Y = positive((rows, m), dtype, 1), positive((rows, n), dtype, 2)
+    W = ops().wgrad(X, Y, 1.0, torch.float32)
+    parts = 3 if dtype == torch.float32 else 1              # hi.hi, lo.hi and hi.lo go to one accumulator
+    assert bias(W, X.double().t() @ Y.double()) < parts * chain / 2 * BIAS
