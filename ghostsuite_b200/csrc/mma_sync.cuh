@@ -32,6 +32,14 @@ __device__ __forceinline__ void mma_16816_new(float (&d)[4], uint32_t a0, uint32
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
 }
 
+// d += a for the four entries of a fragment, two to an instruction
+__device__ __forceinline__ void add_fragment(float (&d)[4], const float (&a)[4]) {
+#pragma unroll
+  for (int e = 0; e < 4; e += 2)
+    asm("{\n\t.reg .b64 x, y;\n\tmov.b64 x, {%0, %1};\n\tmov.b64 y, {%2, %3};\n\tadd.rn.f32x2 x, x, y;\n\tmov.b64 {%0, %1}, x;\n\t}"
+        : "+f"(d[e]), "+f"(d[e + 1]) : "f"(a[e]), "f"(a[e + 1]));
+}
+
 __device__ __forceinline__ uint32_t pack_bf16x2(__nv_bfloat16 x, __nv_bfloat16 y) {
   __nv_bfloat162 h(x, y);
   return *reinterpret_cast<uint32_t*>(&h);

@@ -227,7 +227,7 @@ template <typename PT, bool VEC> struct SimOct {
 // to 64 x 64 scores (again from L2 / L1 for the next block and the neighbouring warps) instead of once
 // per 16 x 16.  All loads of a 32-element step go out together.
 template <typename PT, int MT, int NT, int WM, int WN, bool VEC>
-__global__ void __launch_bounds__(256) proj_similarity_kernel(const SimParams p) {
+__global__ void __launch_bounds__(256, 2) proj_similarity_kernel(const SimParams p) {
   constexpr int WK = 8 / (WM * WN);
   constexpr int BM = 16 * MT * WM, BN = 8 * NT * WN;
   constexpr bool kSplit = sizeof(PT) == 4;
@@ -273,15 +273,24 @@ __global__ void __launch_bounds__(256) proj_similarity_kernel(const SimParams p)
       uint32_t bh[4], bl[4];
       b[n].parts(bh, bl);
 #pragma unroll
-      for (int m = 0; m < MT; ++m)
-#pragma unroll
-        for (int h = 0; h < 4; h += 2) {
-          mma_16816(acc[m][n], ah[2 * m][h], ah[2 * m + 1][h], ah[2 * m][h + 1], ah[2 * m + 1][h + 1], bh[h], bh[h + 1]);
-          if (kSplit) {
-            mma_16816(acc[m][n], al[2 * m][h], al[2 * m + 1][h], al[2 * m][h + 1], al[2 * m + 1][h + 1], bh[h], bh[h + 1]);
-            mma_16816(acc[m][n], ah[2 * m][h], ah[2 * m + 1][h], ah[2 * m][h + 1], ah[2 * m + 1][h + 1], bl[h], bl[h + 1]);
-          }
+      for (int m = 0; m < MT; ++m) {
+        // The tensor core's accumulator truncates, so it holds one step and the sum over the steps is made
+        // here.  16 x 16 scores over 98304 elements: 7.8e-7 -> 4.2e-7 off the 64-bit result (float32), 2.5e-7 ->
+        // 0.9e-7 (bf16); 64 x 64 over 2^20: 5.4e-6 -> 3.8e-7 and 149 -> 156 us (float32, bound by the
+        // splitting of its operands), 1.8e-6 -> 2.4e-7 and 207 -> 82 us (bf16, was bound by the chain).
+        float step[4];
+        if constexpr (kSplit) {
+          mma_16816_new(step, al[2 * m][0], al[2 * m + 1][0], al[2 * m][1], al[2 * m + 1][1], bh[0], bh[1]);
+          mma_16816(step, ah[2 * m][0], ah[2 * m + 1][0], ah[2 * m][1], ah[2 * m + 1][1], bl[0], bl[1]);
+          mma_16816(step, al[2 * m][2], al[2 * m + 1][2], al[2 * m][3], al[2 * m + 1][3], bh[2], bh[3]);
+          mma_16816(step, ah[2 * m][2], ah[2 * m + 1][2], ah[2 * m][3], ah[2 * m + 1][3], bl[2], bl[3]);
+          mma_16816(step, ah[2 * m][0], ah[2 * m + 1][0], ah[2 * m][1], ah[2 * m + 1][1], bh[0], bh[1]);
+        } else {
+          mma_16816_new(step, ah[2 * m][0], ah[2 * m + 1][0], ah[2 * m][1], ah[2 * m + 1][1], bh[0], bh[1]);
         }
+        mma_16816(step, ah[2 * m][2], ah[2 * m + 1][2], ah[2 * m][3], ah[2 * m + 1][3], bh[2], bh[3]);
+        add_fragment(acc[m][n], step);
+      }
     }
   }
   auto add = [&](int i, int j, float v) {

@@ -80,3 +80,12 @@ def test_wgrad_float32_result(m, n, chain, dtype):
     W = ops().wgrad(X, Y, 1.0, torch.float32)
     parts = 3 if dtype == torch.float32 else 1              # hi.hi, lo.hi and hi.lo go to one accumulator
     assert bias(W, X.double().t() @ Y.double()) < parts * chain / 2 * BIAS
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("dim", [9999, 98304])
+@pytest.mark.parametrize("n1,n2", [(8, 8), (16, 64), (32, 32), (64, 64), (100, 7), (128, 20), (3, 100)])
+def test_similarity(n1, n2, dim, dtype):
+    a, b = positive((n1, dim), dtype, 1), positive((n2, dim), dtype, 2)
+    S = ops().projection_similarity(a, b)
+    assert bias(S, a.double() @ b.double().t()) < BIAS
