@@ -102,6 +102,11 @@ __device__ __forceinline__ void pass_row_sums(const ghost_pass_job& j, int f0, i
   }
 }
 
+// Sum of eight values in pairs
+template <typename F> __device__ __forceinline__ float pass_sum8(F&& v) {
+  return ((v(0) + v(1)) + (v(2) + v(3))) + ((v(4) + v(5)) + (v(6) + v(7)));
+}
+
 template <int CAP>
 __global__ void __cluster_dims__(kPassCluster, 1, 1) __launch_bounds__(kPassThreads)
 pass_reduce_kernel(const __grid_constant__ PassJobs<CAP> jobs) {
@@ -144,9 +149,9 @@ pass_reduce_kernel(const __grid_constant__ PassJobs<CAP> jobs) {
     float col = 0.f;                     // rank 0: this thread's share of vec
     int buf = 0;
     for (int v0 = 0; v0 < j.n_val; v0 += 8, buf ^= 1) {
-      float acc[8];
+      float4 acc[8];                     // a sum per quarter of the columns: short chains, as one warp per pair had
 #pragma unroll
-      for (int i = 0; i < 8; ++i) acc[i] = 0.f;
+      for (int i = 0; i < 8; ++i) acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
       for (int f = f0; f < f1; f += kPassSub) {
         const int width = f1 - f < kPassSub ? f1 - f : kPassSub;
         __syncthreads();
@@ -157,28 +162,23 @@ pass_reduce_kernel(const __grid_constant__ PassJobs<CAP> jobs) {
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
             const float4 y = *reinterpret_cast<const float4*>(stage + (32 + i) * kPassPitch + q);
-            acc[i] = fmaf(x.x, y.x, acc[i]); acc[i] = fmaf(x.y, y.y, acc[i]);
-            acc[i] = fmaf(x.z, y.z, acc[i]); acc[i] = fmaf(x.w, y.w, acc[i]);
+            acc[i].x = fmaf(x.x, y.x, acc[i].x); acc[i].y = fmaf(x.y, y.y, acc[i].y);
+            acc[i].z = fmaf(x.z, y.z, acc[i].z); acc[i].w = fmaf(x.w, y.w, acc[i].w);
           }
         }
       }
       __syncthreads();
       float* red = stage;                // [warp][validation row][train lane]
 #pragma unroll
-      for (int i = 0; i < 8; ++i) red[(warp * 8 + i) * 32 + lane] = acc[i];
+      for (int i = 0; i < 8; ++i) red[(warp * 8 + i) * 32 + lane] = (acc[i].x + acc[i].y) + (acc[i].z + acc[i].w);
       __syncthreads();
-      float s = 0.f;                     // thread (warp, lane) now owns pair (v0 + warp, b)
-#pragma unroll
-      for (int w = 0; w < 8; ++w) s += red[(w * 8 + warp) * 32 + lane];
-      part[buf][warp][lane] = s;
+      // thread (warp, lane) now owns pair (v0 + warp, b)
+      part[buf][warp][lane] = pass_sum8([&](int w) { return red[(w * 8 + warp) * 32 + lane]; });
       // one cluster barrier per block: `part` alternates, and rank 0 reads block k's before it
       // arrives at block k + 1's barrier, which every CTA passes before writing that buffer again
       cluster.sync();
       if (rank == 0) {
-        float m = 0.f;
-#pragma unroll
-        for (int r = 0; r < kPassCluster; ++r) m += *cluster.map_shared_rank(&part[buf][warp][lane], r);
-        m *= j.dot_scale;
+        const float m = j.dot_scale * pass_sum8([&](int r) { return *cluster.map_shared_rank(&part[buf][warp][lane], r); });
         if (v0 + warp < j.n_val && live) {
           j.M[static_cast<long long>(v0 + warp) * j.n_train + b] = m;
           col += m;
@@ -188,12 +188,7 @@ pass_reduce_kernel(const __grid_constant__ PassJobs<CAP> jobs) {
     if (rank == 0 && j.vec != nullptr) {
       cols[warp][lane] = col;
       __syncthreads();
-      if (warp == 0 && live) {
-        float s = 0.f;
-#pragma unroll
-        for (int w = 0; w < 8; ++w) s += cols[w][lane];
-        j.vec[b] = s;
-      }
+      if (warp == 0 && live) j.vec[b] = pass_sum8([&](int w) { return cols[w][lane]; });
     }
     if (j.sum_out == nullptr) cluster.sync();   // no CTA leaves while rank 0 still reads its shared memory
   }

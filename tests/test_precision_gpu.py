@@ -4,6 +4,8 @@ The tensor core adds into an accumulator that it truncates, so a long chain of p
 comes out too small by up to 2^-23 per product added (2^-24 on average); float32 additions round to
 nearest and leave no such bias.  The data are therefore positive and the tests look at the mean signed
 error over many entries: chains of a few products stay below 2^-23, rounding averages out."""
+import math
+
 import pytest
 import torch
 
@@ -89,3 +91,19 @@ def test_similarity(n1, n2, dim, dtype):
     a, b = positive((n1, dim), dtype, 1), positive((n2, dim), dtype, 2)
     S = ops().projection_similarity(a, b)
     assert bias(S, a.double() @ b.double().t()) < BIAS
+
+
+@pytest.mark.parametrize("F", [768, 50257])
+def test_end_of_pass_gram(F):
+    """Root mean square error of the matrix of per-sample vectors.  256 accumulators a pair take F / 256
+    products each and are added in pairs.  An addition rounds by 0.29 units in the last place on average,
+    2^-23 / m of a sum whose mantissa is m (the same at every level of the pairs); the squares of the levels
+    add up to twice the last one's.  A quarter on top for the spread of the mantissas."""
+    X = positive((256 + 32, F), torch.float32, 7)
+    M = torch.empty(32, 256, device="cuda")
+    ops().pass_reduce([{"X": X, "n_train": 256, "n_val": 32, "M": M}], [])
+    want = X[256:].double() @ X[:256].double().t()
+    rms = ((M.double() - want) / want).pow(2).mean().sqrt().item()
+    m = want.mean().item()
+    one = 0.29 * BIAS / (m / 2.0 ** math.floor(math.log2(m)))
+    assert rms < 1.25 * one * (2 + F / 256 / 3 / 256) ** 0.5
