@@ -26,6 +26,8 @@ static constexpr int kPassSub = 256;                   // columns staged at a ti
 static constexpr int kPassPitch = kPassSub + 4;        // rows 16 bytes apart modulo 128: no bank conflicts
 static constexpr int kPassSmem = 40 * kPassPitch * 4;  // 32 train rows, then eight validation rows
 
+static constexpr double kPassOneMatrix = 1 << 21;     // products of a single matrix that the clusters take
+
 template <int CAP> struct PassJobs { ghost_pass_job job[CAP]; };
 
 __device__ __forceinline__ const float* pass_val_row(const ghost_pass_job& j, int v) {
@@ -199,6 +201,91 @@ pass_reduce_kernel(const __grid_constant__ PassJobs<CAP> jobs) {
   }
 }
 
+// M[v, b] = scale * <X[n_train + v], X[b]> with a warp per pair: for one matrix on its own, whose blocks above
+// are too few to fill the GPU once a pair is long or the validation rows are many (a cluster goes through
+// them eight at a time).  256 x 256 pairs of 768: 93 us in the clusters, 31 here; 256 x 32 of 50257: 473 and 141;
+// 16384 x 1 of 1024: 49 and 19.  Smaller ones, and every matrix of a batch, stay with the clusters, which fetch a row once.
+__global__ void __launch_bounds__(256) small_gram_kernel(const float* __restrict__ X, int n_train, unsigned pairs, int F,
+                                                         float scale, float* __restrict__ M) {
+  const unsigned pair = blockIdx.x * 8u + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  if (pair >= pairs) return;
+  const unsigned v = pair / static_cast<unsigned>(n_train);
+  const float* xv = X + static_cast<long long>(n_train + v) * F;
+  const float* xb = X + static_cast<long long>(pair - v * n_train) * F;
+  float even[4] = {0.f, 0.f, 0.f, 0.f}, odd[4] = {0.f, 0.f, 0.f, 0.f};      // short chains: 256 sums a pair
+  if ((F & 3) == 0 && (reinterpret_cast<uintptr_t>(X) & 15) == 0) {
+    auto add = [&](int f, float (&sum)[4]) {
+      const float4 x = __ldg(reinterpret_cast<const float4*>(xv) + f), y = __ldg(reinterpret_cast<const float4*>(xb) + f);
+      sum[0] = fmaf(x.x, y.x, sum[0]); sum[1] = fmaf(x.y, y.y, sum[1]);
+      sum[2] = fmaf(x.z, y.z, sum[2]); sum[3] = fmaf(x.w, y.w, sum[3]);
+    };
+    const int F4 = F >> 2;
+    int f = lane;
+#pragma unroll 2
+    for (; f + 32 < F4; f += 64) { add(f, even); add(f + 32, odd); }
+    if (f < F4) add(f, even);
+  } else {
+    for (int f0 = lane; f0 < F; f0 += 512) {     // sixteen loads of either row in flight
+      float x[16], y[16];
+#pragma unroll
+      for (int u = 0; u < 16; ++u) {
+        const bool in = f0 + u * 32 < F;
+        x[u] = in ? __ldg(xv + f0 + u * 32) : 0.f;
+        y[u] = in ? __ldg(xb + f0 + u * 32) : 0.f;
+      }
+#pragma unroll
+      for (int u = 0; u < 16; ++u) {
+        float& sum = (u & 4) ? odd[u & 3] : even[u & 3];
+        sum = fmaf(x[u], y[u], sum);
+      }
+    }
+  }
+  float s = ((even[0] + even[1]) + (even[2] + even[3])) + ((odd[0] + odd[1]) + (odd[2] + odd[3]));
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if (lane == 0) M[pair] = s * scale;
+}
+
+// out[c] = (accumulate ? out[c] : 0) + scale * sum over the rows of X[n, c] for one matrix on its own: the
+// additions of pass_row_sums in their order (the same bits), with a block per COLS columns instead of the
+// blocks that a job's pairs ask for.  4 rows of 1000003: 245 us in the
+// batched kernel, 17 here; 256 of 50257: 68 and 16; 16384 of 1024: 626 and 123.
+template <int COLS>
+__global__ void __launch_bounds__(256) rows_sum_kernel(const float* __restrict__ X, int n_rows, int F, float scale,
+                                                       void* __restrict__ out, int out_is_f32, int accumulate) {
+  constexpr int PER = COLS / 32;
+  __shared__ float red[8][COLS];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const long long c0 = blockIdx.x * static_cast<long long>(COLS);
+  float acc[PER];
+#pragma unroll
+  for (int g = 0; g < PER; ++g) acc[g] = 0.f;
+#pragma unroll 8
+  for (int n = warp; n < n_rows; n += 8) {
+    const float* row = X + static_cast<long long>(n) * F + c0;
+#pragma unroll
+    for (int g = 0; g < PER; ++g)
+      if (c0 + g * 32 + lane < F) acc[g] += __ldg(row + g * 32 + lane);
+  }
+#pragma unroll
+  for (int g = 0; g < PER; ++g) red[warp][g * 32 + lane] = acc[g];
+  __syncthreads();
+  const long long c = c0 + threadIdx.x;
+  if (threadIdx.x >= COLS || c >= F) return;
+  float s = 0.f;
+#pragma unroll
+  for (int w = 0; w < 8; ++w) s += red[w][threadIdx.x];
+  s *= scale;
+  if (out_is_f32) {
+    float* o = static_cast<float*>(out) + c;
+    *o = accumulate ? s + *o : s;
+  } else {
+    __nv_bfloat16* o = static_cast<__nv_bfloat16*>(out) + c;
+    *o = __float2bfloat16_rn(accumulate ? s + __bfloat162float(*o) : s);
+  }
+}
+
 template <int CAP>
 static int launch_pass(const ghost_pass_job* jobs, int n, int blocks, cudaStream_t st) {
   PassJobs<CAP> batch;
@@ -315,8 +402,32 @@ extern "C" int ghost_small_gram_f32(const float* X, int n_train, int n_val, int 
   GB_REQUIRE(X && M_out, "ghost_small_gram_f32: null pointer");
   GB_REQUIRE(n_train > 0, "No training samples to compute dot product, check batch sizes.");
   GB_REQUIRE(n_val > 0 && F > 0, "ghost_small_gram_f32: bad dimensions");
-  const ghost_pass_job j = {X, nullptr, M_out, nullptr, nullptr, 0, n_train, n_val, F, 0, 1, scale, 1.f};
-  return ghost_pass_reduce(&j, 1, stream);
+  const long long pairs = static_cast<long long>(n_train) * n_val;
+  if (static_cast<double>(pairs) * F <= kPassOneMatrix) {
+    const ghost_pass_job j = {X, nullptr, M_out, nullptr, nullptr, 0, n_train, n_val, F, 0, 1, scale, 1.f};
+    return ghost_pass_reduce(&j, 1, stream);
+  }
+  if (!device_state()) return GHOST_ERR_DEVICE;
+  GB_REQUIRE(pairs < (1ll << 32) - 8, "ghost_small_gram_f32: too many pairs");
+  small_gram_kernel<<<ceil_div(pairs, 8), 256, 0, static_cast<cudaStream_t>(stream)>>>(X, n_train, static_cast<unsigned>(pairs), F, scale, M_out);
+  count_launch();
+  return post_launch("small_gram_kernel");
+}
+
+extern "C" int ghost_rows_sum(const float* X, int n_rows, int F, float scale, void* out, int out_is_f32,
+                              int accumulate, void* stream) {
+  const DeviceState* ds = device_state();
+  if (!ds) return GHOST_ERR_DEVICE;
+  GB_REQUIRE(X && out, "ghost_rows_sum: null pointer");
+  GB_REQUIRE(n_rows > 0 && F > 0, "ghost_rows_sum: bad dimensions");
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  // wide blocks read full lines; narrow ones while a row has too few for the GPU
+  if (ceil_div(F, 128) >= ds->sm_count)
+    rows_sum_kernel<128><<<ceil_div(F, 128), 256, 0, st>>>(X, n_rows, F, scale, out, out_is_f32, accumulate);
+  else
+    rows_sum_kernel<32><<<ceil_div(F, 32), 256, 0, st>>>(X, n_rows, F, scale, out, out_is_f32, accumulate);
+  count_launch();
+  return post_launch("rows_sum_kernel");
 }
 
 extern "C" int ghost_matrix_sum(const float* const* mats, int n_mats, int n_val, int n_train, float* total,

@@ -1,7 +1,6 @@
 // Bandwidth-bound kernels of the ghost hot path: dtype cast / bf16 split, per-sample column sums
-// (bias terms), per-sample LayerNorm gradients, and row sums that add per-sample vectors to an
-// averaged train gradient.  All of them stream their inputs once with 16-byte coalesced loads and
-// reduce with warp shuffles / shared memory.
+// (bias terms) and per-sample LayerNorm gradients.  All of them stream their inputs once with
+// 16-byte coalesced loads and reduce with warp shuffles / shared memory.
 #include "common.cuh"
 
 namespace gb {
@@ -468,18 +467,6 @@ layernorm_persample_generic_kernel(const T* __restrict__ A, const T* __restrict_
   }
 }
 
-// out[c] += scale * sum_{n < n_rows} X[n, c]
-template <typename OutT>
-__global__ void rows_sum_kernel(const float* __restrict__ X, int n_rows, int F, float scale,
-                                OutT* __restrict__ out) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= F) return;
-  float s = 0.f;
-#pragma unroll 8
-  for (int n = 0; n < n_rows; ++n) s += __ldg(X + static_cast<long long>(n) * F + c);
-  out[c] = static_cast<OutT>(s * scale + static_cast<float>(out[c]));
-}
-
 }  // namespace gb
 
 using namespace gb;
@@ -660,21 +647,4 @@ extern "C" int ghost_rmsnorm_persample(const void* A, const void* G, int is_f32,
                                        int F, float eps, float* gw, float* gsum, void* ws,
                                        long long ws_bytes, void* stream) {
   return norm_persample("ghost_rmsnorm_persample", A, G, is_f32, N, T, F, eps, gw, gsum, ws, ws_bytes, stream, 1);
-}
-
-extern "C" int ghost_rows_sum(const float* X, int n_rows, int F, float scale, void* out, int out_is_f32,
-                              int accumulate, void* stream) {
-  const DeviceState* ds = device_state();
-  if (!ds) return GHOST_ERR_DEVICE;
-  GB_REQUIRE(X && out, "ghost_rows_sum: null pointer");
-  GB_REQUIRE(n_rows > 0 && F > 0, "ghost_rows_sum: bad dimensions");
-  if (!accumulate) {                     // the batched launch's arithmetic, so both give the same bits
-    const ghost_pass_job j = {X, nullptr, nullptr, nullptr, out, 0, n_rows, 0, F, 0, out_is_f32, 1.f, scale};
-    return ghost_pass_reduce(&j, 1, stream);
-  }
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (out_is_f32) rows_sum_kernel<float><<<ceil_div(F, 64), 64, 0, st>>>(X, n_rows, F, scale, static_cast<float*>(out));
-  else rows_sum_kernel<__nv_bfloat16><<<ceil_div(F, 64), 64, 0, st>>>(X, n_rows, F, scale, static_cast<__nv_bfloat16*>(out));
-  count_launch();
-  return post_launch("rows_sum_kernel");
 }

@@ -773,6 +773,33 @@ def test_small_reduce_batch_matches_single_launches():
             assert torch.equal(job["sum_out"], rec["sum"])
 
 
+# one matrix on its own, beyond what the batched launch's blocks take: vector and scalar loads, remainders
+@pytest.mark.parametrize("n_t,n_v,F", [(300, 30, 772), (2000, 3, 1001), (70, 40, 4100), (5, 3, 150001), (600, 8, 512)])
+def test_small_gram_of_large_vectors(n_t, n_v, F):
+    X = torch.randn(n_t + n_v, F, generator=torch.Generator().manual_seed(3)).cuda()
+    M = ops().small_gram(X, n_v, 0.5)
+    after()
+    want = 0.5 * X[n_t:].double() @ X[:n_t].double().t()
+    # 256 float32 accumulators of F / 256 products each, then pairs: a rounding of 2^-24 per level of the sum
+    bound = (F / 256 + 9) * 2.0 ** -24 * 0.5 * (X[n_t:].double().abs() @ X[:n_t].double().abs().t())
+    assert ((M.double() - want).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("n,F", [(4, 20003), (33, 50257), (300, 100), (9, 1), (7, 18944), (1, 31)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_rows_sum_gives_the_batched_launchs_bits(n, F, dtype):
+    o = ops()
+    X = torch.randn(n, F, generator=torch.Generator().manual_seed(4)).cuda()
+    S = torch.empty(F, dtype=dtype, device="cuda")
+    o.small_reduce_batch([{"X": X, "n_train": n, "n_val": 0, "sum_out": S, "sum_scale": 0.25}])
+    got = o.rows_sum(X, n, 0.25, dtype)
+    after()
+    assert torch.equal(got, S)
+    more = o.rows_sum(X, n, 0.25, dtype, out=got.clone(), accumulate=True)
+    after()
+    assert O.rel_fro(more, 2 * S.double()) < (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -22)
+
+
 def test_error_codes_are_python_exceptions():
     o = ops()
     A = torch.randn(4, 3, 8, device="cuda")
