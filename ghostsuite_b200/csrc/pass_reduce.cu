@@ -116,25 +116,26 @@ pass_reduce_kernel(const __grid_constant__ PassJobs<CAP> jobs) {
   __shared__ float part[2][8][32];       // this CTA's share of F, read by rank 0 of the cluster
   __shared__ float cols[8][32];
   const ghost_pass_job& j = jobs.job[blockIdx.z];
-  const int blk = blockIdx.y;
-  const int n_blk = (j.n_train + 31) / 32;
-  if (blk >= n_blk) return;              // the whole cluster leaves
+  const int n_blk = (j.n_train + 31) / 32, step = gridDim.y;       // one block each, unless a job has more than a grid
+  if (blockIdx.y >= n_blk) return;       // the whole cluster leaves
   const int rank = blockIdx.x;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int b = blk * 32 + lane;
-  const bool live = b < j.n_train;
 
   if (j.X == nullptr) {                  // the matrix exists already: column sums only
     if (rank != 0) return;
-    float s = 0.f;
-    if (live)
-      for (int v = warp; v < j.n_val; v += 8) s += j.M[static_cast<long long>(v) * j.n_train + b];
-    cols[warp][lane] = s;
-    __syncthreads();
-    if (warp == 0 && live) {
+    for (int blk = blockIdx.y; blk < n_blk; blk += step) {
+      const int b = blk * 32 + lane;
+      float s = 0.f;
+      if (b < j.n_train)
+        for (int v = warp; v < j.n_val; v += 8) s += j.M[static_cast<long long>(v) * j.n_train + b];
+      __syncthreads();
+      cols[warp][lane] = s;
+      __syncthreads();
+      if (warp == 0 && b < j.n_train) {
 #pragma unroll
-      for (int w = 1; w < 8; ++w) s += cols[w][lane];
-      j.vec[b] = s;
+        for (int w = 1; w < 8; ++w) s += cols[w][lane];
+        j.vec[b] = s;
+      }
     }
     return;
   }
@@ -148,55 +149,61 @@ pass_reduce_kernel(const __grid_constant__ PassJobs<CAP> jobs) {
   if (j.M != nullptr) {
     cg::cluster_group cluster = cg::this_cluster();
     const bool vec = vec_x && (j.Xv == nullptr || ((reinterpret_cast<uintptr_t>(j.Xv) & 15) == 0 && (j.v_rank_pitch & 3) == 0));
-    float col = 0.f;                     // rank 0: this thread's share of vec
     int buf = 0;
-    for (int v0 = 0; v0 < j.n_val; v0 += 8, buf ^= 1) {
-      float4 acc[8];                     // a sum per quarter of the columns: short chains, as one warp per pair had
+    for (int blk = blockIdx.y; blk < n_blk; blk += step) {
+      const int b = blk * 32 + lane;
+      const bool live = b < j.n_train;
+      float col = 0.f;                     // rank 0: this thread's share of vec
+      for (int v0 = 0; v0 < j.n_val; v0 += 8, buf ^= 1) {
+        float4 acc[8];                     // a sum per quarter of the columns: short chains, as one warp per pair had
 #pragma unroll
-      for (int i = 0; i < 8; ++i) acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-      for (int f = f0; f < f1; f += kPassSub) {
-        const int width = f1 - f < kPassSub ? f1 - f : kPassSub;
-        __syncthreads();
-        pass_stage(j, vec, blk * 32, v0, f, width, stage);
-        __syncthreads();
-        for (int q = warp * 4; q < width; q += 32) {
-          const float4 x = *reinterpret_cast<const float4*>(stage + lane * kPassPitch + q);
+        for (int i = 0; i < 8; ++i) acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int f = f0; f < f1; f += kPassSub) {
+          const int width = f1 - f < kPassSub ? f1 - f : kPassSub;
+          __syncthreads();
+          pass_stage(j, vec, blk * 32, v0, f, width, stage);
+          __syncthreads();
+          for (int q = warp * 4; q < width; q += 32) {
+            const float4 x = *reinterpret_cast<const float4*>(stage + lane * kPassPitch + q);
 #pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const float4 y = *reinterpret_cast<const float4*>(stage + (32 + i) * kPassPitch + q);
-            acc[i].x = fmaf(x.x, y.x, acc[i].x); acc[i].y = fmaf(x.y, y.y, acc[i].y);
-            acc[i].z = fmaf(x.z, y.z, acc[i].z); acc[i].w = fmaf(x.w, y.w, acc[i].w);
+            for (int i = 0; i < 8; ++i) {
+              const float4 y = *reinterpret_cast<const float4*>(stage + (32 + i) * kPassPitch + q);
+              acc[i].x = fmaf(x.x, y.x, acc[i].x); acc[i].y = fmaf(x.y, y.y, acc[i].y);
+              acc[i].z = fmaf(x.z, y.z, acc[i].z); acc[i].w = fmaf(x.w, y.w, acc[i].w);
+            }
+          }
+        }
+        __syncthreads();
+        float* red = stage;                // [warp][validation row][train lane]
+#pragma unroll
+        for (int i = 0; i < 8; ++i) red[(warp * 8 + i) * 32 + lane] = (acc[i].x + acc[i].y) + (acc[i].z + acc[i].w);
+        __syncthreads();
+        // thread (warp, lane) now owns pair (v0 + warp, b)
+        part[buf][warp][lane] = pass_sum8([&](int w) { return red[(w * 8 + warp) * 32 + lane]; });
+        // one cluster barrier per block: `part` alternates, and rank 0 reads block k's before it
+        // arrives at block k + 1's barrier, which every CTA passes before writing that buffer again
+        cluster.sync();
+        if (rank == 0) {
+          const float m = j.dot_scale * pass_sum8([&](int r) { return *cluster.map_shared_rank(&part[buf][warp][lane], r); });
+          if (v0 + warp < j.n_val && live) {
+            j.M[static_cast<long long>(v0 + warp) * j.n_train + b] = m;
+            col += m;
           }
         }
       }
-      __syncthreads();
-      float* red = stage;                // [warp][validation row][train lane]
-#pragma unroll
-      for (int i = 0; i < 8; ++i) red[(warp * 8 + i) * 32 + lane] = (acc[i].x + acc[i].y) + (acc[i].z + acc[i].w);
-      __syncthreads();
-      // thread (warp, lane) now owns pair (v0 + warp, b)
-      part[buf][warp][lane] = pass_sum8([&](int w) { return red[(w * 8 + warp) * 32 + lane]; });
-      // one cluster barrier per block: `part` alternates, and rank 0 reads block k's before it
-      // arrives at block k + 1's barrier, which every CTA passes before writing that buffer again
-      cluster.sync();
-      if (rank == 0) {
-        const float m = j.dot_scale * pass_sum8([&](int r) { return *cluster.map_shared_rank(&part[buf][warp][lane], r); });
-        if (v0 + warp < j.n_val && live) {
-          j.M[static_cast<long long>(v0 + warp) * j.n_train + b] = m;
-          col += m;
-        }
+      if (rank == 0 && j.vec != nullptr) {
+        cols[warp][lane] = col;
+        __syncthreads();
+        if (warp == 0 && live) j.vec[b] = pass_sum8([&](int w) { return cols[w][lane]; });
       }
-    }
-    if (rank == 0 && j.vec != nullptr) {
-      cols[warp][lane] = col;
-      __syncthreads();
-      if (warp == 0 && live) j.vec[b] = pass_sum8([&](int w) { return cols[w][lane]; });
+      __syncthreads();                   // `cols` and the staged rows are free for the next block
     }
     if (j.sum_out == nullptr) cluster.sync();   // no CTA leaves while rank 0 still reads its shared memory
   }
   if (j.sum_out != nullptr) {
-    if (vec_x) pass_row_sums<true>(j, f0, f1, blk, n_blk, stage);
-    else pass_row_sums<false>(j, f0, f1, blk, n_blk, stage);
+    const int share = n_blk < step ? n_blk : step;
+    if (vec_x) pass_row_sums<true>(j, f0, f1, blockIdx.y, share, stage);
+    else pass_row_sums<false>(j, f0, f1, blockIdx.y, share, stage);
     if (j.M != nullptr) cg::this_cluster().sync();
   }
 }
@@ -350,7 +357,6 @@ extern "C" int ghost_pass_reduce(const ghost_pass_job* jobs, int n_jobs, void* s
   for (int i = 0; i < n_jobs; ++i) {
     const ghost_pass_job& j = jobs[i];
     GB_REQUIRE(j.n_train > 0 && j.n_val >= 0 && (j.M == nullptr || j.n_val > 0), "ghost_pass_reduce: job %d has an empty dimension", i);
-    GB_REQUIRE(j.n_train <= 32 * 65535, "ghost_pass_reduce: job %d has too many train samples", i);
     if (j.X == nullptr) {
       GB_REQUIRE(j.M != nullptr && j.vec != nullptr, "ghost_pass_reduce: job %d has no input or no output", i);
       continue;
@@ -370,7 +376,7 @@ extern "C" int ghost_pass_reduce(const ghost_pass_job* jobs, int n_jobs, void* s
     const int n = n_jobs - first < kLarge ? n_jobs - first : kLarge;
     int most = 1;
     for (int i = 0; i < n; ++i) most = jobs[first + i].n_train > most ? jobs[first + i].n_train : most;
-    const int blocks = ceil_div(most, 32);
+    const int blocks = ceil_div(most, 32) < 65535 ? ceil_div(most, 32) : 65535;
     const int rc = n <= 4 ? launch_pass<4>(jobs + first, n, blocks, st)
                  : n <= 40 ? launch_pass<40>(jobs + first, n, blocks, st)
                            : launch_pass<kLarge>(jobs + first, n, blocks, st);

@@ -800,6 +800,22 @@ def test_rows_sum_gives_the_batched_launchs_bits(n, F, dtype):
     assert O.rel_fro(more, 2 * S.double()) < (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -22)
 
 
+def test_more_train_samples_than_a_grid_has_blocks():
+    """Jobs of more than 32 x 65535 train samples: the blocks take several groups of 32 in turn."""
+    o = ops()
+    n_t = 32 * 65535 + 70
+    X = torch.randint(-4, 5, (n_t + 3, 1), generator=torch.Generator().manual_seed(1)).float().cuda()
+    M, S = torch.empty(3, n_t, device="cuda"), torch.empty(1, device="cuda")
+    o.small_reduce_batch([{"X": X, "n_train": n_t, "n_val": 3, "M": M, "sum_out": S}])
+    vec, again = o.pass_reduce([{"X": X, "n_train": n_t, "n_val": 3, "M": (M2 := torch.empty_like(M))}], [M2, M])
+    rows = o.rows_sum(X, n_t, 1.0, torch.float32)
+    after()
+    want = X[n_t:] * X[:n_t].T                       # whole numbers: exact
+    assert torch.equal(M, want) and torch.equal(M2, want)
+    assert torch.equal(vec, want.sum(0)) and torch.equal(again, want.sum(0))
+    assert S.item() == rows.item() == X[:n_t].sum().item()
+
+
 def test_error_codes_are_python_exceptions():
     o = ops()
     A = torch.randn(4, 3, 8, device="cuda")
