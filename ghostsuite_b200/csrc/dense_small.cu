@@ -228,11 +228,20 @@ using namespace gb;
 // gradient (about 12e12 a second here).  Beyond these the fixed costs it avoids -- some 40 us of
 // launches for float32 operands, 20 us for bf16 -- no longer pay for slower arithmetic.  A pair of
 // samples is one block, which walks its token tiles in turn (1.5 us each): at most eight of them.
+//
+// A gradient tile is one block that walks all train rows, 0.045 us each (float32; 0.045 to 0.067 bf16),
+// however few the tiles are; the tensor-core paths split the rows.  GPU time of a hook, this kernel
+// against the better of them: 64 -> 64 float32, one-token samples, 35 / 34 us at 768 rows, 91 / 37 at 2048,
+// 715 / 68 at 16384; 1024 -> 128 45 / 58 us at 1024 rows, 70 / 58 at 1536; with 16 tokens a sample 23 / 21
+// at 512, 45 / 23 at 1024; bf16 64 -> 64 23 / 25 us at 512 rows, 45 / 26 at 1024.
 extern "C" int ghost_dense_small_fits(int is_f32, int n_train, int n_val, long long T, int d, int p) {
   const double pairs = static_cast<double>(n_train) * T * n_val * T;
-  const double macs = static_cast<double>(n_train) * T * d * p;
+  const double train_rows = static_cast<double>(n_train) * T;
+  const double macs = train_rows * d * p;
   const double rows = static_cast<double>(n_train + n_val) * T;
-  return T <= 16 && pairs * (d + p) <= 2e7 && macs <= (is_f32 ? 3e8 : 6e7) && rows * p <= 1e8 ? 1 : 0;
+  const double chain = !is_f32 || T > 4 ? 512 : 700 + 0.6 * (static_cast<double>(d) + p);
+  return T <= 16 && pairs * (static_cast<double>(d) + p) <= 2e7 && macs <= (is_f32 ? 3e8 : 6e7) && rows * p <= 1e8 &&
+         train_rows <= chain ? 1 : 0;
 }
 
 extern "C" int ghost_dense_small(const void* A, const void* B, int is_f32, int n_train, int n_val, long long T, int d,

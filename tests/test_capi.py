@@ -59,3 +59,16 @@ def test_kernel_switches_validate_their_argument():
         assert fn(-1) < 0 and fn(3) < 0
         for mode in (0, 2, default):
             assert fn(mode) == 0
+
+
+def test_small_dense_layers_are_bounded_by_the_rows_of_a_tile():
+    """A gradient tile of the one-launch kernel walks all train rows in turn: long chains are the GEMM's."""
+    from ghostsuite_b200 import _lib
+    fits = _lib.load().ghost_dense_small_fits
+    # (is_f32, n_train, n_val, T, d, p)
+    for args in ((1, 64, 16, 1, 512, 1024), (1, 64, 16, 1, 1024, 10), (1, 768, 8, 1, 64, 64), (1, 1024, 8, 1, 1024, 128),
+                 (1, 32, 8, 16, 64, 64), (0, 512, 8, 1, 64, 64)):
+        assert fits(*args) == 1, args
+    for args in ((1, 16384, 8, 1, 64, 64), (1, 8192, 8, 1, 128, 10), (0, 256, 1, 16, 64, 64), (0, 2048, 1, 8, 128, 10),
+                 (1, 2048, 1, 1, 1024, 128), (0, 1024, 1, 1, 64, 64), (1, 64, 1, 16, 64, 64)):
+        assert fits(*args) == 0, args
