@@ -430,17 +430,19 @@ void dense_paths(const Launch& L, const Operand& A, const Operand& B, long long 
 }
 
 // Everything the backward hook of a Linear / Conv1D layer computes or allocates:
-// (A, B, n_val, weight_is_in_by_out, use_gram, weight grad dtype, grad scale, has_bias, bias grad dtype, any_path)
+// (A, B, n_val, weight_is_in_by_out, use_gram, weight grad dtype, grad scale, has_bias, bias grad dtype, any_path,
+// fuse_colsums)
 // -> (M, weight grad, column sums of B, unfilled bias matrix, unfilled bias grad), None where not wanted.
 PyObject* py_dense_hook(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return guarded([&]() -> PyObject* {
-    need(n, 10, "dense_hook");
+    need(n, 11, "dense_hook");
     const Tensor &A0 = cuda_tensor(a[0]), &B0 = cuda_tensor(a[1]);
     Launch L(A0);
     const Tensor A = as3d(A0), B = as3d(B0);
     const long long n_val = integer(a[2]), N = A.size(0), n_train = N - n_val, p = B.size(2);
     const bool in_by_out = integer(a[3]) != 0, gram = integer(a[4]) != 0, bias = integer(a[7]) != 0;
     const long long gdt = integer(a[5]), bdt = integer(a[8]);
+    const bool fuse = bias && integer(a[10]) != 0;
     const float scale = real(a[6]);
     const Tensor &X = in_by_out ? A : B, &Y = in_by_out ? B : A;
     Tensor M, grad, sums;
@@ -452,12 +454,12 @@ PyObject* py_dense_hook(PyObject*, PyObject* const* a, Py_ssize_t n) {
       M = empty({n_val, n_train}, A, at::kFloat);
       grad = optional_empty({X.size(2), Y.size(2)}, X, gdt);
       // written out even for one float32 token, whose row is the sum: they are read when the pass ends
-      if (bias) sums = empty({N, p}, A, at::kFloat);
+      if (fuse) sums = empty({N, p}, A, at::kFloat);
       check(ghost_dense_small(A.data_ptr(), B.data_ptr(), is_f32(A), static_cast<int>(n_train), static_cast<int>(n_val),
                               A.size(1), dI, pI, in_by_out ? 1 : 0, M.data_ptr<float>(), grad.defined() ? grad.data_ptr() : nullptr,
-                              grad.defined() ? is_f32(grad) : 0, scale, bias ? sums.data_ptr<float>() : nullptr, L.st()));
+                              grad.defined() ? is_f32(grad) : 0, scale, fuse ? sums.data_ptr<float>() : nullptr, L.st()));
     } else {
-      dense_paths(L, Operand(A), Operand(B), n_val, in_by_out, gram, gdt, scale, bias, M, grad, sums);
+      dense_paths(L, Operand(A), Operand(B), n_val, in_by_out, gram, gdt, scale, fuse, M, grad, sums);
     }
     if (bias && !sums.defined()) sums = colsum(L, B);
     Tensor Mb = bias ? empty({n_val, n_train}, A, at::kFloat) : Tensor();

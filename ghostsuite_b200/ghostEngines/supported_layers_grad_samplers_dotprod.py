@@ -467,7 +467,7 @@ def _dense_hook(layer: nn.Module, A: torch.Tensor, B: torch.Tensor, n_val: int, 
     M, grad, colsums, bias_M, bias_grad = ops.dense_hook(
         A, B, n_val, weight_is_in_by_out, layer.use_ghost_computation,
         _grad_dtype(weight, A) if getattr(weight, "initially_requires_grad", True) else None, scale,
-        bias is not None, bias_dtype, PATH_RULE == "cost")
+        bias is not None, bias_dtype, PATH_RULE == "cost", FUSE_BIAS_COLSUMS)
     if grad is not None:
         own["_ghost_cached_train_grad"] = (A.data_ptr(), B.data_ptr(), A.size(0), grad)
     _set_dot(weight, M)

@@ -214,14 +214,15 @@ def _dtype_code(dt: Optional[torch.dtype]) -> int:
 
 def dense_hook(A: torch.Tensor, B: torch.Tensor, n_val: int, weight_is_in_by_out: bool, use_gram: bool,
                grad_dtype: Optional[torch.dtype], grad_scale: float, has_bias: bool,
-               bias_grad_dtype: Optional[torch.dtype], any_path: bool = True):
+               bias_grad_dtype: Optional[torch.dtype], any_path: bool = True, fuse_colsums: bool = True):
     """All that the backward hook of a Linear / Conv1D layer needs, in one native call: ``(M, weight
     gradient, column sums of B, bias matrix, bias gradient)``, None where not wanted (a dtype of None,
     no bias).  With ``any_path`` a layer of few token rows takes the one-launch kernel of
-    ``ghost_dense_small`` whatever ``use_gram`` says.  The last two are allocated only: they are filled by the launch that ends the backward
-    pass (:func:`pass_reduce`)."""
+    ``ghost_dense_small`` whatever ``use_gram`` says.  Without ``fuse_colsums`` the column sums take a launch of
+    their own instead of falling out of another kernel's pass over ``B``.  The last two are allocated
+    only: they are filled by the launch that ends the backward pass (:func:`pass_reduce`)."""
     args = (A, B, n_val, weight_is_in_by_out, use_gram, _dtype_code(grad_dtype), grad_scale, has_bias,
-            _dtype_code(bias_grad_dtype), any_path)
+            _dtype_code(bias_grad_dtype), any_path, fuse_colsums)
     if _timing is None:
         return _native().dense_hook(*args)
     d, p, rows, N = _cols(A), _cols(B), _rows(A), A.shape[0]

@@ -1,6 +1,7 @@
 """Host-side logic that needs no GPU: deferred reduction of the dot-product vectors, the path rule's
 cost model, the flat projection file format."""
 import contextlib
+import inspect
 import io
 
 import numpy as np
@@ -111,3 +112,31 @@ def test_parameter_walk_of_modules_with_tables_of_their_own():
         want, got = list(m.named_parameters()), _lib.named_parameters(m)
         assert [n for n, _ in got] == [n for n, _ in want]
         assert all(a.data_ptr() == b.data_ptr() for (_, a), (_, b) in zip(got, want))
+
+
+_DENSE_HOOK = inspect.signature(L.ops.dense_hook)
+
+
+def _hook_arguments(monkeypatch, layer, dtype=torch.float32, n=6, n_val=2):
+    """What the backward hook of a dense layer asks the native call for."""
+    seen = {}
+
+    def call(*args, **kwargs):
+        bound = _DENSE_HOOK.bind(*args, **kwargs)
+        bound.apply_defaults()
+        seen.update(bound.arguments)
+        return torch.zeros(n_val, n - n_val), None, None, torch.zeros(n_val, n - n_val), None
+
+    monkeypatch.setattr(L.ops, "dense_hook", call)
+    monkeypatch.setattr(L, "_gram_of_vectors", lambda X, n_v, M=None: M)
+    layer._ghost_backprop_scale = 1.0
+    L._compute_linear_dot_product(layer, torch.zeros(n, layer.in_features, dtype=dtype),
+                                  torch.zeros(n, layer.out_features, dtype=dtype), n_val)
+    del layer._ghost_backprop_scale
+    return seen
+
+
+def test_switch_for_fused_column_sums_reaches_the_hook(monkeypatch):
+    assert _hook_arguments(monkeypatch, nn.Linear(8, 8))["fuse_colsums"] is True
+    monkeypatch.setattr(L, "FUSE_BIAS_COLSUMS", False)
+    assert _hook_arguments(monkeypatch, nn.Linear(8, 8))["fuse_colsums"] is False

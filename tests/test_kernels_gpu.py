@@ -816,6 +816,24 @@ def test_more_train_samples_than_a_grid_has_blocks():
     assert S.item() == rows.item() == X[:n_t].sum().item()
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("any_path,use_gram", [(True, True), (False, True), (False, False)])
+def test_dense_hook_with_separate_column_sums(any_path, use_gram, dtype):
+    from ghostsuite_b200 import _lib
+    A, G = make(7, 5, 40, 24, dtype)
+    res, launches = [], []
+    for fuse in (True, False):
+        l0 = _lib.launch_count()
+        res.append(ops().dense_hook(A.cuda(), G.cuda(), 2, False, use_gram, dtype, 1.0, True, dtype, any_path, fuse))
+        launches.append(_lib.launch_count() - l0)
+    after()
+    assert torch.equal(res[0][0], res[1][0]) and torch.equal(res[0][1], res[1][1])
+    for r in res:
+        assert O.rel_fro(r[2], G.double().sum(1)) < 1e-6
+    taken_along = any_path or (not use_gram and dtype == torch.bfloat16)
+    assert launches[1] - launches[0] == (1 if taken_along else 0)
+
+
 def test_error_codes_are_python_exceptions():
     o = ops()
     A = torch.randn(4, 3, 8, device="cuda")
