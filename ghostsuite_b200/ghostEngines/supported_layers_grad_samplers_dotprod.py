@@ -120,7 +120,8 @@ def _should_use_ghost_computation(layer: nn.Module, A: torch.Tensor, B: torch.Te
         per = (2.0 * (n_t + n_v) * T * d * p / _PERSAMPLE_FLOPS
                + 2.0 * d * p * (n_t + n_v) / _TILE_WRITE_BYTES_PER_S
                + 2.0 * d * p * (32 + vr) * passes / _STREAM_BYTES_PER_S)
-    layer.use_ghost_computation = bool(gram <= per)
+    # remembered apart from the choice itself, which a user may set
+    layer.use_ghost_computation = layer._ghost_rule_choice = bool(gram <= per)
 
 
 #: optional observer ``fn(param)`` called every time a layer has added its contribution to
@@ -467,7 +468,8 @@ def _dense_hook(layer: nn.Module, A: torch.Tensor, B: torch.Tensor, n_val: int, 
     M, grad, colsums, bias_M, bias_grad = ops.dense_hook(
         A, B, n_val, weight_is_in_by_out, layer.use_ghost_computation,
         _grad_dtype(weight, A) if getattr(weight, "initially_requires_grad", True) else None, scale,
-        bias is not None, bias_dtype, PATH_RULE == "cost", FUSE_BIAS_COLSUMS)
+        bias is not None, bias_dtype,
+        PATH_RULE == "cost" and own.get("_ghost_rule_choice") is own.get("use_ghost_computation"), FUSE_BIAS_COLSUMS)
     if grad is not None:
         own["_ghost_cached_train_grad"] = (A.data_ptr(), B.data_ptr(), A.size(0), grad)
     _set_dot(weight, M)

@@ -140,3 +140,19 @@ def test_switch_for_fused_column_sums_reaches_the_hook(monkeypatch):
     assert _hook_arguments(monkeypatch, nn.Linear(8, 8))["fuse_colsums"] is True
     monkeypatch.setattr(L, "FUSE_BIAS_COLSUMS", False)
     assert _hook_arguments(monkeypatch, nn.Linear(8, 8))["fuse_colsums"] is False
+
+
+def test_preset_path_is_not_passed_over(monkeypatch):
+    """The one-launch kernel of small layers stands in for the rule's choice, not for a user's."""
+    ruled = nn.Linear(8, 8)
+    assert _hook_arguments(monkeypatch, ruled)["any_path"] is True
+    assert _hook_arguments(monkeypatch, ruled)["any_path"] is True          # the cached choice is still the rule's
+    for choice in (True, False):
+        preset = nn.Linear(8, 8)
+        preset.use_ghost_computation = choice
+        seen = _hook_arguments(monkeypatch, preset)
+        assert seen["any_path"] is False and seen["use_gram"] is choice
+    ruled.use_ghost_computation = not ruled.use_ghost_computation
+    assert _hook_arguments(monkeypatch, ruled)["any_path"] is False
+    monkeypatch.setattr(L, "PATH_RULE", "gram")
+    assert _hook_arguments(monkeypatch, nn.Linear(8, 8))["any_path"] is False
