@@ -827,7 +827,8 @@ def test_dense_hook_with_separate_column_sums(any_path, use_gram, dtype):
         res.append(ops().dense_hook(A.cuda(), G.cuda(), 2, False, use_gram, dtype, 1.0, True, dtype, any_path, fuse))
         launches.append(_lib.launch_count() - l0)
     after()
-    assert torch.equal(res[0][0], res[1][0]) and torch.equal(res[0][1], res[1][1])
+    # the per-sample path adds a handful of blocks' sums in any order: a rounding of 2^-24 each
+    assert O.rel_fro(res[0][0], res[1][0].double()) < 8 * 2.0 ** -24 and torch.equal(res[0][1], res[1][1])
     for r in res:
         assert O.rel_fro(r[2], G.double().sum(1)) < 1e-6
     taken_along = any_path or (not use_gram and dtype == torch.bfloat16)
