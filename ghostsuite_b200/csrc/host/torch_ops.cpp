@@ -116,6 +116,12 @@ Tensor ids2d(const Tensor& x0) {
 bool tma_ready(const Tensor& x) {
   return x.scalar_type() == at::kBFloat16 && x.size(-1) % 8 == 0 && (reinterpret_cast<uintptr_t>(x.data_ptr()) & 15u) == 0;
 }
+// A caller's result buffer, which the kernels write as rows x cols elements from its start.
+void check_result(const Tensor& out, long long rows, long long cols, const Tensor& like, const char* who) {
+  if (out.numel() != rows * cols || !out.is_contiguous() || out.get_device() != like.get_device())
+    invalid(std::string(who) + ": the output must be a contiguous " + std::to_string(rows) + " x " + std::to_string(cols) +
+            " tensor on the operands' device");
+}
 long long pad8(long long n) { return (n + 7) / 8 * 8; }
 Tensor empty(at::IntArrayRef size, const Tensor& like, at::ScalarType dt) { return at::empty(size, like.options().dtype(dt)); }
 
@@ -307,6 +313,7 @@ PyObject* py_wgrad(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (Y.size(0) != X.size(0) || Y.size(1) != X.size(1)) invalid("wgrad operands disagree on the token layout");
     const bool have = present(a[4]);
     Tensor out = have ? cuda_tensor(a[4]) : empty({X.size(2), Y.size(2)}, X, integer(a[3]) ? at::kFloat : at::kBFloat16);
+    if (have) check_result(out, X.size(2), Y.size(2), X, "wgrad");
     wgrad(L, Operand(X), Operand(Y), X.size(0), real(a[2]), out, have && integer(a[5]));
     return wrap(out);
   });
@@ -578,6 +585,9 @@ PyObject* py_embedding_wgrad(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const bool have = present(a[6]);
     Tensor out = have ? cuda_tensor(a[6]) : empty({vocab, d}, G, G.scalar_type());
     if (out.scalar_type() != G.scalar_type()) invalid("embedding_wgrad output must have the dtype of the out-grad");
+    if (have) check_result(out, vocab, d, G, "embedding_wgrad");
+    if (n_train > G.size(0) || ids.size(0) < n_train || ids.size(1) != T)
+      invalid("embedding ids and out-grad do not hold the train samples");
     Workspace ws;
     const long long ws_bytes = ghost_embedding_wgrad_workspace_bytes(static_cast<int>(n_train), T, static_cast<int>(vocab));
     const long long off = ws.plan(ws_bytes);

@@ -835,6 +835,23 @@ def test_dense_hook_with_separate_column_sums(any_path, use_gram, dtype):
     assert launches[1] - launches[0] == (1 if taken_along else 0)
 
 
+def test_result_buffers_and_samples_are_checked_before_anything_is_written():
+    o = ops()
+    X = torch.randn(1, 8, 16).cuda()
+    good = torch.zeros(16, 16).cuda()
+    for out in (torch.zeros(16, 15).cuda(), torch.zeros(16, 32).cuda()[:, :16], good.t()[:8]):
+        with pytest.raises(ValueError):
+            o.wgrad(X, X, 1.0, torch.float32, out=out)
+    assert torch.equal(o.wgrad(X, X, 1.0, torch.float32, out=good.view(256)).view(16, 16), o.wgrad(X, X, 1.0, torch.float32))
+    ids, G = torch.zeros(3, 4, dtype=torch.long).cuda(), torch.randn(3, 4, 8).cuda()
+    for kw in (dict(n_train=4), dict(vocab=6, out=torch.zeros(5, 8).cuda()), dict(ids=ids[:, :3]), dict(ids=ids[:1])):
+        args = dict(ids=ids, G=G, n_train=2, vocab=5, pre_scale=1.0, divisor=2.0)
+        args.update(kw)
+        with pytest.raises(ValueError):
+            o.embedding_wgrad(**args)
+    after()
+
+
 def test_error_codes_are_python_exceptions():
     o = ops()
     A = torch.randn(4, 3, 8, device="cuda")
