@@ -769,13 +769,14 @@ PyObject* py_pass_reduce(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (!PyList_Check(a[0]) || !PyList_Check(a[1])) invalid("pass_reduce takes two lists");
     std::map<int, std::vector<ghost_pass_job>> per_device;
     std::map<int, Tensor> any;               // a tensor of each device, for its stream
-    std::map<const float*, std::pair<int, size_t>> filled;
+    struct Filled { int device; size_t job; PyObject* vec; };
+    std::map<const float*, Filled> filled;
     for (Py_ssize_t i = 0; i < PyList_GET_SIZE(a[0]); ++i) {
       PyObject* d = PyList_GET_ITEM(a[0], i);
       int dev = 0;
       ghost_pass_job j = read_job(d, &dev);
       if (j.M == nullptr && j.sum_out == nullptr) invalid("small_reduce_batch: a job has no output");
-      if (j.M) filled[j.M] = {dev, per_device[dev].size()};
+      if (j.M) filled[j.M] = {dev, per_device[dev].size(), nullptr};
       per_device[dev].push_back(j);
       any.emplace(dev, cuda_tensor(item(d, k_X)));
     }
@@ -797,11 +798,20 @@ PyObject* py_pass_reduce(PyObject*, PyObject* const* a, Py_ssize_t n) {
         Tensor vecs = empty({e - i, first.size(1)}, first, at::kFloat);
         for (Py_ssize_t k = i; k < e; ++k) {
           const Tensor& t = cuda_tensor(PyList_GET_ITEM(a[1], k));
+          auto it = filled.find(t.data_ptr<float>());
+          if (it != filled.end() && it->second.vec != nullptr) {
+            // listed again: a job of its own would read the matrix while the first one writes it
+            Py_INCREF(it->second.vec);
+            PyList_SET_ITEM(out, k, it->second.vec);
+            continue;
+          }
           Tensor v = vecs.select(0, k - i);
           float* vp = v.data_ptr<float>();
-          auto it = filled.find(t.data_ptr<float>());
-          if (it != filled.end() && per_device[it->second.first][it->second.second].vec == nullptr) {
-            per_device[it->second.first][it->second.second].vec = vp;
+          PyObject* wrapped = wrap(v);
+          PyList_SET_ITEM(out, k, wrapped);
+          if (it != filled.end()) {
+            per_device[it->second.device][it->second.job].vec = vp;
+            it->second.vec = wrapped;
           } else {
             ghost_pass_job j = {};
             j.M = t.data_ptr<float>();
@@ -811,7 +821,6 @@ PyObject* py_pass_reduce(PyObject*, PyObject* const* a, Py_ssize_t n) {
             per_device[t.get_device()].push_back(j);
             any.emplace(t.get_device(), t);
           }
-          PyList_SET_ITEM(out, k, wrap(v));
         }
         i = e;
       }

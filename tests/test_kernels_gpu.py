@@ -852,6 +852,15 @@ def test_result_buffers_and_samples_are_checked_before_anything_is_written():
     after()
 
 
+def test_matrix_listed_twice_beside_the_job_that_fills_it():
+    X = torch.randn(37, 96, generator=torch.Generator().manual_seed(2)).cuda()
+    M, other = torch.empty(5, 32, device="cuda"), torch.randn(5, 32).cuda()
+    first, between, second = ops().pass_reduce([{"X": X, "n_train": 32, "n_val": 5, "M": M}], [M, other, M])
+    after()
+    assert torch.equal(first, second) and O.rel_fro(first, M.double().sum(0)) < 1e-6
+    assert O.rel_fro(between, other.double().sum(0)) < 1e-6
+
+
 def test_error_codes_are_python_exceptions():
     o = ops()
     A = torch.randn(4, 3, 8, device="cuda")
