@@ -124,7 +124,7 @@ extern "C" int ghost_conv_tokens_bf16(const void* src, int src_is_f32, long long
   const int Ho = (H + 2 * py - dy * (kh - 1) - 1) / sy + 1, Wo = (W + 2 * px - dx * (kw - 1) - 1) / sx + 1;
   GB_REQUIRE(H + 2 * py > dy * (kh - 1) && W + 2 * px > dx * (kw - 1), "ghost_conv_tokens_bf16: the window is larger than the padded input");
   const long long cols = static_cast<long long>(C) * kh * kw;
-  GB_REQUIRE(cols <= (1 << 22), "ghost_conv_tokens_bf16: too many features per token");
+  GB_REQUIRE(cols <= 64ll * 65535 && cpad <= 64 * 65535, "ghost_conv_tokens_bf16: too many features per token");
   GB_REQUIRE(static_cast<long long>(Ho) * Wo < (1ll << 31) - 64, "ghost_conv_tokens_bf16: too many output positions");
   GB_REQUIRE(parts >= 1 && parts <= 3, "ghost_conv_tokens_bf16: parts must be 1..3");
   GB_REQUIRE(cpad % 8 == 0 && cpad >= cols && ld_dst % 8 == 0 && ld_dst >= (row_stack ? cpad : parts * cpad) &&

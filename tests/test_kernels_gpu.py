@@ -861,6 +861,17 @@ def test_matrix_listed_twice_beside_the_job_that_fills_it():
     assert O.rel_fro(between, other.double().sum(0)) < 1e-6
 
 
+def test_conv_tokens_refuses_what_its_grid_cannot_hold():
+    from ghostsuite_b200 import _lib
+    lib = _lib.load()
+    src, dst = torch.zeros(64, device="cuda"), torch.zeros(64, dtype=torch.bfloat16, device="cuda")
+    for cols, cpad in ((64 * 65535 + 8, 64 * 65535 + 8), (8, 64 * 65535 + 8)):
+        rc = lib.ghost_conv_tokens_bf16(src.data_ptr(), 1, 1, cols, 1, 1, 1, 1, 1, 1, 0, 0, 1, 1, dst.data_ptr(), cpad, cpad, 1,
+                                        0, 0, 0, 0, torch.cuda.current_stream().cuda_stream)
+        assert rc == _lib.GHOST_ERR_INVALID
+    after()
+
+
 def test_error_codes_are_python_exceptions():
     o = ops()
     A = torch.randn(4, 3, 8, device="cuda")
