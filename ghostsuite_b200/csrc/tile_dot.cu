@@ -145,6 +145,7 @@ tile_dot_f32_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_const
         int ok = 1;
         if (lane == 0) ok = mbar_wait(&full_bar[stage], phase, abort_flag, p.err, 132) ? 1 : 0;
         ok = __shfl_sync(0xffffffffu, ok, 0);
+        __syncwarp();                    // the shuffle carries the verdict; this orders the stage's bytes for all lanes
         if (!ok) { alive = false; break; }
         const uint8_t* vbuf = smem + stage * Cfg::kStageBytes + warp * (VR * 128);
         const uint8_t* wbuf = smem + stage * Cfg::kStageBytes + Cfg::kValBytes + warp * (TR * 128);
@@ -384,6 +385,7 @@ tile_dot_mma_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_const
         int ok = 1;
         if (lane == 0) ok = mbar_wait(&full_bar[stage], phase, abort_flag, p.err, 132) ? 1 : 0;
         ok = __shfl_sync(0xffffffffu, ok, 0);
+        __syncwarp();                    // the shuffle carries the verdict; this orders the stage's bytes for all lanes
         if (!ok) { alive = false; break; }
         const uint32_t st = smem_u32(smem + stage * Cfg::kStageBytes);
         uint32_t a[MT][KS][4];
