@@ -195,7 +195,7 @@ def persample_dot(X: torch.Tensor, Y: torch.Tensor, n_val: int, dot_scale: float
     if colsum_of not in _COLSUM_FLAG:
         raise ValueError("colsum_of must be None, 'X' or 'Y'")
     gdt = grad_dtype if grad_dtype is not None else (_BF16 if X.dtype is _BF16 else _F32)
-    if gdt is not _F32 and gdt is not _BF16:
+    if want_grad and gdt is not _F32 and gdt is not _BF16:
         raise ValueError(f"unsupported dtype {gdt}: the kernels take float32 and bfloat16")
     args = (X, Y, n_val, dot_scale, want_grad, grad_scale, gdt is _F32, _COLSUM_FLAG[colsum_of])
     if _timing is None:

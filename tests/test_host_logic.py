@@ -5,6 +5,7 @@ import inspect
 import io
 
 import numpy as np
+import pytest
 import torch
 from torch import nn
 
@@ -156,3 +157,13 @@ def test_preset_path_is_not_passed_over(monkeypatch):
     assert _hook_arguments(monkeypatch, ruled)["any_path"] is False
     monkeypatch.setattr(L, "PATH_RULE", "gram")
     assert _hook_arguments(monkeypatch, nn.Linear(8, 8))["any_path"] is False
+
+
+def test_type_of_an_unwanted_gradient_does_not_matter():
+    """``persample_dot`` without a gradient ignores ``grad_dtype``; here it gets as far as asking for CUDA tensors."""
+    X = torch.zeros(3, 2, 8)
+    for dtype in (torch.float16, torch.float64):
+        with pytest.raises(RuntimeError, match="CUDA"):
+            L.ops.persample_dot(X, X, 1, want_grad=False, grad_dtype=dtype)
+        with pytest.raises(ValueError, match="unsupported dtype"):
+            L.ops.persample_dot(X, X, 1, want_grad=True, grad_dtype=dtype)
