@@ -138,11 +138,9 @@ def named_parameters(module) -> list:
     cost more than what a step does with each parameter.  Walks the live tree, so later changes of
     the model count; without the binding (CPU-only use of the engines' bookkeeping) torch's own."""
     from torch.nn import Module
-    own = type(module)
-    if own.named_parameters is not Module.named_parameters or own.named_modules is not Module.named_modules \
-            or not os.path.exists(BINDING_PATH):
+    if type(module).named_parameters is not Module.named_parameters or not os.path.exists(BINDING_PATH):
         return list(module.named_parameters())
-    found = native().named_parameters(module)
+    found = native().named_parameters(module, Module.named_modules)
     return list(module.named_parameters()) if found is None else found
 
 

@@ -861,18 +861,33 @@ PyObject* py_matrix_sum(PyObject*, PyObject* const* a, Py_ssize_t n) {
   });
 }
 
-// (module) -> [(qualified name, parameter)] as module.named_parameters() gives them: every parameter once,
-// modules in depth-first order.  The engines walk the model three times a step.  False: a module keeps its
-// tables elsewhere than in its dictionary (scripted modules), and the caller asks torch.
-bool walk_parameters(PyObject* module, const std::string& prefix, std::set<PyObject*>& seen, PyObject* out) {
+// (module, torch.nn.Module.named_modules) -> [(qualified name, parameter)] as module.named_parameters() gives
+// them: every parameter once, modules in depth-first order.  The engines walk the model three times a
+// step.  False: a module keeps its tables elsewhere than in its dictionary (scripted modules) or lists its
+// modules in a way of its own, and the caller asks torch.
+struct Walk {
+  PyObject* named_modules;
+  std::set<PyObject*> seen;              // modules and parameters
+  std::set<PyTypeObject*> plain;         // module types with torch's own listing
+};
+bool walk_parameters(PyObject* module, const std::string& prefix, Walk& walk, PyObject* out) {
+  std::set<PyObject*>& seen = walk.seen;
   if (!seen.insert(module).second) return true;
+  if (walk.plain.find(Py_TYPE(module)) == walk.plain.end()) {
+    PyObject* listing = PyObject_GetAttrString(reinterpret_cast<PyObject*>(Py_TYPE(module)), "named_modules");
+    if (!listing) PyErr_Clear();
+    const bool own = listing != walk.named_modules;
+    Py_XDECREF(listing);
+    if (own) return false;
+    walk.plain.insert(Py_TYPE(module));
+  }
   PyObject* dict = PyObject_GetAttrString(module, "__dict__");
   if (!dict) { PyErr_Clear(); return false; }
   PyObject *key, *value;
   Py_ssize_t pos = 0;
   PyObject* params = PyDict_Check(dict) ? PyDict_GetItemString(dict, "_parameters") : nullptr;
   PyObject* modules = PyDict_Check(dict) ? PyDict_GetItemString(dict, "_modules") : nullptr;
-  bool ok = params && PyDict_Check(params) && modules && PyDict_Check(modules);
+  bool ok = params && PyDict_Check(params) && modules && PyDict_Check(modules) && !PyDict_GetItemString(dict, "named_modules");
   if (ok) {
     while (PyDict_Next(params, &pos, &key, &value)) {
       if (value == Py_None || !seen.insert(value).second) continue;
@@ -887,7 +902,7 @@ bool walk_parameters(PyObject* module, const std::string& prefix, std::set<PyObj
     while (ok && PyDict_Next(modules, &pos, &key, &value)) {
       if (value == Py_None) continue;
       const char* name = PyUnicode_AsUTF8(key);
-      ok = walk_parameters(value, prefix + (name ? name : "") + ".", seen, out);
+      ok = walk_parameters(value, prefix + (name ? name : "") + ".", walk, out);
     }
   }
   Py_DECREF(dict);
@@ -896,12 +911,12 @@ bool walk_parameters(PyObject* module, const std::string& prefix, std::set<PyObj
 
 PyObject* py_named_parameters(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return guarded([&]() -> PyObject* {
-    need(n, 1, "named_parameters");
+    need(n, 2, "named_parameters");
     PyObject* out = PyList_New(0);
     if (!out) throw std::bad_alloc();
-    std::set<PyObject*> seen;
+    Walk walk{a[1], {}, {}};
     try {
-      if (!walk_parameters(a[0], "", seen, out)) {
+      if (!walk_parameters(a[0], "", walk, out)) {
         Py_DECREF(out);
         Py_RETURN_NONE;
       }

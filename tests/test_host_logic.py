@@ -3,6 +3,7 @@ cost model, the flat projection file format."""
 import contextlib
 import inspect
 import io
+import os
 
 import numpy as np
 import pytest
@@ -167,3 +168,33 @@ def test_type_of_an_unwanted_gradient_does_not_matter():
             L.ops.persample_dot(X, X, 1, want_grad=False, grad_dtype=dtype)
         with pytest.raises(ValueError, match="unsupported dtype"):
             L.ops.persample_dot(X, X, 1, want_grad=True, grad_dtype=dtype)
+
+
+class _Listing(nn.Module):
+    """A wrapper that lists its modules under names of its own and leaves one out."""
+
+    def __init__(self):
+        super().__init__()
+        self.inner, self.hidden = nn.Linear(2, 2), nn.Linear(2, 2)
+
+    def named_modules(self, memo=None, prefix="", remove_duplicate=True):
+        yield prefix, self
+        yield prefix + ".renamed", self.inner
+
+
+def test_native_parameter_walk_agrees_with_torch():
+    from ghostsuite_b200 import _lib
+    if not os.path.exists(_lib.BINDING_PATH):
+        pytest.skip("the torch binding is not built")
+    tied = nn.Sequential(nn.Linear(2, 2), nn.Linear(2, 2), nn.LayerNorm(2))
+    tied[1].weight = tied[0].weight
+    shared = nn.Sequential(tied[0], nn.ModuleDict({"again": tied[0], "none": nn.Identity()}), nn.TransformerEncoderLayer(4, 2))
+    shared.register_parameter("absent", None)
+    for m in (tied, shared):                               # walked
+        found = _lib.native().named_parameters(m, nn.Module.named_modules)
+        assert [(n, id(p)) for n, p in found] == [(n, id(p)) for n, p in m.named_parameters()]
+    late = nn.Sequential(nn.Linear(2, 2))
+    late[0].named_modules = lambda *args, **kwargs: iter(())
+    for m in (_Listing(), nn.Sequential(nn.Linear(2, 2), _Listing()), late):          # torch's to list
+        assert _lib.native().named_parameters(m, nn.Module.named_modules) is None
+        assert [n for n, _ in _lib.named_parameters(m)] == [n for n, _ in m.named_parameters()]
