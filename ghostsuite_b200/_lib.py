@@ -116,6 +116,12 @@ def load() -> C.CDLL:
     return lib
 
 
+def binding_built_for(version: str, path: str = BINDING_PATH) -> bool:
+    """Whether the torch binding at ``path`` was compiled against this torch release's C++ headers."""
+    with open(path, "rb") as f:
+        return f"ghost_torch built for torch {version}\n".encode() in f.read()
+
+
 def native():
     """The torch binding (``_ghost_torch.so``), loaded once; raises RuntimeError when it is absent."""
     global _native
@@ -124,7 +130,10 @@ def native():
         if not os.path.exists(BINDING_PATH):
             raise RuntimeError(f"{BINDING_PATH} is missing: build it with `python -m ghostsuite_b200.build`. "
                                "There is no CPU or PyTorch fallback.")
-        import torch  # noqa: F401  (the binding resolves its torch symbols from the loaded libraries)
+        import torch  # (the binding resolves its torch symbols from the loaded libraries)
+        if not binding_built_for(torch.__version__):
+            raise RuntimeError(f"{BINDING_PATH} was built for another torch than {torch.__version__}: "
+                               "build it again with `python -m ghostsuite_b200.build`.")
         loader = importlib.machinery.ExtensionFileLoader("_ghost_torch", BINDING_PATH)
         module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_ghost_torch", loader))
         loader.exec_module(module)

@@ -4,10 +4,13 @@ from __future__ import annotations
 
 import importlib.util
 import os
+import re
 import shutil
 import subprocess
 import sys
 import sysconfig
+
+from ._lib import binding_built_for
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
@@ -33,17 +36,29 @@ def _stale(target: str, sources) -> bool:
     return any(os.path.getmtime(d) > t for d in deps)
 
 
-def _start_binding():
-    """Start compiling the torch binding; it needs the library's header only, so it runs beside nvcc."""
+def _torch():
+    """``(installation root, version)`` of torch, without importing it."""
     spec = importlib.util.find_spec("torch")
     if spec is None:
         raise RuntimeError("torch is not importable: its headers are needed for _ghost_torch.so")
     root = os.path.dirname(spec.origin)
+    with open(os.path.join(root, "version.py")) as f:
+        return root, re.search(r"__version__\s*=\s*['\"]([^'\"]+)", f.read()).group(1)
+
+
+def _binding_stale() -> bool:
+    return _stale(BINDING, [BINDING_SOURCE, HEADERS[-1]]) or not binding_built_for(_torch()[1], BINDING)
+
+
+def _start_binding():
+    """Start compiling the torch binding; it needs the library's header only, so it runs beside nvcc."""
+    root, version = _torch()
     cuda = os.path.dirname(os.path.dirname(_nvcc()))
     obj = os.path.join(HERE, "build", "torch_ops.o")
     include = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
                os.path.join(cuda, "include"), sysconfig.get_paths()["include"]]
-    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden", "-c", os.path.join(CSRC, BINDING_SOURCE), "-o", obj]
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden", f'-DGHOST_TORCH_VERSION="{version}"',
+           "-c", os.path.join(CSRC, BINDING_SOURCE), "-o", obj]
     cmd += [f"-I{d}" for d in include]
     link = ["g++", "-shared", obj, "-o", BINDING, f"-L{HERE}", "-l:libghost_b200.so", f"-L{os.path.join(root, 'lib')}",
             "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python", "-Wl,-rpath,$ORIGIN"]
@@ -54,7 +69,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
     """Compile every .cu under csrc/ for sm_100a and link libghost_b200.so next to this file, then the
     torch binding."""
     lib_stale = force or _stale(LIB, SOURCES + HEADERS)
-    binding_stale = lib_stale or _stale(BINDING, [BINDING_SOURCE, HEADERS[-1]])
+    binding_stale = lib_stale or _binding_stale()
     if not lib_stale and not binding_stale:
         return LIB
     os.makedirs(os.path.join(HERE, "build"), exist_ok=True)

@@ -954,6 +954,10 @@ PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_ghost_torch", nullptr, -1, kMeth
 
 }  // namespace
 
+// The torch release whose headers this was compiled against; looked for in the file before it is loaded.
+extern "C" __attribute__((visibility("default"), used)) const char ghost_torch_built_for[] =
+    "ghost_torch built for torch " GHOST_TORCH_VERSION "\n";
+
 PyMODINIT_FUNC PyInit__ghost_torch() {
   struct { PyObject** at; const char* name; } keys[] = {{&k_X, "X"}, {&k_M, "M"}, {&k_sum_out, "sum_out"}, {&k_n_train, "n_train"},
                                                         {&k_n_val, "n_val"}, {&k_dot_scale, "dot_scale"},

@@ -72,3 +72,19 @@ def test_small_dense_layers_are_bounded_by_the_rows_of_a_tile():
     for args in ((1, 16384, 8, 1, 64, 64), (1, 8192, 8, 1, 128, 10), (0, 256, 1, 16, 64, 64), (0, 2048, 1, 8, 128, 10),
                  (1, 2048, 1, 1, 1024, 128), (0, 1024, 1, 1, 64, 64), (1, 64, 1, 16, 64, 64)):
         assert fits(*args) == 0, args
+
+
+def test_binding_of_another_torch_is_stale(tmp_path, monkeypatch):
+    """The binding is compiled against torch's C++ headers: after an upgrade it is built again, not loaded."""
+    import shutil
+    import torch
+    from ghostsuite_b200 import _lib, build
+    build.build()
+    assert build._torch()[1] == torch.__version__
+    assert _lib.binding_built_for(torch.__version__) and not build._binding_stale()
+    other = tmp_path / "_ghost_torch.so"
+    shutil.copyfile(build.BINDING, other)
+    os.utime(other)
+    other.write_bytes(other.read_bytes().replace(b"built for torch " + torch.__version__.encode(), b"built for torch 0"))
+    monkeypatch.setattr(build, "BINDING", str(other))
+    assert build._binding_stale() and not _lib.binding_built_for(torch.__version__, str(other))
