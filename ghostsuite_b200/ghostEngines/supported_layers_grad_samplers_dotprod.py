@@ -66,20 +66,22 @@ def _token_count(A: torch.Tensor) -> int:
     return t
 
 
-def _fp32_path_seconds(n_t: int, n_v: int, T: int, d: int, p: int):
-    """``(per-sample path, Gram path)``: measured cost of a float32 layer of short samples, train gradient
-    included.  At these sizes the fixed launches, the padding of the tiles and the second conversion of
+def _fp32_path_seconds(n_t: int, n_v: int, T: int, rows: int, cols: int):
+    """``(per-sample path, Gram path)``: measured cost of a float32 layer of short samples with a weight of
+    ``rows x cols``, train gradient included.  At these sizes the fixed launches, the padding of the tiles and the second conversion of
     both operands (the Gram path lays them out once for the Grams and once for the gradient) decide;
     the rates alone chose the Gram path for 24 + 5 samples of 197 x (768 -> 1000), 171 us against 103.
 
     Only for ``T <= 256`` and ``2 T <= d + p``: the tensor cores' float32 accumulation leaves a relative error
     of about 1e-8 per contracted token in the per-sample products and 5e-9 per feature in the Grams (70
     shapes against 64 bits), so below that line the per-sample path is the more accurate one as well
-    (1.9e-6 against 8.7e-6 in the example)."""
-    tiles = -(-p // 128) * -(-d // 256)
+    (1.9e-6 against 8.7e-6 in the example).  For the same reason only a choice of the Gram path is looked at
+    again with this model."""
+    tiles = -(-rows // 128) * -(-cols // 256)
     tile_bytes = 131072.0 * tiles * (n_t + n_v)
     per = 28e-6 + tile_bytes * (1 / 3.0e12 + 1 / 5.0e12) + (-(-3 * T // 64) * 64) * tile_bytes / 2 / 0.9e15
-    gram = 60e-6 + 20e-9 * (d + p) + 6.0 * n_t * n_v * T * T * (d + p) / 0.45e15 + 6.0 * n_t * T * d * p / 0.9e15
+    gram = 60e-6 + 20e-9 * (rows + cols) + 6.0 * n_t * n_v * T * T * (rows + cols) / 0.45e15 \
+        + 6.0 * n_t * T * rows * cols / 0.9e15
     return per, gram
 
 
@@ -113,7 +115,8 @@ def _should_use_ghost_computation(layer: nn.Module, A: torch.Tensor, B: torch.Te
         per = (6.0 * (n_t + n_v) * T * d * p / _PERSAMPLE_FLOPS + float(n_v) * n_t * d * p / _DOT_PRODUCTS_PER_S
                + 8.0 * (n_t + n_v) * d * p / _TILE_BYTES_PER_S)
         if gram <= per and T <= 256 and 2 * T <= d + p:
-            per, gram = _fp32_path_seconds(n_t, n_v, T, d, p)
+            in_by_out = _HFConv1D is not None and isinstance(layer, _HFConv1D)
+            per, gram = _fp32_path_seconds(n_t, n_v, T, *((d, p) if in_by_out else (p, d)))
     else:
         vr = 8 if n_v <= 8 else (16 if n_v <= 16 else 32)
         passes = -(-n_v // vr) * -(-n_t // 32)

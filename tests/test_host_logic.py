@@ -198,3 +198,17 @@ def test_native_parameter_walk_agrees_with_torch():
     for m in (_Listing(), nn.Sequential(nn.Linear(2, 2), _Listing()), late):          # torch's to list
         assert _lib.native().named_parameters(m, nn.Module.named_modules) is None
         assert [n for n, _ in _lib.named_parameters(m)] == [n for n, _ in m.named_parameters()]
+
+
+def test_path_rule_goes_by_the_layout_of_the_weight():
+    """A Conv1D d -> p has the tiles of a Linear p -> d, and the same costs otherwise."""
+    from transformers.pytorch_utils import Conv1D
+    choices = set()
+    for n_t, n_v, T in ((64, 1, 32), (64, 1, 100), (24, 5, 60), (24, 5, 197)):
+        for d, p in ((300, 1000), (1000, 300), (100, 2000), (768, 768)):
+            conv = Conv1D(p, d)
+            L._should_use_ghost_computation(conv, torch.empty(n_t + n_v, T, d, device="meta"),
+                                            torch.empty(n_t + n_v, T, p, device="meta"), val_batch_size=n_v)
+            assert conv.use_ghost_computation is _decide(n_t, n_v, T, p, d, dtype=torch.float32), (n_t, n_v, T, d, p)
+            choices.add(conv.use_ghost_computation)
+    assert choices == {True, False}
