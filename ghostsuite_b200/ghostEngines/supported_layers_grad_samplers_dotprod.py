@@ -532,9 +532,10 @@ def _compute_embedding_dot_product(layer: nn.Embedding, A: torch.Tensor, B: torc
     """nn.Embedding: id-equality-masked Gram of the out-grad rows (reference :181-211)."""
     _check_batch(A, B, val_batch_size)
     own = layer.__dict__
-    if "_ghost_backprop_scale" in own and val_batch_size > 0 \
+    if "_ghost_backprop_scale" in own and val_batch_size > 0 and A.numel() < 2 ** 31 - 1 \
             and getattr(layer.weight, "initially_requires_grad", layer.weight.requires_grad):
-        # inside a backward hook: the train gradient is asked for next and needs the same buckets
+        # inside a backward hook: the train gradient is asked for next and needs the same buckets (whose
+        # token indices are 32-bit for the whole batch; on their own either half may have as many)
         M, grad = ops.embedding_hook(A, B, val_batch_size, layer.weight.shape[0], own["_ghost_backprop_scale"])
         own["_ghost_cached_train_grad"] = (A.data_ptr(), B.data_ptr(), A.size(0), grad)
         _set_dot(layer.weight, M)

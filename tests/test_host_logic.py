@@ -212,3 +212,20 @@ def test_path_rule_goes_by_the_layout_of_the_weight():
             assert conv.use_ghost_computation is _decide(n_t, n_v, T, p, d, dtype=torch.float32), (n_t, n_v, T, d, p)
             choices.add(conv.use_ghost_computation)
     assert choices == {True, False}
+
+
+def test_embedding_batch_beyond_one_set_of_buckets(monkeypatch):
+    """Train and validation tokens that only together pass 31 bits go through the two separate calls."""
+    calls = []
+    monkeypatch.setattr(L.ops, "embedding_hook", lambda ids, G, n_val, *a: calls.append("hook") or (torch.zeros(n_val, 3), torch.zeros(4, 8)))
+    monkeypatch.setattr(L.ops, "embedding_dot", lambda ids, G, n_val, *a: calls.append("dot") or torch.zeros(n_val, 3))
+    monkeypatch.setattr(L.ops, "embedding_wgrad", lambda *a: calls.append("wgrad") or torch.zeros(4, 8))
+    layer = nn.Embedding(4, 8)
+    layer._ghost_backprop_scale = 1.0
+    for T, want in ((2 ** 28, ["hook"]), (2 ** 29, ["dot", "wgrad"])):
+        calls.clear()
+        A = torch.zeros(1, dtype=torch.long).expand(4, T)
+        B = torch.zeros(1).expand(4, T, 8)
+        L._compute_embedding_dot_product(layer, A, B, 1)
+        L._compute_embedding_train_grad(layer, A, B, 1)
+        assert calls == want
