@@ -21,7 +21,7 @@ struct SmallDense {
   float* colsums;                       // [N, p]; null: not wanted
   // blocks [0, gram_blocks): pairs of sample groups; then wgrad_blocks tiles of 64 x 64; then column sums
   int sv, sb, groups_b, gram_blocks;    // samples of a group (validation, train)
-  int tiles_n, wgrad_blocks, col_blocks;
+  int tiles_n, wgrad_blocks;
 };
 
 __device__ __forceinline__ float sd_f32(float v) { return v; }
@@ -272,7 +272,6 @@ extern "C" int ghost_dense_small(const void* A, const void* B, int is_f32, int n
   GB_REQUIRE(gram + wgrad + col < (1ll << 31), "ghost_dense_small: too many blocks");
   q.gram_blocks = static_cast<int>(gram);
   q.wgrad_blocks = static_cast<int>(wgrad);
-  q.col_blocks = static_cast<int>(col);
   const uintptr_t align = is_f32 ? 15 : 7;
   const bool vec = d % 4 == 0 && p % 4 == 0 && (reinterpret_cast<uintptr_t>(A) & align) == 0 && (reinterpret_cast<uintptr_t>(B) & align) == 0;
   const unsigned grid = static_cast<unsigned>(gram + wgrad + col);

@@ -368,7 +368,7 @@ extern "C" int ghost_pass_reduce(const ghost_pass_job* jobs, int n_jobs, void* s
                "ghost_pass_reduce: job %d has separate validation rows without a valid layout", i);
   }
   // Kernel parameters are copied whole whatever the job count, so short lists take a small block.
-  // A few jobs are one layer called on its own; the largest block (28 KB of the 32 KB a launch
+  // A few jobs are one layer called on its own; the largest block (24 KB of the 32 KB a launch
   // takes) holds all parameters of a GPT-2-sized model.
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   constexpr int kLarge = 300;

@@ -78,7 +78,8 @@ struct TdF32Cfg {
 //
 // What bounds it: the stream and, on small layers, the latency of a handful of stages.  With a warp
 // per four train rows, which read all validation rows and met at two barriers per stage, the pass over 64 + 16
-// samples of 128 x 576 float32 took 39 us; it takes 14.7 us now (24 MB, L2-resident).
+// samples of 128 x 576 float32 took 39 us; it takes 14.7 us now (31 MB: three 256-column tiles
+// hold the 576 columns; L2-resident).
 template <int VR>
 __global__ void __launch_bounds__(288, 1)
 tile_dot_f32_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_w,

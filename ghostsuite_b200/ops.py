@@ -569,8 +569,9 @@ def gradproj_embedding(ids: torch.Tensor, G: torch.Tensor, P_o_prepared: torch.T
         return _native().gradproj_embedding(ids, G, P_o_prepared, P_i_t, k_o, k_i, scale, out)
 
 
-#: largest block (rows of either operand) the similarity kernel is used for; beyond it the operands
-#: would be re-read once per 16 x 16 output block and a library GEMM is the better tool
+#: largest block (rows of either operand) the similarity kernel is used for.  Beyond it a library GEMM
+#: takes bf16 operands faster (192 x 192 scores over 98304 elements: 28 us against 69) and float32 ones
+#: more accurately (1.1e-6 off the 64-bit result against 4.4e-6; 486 us against 146)
 SIMILARITY_KERNEL_MAX_ROWS = 128
 
 
