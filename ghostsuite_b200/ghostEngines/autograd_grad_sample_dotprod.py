@@ -110,7 +110,10 @@ def register_hook_pair(layer: nn.Module, capture, backward_hook, slot: str):
             own[slot] = value if own.pop(due, False) else None
             backward_hook(layer, None, (grad,))
 
-        node.register_prehook(on_gradients)
+        if node is None:                 # a leaf handed through (a layer that returns its parameter)
+            out.register_hook(lambda grad: on_gradients((grad,)))
+        else:
+            node.register_prehook(on_gradients)
 
     return [layer.register_forward_hook(forward_hook)]
 

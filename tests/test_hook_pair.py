@@ -174,3 +174,18 @@ def test_two_pairs_on_one_layer():
     (h.layer(h.x) ** 2).sum().backward()
     h.check()
     assert torch.equal(other[0], h.x)
+
+
+def test_layer_that_returns_its_parameter():
+    class Table(nn.Linear):
+        def forward(self, x):
+            return self.weight
+
+    LAYERS["table"] = lambda: Table(4, 4)
+    try:
+        h = Hooked("table", "2d")
+    finally:
+        del LAYERS["table"]
+    (h.layer(h.x) * 3).sum().backward()
+    (A, g), = h.seen
+    assert torch.equal(A, h.x) and torch.equal(g, torch.full((4, 4), 3.0))
