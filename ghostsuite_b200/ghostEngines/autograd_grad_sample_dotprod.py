@@ -89,6 +89,9 @@ def register_hook_pair(layer: nn.Module, capture, backward_hook, slot: str):
     due = slot + "_due"
 
     def forward_hook(layer, inputs, outputs):
+        if torch._C._get_tracing_state() is not None:
+            # as torch says of full backward hooks: the trace would run on without them
+            raise ValueError(f"Modules that have backward hooks assigned can't be compiled: {layer}")
         capture(layer, inputs, outputs)
         out = outputs if torch.is_tensor(outputs) else next((o for o in outputs if torch.is_tensor(o)), None)
         if out is None or not out.requires_grad or not torch.is_grad_enabled():

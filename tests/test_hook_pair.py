@@ -189,3 +189,15 @@ def test_layer_that_returns_its_parameter():
     (h.layer(h.x) * 3).sum().backward()
     (A, g), = h.seen
     assert torch.equal(A, h.x) and torch.equal(g, torch.full((4, 4), 3.0))
+
+
+@every_layer
+def test_tracing_a_hooked_layer_is_refused(kind):
+    h = Hooked(kind, "3d")
+    with pytest.raises(ValueError, match="backward hooks"):
+        torch.jit.trace(nn.Sequential(h.layer), (h.x.detach(),))
+    (h.layer(h.x) ** 2).sum().backward()          # and it goes on as before
+    h.check()
+    for handle in h.handles:
+        handle.remove()
+    torch.jit.trace(nn.Sequential(h.layer), (h.x.detach(),))
