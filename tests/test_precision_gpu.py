@@ -107,3 +107,28 @@ def test_end_of_pass_gram(F):
     m = want.mean().item()
     one = 0.29 * BIAS / (m / 2.0 ** math.floor(math.log2(m)))
     assert rms < 1.25 * one * (2 + F / 256 / 3 / 256) ** 0.5
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("rms", [False, True])
+@pytest.mark.parametrize("N,T,F,splits", [(148, 1024, 1032, 2), (148, 1024, 731, 2), (148, 512, 4104, 1), (40, 160, 2048, 7)])
+def test_wide_norm_vectors(N, T, F, splits, rms, dtype):
+    """Sums over the tokens of terms of either sign: the partial sums grow with the root of their length, so n additions
+    in a row leave 2.45e-8 (0.29 ulp of a sum with an average mantissa) times the root of n / 2 of the
+    result.  32 rows in registers, the groups of a split, the splits; each term carries another eight
+    roundings (mean, variance, root, products).  Half on top."""
+    g = torch.Generator(device="cuda").manual_seed(9)
+    A, G = (torch.randn((N, T, F), generator=g, device="cuda").to(dtype) for _ in range(2))
+    got, _ = ops().layernorm_persample(A, G, 1e-5, rms=rms)
+    num = den = 0.0
+    for n in range(N):
+        x = A[n].double()
+        if not rms:
+            x = x - x.mean(-1, keepdim=True)
+        x = x * torch.rsqrt((x * x).mean(-1, keepdim=True) + 1e-5)
+        want = (G[n].double() * x).sum(0)
+        num += (got[n].double() - want).pow(2).sum().item()
+        den += want.pow(2).sum().item()
+    rows = T / splits
+    bound = 2.45e-8 * (min(rows, 32) / 2 + rows / 32 / 2 + splits / 2 + 8) ** 0.5
+    assert (num / den) ** 0.5 < 1.5 * bound
