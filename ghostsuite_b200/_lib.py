@@ -142,12 +142,17 @@ def native():
     return _native
 
 
+def binding_present() -> bool:
+    """Whether the torch binding is loaded or can be (CPU-only use of the engines' bookkeeping does without)."""
+    return _native is not None or os.path.exists(BINDING_PATH)
+
+
 def named_parameters(module) -> list:
     """``list(module.named_parameters())`` for a module on a GPU without its nested generators, which
     cost more than what a step does with each parameter.  Walks the live tree, so later changes of
     the model count; without the binding (CPU-only use of the engines' bookkeeping) torch's own."""
     from torch.nn import Module
-    if type(module).named_parameters is not Module.named_parameters or not os.path.exists(BINDING_PATH):
+    if type(module).named_parameters is not Module.named_parameters or not binding_present():
         return list(module.named_parameters())
     found = native().named_parameters(module, Module.named_modules)
     return list(module.named_parameters()) if found is None else found

@@ -10,7 +10,11 @@
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/function.h>
+#include <torch/csrc/autograd/function_hook.h>
 #include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/autograd/variable.h>
 
 #include <algorithm>
 #include <map>
@@ -928,6 +932,65 @@ PyObject* py_named_parameters(PyObject*, PyObject* const* a, Py_ssize_t n) {
   });
 }
 
+// ---- the gradient of a layer's output -----------------------------------------------------------------------
+// Calls fn(gradient in the output's shape, or None) before the node runs.
+class OutputHook : public torch::autograd::FunctionPreHook {
+ public:
+  OutputHook(PyObject* fn, size_t index, at::IntArrayRef shape) : fn_(fn), index_(index), shape_(shape.vec()) { Py_INCREF(fn_); }
+  ~OutputHook() override {
+    if (!Py_IsInitialized()) return;
+    const PyGILState_STATE gil = PyGILState_Ensure();
+    Py_DECREF(fn_);
+    PyGILState_Release(gil);
+  }
+  torch::autograd::variable_list operator()(const torch::autograd::variable_list& grads) override {
+    const PyGILState_STATE gil = PyGILState_Ensure();
+    try {
+      call(grads[index_]);
+    } catch (...) {
+      PyGILState_Release(gil);
+      throw;
+    }
+    PyGILState_Release(gil);
+    return grads;
+  }
+
+ private:
+  void call(const Tensor& grad) const {
+    PyObject* arg = !grad.defined() ? Py_NewRef(Py_None) : wrap(grad.sizes() == shape_ ? grad : grad.reshape(shape_));
+    PyObject* result = arg ? PyObject_CallOneArg(fn_, arg) : nullptr;
+    Py_XDECREF(arg);
+    if (!result) {
+      python_error error;
+      error.persist();
+      throw std::move(error);
+    }
+    Py_DECREF(result);
+  }
+  PyObject* fn_;
+  size_t index_;
+  std::vector<int64_t> shape_;
+};
+
+// (output, fn): hook the node that hands the output's gradient on.  Linear layers return a reshaped view of
+// their product; an in-place operation on a view gives it a new node and drops the old one with its hooks, so
+// there the base's node is taken.  False: no node has produced it.
+PyObject* py_hook_output(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    need(n, 2, "hook_output");
+    const Tensor& out = tensor(a[0]);
+    torch::autograd::Edge edge = torch::autograd::impl::gradient_edge(out);
+    if (out.is_view()) {
+      const Tensor base(out._base());
+      if (base.requires_grad() && base.grad_fn() && base.numel() == out.numel() && base.is_contiguous() && out.is_contiguous())
+        edge = torch::autograd::impl::gradient_edge(base);
+    }
+    if (!out.grad_fn()) Py_RETURN_FALSE;
+    edge.function->add_pre_hook(std::make_unique<OutputHook>(a[1], edge.input_nr, out.sizes()));
+    Py_RETURN_TRUE;
+  });
+}
+
 PyObject* py_set_kernel_error(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (n == 1) {
     Py_XDECREF(g_kernel_error);
@@ -948,6 +1011,7 @@ PyMethodDef kMethods[] = {
     GB_METHOD(dense_hook),        GB_METHOD(conv_hook),
     GB_METHOD(norm_hook),
     GB_METHOD(embedding_hook),    GB_METHOD(named_parameters),
+    GB_METHOD(hook_output),
     GB_METHOD(arena_clear),       GB_METHOD(set_kernel_error),
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_ghost_torch", nullptr, -1, kMethods, nullptr, nullptr, nullptr, nullptr};

@@ -13,12 +13,13 @@ kernels fold it into their epilogue scale.
 """
 from __future__ import annotations
 
+import weakref
 from typing import Tuple
 
 import torch
 import torch.nn as nn
 
-from .. import ops
+from .. import _lib, ops
 from . import supported_layers_grad_samplers_dotprod as _layers
 from .supported_layers_grad_samplers_dotprod import (
     _supported_layers_dotprod,
@@ -98,39 +99,49 @@ def register_hook_pair(layer: nn.Module, capture, backward_hook, slot: str):
             return
         own = layer.__dict__
         own[due] = True
-        # a list, emptied by the hook: a graph that outlives its backward pass keeps no input alive
-        kept = [own.get(slot)]
+        # The graph holds what follows, and the collector does not look into it: the layer is held weakly (it may
+        # hold the graph), and the input in a list that the hook empties (a graph may outlive its backward pass).
+        ref, kept = weakref.ref(layer), [own.get(slot)]
         if torch._C._current_graph_task_id() != -1:
             own.pop(slot, None)          # recomputed: no hook may follow that would clear it
-        node, index = _producing_node(out)
-        shape = out.shape
 
-        def on_gradients(grads):
-            grad = grads[index]
-            if grad is not None and grad.shape != shape:
-                grad = grad.reshape(shape)
-            value = kept.pop() if kept else None
+        def on_gradient(grad):
+            value, layer = kept.pop() if kept else None, ref()
+            if layer is None:
+                return
+            own = layer.__dict__
             own[slot] = value if own.pop(due, False) else None
             backward_hook(layer, None, (grad,))
 
-        if node is None:                 # a leaf handed through (a layer that returns its parameter)
-            out.register_hook(lambda grad: on_gradients((grad,)))
-        else:
-            node.register_prehook(on_gradients)
+        _hook_output(out, on_gradient)
 
     return [layer.register_forward_hook(forward_hook)]
 
 
-def _producing_node(out: torch.Tensor):
-    """``(node, output index)`` that hands on the gradient of ``out``.  Linear layers return a reshaped view
-    of their product; an in-place operation on a view gives it a new node and drops the old one with
-    its hooks, so there the base's node is taken."""
+def _hook_output(out: torch.Tensor, fn) -> None:
+    """``fn(gradient)`` when the node that hands on the gradient of ``out`` is about to run.  Linear layers return a
+    reshaped view of their product; an in-place operation on a view gives it a new node and drops the old
+    one with its hooks, so there the base's node is taken.  The native form of this saves 5 us of host
+    time per layer and step; the compiler traces the one here."""
+    if _lib.binding_present() and not torch.compiler.is_compiling():
+        if not _lib.native().hook_output(out, fn):
+            out.register_hook(fn)           # a leaf handed through (a layer that returns its parameter)
+        return
+    node, index, shape = out.grad_fn, out.output_nr, out.shape
     if out._is_view():
         base = out._base
         if base.requires_grad and base.grad_fn is not None and base.numel() == out.numel() \
                 and base.is_contiguous() and out.is_contiguous():
-            return base.grad_fn, base.output_nr
-    return out.grad_fn, out.output_nr
+            node, index = base.grad_fn, base.output_nr
+    if node is None:
+        out.register_hook(fn)
+        return
+
+    def on_gradients(grads):
+        grad = grads[index]
+        fn(grad if grad is None or grad.shape == shape else grad.reshape(shape))
+
+    node.register_prehook(on_gradients)
 
 
 def remove_hooks(model: nn.Module):

@@ -1,5 +1,8 @@
 """The pair of hooks that both engines put on a layer: which gradient and which input the backward hook
 gets.  Its product must be the weight gradient that autograd itself computes."""
+import gc
+import weakref
+
 import pytest
 import torch
 import torch.nn.functional as F
@@ -7,7 +10,18 @@ from torch import nn
 from torch.utils.checkpoint import checkpoint
 from transformers.pytorch_utils import Conv1D
 
+from ghostsuite_b200 import _lib
 from ghostsuite_b200.ghostEngines.autograd_grad_sample_dotprod import register_hook_pair
+
+
+@pytest.fixture(autouse=True, params=["native", "python"])
+def form(request, monkeypatch):
+    """The hook on the node in both its forms."""
+    if request.param == "python":
+        monkeypatch.setattr(_lib, "binding_present", lambda: False)
+    elif not _lib.binding_present():
+        pytest.skip("the torch binding is not built")
+
 
 LAYERS = {"linear": lambda: nn.Linear(4, 4), "linear_no_bias": lambda: nn.Linear(4, 4, bias=False),
           "conv1d": lambda: Conv1D(4, 4)}
@@ -201,3 +215,47 @@ def test_tracing_a_hooked_layer_is_refused(kind):
     for handle in h.handles:
         handle.remove()
     torch.jit.trace(nn.Sequential(h.layer), (h.x.detach(),))
+
+
+def test_exceptions_of_the_hook_reach_the_caller():
+    layer = nn.Linear(4, 4)
+
+    def fail(m, grad_input, grad_output):
+        raise KeyError("from the hook")
+
+    register_hook_pair(layer, Hooked.capture, fail, "kept")
+    with pytest.raises(KeyError, match="from the hook"):
+        layer(torch.randn(3, 4, requires_grad=True)).sum().backward()
+
+
+def test_compiled_model():
+    h = Hooked("linear", "3d")
+    torch._dynamo.reset()
+    (torch.compile(nn.Sequential(h.layer, nn.Tanh()), backend="eager")(h.x) ** 2).sum().backward()
+    h.check()
+
+
+@pytest.mark.parametrize("backward", [False, True])
+def test_a_layer_that_holds_its_output_is_collected(backward):
+    """The hook sits in the graph, the graph on the output, the output on the layer."""
+    seen = []
+    layer = nn.Linear(4, 4)
+    register_hook_pair(layer, Hooked.capture, lambda m, grad_input, grad: seen.append(m.__dict__.pop("kept").shape), "kept")
+    layer.seen_output = layer(torch.randn(3, 2, 4))
+    if backward:
+        layer.seen_output.sum().backward()
+        assert seen == [(3, 2, 4)]
+    gone = weakref.ref(layer)
+    del layer
+    gc.collect()
+    assert gone() is None
+
+
+def test_a_graph_that_outlives_its_backward_pass_keeps_no_input():
+    h = Hooked("linear", "3d")
+    loss = (h.layer(h.x * 2) ** 2).sum()
+    kept = weakref.ref(h.layer.__dict__["kept"])
+    loss.backward()
+    h.seen.clear()
+    gc.collect()
+    assert kept() is None and loss.grad_fn is not None
