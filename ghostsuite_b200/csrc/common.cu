@@ -137,7 +137,7 @@ int make_tmap_plain_2d(CUtensorMap* out, const void* base, int elem_bytes, uint6
   return GHOST_OK;
 }
 
-int make_tmap_bf16_store_2d(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows) {
+static int make_tmap_store_2d(CUtensorMap* out, const void* base, int elem_bytes, uint64_t rows, uint64_t cols, uint32_t box_rows) {
   EncodeTiledFn fn = encode_fn();
   if (!fn) return fail(GHOST_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
   if ((reinterpret_cast<uintptr_t>(base) & 15u) != 0 || cols % 32 != 0)
@@ -146,15 +146,23 @@ int make_tmap_bf16_store_2d(CUtensorMap* out, const void* base, uint64_t rows, u
   if (rows == 0 || rows >= (1ull << 32) || box_rows == 0 || box_rows > 256)
     return fail(GHOST_ERR_INVALID, "bad TMA store map (rows=%llu box_rows=%u)", (unsigned long long)rows, box_rows);
   cuuint64_t dims[2] = {cols, rows};
-  cuuint64_t strides[1] = {cols * 2};
+  cuuint64_t strides[1] = {cols * elem_bytes};
   cuuint32_t box[2] = {32, box_rows};
   cuuint32_t estr[2] = {1, 1};
-  CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+  CUresult r = fn(out, elem_bytes == 2 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(base),
+                  dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                  elem_bytes == 2 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS)
     return fail(GHOST_ERR_CUDA, "cuTensorMapEncodeTiled(store) failed with CUresult %d", (int)r);
   return GHOST_OK;
+}
+
+int make_tmap_bf16_store_2d(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows) {
+  return make_tmap_store_2d(out, base, 2, rows, cols, box_rows);
+}
+int make_tmap_f32_store_2d(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows) {
+  return make_tmap_store_2d(out, base, 4, rows, cols, box_rows);
 }
 
 int make_tmap_f32_tiles(CUtensorMap* out, const void* base, uint64_t tiles, uint64_t samples, uint32_t box_rows) {
@@ -222,6 +230,25 @@ int make_tmap_bf16_blocks(CUtensorMap* out, const void* base, uint64_t samples, 
                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS)
     return fail(GHOST_ERR_CUDA, "cuTensorMapEncodeTiled(blocked 4d) failed with CUresult %d", (int)r);
+  return GHOST_OK;
+}
+
+int make_tmap_bf16_parts(CUtensorMap* out, const void* base, uint64_t samples, uint64_t rows, uint64_t cols,
+                         uint32_t box_rows, uint32_t box_blocks) {
+  EncodeTiledFn fn = encode_fn();
+  if (!fn) return fail(GHOST_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
+  if ((reinterpret_cast<uintptr_t>(base) & 15u) != 0)
+    return fail(GHOST_ERR_INVALID, "TMA operand base %p is not 16-byte aligned", base);
+  if (rows == 0 || cols == 0 || samples == 0 || cols % 64 != 0)
+    return fail(GHOST_ERR_INVALID, "split TMA operand needs a column count that is a multiple of 64");
+  cuuint64_t dims[5] = {64, rows, cols / 64, 2, samples};
+  cuuint64_t strides[4] = {cols * 2, 128, rows * cols * 2, 2 * rows * cols * 2};
+  cuuint32_t box[5] = {64, box_rows, box_blocks, 2, 1};
+  cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+  CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<void*>(base), dims, strides, box, estr,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return fail(GHOST_ERR_CUDA, "cuTensorMapEncodeTiled(split 5d) failed with CUresult %d", (int)r);
   return GHOST_OK;
 }
 

@@ -65,6 +65,12 @@ int make_tmap_bf16_3d(CUtensorMap* out, const void* base, uint64_t samples, uint
 int make_tmap_bf16_blocks(CUtensorMap* out, const void* base, uint64_t samples, uint64_t rows,
                           uint64_t cols, uint64_t ld, uint32_t box_rows, uint32_t box_blocks);
 
+// float32 operands as two bf16 parts (value and residual), [samples, 2, rows, cols] with cols a multiple of 64
+// (zero-padded): a box covers both parts of `box_blocks` adjacent 64-column blocks of `box_rows` rows, the
+// value panels first.  Rows past the end of a sample read as zero.  Coordinates: (0, row, block, 0, sample).
+int make_tmap_bf16_parts(CUtensorMap* out, const void* base, uint64_t samples, uint64_t rows, uint64_t cols,
+                         uint32_t box_rows, uint32_t box_blocks);
+
 // Validation tiles as an all-gather leaves them: [ranks][tiles][per_rank samples][32768] bf16, seen as
 // [64, per_rank, ranks, 512 panels, tiles]; a box holds `box_rows` consecutive validation samples
 // (global index = rank * per_rank + sample) of `box_blocks` panels, each panel a swizzled
@@ -80,6 +86,9 @@ int make_tmap_plain_2d(CUtensorMap* out, const void* base, int elem_bytes, uint6
 // rows) from shared memory written with the 64-byte swizzle: 16-byte chunk c of row r sits at
 // r * 64 + ((c ^ ((r >> 1) & 3)) * 16).
 int make_tmap_bf16_store_2d(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows);
+// The same for fp32: boxes of [box_rows, 32 columns] (128-byte rows) written with the 128-byte swizzle, chunk c of row r at
+// r * 128 + ((c ^ (r & 7)) * 16).
+int make_tmap_f32_store_2d(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows);
 // Per-sample fp32 tiles [tiles][samples][32768], seen as [tiles, 1024 panels, samples, 32]: a box holds
 // eight panels (256 elements) of `box_rows` samples, each panel a swizzled [box_rows][32] block.
 // Coordinates: (0, sample, panel, tile).

@@ -83,8 +83,8 @@ __global__ void __launch_bounds__(256) conv_tokens_kernel(const ConvTokens q) {
       hw[e] = *reinterpret_cast<const uint32_t*>(&hi);
       lw[e] = *reinterpret_cast<const uint32_t*>(&lo);
     }
-    const long long stride = q.row_stack ? q.T * q.ld_dst : q.cpad;
-    __nv_bfloat16* dst = q.dst + (q.row_stack ? n * q.parts * q.T + t : n * q.T + t) * q.ld_dst + f0 + fl;
+    const long long stride = q.row_stack == 2 ? gridDim.z * q.T * q.ld_dst : q.row_stack ? q.T * q.ld_dst : q.cpad;
+    __nv_bfloat16* dst = q.dst + (q.row_stack == 1 ? n * q.parts * q.T + t : n * q.T + t) * q.ld_dst + f0 + fl;
 #pragma unroll
     for (int part = 0; part < 3; ++part) {
       if (part >= q.parts) break;

@@ -177,6 +177,7 @@ PyObject* py_arena_clear(PyObject*, PyObject* const*, Py_ssize_t) {
 constexpr int kSplitLeft[3] = {0, 1, 0};
 constexpr int kSplitRight[3] = {0, 0, 1};
 constexpr int kPlain[3] = {0, 0, 0};
+enum { kSideBySide = 0, kStackRows = 1, kStackBatch = 2 };     // where the parts of a copy lie (kStackBatch: convolutions)
 
 // An operand [N, T, cols] of the layer math: a tensor with exactly these dimensions, or a convolution
 // operand [N, C, H, W] whose tokens are the output positions.
@@ -193,10 +194,10 @@ struct Operand {
   bool ready() const { return conv == nullptr && tma_ready(t); }
   // bf16 copy of samples [first, first + samples)
   void cast(long long first, long long samples, void* dst, long long ld_dst, long long cpad, int parts, const int (&kinds)[3],
-            bool row_stack, void* st) const {
+            int stack, void* st) const {
     const long long per = conv ? static_cast<long long>(conv->C) * conv->H * conv->W : T * cols;
     const char* p = static_cast<const char*>(t.data_ptr()) + first * per * t.element_size();
-    const int cp = static_cast<int>(cpad), stack = row_stack ? 1 : 0;
+    const int cp = static_cast<int>(cpad);
     if (conv)
       check(ghost_conv_tokens_bf16(p, f32(), samples, conv->C, conv->H, conv->W, conv->kh, conv->kw, conv->sy, conv->sx,
                                    conv->py, conv->px, conv->dy, conv->dx, dst, ld_dst, cp, parts, kinds[0], kinds[1],
@@ -240,13 +241,13 @@ Tensor gram_dot(const Launch& L, const Operand& A, const Operand& G, long long n
     const Operand& x = *xs[i];
     const long long cp = op[i].cp;
     if (op[i].kind == 2) {
-      x.cast(0, n_train, base + op[i].off_t, 3 * cp, cp, 3, kSplitLeft, false, L.st());
-      x.cast(n_train, n_val, base + op[i].off_v, 3 * cp, cp, 3, kSplitRight, false, L.st());
+      x.cast(0, n_train, base + op[i].off_t, 3 * cp, cp, 3, kSplitLeft, kSideBySide, L.st());
+      x.cast(n_train, n_val, base + op[i].off_v, 3 * cp, cp, 3, kSplitRight, kSideBySide, L.st());
       pt[i] = base + op[i].off_t;
       pv[i] = base + op[i].off_v;
       k[i] = 3 * cp;
     } else {
-      if (op[i].kind == 1) x.cast(0, N, base + op[i].off_t, cp, cp, 1, kPlain, false, L.st());
+      if (op[i].kind == 1) x.cast(0, N, base + op[i].off_t, cp, cp, 1, kPlain, kSideBySide, L.st());
       pt[i] = op[i].kind == 1 ? base + op[i].off_t : static_cast<const char*>(x.t.data_ptr());
       pv[i] = pt[i] + n_train * T * cp * 2;
       k[i] = cp;
@@ -269,28 +270,39 @@ PyObject* py_gram_dot(PyObject*, PyObject* const* a, Py_ssize_t n) {
 }
 
 // ---- token-contracted GEMMs --------------------------------------------------------------------------
+// Operands of the entry points that take one or two bf16 parts.  A float32 operand makes both two parts; otherwise
+// what is not readable as it is is copied with its rows padded.  `merged`: one sample holding all rows.
 struct XtyOperands {
   const Operand* x[2];
-  long long samples, T, cp[2], off[2] = {0, 0};
-  int kind[2];                      // 0 as it is, 1 padded copy, 2 split
-  bool split;
-  XtyOperands(Workspace& ws, const Operand& X, const Operand& Y, long long samples_) : samples(samples_), T(X.T) {
+  long long count, samples, T, ld[2], off[2] = {0, 0};      // samples that are read; samples and tokens of the layout
+  bool copy[2], split;
+  XtyOperands(Workspace& ws, const Operand& X, const Operand& Y, long long count_, bool merged)
+      : count(count_), samples(merged ? 1 : count_), T(merged ? count_ * X.T : X.T) {
     x[0] = &X;
     x[1] = &Y;
     split = X.f32() || Y.f32();
     for (int i = 0; i < 2; ++i) {
-      cp[i] = pad8(x[i]->cols);
-      kind[i] = split ? 2 : x[i]->ready() ? 0 : 1;
-      if (kind[i]) off[i] = ws.plan(samples * (split ? 3 : 1) * T * cp[i] * 2);
+      copy[i] = split || !x[i]->ready();
+      ld[i] = copy[i] ? (x[i]->cols + 63) / 64 * 64 : x[i]->cols;
+      if (copy[i]) off[i] = ws.plan(samples * parts() * T * ld[i] * 2);
     }
   }
-  const void* get(int i, char* base, void* st) const {
-    if (kind[i] == 0) return x[i]->t.data_ptr();
-    if (kind[i] == 1) x[i]->cast(0, samples, base + off[i], cp[i], cp[i], 1, kPlain, true, st);
-    else x[i]->cast(0, samples, base + off[i], cp[i], cp[i], 3, i == 0 ? kSplitLeft : kSplitRight, true, st);
-    return base + off[i];
+  int parts() const { return split ? 2 : 1; }
+  const void* where(int i, char* base) const { return copy[i] ? static_cast<const void*>(base + off[i]) : x[i]->t.data_ptr(); }
+  // Lays out what has to be copied, with the column sums of operand sums_of (1 or 2, both operands copied) on the way
+  void prepare(char* base, void* st, int sums_of = 0, float* sums = nullptr) const {
+    if (x[0]->conv || x[1]->conv) {
+      const int kinds[3] = {0, 1, 0};
+      for (int i = 0; i < 2; ++i)
+        if (copy[i]) x[i]->cast(0, count, base + off[i], ld[i], ld[i], parts(), kinds, samples == 1 ? kStackBatch : kStackRows, st);
+    } else if (copy[0] || copy[1]) {
+      auto src = [&](int i) { return copy[i] ? x[i]->t.data_ptr() : nullptr; };
+      auto dst = [&](int i) { return copy[i] ? base + off[i] : nullptr; };
+      check(ghost_split_operands(src(0), x[0]->f32(), static_cast<int>(x[0]->cols), src(1), x[1]->f32(), static_cast<int>(x[1]->cols),
+                                 parts(), samples, T, dst(0), dst(1), sums_of == 1 ? sums : nullptr,
+                                 sums_of == 2 ? sums : nullptr, st));
+    }
   }
-  long long tokens() const { return split ? 3 * T : T; }
 };
 
 // scale * sum over the first `samples` samples of X^T Y, into out
@@ -299,12 +311,11 @@ void wgrad(const Launch& L, const Operand& X, const Operand& Y, long long sample
   Workspace ws;
   const long long ws_bytes = ghost_wgrad_workspace_bytes(m, n);
   const long long off_ws = ws.plan(ws_bytes);
-  XtyOperands ops(ws, X, Y, samples);
+  XtyOperands ops(ws, X, Y, samples, true);
   char* base = ws.commit(L, X.t);
-  const void* xp = ops.get(0, base, L.st());
-  const void* yp = ops.get(1, base, L.st());
-  check(ghost_wgrad_bf16(xp, yp, samples * ops.tokens(), m, n, ops.cp[0], ops.cp[1], scale, accumulate ? 1 : 0,
-                         out.data_ptr(), is_f32(out), base + off_ws, ws_bytes, L.st()));
+  ops.prepare(base, L.st());
+  check(ghost_wgrad_parts(ops.where(0, base), ops.where(1, base), ops.parts(), ops.samples * ops.T, m, n, ops.ld[0], ops.ld[1], scale, accumulate ? 1 : 0,
+                          out.data_ptr(), is_f32(out), base + off_ws, ws_bytes, L.st()));
 }
 
 // (X, Y, scale, f32_out, out or None, accumulate)
@@ -327,7 +338,7 @@ PyObject* py_wgrad(PyObject*, PyObject* const* a, Py_ssize_t n) {
 struct PerSample { Tensor M, grad, colsums; };
 
 PerSample persample_dot(const Launch& L, const Operand& X, const Operand& Y, long long n_val, float dot_scale, bool want_grad,
-                        float grad_scale, at::ScalarType grad_dt, int colsum_of) {
+                        float grad_scale, at::ScalarType grad_dt, int colsum_of, int split_sums_of) {
   const long long N = X.N, T = X.T, n_train = N - n_val;
   const int m = static_cast<int>(X.cols), n = static_cast<int>(Y.cols);
   check_split(n_train, n_val, "persample_dot");
@@ -336,18 +347,22 @@ PerSample persample_dot(const Launch& L, const Operand& X, const Operand& Y, lon
   r.M = empty({n_val, n_train}, X.t, at::kFloat);
   if (want_grad) r.grad = empty({m, n}, X.t, grad_dt);
   Workspace ws;
-  XtyOperands ops(ws, X, Y, N);
+  XtyOperands ops(ws, X, Y, N, false);
   const int f32 = ops.split ? 1 : 0;
   const long long ws_bytes = ghost_persample_workspace_bytes(static_cast<int>(n_train), static_cast<int>(n_val), m, n, f32);
   const long long off_ws = ws.plan(ws_bytes);
   char* base = ws.commit(L, X.t);
-  if (colsum_of && !ops.split) r.colsums = empty({N, colsum_of == 1 ? m : n}, X.t, at::kFloat);
-  const void* xp = ops.get(0, base, L.st());
-  const void* yp = ops.get(1, base, L.st());
-  check(ghost_persample_dot_bf16(xp, yp, static_cast<int>(n_train), static_cast<int>(n_val), ops.tokens(), m, n, ops.cp[0],
-                                 ops.cp[1], dot_scale, r.M.data_ptr<float>(), f32, want_grad ? r.grad.data_ptr() : nullptr,
-                                 want_grad ? is_f32(r.grad) : 0, grad_scale, 0, r.colsums.defined() ? colsum_of : 0,
-                                 r.colsums.defined() ? r.colsums.data_ptr<float>() : nullptr, base + off_ws, ws_bytes, L.st()));
+  // Column sums: of bf16 operands the GEMM pass takes them along (colsum_of), of float32 ones their conversion does
+  // (split_sums_of) unless a sample has too few rows for a block of it.
+  const int sums_of = !ops.split ? colsum_of : T >= 16 && !X.conv ? split_sums_of : 0;
+  if (sums_of) r.colsums = empty({N, ops.x[sums_of - 1]->cols}, X.t, at::kFloat);
+  float* sums = sums_of ? r.colsums.data_ptr<float>() : nullptr;
+  if (ops.split) ops.prepare(base, L.st(), sums_of, sums);
+  else ops.prepare(base, L.st());
+  check(ghost_persample_dot_parts(ops.where(0, base), ops.where(1, base), ops.parts(), static_cast<int>(n_train),
+                                  static_cast<int>(n_val), T, m, n, ops.ld[0], ops.ld[1], dot_scale, r.M.data_ptr<float>(),
+                                  want_grad ? r.grad.data_ptr() : nullptr, want_grad ? is_f32(r.grad) : 0, grad_scale, 0,
+                                  ops.split ? 0 : sums_of, ops.split ? nullptr : sums, base + off_ws, ws_bytes, L.st()));
   return r;
 }
 
@@ -359,7 +374,7 @@ PyObject* py_persample_dot(PyObject*, PyObject* const* a, Py_ssize_t n) {
     Launch L(X0);
     const Tensor X = as3d(X0), Y = as3d(Y0);
     PerSample r = persample_dot(L, Operand(X), Operand(Y), integer(a[2]), real(a[3]), integer(a[4]) != 0, real(a[5]),
-                                integer(a[6]) ? at::kFloat : at::kBFloat16, static_cast<int>(integer(a[7])));
+                                integer(a[6]) ? at::kFloat : at::kBFloat16, static_cast<int>(integer(a[7])), 0);
     return Py_BuildValue("(NNN)", wrap(r.M), wrap_or_none(r.grad), wrap_or_none(r.colsums));
   });
 }
@@ -423,9 +438,9 @@ Tensor optional_empty(at::IntArrayRef size, const Tensor& like, long long dt) {
 }
 
 // One of the two tensor-core paths, with the train gradient (dtype code gdt) and, where it costs nothing
-// extra, the column sums of B.
+// extra, the column sums of B for a layer with a bias (`fuse`: also those that a GEMM pass takes along).
 void dense_paths(const Launch& L, const Operand& A, const Operand& B, long long n_val, bool in_by_out, bool gram, long long gdt,
-                 float scale, bool want_sums, Tensor& M, Tensor& grad, Tensor& sums) {
+                 float scale, bool bias, bool fuse, Tensor& M, Tensor& grad, Tensor& sums) {
   const Operand &X = in_by_out ? A : B, &Y = in_by_out ? B : A;
   if (gram) {
     M = gram_dot(L, A, B, n_val, 0, 1.f);
@@ -433,7 +448,7 @@ void dense_paths(const Launch& L, const Operand& A, const Operand& B, long long 
     if (grad.defined()) wgrad(L, X, Y, A.N - n_val, scale, grad, false);
   } else {
     PerSample r = persample_dot(L, X, Y, n_val, 1.f, gdt >= 0, scale, gdt == 0 ? at::kBFloat16 : at::kFloat,
-                                !want_sums ? 0 : in_by_out ? 2 : 1);
+                                !fuse ? 0 : in_by_out ? 2 : 1, !bias ? 0 : in_by_out ? 2 : 1);
     M = r.M;
     grad = r.grad;
     sums = r.colsums;
@@ -470,7 +485,7 @@ PyObject* py_dense_hook(PyObject*, PyObject* const* a, Py_ssize_t n) {
                               A.size(1), dI, pI, in_by_out ? 1 : 0, M.data_ptr<float>(), grad.defined() ? grad.data_ptr() : nullptr,
                               grad.defined() ? is_f32(grad) : 0, scale, fuse ? sums.data_ptr<float>() : nullptr, L.st()));
     } else {
-      dense_paths(L, Operand(A), Operand(B), n_val, in_by_out, gram, gdt, scale, fuse, M, grad, sums);
+      dense_paths(L, Operand(A), Operand(B), n_val, in_by_out, gram, gdt, scale, bias, fuse, M, grad, sums);
     }
     if (bias && !sums.defined()) sums = colsum(L, B);
     Tensor Mb = bias ? empty({n_val, n_train}, A, at::kFloat) : Tensor();
@@ -501,7 +516,7 @@ PyObject* py_conv_hook(PyObject*, PyObject* const* a, Py_ssize_t n) {
     check_split(n_train, n_val, "conv_hook");
     const bool bias = integer(a[7]) != 0;
     Tensor M, grad, sums;
-    dense_paths(L, Operand(A, ca, T), Operand(B, cb, T), n_val, false, integer(a[4]) != 0, integer(a[5]), real(a[6]), false, M,
+    dense_paths(L, Operand(A, ca, T), Operand(B, cb, T), n_val, false, integer(a[4]) != 0, integer(a[5]), real(a[6]), false, false, M,
                 grad, sums);
     if (bias) {
       sums = empty({N, p}, A, at::kFloat);
@@ -637,8 +652,8 @@ PyObject* py_gradproj_dense(PyObject*, PyObject* const* a, Py_ssize_t n) {
     for (int i = 0; i < 2; ++i) {
       len[i] = split ? 3 * cp[i] : cp[i];
       p[i] = kind[i] ? static_cast<const void*>(base + off[i]) : x[i]->data_ptr();
-      if (kind[i] == 1) Operand(*x[i]).cast(0, B, base + off[i], cp[i], cp[i], 1, kPlain, false, L.st());
-      else if (kind[i] == 2) Operand(*x[i]).cast(0, B, base + off[i], 3 * cp[i], cp[i], 3, kSplitLeft, false, L.st());
+      if (kind[i] == 1) Operand(*x[i]).cast(0, B, base + off[i], cp[i], cp[i], 1, kPlain, kSideBySide, L.st());
+      else if (kind[i] == 2) Operand(*x[i]).cast(0, B, base + off[i], 3 * cp[i], cp[i], 3, kSplitLeft, kSideBySide, L.st());
     }
     if (P_r.size(1) != len[0] || P_c.size(1) != len[1])
       invalid("projection matrices were prepared for a different dtype/feature size");

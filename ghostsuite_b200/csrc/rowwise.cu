@@ -93,6 +93,130 @@ __global__ void cast_split_kernel(const CastParams p) {
   }
 }
 
+// Both operands of a token-contracted GEMM in one launch: rows zero-padded to ld (a multiple of 64) columns, as the
+// values alone (PARTS = 1) or as values and residuals, [samples, 2, T, ld].  A block takes a panel of 128 columns of
+// some rows, a thread eight columns of every 16th row, four rows in flight.  Where the column sums of an operand are
+// wanted the rows are one sample's (or a chunk of it, added with atomics), and they cost no second pass over it.
+// Bound by HBM and, on small layers, by the round trip of one round of loads: 8 x 2048 rows of (1024, 2048) float32 at
+// 5.5 TB/s, 29 x 197 of (768, 1000) 22.5 us from cold caches (two launches of cast_split_kernel with three parts
+// 17.4, and 8.5 for the sums in a pass of their own).
+static constexpr int kSplitCols = 128, kSplitLanes = 16;       // columns and row lanes of a block
+struct SplitJob {
+  const void* src;
+  __nv_bfloat16* dst;
+  float* sums;             // [samples, cols] or null
+  int is_f32, cols, ld, panels;
+  int vec;                 // rows on 16-byte boundaries
+  long long rows, per;     // all rows; rows of a block
+  int chunks;              // blocks that share a sample (sums only)
+  long long blocks;
+};
+struct SplitParams {
+  SplitJob job[2];
+  long long T;
+};
+
+template <typename E, int PARTS, bool VEC>
+__device__ __forceinline__ void split_rows(const SplitJob& j, long long T, long long r0, long long r1, int c0, float (&sum)[8]) {
+  const E* src = static_cast<const E*>(j.src) + c0;
+  const bool inside = c0 + 8 <= j.cols;
+  // sample s of two parts of T rows: row + s * T.  The sample of this thread's first row, then step by step.
+  long long sample = 0, end = T;
+  const long long first = r0 + (threadIdx.x / (kSplitCols / 8));
+  if (PARTS == 2) {
+    sample = j.rows < (1ll << 32) ? static_cast<unsigned>(first) / static_cast<unsigned>(T) : first / T;
+    end = (sample + 1) * T;
+  }
+  float part[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};      // of up to eight rounds: short chains
+  int rounds = 0;
+  for (long long row = first; row < r1; row += 4 * kSplitLanes) {
+    float x[4][8];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) x[q][e] = 0.f;
+      const E* p = src + (row + kSplitLanes * q) * j.cols;
+      if (row + kSplitLanes * q < r1) {
+        if (VEC && inside) {
+          Vec8<E>::load(p, x[q]);
+        } else {
+#pragma unroll
+          for (int e = 0; e < 8; ++e)
+            if (c0 + e < j.cols) x[q][e] = to_f32<E>(p[e]);
+        }
+      }
+    }
+#pragma unroll
+    for (int e = 0; e < 8; ++e) part[e] += (x[0][e] + x[1][e]) + (x[2][e] + x[3][e]);
+    if (++rounds % 8 == 0) {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) { sum[e] += part[e]; part[e] = 0.f; }
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const long long r = row + kSplitLanes * q;
+      if (r >= r1) break;
+      uint32_t hw[4], lw[4];             // the values as bf16, and what that leaves of them
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float a = x[q][2 * e], b = x[q][2 * e + 1];
+        const __nv_bfloat162 hi = __floats2bfloat162_rn(a, b);
+        const __nv_bfloat162 lo = __floats2bfloat162_rn(a - __bfloat162float(hi.x), b - __bfloat162float(hi.y));
+        hw[e] = *reinterpret_cast<const uint32_t*>(&hi);
+        lw[e] = *reinterpret_cast<const uint32_t*>(&lo);
+      }
+      long long at = r;
+      if (PARTS == 2) {
+        while (r >= end) { ++sample; end += T; }
+        at += sample * T;
+      }
+      __nv_bfloat16* dst = j.dst + at * j.ld + c0;
+      *reinterpret_cast<uint4*>(dst) = make_uint4(hw[0], hw[1], hw[2], hw[3]);
+      if (PARTS == 2) *reinterpret_cast<uint4*>(dst + T * j.ld) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
+    }
+  }
+#pragma unroll
+  for (int e = 0; e < 8; ++e) sum[e] += part[e];
+}
+
+template <int PARTS>
+__global__ void __launch_bounds__(256) split_pair_kernel(const SplitParams p) {
+  __shared__ float red[8][kSplitCols];
+  const bool second = blockIdx.x >= p.job[0].blocks;
+  const SplitJob& j = p.job[second ? 1 : 0];
+  const unsigned at = blockIdx.x - (second ? static_cast<unsigned>(p.job[0].blocks) : 0u);
+  const unsigned panel = at % j.panels, rest = at / j.panels;
+  const int oct = threadIdx.x % (kSplitCols / 8), c0 = static_cast<int>(panel) * kSplitCols + oct * 8;
+  long long sample = 0, r0 = rest * j.per, r1 = j.rows;
+  if (j.sums) {
+    sample = rest / j.chunks;
+    r0 = sample * p.T + rest % j.chunks * j.per;
+    r1 = (sample + 1) * p.T;
+  }
+  if (r0 + j.per < r1) r1 = r0 + j.per;
+  float sum[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  if (c0 < j.ld) {
+    if (j.is_f32 && j.vec) split_rows<float, PARTS, true>(j, p.T, r0, r1, c0, sum);
+    else if (j.is_f32) split_rows<float, PARTS, false>(j, p.T, r0, r1, c0, sum);
+    else if (j.vec) split_rows<__nv_bfloat16, PARTS, true>(j, p.T, r0, r1, c0, sum);
+    else split_rows<__nv_bfloat16, PARTS, false>(j, p.T, r0, r1, c0, sum);
+  }
+  if (!j.sums) return;
+#pragma unroll
+  for (int e = 0; e < 8; ++e) sum[e] += __shfl_xor_sync(0xffffffffu, sum[e], 16);
+  if ((threadIdx.x & 31) < 16)
+#pragma unroll
+    for (int e = 0; e < 8; ++e) red[threadIdx.x >> 5][oct * 8 + e] = sum[e];
+  __syncthreads();
+  const int t = threadIdx.x, c = static_cast<int>(panel) * kSplitCols + t;
+  if (t < kSplitCols && c < j.cols) {
+    const float v = ((red[0][t] + red[1][t]) + (red[2][t] + red[3][t])) + ((red[4][t] + red[5][t]) + (red[6][t] + red[7][t]));
+    float* out = j.sums + sample * j.cols + c;
+    if (j.chunks == 1) *out = v;
+    else atomicAdd(out, v);
+  }
+}
+
 // ------------------------------------------------------------------------------------------
 // per-sample column sums: out[n, c] += sum_{t in split} G[n, t, c]
 // ------------------------------------------------------------------------------------------
@@ -546,6 +670,53 @@ static int pick_splits(long long Tn, long long ctas_without_split, int sm_count,
   if (want < 1) want = 1;
   if (want > 65535) want = 65535;
   return static_cast<int>(want);
+}
+
+extern "C" int ghost_split_operands(const void* X, int x_is_f32, int x_cols, const void* Y, int y_is_f32, int y_cols, int parts,
+                                    long long samples, long long T, void* X_out, void* Y_out, float* x_sums, float* y_sums,
+                                    void* stream) {
+  const DeviceState* ds = device_state();
+  if (!ds) return GHOST_ERR_DEVICE;
+  GB_REQUIRE((X == nullptr) == (X_out == nullptr) && (Y == nullptr) == (Y_out == nullptr) && (X || Y), "ghost_split_operands: null pointer");
+  GB_REQUIRE((X || !x_sums) && (Y || !y_sums), "ghost_split_operands: sums of an operand that is not there");
+  GB_REQUIRE(samples > 0 && T > 0 && (!X || x_cols > 0) && (!Y || y_cols > 0), "ghost_split_operands: empty dimension");
+  GB_REQUIRE(parts == 1 || parts == 2, "ghost_split_operands: one or two parts");
+  GB_REQUIRE(((reinterpret_cast<uintptr_t>(X_out) | reinterpret_cast<uintptr_t>(Y_out)) & 15u) == 0,
+             "ghost_split_operands: destinations must be 16-byte aligned");
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  SplitParams p = {};
+  p.T = T;
+  auto fill = [&](SplitJob& j, const void* src, int f32, int cols, void* dst, float* sums) {
+    j.panels = 1;
+    if (!src) return;
+    j.src = src;
+    j.dst = static_cast<__nv_bfloat16*>(dst);
+    j.sums = sums;
+    j.is_f32 = f32;
+    j.cols = cols;
+    j.panels = ceil_div(cols, kSplitCols);
+    j.ld = (cols + 63) / 64 * 64;
+    j.rows = samples * T;
+    j.vec = cols % (f32 ? 4 : 8) == 0 && (reinterpret_cast<uintptr_t>(src) & 15u) == 0;
+    // 64 rows to a block (four a thread, one round of loads) while that is a few waves of blocks, more rows beyond it.
+    // Sums: a sample to a block and no atomics where that fills the GPU.
+    const long long units = sums ? T : j.rows, each = (sums ? samples : 1) * j.panels, wave = 6ll * ds->sm_count;
+    j.per = 4 * kSplitLanes;
+    if (sums && each >= wave) j.per = (units + 63) / 64 * 64;
+    while (j.per < units && (units + j.per - 1) / j.per * each > 8 * wave) j.per *= 2;
+    j.chunks = static_cast<int>((units + j.per - 1) / j.per);
+    j.blocks = j.chunks * each;
+  };
+  fill(p.job[0], X, x_is_f32, x_cols, X_out, x_sums);
+  fill(p.job[1], Y, y_is_f32, y_cols, Y_out, y_sums);
+  const long long blocks = p.job[0].blocks + p.job[1].blocks;
+  GB_REQUIRE(blocks < (1ll << 31), "ghost_split_operands: too many rows");
+  for (const SplitJob& j : p.job)
+    if (j.sums && j.chunks > 1) GB_CUDA_OK(cudaMemsetAsync(j.sums, 0, sizeof(float) * static_cast<size_t>(samples) * j.cols, st));
+  if (parts == 1) split_pair_kernel<1><<<static_cast<unsigned>(blocks), 256, 0, st>>>(p);
+  else split_pair_kernel<2><<<static_cast<unsigned>(blocks), 256, 0, st>>>(p);
+  count_launch();
+  return post_launch("split_pair_kernel");
 }
 
 extern "C" int ghost_colsum(const void* G, int is_f32, int N, long long T, int cols, long long ld,

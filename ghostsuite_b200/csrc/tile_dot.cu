@@ -65,7 +65,10 @@ struct TdF32Cfg {
   static constexpr int kPanels = kTdCols / 32;
   static constexpr int kValBytes = kPanels * VR * 128;
   static constexpr int kStageBytes = kValBytes + kPanels * kTdTrainRows * 128;   // 40 / 48 KB
-  static constexpr int kStages = 4;
+  // Eight validation rows leave registers for two CTAs per SM, of two stages each: with one CTA's eight warps the
+  // schedulers had two warps each to hide a stage's chain of loads, products and shuffles behind.
+  static constexpr int kCtas = VR == 8 ? 2 : 1;
+  static constexpr int kStages = 4 / kCtas;
   static constexpr int kRedBytes = 8 * kTdTrainRows * VR * 4;                    // per-warp partial dot blocks
   static constexpr int kSmemBytes = kStages * kStageBytes + kRedBytes + 1024 + 256;
 };
@@ -81,7 +84,7 @@ struct TdF32Cfg {
 // samples of 128 x 576 float32 took 39 us; it takes 14.7 us now (31 MB: three 256-column tiles
 // hold the 576 columns; L2-resident).
 template <int VR>
-__global__ void __launch_bounds__(288, 1)
+__global__ void __launch_bounds__(288, TdF32Cfg<VR>::kCtas)
 tile_dot_f32_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_w,
                     const TileDotParams p) {
   using Cfg = TdF32Cfg<VR>;
@@ -524,7 +527,7 @@ static int launch_tile_dot_f32(const void* V, int v_samples, const void* W, int 
     GB_CUDA_OK(cudaFuncSetAttribute(tile_dot_f32_kernel<VR>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes));
     attr_set[ds->device] = true;
   }
-  long long ctas = ds->sm_count;
+  long long ctas = static_cast<long long>(ds->sm_count) * Cfg::kCtas;
   if (ctas > p.stages) ctas = p.stages;
   p.stages_per_cta = (p.stages + ctas - 1) / ctas;
   ctas = (p.stages + p.stages_per_cta - 1) / p.stages_per_cta;

@@ -22,6 +22,7 @@
 #include "common.cuh"
 #include "sm100_ptx.cuh"
 #include "xty_colsum.cuh"
+#include "xty_operands.cuh"
 #include "xty_store.cuh"
 
 namespace gb {
@@ -44,25 +45,29 @@ struct XtyParams {
   // kEpiDirect: the result [m_cols, n_cols]; kEpiStoreTiles: tile-major [tile][sample][128][256]
   void* vgrad;
   int v_is_f32;
+  int tma_store;             // float32 tiles of two-part operands: stored by the copy engine
   float out_scale;           // kEpiDirect
   int out_accumulate, out_vec;
   int sample_major;          // unit order (sample, tile), dealt round-robin to the CTAs; needs k_splits == 1
-  // per-sample column sums of one operand (bias terms), taken by four extra warps that read the
-  // operand rows through L2: 0 = none, 1 = X, 2 = Y; out [all samples, cols of that operand] fp32
-  int colsum_of;
-  float* colsum_out;
-  const __nv_bfloat16* cs_src;   // that operand, [all samples, T, cols], row pitch cs_ld
+  // per-sample column sums of one operand (bias terms), taken by four extra warps that read the rows through L2
+  XtyColsum cs;
+  const __nv_bfloat16* cs_src;
   long long cs_ld;
+  float* zero;               // cleared for the kernel that follows (the matrix it adds into), or null
+  long long zero_n;
   int blocked_x, blocked_y;  // operand map is the blocked 4-D form: one TMA per stage instead of one per 64 columns
   int* err;
 };
 
+// PARTS = 2: operands in two bf16 parts, three products (see XtyPairCfg)
+template <int PARTS>
 struct XtyCfg {
-  static constexpr int BM = 128, BN = 256, BK = 64;
-  static constexpr int kStageBytes = (BM + BN) * BK * 2;   // 48 KB
+  static constexpr int BM = 128, BN = 256, BK = 64 / PARTS;
+  static constexpr int kStageBytes = (BM + BN) * BK * 2 * PARTS;   // 48 KB
   static constexpr int kStages = 4;
-  static constexpr int kColsumBytes = 8 * 128 * 4;          // reduction scratch of the column-sum warps
-  static constexpr int kSmemBytes = kStages * kStageBytes + 1024 + 256 + kColsumBytes;
+  static constexpr int kColsumBytes = PARTS == 1 ? 8 * 128 * 4 : 0;      // reduction scratch of the column-sum warps
+  static constexpr int kBoxBytes = PARTS * 4 * 32 * 32 * 4;  // store_grad_block32 (a box per epilogue warp), store_tile_f32
+  static constexpr int kSmemBytes = kStages * kStageBytes + 1024 + 256 + kColsumBytes + kBoxBytes;
 };
 
 // one 256-bit store (the address must be 32-byte aligned)
@@ -92,16 +97,17 @@ __device__ __forceinline__ void red_add_row32(float* dst, const uint32_t (&r)[32
   }
 }
 
-template <bool kColsum>
+template <bool kColsum, int PARTS>
 __global__ void __launch_bounds__(kColsum ? 320 : 192, 1)
 xty_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_y,
-                const XtyParams p) {
-  using Cfg = XtyCfg;
+                const __grid_constant__ CUtensorMap tm_out, const XtyParams p) {
+  using Cfg = XtyCfg<PARTS>;
   constexpr int BM = Cfg::BM, BN = Cfg::BN, BK = Cfg::BK, kStages = Cfg::kStages;
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kStages * Cfg::kStageBytes);
+  uint8_t* store_box = smem + kStages * Cfg::kStageBytes;      // 1024-byte aligned
+  uint64_t* bars = reinterpret_cast<uint64_t*>(store_box + Cfg::kBoxBytes);
   uint64_t* full_bar = bars;
   uint64_t* empty_bar = bars + kStages;
   uint64_t* acc_full = bars + 2 * kStages;     // [2]
@@ -136,6 +142,9 @@ xty_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant_
     *abort_flag = 0;
     fence_barrier_init();
   }
+  if (p.zero != nullptr)
+    for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < p.zero_n; i += gridDim.x * blockDim.x)
+      p.zero[i] = 0.f;
   if (warp == 5) {
     tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
@@ -190,14 +199,18 @@ xty_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant_
           const int z = p.sample0 + sample;
           // Every TMA instruction costs the issuing thread on the order of 100 cycles whatever its
           // size, and six of them per stage would take longer than the stage's MMAs.
-          if (p.blocked_x) {
+          if constexpr (PARTS == 2) {
+            tma_load_5d(st, &tm_x, &full_bar[stage], 0, row, m0 / 64, 0, z);
+          } else if (p.blocked_x) {
             tma_load_4d(st, &tm_x, &full_bar[stage], 0, row, m0 / 64, z);
           } else {
 #pragma unroll
             for (int j = 0; j < BM / 64; ++j)
               tma_load_3d(st + j * (BK * 128), &tm_x, &full_bar[stage], m0 + j * 64, row, z);
           }
-          if (p.blocked_y) {
+          if constexpr (PARTS == 2) {
+            tma_load_5d(st + BM * BK * 4, &tm_y, &full_bar[stage], 0, row, n0 / 64, 0, z);
+          } else if (p.blocked_y) {
             tma_load_4d(st + BM * BK * 2, &tm_y, &full_bar[stage], 0, row, n0 / 64, z);
           } else {
 #pragma unroll
@@ -228,11 +241,26 @@ xty_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant_
           const uint32_t sa = smem_u32(smem + stage * Cfg::kStageBytes);
           // MN-major: LBO = distance between 64-column slabs (one TMA box), SBO = 8 token rows
           const uint64_t adesc = make_smem_desc_sw128(sa, BK * 128, 1024);
-          const uint64_t bdesc = make_smem_desc_sw128(sa + BM * BK * 2, BK * 128, 1024);
+          const uint64_t bdesc = make_smem_desc_sw128(sa + BM * BK * 2 * PARTS, BK * 128, 1024);
+          auto step = [&](int k) {
+            const uint64_t a = adesc + k * (16 * 128 / 16), b = bdesc + k * (16 * 128 / 16);
+            const uint32_t add = (kb == kb0 && k == 0) ? 0u : 1u;
+            if constexpr (PARTS == 2) {      // residual parts lie behind the values
+              umma_bf16(dst, a + BM * BK * 2 / 16, b, idesc, add);
+              umma_bf16(dst, a, b + BN * BK * 2 / 16, idesc, 1u);
+              umma_bf16(dst, a, b, idesc, 1u);
+            } else {
+              umma_bf16(dst, a, b, idesc, add);
+            }
+          };
+          const long long left = p.T - static_cast<long long>(kb) * BK;
+          if (left >= BK) {
 #pragma unroll
-          for (int k = 0; k < BK / 16; ++k)
-            umma_bf16(dst, adesc + k * (16 * 128 / 16), bdesc + k * (16 * 128 / 16), idesc,
-                      (kb == kb0 && k == 0) ? 0u : 1u);
+            for (int k = 0; k < BK / 16; ++k) step(k);
+          } else {                        // steps past the last token hold zeros only
+#pragma unroll 1
+            for (int k = 0; k < (static_cast<int>(left) + 15) / 16; ++k) step(k);
+          }
           umma_commit(&empty_bar[stage]);
           if (++stage == kStages) { stage = 0; phase ^= 1; }
         }
@@ -242,39 +270,41 @@ xty_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant_
     }
   } else if (kColsum && warp >= 6) {
     // ---------------------------------------------------------------- column sums (warps 6-9)
-    // Every unit adds its share of the sample's token rows to the sums of its column block; see
-    // xty_colsum.cuh.
-    float* red = reinterpret_cast<float*>(smem + kStages * Cfg::kStageBytes + 1024 + 256);
+    // see xty_colsum.cuh
+    float* red = reinterpret_cast<float*>(smem + kStages * Cfg::kStageBytes + Cfg::kBoxBytes + 1024 + 256);
     const int ct = static_cast<int>(threadIdx.x) - 192;
-    const bool of_y = p.colsum_of == 2;
+    const bool of_y = p.cs.of == 2;
     const int total_cols = of_y ? p.n_cols : p.m_cols;
     for (long long u = u_begin; u < u_end; u += u_step) {
       int tile, sample, kb0, kb1;
       decode(u, tile, sample, kb0, kb1);
       const int tm = tile / p.n_tiles, tn = tile % p.n_tiles;
-      // the units that share this (sample, column block) split the sample's token rows among them
-      const int part = of_y ? tm : tn, parts = of_y ? p.m_tiles : p.n_tiles;
-      const long long per = ((p.T + parts - 1) / parts + 7) / 8 * 8;
-      const long long t0 = part * per;
-      const long long t1 = (t0 + per < p.T) ? t0 + per : p.T;
-      if (t0 >= t1) continue;
+      const int parts = of_y ? p.m_tiles : p.n_tiles;
+      const XtyRows rows = xty_colsum_rows(of_y ? tm : tn, parts, p.T);
+      if (rows.t0 >= rows.t1) continue;
       const long long s_idx = p.sample0 + sample;
+      float* out = p.cs.out + s_idx * total_cols;
       const int width = of_y ? BN : BM;
-      for (int half = 0; half < width; half += 128)
-        xty_colsum_128(p.cs_src + s_idx * p.T * p.cs_ld, t0, t1, p.cs_ld, (of_y ? tn * BN : tm * BM) + half, total_cols,
-                       red, p.colsum_out + s_idx * total_cols, ct, 1);
+      for (int half = 0; half < width; half += 128) {
+        xty_colsum_128(p.cs_src + s_idx * p.T * p.cs_ld, rows, parts == 1, p.cs_ld, (of_y ? tn * BN : tm * BM) + half, total_cols,
+                       red, out, ct, 1);
+      }
     }
   } else {
     // ---------------------------------------------------------------- epilogue
     int acc = 0;
     uint32_t acc_phase = 0;
+    uint32_t boxes = 0;          // boxes handed to the copy engine so far (selects the staging buffer)
     const uint32_t lane_base = static_cast<uint32_t>(warp * 32) << 16;
     for (long long u = u_begin; u < u_end; u += u_step) {
       int tile, sample, kb0, kb1;
       decode(u, tile, sample, kb0, kb1);
       const int m0 = (tile / p.n_tiles) * BM;
       const int n0 = (tile % p.n_tiles) * BN;
-      if (!mbar_wait_warp(&acc_full[acc], acc_phase, abort_flag, p.err, 114)) break;
+      bool ok = mbar_wait_warp(&acc_full[acc], acc_phase, abort_flag, p.err, 114);
+      // the staged store synchronises the four warps on a named barrier: they leave together
+      if (PARTS == 2 && p.tma_store) ok = named_bar_and(2, 128, ok);
+      if (!ok) break;
       tc_fence_after_sync();
       const int m = m0 + threadIdx.x;
       const bool m_ok = m < p.m_cols;
@@ -298,10 +328,16 @@ xty_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant_
           uint32_t r[32];
           tmem_ld32(t_acc + c0, r);
           tmem_ld_wait();
-          if (m_ok)
+          if (!p.out_vec)
+            store_grad_block32(p.vgrad, p.v_is_f32, p.out_accumulate, p.out_scale,
+                               static_cast<long long>(m0 + warp * 32) * p.n_cols + n0 + c0, p.n_cols, r, p.m_cols - (m0 + warp * 32),
+                               p.n_cols - (n0 + c0), reinterpret_cast<float*>(store_box) + warp * 1024);
+          else if (m_ok)
             store_grad_row32(p.vgrad, p.v_is_f32, p.out_accumulate, p.out_scale,
                              static_cast<long long>(m) * p.n_cols + n0 + c0, r, p.n_cols - (n0 + c0), p.out_vec != 0);
         }
+      } else if (PARTS == 2 && p.tma_store) {
+        store_tile_f32(&tm_out, store_box, t_acc, static_cast<int>((static_cast<long long>(tile) * p.samples + sample) * BM), boxes);
       } else {
         // kEpiStoreTiles: the whole 128 x 256 tile (zero padded), tile-major:
         //   dst[(tile * samples + sample)][row][col], one 512- or 1024-byte row per thread
@@ -344,6 +380,8 @@ xty_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant_
       if (lane == 0) mbar_arrive(&acc_empty[acc]);
       if (++acc == 2) { acc = 0; acc_phase ^= 1; }
     }
+    // the boxes still in flight are written out before the CTA gives up its shared memory
+    if (threadIdx.x == 0) bulk_wait_group<0>();
   }
 
   tc_fence_before_sync();
@@ -368,56 +406,54 @@ __global__ void xty_finalize_kernel(const float* __restrict__ ws, long long ld_w
   }
 }
 
-// CTA-pair variant of the tile-store pass (xty_gemm_pair.cu)
-int launch_xty_pair_tiles(const void* X, const void* Y, long long n_samples_total, long long T, int m_cols,
-                          int n_cols, long long ldx, long long ldy, int samples, int sample0, void* vgrad,
-                          int v_is_f32, int colsum_of, float* colsum_out, const DeviceState* ds, cudaStream_t st);
-int launch_xty_pair_wgrad(const void* X, const void* Y, long long n_rows, int m_cols, int n_cols, long long ldx,
-                          long long ldy, int splits, float* acc_ws, long long ld_acc, void* out, int out_is_f32,
-                          float scale, int accumulate, const DeviceState* ds, cudaStream_t st);
+// CTA-pair variant of both passes (xty_gemm_pair.cu)
+int launch_xty_pair_tiles(const XtyOperands& o, long long n_samples_total, long long T, int samples, int sample0, void* vgrad,
+                          int v_is_f32, const XtyColsum& cs, float* zero, long long zero_n, const DeviceState* ds, cudaStream_t st);
+int launch_xty_pair_wgrad(const XtyOperands& o, long long n_rows, int splits, float* acc_ws, long long ld_acc, void* out,
+                          int out_is_f32, float scale, int accumulate, const DeviceState* ds, cudaStream_t st);
 bool xty_pair_usable(const DeviceState* ds);
 static int g_wgrad_pair_mode = 1;      // same meaning as below
 static int g_persample_pair_mode = 1;  // 0 off, 1 where no half of a pair would idle, 2 wherever applicable
 
-// Operand maps: the blocked form (one TMA instruction per operand and stage) when the column count
-// is a multiple of 64, else one box per 64 columns with the tail zero-filled by the bounds check.
-static int make_xty_maps(CUtensorMap* tx, CUtensorMap* ty, XtyParams& p, const void* X, const void* Y,
-                         long long samples, long long rows, long long ldx, long long ldy) {
-  int rc;
-  p.blocked_x = (p.m_cols % 64 == 0) ? 1 : 0;
-  p.blocked_y = (p.n_cols % 64 == 0) ? 1 : 0;
-  rc = p.blocked_x ? make_tmap_bf16_blocks(tx, X, samples, rows, p.m_cols, ldx, XtyCfg::BK, XtyCfg::BM / 64)
-                   : make_tmap_bf16_3d(tx, X, samples, rows, p.m_cols, ldx, XtyCfg::BK);
-  if (rc != GHOST_OK) return rc;
-  return p.blocked_y ? make_tmap_bf16_blocks(ty, Y, samples, rows, p.n_cols, ldy, XtyCfg::BK, XtyCfg::BN / 64)
-                     : make_tmap_bf16_3d(ty, Y, samples, rows, p.n_cols, ldy, XtyCfg::BK);
-}
-
-static int launch_xty(const CUtensorMap& tx, const CUtensorMap& ty, XtyParams p,
-                      const DeviceState* ds, cudaStream_t st) {
+template <bool kColsum, int PARTS>
+static int launch_xty_t(const CUtensorMap& tx, const CUtensorMap& ty, const CUtensorMap& tout, const XtyParams& p, int grid, const DeviceState* ds, cudaStream_t st) {
   static bool attr_set[64] = {};
   if (!attr_set[ds->device]) {
-    GB_CUDA_OK(cudaFuncSetAttribute(xty_gemm_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    XtyCfg::kSmemBytes));
-    GB_CUDA_OK(cudaFuncSetAttribute(xty_gemm_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    XtyCfg::kSmemBytes));
+    GB_CUDA_OK(cudaFuncSetAttribute(xty_gemm_kernel<kColsum, PARTS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    XtyCfg<PARTS>::kSmemBytes));
     attr_set[ds->device] = true;
   }
+  xty_gemm_kernel<kColsum, PARTS><<<grid, kColsum ? 320 : 192, XtyCfg<PARTS>::kSmemBytes, st>>>(tx, ty, tout, p);
+  count_launch();
+  return post_launch("xty_gemm_kernel");
+}
+
+// rows: token rows of one of the `total` samples that the operands hold
+static int launch_xty(const XtyOperands& o, long long total, long long rows, XtyParams p, const DeviceState* ds, cudaStream_t st) {
+  CUtensorMap tx, ty;
+  int rc;
+  p.blocked_x = o.blocked(0) ? 1 : 0;
+  p.blocked_y = o.blocked(1) ? 1 : 0;
+  const int bk = o.parts == 2 ? XtyCfg<2>::BK : XtyCfg<1>::BK;
+  if ((rc = xty_operand_map(&tx, o, 0, total, rows, bk, XtyCfg<1>::BM / 64)) != GHOST_OK) return rc;
+  if ((rc = xty_operand_map(&ty, o, 1, total, rows, bk, XtyCfg<1>::BN / 64)) != GHOST_OK) return rc;
   const long long units = static_cast<long long>(p.m_tiles) * p.n_tiles * p.samples * p.k_splits;
   int grid = static_cast<int>(units < ds->sm_count ? units : ds->sm_count);
   p.units_per_cta = static_cast<int>((units + grid - 1) / grid);
   if (!p.sample_major) grid = static_cast<int>((units + p.units_per_cta - 1) / p.units_per_cta);
-  if (p.colsum_of != 0 && p.colsum_out != nullptr) {
-    // the column-sum warps add into the output: zero the rows of this launch's samples first
-    const int cs_cols = p.colsum_of == 2 ? p.n_cols : p.m_cols;
-    GB_CUDA_OK(cudaMemsetAsync(p.colsum_out + static_cast<long long>(p.sample0) * cs_cols, 0,
-                               sizeof(float) * static_cast<size_t>(p.samples) * cs_cols, st));
-    xty_gemm_kernel<true><<<grid, 320, XtyCfg::kSmemBytes, st>>>(tx, ty, p);
+  if ((rc = xty_colsum_clear(p.cs, p.cs.of == 1 ? p.n_tiles : p.m_tiles, p.sample0, p.samples, p.cs.of == 1 ? p.m_cols : p.n_cols, st)) !=
+      GHOST_OK)
+    return rc;
+  if (p.cs.of) {
+    p.cs_src = static_cast<const __nv_bfloat16*>(o.ptr[p.cs.of - 1]);
+    p.cs_ld = o.ld[p.cs.of - 1];
   }
-  else
-    xty_gemm_kernel<false><<<grid, 192, XtyCfg::kSmemBytes, st>>>(tx, ty, p);
-  count_launch();
-  return post_launch("xty_gemm_kernel");
+  CUtensorMap tout = tx;
+  const unsigned long long out_rows = static_cast<unsigned long long>(p.m_tiles) * p.n_tiles * p.samples * XtyCfg<1>::BM;
+  p.tma_store = o.parts == 2 && p.mode == kEpiStoreTiles && p.v_is_f32 && out_rows < (1ull << 31) ? 1 : 0;
+  if (p.tma_store && (rc = make_tmap_f32_store_2d(&tout, p.vgrad, out_rows, XtyCfg<1>::BN, XtyCfg<1>::BM)) != GHOST_OK) return rc;
+  if (o.parts == 2) return launch_xty_t<false, 2>(tx, ty, tout, p, grid, ds, st);
+  return p.cs.of ? launch_xty_t<true, 1>(tx, ty, tout, p, grid, ds, st) : launch_xty_t<false, 1>(tx, ty, tout, p, grid, ds, st);
 }
 
 int finalize_xty(const float* ws, long long ld_ws, void* out, int out_is_f32, int rows, int cols,
@@ -440,10 +476,19 @@ static inline long long round_up(long long x, long long m) { return (x + m - 1) 
 
 // a pair covers two 128-row tiles of X's columns: with an odd tile count the last pair's second CTA
 // idles, which costs more than the pair saves unless there are many tiles
-static bool pair_kernel_fits(int mode, int m_cols, int n_cols) {
-  if (mode == 0 || m_cols % 64 != 0 || n_cols % 64 != 0) return false;
-  const int m_tiles128 = (m_cols + 127) / 128;
-  return mode == 2 || m_tiles128 % 2 == 0 || m_tiles128 >= 15;
+static bool pair_kernel_fits(int mode, const XtyOperands& o, const DeviceState* ds) {
+  if (mode == 0 || !o.blocked(0) || !o.blocked(1)) return false;
+  const int m_tiles128 = (o.cols[0] + 127) / 128;
+  return (mode == 2 || m_tiles128 % 2 == 0 || m_tiles128 >= 15) && xty_pair_usable(ds);
+}
+
+static int check_parts(const void* X, const void* Y, int parts, int m_cols, int n_cols, long long ldx, long long ldy) {
+  GB_REQUIRE(parts == 1 || parts == 2, "split operands have one or two parts");
+  GB_REQUIRE(ldx % 8 == 0 && ldy % 8 == 0 && ldx >= m_cols && ldy >= n_cols, "operand pitch smaller than its rows or no multiple of 8");
+  GB_REQUIRE(parts == 1 || (ldx == round_up(m_cols, 64) && ldy == round_up(n_cols, 64)),
+             "operands in two parts have their rows padded to the next multiple of 64 columns");
+  GB_REQUIRE(((reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(Y)) & 15u) == 0, "operands must be 16-byte aligned");
+  return GHOST_OK;
 }
 
 extern "C" int ghost_set_wgrad_pair_mode(int mode) {
@@ -457,12 +502,12 @@ extern "C" long long ghost_wgrad_workspace_bytes(int m_cols, int n_cols) {
 }
 
 // D[m_cols, n_cols] = scale * sum_{rows < n_rows} X[row, :]^T Y[row, :]
-extern "C" int ghost_wgrad_bf16(const void* X, const void* Y, long long n_rows, int m_cols, int n_cols,
-                                long long ldx, long long ldy, float scale, int accumulate, void* out,
-                                int out_is_f32, void* ws, long long ws_bytes, void* stream) {
+static int wgrad(const XtyOperands& o, long long n_rows, float scale, int accumulate, void* out, int out_is_f32, void* ws,
+                 long long ws_bytes, void* stream) {
   const DeviceState* ds = device_state();
   if (!ds) return GHOST_ERR_DEVICE;
-  GB_REQUIRE(X && Y && out && ws, "ghost_wgrad_bf16: null pointer");
+  const int m_cols = o.cols[0], n_cols = o.cols[1];
+  GB_REQUIRE(o.ptr[0] && o.ptr[1] && out && ws, "ghost_wgrad_bf16: null pointer");
   GB_REQUIRE(n_rows > 0 && m_cols > 0 && n_cols > 0, "ghost_wgrad_bf16: empty dimension");
   GB_REQUIRE(n_rows < (1ll << 31) - 64, "ghost_wgrad_bf16: more than 2^31 token rows");
   GB_REQUIRE(ws_bytes >= ghost_wgrad_workspace_bytes(m_cols, n_cols), "ghost_wgrad_bf16: workspace too small");
@@ -471,12 +516,11 @@ extern "C" int ghost_wgrad_bf16(const void* X, const void* Y, long long n_rows, 
   p.mode = kEpiAccumulate;
   p.m_cols = m_cols;
   p.n_cols = n_cols;
-  p.m_tiles = ceil_div(m_cols, XtyCfg::BM);
-  p.n_tiles = ceil_div(n_cols, XtyCfg::BN);
+  p.m_tiles = ceil_div(m_cols, XtyCfg<1>::BM);
+  p.n_tiles = ceil_div(n_cols, XtyCfg<1>::BN);
   p.samples = 1;
-  p.sample0 = 0;
   p.T = n_rows;
-  const int kb = ceil_div(n_rows, XtyCfg::BK);
+  const int kb = ceil_div(n_rows, o.parts == 2 ? XtyCfg<2>::BK : XtyCfg<1>::BK);
   const int tiles = p.m_tiles * p.n_tiles;
   const double elems = static_cast<double>(m_cols) * n_cols;
   p.acc_ws = static_cast<float*>(ws);
@@ -487,25 +531,38 @@ extern "C" int ghost_wgrad_bf16(const void* X, const void* Y, long long n_rows, 
   p.out_accumulate = accumulate;
   p.out_vec = n_cols % 8 == 0 && (reinterpret_cast<uintptr_t>(out) & 15u) == 0;
   p.err = ds->err_word;
-  CUtensorMap tx, ty;
   int rc;
-  if ((rc = make_xty_maps(&tx, &ty, p, X, Y, 1, n_rows, ldx, ldy)) != GHOST_OK) return rc;
-  const bool pair = pair_kernel_fits(g_wgrad_pair_mode, m_cols, n_cols) && p.blocked_x && p.blocked_y && xty_pair_usable(ds);
-  const int splits = pair ? pick_k_splits(static_cast<long long>(ceil_div(m_cols, 256)) * p.n_tiles, ds->sm_count / 2,
-                                          ceil_div(n_rows, 128), 32, elems, out_is_f32 != 0)
+  const bool pair = pair_kernel_fits(g_wgrad_pair_mode, o, ds);
+  // in row blocks of the kernel; a block of two-part operands is half as many tokens and three products
+  const int kb_pair = ceil_div(n_rows, o.parts == 2 ? 64 : 128);
+  const int splits = pair ? pick_k_splits(static_cast<long long>(ceil_div(m_cols, 256)) * p.n_tiles, ds->sm_count / 2, kb_pair, 32,
+                                          elems, out_is_f32 != 0)
                           : pick_k_splits(tiles, ds->sm_count, kb, 64, elems, out_is_f32 != 0);
   if (splits > 1) GB_CUDA_OK(cudaMemsetAsync(ws, 0, static_cast<size_t>(m_cols) * p.ld_acc * 4, st));
   else p.mode = kEpiDirect;
   if (pair) {
-    rc = launch_xty_pair_wgrad(X, Y, n_rows, m_cols, n_cols, ldx, ldy, splits, p.acc_ws, p.ld_acc, out, out_is_f32, scale,
-                               accumulate, ds, st);
+    rc = launch_xty_pair_wgrad(o, n_rows, splits, p.acc_ws, p.ld_acc, out, out_is_f32, scale, accumulate, ds, st);
   } else {
     p.kb_per_split = ceil_div(kb, splits);
     p.k_splits = ceil_div(kb, p.kb_per_split);
-    rc = launch_xty(tx, ty, p, ds, st);
+    rc = launch_xty(o, 1, n_rows, p, ds, st);
   }
   if (rc != GHOST_OK || splits == 1) return rc;
   return finalize_xty(p.acc_ws, p.ld_acc, out, out_is_f32, m_cols, n_cols, scale, accumulate, st);
+}
+
+extern "C" int ghost_wgrad_bf16(const void* X, const void* Y, long long n_rows, int m_cols, int n_cols,
+                                long long ldx, long long ldy, float scale, int accumulate, void* out,
+                                int out_is_f32, void* ws, long long ws_bytes, void* stream) {
+  return wgrad(XtyOperands{{X, Y}, {m_cols, n_cols}, {ldx, ldy}, 1, false}, n_rows, scale, accumulate, out, out_is_f32, ws, ws_bytes, stream);
+}
+
+extern "C" int ghost_wgrad_parts(const void* X, const void* Y, int parts, long long n_rows, int m_cols, int n_cols, long long ldx,
+                                 long long ldy, float scale, int accumulate, void* out, int out_is_f32, void* ws,
+                                 long long ws_bytes, void* stream) {
+  const int rc = check_parts(X, Y, parts, m_cols, n_cols, ldx, ldy);
+  if (rc != GHOST_OK) return rc;
+  return wgrad(XtyOperands{{X, Y}, {m_cols, n_cols}, {ldx, ldy}, parts, true}, n_rows, scale, accumulate, out, out_is_f32, ws, ws_bytes, stream);
 }
 
 namespace gb {
@@ -538,7 +595,7 @@ extern "C" int ghost_set_persample_budget_bytes(long long bytes) {
 }
 
 extern "C" long long ghost_persample_workspace_bytes(int n_train, int n_val, int m_cols, int n_cols, int v_is_f32) {
-  const long long tiles = static_cast<long long>(ceil_div(m_cols, XtyCfg::BM)) * ceil_div(n_cols, XtyCfg::BN);
+  const long long tiles = static_cast<long long>(ceil_div(m_cols, XtyCfg<1>::BM)) * ceil_div(n_cols, XtyCfg<1>::BN);
   const int esize = v_is_f32 ? 4 : 2;
   const int g = persample_group(n_train, n_val, tiles, esize, kPersampleBudget);
   return tiles * kTileElems * 4 + (static_cast<long long>(n_val) + g) * tiles * kTileElems * esize + 512;
@@ -553,16 +610,14 @@ extern "C" int ghost_set_persample_pair_mode(int mode) {
 // Per-sample-gradient path.  X, Y: [n_train + n_val, T, cols] (train first).  Produces
 // M[v, b] = dot_scale * <X_v^T Y_v, X_b^T Y_b> and, if grad_out != null, the train gradient
 // grad_scale * sum_b X_b^T Y_b (written or accumulated, cast to the parameter dtype).
-extern "C" int ghost_persample_dot_bf16(const void* X, const void* Y, int n_train, int n_val, long long T,
-                                        int m_cols, int n_cols, long long ldx, long long ldy,
-                                        float dot_scale, float* M_out, int v_is_f32, void* grad_out,
-                                        int grad_is_f32, float grad_scale, int grad_accumulate,
-                                        int colsum_of, float* colsum_out,
-                                        void* ws, long long ws_bytes, void* stream) {
+static int persample_dot(const XtyOperands& o, int n_train, int n_val, long long T, float dot_scale, float* M_out, int v_is_f32,
+                         void* grad_out, int grad_is_f32, float grad_scale, int grad_accumulate, const XtyColsum& cs, void* ws,
+                         long long ws_bytes, void* stream) {
   const DeviceState* ds = device_state();
   if (!ds) return GHOST_ERR_DEVICE;
-  GB_REQUIRE(X && Y && M_out && ws, "ghost_persample_dot_bf16: null pointer");
-  GB_REQUIRE(colsum_of >= 0 && colsum_of <= 2 && (colsum_of == 0 || colsum_out != nullptr),
+  const int m_cols = o.cols[0], n_cols = o.cols[1];
+  GB_REQUIRE(o.ptr[0] && o.ptr[1] && M_out && ws, "ghost_persample_dot_bf16: null pointer");
+  GB_REQUIRE(cs.of >= 0 && cs.of <= 2 && (cs.of == 0 || (cs.out != nullptr && o.parts == 1)),
              "ghost_persample_dot_bf16: colsum_of must be 0, 1 (X) or 2 (Y) with an output buffer");
   GB_REQUIRE(n_train > 0, "No training samples to compute dot product, check batch sizes.");
   GB_REQUIRE(n_val > 0 && T > 0 && m_cols > 0 && n_cols > 0, "ghost_persample_dot_bf16: empty dimension");
@@ -576,36 +631,33 @@ extern "C" int ghost_persample_dot_bf16(const void* X, const void* Y, int n_trai
   p.mode = kEpiStoreTiles;
   p.m_cols = m_cols;
   p.n_cols = n_cols;
-  p.m_tiles = ceil_div(m_cols, XtyCfg::BM);
-  p.n_tiles = ceil_div(n_cols, XtyCfg::BN);
+  p.m_tiles = ceil_div(m_cols, XtyCfg<1>::BM);
+  p.n_tiles = ceil_div(n_cols, XtyCfg<1>::BN);
   p.T = T;
   p.k_splits = 1;
   p.sample_major = 1;
-  p.kb_per_split = ceil_div(T, XtyCfg::BK);
+  p.kb_per_split = ceil_div(T, o.parts == 2 ? XtyCfg<2>::BK : XtyCfg<1>::BK);
   p.v_is_f32 = v_is_f32;
-  p.colsum_of = colsum_of;
-  p.colsum_out = colsum_out;
-  p.cs_src = static_cast<const __nv_bfloat16*>(colsum_of == 1 ? X : Y);
-  p.cs_ld = (colsum_of == 1) ? ldx : ldy;
+  p.cs = cs;
   p.err = ds->err_word;
   const long long tiles = static_cast<long long>(p.m_tiles) * p.n_tiles;
   const int group = persample_group(n_train, n_val, tiles, esize, kPersampleBudget);
   float* sum = static_cast<float*>(ws);
   uint8_t* vws = static_cast<uint8_t*>(ws) + tiles * kTileElems * 4;
   uint8_t* wws = vws + static_cast<long long>(n_val) * tiles * kTileElems * esize;
-  CUtensorMap tx, ty;
   int rc;
   const long long N = static_cast<long long>(n_train) + n_val;
-  if ((rc = make_xty_maps(&tx, &ty, p, X, Y, N, T, ldx, ldy)) != GHOST_OK) return rc;
-  GB_CUDA_OK(cudaMemsetAsync(M_out, 0, sizeof(float) * static_cast<size_t>(n_val) * n_train, st));
+  // The first tile pass clears M, which the streaming pass adds into (a memset before it cost its launch and a gap).
+  const long long m_elems = static_cast<long long>(n_val) * n_train;
+  p.zero = M_out;
+  p.zero_n = m_elems;
   // tile pass: the CTA-pair kernel when it is selected and applicable, else the single-CTA kernel
-  const bool use_pair = pair_kernel_fits(g_persample_pair_mode, m_cols, n_cols) && p.blocked_x && p.blocked_y &&
-                        xty_pair_usable(ds);
-  auto tile_pass = [&](const XtyParams& q) -> int {
-    if (use_pair)
-      return launch_xty_pair_tiles(X, Y, N, T, m_cols, n_cols, ldx, ldy, q.samples, q.sample0, q.vgrad,
-                                   v_is_f32, colsum_of, colsum_out, ds, st);
-    return launch_xty(tx, ty, q, ds, st);
+  const bool use_pair = pair_kernel_fits(g_persample_pair_mode, o, ds);
+  auto tile_pass = [&](XtyParams& q) -> int {
+    const int status = use_pair ? launch_xty_pair_tiles(o, N, T, q.samples, q.sample0, q.vgrad, v_is_f32, cs, q.zero, q.zero_n, ds, st)
+                                : launch_xty(o, N, T, q, ds, st);
+    q.zero = nullptr;
+    return status;
   };
   if (group == n_train) {
     // everything fits: one GEMM pass over all samples (train first, validation last) into one
@@ -649,6 +701,28 @@ extern "C" int ghost_persample_dot_bf16(const void* X, const void* Y, int n_trai
   return GHOST_OK;
 }
 
+extern "C" int ghost_persample_dot_bf16(const void* X, const void* Y, int n_train, int n_val, long long T,
+                                        int m_cols, int n_cols, long long ldx, long long ldy,
+                                        float dot_scale, float* M_out, int v_is_f32, void* grad_out,
+                                        int grad_is_f32, float grad_scale, int grad_accumulate,
+                                        int colsum_of, float* colsum_out,
+                                        void* ws, long long ws_bytes, void* stream) {
+  const XtyColsum cs = {colsum_of, colsum_out};
+  return persample_dot(XtyOperands{{X, Y}, {m_cols, n_cols}, {ldx, ldy}, 1, false}, n_train, n_val, T, dot_scale, M_out, v_is_f32,
+                       grad_out, grad_is_f32, grad_scale, grad_accumulate, cs, ws, ws_bytes, stream);
+}
+
+extern "C" int ghost_persample_dot_parts(const void* X, const void* Y, int parts, int n_train, int n_val, long long T, int m_cols,
+                                         int n_cols, long long ldx, long long ldy, float dot_scale, float* M_out,
+                                         void* grad_out, int grad_is_f32, float grad_scale, int grad_accumulate, int colsum_of,
+                                         float* colsum_out, void* ws, long long ws_bytes, void* stream) {
+  const int rc = check_parts(X, Y, parts, m_cols, n_cols, ldx, ldy);
+  if (rc != GHOST_OK) return rc;
+  const XtyColsum cs = {colsum_of, colsum_out};
+  return persample_dot(XtyOperands{{X, Y}, {m_cols, n_cols}, {ldx, ldy}, parts, true}, n_train, n_val, T, dot_scale, M_out,
+                       parts == 2 ? 1 : 0, grad_out, grad_is_f32, grad_scale, grad_accumulate, cs, ws, ws_bytes, stream);
+}
+
 // ---- the two passes as separate calls ---------------------------------------------------------------
 // For callers that put something between the passes: a data-parallel run whose ranks each hold a
 // part of the validation batch computes its own validation tiles, all-gathers them, and only then
@@ -656,7 +730,7 @@ extern "C" int ghost_persample_dot_bf16(const void* X, const void* Y, int n_trai
 
 extern "C" long long ghost_persample_tiles_bytes(int samples, int m_cols, int n_cols) {
   if (samples <= 0 || m_cols <= 0 || n_cols <= 0) return 0;
-  const long long tiles = static_cast<long long>(ceil_div(m_cols, XtyCfg::BM)) * ceil_div(n_cols, XtyCfg::BN);
+  const long long tiles = static_cast<long long>(ceil_div(m_cols, XtyCfg<1>::BM)) * ceil_div(n_cols, XtyCfg<1>::BN);
   return tiles * samples * kTileElems * 2;
 }
 
@@ -680,28 +754,22 @@ extern "C" int ghost_persample_tiles_bf16(const void* X, const void* Y, int n_sa
   p.mode = kEpiStoreTiles;
   p.m_cols = m_cols;
   p.n_cols = n_cols;
-  p.m_tiles = ceil_div(m_cols, XtyCfg::BM);
-  p.n_tiles = ceil_div(n_cols, XtyCfg::BN);
+  p.m_tiles = ceil_div(m_cols, XtyCfg<1>::BM);
+  p.n_tiles = ceil_div(n_cols, XtyCfg<1>::BN);
   p.T = T;
   p.k_splits = 1;
   p.sample_major = 1;
-  p.kb_per_split = ceil_div(T, XtyCfg::BK);
+  p.kb_per_split = ceil_div(T, XtyCfg<1>::BK);
   p.v_is_f32 = 0;
-  p.colsum_of = colsum_of;
-  p.colsum_out = colsum_out;
-  p.cs_src = static_cast<const __nv_bfloat16*>(colsum_of == 1 ? X : Y);
-  p.cs_ld = (colsum_of == 1) ? ldx : ldy;
+  p.cs = XtyColsum{colsum_of, colsum_out};
   p.err = ds->err_word;
   p.samples = samples;
   p.sample0 = sample0;
   p.vgrad = tiles_out;
-  CUtensorMap tx, ty;
-  int rc;
-  if ((rc = make_xty_maps(&tx, &ty, p, X, Y, n_samples_total, T, ldx, ldy)) != GHOST_OK) return rc;
-  if (pair_kernel_fits(g_persample_pair_mode, m_cols, n_cols) && p.blocked_x && p.blocked_y && xty_pair_usable(ds))
-    return launch_xty_pair_tiles(X, Y, n_samples_total, T, m_cols, n_cols, ldx, ldy, samples, sample0, tiles_out, 0,
-                                 colsum_of, colsum_out, ds, st);
-  return launch_xty(tx, ty, p, ds, st);
+  const XtyOperands o = {{X, Y}, {m_cols, n_cols}, {ldx, ldy}, 1, false};
+  if (pair_kernel_fits(g_persample_pair_mode, o, ds))
+    return launch_xty_pair_tiles(o, n_samples_total, T, samples, sample0, tiles_out, 0, p.cs, nullptr, 0, ds, st);
+  return launch_xty(o, n_samples_total, T, p, ds, st);
 }
 
 extern "C" int ghost_tile_dot_bf16(const void* V, int v_ranks, int v_per_rank, const void* W, int n_train, int m_cols,
@@ -721,8 +789,8 @@ extern "C" int ghost_tile_dot_bf16(const void* V, int v_ranks, int v_per_rank, c
   GB_REQUIRE((reinterpret_cast<uintptr_t>(V) & 255u) == 0 && (reinterpret_cast<uintptr_t>(W) & 255u) == 0,
              "ghost_tile_dot_bf16: tile buffers must be 256-byte aligned");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const int n_tiles_n = ceil_div(n_cols, XtyCfg::BN);
-  const long long tiles = static_cast<long long>(ceil_div(m_cols, XtyCfg::BM)) * n_tiles_n;
+  const int n_tiles_n = ceil_div(n_cols, XtyCfg<1>::BN);
+  const long long tiles = static_cast<long long>(ceil_div(m_cols, XtyCfg<1>::BM)) * n_tiles_n;
   GB_CUDA_OK(cudaMemsetAsync(M_out, 0, sizeof(float) * static_cast<size_t>(n_val) * n_train, st));
   return launch_tile_dot(V, n_val, 0, W, n_train, 0, tiles, n_val, n_train, 0, n_train, dot_scale, M_out, nullptr, 1,
                          grad_out, grad_is_f32, grad_accumulate, m_cols, n_cols, n_tiles_n, grad_scale, ds, st,

@@ -28,6 +28,7 @@
 #include "common.cuh"
 #include "sm100_ptx.cuh"
 #include "xty_colsum.cuh"
+#include "xty_operands.cuh"
 #include "xty_store.cuh"
 
 namespace gb {
@@ -40,7 +41,7 @@ struct XtyPairParams {
   long long T;
   void* vgrad;
   int v_is_f32;
-  int tma_store;             // bf16 tiles: staged in shared memory and stored by the copy engine
+  int tma_store;             // tiles: staged in shared memory and stored by the copy engine
   int accumulate;            // 0: store tiles; 1: add into acc_ws ("samples" = k_splits, one real sample);
                              // 2: one split, stored to `out`
   void* out;                 // [m_cols, n_cols]
@@ -56,21 +57,30 @@ struct XtyPairParams {
   long long cs_ld;
   int cs_cols;
   float* cs_out;             // [n_samples_total, cs_cols] fp32
+  float* zero;               // cleared for the kernel that follows (the matrix it adds into), or null
+  long long zero_n;
   int* err;
 };
 
+// PARTS = 2: float32 operands as two bf16 parts each (make_tmap_bf16_parts), three products per token block --
+// residual x value, value x residual, value x value -- into the same accumulator.  Both parts of an operand are
+// fetched once and used twice; the same products over operands stacked three deep ([value; residual;
+// value] against [value; value; residual]) fetch six blocks for these four, and the kernel is bound by what
+// crosses the L2: 24 + 5 samples of 197 tokens, 768 x 1000, went from 45 us (single CTAs, tiles stored a row a lane) to
+// 35.6 with the copy engine storing the float32 tiles.
+template <int PARTS>
 struct XtyPairCfg {
   static constexpr int BM = 128;           // X columns per CTA
   static constexpr int BNH = 128;          // Y columns loaded per CTA (half of N = 256)
   static constexpr int BN = 256;
-  static constexpr int BK = 128;           // tokens per stage: eight MMAs per barrier round trip
-  static constexpr int kStageBytes = (BM + BNH) * BK * 2;   // 64 KB
+  static constexpr int BK = 128 / PARTS;   // tokens per stage: eight (twelve) MMAs per barrier round trip
+  static constexpr int kStageBytes = (BM + BNH) * BK * 2 * PARTS;   // 64 KB
   static constexpr int kStages = 3;
-  static constexpr int kColsumBytes = 8 * 128 * 4;          // cross-row-lane reduction of the column-sum warps
-  // bf16 tiles leave through shared memory: two [128 rows][32 columns] boxes (64-byte rows, 64-byte
-  // swizzle) that the epilogue warps fill alternately and one thread hands to the copy engine
-  static constexpr int kStoreBoxBytes = 128 * 32 * 2;
+  // tiles leave through shared memory: two [128 rows][32 columns] boxes (64- or 128-byte rows, swizzled)
+  // that the epilogue warps fill alternately and one thread hands to the copy engine
+  static constexpr int kStoreBoxBytes = 128 * 32 * 2 * PARTS;
   static constexpr int kStoreBytes = 2 * kStoreBoxBytes;
+  static constexpr int kColsumBytes = PARTS == 1 ? 8 * 128 * 4 : 0;      // cross-row-lane reduction of the column-sum warps
   static constexpr int kSmemBytes = kStages * kStageBytes + kStoreBytes + 1024 + 256 + kColsumBytes;
 };
 
@@ -94,10 +104,11 @@ __device__ __forceinline__ void red_add_row32_pair(float* dst, const uint32_t (&
   }
 }
 
+template <int PARTS>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(320, 1)
 xty_gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_y,
                      const __grid_constant__ CUtensorMap tm_out, const XtyPairParams p) {
-  using Cfg = XtyPairCfg;
+  using Cfg = XtyPairCfg<PARTS>;
   constexpr int BM = Cfg::BM, BN = Cfg::BN, BK = Cfg::BK, kStages = Cfg::kStages;
 
   extern __shared__ uint8_t smem_raw[];
@@ -151,6 +162,9 @@ xty_gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
     *abort_flag = 0;
     fence_barrier_init();
   }
+  if (p.zero != nullptr)
+    for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < p.zero_n; i += gridDim.x * blockDim.x)
+      p.zero[i] = 0.f;
   if (warp == 5) {
     tmem_alloc_pair(tmem_slot, 512);
     tmem_relinquish_pair();
@@ -186,8 +200,13 @@ xty_gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
           // the leader's barrier collects both CTAs' bytes
           if (leader) mbar_arrive_expect_tx(&full_bar[stage], 2 * Cfg::kStageBytes);
           const uint32_t bar = map_to_cta(smem_u32(&full_bar[stage]), 0);
-          tma_load_4d_pair(st, &tm_x, bar, 0, kb * BK, xblk, z);
-          tma_load_4d_pair(st + BM * BK * 2, &tm_y, bar, 0, kb * BK, yblk, z);
+          if constexpr (PARTS == 2) {
+            tma_load_5d_pair(st, &tm_x, bar, 0, kb * BK, xblk, 0, z);
+            tma_load_5d_pair(st + BM * BK * 4, &tm_y, bar, 0, kb * BK, yblk, 0, z);
+          } else {
+            tma_load_4d_pair(st, &tm_x, bar, 0, kb * BK, xblk, z);
+            tma_load_4d_pair(st + BM * BK * 2, &tm_y, bar, 0, kb * BK, yblk, z);
+          }
           if (++stage == kStages) { stage = 0; phase ^= 1; }
         }
       }
@@ -212,11 +231,26 @@ xty_gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
           const uint32_t sa = smem_u32(smem + stage * Cfg::kStageBytes);
           // MN-major: LBO = distance between 64-column panels, SBO = 8 token rows
           const uint64_t adesc = make_smem_desc_sw128(sa, BK * 128, 1024);
-          const uint64_t bdesc = make_smem_desc_sw128(sa + BM * BK * 2, BK * 128, 1024);
+          const uint64_t bdesc = make_smem_desc_sw128(sa + BM * BK * 2 * PARTS, BK * 128, 1024);
+          auto step = [&](int k) {
+            const uint64_t a = adesc + k * (16 * 128 / 16), b = bdesc + k * (16 * 128 / 16);
+            const uint32_t add = (kb == kb0 && k == 0) ? 0u : 1u;
+            if constexpr (PARTS == 2) {      // residual parts lie behind the values
+              umma_bf16_pair(dst, a + BM * BK * 2 / 16, b, idesc, add);
+              umma_bf16_pair(dst, a, b + Cfg::BNH * BK * 2 / 16, idesc, 1u);
+              umma_bf16_pair(dst, a, b, idesc, 1u);
+            } else {
+              umma_bf16_pair(dst, a, b, idesc, add);
+            }
+          };
+          const long long left = p.T - static_cast<long long>(kb) * BK;
+          if (left >= BK) {
 #pragma unroll
-          for (int k = 0; k < BK / 16; ++k)
-            umma_bf16_pair(dst, adesc + k * (16 * 128 / 16), bdesc + k * (16 * 128 / 16), idesc,
-                           (kb == kb0 && k == 0) ? 0u : 1u);
+            for (int k = 0; k < BK / 16; ++k) step(k);
+          } else {                        // steps past the last token hold zeros only
+#pragma unroll 1
+            for (int k = 0; k < (static_cast<int>(left) + 15) / 16; ++k) step(k);
+          }
           umma_commit_pair(&empty_bar[stage], 3);      // frees the stage in both CTAs
           if (++stage == kStages) { stage = 0; phase ^= 1; }
         }
@@ -226,23 +260,20 @@ xty_gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
     }
   } else if (warp >= 6) {
     // ------------------------------------------------------------------ column sums (warps 6-9, both CTAs)
-    // Present only in launches that ask for them (320 threads).  Every unit adds its share of the
-    // sample's token rows of the chosen operand's 256-column block to the sums: CTA r the 128
-    // columns it also loads for the tensor core.
+    // Present only in launches that ask for them (320 threads): CTA r takes the 128 columns of a 256-column block
+    // that it also loads for the tensor core.
     float* red = reinterpret_cast<float*>(smem + kStages * Cfg::kStageBytes + Cfg::kStoreBytes + 1024 + 256);
     const int ct = static_cast<int>(threadIdx.x) - 192;
     for (long long u = pair; u < units; u += num_pairs) {
       int sample, tm, tn;
       decode(u, sample, tm, tn);
-      // the units that share this (sample, column block) split the sample's token rows among them
-      const int part = (p.cs_of == 1) ? tn : tm, parts = (p.cs_of == 1) ? p.n_tiles : p.m_tiles;
-      const long long per = ((p.T + parts - 1) / parts + 7) / 8 * 8;
-      const long long t0 = part * per;
-      const long long t1 = (t0 + per < p.T) ? t0 + per : p.T;
-      if (t0 >= t1) continue;
-      const int cbase = ((p.cs_of == 1) ? tm : tn) * BN + static_cast<int>(rank) * 128;
+      const bool of_x = p.cs_of == 1;
+      const int parts = of_x ? p.n_tiles : p.m_tiles;
+      const XtyRows rows = xty_colsum_rows(of_x ? tn : tm, parts, p.T);
+      if (rows.t0 >= rows.t1) continue;
+      const int cbase = (of_x ? tm : tn) * BN + static_cast<int>(rank) * 128;
       const long long s_idx = p.sample0 + sample;
-      xty_colsum_128(p.cs_src + s_idx * p.T * p.cs_ld, t0, t1, p.cs_ld, cbase, p.cs_cols, red,
+      xty_colsum_128(p.cs_src + s_idx * p.T * p.cs_ld, rows, parts == 1, p.cs_ld, cbase, p.cs_cols, red,
                      p.cs_out + s_idx * p.cs_cols, ct, 1);
     }
   } else {
@@ -273,13 +304,21 @@ xty_gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
           uint32_t r[32];
           tmem_ld32(t_acc + c0, r);
           tmem_ld_wait();
-          if (live && p.accumulate == 2)
+          if (p.accumulate == 2 && !p.out_vec) {
+            const int m_first = tile128 * BM + warp * 32;
+            if (kb0 < kb1)
+              store_grad_block32(p.out, p.out_is_f32, p.out_accumulate, p.out_scale,
+                                 static_cast<long long>(m_first) * p.n_cols + n0 + c0, p.n_cols, r, p.m_cols - m_first,
+                                 p.n_cols - (n0 + c0), reinterpret_cast<float*>(store_box) + warp * 1024);
+          } else if (live && p.accumulate == 2)
             store_grad_row32(p.out, p.out_is_f32, p.out_accumulate, p.out_scale, static_cast<long long>(m) * p.n_cols + n0 + c0,
                              r, p.n_cols - (n0 + c0), p.out_vec != 0);
           else if (live)
             red_add_row32_pair(p.acc_ws + static_cast<long long>(m) * p.ld_acc + n0 + c0, r, p.n_cols - (n0 + c0));
         }
-      } else if (tile128 < p.m_tiles128 && p.tma_store) {
+      } else if (PARTS == 2 && tile128 < p.m_tiles128 && p.tma_store) {
+        store_tile_f32(&tm_out, store_box, tmem_base + lane_base + acc * BN, ((tile128 * p.n_tiles + tn) * p.samples + sample) * BM, boxes);
+      } else if (PARTS == 1 && tile128 < p.m_tiles128 && p.tma_store) {
         // Tile rows of 512 bytes lie 512 bytes apart: a warp-wide st.global touches 32 lines, and
         // its passes through the L1 data path compete with the column-sum warps' loads and the
         // operand traffic of the tensor core.  Instead every thread writes its row's 64 bytes into
@@ -370,8 +409,10 @@ xty_gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
 static int pair_kernel_smem_attr(const DeviceState* ds) {
   static bool attr_set[64] = {};
   if (!attr_set[ds->device]) {
-    GB_CUDA_OK(cudaFuncSetAttribute(xty_gemm_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    XtyPairCfg::kSmemBytes));
+    GB_CUDA_OK(cudaFuncSetAttribute(xty_gemm_pair_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    XtyPairCfg<1>::kSmemBytes));
+    GB_CUDA_OK(cudaFuncSetAttribute(xty_gemm_pair_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    XtyPairCfg<2>::kSmemBytes));
     attr_set[ds->device] = true;
   }
   return GHOST_OK;
@@ -389,7 +430,7 @@ bool xty_pair_usable(const DeviceState* ds) {
       cudaLaunchConfig_t cfg = {};
       cfg.gridDim = dim3(2, 1, 1);
       cfg.blockDim = dim3(192, 1, 1);
-      cfg.dynamicSmemBytes = XtyPairCfg::kSmemBytes;
+      cfg.dynamicSmemBytes = XtyPairCfg<2>::kSmemBytes;     // the larger of the two instantiations
       cudaLaunchAttribute attr;
       attr.id = cudaLaunchAttributeClusterDimension;
       attr.val.clusterDim.x = 2;
@@ -398,7 +439,7 @@ bool xty_pair_usable(const DeviceState* ds) {
       cfg.attrs = &attr;
       cfg.numAttrs = 1;
       int clusters = 0;
-      if (cudaOccupancyMaxActiveClusters(&clusters, xty_gemm_pair_kernel, &cfg) == cudaSuccess && clusters > 0)
+      if (cudaOccupancyMaxActiveClusters(&clusters, xty_gemm_pair_kernel<2>, &cfg) == cudaSuccess && clusters > 0)
         st = 1;
       else
         (void)cudaGetLastError();
@@ -407,103 +448,86 @@ bool xty_pair_usable(const DeviceState* ds) {
   return st == 1;
 }
 
-// X: [n_samples_total, T, m_cols], Y: [n_samples_total, T, n_cols] bf16, both column counts multiples
-// of 64.  Writes the tiles of samples [sample0, sample0 + samples) to vgrad ([tile][samples][128][256]).
-int launch_xty_pair_tiles(const void* X, const void* Y, long long n_samples_total, long long T, int m_cols,
-                          int n_cols, long long ldx, long long ldy, int samples, int sample0, void* vgrad,
-                          int v_is_f32, int colsum_of, float* colsum_out, const DeviceState* ds, cudaStream_t st) {
-  using Cfg = XtyPairCfg;
-  XtyPairParams p;
-  p.m_cols = m_cols;
-  p.n_cols = n_cols;
-  p.m_tiles128 = ceil_div(m_cols, 128);
-  p.m_tiles = ceil_div(m_cols, 256);
-  p.n_tiles = ceil_div(n_cols, 256);
+template <int PARTS>
+static int launch_pair(const XtyOperands& o, long long samples, long long rows, const CUtensorMap* tout, const XtyPairParams& p,
+                       const DeviceState* ds, cudaStream_t st) {
+  using Cfg = XtyPairCfg<PARTS>;
+  CUtensorMap tx, ty;
+  int rc;
+  if ((rc = xty_operand_map(&tx, o, 0, samples, rows, Cfg::BK, Cfg::BM / 64)) != GHOST_OK) return rc;
+  if ((rc = xty_operand_map(&ty, o, 1, samples, rows, Cfg::BK, Cfg::BNH / 64)) != GHOST_OK) return rc;
+  if ((rc = pair_kernel_smem_attr(ds)) != GHOST_OK) return rc;
+  const long long units = static_cast<long long>(p.m_tiles) * p.n_tiles * p.samples;
+  long long pairs = ds->sm_count / 2;
+  if (pairs > units) pairs = units;
+  xty_gemm_pair_kernel<PARTS><<<static_cast<int>(2 * pairs), p.cs_of ? 320 : 192, Cfg::kSmemBytes, st>>>(tx, ty, tout ? *tout : tx, p);
+  count_launch();
+  return post_launch("xty_gemm_pair_kernel");
+}
+
+static XtyPairParams pair_params(const XtyOperands& o, const DeviceState* ds) {
+  XtyPairParams p = {};
+  p.m_cols = o.cols[0];
+  p.n_cols = o.cols[1];
+  p.m_tiles128 = ceil_div(p.m_cols, 128);
+  p.m_tiles = ceil_div(p.m_cols, 256);
+  p.n_tiles = ceil_div(p.n_cols, 256);
+  p.out_scale = 1.f;
+  p.err = ds->err_word;
+  return p;
+}
+
+// Writes the tiles of samples [sample0, sample0 + samples) of the n_samples_total that the operands hold to
+// vgrad ([tile][samples][128][256]); operands in the blocked layout only (XtyOperands::blocked).
+int launch_xty_pair_tiles(const XtyOperands& o, long long n_samples_total, long long T, int samples, int sample0, void* vgrad,
+                          int v_is_f32, const XtyColsum& cs, float* zero, long long zero_n, const DeviceState* ds, cudaStream_t st) {
+  using Cfg = XtyPairCfg<1>;
+  XtyPairParams p = pair_params(o, ds);
   p.samples = samples;
   p.sample0 = sample0;
   p.T = T;
   p.vgrad = vgrad;
   p.v_is_f32 = v_is_f32;
-  // bf16 tiles go out through the copy engine (row counts up to 2^31 keep the box coordinate an int)
+  // tiles go out through the copy engine (row counts up to 2^31 keep the box coordinate an int), but for float32 tiles
+  // of operands that are one part (stacked by the caller)
   const unsigned long long out_rows = static_cast<unsigned long long>(p.m_tiles128) * p.n_tiles * samples * Cfg::BM;
-  p.tma_store = (!v_is_f32 && out_rows < (1ull << 31)) ? 1 : 0;
-  p.accumulate = 0;
-  p.out = nullptr;
-  p.out_is_f32 = p.out_accumulate = p.out_vec = 0;
-  p.out_scale = 1.f;
-  p.kb_per_split = 0;
-  p.acc_ws = nullptr;
-  p.ld_acc = 0;
-  p.cs_of = (colsum_out != nullptr) ? colsum_of : 0;
-  p.cs_src = static_cast<const __nv_bfloat16*>(p.cs_of == 1 ? X : Y);
-  p.cs_ld = (p.cs_of == 1) ? ldx : ldy;
-  p.cs_cols = (p.cs_of == 1) ? m_cols : n_cols;
-  p.cs_out = colsum_out;
-  p.err = ds->err_word;
-  if (p.cs_of)
-    GB_CUDA_OK(cudaMemsetAsync(colsum_out + static_cast<long long>(sample0) * p.cs_cols, 0,
-                               sizeof(float) * static_cast<size_t>(samples) * p.cs_cols, st));
-  CUtensorMap tx, ty;
+  p.tma_store = (v_is_f32 == (o.parts == 2 ? 1 : 0) && out_rows < (1ull << 31)) ? 1 : 0;
+  p.cs_of = cs.of;
+  if (cs.of) {
+    p.cs_src = static_cast<const __nv_bfloat16*>(o.ptr[cs.of - 1]);
+    p.cs_ld = o.ld[cs.of - 1];
+    p.cs_cols = o.cols[cs.of - 1];
+  }
+  p.cs_out = cs.out;
+  p.zero = zero;
+  p.zero_n = zero_n;
+  CUtensorMap tout;
   int rc;
-  if ((rc = make_tmap_bf16_blocks(&tx, X, n_samples_total, T, m_cols, ldx, Cfg::BK, Cfg::BM / 64)) != GHOST_OK) return rc;
-  if ((rc = make_tmap_bf16_blocks(&ty, Y, n_samples_total, T, n_cols, ldy, Cfg::BK, Cfg::BNH / 64)) != GHOST_OK) return rc;
-  CUtensorMap tout = tx;
-  if (p.tma_store && (rc = make_tmap_bf16_store_2d(&tout, vgrad, out_rows, Cfg::BN, Cfg::BM)) != GHOST_OK) return rc;
-  if ((rc = pair_kernel_smem_attr(ds)) != GHOST_OK) return rc;
-  const long long units = static_cast<long long>(p.m_tiles) * p.n_tiles * samples;
-  long long pairs = ds->sm_count / 2;
-  if (pairs > units) pairs = units;
-  xty_gemm_pair_kernel<<<static_cast<int>(2 * pairs), p.cs_of ? 320 : 192, Cfg::kSmemBytes, st>>>(tx, ty, tout, p);
-  count_launch();
-  return post_launch("xty_gemm_pair_kernel");
+  if ((rc = xty_colsum_clear(cs, p.cs_of == 1 ? p.n_tiles : p.m_tiles, sample0, samples, p.cs_cols, st)) != GHOST_OK) return rc;
+  if (p.tma_store && (rc = (v_is_f32 ? make_tmap_f32_store_2d : make_tmap_bf16_store_2d)(&tout, vgrad, out_rows, Cfg::BN, Cfg::BM)) != GHOST_OK)
+    return rc;
+  const CUtensorMap* t = p.tma_store ? &tout : nullptr;
+  return o.parts == 2 ? launch_pair<2>(o, n_samples_total, T, t, p, ds, st) : launch_pair<1>(o, n_samples_total, T, t, p, ds, st);
 }
 
-// Train-gradient pass over n_rows token rows, both column counts multiples of 64: one split stores
+// Train-gradient pass over n_rows token rows (one sample), operands in the blocked layout: one split stores
 // scale * X^T Y to `out`, more of them add into acc_ws[m_cols, ld_acc] (fp32, zeroed by the caller).
-int launch_xty_pair_wgrad(const void* X, const void* Y, long long n_rows, int m_cols, int n_cols, long long ldx,
-                          long long ldy, int splits, float* acc_ws, long long ld_acc, void* out, int out_is_f32,
-                          float scale, int accumulate, const DeviceState* ds, cudaStream_t st) {
-  using Cfg = XtyPairCfg;
-  XtyPairParams p;
-  p.m_cols = m_cols;
-  p.n_cols = n_cols;
-  p.m_tiles128 = ceil_div(m_cols, 128);
-  p.m_tiles = ceil_div(m_cols, 256);
-  p.n_tiles = ceil_div(n_cols, 256);
-  p.sample0 = 0;
+int launch_xty_pair_wgrad(const XtyOperands& o, long long n_rows, int splits, float* acc_ws, long long ld_acc, void* out,
+                          int out_is_f32, float scale, int accumulate, const DeviceState* ds, cudaStream_t st) {
+  XtyPairParams p = pair_params(o, ds);
   p.T = n_rows;
-  p.vgrad = nullptr;
-  p.v_is_f32 = 0;
-  p.tma_store = 0;
   p.accumulate = splits == 1 ? 2 : 1;
   p.out = out;
   p.out_is_f32 = out_is_f32;
   p.out_accumulate = accumulate;
-  p.out_vec = (reinterpret_cast<uintptr_t>(out) & 15u) == 0;
+  p.out_vec = p.n_cols % 8 == 0 && (reinterpret_cast<uintptr_t>(out) & 15u) == 0;
   p.out_scale = scale;
   p.acc_ws = acc_ws;
   p.ld_acc = ld_acc;
-  p.cs_of = 0;
-  p.cs_src = nullptr;
-  p.cs_ld = 0;
-  p.cs_cols = 0;
-  p.cs_out = nullptr;
-  p.err = ds->err_word;
-  const long long pairs_max = ds->sm_count / 2;
-  const int kb = static_cast<int>(ceil_div(n_rows, static_cast<long long>(Cfg::BK)));
-  const long long blocks = static_cast<long long>(p.m_tiles) * p.n_tiles;
+  const int kb = ceil_div(n_rows, o.parts == 2 ? XtyPairCfg<2>::BK : XtyPairCfg<1>::BK);
   p.kb_per_split = ceil_div(kb, splits);
   p.samples = ceil_div(kb, p.kb_per_split);
-  CUtensorMap tx, ty;
-  int rc;
-  if ((rc = make_tmap_bf16_blocks(&tx, X, 1, n_rows, m_cols, ldx, Cfg::BK, Cfg::BM / 64)) != GHOST_OK) return rc;
-  if ((rc = make_tmap_bf16_blocks(&ty, Y, 1, n_rows, n_cols, ldy, Cfg::BK, Cfg::BNH / 64)) != GHOST_OK) return rc;
-  if ((rc = pair_kernel_smem_attr(ds)) != GHOST_OK) return rc;
-  const long long units = blocks * p.samples;
-  const long long pairs = pairs_max < units ? pairs_max : units;
-  xty_gemm_pair_kernel<<<static_cast<int>(2 * pairs), 192, Cfg::kSmemBytes, st>>>(tx, ty, tx, p);
-  count_launch();
-  return post_launch("xty_gemm_pair_kernel");
+  return o.parts == 2 ? launch_pair<2>(o, 1, n_rows, nullptr, p, ds, st) : launch_pair<1>(o, 1, n_rows, nullptr, p, ds, st);
 }
 
 }  // namespace gb

@@ -63,10 +63,20 @@ int ghost_cast_split_bf16(const void* src, int src_is_f32, long long samples, lo
                           long long ld_src, void* dst, long long ld_dst, int cpad, int parts,
                           int kind0, int kind1, int kind2, int row_stack, void* stream);
 
+/* Both operands of a GEMM over tokens in one launch: X [samples, T, x_cols] and Y [samples, T, y_cols] (dense, fp32
+ * or bf16; either may be NULL with its destination) as [samples, parts, T, cols rounded up to 64] bf16, zero-padded:
+ * the values, and with parts = 2 behind each sample's values their residuals bf16(x - bf16(x)).  This is the layout of
+ * ghost_persample_dot_parts and ghost_wgrad_parts (samples = 1 and T = all rows there).  x_sums / y_sums, if not
+ * NULL, receive the operand's column sums per sample (fp32, [samples, cols]) on the way.  Same reference lines. */
+int ghost_split_operands(const void* X, int x_is_f32, int x_cols, const void* Y, int y_is_f32, int y_cols, int parts,
+                         long long samples, long long T, void* X_out, void* Y_out, float* x_sums, float* y_sums,
+                         void* stream);
+
 /* The same from a convolution operand: token (oy, ox) of sample n holds the C * kh * kw inputs of
  * src [samples, C, H, W] (dense) under the kernel window, in the order of torch's unfold; tokens per
  * sample are Ho * Wo of a convolution with strides (sy, sx), zero paddings (py, px) and dilations
- * (dy, dx).  A 1 x 1 window turns an [N, p, Ho, Wo] out-grad into tokens.  Replaces the F.unfold of
+ * (dy, dx).  row_stack = 2 stacks the parts over the whole batch, [parts, samples * tokens, cpad].
+ * A 1 x 1 window turns an [N, p, Ho, Wo] out-grad into tokens.  Replaces the F.unfold of
  * ghostEngines/supported_layers_grad_samplers_dotprod.py:513-592 and the casts after it. */
 int ghost_conv_tokens_bf16(const void* src, int src_is_f32, long long samples, int C, int H, int W, int kh,
                            int kw, int sy, int sx, int py, int px, int dy, int dx, void* dst,
@@ -104,6 +114,13 @@ int ghost_wgrad_bf16(const void* X, const void* Y, long long n_rows, int m_cols,
                      long long ldx, long long ldy, float scale, int accumulate, void* out,
                      int out_is_f32, void* ws, long long ws_bytes, void* stream);
 
+/* The same over operands as ghost_split_operands lays them out: X [parts, n_rows, ldx], the pitch a multiple of 64
+ * and zero beyond the columns (parts = 1: an operand whose pitch is smaller than that is read as it is).
+ * parts = 2 contracts value x value + value x residual + residual x value. */
+int ghost_wgrad_parts(const void* X, const void* Y, int parts, long long n_rows, int m_cols, int n_cols, long long ldx,
+                      long long ldy, float scale, int accumulate, void* out, int out_is_f32, void* ws, long long ws_bytes,
+                      void* stream);
+
 /* ---- Linear / Conv1D weight dot product, per-sample-gradient path ---------------------------- */
 /* X, Y: [n_train + n_val, T, cols] bf16.  M[v,b] = dot_scale * <X_v^T Y_v, X_b^T Y_b>.  Per-sample
  * weight-gradient tiles are formed in TMEM by a tcgen05 GEMM over each sample's tokens and written
@@ -136,6 +153,13 @@ int ghost_persample_dot_bf16(const void* X, const void* Y, int n_train, int n_va
                              float* M_out, int v_is_f32, void* grad_out, int grad_is_f32,
                              float grad_scale, int grad_accumulate, int colsum_of, float* colsum_out,
                              void* ws, long long ws_bytes, void* stream);
+
+/* The same over operands as ghost_split_operands lays them out ([n_train + n_val, parts, T, ld]); parts = 2 stores
+ * fp32 tiles (workspace with v_is_f32 = 1) and takes no column sums, parts = 1 bf16 ones. */
+int ghost_persample_dot_parts(const void* X, const void* Y, int parts, int n_train, int n_val, long long T, int m_cols,
+                              int n_cols, long long ldx, long long ldy, float dot_scale, float* M_out, void* grad_out,
+                              int grad_is_f32, float grad_scale, int grad_accumulate, int colsum_of,
+                              float* colsum_out, void* ws, long long ws_bytes, void* stream);
 
 /* The same path as two calls, for callers that put something between the passes: in a data-parallel
  * run whose ranks each hold a part of the validation batch, a rank computes the tiles of its own

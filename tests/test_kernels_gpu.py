@@ -193,6 +193,49 @@ def test_persample_dot_column_sums(case, which):
     assert res[2] is None
 
 
+# token counts around a step of 16, a stage of 32 / 64 and one of 128; columns around a panel of 64, one and two
+# tiles of 128; every operand needs a copy, so the padded and the two-part layouts are what runs
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("case", [(3, 2, 1, 63, 65), (2, 1, 16, 127, 129), (3, 1, 17, 257, 63), (2, 2, 33, 130, 70),
+                                  (2, 1, 63, 65, 257), (2, 1, 129, 300, 140), (33, 3, 5, 71, 199), (2, 1, 260, 190, 510)])
+def test_padded_and_split_operands(case, dtype):
+    """Padded bf16 copies and two-part float32 operands: matrix, train gradient, column sums, and the
+    gradient GEMM with results that no 16-byte store fits, through both tile kernels."""
+    from ghostsuite_b200 import _lib
+    lib = _lib.load()
+    n_t, n_v, T, d, p = case
+    A, G = make(n_t + n_v, T, d, p, dtype, seed=31)
+    # values and residuals are 8 bits each and the product of two residuals is left out: 2^-16 a product, and
+    # the bf16 path stores its tiles in 8 bits
+    tol = 2 * 2.0 ** -16 if dtype == torch.float32 else 2 * 2.0 ** -8
+    S = torch.einsum("ntp,ntd->npd", G.double(), A.double())
+    ref, gref, cref = torch.einsum("vpd,bpd->vb", S[n_t:], S[:n_t]), S[:n_t].sum(0), G.double().sum(1)
+    size = (S[n_t:].flatten(1).norm(dim=1)[:, None] * S[:n_t].flatten(1).norm(dim=1)[None]).norm()
+    old = torch.full((p, d), 0.25, dtype=dtype, device="cuda")
+    try:
+        for mode in (0, 2):
+            _lib.check(lib.ghost_set_persample_pair_mode(mode))
+            _lib.check(lib.ghost_set_wgrad_pair_mode(mode))
+            M, grad, sums = ops().persample_dot(G.cuda(), A.cuda(), n_v, want_grad=True, grad_scale=0.5,
+                                                grad_dtype=torch.float32, colsum_of="X")
+            hook = ops().dense_hook(A.cuda(), G.cuda(), n_v, False, False, torch.float32, 0.5, True, torch.float32,
+                                    False, True)
+            out = ops().wgrad(G[:n_t].cuda(), A[:n_t].cuda(), 0.5, dtype)
+            acc = ops().wgrad(G[:n_t].cuda(), A[:n_t].cuda(), 0.5, dtype, out=old.clone(), accumulate=True)
+            after()
+            assert (M.cpu().double() - ref).norm() < tol * size
+            assert O.rel_fro(grad, 0.5 * gref) < tol
+            assert (hook[0].cpu().double() - ref).norm() < tol * size and O.rel_fro(hook[1], 0.5 * gref) < tol
+            for got in ([sums] if sums is not None else []) + [hook[2]]:
+                assert O.rel_fro(got, cref) < 1e-6
+            assert O.rel_fro(out, 0.5 * gref) < tol
+            assert O.rel_fro(acc.float() - 0.25, 0.5 * gref) < tol + 2 * 0.25 * (p * d) ** 0.5 / gref.norm() * (
+                2.0 ** -24 if dtype == torch.float32 else 2.0 ** -9) * 2
+    finally:
+        _lib.check(lib.ghost_set_persample_pair_mode(1))
+        _lib.check(lib.ghost_set_wgrad_pair_mode(1))
+
+
 @pytest.mark.parametrize("sizes", [(37, 11, 70, 136, 264), (70, 35, 12, 72, 264)])
 def test_persample_dot_in_groups(sizes):
     """A small workspace budget forces the train samples through in several groups (and several
