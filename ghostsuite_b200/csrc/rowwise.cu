@@ -282,22 +282,43 @@ __global__ void colsum_kernel(const T* __restrict__ G, long long Tn, int cols, l
 // LayerNorm per-sample gradients, one warp per token row, F <= 256 * NCHUNK, F % 8 == 0.
 //   gw[n, f] += sum_t G[n,t,f] * xhat[n,t,f],   gb[n, f] += sum_t G[n,t,f]
 // ------------------------------------------------------------------------------------------
-__device__ __forceinline__ void cp_async16(void* smem_dst, const void* gmem_src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(smem_dst))),
-               "l"(gmem_src) : "memory");
-}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+// Two float32 operations an instruction, each rounded as the single one is
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  float2 d;
+  asm("{\n\t.reg .b64 x, y;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tadd.rn.f32x2 x, x, y;\n\tmov.b64 {%0, %1}, x;\n\t}"
+      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  float2 d;
+  asm("{\n\t.reg .b64 x, y;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmul.rn.f32x2 x, x, y;\n\tmov.b64 {%0, %1}, x;\n\t}"
+      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmov.b64 z, {%6, %7};\n\tfma.rn.f32x2 x, x, y, z;\n\t"
+      "mov.b64 {%0, %1}, x;\n\t}"
+      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return d;
 }
 
 // Each warp streams its token rows through a private three-slot ring in shared memory filled with
 // cp.async: the loads of the next two rows are in flight while the current row goes through its two
 // dependent shuffle reductions.  A lane reads back exactly the 16-byte pieces it copied itself, so
 // the ring needs no synchronisation beyond cp.async.wait_group.
+//
+// Bound by issue slots before HBM: 388 instructions a row of 768 bf16 features kept the schedulers 60 % busy at
+// 4.35 TB/s.  So features go in pairs (f32x2), and a width that fills the lanes (FULL: F = 256 NCHUNK) has no tests:
+// 40 x 1024 rows went from 30.1 to 24.2 us (5.2 TB/s).
 constexpr int kLnSlots = 3;
 
-template <typename T, int NCHUNK>
+template <typename T, int NCHUNK, bool FULL>
 __global__ void __launch_bounds__(256, NCHUNK <= 3 ? 2 : 1)
 layernorm_persample_kernel(const T* __restrict__ A, const T* __restrict__ G, long long Tn, int F,
                            float eps, float* __restrict__ gw, float* __restrict__ gb,
@@ -310,77 +331,83 @@ layernorm_persample_kernel(const T* __restrict__ A, const T* __restrict__ G, lon
   const long long per = (Tn + t_splits - 1) / t_splits;
   const long long t0 = split * per;
   const long long t1 = (t0 + per < Tn) ? t0 + per : Tn;
-  float aw[NCHUNK][8], ab[NCHUNK][8];
+  float2 aw[NCHUNK][4], ab[NCHUNK][4];
 #pragma unroll
   for (int i = 0; i < NCHUNK; ++i)
 #pragma unroll
-    for (int j = 0; j < 8; ++j) { aw[i][j] = 0.f; ab[i][j] = 0.f; }
+    for (int j = 0; j < 4; ++j) aw[i][j] = ab[i][j] = make_float2(0.f, 0.f);
   const float invF = 1.f / static_cast<float>(F);
+  auto inside = [&](int i) { return FULL || (i * 32 + lane) * 8 < F; };
 
-  auto issue = [&](long long t, int slot) {
-    if (t < t1) {
-      const long long off = (static_cast<long long>(n) * Tn + t) * F;
-      T* sa = ring + static_cast<size_t>(slot) * 2 * F;
-      T* sg = sa + F;
+  long long t = t0 + warp, ahead = t;                  // row at work, row to fetch next
+  const T *pa = A + (static_cast<long long>(n) * Tn + t) * F + lane * 8, *pg = G + (pa - A);
+  const uint32_t ring0 = static_cast<uint32_t>(__cvta_generic_to_shared(ring + lane * 8)), slot_bytes = 2 * F * sizeof(T);
+  const uint32_t row_bytes = F * sizeof(T);
+  auto issue = [&](int slot) {
+    if (ahead < t1) {
+      const uint32_t dst = ring0 + slot * slot_bytes;
 #pragma unroll
       for (int i = 0; i < NCHUNK; ++i) {
-        const int f = (i * 32 + lane) * 8;
-        if (f < F) {
+        if (inside(i)) {
 #pragma unroll
           for (int b = 0; b < static_cast<int>(8 * sizeof(T)); b += 16) {
-            cp_async16(reinterpret_cast<unsigned char*>(sa + f) + b, reinterpret_cast<const unsigned char*>(A + off + f) + b);
-            cp_async16(reinterpret_cast<unsigned char*>(sg + f) + b, reinterpret_cast<const unsigned char*>(G + off + f) + b);
+            const int at = i * 256 * static_cast<int>(sizeof(T)) + b;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + at), "l"(reinterpret_cast<const unsigned char*>(pa) + at) : "memory");
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + row_bytes + at), "l"(reinterpret_cast<const unsigned char*>(pg) + at) : "memory");
           }
         }
       }
     }
     cp_async_commit();      // an empty group keeps the group count uniform at the tail
+    ahead += 8;
+    pa += 8ll * F;
+    pg += 8ll * F;
   };
 
-  long long t = t0 + warp;
-  issue(t, 0);
-  issue(t + 8, 1);
+  issue(0);
+  issue(1);
   int slot = 0;
   for (; t < t1; t += 8) {
-    issue(t + 16, slot == 0 ? 2 : slot - 1);
+    issue(slot == 0 ? 2 : slot - 1);
     cp_async_wait<kLnSlots - 1>();
     const T* sa = ring + static_cast<size_t>(slot) * 2 * F;
     const T* sg = sa + F;
     slot = (slot + 1 == kLnSlots) ? 0 : slot + 1;
-    float x[NCHUNK][8], g[NCHUNK][8];
-    float s = 0.f;
+    float2 x[NCHUNK][4], g[NCHUNK][4];
+    auto load = [&](const T* row, int i, float2 (&v)[4]) {
+      float e[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+      if (inside(i)) Vec8<T>::load(row + (i * 32 + lane) * 8, e);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) v[j] = make_float2(e[2 * j], e[2 * j + 1]);
+    };
+    float2 s = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int i = 0; i < NCHUNK; ++i) load(sa, i, x[i]);
+#pragma unroll
+    for (int i = 0; i < NCHUNK; ++i) load(sg, i, g[i]);
+    float mean = 0.f;                                  // RMS norm: no centring
+    if (!rms) {
+#pragma unroll
+      for (int i = 0; i < NCHUNK; ++i) s = add2(s, add2(add2(x[i][0], x[i][1]), add2(x[i][2], x[i][3])));
+      mean = warp_sum(s.x + s.y) * invF;
+    }
+    const float2 centre = make_float2(-mean, -mean);
+    float2 q = make_float2(0.f, 0.f);
 #pragma unroll
     for (int i = 0; i < NCHUNK; ++i) {
-      const int f = (i * 32 + lane) * 8;
-      if (f < F) {
-        Vec8<T>::load(sa + f, x[i]);
-        Vec8<T>::load(sg + f, g[i]);
-      } else {
+      if (inside(i)) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) { x[i][j] = 0.f; g[i][j] = 0.f; }
+        for (int j = 0; j < 4; ++j) { x[i][j] = add2(x[i][j], centre); q = fma2(x[i][j], x[i][j], q); }
       }
     }
+    const float rstd = rsqrtf(warp_sum(q.x + q.y) * invF + eps);
+    const float2 scale = make_float2(rstd, rstd);
 #pragma unroll
     for (int i = 0; i < NCHUNK; ++i)
 #pragma unroll
-      for (int j = 0; j < 8; ++j) s += x[i][j];
-    const float mean = rms ? 0.f : warp_sum(s) * invF;     // RMS norm: no centring
-    float q = 0.f;
-#pragma unroll
-    for (int i = 0; i < NCHUNK; ++i) {
-      const int f = (i * 32 + lane) * 8;
-      if (f < F) {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) { x[i][j] -= mean; q += x[i][j] * x[i][j]; }
-      }
-    }
-    const float rstd = rsqrtf(warp_sum(q) * invF + eps);
-#pragma unroll
-    for (int i = 0; i < NCHUNK; ++i)
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        aw[i][j] = fmaf(g[i][j], x[i][j] * rstd, aw[i][j]);
-        ab[i][j] += g[i][j];
+      for (int j = 0; j < 4; ++j) {
+        aw[i][j] = fma2(g[i][j], mul2(x[i][j], scale), aw[i][j]);
+        ab[i][j] = add2(ab[i][j], g[i][j]);
       }
   }
   cp_async_wait<0>();
@@ -391,7 +418,10 @@ layernorm_persample_kernel(const T* __restrict__ A, const T* __restrict__ G, lon
     const int f = (i * 32 + lane) * 8;
     if (f < F) {
 #pragma unroll
-      for (int j = 0; j < 8; ++j) { mine[f + j] = aw[i][j]; mine[F + f + j] = ab[i][j]; }
+      for (int j = 0; j < 4; ++j) {
+        *reinterpret_cast<float2*>(mine + f + 2 * j) = aw[i][j];
+        *reinterpret_cast<float2*>(mine + F + f + 2 * j) = ab[i][j];
+      }
     }
   }
   __syncthreads();
@@ -778,6 +808,18 @@ static int launch_norm_wide(dim3 grid, const T* A, const T* G, long long Tn, int
   return launch_norm_wide_of<T, VEC, 16, 512>(grid, A, G, Tn, F, eps, gw, gb, ws, splits, ds, st, rms);
 }
 
+template <typename T, int NCHUNK, bool FULL>
+static int launch_ln_warp(dim3 grid, size_t smem, const T* A, const T* G, long long Tn, int F, float eps, float* gw, float* gb, float* ws,
+                          int splits, const DeviceState* ds, cudaStream_t st, int rms) {
+  static bool attr_set[64] = {};
+  if (!attr_set[ds->device]) {
+    GB_CUDA_OK(cudaFuncSetAttribute(layernorm_persample_kernel<T, NCHUNK, FULL>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    attr_set[ds->device] = true;
+  }
+  layernorm_persample_kernel<T, NCHUNK, FULL><<<grid, 256, smem, st>>>(A, G, Tn, F, eps, gw, gb, ws, splits, rms);
+  return GHOST_OK;
+}
+
 template <typename T>
 static int launch_ln(const T* A, const T* G, int N, long long Tn, int F, float eps, float* gw, float* gb,
                      float* ws, long long ws_bytes, const DeviceState* ds, cudaStream_t st, int rms) {
@@ -795,12 +837,8 @@ static int launch_ln(const T* A, const T* G, int N, long long Tn, int F, float e
     const int nchunk = aligned ? (F + 255) / 256 : 0;
     int rc = GHOST_OK;
 #define GB_LN_LAUNCH(NC)                                                                              \
-    do {                                                                                              \
-      if (smem > 48 * 1024)                                                                           \
-        GB_CUDA_OK(cudaFuncSetAttribute(layernorm_persample_kernel<T, NC>,                            \
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));    \
-      layernorm_persample_kernel<T, NC><<<grid, 256, smem, st>>>(A, G, Tn, F, eps, gw, gb, ws, splits, rms); \
-    } while (0)
+    rc = F == 256 * NC ? launch_ln_warp<T, NC, true>(grid, smem, A, G, Tn, F, eps, gw, gb, ws, splits, ds, st, rms) \
+                       : launch_ln_warp<T, NC, false>(grid, smem, A, G, Tn, F, eps, gw, gb, ws, splits, ds, st, rms)
     switch (nchunk) {
       case 0: rc = launch_norm_wide<T, false>(grid, A, G, Tn, F, eps, gw, gb, ws, splits, ds, st, rms); break;
       case 1: GB_LN_LAUNCH(1); break;
