@@ -85,6 +85,7 @@ PROTOTYPES = {
     "ghost_embedding_pass_workspace_bytes": (_ll, [_i, _i, _ll, _i, _i]),
     "ghost_embedding_pass": (_i, [_vp, _vp, _i, _i, _i, _ll, _i, _i, _f, _vp, _f, _f, _i, _vp, _vp, _ll, _vp]),
     "ghost_gradproj_dense_bf16": (_i, [_vp, _vp, _i, _ll, _i, _i, _ll, _ll, _vp, _vp, _i, _i, _ll, _ll, _f, _vp, _ll, _vp]),
+    "ghost_gradproj_dense": (_i, [_vp, _vp, _i, _i, _ll, _i, _i, _ll, _ll, _vp, _vp, _i, _i, _ll, _ll, _i, _i, _f, _vp, _ll, _vp]),
     "ghost_gradproj_embedding": (_i, [_vp, _vp, _i, _i, _ll, _i, _ll, _vp, _ll, _i, _i, _vp, _ll, _i, _i, _i, _f,
                                       _i, _vp, _ll, _i, _vp]),
     "ghost_projection_similarity": (_i, [_vp, _vp, _i, _i, _i, _ll, _ll, _ll, _f, _vp, _ll, _vp]),

@@ -17,7 +17,18 @@
 // The embedding form (kEmb) has token ids in place of A: the rows of P_c^T are gathered by id straight into
 // the staged block, out[b] = scale * sum_t (P_r g_t)(P_c[:, id_t])^T, and only G is streamed.
 //
-// CTA layout (192 threads): warps 0-3 epilogue, warp 4 TMA producer, warp 5 MMA issuer.
+// float32 rows, and bf16 rows that TMA cannot read, come through the registers of eight more warps (kSrc), which write
+// the swizzled bf16 blocks -- of float32 data value and residual, three products -- so that such operands too are
+// read once: copies in parts beforehand moved 16 bytes for every element of four (8 x 4096 tokens of 1024 + 1024
+// float32, k = 32: 189 -> 97 us; token table of 1024 float32 features, 16 x 2048 tokens: 107 -> 56 with mma.sync before).
+//
+// Few (sample, 128-token) units: a unit is one CTA's chain over all columns of G and A, whatever the number of
+// tokens in it, so a small batch leaves the GPU idle for the length of that chain.  There (kCluster) a cluster of
+// up to eight CTAs shares a unit: each projects its part of the columns, the partial [128, k] blocks are added through
+// distributed shared memory in rank order, and every CTA contracts its share of the tokens (10 tokens of 4407 + 452
+// float32, k = 44: 77 -> 22 us; 6 x 54 tokens of 2944 + 6528 bf16, k = 13: 47 -> 15).
+//
+// CTA layout: warps 0-3 epilogue, warp 4 TMA producer, warp 5 MMA issuer, warps 6-13 loaders where kSrc asks for them.
 #include "common.cuh"
 #include "sm100_ptx.cuh"
 
@@ -33,6 +44,11 @@ struct GpParams {
   long long units;         // B * chunks_per_sample
   int units_per_cta;       // base number of units per CTA
   int units_extra;         // the first `units_extra` CTAs take one more
+  // register loaders: the operands themselves, and where the residual part of P_r / P_c starts (kSrcF32)
+  const void *g, *a;
+  long long ldg, lda;
+  int lo_r, lo_c;
+  int vec_g, vec_a;        // rows on 16-byte (float32) / 8-byte (bf16) boundaries
   float scale;
   float* out;              // sample b at out + b * out_stride, [k_r, k_c] row-major
   long long out_stride;
@@ -45,25 +61,30 @@ struct GpParams {
   int* err;
 };
 
-template <int KMAX>   // largest padded rank this instantiation handles (32, 64 or 128)
+enum { kSrcTma = 0, kSrcF32 = 1, kSrcBf16 = 2 };      // how the rows of G and A reach shared memory
+
+template <int KMAX, int kSrc, bool kCluster>   // KMAX: largest padded rank this instantiation handles (32, 64 or 128)
 struct GpCfg {
   static constexpr int BM = 128, BK = 64;                  // BK: one 128-byte swizzle atom of bf16
+  static constexpr int PARTS = kSrc == kSrcF32 ? 2 : 1;    // bf16 parts of an element
   // Columns per pipeline stage = ATOMS * 64.  The single threads that drive the pipeline pay a few
   // hundred cycles per stage for the barrier round trip, so a stage carries two atoms when the
   // shared memory allows it.
-  static constexpr int ATOMS = (KMAX == 128) ? 1 : 2;
+  static constexpr int ATOMS = (KMAX == 128 || kSrc != kSrcTma) ? 1 : 2;
   static constexpr int kActAtomBytes = BM * BK * 2;
   static constexpr int kProjAtomBytes = KMAX * BK * 2;
-  static constexpr int kStageBytes = ATOMS * (kActAtomBytes + kProjAtomBytes);
+  static constexpr int kStageBytes = ATOMS * PARTS * (kActAtomBytes + kProjAtomBytes);
   // The pipeline is bound by how many bytes are in flight per SM, so the fp32 staging of the
-  // projected blocks is kept to half a tile (64 tokens at a time) and the rest goes to stages.
-  static constexpr int kStageRows = 64;
+  // projected blocks is kept to half a tile (64 tokens at a time; a cluster's partial blocks are
+  // staged whole) and the rest goes to stages: it fills the 227 KB of shared memory.
+  static constexpr int kStageRows = kCluster ? 128 : 64;
   static constexpr int kProjBytes = 2 * kStageRows * KMAX * 4;
-  static constexpr int kStages = (KMAX == 32) ? 5 : (KMAX == 64 ? 4 : 5);     // fills the 227 KB of shared memory
+  static constexpr int kRoom = (232448 - 1280 - kProjBytes) / kStageBytes;
+  static constexpr int kStages = kRoom < 8 ? kRoom : 8;
   static constexpr int kSmemBytes = kStages * kStageBytes + kProjBytes + 1024 + 256;
+  static constexpr int kThreads = kSrc == kSrcTma ? 192 : 448;
   static constexpr int RT = KMAX / 16;   // output rows per thread (16 thread rows)
   static constexpr int CT = KMAX / 8;    // output cols per thread (8 thread cols)
-  static constexpr int NCH = KMAX / 4;   // float4 chunks per staged row
 };
 
 // Staged fp32 rows are stored with their float4 chunks XOR-permuted by the row index, so that the
@@ -73,19 +94,98 @@ __device__ __forceinline__ int gp_staged_index(int row, int elem) {
   return row * KMAX + ((((elem >> 2) ^ row) & (KMAX / 4 - 1)) << 2) + (elem & 3);
 }
 
-template <int KMAX, bool kEmb>
-__global__ void __launch_bounds__(192, 1)
+// A loader warp's share of a stage, 16 rows of 64 columns, held in registers between its load and its store; nothing looks
+// at a loaded value before the store.  float32: lane l has columns 4 (l % 16) .. + 3 of rows l / 16 + 2 i, a vector where
+// rows are on its boundaries.  bf16 rows the same way, but element by element where they are not: there a lane has
+// columns l and l + 32 of all rows, so that a load of the warp covers neighbouring elements.
+template <int kSrc> struct GpRows;
+template <> struct GpRows<kSrcF32> {
+  float4 v[8];
+  // base + at: the warp's first row, column of the stage's first column; `left` columns and `rows` rows from there on
+  __device__ __forceinline__ void load(const void* base, long long at, long long ld, int left, long long rows, bool vec, int lane) {
+    const int r0 = lane >> 4, c = (lane & 15) * 4, cols = left - c;
+    const float* p = static_cast<const float*>(base) + at + r0 * ld + c;
+#pragma unroll
+    for (int i = 0; i < 8; ++i, p += 2 * ld) {
+      const bool in = r0 + 2 * i < rows;
+      if (vec) {                           // widths are multiples of four here
+        v[i] = in && cols > 0 ? __ldg(reinterpret_cast<const float4*>(p)) : make_float4(0.f, 0.f, 0.f, 0.f);
+      } else {
+        v[i].x = in && cols > 0 ? __ldg(p) : 0.f;
+        v[i].y = in && cols > 1 ? __ldg(p + 1) : 0.f;
+        v[i].z = in && cols > 2 ? __ldg(p + 2) : 0.f;
+        v[i].w = in && cols > 3 ? __ldg(p + 3) : 0.f;
+      }
+    }
+  }
+  // into the stage's two [128 rows][64 columns] swizzled blocks; first: the warp's first row in them
+  __device__ __forceinline__ void store(uint8_t* block, int lo_bytes, int first, int lane) const {
+    const int c = (lane & 15) * 4;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int row = first + (lane >> 4) + 2 * i;
+      uint8_t* dst = block + row * 128 + (((c >> 3) ^ (row & 7)) << 4) + (c & 4) * 2;
+      const __nv_bfloat162 h0 = __floats2bfloat162_rn(v[i].x, v[i].y), h1 = __floats2bfloat162_rn(v[i].z, v[i].w);
+      const __nv_bfloat162 l0 = __floats2bfloat162_rn(v[i].x - __bfloat162float(h0.x), v[i].y - __bfloat162float(h0.y));
+      const __nv_bfloat162 l1 = __floats2bfloat162_rn(v[i].z - __bfloat162float(h1.x), v[i].w - __bfloat162float(h1.y));
+      *reinterpret_cast<uint2*>(dst) = make_uint2(*reinterpret_cast<const uint32_t*>(&h0), *reinterpret_cast<const uint32_t*>(&h1));
+      *reinterpret_cast<uint2*>(dst + lo_bytes) = make_uint2(*reinterpret_cast<const uint32_t*>(&l0), *reinterpret_cast<const uint32_t*>(&l1));
+    }
+  }
+};
+template <> struct GpRows<kSrcBf16> {
+  uint32_t v[32];
+  bool vec;
+  __device__ __forceinline__ void load(const void* base, long long at, long long ld, int left, long long rows, bool by_vector, int lane) {
+    const unsigned short* p = static_cast<const unsigned short*>(base) + at;
+    vec = by_vector;
+    if (vec) {
+      const int r0 = lane >> 4, c = (lane & 15) * 4;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const bool in = r0 + 2 * i < rows && c < left;         // widths are multiples of four here
+        const uint2 w = in ? __ldg(reinterpret_cast<const uint2*>(p + (r0 + 2 * i) * ld + c)) : make_uint2(0u, 0u);
+        v[2 * i] = w.x; v[2 * i + 1] = w.y;
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < 32; ++i) {
+        const int r = i >> 1, c = (i & 1) * 32 + lane;
+        v[i] = r < rows && c < left ? __ldg(p + r * ld + c) : 0u;
+      }
+    }
+  }
+  __device__ __forceinline__ void store(uint8_t* block, int, int first, int lane) const {
+#pragma unroll
+    for (int i = 0; i < 32; ++i) {
+      if (vec && i >= 8) break;
+      const int row = vec ? first + (lane >> 4) + 2 * i : first + (i >> 1), c = vec ? (lane & 15) * 4 : (i & 1) * 32 + lane;
+      uint8_t* dst = block + row * 128 + (((c >> 3) ^ (row & 7)) << 4) + (c & 7) * 2;
+      if (vec) *reinterpret_cast<uint2*>(dst) = make_uint2(v[(2 * i) & 31], v[(2 * i + 1) & 31]);
+      else *reinterpret_cast<unsigned short*>(dst) = static_cast<unsigned short>(v[i]);
+    }
+  }
+};
+
+__device__ __forceinline__ float4 gp_ld_cluster(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+  return v;
+}
+
+template <int KMAX, int kSrc, bool kEmb, bool kCluster>
+__global__ void __launch_bounds__(kSrc == kSrcTma ? 192 : 448, 1)
 gradproj_kernel(const __grid_constant__ CUtensorMap tm_g, const __grid_constant__ CUtensorMap tm_pr,
                 const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_pc,
                 const GpParams p) {
-  using Cfg = GpCfg<KMAX>;
+  using Cfg = GpCfg<KMAX, kSrc, kCluster>;
   constexpr int BM = Cfg::BM, BK = Cfg::BK, kStages = Cfg::kStages, RT = Cfg::RT, CT = Cfg::CT;
-  constexpr int ATOMS = Cfg::ATOMS;
+  constexpr int ATOMS = Cfg::ATOMS, PARTS = Cfg::PARTS;
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  float* s_r = reinterpret_cast<float*>(smem + kStages * Cfg::kStageBytes);   // [64][KMAX]
-  float* s_c = s_r + Cfg::kStageRows * KMAX;                                  // [64][KMAX]
+  float* s_r = reinterpret_cast<float*>(smem + kStages * Cfg::kStageBytes);   // [kStageRows][KMAX]
+  float* s_c = s_r + Cfg::kStageRows * KMAX;                                  // [kStageRows][KMAX]
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kStages * Cfg::kStageBytes + Cfg::kProjBytes);
   uint64_t* full_bar = bars;
   uint64_t* empty_bar = bars + kStages;
@@ -95,23 +195,37 @@ gradproj_kernel(const __grid_constant__ CUtensorMap tm_g, const __grid_constant_
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const long long bx = blockIdx.x;
-  const long long u0 = bx * p.units_per_cta + (bx < p.units_extra ? bx : p.units_extra);
-  long long u1 = u0 + p.units_per_cta + (bx < p.units_extra ? 1 : 0);
-  if (u1 > p.units) u1 = p.units;
   const int kb_r = (p.n_r + ATOMS * BK - 1) / (ATOMS * BK);            // pipeline stages over G's columns
   const int kb_total = kEmb ? kb_r : kb_r + (p.n_c + ATOMS * BK - 1) / (ATOMS * BK);
+  // units of this CTA and its stages [kb0, kb1) of each: all of them, or in a cluster (one unit) its rank's share
+  long long u0, u1;
+  int kb0 = 0, kb1 = kb_total;
+  uint32_t rank = 0, ranks = 1;
+  if constexpr (kCluster) {
+    rank = cluster_ctarank();
+    asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(ranks));
+    u0 = blockIdx.x / ranks;
+    u1 = u0 + 1;
+    kb0 = static_cast<int>(rank * kb_total / ranks);
+    kb1 = static_cast<int>((rank + 1) * kb_total / ranks);
+  } else {
+    const long long bx = blockIdx.x;
+    u0 = bx * p.units_per_cta + (bx < p.units_extra ? bx : p.units_extra);
+    u1 = u0 + p.units_per_cta + (bx < p.units_extra ? 1 : 0);
+    if (u1 > p.units) u1 = p.units;
+  }
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < kStages; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
+    for (int s = 0; s < kStages; ++s) { mbar_init(&full_bar[s], kSrc == kSrcTma ? 1 : 9); mbar_init(&empty_bar[s], 1); }
     for (int a = 0; a < 2; ++a) { mbar_init(&acc_full[a], 1); mbar_init(&acc_empty[a], 4); }
     *abort_flag = 0;
     fence_barrier_init();
   }
   if (warp == 5) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
   if (warp == 4 && lane == 0) {
-    tma_prefetch_desc(&tm_g); tma_prefetch_desc(&tm_pr);
-    if (!kEmb) { tma_prefetch_desc(&tm_a); tma_prefetch_desc(&tm_pc); }
+    tma_prefetch_desc(&tm_pr);
+    if (!kEmb) tma_prefetch_desc(&tm_pc);
+    if (kSrc == kSrcTma) { tma_prefetch_desc(&tm_g); if (!kEmb) tma_prefetch_desc(&tm_a); }
   }
   tc_fence_before_sync();
   __syncthreads();
@@ -119,33 +233,87 @@ gradproj_kernel(const __grid_constant__ CUtensorMap tm_g, const __grid_constant_
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 4) {
-    // Producer warp.  Lane 0 owns the barriers; lanes [0, ATOMS) each issue the TMA of one
-    // activation atom and lanes [ATOMS, 2*ATOMS) the TMA of one projection atom -- one warp
-    // instruction per stage instead of one thread issuing the boxes back to back.
-    const bool is_p = lane >= ATOMS;
-    const int atom = is_p ? lane - ATOMS : lane;
-    const uint32_t dst_off = is_p ? ATOMS * Cfg::kActAtomBytes + atom * Cfg::kProjAtomBytes
-                                  : atom * Cfg::kActAtomBytes;
+    // Producer warp.  Lane 0 owns the barriers; each of the first lanes issues the TMA of one box -- activation
+    // atoms (kSrcTma), then projection atoms or, of float32 operands, the two parts of the one atom -- in one
+    // warp instruction per stage instead of one thread issuing the boxes back to back.
+    constexpr int kActBoxes = kSrc == kSrcTma ? ATOMS : 0, kProjBoxes = ATOMS * PARTS;
+    const bool is_p = lane >= kActBoxes;
+    const int box = is_p ? lane - kActBoxes : lane;
+    const uint32_t dst_off = is_p ? ATOMS * PARTS * Cfg::kActAtomBytes + box * Cfg::kProjAtomBytes
+                                  : box * Cfg::kActAtomBytes;
     int stage = 0; uint32_t phase = 0; bool ok = true;
     for (long long u = u0; u < u1 && ok; ++u) {
       const int b = static_cast<int>(u / p.chunks_per_sample);
       const int row0 = static_cast<int>(u % p.chunks_per_sample) * BM;
-      for (int kb = 0; kb < kb_total; ++kb) {
+      for (int kb = kb0; kb < kb1; ++kb) {
         int w = 1;
         if (lane == 0) w = mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag, p.err, 421) ? 1 : 0;
         w = __shfl_sync(0xffffffffu, w, 0);
         if (!w) { ok = false; break; }
         const bool first = kb < kb_r;
-        if (lane == 0)
-          mbar_arrive_expect_tx(&full_bar[stage], ATOMS * (BM + (first ? p.kr_pad : p.kc_pad)) * BK * 2);
-        if (lane < 2 * ATOMS) {
-          // an atom past the last column starts out of range and is zero-filled
-          const int col = ((first ? kb : kb - kb_r) * ATOMS + atom) * BK;
+        const int kpad = first ? p.kr_pad : p.kc_pad;
+        if (lane == 0) mbar_arrive_expect_tx(&full_bar[stage], (kActBoxes * BM + kProjBoxes * kpad) * BK * 2);
+        __syncwarp();
+        if (lane < kActBoxes + kProjBoxes) {
+          // an atom past the last column starts out of range and is zero-filled; what a residual box reads beyond
+          // its part meets zeros of the operand
+          int col = (first ? kb : kb - kb_r) * ATOMS * BK;
+          if (kSrc == kSrcF32) col += box == 0 ? 0 : (first ? p.lo_r : p.lo_c);
+          else col += box * BK;
           const CUtensorMap* m = first ? (is_p ? &tm_pr : &tm_g) : (is_p ? &tm_pc : &tm_a);
           tma_load_3d(smem + stage * Cfg::kStageBytes + dst_off, m, &full_bar[stage], col,
                       is_p ? 0 : row0, is_p ? 0 : b);
         }
         if (++stage == kStages) { stage = 0; phase ^= 1; }
+      }
+    }
+  } else if (kSrc != kSrcTma && warp >= 6) {
+    // Loader warps: 16 rows of a unit each.  The loads of the next stage are in flight while a stage is converted
+    // and stored: two register sets.
+    if constexpr (kSrc != kSrcTma) {
+      const int lw = warp - 6;
+      GpRows<kSrc> set[2];
+      long long row = 0, rows_left = 0;                  // of the unit being fetched: this warp's first row, rows from there on
+      auto fetch = [&](int kb, GpRows<kSrc>& q) {
+        const bool first = kb < kb_r;
+        const int col = (first ? kb : kb - kb_r) * BK;
+        const long long ld = first ? p.ldg : p.lda;
+        q.load(first ? p.g : p.a, row * ld + col, ld, (first ? p.n_r : p.n_c) - col, rows_left, first ? p.vec_g : p.vec_a, lane);
+      };
+      int stage = 0; uint32_t phase = 0;
+      auto put = [&](const GpRows<kSrc>& q) -> bool {
+        int w = 1;
+        if (lane == 0) w = mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag, p.err, 621) ? 1 : 0;
+        w = __shfl_sync(0xffffffffu, w, 0);
+        __syncwarp();
+        if (!w) return false;
+        q.store(smem + stage * Cfg::kStageBytes, Cfg::kActAtomBytes, lw * 16, lane);
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&full_bar[stage]);
+        if (++stage == kStages) { stage = 0; phase ^= 1; }
+        return true;
+      };
+      const long long n = (u1 - u0) * (kb1 - kb0);       // this CTA's stages
+      long long fu = u0;
+      int fk = kb0;
+      auto advance = [&](GpRows<kSrc>& q) {
+        if (fu >= u1) return;
+        if (fk == kb0) {
+          const long long b = fu / p.chunks_per_sample, t0 = (fu - b * p.chunks_per_sample) * BM + lw * 16;
+          row = b * p.T + t0;
+          rows_left = p.T - t0;
+        }
+        fetch(fk, q);
+        if (++fk == kb1) { fk = kb0; ++fu; }
+      };
+      if (n > 0) advance(set[0]);
+      for (long long i = 0; i < n; i += 2) {
+        advance(set[1]);
+        if (!put(set[0])) break;
+        if (i + 1 >= n) break;
+        advance(set[0]);
+        if (!put(set[1])) break;
       }
     }
   } else if (warp == 5) {
@@ -158,21 +326,29 @@ gradproj_kernel(const __grid_constant__ CUtensorMap tm_g, const __grid_constant_
         tc_fence_after_sync();
         const uint32_t d_r = tmem_base + acc * 256;
         const uint32_t d_c = d_r + 128;
-        for (int kb = 0; kb < kb_total; ++kb) {
+        for (int kb = kb0; kb < kb1; ++kb) {
           if (!mbar_wait(&full_bar[stage], phase, abort_flag, p.err, 523)) { ok = false; break; }
           tc_fence_after_sync();
           const uint32_t sa = smem_u32(smem + stage * Cfg::kStageBytes);
           const bool first = kb < kb_r;
-          const bool fresh = (kb == 0) || (kb == kb_r);
+          const bool fresh = (kb == kb0) || (kb == kb_r);
           const uint32_t d = first ? d_r : d_c;
           const uint32_t idesc = first ? idesc_r : idesc_c;
 #pragma unroll
           for (int at = 0; at < ATOMS; ++at) {
             const uint64_t adesc = make_smem_desc_sw128(sa + at * Cfg::kActAtomBytes, 16, 1024);
-            const uint64_t bdesc = make_smem_desc_sw128(sa + ATOMS * Cfg::kActAtomBytes + at * Cfg::kProjAtomBytes, 16, 1024);
+            const uint64_t bdesc = make_smem_desc_sw128(sa + ATOMS * PARTS * Cfg::kActAtomBytes + at * Cfg::kProjAtomBytes, 16, 1024);
 #pragma unroll
-            for (int k = 0; k < BK / 16; ++k)
-              umma_bf16(d, adesc + 2 * k, bdesc + 2 * k, idesc, (fresh && at == 0 && k == 0) ? 0u : 1u);
+            for (int k = 0; k < BK / 16; ++k) {
+              const uint32_t add = (fresh && at == 0 && k == 0) ? 0u : 1u;
+              if constexpr (PARTS == 2) {      // residual parts lie behind the values
+                umma_bf16(d, adesc + 2 * k + Cfg::kActAtomBytes / 16, bdesc + 2 * k, idesc, add);
+                umma_bf16(d, adesc + 2 * k, bdesc + 2 * k + Cfg::kProjAtomBytes / 16, idesc, 1u);
+                umma_bf16(d, adesc + 2 * k, bdesc + 2 * k, idesc, 1u);
+              } else {
+                umma_bf16(d, adesc + 2 * k, bdesc + 2 * k, idesc, add);
+              }
+            }
           }
           umma_commit(&empty_bar[stage]);
           if (++stage == kStages) { stage = 0; phase ^= 1; }
@@ -218,7 +394,7 @@ gradproj_kernel(const __grid_constant__ CUtensorMap tm_g, const __grid_constant_
 #pragma unroll
         for (int j = 0; j < 32; j += 4)
           if (c0 + j < KMAX)
-            *reinterpret_cast<float4*>(&dst[gp_staged_index<KMAX>(tid & 63, c0 + j)]) =
+            *reinterpret_cast<float4*>(&dst[gp_staged_index<KMAX>(tid & (Cfg::kStageRows - 1), c0 + j)]) =
                 make_float4(__uint_as_float(r[j]), __uint_as_float(r[j + 1]), __uint_as_float(r[j + 2]), __uint_as_float(r[j + 3]));
       }
     };
@@ -249,8 +425,78 @@ gradproj_kernel(const __grid_constant__ CUtensorMap tm_g, const __grid_constant_
       }
     };
 
+    // out[r, c] += sum over staged rows [t0, t1) of s_r[t][r] * s_c[t][c]
+    auto contract = [&](int t0, int t1) {
+#pragma unroll 4
+      for (int t = t0; t < t1; ++t) {
+        float rr[RT], cc[CT];
+        if constexpr (RT >= 4) {
+#pragma unroll
+          for (int i = 0; i < RT; i += 4)
+            *reinterpret_cast<float4*>(&rr[i]) = *reinterpret_cast<const float4*>(&s_r[gp_staged_index<KMAX>(t, ty * RT + i)]);
+        } else {
+          *reinterpret_cast<float2*>(&rr[0]) = *reinterpret_cast<const float2*>(&s_r[gp_staged_index<KMAX>(t, ty * RT)]);
+        }
+#pragma unroll
+        for (int j = 0; j < CT; j += 4)
+          *reinterpret_cast<float4*>(&cc[j]) = *reinterpret_cast<const float4*>(&s_c[gp_staged_index<KMAX>(t, tx * CT + j)]);
+#pragma unroll
+        for (int i = 0; i < RT; ++i)
+#pragma unroll
+          for (int j = 0; j < CT; ++j) o[i][j] = fmaf(rr[i], cc[j], o[i][j]);
+      }
+    };
+
+    if constexpr (kCluster) {
+      // One unit.  Row `tid` of this CTA's partial blocks is staged; rows [first, first + share) of all CTAs' blocks are
+      // then added up here, in place: nobody else reads them from this CTA.
+      const int share = BM / static_cast<int>(ranks), first = static_cast<int>(rank) * share;
+      const int b = static_cast<int>(u0 / p.chunks_per_sample);
+      const long long t_first = u0 % p.chunks_per_sample * BM;
+      const bool owned = tid >= first && tid < first + share;
+      if constexpr (kEmb) { if (owned) gather(b, t_first + tid); }
+      bool alive = true;
+      if (kb1 > kb0) alive = named_bar_and(2, 128, mbar_wait(&acc_full[0], 0, abort_flag, p.err, 124));
+      if (alive) {
+        tc_fence_after_sync();
+        const uint32_t t_r = tmem_base + lane_base;
+        if (kb0 < kb_r && kb0 < kb1) stage_block(t_r, p.kr_pad, s_r);
+        if (!kEmb && kb1 > kb_r) stage_block(t_r + 128, p.kc_pad, s_c);
+        if constexpr (kEmb) {
+          if (owned)
+#pragma unroll
+            for (int q = 0; q < kRowQuads; ++q) *reinterpret_cast<float4*>(&s_c[gp_staged_index<KMAX>(tid, 4 * q)]) = mine[q];
+        }
+      }
+      __syncwarp();
+      cluster_sync_all();
+      if (alive) {
+        // ranks [0, last_r] hold columns of G, [first_c, ranks) columns of A
+        auto begin = [&](int r) { return static_cast<int>(static_cast<unsigned>(r) * kb_total / ranks); };
+        auto add_up = [&](float* block, int kpad, bool of_r) {
+          const int quads = kpad / 4;
+          for (int i = tid; i < share * quads; i += 128) {
+            float* at = &block[gp_staged_index<KMAX>(first + i / quads, i % quads * 4)];
+            float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+            for (int r = 0; r < static_cast<int>(ranks); ++r) {
+              const int s0 = begin(r), s1 = begin(r + 1);
+              if (s0 == s1 || (of_r ? s0 >= kb_r : s1 <= kb_r)) continue;
+              const float4 v = gp_ld_cluster(map_to_cta(smem_u32(at), r));
+              sum.x += v.x; sum.y += v.y; sum.z += v.z; sum.w += v.w;
+            }
+            *reinterpret_cast<float4*>(at) = sum;
+          }
+        };
+        add_up(s_r, p.kr_pad, true);
+        if (!kEmb) add_up(s_c, p.kc_pad, false);
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+        contract(first, first + share);
+        flush(b);
+      }
+    }
     bool alive = true;
-    for (long long u = u0; u < u1; ++u) {
+    for (long long u = u0; u < u1 && !kCluster; ++u) {
       const int b = static_cast<int>(u / p.chunks_per_sample);
       if (b != cur_b) { if (cur_b >= 0) flush(cur_b); cur_b = b; }
       if constexpr (kEmb) gather(b, u % p.chunks_per_sample * BM + tid);
@@ -274,25 +520,7 @@ gradproj_kernel(const __grid_constant__ CUtensorMap tm_g, const __grid_constant_
           if (lane == 0) mbar_arrive(&acc_empty[acc]);     // four arrivals per tile, one per warp
         }
         asm volatile("bar.sync 1, 128;" ::: "memory");     // the four epilogue warps only
-        // out[r, c] += sum_t s_r[t][r] * s_c[t][c]
-#pragma unroll 4
-        for (int t = 0; t < Cfg::kStageRows; ++t) {
-          float rr[RT], cc[CT];
-          if constexpr (RT >= 4) {
-#pragma unroll
-            for (int i = 0; i < RT; i += 4)
-              *reinterpret_cast<float4*>(&rr[i]) = *reinterpret_cast<const float4*>(&s_r[gp_staged_index<KMAX>(t, ty * RT + i)]);
-          } else {
-            *reinterpret_cast<float2*>(&rr[0]) = *reinterpret_cast<const float2*>(&s_r[gp_staged_index<KMAX>(t, ty * RT)]);
-          }
-#pragma unroll
-          for (int j = 0; j < CT; j += 4)
-            *reinterpret_cast<float4*>(&cc[j]) = *reinterpret_cast<const float4*>(&s_c[gp_staged_index<KMAX>(t, tx * CT + j)]);
-#pragma unroll
-          for (int i = 0; i < RT; ++i)
-#pragma unroll
-            for (int j = 0; j < CT; ++j) o[i][j] = fmaf(rr[i], cc[j], o[i][j]);
-        }
+        contract(0, Cfg::kStageRows);
         asm volatile("bar.sync 1, 128;" ::: "memory");
       }
       if (++acc == 2) { acc = 0; acc_phase ^= 1; }
@@ -300,56 +528,141 @@ gradproj_kernel(const __grid_constant__ CUtensorMap tm_g, const __grid_constant_
     if (alive && cur_b >= 0) flush(cur_b);
   }
 
+  if constexpr (kCluster) {
+    __syncwarp();
+    if (warp >= 4) cluster_sync_all();     // the epilogue's barrier before the partial blocks are added up
+    cluster_sync_all();                    // no CTA leaves while another reads its blocks
+  }
   tc_fence_before_sync();
   __syncthreads();
   if (warp == 5) { tc_fence_after_sync(); tmem_dealloc(tmem_base, 512); }
 }
 
-template <int KMAX, bool kEmb>
-static int launch_gradproj(const CUtensorMap& tg, const CUtensorMap& tpr, const CUtensorMap& ta,
-                           const CUtensorMap& tpc, GpParams& p, const DeviceState* ds, cudaStream_t st) {
-  using Cfg = GpCfg<KMAX>;
+template <int KMAX, int kSrc, bool kEmb, bool kCluster>
+static int launch_gradproj_t(const CUtensorMap& tg, const CUtensorMap& tpr, const CUtensorMap& ta, const CUtensorMap& tpc,
+                             GpParams& p, int ranks, const DeviceState* ds, cudaStream_t st) {
+  using Cfg = GpCfg<KMAX, kSrc, kCluster>;
   static bool attr_set[64] = {};
   if (!attr_set[ds->device]) {
-    GB_CUDA_OK(cudaFuncSetAttribute(gradproj_kernel<KMAX, kEmb>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes));
+    GB_CUDA_OK(cudaFuncSetAttribute(gradproj_kernel<KMAX, kSrc, kEmb, kCluster>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    Cfg::kSmemBytes));
     attr_set[ds->device] = true;
   }
-  const int grid = static_cast<int>(p.units < ds->sm_count ? p.units : ds->sm_count);
-  p.units_per_cta = static_cast<int>(p.units / grid);
-  p.units_extra = static_cast<int>(p.units % grid);
-  gradproj_kernel<KMAX, kEmb><<<grid, 192, Cfg::kSmemBytes, st>>>(tg, tpr, ta, tpc, p);
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr;
+  cfg.blockDim = dim3(Cfg::kThreads, 1, 1);
+  cfg.dynamicSmemBytes = Cfg::kSmemBytes;
+  cfg.stream = st;
+  if (kCluster) {
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = ranks;
+    attr.val.clusterDim.y = 1;
+    attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    cfg.gridDim = dim3(static_cast<unsigned>(p.units * ranks), 1, 1);
+  } else {
+    const int grid = static_cast<int>(p.units < ds->sm_count ? p.units : ds->sm_count);
+    p.units_per_cta = static_cast<int>(p.units / grid);
+    p.units_extra = static_cast<int>(p.units % grid);
+    cfg.gridDim = dim3(grid, 1, 1);
+  }
+  GB_CUDA_OK(cudaLaunchKernelEx(&cfg, gradproj_kernel<KMAX, kSrc, kEmb, kCluster>, tg, tpr, ta, tpc, p));
   count_launch();
   return post_launch("gradproj_kernel");
 }
 
-// The embedding form for bf16 rows that TMA can read (proj_extras.cu holds the entry point and the
-// kernel for the rest).  16 x 2048 tokens of 1024 features, k = 32: bound by streaming G once.
-int launch_gradproj_embedding(const long long* ids, const void* G, int B, long long T, int d, long long ldg, const void* P_o,
-                              long long ldp_o, const float* P_i_t, long long ld_pit, int vocab, int k_o, int k_i, float scale,
-                              float* out, long long out_stride, int out_ld, const DeviceState* ds, cudaStream_t st) {
-  GpParams p = {};
-  p.B = B; p.T = T; p.n_r = d; p.n_c = 0; p.k_r = k_o; p.k_c = k_i;
-  p.kr_pad = (k_o + 15) / 16 * 16;
-  p.kc_pad = (k_i + 15) / 16 * 16;
-  p.chunks_per_sample = ceil_div(T, 128);
-  p.units = static_cast<long long>(B) * p.chunks_per_sample;
-  p.scale = scale;
-  p.out = out; p.out_stride = out_stride; p.out_ld = out_ld;
-  p.ids = ids; p.rows = P_i_t; p.ld_rows = ld_pit; p.vocab = vocab;
-  p.rows_vec = k_i % 4 == 0 && ld_pit % 4 == 0 && (reinterpret_cast<uintptr_t>(P_i_t) & 15u) == 0;
-  p.err = ds->err_word;
-  CUtensorMap tg, tp;
+// CTAs that share a unit: as many as keep the GPU's SMs busy with one unit per cluster.  A GPC has 16 to 20 SMs, so about
+// 16 clusters of eight and 34 of four are resident at once.  The cluster's two barriers and the exchange cost about
+// 2 us; a stage is 0.5 us of a unit's chain, and the contraction of 128 tokens, which the CTAs share too, 3 us at
+// 64 x 64 and 1 us at 32 x 32 (32 x 64 tokens of 256 + 256 columns, four stages, k = 32: 10.3 us alone, 11.3 in pairs;
+// 12 x 1 token of 128 + 2112, k = 44: 23.6 and 13.1 in eights).
+static int gradproj_ranks(long long units, int stages, int kmax) {
+  if (stages < 8 && kmax <= 32) return 1;
+  return units <= 16 ? 8 : units <= 34 ? 4 : units <= 74 ? 2 : 1;
+}
+
+// Operands of one projection as the entry points get them.
+struct GpOperands {
+  const void *G, *A;               // A null: the embedding form
+  int is_f32;
+  long long ldg, lda;
+  const void *P_r, *P_c;
+  long long ldpr, ldpc;
+  int pr_cols, pc_cols;            // columns of the P matrices that belong to the operand's (padded) columns
+};
+
+template <int KMAX, int kSrc, bool kEmb>
+static int launch_gradproj_src(const GpOperands& o, GpParams& p, const DeviceState* ds, cudaStream_t st) {
+  CUtensorMap tg = {}, tpr, ta = {}, tpc = {};
   int rc;
-  if ((rc = make_tmap_bf16_3d(&tg, G, B, T, d, ldg, 128)) != GHOST_OK) return rc;
-  if ((rc = make_tmap_bf16_3d(&tp, P_o, 1, k_o, d, ldp_o, p.kr_pad)) != GHOST_OK) return rc;
+  // the projection matrices as one-sample 3-D operands, so that one TMA instruction form serves all four
+  if ((rc = make_tmap_bf16_3d(&tpr, o.P_r, 1, p.k_r, o.pr_cols, o.ldpr, p.kr_pad)) != GHOST_OK) return rc;
+  if (!kEmb && (rc = make_tmap_bf16_3d(&tpc, o.P_c, 1, p.k_c, o.pc_cols, o.ldpc, p.kc_pad)) != GHOST_OK) return rc;
+  if (kSrc == kSrcTma) {
+    if ((rc = make_tmap_bf16_3d(&tg, o.G, p.B, p.T, p.n_r, o.ldg, 128)) != GHOST_OK) return rc;
+    if (!kEmb && (rc = make_tmap_bf16_3d(&ta, o.A, p.B, p.T, p.n_c, o.lda, 128)) != GHOST_OK) return rc;
+  }
+  constexpr int kCols = GpCfg<KMAX, kSrc, false>::ATOMS * 64;
+  const int stages = ceil_div(p.n_r, kCols) + (kEmb ? 0 : ceil_div(p.n_c, kCols));
+  const int ranks = gradproj_ranks(p.units, stages, KMAX);
+  if (ranks > 1) return launch_gradproj_t<KMAX, kSrc, kEmb, true>(tg, tpr, ta, tpc, p, ranks, ds, st);
+  return launch_gradproj_t<KMAX, kSrc, kEmb, false>(tg, tpr, ta, tpc, p, 1, ds, st);
+}
+
+template <int kSrc, bool kEmb>
+static int launch_gradproj_k(const GpOperands& o, GpParams& p, const DeviceState* ds, cudaStream_t st) {
   const int kmax = p.kr_pad > p.kc_pad ? p.kr_pad : p.kc_pad;
-  if (kmax <= 32) return launch_gradproj<32, true>(tg, tp, tg, tp, p, ds, st);
-  return launch_gradproj<64, true>(tg, tp, tg, tp, p, ds, st);
+  if (kmax <= 32) return launch_gradproj_src<32, kSrc, kEmb>(o, p, ds, st);
+  if constexpr (!kEmb && kSrc == kSrcTma) { if (kmax > 64) return launch_gradproj_src<128, kSrc, kEmb>(o, p, ds, st); }
+  return launch_gradproj_src<64, kSrc, kEmb>(o, p, ds, st);
+}
+
+// Chooses how the rows are read: bf16 through TMA where it can, else through registers
+template <bool kEmb>
+static int launch_gradproj(const GpOperands& o, GpParams& p, const DeviceState* ds, cudaStream_t st) {
+  p.kr_pad = (p.k_r + 15) / 16 * 16;
+  p.kc_pad = (p.k_c + 15) / 16 * 16;
+  const long long chunks = (p.T + 127) / 128;
+  GB_REQUIRE(chunks < (1ll << 31) && chunks * p.B < (1ll << 31) * 128, "gradproj: too many tokens");
+  p.chunks_per_sample = static_cast<int>(chunks);
+  p.units = chunks * p.B;
+  p.g = o.G; p.a = o.A; p.ldg = o.ldg; p.lda = o.lda;
+  p.err = ds->err_word;
+  auto aligned = [](const void* x, long long ld, long long bytes, long long elem) {
+    return (reinterpret_cast<uintptr_t>(x) % bytes) == 0 && ld * elem % bytes == 0;
+  };
+  if (o.is_f32) {
+    p.vec_g = aligned(o.G, o.ldg, 16, 4) && p.n_r % 4 == 0;
+    p.vec_a = aligned(o.A, o.lda, 16, 4) && p.n_c % 4 == 0;
+    return launch_gradproj_k<kSrcF32, kEmb>(o, p, ds, st);
+  }
+  if (aligned(o.G, o.ldg, 16, 2) && (kEmb || aligned(o.A, o.lda, 16, 2)) && p.T < (1ll << 31) - 128)
+    return launch_gradproj_k<kSrcTma, kEmb>(o, p, ds, st);
+  p.vec_g = aligned(o.G, o.ldg, 8, 2) && p.n_r % 4 == 0;
+  p.vec_a = aligned(o.A, o.lda, 8, 2) && p.n_c % 4 == 0;
+  return launch_gradproj_k<kSrcBf16, kEmb>(o, p, ds, st);
 }
 
 }  // namespace gb
 
 using namespace gb;
+
+static int gradproj_dense(const GpOperands& o, GpParams& p, long long out_stride, void* stream) {
+  const DeviceState* ds = device_state();
+  if (!ds) return GHOST_ERR_DEVICE;
+  GB_REQUIRE(o.G && o.A && o.P_r && o.P_c && p.out, "ghost_gradproj_dense_bf16: null pointer");
+  GB_REQUIRE(p.B > 0 && p.T > 0 && p.n_r > 0 && p.n_c > 0 && p.k_r > 0 && p.k_c > 0, "ghost_gradproj_dense_bf16: empty dimension");
+  GB_REQUIRE(p.k_r <= 128 && p.k_c <= 128, "ghost_gradproj_dense_bf16: projection ranks above 128 are not supported");
+  GB_REQUIRE(out_stride >= static_cast<long long>(p.k_r) * p.k_c, "ghost_gradproj_dense_bf16: out_stride smaller than k_r * k_c");
+  GB_REQUIRE(p.T < (1ll << 31) - 128, "ghost_gradproj_dense_bf16: T too large");
+  GB_REQUIRE(o.ldg >= p.n_r && o.lda >= p.n_c, "ghost_gradproj_dense_bf16: pitch smaller than the row it holds");
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  p.out_stride = out_stride;
+  p.out_ld = p.k_c;
+  GB_CUDA_OK(cudaMemset2DAsync(p.out, out_stride * sizeof(float), 0, static_cast<size_t>(p.k_r) * p.k_c * sizeof(float), p.B, st));
+  return launch_gradproj<false>(o, p, ds, st);
+}
 
 // G: [B, T, n_r] bf16 (pitch ldg), A: [B, T, n_c] bf16 (pitch lda), P_r: [k_r, n_r] bf16 (pitch ldpr),
 // P_c: [k_c, n_c] bf16 (pitch ldpc).  out + b * out_stride receives [k_r, k_c] fp32 (overwritten).
@@ -357,35 +670,63 @@ extern "C" int ghost_gradproj_dense_bf16(const void* G, const void* A, int B, lo
                                          long long ldg, long long lda, const void* P_r, const void* P_c,
                                          int k_r, int k_c, long long ldpr, long long ldpc, float scale,
                                          float* out, long long out_stride, void* stream) {
+  GB_REQUIRE(((reinterpret_cast<uintptr_t>(G) | reinterpret_cast<uintptr_t>(A)) & 15u) == 0 && ldg % 8 == 0 && lda % 8 == 0,
+             "ghost_gradproj_dense_bf16: operands must be 16-byte aligned with pitches that are multiples of 8");
+  GpParams p = {};
+  p.B = B; p.T = T; p.n_r = n_r; p.n_c = n_c; p.k_r = k_r; p.k_c = k_c; p.scale = scale; p.out = out;
+  const GpOperands o = {G, A, 0, ldg, lda, P_r, P_c, ldpr, ldpc, n_r, n_c};
+  return gradproj_dense(o, p, out_stride, stream);
+}
+
+extern "C" int ghost_gradproj_dense(const void* G, const void* A, int is_f32, int B, long long T, int n_r, int n_c, long long ldg,
+                                    long long lda, const void* P_r, const void* P_c, int k_r, int k_c, long long ldpr,
+                                    long long ldpc, int lo_r, int lo_c, float scale, float* out, long long out_stride,
+                                    void* stream) {
+  GB_REQUIRE(n_r <= ldpr && n_c <= ldpc && ldpr % 8 == 0 && ldpc % 8 == 0, "ghost_gradproj_dense: bad layout of the projection matrices");
+  GB_REQUIRE(!is_f32 || (lo_r % 8 == 0 && lo_c % 8 == 0 && lo_r >= n_r && lo_c >= n_c && lo_r + n_r <= ldpr && lo_c + n_c <= ldpc),
+             "ghost_gradproj_dense: float32 operands need the residual parts of the projection matrices inside their rows");
+  GpParams p = {};
+  p.B = B; p.T = T; p.n_r = n_r; p.n_c = n_c; p.k_r = k_r; p.k_c = k_c; p.scale = scale; p.out = out;
+  p.lo_r = lo_r; p.lo_c = lo_c;
+  // The loaders' threads leave the epilogue 128 registers, which a block of 128 x 128 does not fit: 32 x 2048 tokens of
+  // 1024 + 1024 float32 took 639 us against 462 for copies of the operands in three parts.
+  GB_REQUIRE(k_r <= 64 && k_c <= 64, "ghost_gradproj_dense: projection ranks above 64 are left to ghost_gradproj_dense_bf16");
+  const GpOperands o = {G, A, is_f32, ldg, lda, P_r, P_c, ldpr, ldpc, static_cast<int>(ldpr), static_cast<int>(ldpc)};
+  return gradproj_dense(o, p, out_stride, stream);
+}
+
+extern "C" int ghost_gradproj_embedding(const long long* ids, const void* G, int g_is_f32, int B, long long T,
+                                        int d, long long ldg, const void* P_o, long long ldp_o, int p_cols,
+                                        int p_lo_offset, const float* P_i_t, long long ld_pit, int vocab, int k_o,
+                                        int k_i, float scale, int accumulate, float* out, long long out_stride,
+                                        int out_ld, void* stream) {
   const DeviceState* ds = device_state();
   if (!ds) return GHOST_ERR_DEVICE;
-  GB_REQUIRE(G && A && P_r && P_c && out, "ghost_gradproj_dense_bf16: null pointer");
-  GB_REQUIRE(B > 0 && T > 0 && n_r > 0 && n_c > 0 && k_r > 0 && k_c > 0, "ghost_gradproj_dense_bf16: empty dimension");
-  GB_REQUIRE(k_r <= 128 && k_c <= 128, "ghost_gradproj_dense_bf16: projection ranks above 128 are not supported");
-  GB_REQUIRE(out_stride >= static_cast<long long>(k_r) * k_c, "ghost_gradproj_dense_bf16: out_stride smaller than k_r * k_c");
-  GB_REQUIRE(T < (1ll << 31) - 128, "ghost_gradproj_dense_bf16: T too large");
+  GB_REQUIRE(ids && G && P_o && P_i_t && out, "ghost_gradproj_embedding: null pointer");
+  GB_REQUIRE(B > 0 && T > 0 && d > 0 && vocab > 0, "ghost_gradproj_embedding: empty dimension");
+  GB_REQUIRE(k_o >= 1 && k_o <= 64 && k_i >= 1 && k_i <= 64,
+             "ghost_gradproj_embedding: k_o and k_i must be between 1 and 64 (got %d, %d)", k_o, k_i);
+  GB_REQUIRE(ldg >= d && ld_pit >= k_i && out_ld >= k_i &&
+                 out_stride >= static_cast<long long>(k_o - 1) * out_ld + k_i,
+             "ghost_gradproj_embedding: pitch smaller than the row it holds");
+  GB_REQUIRE(accumulate || out_ld == k_i,
+             "ghost_gradproj_embedding: a block inside wider rows (out_ld > k_i) must be zeroed by the caller "
+             "and passed with accumulate = 1");
+  GB_REQUIRE(p_cols >= d && p_cols % 8 == 0 && ldp_o % 8 == 0 && ldp_o >= p_cols &&
+                 (reinterpret_cast<uintptr_t>(P_o) & 15u) == 0,
+             "ghost_gradproj_embedding: P_o must be 16-byte aligned bf16 with columns padded to a multiple of 8");
+  GB_REQUIRE(!g_is_f32 || (p_lo_offset % 8 == 0 && p_lo_offset >= p_cols && p_lo_offset + p_cols <= ldp_o),
+             "ghost_gradproj_embedding: float out-grads need the residual part of P_o inside its rows");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (!accumulate)
+    GB_CUDA_OK(cudaMemset2DAsync(out, static_cast<size_t>(out_stride) * 4, 0, static_cast<size_t>(k_o) * k_i * 4,
+                                 static_cast<size_t>(B), st));
   GpParams p = {};
-  p.B = B; p.T = T; p.n_r = n_r; p.n_c = n_c; p.k_r = k_r; p.k_c = k_c;
-  p.kr_pad = (k_r + 15) / 16 * 16;
-  p.kc_pad = (k_c + 15) / 16 * 16;
-  p.chunks_per_sample = ceil_div(T, 128);
-  p.units = static_cast<long long>(B) * p.chunks_per_sample;
-  p.scale = scale;
-  p.out = out;
-  p.out_stride = out_stride;
-  p.out_ld = k_c;
-  p.err = ds->err_word;
-  CUtensorMap tg, tpr, ta, tpc;
-  int rc;
-  if ((rc = make_tmap_bf16_3d(&tg, G, B, T, n_r, ldg, 128)) != GHOST_OK) return rc;
-  if ((rc = make_tmap_bf16_3d(&ta, A, B, T, n_c, lda, 128)) != GHOST_OK) return rc;
-  // the projection matrices as one-sample 3-D operands, so that one TMA instruction form serves all four
-  if ((rc = make_tmap_bf16_3d(&tpr, P_r, 1, k_r, n_r, ldpr, p.kr_pad)) != GHOST_OK) return rc;
-  if ((rc = make_tmap_bf16_3d(&tpc, P_c, 1, k_c, n_c, ldpc, p.kc_pad)) != GHOST_OK) return rc;
-  GB_CUDA_OK(cudaMemset2DAsync(out, out_stride * sizeof(float), 0, static_cast<size_t>(k_r) * k_c * sizeof(float), B, st));
-  const int kmax = p.kr_pad > p.kc_pad ? p.kr_pad : p.kc_pad;
-  if (kmax <= 32) return launch_gradproj<32, false>(tg, tpr, ta, tpc, p, ds, st);
-  if (kmax <= 64) return launch_gradproj<64, false>(tg, tpr, ta, tpc, p, ds, st);
-  return launch_gradproj<128, false>(tg, tpr, ta, tpc, p, ds, st);
+  p.B = B; p.T = T; p.n_r = d; p.k_r = k_o; p.k_c = k_i; p.scale = scale;
+  p.out = out; p.out_stride = out_stride; p.out_ld = out_ld;
+  p.lo_r = p_lo_offset;
+  p.ids = ids; p.rows = P_i_t; p.ld_rows = ld_pit; p.vocab = vocab;
+  p.rows_vec = k_i % 4 == 0 && ld_pit % 4 == 0 && (reinterpret_cast<uintptr_t>(P_i_t) & 15u) == 0;
+  const GpOperands o = {G, nullptr, g_is_f32, ldg, 0, P_o, nullptr, ldp_o, 0, g_is_f32 ? static_cast<int>(ldp_o) : p_cols, 0};
+  return launch_gradproj<true>(o, p, ds, st);
 }

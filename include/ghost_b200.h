@@ -333,6 +333,14 @@ int ghost_gradproj_dense_bf16(const void* G, const void* A, int B, long long T, 
                               long long ldg, long long lda, const void* P_r, const void* P_c, int k_r,
                               int k_c, long long ldpr, long long ldpc, float scale, float* out,
                               long long out_stride, void* stream);
+/* The same for operands of any alignment and pitch, bf16 or (is_f32) fp32, without copies of them.  P_r and P_c: bf16
+ * rows of whole pitches, for fp32 operands bf16(P) in columns [0, n) and the residual P - bf16(P) in columns
+ * [lo, lo + n), finite values elsewhere (ghost_cast_split_bf16 with parts side by side leaves hi, hi, lo: lo = 2 cpad);
+ * for bf16 operands zero beyond column n.  Ranks up to 64. */
+int ghost_gradproj_dense(const void* G, const void* A, int is_f32, int B, long long T, int n_r, int n_c, long long ldg,
+                         long long lda, const void* P_r, const void* P_c, int k_r, int k_c, long long ldpr,
+                         long long ldpc, int lo_r, int lo_c, float scale, float* out, long long out_stride,
+                         void* stream);
 /* out + b * out_stride + o * out_ld + i (+)= scale * sum_t (P_o g_bt)[o] * P_i[i, id_bt] for every sample
  * b, o < k_o, i < k_i: the projected gradient of an embedding table.  ids: [B, T] int64; G: [B, T, d]
  * out-grad rows (fp32 or bf16, row pitch ldg); P_o: bf16 [k_o, ldp_o] as ghost_cast_split_bf16 lays

@@ -1041,3 +1041,45 @@ def test_norm_wide_rows(dtype, rms, N, T, F):
     # float32 sums of F values and of T rows around values of order one: a few ulp of sqrt(F + T)
     assert O.rel_fro(gw, (g * x).sum(1)) < 2e-6
     assert O.rel_fro(gb, g.sum(1)) < 2e-6
+
+
+# (B, T, columns of G, of A, k_r, k_c): one unit of 128 tokens to more than the GPU has SMs, so that every cluster size
+# and none is met, with fewer stages of columns than CTAs among them; token counts around a unit; columns that no
+# 16-byte load fits; ranks on both sides of each instantiation's largest
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("case", [(1, 1, 7, 5, 1, 1), (1, 10, 4407, 452, 44, 44), (2, 129, 333, 1000, 16, 17), (16, 127, 130, 70, 33, 9),
+                                  (17, 128, 512, 300, 64, 64), (35, 100, 260, 516, 5, 60), (3, 300, 2050, 3072, 32, 48),
+                                  (75, 64, 200, 136, 20, 20), (160, 33, 97, 104, 9, 4), (5, 140, 640, 259, 100, 128),
+                                  (80, 200, 321, 192, 128, 65)])
+def test_gradproj_dense_unit_counts_and_widths(case, dtype):
+    B, T, n_r, n_c, k_r, k_c = case
+    g = torch.Generator().manual_seed(17)
+    G, A = torch.randn(B, T, n_r, generator=g).to(dtype), torch.randn(B, T, n_c, generator=g).to(dtype)
+    P_r, P_c = torch.randn(k_r, n_r, generator=g) / k_r ** 0.5, torch.randn(k_c, n_c, generator=g) / k_c ** 0.5
+    out = torch.full((B, k_r * k_c + 3), 7.0, device="cuda")
+    split = dtype == torch.float32
+    ops().gradproj_dense(G.cuda(), A.cuda(), ops().prepare_projection(P_r.cuda(), split), ops().prepare_projection(P_c.cuda(), split),
+                         k_r, k_c, 0.5, out[:, :k_r * k_c])
+    after()
+    ref = 0.5 * torch.einsum("btr,btc->brc", G.double() @ P_r.double().t(), A.double() @ P_c.double().t())
+    # every factor of a product is rounded once: to 8 bits (P of a bf16 layer), or to two parts of 8 bits
+    assert O.rel_fro(out[:, :k_r * k_c], ref.flatten(1)) < (2 * 2.0 ** -15 if split else 2 * 2.0 ** -8)
+    assert (out[:, k_r * k_c:] == 7.0).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("case", [(1, 3, 5, 1, 1), (2, 63, 1920, 57, 57), (4, 36, 307, 9, 9), (2, 1212, 717, 26, 26), (16, 130, 64, 64, 33),
+                                  (40, 128, 230, 16, 16), (90, 200, 136, 32, 64)])
+def test_gradproj_embedding_unit_counts_and_widths(case, dtype):
+    B, T, d, k_o, k_i = case
+    g = torch.Generator().manual_seed(18)
+    vocab = 211
+    ids = torch.randint(0, vocab, (B, T), generator=g)
+    G = torch.randn(B, T, d, generator=g).to(dtype)
+    P_o, P_i = torch.randn(k_o, d, generator=g) / k_o ** 0.5, torch.randn(k_i, vocab, generator=g)
+    split = dtype == torch.float32
+    out = ops().gradproj_embedding(ids.cuda(), G.cuda(), ops().prepare_projection(P_o.cuda(), split),
+                                   ops().prepare_embedding_projection(P_i.cuda()), k_o, k_i)
+    after()
+    ref = torch.einsum("bto,bti->boi", G.double() @ P_o.double().t(), P_i.double().t()[ids])
+    assert O.rel_fro(out, ref.flatten(1)) < (2 * 2.0 ** -15 if split else 2 * 2.0 ** -8)
