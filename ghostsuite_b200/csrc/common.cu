@@ -233,8 +233,24 @@ int make_tmap_bf16_blocks(CUtensorMap* out, const void* base, uint64_t samples, 
   return GHOST_OK;
 }
 
-int make_tmap_bf16_parts(CUtensorMap* out, const void* base, uint64_t samples, uint64_t rows, uint64_t cols,
-                         uint32_t box_rows, uint32_t box_blocks) {
+int make_tmap_bf16_part_rows(CUtensorMap* out, const void* base, uint64_t part_rows, uint64_t rows, uint64_t ld, uint32_t box_rows) {
+  EncodeTiledFn fn = encode_fn();
+  if (!fn) return fail(GHOST_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
+  if ((reinterpret_cast<uintptr_t>(base) & 15u) != 0 || ld % 64 != 0 || rows == 0 || rows > part_rows)
+    return fail(GHOST_ERR_INVALID, "split TMA rows need 16-byte alignment and a pitch that is a multiple of 64");
+  cuuint64_t dims[3] = {ld, rows, 2};
+  cuuint64_t strides[2] = {ld * 2, part_rows * ld * 2};
+  cuuint32_t box[3] = {64, box_rows, 2};
+  cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return fail(GHOST_ERR_CUDA, "cuTensorMapEncodeTiled(split rows) failed with CUresult %d", (int)r);
+  return GHOST_OK;
+}
+
+int make_tmap_bf16_parts(CUtensorMap* out, const void* base, uint64_t samples, uint64_t part_rows, uint64_t rows,
+                         uint64_t cols, uint32_t box_rows, uint32_t box_blocks) {
   EncodeTiledFn fn = encode_fn();
   if (!fn) return fail(GHOST_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
   if ((reinterpret_cast<uintptr_t>(base) & 15u) != 0)
@@ -242,7 +258,7 @@ int make_tmap_bf16_parts(CUtensorMap* out, const void* base, uint64_t samples, u
   if (rows == 0 || cols == 0 || samples == 0 || cols % 64 != 0)
     return fail(GHOST_ERR_INVALID, "split TMA operand needs a column count that is a multiple of 64");
   cuuint64_t dims[5] = {64, rows, cols / 64, 2, samples};
-  cuuint64_t strides[4] = {cols * 2, 128, rows * cols * 2, 2 * rows * cols * 2};
+  cuuint64_t strides[4] = {cols * 2, 128, part_rows * cols * 2, 2 * part_rows * cols * 2};
   cuuint32_t box[5] = {64, box_rows, box_blocks, 2, 1};
   cuuint32_t estr[5] = {1, 1, 1, 1, 1};
   CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<void*>(base), dims, strides, box, estr,

@@ -65,11 +65,15 @@ int make_tmap_bf16_3d(CUtensorMap* out, const void* base, uint64_t samples, uint
 int make_tmap_bf16_blocks(CUtensorMap* out, const void* base, uint64_t samples, uint64_t rows,
                           uint64_t cols, uint64_t ld, uint32_t box_rows, uint32_t box_blocks);
 
-// float32 operands as two bf16 parts (value and residual), [samples, 2, rows, cols] with cols a multiple of 64
-// (zero-padded): a box covers both parts of `box_blocks` adjacent 64-column blocks of `box_rows` rows, the
+// Rows of a float32 matrix as two bf16 parts `part_rows` rows apart (columns zero-padded to the pitch), for K-major
+// tiles: a box covers 64 columns of `box_rows` rows of both parts, the values first.  Coordinates: (column, row, 0).
+int make_tmap_bf16_part_rows(CUtensorMap* out, const void* base, uint64_t part_rows, uint64_t rows, uint64_t ld, uint32_t box_rows);
+
+// float32 operands as two bf16 parts (value and residual), [samples, 2, part_rows, cols] with cols a multiple of 64
+// (zero-padded), of which the first `rows` of a part count: a box covers both parts of `box_blocks` adjacent 64-column blocks of `box_rows` rows, the
 // value panels first.  Rows past the end of a sample read as zero.  Coordinates: (0, row, block, 0, sample).
-int make_tmap_bf16_parts(CUtensorMap* out, const void* base, uint64_t samples, uint64_t rows, uint64_t cols,
-                         uint32_t box_rows, uint32_t box_blocks);
+int make_tmap_bf16_parts(CUtensorMap* out, const void* base, uint64_t samples, uint64_t part_rows, uint64_t rows,
+                         uint64_t cols, uint32_t box_rows, uint32_t box_blocks);
 
 // Validation tiles as an all-gather leaves them: [ranks][tiles][per_rank samples][32768] bf16, seen as
 // [64, per_rank, ranks, 512 panels, tiles]; a box holds `box_rows` consecutive validation samples

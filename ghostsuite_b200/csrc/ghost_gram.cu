@@ -34,26 +34,29 @@ struct GramParams {
   int* err;
 };
 
-template <int BN>
+// PARTS = 2: float32 rows as two bf16 parts, three products per K step into the same accumulator; a stage holds both
+// parts of 64 K elements.  (Parts stacked along K, three per operand, fetched the values twice.)
+template <int BN, int PARTS>
 struct GramCfg {
   static constexpr int BM = 128;
   static constexpr int kAtomK = 64;                        // K elements of one 128-byte swizzle atom
   // K elements per stage.  BN = 128: two atoms per operand (64 KB stages), so the issuing thread
   // does one barrier round trip per eight MMAs; BN = 256 keeps one atom (48 KB stages), two would
   // leave room for two stages only.
-  static constexpr int BK = (BN == 256) ? 64 : 128;
-  static constexpr int kStageBytes = (BM + BN) * BK * 2;
+  static constexpr int BK = (BN == 256 || PARTS == 2) ? 64 : 128;
+  static constexpr int kStageBytes = (BM + BN) * BK * 2 * PARTS;
   static constexpr int kStages = (BN == 256) ? 4 : 3;
   static constexpr int kAccBufs = 512 / (2 * BN);          // 1 (BN=256) or 2 (BN=128)
   static constexpr int kSmemBytes = kStages * kStageBytes + 1024 /*align*/ + 256 /*barriers*/;
 };
 
-template <int BN>
+template <int BN, int PARTS>
 __global__ void __launch_bounds__(192, 1)
 ghost_gram_kernel(const __grid_constant__ CUtensorMap tm_at, const __grid_constant__ CUtensorMap tm_av,
                   const __grid_constant__ CUtensorMap tm_gt, const __grid_constant__ CUtensorMap tm_gv,
                   const GramParams p) {
-  using Cfg = GramCfg<BN>;
+  using Cfg = GramCfg<BN, PARTS>;
+  static_assert(PARTS == 1 || BN == 128, "two parts of wider tiles leave two stages");
   constexpr int BM = Cfg::BM, BK = Cfg::BK, kStages = Cfg::kStages, kAccBufs = Cfg::kAccBufs;
 
   extern __shared__ uint8_t smem_raw[];
@@ -131,8 +134,12 @@ ghost_gram_kernel(const __grid_constant__ CUtensorMap tm_at, const __grid_consta
           const CUtensorMap* mt = (kb < kb_a) ? &tm_at : &tm_gt;
           const CUtensorMap* mv = (kb < kb_a) ? &tm_av : &tm_gv;
           const int k0 = ((kb < kb_a) ? kb : kb - kb_a) * BK;
+          if constexpr (PARTS == 2) {
+            tma_load_3d(st, mt, &full_bar[stage], k0, m0, 0);
+            tma_load_3d(st + BM * BK * 4, mv, &full_bar[stage], k0, n0, 0);
+          }
 #pragma unroll
-          for (int a = 0; a < BK / Cfg::kAtomK; ++a) {
+          for (int a = 0; a < (PARTS == 2 ? 0 : BK / Cfg::kAtomK); ++a) {
             tma_load_2d(st + a * (BM * Cfg::kAtomK * 2), mt, &full_bar[stage], k0 + a * Cfg::kAtomK, m0);
             tma_load_2d(st + BM * BK * 2 + a * (BN * Cfg::kAtomK * 2), mv, &full_bar[stage],
                         k0 + a * Cfg::kAtomK, n0);
@@ -164,10 +171,18 @@ ghost_gram_kernel(const __grid_constant__ CUtensorMap tm_at, const __grid_consta
 #pragma unroll
           for (int a = 0; a < BK / Cfg::kAtomK; ++a) {
             const uint64_t adesc = make_smem_desc_sw128(sa + a * (BM * Cfg::kAtomK * 2), 16, 1024);
-            const uint64_t bdesc = make_smem_desc_sw128(sa + BM * BK * 2 + a * (BN * Cfg::kAtomK * 2), 16, 1024);
+            const uint64_t bdesc = make_smem_desc_sw128(sa + BM * BK * 2 * PARTS + a * (BN * Cfg::kAtomK * 2), 16, 1024);
 #pragma unroll
-            for (int k = 0; k < Cfg::kAtomK / 16; ++k)
-              umma_bf16(dst, adesc + 2 * k, bdesc + 2 * k, idesc, (first && a == 0 && k == 0) ? 0u : 1u);
+            for (int k = 0; k < Cfg::kAtomK / 16; ++k) {
+              const uint32_t add = (first && a == 0 && k == 0) ? 0u : 1u;
+              if constexpr (PARTS == 2) {      // residual parts lie behind the values
+                umma_bf16(dst, adesc + 2 * k + BM * BK * 2 / 16, bdesc + 2 * k, idesc, add);
+                umma_bf16(dst, adesc + 2 * k, bdesc + 2 * k + BN * BK * 2 / 16, idesc, 1u);
+                umma_bf16(dst, adesc + 2 * k, bdesc + 2 * k, idesc, 1u);
+              } else {
+                umma_bf16(dst, adesc + 2 * k, bdesc + 2 * k, idesc, add);
+              }
+            }
           }
           umma_commit(&empty_bar[stage]);   // frees the stage once these MMAs have read it
           if (++stage == kStages) { stage = 0; phase ^= 1; }
@@ -262,56 +277,98 @@ ghost_gram_kernel(const __grid_constant__ CUtensorMap tm_at, const __grid_consta
   }
 }
 
-template <int BN>
-static int launch_gram(const void* a_t, const void* a_v, const void* g_t, const void* g_v,
-                       int n_train, int n_val, long long T, int ka, int kg, long long ld_at,
-                       long long ld_av, long long ld_gt, long long ld_gv, int round_mode, float scale,
-                       float* M, const DeviceState* ds, cudaStream_t stream) {
-  using Cfg = GramCfg<BN>;
+// Operands of the two Grams: rows of train and validation tokens
+struct GramOperands {
+  const void *a_t, *a_v, *g_t, *g_v;
+  long long ld_at, ld_av, ld_gt, ld_gv;
+  int ka, kg;
+  int parts;
+  long long part_rows;     // parts == 2: rows of a part in memory
+};
+static int gram_map(CUtensorMap* t, const GramOperands& o, const void* base, long long rows, int k, long long ld, int box_rows) {
+  return o.parts == 2 ? make_tmap_bf16_part_rows(t, base, o.part_rows, rows, ld, box_rows)
+                      : make_tmap_bf16_2d(t, base, rows, k, ld, box_rows);
+}
+// Maps of the four operands: train rows in boxes of box_t, validation rows of box_v
+int gram_maps(CUtensorMap (&t)[4], const GramOperands& o, long long rows_t, long long rows_v, int box_t, int box_v) {
+  int rc;
+  if ((rc = gram_map(&t[0], o, o.a_t, rows_t, o.ka, o.ld_at, box_t)) != GHOST_OK) return rc;
+  if ((rc = gram_map(&t[1], o, o.a_v, rows_v, o.ka, o.ld_av, box_v)) != GHOST_OK) return rc;
+  if ((rc = gram_map(&t[2], o, o.g_t, rows_t, o.kg, o.ld_gt, box_t)) != GHOST_OK) return rc;
+  return gram_map(&t[3], o, o.g_v, rows_v, o.kg, o.ld_gv, box_v);
+}
+
+template <int BN, int PARTS>
+static int launch_gram(const GramOperands& o, int n_train, int n_val, long long T, int round_mode, float scale, float* M,
+                       const DeviceState* ds, cudaStream_t stream) {
+  using Cfg = GramCfg<BN, PARTS>;
   GramParams p;
   p.rows_t = static_cast<long long>(n_train) * T;
   p.rows_v = static_cast<long long>(n_val) * T;
   p.T = T;
   p.n_train = n_train;
   p.n_val = n_val;
-  p.ka = ka;
-  p.kg = kg;
+  p.ka = o.ka;
+  p.kg = o.kg;
   p.m_tiles = ceil_div(p.rows_t, Cfg::BM);
   p.n_tiles = ceil_div(p.rows_v, BN);
   p.round_mode = round_mode;
   p.scale = scale;
   p.M = M;
   p.err = ds->err_word;
-  CUtensorMap tm_at, tm_av, tm_gt, tm_gv;
-  int rc;
-  if ((rc = make_tmap_bf16_2d(&tm_at, a_t, p.rows_t, ka, ld_at, Cfg::BM)) != GHOST_OK) return rc;
-  if ((rc = make_tmap_bf16_2d(&tm_av, a_v, p.rows_v, ka, ld_av, BN)) != GHOST_OK) return rc;
-  if ((rc = make_tmap_bf16_2d(&tm_gt, g_t, p.rows_t, kg, ld_gt, Cfg::BM)) != GHOST_OK) return rc;
-  if ((rc = make_tmap_bf16_2d(&tm_gv, g_v, p.rows_v, kg, ld_gv, BN)) != GHOST_OK) return rc;
-
+  CUtensorMap t[4];
+  const int rc = gram_maps(t, o, p.rows_t, p.rows_v, Cfg::BM, BN);
+  if (rc != GHOST_OK) return rc;
   static bool attr_set[64] = {};
   if (!attr_set[ds->device]) {
-    GB_CUDA_OK(cudaFuncSetAttribute(ghost_gram_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    GB_CUDA_OK(cudaFuncSetAttribute(ghost_gram_kernel<BN, PARTS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     Cfg::kSmemBytes));
     attr_set[ds->device] = true;
   }
   const long long tiles = static_cast<long long>(p.m_tiles) * p.n_tiles;
   const int grid = static_cast<int>(tiles < ds->sm_count ? tiles : ds->sm_count);
-  ghost_gram_kernel<BN><<<grid, 192, Cfg::kSmemBytes, stream>>>(tm_at, tm_av, tm_gt, tm_gv, p);
+  ghost_gram_kernel<BN, PARTS><<<grid, 192, Cfg::kSmemBytes, stream>>>(t[0], t[1], t[2], t[3], p);
   count_launch();
   return post_launch("ghost_gram_kernel");
 }
 
-int launch_gram_pair(const void* a_t, const void* a_v, const void* g_t, const void* g_v, int n_train, int n_val,
-                     long long T, int ka, int kg, long long ld_at, long long ld_av, long long ld_gt,
-                     long long ld_gv, int round_mode, float scale, float* M, const DeviceState* ds,
-                     cudaStream_t stream);
+int launch_gram_pair(const GramOperands& o, int n_train, int n_val, long long T, int round_mode, float scale, float* M,
+                     const DeviceState* ds, cudaStream_t stream);
 
 // 0: single-CTA kernels only; 1: CTA-pair kernel for problems with at least 512 train tokens and 256
 // to 8192 validation tokens (where it measured faster: 1474 against 1339 TFLOP/s with 32768 x 4096
 // tokens, 985 against 1117 with 131072 x 16384); 2: CTA-pair kernel from 512 x 256 tokens up
 static int g_gram_pair_mode = 1;
 bool xty_pair_usable(const DeviceState* ds);     // a cluster of two ~198 KB CTAs fits on the device
+
+static int gram_dot(const GramOperands& o, int n_train, int n_val, long long T, int round_mode, float scale, float* M_out, void* stream) {
+  const DeviceState* ds = device_state();
+  if (!ds) return GHOST_ERR_DEVICE;
+  GB_REQUIRE(o.a_t && o.a_v && o.g_t && o.g_v && M_out, "ghost_gram_dot_bf16: null pointer");
+  GB_REQUIRE(n_train > 0, "No training samples to compute dot product, check batch sizes.");
+  GB_REQUIRE(n_val > 0 && T > 0 && o.ka > 0 && o.kg > 0, "ghost_gram_dot_bf16: empty dimension");
+  GB_REQUIRE(round_mode == 0 || round_mode == 1, "ghost_gram_dot_bf16: round_mode must be 0 or 1");
+  GB_REQUIRE(static_cast<long long>(n_train) * T < (1ll << 31) - 256 &&
+             static_cast<long long>(n_val) * T < (1ll << 31) - 256,
+             "ghost_gram_dot_bf16: more than 2^31 tokens");
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  GB_CUDA_OK(cudaMemsetAsync(M_out, 0, sizeof(float) * static_cast<size_t>(n_val) * n_train, st));
+  const long long rows_t = static_cast<long long>(n_train) * T, rows_v = static_cast<long long>(n_val) * T;
+  // Rounds of tiles over the GPU times the cycles of a K step of a tile (128 for 256 x 256 on a pair and 128 x 256 on one
+  // SM, 64 for 128 x 128, a tenth more for its operand traffic): 2048 x 1024 tokens are 32 tiles of 256 x 256 on 74
+  // pairs, and 128 of 128 x 128 on 148 SMs.
+  auto tiles = [&](int bm, int bn) { return ((rows_t + bm - 1) / bm) * ((rows_v + bn - 1) / bn); };
+  auto rounds = [](long long n, long long workers) { return static_cast<double>((n + workers - 1) / workers); };
+  const double small_tiles = rounds(tiles(128, 128), ds->sm_count) * 70.;
+  const bool pair_wanted = g_gram_pair_mode == 2 || (g_gram_pair_mode == 1 && rows_v <= 8192 &&
+                                                     rounds(tiles(256, 256), ds->sm_count / 2) * 128. < small_tiles * 1.1);
+  if (pair_wanted && rows_v >= 256 && rows_t >= 512 && xty_pair_usable(ds))
+    return launch_gram_pair(o, n_train, n_val, T, round_mode, scale, M_out, ds, st);
+  if (o.parts == 2) return launch_gram<128, 2>(o, n_train, n_val, T, round_mode, scale, M_out, ds, st);
+  if (rows_v <= 128 || small_tiles * 1.1 < rounds(tiles(128, 256), ds->sm_count) * 128.)
+    return launch_gram<128, 1>(o, n_train, n_val, T, round_mode, scale, M_out, ds, st);
+  return launch_gram<256, 1>(o, n_train, n_val, T, round_mode, scale, M_out, ds, st);
+}
 
 }  // namespace gb
 
@@ -326,26 +383,20 @@ extern "C" int ghost_gram_dot_bf16(const void* a_train, const void* a_val, const
                                    int kg, long long ld_at, long long ld_av, long long ld_gt,
                                    long long ld_gv, int round_mode, float scale, float* M_out,
                                    void* stream) {
+  const gb::GramOperands o = {a_train, a_val, g_train, g_val, ld_at, ld_av, ld_gt, ld_gv, ka, kg, 1, 0};
+  return gb::gram_dot(o, n_train, n_val, T, round_mode, scale, M_out, stream);
+}
+
+extern "C" int ghost_gram_dot_parts(const void* A, const void* G, int parts, int n_train, int n_val, long long T, int d, int p,
+                                    long long ld_a, long long ld_g, int round_mode, float scale, float* M_out, void* stream) {
   using namespace gb;
-  const DeviceState* ds = device_state();
-  if (!ds) return GHOST_ERR_DEVICE;
-  GB_REQUIRE(a_train && a_val && g_train && g_val && M_out, "ghost_gram_dot_bf16: null pointer");
+  GB_REQUIRE(A && G, "ghost_gram_dot_parts: null pointer");
+  GB_REQUIRE(parts == 1 || parts == 2, "ghost_gram_dot_parts: one or two parts");
   GB_REQUIRE(n_train > 0, "No training samples to compute dot product, check batch sizes.");
-  GB_REQUIRE(n_val > 0 && T > 0 && ka > 0 && kg > 0, "ghost_gram_dot_bf16: empty dimension");
-  GB_REQUIRE(round_mode == 0 || round_mode == 1, "ghost_gram_dot_bf16: round_mode must be 0 or 1");
-  GB_REQUIRE(static_cast<long long>(n_train) * T < (1ll << 31) - 256 &&
-             static_cast<long long>(n_val) * T < (1ll << 31) - 256,
-             "ghost_gram_dot_bf16: more than 2^31 tokens");
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  GB_CUDA_OK(cudaMemsetAsync(M_out, 0, sizeof(float) * static_cast<size_t>(n_val) * n_train, st));
-  const long long rows_v = static_cast<long long>(n_val) * T;
-  const bool pair_wanted = g_gram_pair_mode == 2 || (g_gram_pair_mode == 1 && rows_v <= 8192);
-  if (pair_wanted && rows_v >= 256 && static_cast<long long>(n_train) * T >= 512 && xty_pair_usable(ds))
-    return launch_gram_pair(a_train, a_val, g_train, g_val, n_train, n_val, T, ka, kg, ld_at, ld_av, ld_gt,
-                            ld_gv, round_mode, scale, M_out, ds, st);
-  if (rows_v <= 128)
-    return launch_gram<128>(a_train, a_val, g_train, g_val, n_train, n_val, T, ka, kg, ld_at, ld_av,
-                            ld_gt, ld_gv, round_mode, scale, M_out, ds, st);
-  return launch_gram<256>(a_train, a_val, g_train, g_val, n_train, n_val, T, ka, kg, ld_at, ld_av,
-                          ld_gt, ld_gv, round_mode, scale, M_out, ds, st);
+  GB_REQUIRE(n_val > 0 && T > 0 && d > 0 && p > 0 && ld_a >= d && ld_g >= p, "ghost_gram_dot_parts: bad dimensions");
+  const long long rows_t = static_cast<long long>(n_train) * T;
+  const char *a = static_cast<const char*>(A), *g = static_cast<const char*>(G);
+  const GramOperands o = {a, a + rows_t * ld_a * 2, g, g + rows_t * ld_g * 2, ld_a, ld_a, ld_g, ld_g, d, p, parts,
+                          rows_t + static_cast<long long>(n_val) * T};
+  return gram_dot(o, n_train, n_val, T, round_mode, scale, M_out, stream);
 }

@@ -27,22 +27,24 @@ struct GramPairParams {
   int* err;
 };
 
+template <int PARTS>      // as in ghost_gram.cu
 struct GramPairCfg {
   static constexpr int BM = 128;           // rows per CTA
   static constexpr int BNH = 128;          // validation rows loaded per CTA (half of N = 256)
   static constexpr int BN = 256;
-  static constexpr int BK = 128;           // K elements per stage = two 64-element swizzle atoms per operand
+  static constexpr int BK = 128 / PARTS;   // K elements per stage: two 64-element swizzle atoms per operand, or both parts of one
   static constexpr int kAtomK = 64;
-  static constexpr int kStageBytes = (BM + BNH) * BK * 2;   // 64 KB
+  static constexpr int kStageBytes = (BM + BNH) * BK * 2 * PARTS;   // 64 KB
   static constexpr int kStages = 3;
   static constexpr int kSmemBytes = kStages * kStageBytes + 1024 + 256;
 };
 
+template <int PARTS>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1)
 ghost_gram_pair_kernel(const __grid_constant__ CUtensorMap tm_at, const __grid_constant__ CUtensorMap tm_av,
                        const __grid_constant__ CUtensorMap tm_gt, const __grid_constant__ CUtensorMap tm_gv,
                        const GramPairParams p) {
-  using Cfg = GramPairCfg;
+  using Cfg = GramPairCfg<PARTS>;
   constexpr int BM = Cfg::BM, BNH = Cfg::BNH, BN = Cfg::BN, BK = Cfg::BK, kStages = Cfg::kStages;
 
   extern __shared__ uint8_t smem_raw[];
@@ -121,8 +123,12 @@ ghost_gram_pair_kernel(const __grid_constant__ CUtensorMap tm_at, const __grid_c
           const CUtensorMap* mt = (kb < kb_a) ? &tm_at : &tm_gt;
           const CUtensorMap* mv = (kb < kb_a) ? &tm_av : &tm_gv;
           const int k0 = ((kb < kb_a) ? kb : kb - kb_a) * BK;
+          if constexpr (PARTS == 2) {
+            tma_load_3d_pair(st, mt, bar, k0, m0, 0);
+            tma_load_3d_pair(st + BM * BK * 4, mv, bar, k0, n0, 0);
+          }
 #pragma unroll
-          for (int a = 0; a < BK / Cfg::kAtomK; ++a) {
+          for (int a = 0; a < (PARTS == 2 ? 0 : BK / Cfg::kAtomK); ++a) {
             tma_load_2d_pair(st + a * (BM * Cfg::kAtomK * 2), mt, bar, k0 + a * Cfg::kAtomK, m0);
             tma_load_2d_pair(st + BM * BK * 2 + a * (BNH * Cfg::kAtomK * 2), mv, bar, k0 + a * Cfg::kAtomK, n0);
           }
@@ -151,10 +157,18 @@ ghost_gram_pair_kernel(const __grid_constant__ CUtensorMap tm_at, const __grid_c
 #pragma unroll
           for (int a = 0; a < BK / Cfg::kAtomK; ++a) {
             const uint64_t adesc = make_smem_desc_sw128(sa + a * (BM * Cfg::kAtomK * 2), 16, 1024);
-            const uint64_t bdesc = make_smem_desc_sw128(sa + BM * BK * 2 + a * (BNH * Cfg::kAtomK * 2), 16, 1024);
+            const uint64_t bdesc = make_smem_desc_sw128(sa + BM * BK * 2 * PARTS + a * (BNH * Cfg::kAtomK * 2), 16, 1024);
 #pragma unroll
-            for (int k = 0; k < Cfg::kAtomK / 16; ++k)
-              umma_bf16_pair(dst, adesc + 2 * k, bdesc + 2 * k, idesc, (first && a == 0 && k == 0) ? 0u : 1u);
+            for (int k = 0; k < Cfg::kAtomK / 16; ++k) {
+              const uint32_t add = (first && a == 0 && k == 0) ? 0u : 1u;
+              if constexpr (PARTS == 2) {      // residual parts lie behind the values
+                umma_bf16_pair(dst, adesc + 2 * k + BM * BK * 2 / 16, bdesc + 2 * k, idesc, add);
+                umma_bf16_pair(dst, adesc + 2 * k, bdesc + 2 * k + BNH * BK * 2 / 16, idesc, 1u);
+                umma_bf16_pair(dst, adesc + 2 * k, bdesc + 2 * k, idesc, 1u);
+              } else {
+                umma_bf16_pair(dst, adesc + 2 * k, bdesc + 2 * k, idesc, add);
+              }
+            }
           }
           umma_commit_pair(&empty_bar[stage], 3);      // frees the stage in both CTAs
           if (++stage == kStages) { stage = 0; phase ^= 1; }
@@ -248,43 +262,53 @@ ghost_gram_pair_kernel(const __grid_constant__ CUtensorMap tm_at, const __grid_c
   }
 }
 
-int launch_gram_pair(const void* a_t, const void* a_v, const void* g_t, const void* g_v, int n_train, int n_val,
-                     long long T, int ka, int kg, long long ld_at, long long ld_av, long long ld_gt,
-                     long long ld_gv, int round_mode, float scale, float* M, const DeviceState* ds,
-                     cudaStream_t stream) {
-  using Cfg = GramPairCfg;
-  GramPairParams p;
-  p.rows_t = static_cast<long long>(n_train) * T;
-  p.rows_v = static_cast<long long>(n_val) * T;
-  p.T = T;
-  p.n_train = n_train;
-  p.n_val = n_val;
-  p.ka = ka;
-  p.kg = kg;
-  p.m_tiles = ceil_div(p.rows_t, 2 * Cfg::BM);
-  p.n_tiles = ceil_div(p.rows_v, Cfg::BN);
-  p.round_mode = round_mode;
-  p.scale = scale;
-  p.M = M;
-  p.err = ds->err_word;
-  CUtensorMap tm_at, tm_av, tm_gt, tm_gv;
-  int rc;
-  if ((rc = make_tmap_bf16_2d(&tm_at, a_t, p.rows_t, ka, ld_at, Cfg::BM)) != GHOST_OK) return rc;
-  if ((rc = make_tmap_bf16_2d(&tm_av, a_v, p.rows_v, ka, ld_av, Cfg::BNH)) != GHOST_OK) return rc;
-  if ((rc = make_tmap_bf16_2d(&tm_gt, g_t, p.rows_t, kg, ld_gt, Cfg::BM)) != GHOST_OK) return rc;
-  if ((rc = make_tmap_bf16_2d(&tm_gv, g_v, p.rows_v, kg, ld_gv, Cfg::BNH)) != GHOST_OK) return rc;
+struct GramOperands {      // as in ghost_gram.cu
+  const void *a_t, *a_v, *g_t, *g_v;
+  long long ld_at, ld_av, ld_gt, ld_gv;
+  int ka, kg;
+  int parts;
+  long long part_rows;
+};
+int gram_maps(CUtensorMap (&t)[4], const GramOperands& o, long long rows_t, long long rows_v, int box_t, int box_v);
+
+template <int PARTS>
+static int launch_gram_pair_t(const CUtensorMap (&t)[4], const GramPairParams& p, const DeviceState* ds, cudaStream_t stream) {
+  using Cfg = GramPairCfg<PARTS>;
   static bool attr_set[64] = {};
   if (!attr_set[ds->device]) {
-    GB_CUDA_OK(cudaFuncSetAttribute(ghost_gram_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    GB_CUDA_OK(cudaFuncSetAttribute(ghost_gram_pair_kernel<PARTS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     Cfg::kSmemBytes));
     attr_set[ds->device] = true;
   }
   const long long tiles = static_cast<long long>(p.m_tiles) * p.n_tiles;
   long long pairs = ds->sm_count / 2;
   if (pairs > tiles) pairs = tiles;
-  ghost_gram_pair_kernel<<<static_cast<int>(2 * pairs), 192, Cfg::kSmemBytes, stream>>>(tm_at, tm_av, tm_gt, tm_gv, p);
+  ghost_gram_pair_kernel<PARTS><<<static_cast<int>(2 * pairs), 192, Cfg::kSmemBytes, stream>>>(t[0], t[1], t[2], t[3], p);
   count_launch();
   return post_launch("ghost_gram_pair_kernel");
+}
+
+int launch_gram_pair(const GramOperands& o, int n_train, int n_val, long long T, int round_mode, float scale, float* M,
+                     const DeviceState* ds, cudaStream_t stream) {
+  using Cfg = GramPairCfg<1>;
+  GramPairParams p;
+  p.rows_t = static_cast<long long>(n_train) * T;
+  p.rows_v = static_cast<long long>(n_val) * T;
+  p.T = T;
+  p.n_train = n_train;
+  p.n_val = n_val;
+  p.ka = o.ka;
+  p.kg = o.kg;
+  p.m_tiles = ceil_div(p.rows_t, 2 * Cfg::BM);
+  p.n_tiles = ceil_div(p.rows_v, Cfg::BN);
+  p.round_mode = round_mode;
+  p.scale = scale;
+  p.M = M;
+  p.err = ds->err_word;
+  CUtensorMap t[4];
+  const int rc = gram_maps(t, o, p.rows_t, p.rows_v, Cfg::BM, Cfg::BNH);
+  if (rc != GHOST_OK) return rc;
+  return o.parts == 2 ? launch_gram_pair_t<2>(t, p, ds, stream) : launch_gram_pair_t<1>(t, p, ds, stream);
 }
 
 }  // namespace gb

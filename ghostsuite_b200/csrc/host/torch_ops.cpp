@@ -175,7 +175,6 @@ PyObject* py_arena_clear(PyObject*, PyObject* const*, Py_ssize_t) {
 
 // hi/lo layouts of an fp32 operand pair so that sum_k L[k] R[k] = hi*hi + lo*hi + hi*lo
 constexpr int kSplitLeft[3] = {0, 1, 0};
-constexpr int kSplitRight[3] = {0, 0, 1};
 constexpr int kPlain[3] = {0, 0, 0};
 enum { kSideBySide = 0, kStackRows = 1, kStackBatch = 2 };     // where the parts of a copy lie (kStackBatch: convolutions)
 
@@ -213,49 +212,59 @@ void check_split(long long n_train, long long n_val, const char* who) {
   if (n_val <= 0) invalid(std::string(who) + " needs at least one validation sample");
 }
 
+// ---- operands of the tensor-core paths -----------------------------------------------------------------
+// Two operands of the entry points that take one or two bf16 parts.  A float32 operand makes both two parts; otherwise
+// what is not readable as it is is copied with its rows padded.  `merged`: one sample holding all rows.
+struct XtyOperands {
+  const Operand* x[2];
+  long long count, T, ld[2], off[2] = {0, 0};      // samples that are read and their tokens
+  bool merged, copy[2], split;
+  XtyOperands(Workspace& ws, const Operand& X, const Operand& Y, long long count_, bool merged_)
+      : count(count_), T(X.T), merged(merged_) {
+    x[0] = &X;
+    x[1] = &Y;
+    split = X.f32() || Y.f32();
+    for (int i = 0; i < 2; ++i) {
+      copy[i] = split || !x[i]->ready();
+      ld[i] = copy[i] ? (x[i]->cols + 63) / 64 * 64 : x[i]->cols;
+      if (copy[i]) off[i] = ws.plan(count * parts() * T * ld[i] * 2);
+    }
+  }
+  int parts() const { return split ? 2 : 1; }
+  const void* where(int i, char* base) const { return copy[i] ? static_cast<const void*>(base + off[i]) : x[i]->t.data_ptr(); }
+  // Lays out what has to be copied, with the column sums of operand sums_of (1 or 2, both operands copied) on the way
+  void prepare(char* base, void* st, int sums_of = 0, float* sums = nullptr) const {
+    if (x[0]->conv || x[1]->conv) {
+      const int kinds[3] = {0, 1, 0};
+      for (int i = 0; i < 2; ++i)
+        if (copy[i]) x[i]->cast(0, count, base + off[i], ld[i], ld[i], parts(), kinds, merged ? kStackBatch : kStackRows, st);
+    } else if (copy[0] || copy[1]) {
+      auto src = [&](int i) { return copy[i] ? x[i]->t.data_ptr() : nullptr; };
+      auto dst = [&](int i) { return copy[i] ? base + off[i] : nullptr; };
+      check(ghost_split_operands(src(0), x[0]->f32(), static_cast<int>(x[0]->cols), src(1), x[1]->f32(), static_cast<int>(x[1]->cols),
+                                 parts(), count, T, merged ? 1 : 0, dst(0), dst(1), sums_of == 1 ? sums : nullptr,
+                                 sums_of == 2 ? sums : nullptr, st));
+    }
+  }
+};
+
 // ---- Gram path -----------------------------------------------------------------------------------------
+void launch_gram(const Launch& L, const XtyOperands& ops, int a, char* base, long long n_val, int round_mode, float scale, Tensor& M) {
+  const int g = 1 - a;
+  check(ghost_gram_dot_parts(ops.where(a, base), ops.where(g, base), ops.parts(), static_cast<int>(ops.count - n_val),
+                             static_cast<int>(n_val), ops.T, static_cast<int>(ops.x[a]->cols), static_cast<int>(ops.x[g]->cols),
+                             ops.ld[a], ops.ld[g], round_mode, scale, M.data_ptr<float>(), L.st()));
+}
+
 Tensor gram_dot(const Launch& L, const Operand& A, const Operand& G, long long n_val, int round_mode, float scale) {
-  const long long N = A.N, T = A.T, n_train = N - n_val;
-  check_split(n_train, n_val, "gram_dot");
-  if (G.N != N || G.T != T) invalid("gram_dot: activation and out-grad disagree on [batch, tokens]");
-  Tensor M = empty({n_val, n_train}, A.t, at::kFloat);
+  check_split(A.N - n_val, n_val, "gram_dot");
+  if (G.N != A.N || G.T != A.T) invalid("gram_dot: activation and out-grad disagree on [batch, tokens]");
+  Tensor M = empty({n_val, A.N - n_val}, A.t, at::kFloat);
   Workspace ws;
-  struct Plan { int kind; long long cp, off_t, off_v; } op[2];      // kind 0 as it is, 1 padded copy, 2 split
-  const Operand* xs[2] = {&A, &G};
-  for (int i = 0; i < 2; ++i) {
-    const Operand& x = *xs[i];
-    const long long cp = pad8(x.cols);
-    if (x.f32()) {
-      op[i] = {2, cp, ws.plan(n_train * T * 3 * cp * 2), 0};
-      op[i].off_v = ws.plan(n_val * T * 3 * cp * 2);
-    } else if (x.ready()) {
-      op[i] = {0, cp, 0, 0};
-    } else {
-      op[i] = {1, cp, ws.plan(N * T * cp * 2), 0};
-    }
-  }
+  XtyOperands ops(ws, A, G, A.N, true);
   char* base = ws.commit(L, A.t);
-  const char *pt[2], *pv[2];
-  long long k[2];
-  for (int i = 0; i < 2; ++i) {
-    const Operand& x = *xs[i];
-    const long long cp = op[i].cp;
-    if (op[i].kind == 2) {
-      x.cast(0, n_train, base + op[i].off_t, 3 * cp, cp, 3, kSplitLeft, kSideBySide, L.st());
-      x.cast(n_train, n_val, base + op[i].off_v, 3 * cp, cp, 3, kSplitRight, kSideBySide, L.st());
-      pt[i] = base + op[i].off_t;
-      pv[i] = base + op[i].off_v;
-      k[i] = 3 * cp;
-    } else {
-      if (op[i].kind == 1) x.cast(0, N, base + op[i].off_t, cp, cp, 1, kPlain, kSideBySide, L.st());
-      pt[i] = op[i].kind == 1 ? base + op[i].off_t : static_cast<const char*>(x.t.data_ptr());
-      pv[i] = pt[i] + n_train * T * cp * 2;
-      k[i] = cp;
-    }
-  }
-  check(ghost_gram_dot_bf16(pt[0], pv[0], pt[1], pv[1], static_cast<int>(n_train), static_cast<int>(n_val), T,
-                            static_cast<int>(k[0]), static_cast<int>(k[1]), k[0], k[0], k[1], k[1], round_mode, scale,
-                            M.data_ptr<float>(), L.st()));
+  ops.prepare(base, L.st());
+  launch_gram(L, ops, 0, base, n_val, round_mode, scale, M);
   return M;
 }
 
@@ -270,41 +279,6 @@ PyObject* py_gram_dot(PyObject*, PyObject* const* a, Py_ssize_t n) {
 }
 
 // ---- token-contracted GEMMs --------------------------------------------------------------------------
-// Operands of the entry points that take one or two bf16 parts.  A float32 operand makes both two parts; otherwise
-// what is not readable as it is is copied with its rows padded.  `merged`: one sample holding all rows.
-struct XtyOperands {
-  const Operand* x[2];
-  long long count, samples, T, ld[2], off[2] = {0, 0};      // samples that are read; samples and tokens of the layout
-  bool copy[2], split;
-  XtyOperands(Workspace& ws, const Operand& X, const Operand& Y, long long count_, bool merged)
-      : count(count_), samples(merged ? 1 : count_), T(merged ? count_ * X.T : X.T) {
-    x[0] = &X;
-    x[1] = &Y;
-    split = X.f32() || Y.f32();
-    for (int i = 0; i < 2; ++i) {
-      copy[i] = split || !x[i]->ready();
-      ld[i] = copy[i] ? (x[i]->cols + 63) / 64 * 64 : x[i]->cols;
-      if (copy[i]) off[i] = ws.plan(samples * parts() * T * ld[i] * 2);
-    }
-  }
-  int parts() const { return split ? 2 : 1; }
-  const void* where(int i, char* base) const { return copy[i] ? static_cast<const void*>(base + off[i]) : x[i]->t.data_ptr(); }
-  // Lays out what has to be copied, with the column sums of operand sums_of (1 or 2, both operands copied) on the way
-  void prepare(char* base, void* st, int sums_of = 0, float* sums = nullptr) const {
-    if (x[0]->conv || x[1]->conv) {
-      const int kinds[3] = {0, 1, 0};
-      for (int i = 0; i < 2; ++i)
-        if (copy[i]) x[i]->cast(0, count, base + off[i], ld[i], ld[i], parts(), kinds, samples == 1 ? kStackBatch : kStackRows, st);
-    } else if (copy[0] || copy[1]) {
-      auto src = [&](int i) { return copy[i] ? x[i]->t.data_ptr() : nullptr; };
-      auto dst = [&](int i) { return copy[i] ? base + off[i] : nullptr; };
-      check(ghost_split_operands(src(0), x[0]->f32(), static_cast<int>(x[0]->cols), src(1), x[1]->f32(), static_cast<int>(x[1]->cols),
-                                 parts(), samples, T, dst(0), dst(1), sums_of == 1 ? sums : nullptr,
-                                 sums_of == 2 ? sums : nullptr, st));
-    }
-  }
-};
-
 // scale * sum over the first `samples` samples of X^T Y, into out
 void wgrad(const Launch& L, const Operand& X, const Operand& Y, long long samples, float scale, Tensor& out, bool accumulate) {
   const int m = static_cast<int>(X.cols), n = static_cast<int>(Y.cols);
@@ -314,7 +288,7 @@ void wgrad(const Launch& L, const Operand& X, const Operand& Y, long long sample
   XtyOperands ops(ws, X, Y, samples, true);
   char* base = ws.commit(L, X.t);
   ops.prepare(base, L.st());
-  check(ghost_wgrad_parts(ops.where(0, base), ops.where(1, base), ops.parts(), ops.samples * ops.T, m, n, ops.ld[0], ops.ld[1], scale, accumulate ? 1 : 0,
+  check(ghost_wgrad_parts(ops.where(0, base), ops.where(1, base), ops.parts(), samples * ops.T, samples * ops.T, m, n, ops.ld[0], ops.ld[1], scale, accumulate ? 1 : 0,
                           out.data_ptr(), is_f32(out), base + off_ws, ws_bytes, L.st()));
 }
 
@@ -443,9 +417,23 @@ void dense_paths(const Launch& L, const Operand& A, const Operand& B, long long 
                  float scale, bool bias, bool fuse, Tensor& M, Tensor& grad, Tensor& sums) {
   const Operand &X = in_by_out ? A : B, &Y = in_by_out ? B : A;
   if (gram) {
-    M = gram_dot(L, A, B, n_val, 0, 1.f);
+    // one copy of what has to be copied serves the Grams and the gradient, and gives the bias its sums
+    const long long N = A.N, rows = (N - n_val) * A.T;
+    const int m = static_cast<int>(X.cols), n = static_cast<int>(Y.cols), b = in_by_out ? 1 : 0;
+    check_split(N - n_val, n_val, "gram_dot");
+    M = empty({n_val, N - n_val}, A.t, at::kFloat);
     grad = optional_empty({X.cols, Y.cols}, X.t, gdt);
-    if (grad.defined()) wgrad(L, X, Y, A.N - n_val, scale, grad, false);
+    Workspace ws;
+    const long long ws_bytes = grad.defined() ? ghost_wgrad_workspace_bytes(m, n) : 0, off_ws = ws.plan(ws_bytes);
+    XtyOperands ops(ws, X, Y, N, true);
+    char* base = ws.commit(L, A.t);
+    const bool take = bias && ops.split && A.T >= 16 && !A.conv;
+    if (take) sums = empty({N, B.cols}, A.t, at::kFloat);
+    ops.prepare(base, L.st(), take ? b + 1 : 0, take ? sums.data_ptr<float>() : nullptr);
+    launch_gram(L, ops, 1 - b, base, n_val, 0, 1.f, M);
+    if (grad.defined())
+      check(ghost_wgrad_parts(ops.where(0, base), ops.where(1, base), ops.parts(), N * A.T, rows, m, n, ops.ld[0], ops.ld[1], scale, 0,
+                              grad.data_ptr(), is_f32(grad), base + off_ws, ws_bytes, L.st()));
   } else {
     PerSample r = persample_dot(L, X, Y, n_val, 1.f, gdt >= 0, scale, gdt == 0 ? at::kBFloat16 : at::kFloat,
                                 !fuse ? 0 : in_by_out ? 2 : 1, !bias ? 0 : in_by_out ? 2 : 1);

@@ -94,8 +94,8 @@ __global__ void cast_split_kernel(const CastParams p) {
 }
 
 // Both operands of a token-contracted GEMM in one launch: rows zero-padded to ld (a multiple of 64) columns, as the
-// values alone (PARTS = 1) or as values and residuals, [samples, 2, T, ld].  A block takes a panel of 128 columns of
-// some rows, a thread eight columns of every 16th row, four rows in flight.  Where the column sums of an operand are
+// values alone (PARTS = 1) or as values and residuals, [samples, 2, T, ld] or [2, samples * T, ld].  A block takes a panel of 128 columns of
+// some rows, a thread eight columns of every 16th row, two rows in flight.  Where the column sums of an operand are
 // wanted the rows are one sample's (or a chunk of it, added with atomics), and they cost no second pass over it.
 // Bound by HBM and, on small layers, by the round trip of one round of loads: 8 x 2048 rows of (1024, 2048) float32 at
 // 5.5 TB/s, 29 x 197 of (768, 1000) 22.5 us from cold caches (two launches of cast_split_kernel with three parts
@@ -113,74 +113,67 @@ struct SplitJob {
 };
 struct SplitParams {
   SplitJob job[2];
-  long long T;
+  long long T;             // rows of a sample
+  long long part_rows;     // rows of a part: T, or those of all samples
 };
 
 template <typename E, int PARTS, bool VEC>
 __device__ __forceinline__ void split_rows(const SplitJob& j, long long T, long long r0, long long r1, int c0, float (&sum)[8]) {
-  const E* src = static_cast<const E*>(j.src) + c0;
+  constexpr int R = 2;                   // rows in flight of a thread
   const bool inside = c0 + 8 <= j.cols;
-  // sample s of two parts of T rows: row + s * T.  The sample of this thread's first row, then step by step.
-  long long sample = 0, end = T;
   const long long first = r0 + (threadIdx.x / (kSplitCols / 8));
-  if (PARTS == 2) {
-    sample = j.rows < (1ll << 32) ? static_cast<unsigned>(first) / static_cast<unsigned>(T) : first / T;
-    end = (sample + 1) * T;
-  }
-  float part[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};      // of up to eight rounds: short chains
-  int rounds = 0;
-  for (long long row = first; row < r1; row += 4 * kSplitLanes) {
-    float x[4][8];
+  int left = r1 - first > 0 ? static_cast<int>(r1 - first) : 0;          // a block has far fewer than 2^31 rows
+  const E* src = static_cast<const E*>(j.src) + first * j.cols + c0;
+  // sample s of two parts of T rows: row + s * T.  The sample of this thread's first row, then step by step.
+  long long sample = 0;
+  if (PARTS == 2) sample = j.rows < (1ll << 32) ? static_cast<unsigned>(first) / static_cast<unsigned>(T) : first / T;
+  long long in_sample = T - (first - sample * T);                        // rows of it from here on
+  __nv_bfloat16* dst = j.dst + (first + (PARTS == 2 ? sample * T : 0)) * j.ld + c0;
+  const long long row_src = static_cast<long long>(kSplitLanes) * j.cols, row_dst = static_cast<long long>(kSplitLanes) * j.ld, lo = T * j.ld;
+  for (; left > 0; left -= R * kSplitLanes) {
+    float x[R][8];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
+    for (int q = 0; q < R; ++q, src += row_src) {
 #pragma unroll
       for (int e = 0; e < 8; ++e) x[q][e] = 0.f;
-      const E* p = src + (row + kSplitLanes * q) * j.cols;
-      if (row + kSplitLanes * q < r1) {
+      if (kSplitLanes * q < left) {
         if (VEC && inside) {
-          Vec8<E>::load(p, x[q]);
+          Vec8<E>::load(src, x[q]);
         } else {
 #pragma unroll
           for (int e = 0; e < 8; ++e)
-            if (c0 + e < j.cols) x[q][e] = to_f32<E>(p[e]);
+            if (c0 + e < j.cols) x[q][e] = to_f32<E>(src[e]);
         }
       }
     }
 #pragma unroll
-    for (int e = 0; e < 8; ++e) part[e] += (x[0][e] + x[1][e]) + (x[2][e] + x[3][e]);
-    if (++rounds % 8 == 0) {
+    for (int e = 0; e < 8; ++e) sum[e] += x[0][e] + x[1][e];
 #pragma unroll
-      for (int e = 0; e < 8; ++e) { sum[e] += part[e]; part[e] = 0.f; }
-    }
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const long long r = row + kSplitLanes * q;
-      if (r >= r1) break;
+    for (int q = 0; q < R; ++q) {
       uint32_t hw[4], lw[4];             // the values as bf16, and what that leaves of them
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         const float a = x[q][2 * e], b = x[q][2 * e + 1];
         const __nv_bfloat162 hi = __floats2bfloat162_rn(a, b);
-        const __nv_bfloat162 lo = __floats2bfloat162_rn(a - __bfloat162float(hi.x), b - __bfloat162float(hi.y));
+        const __nv_bfloat162 lv = __floats2bfloat162_rn(a - __bfloat162float(hi.x), b - __bfloat162float(hi.y));
         hw[e] = *reinterpret_cast<const uint32_t*>(&hi);
-        lw[e] = *reinterpret_cast<const uint32_t*>(&lo);
+        lw[e] = *reinterpret_cast<const uint32_t*>(&lv);
       }
-      long long at = r;
+      if (kSplitLanes * q < left) {
+        *reinterpret_cast<uint4*>(dst) = make_uint4(hw[0], hw[1], hw[2], hw[3]);
+        if (PARTS == 2) *reinterpret_cast<uint4*>(dst + lo) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
+      }
+      dst += row_dst;
       if (PARTS == 2) {
-        while (r >= end) { ++sample; end += T; }
-        at += sample * T;
+        in_sample -= kSplitLanes;
+        while (in_sample <= 0) { in_sample += T; dst += lo; }
       }
-      __nv_bfloat16* dst = j.dst + at * j.ld + c0;
-      *reinterpret_cast<uint4*>(dst) = make_uint4(hw[0], hw[1], hw[2], hw[3]);
-      if (PARTS == 2) *reinterpret_cast<uint4*>(dst + T * j.ld) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
     }
   }
-#pragma unroll
-  for (int e = 0; e < 8; ++e) sum[e] += part[e];
 }
 
 template <int PARTS>
-__global__ void __launch_bounds__(256) split_pair_kernel(const SplitParams p) {
+__global__ void __launch_bounds__(256, 4) split_pair_kernel(const SplitParams p) {
   __shared__ float red[8][kSplitCols];
   const bool second = blockIdx.x >= p.job[0].blocks;
   const SplitJob& j = p.job[second ? 1 : 0];
@@ -196,10 +189,10 @@ __global__ void __launch_bounds__(256) split_pair_kernel(const SplitParams p) {
   if (r0 + j.per < r1) r1 = r0 + j.per;
   float sum[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   if (c0 < j.ld) {
-    if (j.is_f32 && j.vec) split_rows<float, PARTS, true>(j, p.T, r0, r1, c0, sum);
-    else if (j.is_f32) split_rows<float, PARTS, false>(j, p.T, r0, r1, c0, sum);
-    else if (j.vec) split_rows<__nv_bfloat16, PARTS, true>(j, p.T, r0, r1, c0, sum);
-    else split_rows<__nv_bfloat16, PARTS, false>(j, p.T, r0, r1, c0, sum);
+    if (j.is_f32 && j.vec) split_rows<float, PARTS, true>(j, p.part_rows, r0, r1, c0, sum);
+    else if (j.is_f32) split_rows<float, PARTS, false>(j, p.part_rows, r0, r1, c0, sum);
+    else if (j.vec) split_rows<__nv_bfloat16, PARTS, true>(j, p.part_rows, r0, r1, c0, sum);
+    else split_rows<__nv_bfloat16, PARTS, false>(j, p.part_rows, r0, r1, c0, sum);
   }
   if (!j.sums) return;
 #pragma unroll
@@ -703,8 +696,8 @@ static int pick_splits(long long Tn, long long ctas_without_split, int sm_count,
 }
 
 extern "C" int ghost_split_operands(const void* X, int x_is_f32, int x_cols, const void* Y, int y_is_f32, int y_cols, int parts,
-                                    long long samples, long long T, void* X_out, void* Y_out, float* x_sums, float* y_sums,
-                                    void* stream) {
+                                    long long samples, long long T, int merged, void* X_out, void* Y_out, float* x_sums,
+                                    float* y_sums, void* stream) {
   const DeviceState* ds = device_state();
   if (!ds) return GHOST_ERR_DEVICE;
   GB_REQUIRE((X == nullptr) == (X_out == nullptr) && (Y == nullptr) == (Y_out == nullptr) && (X || Y), "ghost_split_operands: null pointer");
@@ -716,6 +709,7 @@ extern "C" int ghost_split_operands(const void* X, int x_is_f32, int x_cols, con
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   SplitParams p = {};
   p.T = T;
+  p.part_rows = merged ? samples * T : T;
   auto fill = [&](SplitJob& j, const void* src, int f32, int cols, void* dst, float* sums) {
     j.panels = 1;
     if (!src) return;
@@ -728,12 +722,12 @@ extern "C" int ghost_split_operands(const void* X, int x_is_f32, int x_cols, con
     j.ld = (cols + 63) / 64 * 64;
     j.rows = samples * T;
     j.vec = cols % (f32 ? 4 : 8) == 0 && (reinterpret_cast<uintptr_t>(src) & 15u) == 0;
-    // 64 rows to a block (four a thread, one round of loads) while that is a few waves of blocks, more rows beyond it.
-    // Sums: a sample to a block and no atomics where that fills the GPU.
-    const long long units = sums ? T : j.rows, each = (sums ? samples : 1) * j.panels, wave = 6ll * ds->sm_count;
-    j.per = 4 * kSplitLanes;
-    if (sums && each >= wave) j.per = (units + 63) / 64 * 64;
-    while (j.per < units && (units + j.per - 1) / j.per * each > 8 * wave) j.per *= 2;
+    // 64 rows to a block (two rounds of loads) while that is a few waves of blocks, more rows beyond it.  Sums: a sample to a
+    // block and no atomics where that fills the GPU; up to 512 rows, so that a chain of additions has sixteen at most.
+    const long long units = sums ? T : j.rows, each = (sums ? samples : 1) * j.panels, wave = 4ll * ds->sm_count;
+    j.per = 64;
+    if (sums && each >= wave && T <= 512) j.per = (units + 63) / 64 * 64;
+    while (j.per < (sums ? 512 : units) && (units + j.per - 1) / j.per * each > 16 * wave) j.per *= 2;
     j.chunks = static_cast<int>((units + j.per - 1) / j.per);
     j.blocks = j.chunks * each;
   };

@@ -554,15 +554,16 @@ static int wgrad(const XtyOperands& o, long long n_rows, float scale, int accumu
 extern "C" int ghost_wgrad_bf16(const void* X, const void* Y, long long n_rows, int m_cols, int n_cols,
                                 long long ldx, long long ldy, float scale, int accumulate, void* out,
                                 int out_is_f32, void* ws, long long ws_bytes, void* stream) {
-  return wgrad(XtyOperands{{X, Y}, {m_cols, n_cols}, {ldx, ldy}, 1, false}, n_rows, scale, accumulate, out, out_is_f32, ws, ws_bytes, stream);
+  return wgrad(XtyOperands{{X, Y}, {m_cols, n_cols}, {ldx, ldy}, 1, 0, false}, n_rows, scale, accumulate, out, out_is_f32, ws, ws_bytes, stream);
 }
 
-extern "C" int ghost_wgrad_parts(const void* X, const void* Y, int parts, long long n_rows, int m_cols, int n_cols, long long ldx,
+extern "C" int ghost_wgrad_parts(const void* X, const void* Y, int parts, long long part_rows, long long n_rows, int m_cols, int n_cols, long long ldx,
                                  long long ldy, float scale, int accumulate, void* out, int out_is_f32, void* ws,
                                  long long ws_bytes, void* stream) {
   const int rc = check_parts(X, Y, parts, m_cols, n_cols, ldx, ldy);
   if (rc != GHOST_OK) return rc;
-  return wgrad(XtyOperands{{X, Y}, {m_cols, n_cols}, {ldx, ldy}, parts, true}, n_rows, scale, accumulate, out, out_is_f32, ws, ws_bytes, stream);
+  GB_REQUIRE(part_rows >= n_rows, "ghost_wgrad_parts: more rows than a part has");
+  return wgrad(XtyOperands{{X, Y}, {m_cols, n_cols}, {ldx, ldy}, parts, part_rows, true}, n_rows, scale, accumulate, out, out_is_f32, ws, ws_bytes, stream);
 }
 
 namespace gb {
@@ -708,7 +709,7 @@ extern "C" int ghost_persample_dot_bf16(const void* X, const void* Y, int n_trai
                                         int colsum_of, float* colsum_out,
                                         void* ws, long long ws_bytes, void* stream) {
   const XtyColsum cs = {colsum_of, colsum_out};
-  return persample_dot(XtyOperands{{X, Y}, {m_cols, n_cols}, {ldx, ldy}, 1, false}, n_train, n_val, T, dot_scale, M_out, v_is_f32,
+  return persample_dot(XtyOperands{{X, Y}, {m_cols, n_cols}, {ldx, ldy}, 1, 0, false}, n_train, n_val, T, dot_scale, M_out, v_is_f32,
                        grad_out, grad_is_f32, grad_scale, grad_accumulate, cs, ws, ws_bytes, stream);
 }
 
@@ -719,7 +720,7 @@ extern "C" int ghost_persample_dot_parts(const void* X, const void* Y, int parts
   const int rc = check_parts(X, Y, parts, m_cols, n_cols, ldx, ldy);
   if (rc != GHOST_OK) return rc;
   const XtyColsum cs = {colsum_of, colsum_out};
-  return persample_dot(XtyOperands{{X, Y}, {m_cols, n_cols}, {ldx, ldy}, parts, true}, n_train, n_val, T, dot_scale, M_out,
+  return persample_dot(XtyOperands{{X, Y}, {m_cols, n_cols}, {ldx, ldy}, parts, 0, true}, n_train, n_val, T, dot_scale, M_out,
                        parts == 2 ? 1 : 0, grad_out, grad_is_f32, grad_scale, grad_accumulate, cs, ws, ws_bytes, stream);
 }
 
@@ -766,7 +767,7 @@ extern "C" int ghost_persample_tiles_bf16(const void* X, const void* Y, int n_sa
   p.samples = samples;
   p.sample0 = sample0;
   p.vgrad = tiles_out;
-  const XtyOperands o = {{X, Y}, {m_cols, n_cols}, {ldx, ldy}, 1, false};
+  const XtyOperands o = {{X, Y}, {m_cols, n_cols}, {ldx, ldy}, 1, 0, false};
   if (pair_kernel_fits(g_persample_pair_mode, o, ds))
     return launch_xty_pair_tiles(o, n_samples_total, T, samples, sample0, tiles_out, 0, p.cs, nullptr, 0, ds, st);
   return launch_xty(o, n_samples_total, T, p, ds, st);

@@ -9,6 +9,7 @@ struct XtyOperands {
   int cols[2];
   long long ld[2];         // row pitch
   int parts;
+  long long part_rows;     // rows of a part in memory (parts == 2); 0: those that are read
   // Whether one TMA box may cover several 64-column blocks: the columns are a multiple of 64, or the rows are zero
   // up to the next one (`padded`, which the split layout always is).
   bool padded;
@@ -32,7 +33,7 @@ inline int xty_colsum_clear(const XtyColsum& cs, int parts, int sample0, int sam
 
 // Map of operand i for boxes of `rows_box` tokens and `blocks` 64-column blocks (both parts of a split operand)
 inline int xty_operand_map(CUtensorMap* t, const XtyOperands& o, int i, long long samples, long long rows, int rows_box, int blocks) {
-  if (o.parts == 2) return make_tmap_bf16_parts(t, o.ptr[i], samples, rows, o.ld[i], rows_box, blocks);
+  if (o.parts == 2) return make_tmap_bf16_parts(t, o.ptr[i], samples, o.part_rows ? o.part_rows : rows, rows, o.ld[i], rows_box, blocks);
   if (!o.blocked(i)) return make_tmap_bf16_3d(t, o.ptr[i], samples, rows, o.cols[i], o.ld[i], rows_box);
   return make_tmap_bf16_blocks(t, o.ptr[i], samples, rows, o.padded_cols(i), o.ld[i], rows_box, blocks);
 }

@@ -65,12 +65,13 @@ int ghost_cast_split_bf16(const void* src, int src_is_f32, long long samples, lo
 
 /* Both operands of a GEMM over tokens in one launch: X [samples, T, x_cols] and Y [samples, T, y_cols] (dense, fp32
  * or bf16; either may be NULL with its destination) as [samples, parts, T, cols rounded up to 64] bf16, zero-padded:
- * the values, and with parts = 2 behind each sample's values their residuals bf16(x - bf16(x)).  This is the layout of
- * ghost_persample_dot_parts and ghost_wgrad_parts (samples = 1 and T = all rows there).  x_sums / y_sums, if not
+ * the values, and with parts = 2 behind each sample's values their residuals bf16(x - bf16(x)); `merged` lays out
+ * [parts, samples * T, ld] instead.  The first is the layout of ghost_persample_dot_parts, the second that of
+ * ghost_wgrad_parts and ghost_gram_dot_parts.  x_sums / y_sums, if not
  * NULL, receive the operand's column sums per sample (fp32, [samples, cols]) on the way.  Same reference lines. */
 int ghost_split_operands(const void* X, int x_is_f32, int x_cols, const void* Y, int y_is_f32, int y_cols, int parts,
-                         long long samples, long long T, void* X_out, void* Y_out, float* x_sums, float* y_sums,
-                         void* stream);
+                         long long samples, long long T, int merged, void* X_out, void* Y_out, float* x_sums,
+                         float* y_sums, void* stream);
 
 /* The same from a convolution operand: token (oy, ox) of sample n holds the C * kh * kw inputs of
  * src [samples, C, H, W] (dense) under the kernel window, in the order of torch's unfold; tokens per
@@ -97,9 +98,16 @@ int ghost_gram_dot_bf16(const void* a_train, const void* a_val, const void* g_tr
                         long long ld_at, long long ld_av, long long ld_gt, long long ld_gv,
                         int round_mode, float scale, float* M_out, void* stream);
 
-/* Selects the kernel behind ghost_gram_dot_bf16: 0 = one CTA per 128 x 256 tile; 1 (default) = a
- * CTA pair (tcgen05 cta_group::2) per 256 x 256 tile for problems of at least 512 train tokens and
- * 256 to 8192 validation tokens; 2 = the pair kernel from 512 x 256 tokens up.  Process-wide. */
+/* The same over operands as ghost_split_operands lays them out merged: A [parts, (n_train + n_val) * T, ld_a],
+ * train samples first.  parts = 2 contracts value x value + value x residual + residual x value (pitches that are
+ * multiples of 64, zero beyond the columns). */
+int ghost_gram_dot_parts(const void* A, const void* G, int parts, int n_train, int n_val, long long T, int d, int p,
+                         long long ld_a, long long ld_g, int round_mode, float scale, float* M_out, void* stream);
+
+/* Selects the kernels behind ghost_gram_dot_bf16: 0 = one CTA per tile of 128 x 256 (or 128); 1 (default) = also a
+ * CTA pair (tcgen05 cta_group::2) per 256 x 256 tile for problems of at least 512 train tokens and 256 to 8192
+ * validation tokens, unless smaller tiles fill the GPU better; 2 = the pair kernel from 512 x 256 tokens up.
+ * Process-wide. */
 int ghost_set_gram_pair_mode(int mode);
 
 /* ---- train-gradient recovery ------------------------------------------------------------------- */
@@ -114,10 +122,11 @@ int ghost_wgrad_bf16(const void* X, const void* Y, long long n_rows, int m_cols,
                      long long ldx, long long ldy, float scale, int accumulate, void* out,
                      int out_is_f32, void* ws, long long ws_bytes, void* stream);
 
-/* The same over operands as ghost_split_operands lays them out: X [parts, n_rows, ldx], the pitch a multiple of 64
+/* The same over operands as ghost_split_operands lays them out: X [parts, part_rows, ldx] (the first
+ * n_rows of a part are read), the pitch a multiple of 64
  * and zero beyond the columns (parts = 1: an operand whose pitch is smaller than that is read as it is).
  * parts = 2 contracts value x value + value x residual + residual x value. */
-int ghost_wgrad_parts(const void* X, const void* Y, int parts, long long n_rows, int m_cols, int n_cols, long long ldx,
+int ghost_wgrad_parts(const void* X, const void* Y, int parts, long long part_rows, long long n_rows, int m_cols, int n_cols, long long ldx,
                       long long ldy, float scale, int accumulate, void* out, int out_is_f32, void* ws, long long ws_bytes,
                       void* stream);
 

@@ -54,6 +54,27 @@ def test_gram_dot(case, dtype):
     assert O.rel_fro(M, ref) < TOL[dtype]
 
 
+# token counts on both sides of what chooses the tile shape: one tile of 128 x 128, fewer tiles of 256 x 256 than CTA
+# pairs, a full round of them; both operands and their sums through the layer's hook, which shares their copies
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("case", [(2, 1, 17, 63, 65), (5, 4, 64, 130, 64), (4, 2, 512, 96, 72), (40, 10, 100, 64, 200), (300, 40, 31, 65, 70)])
+@pytest.mark.parametrize("in_by_out", [False, True])
+def test_gram_hook_tile_shapes(in_by_out, case, dtype):
+    n_t, n_v, T, d, p = case
+    A, G = make(n_t + n_v, T, d, p, dtype, seed=33)
+    M, grad, sums, _, _ = ops().dense_hook(A.cuda(), G.cuda(), n_v, in_by_out, True, torch.float32, 0.5, True, torch.float32, False, True)
+    after()
+    S = torch.einsum("ntp,ntd->npd", G.cuda().double(), A.cuda().double()).flatten(1)
+    ref, gref = S[n_t:] @ S[:n_t].t(), 0.5 * S[:n_t].sum(0).view(p, d)
+    # entries cancel over the token pairs: errors are relative to the norms of the pair's gradients.  float32 carries two
+    # parts of 8 bits; a Gram entry sums d (p) products in float32 that the tensor core truncates
+    tol = (2 * 2.0 ** -16 if dtype == torch.float32 else 0.) + max(d, p) * 2.0 ** -23
+    scale = (A.cuda().double().flatten(1).norm(dim=1) * G.cuda().double().flatten(1).norm(dim=1))
+    assert ((M.double() - ref).abs() <= tol * scale[n_t:, None] * scale[None, :n_t]).all()
+    assert O.rel_fro(grad if not in_by_out else grad.t(), gref) < 2 * 2.0 ** -16 + T * n_t * 2.0 ** -23
+    assert O.rel_fro(sums, G.double().sum(1)) < 1e-6
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("case", [(5, 3, 130, 72, 40), (4, 2, 256, 128, 64), (9, 2, 300, 200, 136),
                                   (700, 300, 1, 64, 48), (3, 5, 513, 96, 256)])
