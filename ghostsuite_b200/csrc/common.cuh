@@ -93,6 +93,9 @@ int make_tmap_bf16_store_2d(CUtensorMap* out, const void* base, uint64_t rows, u
 // The same for fp32: boxes of [box_rows, 32 columns] (128-byte rows) written with the 128-byte swizzle, chunk c of row r at
 // r * 128 + ((c ^ (r & 7)) * 16).
 int make_tmap_f32_store_2d(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows);
+// 2-D map of a row-major matrix of 2- or 4-byte elements for boxes of 128 bytes of columns and `box_rows` rows with the
+// 128-byte swizzle.  Coordinates: (column, row).
+int make_tmap_rows(CUtensorMap* out, const void* base, int elem_bytes, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows);
 // Per-sample fp32 tiles [tiles][samples][32768], seen as [tiles, 1024 panels, samples, 32]: a box holds
 // eight panels (256 elements) of `box_rows` samples, each panel a swizzled [box_rows][32] block.
 // Coordinates: (0, sample, panel, tile).

@@ -802,6 +802,25 @@ def test_projection_similarity_block_shapes(case, dtype):
     assert (err <= 2.0 ** -15 * a.double().norm(dim=1)[:, None] * b.double().norm(dim=1)[None]).all()
 
 
+# one stage, one cluster and many of them; rows that TMA reads and rows that it cannot (odd lengths, odd pitches), each at
+# the ends of a panel of 32 floats / 64 bf16 elements; scores with and without whole 16-byte pieces per row
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("D", [8, 31, 256, 257, 2055, 4096, 65536 + 24, 65536 + 25])
+@pytest.mark.parametrize("n", [(2, 3), (18, 74), (40, 33), (64, 64)])
+def test_projection_similarity_splits_and_pitches(n, D, dtype):
+    g = torch.Generator(device="cuda").manual_seed(24)
+    a, b = (torch.randn(k, D, generator=g, device="cuda").to(dtype) for k in n)
+    wide = torch.full((n[0], D + 3), 1e30, device="cuda").to(dtype)
+    wide[:, 2:2 + D] = a
+    ref = a.double() @ b.double().t()
+    bound = 2.0 ** -15 * a.double().norm(dim=1)[:, None] * b.double().norm(dim=1)[None]
+    for rows in (a, wide[:, 2:2 + D]):
+        S = ops().projection_similarity(rows, b)
+        after()
+        assert ((S.double() - ref).abs() <= bound).all()
+
+
+
 def test_small_reduce_batch_matches_single_launches():
     """One batched launch for many layers' small reductions against the per-layer kernels: more jobs
     than fit one launch, mixed sizes, Gram only / sum only / both, bf16 and fp32 sums."""
