@@ -28,6 +28,7 @@ template <> __device__ __forceinline__ float ct_f32<__nv_bfloat16>(__nv_bfloat16
 // once an element.  The library unfold before it ran one launch per sample and two more passes: 575 us.
 template <typename E>
 __global__ void __launch_bounds__(256) conv_tokens_kernel(const ConvTokens q) {
+  stream_order();
   __shared__ float tile[64][65];
   __shared__ long long s_off[64];        // of a feature: channel and window position as an offset into the sample
   __shared__ int2 s_ij[64];              // and the position alone; far outside for the padding features
@@ -99,6 +100,7 @@ __global__ void __launch_bounds__(256) conv_tokens_kernel(const ConvTokens q) {
 // One warp per row; the rows are contiguous, so the loads are.
 template <typename E>
 __global__ void __launch_bounds__(256) row_sums_kernel(const E* __restrict__ x, long long rows, long long len, float* __restrict__ out) {
+  stream_order();
   const long long r = blockIdx.x * 8ll + (threadIdx.x >> 5);
   if (r >= rows) return;
   float s = 0.f;
@@ -143,8 +145,8 @@ extern "C" int ghost_conv_tokens_bf16(const void* src, int src_is_f32, long long
   q.row_stack = row_stack;
   const dim3 grid(ceil_div(q.T, 64), ceil_div(cpad, 64), static_cast<unsigned>(samples));
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (src_is_f32) conv_tokens_kernel<float><<<grid, 256, 0, st>>>(q);
-  else conv_tokens_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(q);
+  if (src_is_f32) GB_CUDA_OK(launch_next(conv_tokens_kernel<float>, dim3(grid), dim3(256), 0, st, q));
+  else GB_CUDA_OK(launch_next(conv_tokens_kernel<__nv_bfloat16>, dim3(grid), dim3(256), 0, st, q));
   count_launch();
   return post_launch("conv_tokens_kernel");
 }
@@ -155,8 +157,8 @@ extern "C" int ghost_row_sums(const void* x, int is_f32, long long rows, long lo
   GB_REQUIRE(x && out && rows > 0 && len > 0 && rows < (1ll << 33), "ghost_row_sums: bad arguments");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const unsigned grid = static_cast<unsigned>((rows + 7) / 8);
-  if (is_f32) row_sums_kernel<float><<<grid, 256, 0, st>>>(static_cast<const float*>(x), rows, len, out);
-  else row_sums_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(static_cast<const __nv_bfloat16*>(x), rows, len, out);
+  if (is_f32) GB_CUDA_OK(launch_next(row_sums_kernel<float>, dim3(grid), dim3(256), 0, st, static_cast<const float*>(x), rows, len, out));
+  else GB_CUDA_OK(launch_next(row_sums_kernel<__nv_bfloat16>, dim3(grid), dim3(256), 0, st, static_cast<const __nv_bfloat16*>(x), rows, len, out));
   count_launch();
   return post_launch("row_sums_kernel");
 }

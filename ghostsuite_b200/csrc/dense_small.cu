@@ -84,6 +84,7 @@ __device__ __forceinline__ float sd_gram(const E* X, int K, long long row_v, int
 
 template <typename E, bool VEC>
 __global__ void __launch_bounds__(256, 2) dense_small_kernel(const SmallDense q) {
+  stream_order();
   __shared__ __align__(16) float sm[2 * 2 * 16 * 64];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const E* A = static_cast<const E*>(q.A);
@@ -277,11 +278,11 @@ extern "C" int ghost_dense_small(const void* A, const void* B, int is_f32, int n
   const unsigned grid = static_cast<unsigned>(gram + wgrad + col);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (is_f32) {
-    if (vec) dense_small_kernel<float, true><<<grid, 256, 0, st>>>(q);
-    else dense_small_kernel<float, false><<<grid, 256, 0, st>>>(q);
+    if (vec) GB_CUDA_OK(launch_next(dense_small_kernel<float, true>, dim3(grid), dim3(256), 0, st, q));
+    else GB_CUDA_OK(launch_next(dense_small_kernel<float, false>, dim3(grid), dim3(256), 0, st, q));
   } else {
-    if (vec) dense_small_kernel<__nv_bfloat16, true><<<grid, 256, 0, st>>>(q);
-    else dense_small_kernel<__nv_bfloat16, false><<<grid, 256, 0, st>>>(q);
+    if (vec) GB_CUDA_OK(launch_next(dense_small_kernel<__nv_bfloat16, true>, dim3(grid), dim3(256), 0, st, q));
+    else GB_CUDA_OK(launch_next(dense_small_kernel<__nv_bfloat16, false>, dim3(grid), dim3(256), 0, st, q));
   }
   count_launch();
   return post_launch("dense_small_kernel");

@@ -113,6 +113,7 @@ ghost_gram_kernel(const __grid_constant__ CUtensorMap tm_at, const __grid_consta
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  stream_order();
 
   if (warp == 4) {
     // ------------------------------------------------------------------ TMA producer
@@ -327,7 +328,7 @@ static int launch_gram(const GramOperands& o, int n_train, int n_val, long long 
   }
   const long long tiles = static_cast<long long>(p.m_tiles) * p.n_tiles;
   const int grid = static_cast<int>(tiles < ds->sm_count ? tiles : ds->sm_count);
-  ghost_gram_kernel<BN, PARTS><<<grid, 192, Cfg::kSmemBytes, stream>>>(t[0], t[1], t[2], t[3], p);
+  GB_CUDA_OK(launch_next(ghost_gram_kernel<BN, PARTS>, dim3(grid), dim3(192), Cfg::kSmemBytes, stream, t[0], t[1], t[2], t[3], p));
   count_launch();
   return post_launch("ghost_gram_kernel");
 }

@@ -100,6 +100,7 @@ ghost_gram_pair_kernel(const __grid_constant__ CUtensorMap tm_at, const __grid_c
   cluster_sync_all();          // both CTAs' barriers are initialised before anyone signals them
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  stream_order();
 
   if (warp == 4) {
     // ------------------------------------------------------------------ TMA producer (both CTAs)
@@ -283,7 +284,7 @@ static int launch_gram_pair_t(const CUtensorMap (&t)[4], const GramPairParams& p
   const long long tiles = static_cast<long long>(p.m_tiles) * p.n_tiles;
   long long pairs = ds->sm_count / 2;
   if (pairs > tiles) pairs = tiles;
-  ghost_gram_pair_kernel<PARTS><<<static_cast<int>(2 * pairs), 192, Cfg::kSmemBytes, stream>>>(t[0], t[1], t[2], t[3], p);
+  GB_CUDA_OK(launch_next(ghost_gram_pair_kernel<PARTS>, dim3(static_cast<int>(2 * pairs)), dim3(192), Cfg::kSmemBytes, stream, t[0], t[1], t[2], t[3], p));
   count_launch();
   return post_launch("ghost_gram_pair_kernel");
 }

@@ -231,6 +231,7 @@ gradproj_kernel(const __grid_constant__ CUtensorMap tm_g, const __grid_constant_
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  stream_order();
 
   if (warp == 4) {
     // Producer warp.  Lane 0 owns the barriers; each of the first lanes issues the TMA of one box -- activation
@@ -549,17 +550,18 @@ static int launch_gradproj_t(const CUtensorMap& tg, const CUtensorMap& tpr, cons
     attr_set[ds->device] = true;
   }
   cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr;
+  cudaLaunchAttribute attr[2];
+  cfg.attrs = attr;
+  cfg.numAttrs = early_start(attr, st);
   cfg.blockDim = dim3(Cfg::kThreads, 1, 1);
   cfg.dynamicSmemBytes = Cfg::kSmemBytes;
   cfg.stream = st;
   if (kCluster) {
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = ranks;
-    attr.val.clusterDim.y = 1;
-    attr.val.clusterDim.z = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
+    cudaLaunchAttribute& cluster = attr[cfg.numAttrs++];
+    cluster.id = cudaLaunchAttributeClusterDimension;
+    cluster.val.clusterDim.x = ranks;
+    cluster.val.clusterDim.y = 1;
+    cluster.val.clusterDim.z = 1;
     cfg.gridDim = dim3(static_cast<unsigned>(p.units * ranks), 1, 1);
   } else {
     const int grid = static_cast<int>(p.units < ds->sm_count ? p.units : ds->sm_count);

@@ -136,6 +136,7 @@ __global__ void __cluster_dims__(kPassCluster, 1, 1) __launch_bounds__(kPassThre
 pass_reduce_kernel(const __grid_constant__ PassJobs<CAP> jobs) {
   extern __shared__ __align__(16) float stage[];       // pass_smem(sub) bytes
   const int pitch = pass_pitch(jobs.sub);
+  stream_order();
   __shared__ float part[2][8][32];       // this CTA's share of F, read by rank 0 of the cluster
   __shared__ float cols[8][32];
   const ghost_pass_job& j = jobs.job[blockIdx.z];
@@ -240,6 +241,7 @@ pass_reduce_kernel(const __grid_constant__ PassJobs<CAP> jobs) {
 // 16384 x 1 of 1024: 49 and 19.  Smaller ones, and every matrix of a batch, stay with the clusters, which fetch a row once.
 __global__ void __launch_bounds__(256) small_gram_kernel(const float* __restrict__ X, int n_train, unsigned pairs, int F,
                                                          float scale, float* __restrict__ M) {
+  stream_order();
   const unsigned pair = blockIdx.x * 8u + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (pair >= pairs) return;
@@ -287,6 +289,7 @@ __global__ void __launch_bounds__(256) small_gram_kernel(const float* __restrict
 template <int COLS>
 __global__ void __launch_bounds__(256) rows_sum_kernel(const float* __restrict__ X, int n_rows, int F, float scale,
                                                        void* __restrict__ out, int out_is_f32, int accumulate) {
+  stream_order();
   constexpr int PER = COLS / 32;
   __shared__ float red[8][COLS];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -334,7 +337,7 @@ static int launch_pass(const ghost_pass_job* jobs, int n, int blocks, const Devi
   const int sub = (pass_chunk(longest) + 31) / 32 * 32;
   // the row sums of longer lists reduce 8 x 4 x 128 partial sums in the same memory
   batch.sub = sub < 128 ? 128 : sub > kPassMost ? kPassMost : sub;
-  pass_reduce_kernel<CAP><<<dim3(kPassCluster, blocks, n), kPassThreads, pass_smem(batch.sub), st>>>(batch);
+  GB_CUDA_OK(launch_next(pass_reduce_kernel<CAP>, dim3(dim3(kPassCluster, blocks, n)), dim3(kPassThreads), pass_smem(batch.sub), st, batch));
   count_launch();
   return post_launch("pass_reduce_kernel");
 }
@@ -348,6 +351,7 @@ struct MatrixList { const float* m[kSumPointers]; };
 __global__ void __launch_bounds__(1024)
 matrix_sum_kernel(const __grid_constant__ MatrixList list, int n, int n_val, int n_train, int accumulate,
                   float* total, float* vec, const int* err_word, int* err_out) {
+  stream_order();
   __shared__ float red[4][8][32];
   __shared__ float cols[8][32];
   const int lane = threadIdx.x & 31, row = (threadIdx.x >> 5) & 7, grp = threadIdx.x >> 8;
@@ -452,7 +456,7 @@ extern "C" int ghost_small_gram_f32(const float* X, int n_train, int n_val, int 
   }
   if (!device_state()) return GHOST_ERR_DEVICE;
   GB_REQUIRE(pairs < (1ll << 32) - 8, "ghost_small_gram_f32: too many pairs");
-  small_gram_kernel<<<ceil_div(pairs, 8), 256, 0, static_cast<cudaStream_t>(stream)>>>(X, n_train, static_cast<unsigned>(pairs), F, scale, M_out);
+  GB_CUDA_OK(launch_next(small_gram_kernel, dim3(ceil_div(pairs, 8)), dim3(256), 0, static_cast<cudaStream_t>(stream), X, n_train, static_cast<unsigned>(pairs), F, scale, M_out));
   count_launch();
   return post_launch("small_gram_kernel");
 }
@@ -466,9 +470,9 @@ extern "C" int ghost_rows_sum(const float* X, int n_rows, int F, float scale, vo
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   // wide blocks read full lines; narrow ones while a row has too few for the GPU
   if (ceil_div(F, 128) >= ds->sm_count)
-    rows_sum_kernel<128><<<ceil_div(F, 128), 256, 0, st>>>(X, n_rows, F, scale, out, out_is_f32, accumulate);
+    GB_CUDA_OK(launch_next(rows_sum_kernel<128>, dim3(ceil_div(F, 128)), dim3(256), 0, st, X, n_rows, F, scale, out, out_is_f32, accumulate));
   else
-    rows_sum_kernel<32><<<ceil_div(F, 32), 256, 0, st>>>(X, n_rows, F, scale, out, out_is_f32, accumulate);
+    GB_CUDA_OK(launch_next(rows_sum_kernel<32>, dim3(ceil_div(F, 32)), dim3(256), 0, st, X, n_rows, F, scale, out, out_is_f32, accumulate));
   count_launch();
   return post_launch("rows_sum_kernel");
 }
@@ -485,8 +489,8 @@ extern "C" int ghost_matrix_sum(const float* const* mats, int n_mats, int n_val,
     MatrixList list;
     memcpy(list.m, mats + first, sizeof(float*) * n);
     const bool last = first + n == n_mats;
-    matrix_sum_kernel<<<ceil_div(n_train, 32), 1024, 0, st>>>(list, n, n_val, n_train, first > 0 ? 1 : 0, total, vec,
-                                                              ds->err_word, last ? err_out : nullptr);
+    GB_CUDA_OK(launch_next(matrix_sum_kernel, dim3(ceil_div(n_train, 32)), dim3(1024), 0, st, list, n, n_val, n_train, first > 0 ? 1 : 0, total, vec,
+                                                              ds->err_word, last ? err_out : nullptr));
     count_launch();
     const int rc = post_launch("matrix_sum_kernel");
     if (rc != GHOST_OK) return rc;

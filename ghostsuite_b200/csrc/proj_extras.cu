@@ -123,6 +123,7 @@ __global__ void __launch_bounds__(256, 2) proj_similarity_kernel(const SimParams
   constexpr int BM = 16 * MT * WM, BN = 8 * NT * WN;
   constexpr bool kSplit = sizeof(PT) == 4;
   __shared__ __align__(16) float part[WK * BM * BN];
+  stream_order();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, c = lane & 3;
   const int wk = warp / (WM * WN), wm = warp % (WM * WN) / WN, wn = warp % WN;
@@ -257,6 +258,7 @@ proj_similarity_tma_kernel(const __grid_constant__ CUtensorMap tm_a, const __gri
   }
   if (warp == 8 && lane == 0) { tma_prefetch_desc(&tm_a); tma_prefetch_desc(&tm_b); }
   __syncthreads();
+  stream_order();
 
   float acc[MT][NT][4];
   if (warp >= 8) {
@@ -369,17 +371,20 @@ static int sim_launch(K kernel, const SimParams& p, SimGrid g, int bi, int bj, i
   if (!p.direct)
     GB_CUDA_OK(cudaMemset2DAsync(p.S, static_cast<size_t>(p.ld_s) * 4, 0, static_cast<size_t>(p.n2) * 4, static_cast<size_t>(p.n1), st));
   cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr;
+  cudaLaunchAttribute attr[2];
   cfg.gridDim = dim3(static_cast<unsigned>(g.splits), static_cast<unsigned>(bi), static_cast<unsigned>(bj));
   cfg.blockDim = dim3(threads, 1, 1);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = g.ranks;
-  attr.val.clusterDim.y = 1;
-  attr.val.clusterDim.z = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = g.ranks > 1 ? 1 : 0;
+  cfg.attrs = attr;
+  cfg.numAttrs = early_start(attr, st);
+  if (g.ranks > 1) {
+    cudaLaunchAttribute& cluster = attr[cfg.numAttrs++];
+    cluster.id = cudaLaunchAttributeClusterDimension;
+    cluster.val.clusterDim.x = g.ranks;
+    cluster.val.clusterDim.y = 1;
+    cluster.val.clusterDim.z = 1;
+  }
   GB_CUDA_OK(cudaLaunchKernelEx(&cfg, kernel, args...));
   count_launch();
   return post_launch("proj_similarity_kernel");

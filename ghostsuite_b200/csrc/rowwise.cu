@@ -57,6 +57,7 @@ struct CastParams {
 // operands of 29 samples of 197 x (768, 1000) float32: 18.8 us before, 14.4 now).
 template <typename T, typename I>
 __global__ void cast_split_kernel(const CastParams p) {
+  stream_order();
   const I cvec = static_cast<I>(p.cpad / 8);
   const I total = static_cast<I>(p.samples * p.T) * cvec;
   const bool stacked = p.row_stack && p.parts > 1;
@@ -175,6 +176,7 @@ __device__ __forceinline__ void split_rows(const SplitJob& j, long long T, long 
 template <int PARTS>
 __global__ void __launch_bounds__(256, 4) split_pair_kernel(const SplitParams p) {
   __shared__ float red[8][kSplitCols];
+  stream_order();
   const bool second = blockIdx.x >= p.job[0].blocks;
   const SplitJob& j = p.job[second ? 1 : 0];
   const unsigned at = blockIdx.x - (second ? static_cast<unsigned>(p.job[0].blocks) : 0u);
@@ -218,6 +220,7 @@ __global__ void colsum_kernel(const T* __restrict__ G, long long Tn, int cols, l
                               float* __restrict__ out, int t_splits) {
   // block: 32 column vectors (256 columns) x 8 row lanes
   __shared__ float red[8][256 + 8];
+  stream_order();
   const int n = blockIdx.z;
   const int split = blockIdx.y;
   const int cx = threadIdx.x & 31, ry = threadIdx.x >> 5;
@@ -316,6 +319,7 @@ __global__ void __launch_bounds__(256, NCHUNK <= 3 ? 2 : 1)
 layernorm_persample_kernel(const T* __restrict__ A, const T* __restrict__ G, long long Tn, int F,
                            float eps, float* __restrict__ gw, float* __restrict__ gb,
                            float* __restrict__ part, int t_splits, int rms) {
+  stream_order();
   extern __shared__ __align__(16) unsigned char sm_raw[];   // rings [8 warps][3][2][F] of T, then [8][2][F] floats
   float* sm = reinterpret_cast<float*>(sm_raw);
   const int n = blockIdx.y, split = blockIdx.x;
@@ -435,6 +439,7 @@ layernorm_persample_kernel(const T* __restrict__ A, const T* __restrict__ G, lon
 // second stage: sum the per-split partials in a fixed order (deterministic)
 __global__ void layernorm_reduce_kernel(const float* __restrict__ part, int N, int F, int t_splits,
                                         float* __restrict__ gw, float* __restrict__ gb) {
+  stream_order();
   const long long total = static_cast<long long>(N) * 2 * F;
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
        i += static_cast<long long>(gridDim.x) * blockDim.x) {
@@ -463,6 +468,7 @@ norm_wide_kernel(const T* __restrict__ A, const T* __restrict__ G, long long Tn,
   // error of the kernel before (4096 rows of 8192 in nine splits: 3.9e-7 against 2.3e-7; 1.5e-7 now).
   constexpr int kChain = 32;
   __shared__ float red[2][R][W];
+  stream_order();
   extern __shared__ float s_total[];     // [2][PT][THREADS]: a thread's own totals, where they cost no registers
   const int n = blockIdx.y, split = blockIdx.x;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -676,11 +682,11 @@ extern "C" int ghost_cast_split_bf16(const void* src, int src_is_f32, long long 
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int grid = static_cast<int>(blocks);
   if (total < (1ll << 31) && samples * T < (1ll << 31)) {      // a grid stride further still fits 32 bits
-    if (src_is_f32) cast_split_kernel<float, unsigned><<<grid, 256, 0, st>>>(p);
-    else cast_split_kernel<__nv_bfloat16, unsigned><<<grid, 256, 0, st>>>(p);
+    if (src_is_f32) GB_CUDA_OK(launch_next(cast_split_kernel<float, unsigned>, dim3(grid), dim3(256), 0, st, p));
+    else GB_CUDA_OK(launch_next(cast_split_kernel<__nv_bfloat16, unsigned>, dim3(grid), dim3(256), 0, st, p));
   } else {
-    if (src_is_f32) cast_split_kernel<float, long long><<<grid, 256, 0, st>>>(p);
-    else cast_split_kernel<__nv_bfloat16, long long><<<grid, 256, 0, st>>>(p);
+    if (src_is_f32) GB_CUDA_OK(launch_next(cast_split_kernel<float, long long>, dim3(grid), dim3(256), 0, st, p));
+    else GB_CUDA_OK(launch_next(cast_split_kernel<__nv_bfloat16, long long>, dim3(grid), dim3(256), 0, st, p));
   }
   count_launch();
   return post_launch("cast_split_kernel");
@@ -737,8 +743,8 @@ extern "C" int ghost_split_operands(const void* X, int x_is_f32, int x_cols, con
   GB_REQUIRE(blocks < (1ll << 31), "ghost_split_operands: too many rows");
   for (const SplitJob& j : p.job)
     if (j.sums && j.chunks > 1) GB_CUDA_OK(cudaMemsetAsync(j.sums, 0, sizeof(float) * static_cast<size_t>(samples) * j.cols, st));
-  if (parts == 1) split_pair_kernel<1><<<static_cast<unsigned>(blocks), 256, 0, st>>>(p);
-  else split_pair_kernel<2><<<static_cast<unsigned>(blocks), 256, 0, st>>>(p);
+  if (parts == 1) GB_CUDA_OK(launch_next(split_pair_kernel<1>, dim3(static_cast<unsigned>(blocks)), dim3(256), 0, st, p));
+  else GB_CUDA_OK(launch_next(split_pair_kernel<2>, dim3(static_cast<unsigned>(blocks)), dim3(256), 0, st, p));
   count_launch();
   return post_launch("split_pair_kernel");
 }
@@ -754,8 +760,8 @@ extern "C" int ghost_colsum(const void* G, int is_f32, int N, long long T, int c
   const int splits = pick_splits(T, static_cast<long long>(cblocks) * N, ds->sm_count, 64);
   if (splits > 1) GB_CUDA_OK(cudaMemsetAsync(out, 0, sizeof(float) * static_cast<size_t>(N) * cols, st));
   dim3 grid(cblocks, splits, N);
-  if (is_f32) colsum_kernel<float><<<grid, 256, 0, st>>>(static_cast<const float*>(G), T, cols, ld, out, splits);
-  else colsum_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(static_cast<const __nv_bfloat16*>(G), T, cols, ld, out, splits);
+  if (is_f32) GB_CUDA_OK(launch_next(colsum_kernel<float>, dim3(grid), dim3(256), 0, st, static_cast<const float*>(G), T, cols, ld, out, splits));
+  else GB_CUDA_OK(launch_next(colsum_kernel<__nv_bfloat16>, dim3(grid), dim3(256), 0, st, static_cast<const __nv_bfloat16*>(G), T, cols, ld, out, splits));
   count_launch();
   return post_launch("colsum_kernel");
 }
@@ -790,7 +796,7 @@ static int launch_norm_wide_of(dim3 grid, const T* A, const T* G, long long Tn, 
     GB_CUDA_OK(cudaFuncSetAttribute(norm_wide_kernel<T, VEC, PT, THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
     attr_set[ds->device] = true;
   }
-  norm_wide_kernel<T, VEC, PT, THREADS><<<grid, THREADS, kSmem, st>>>(A, G, Tn, F, eps, gw, gb, ws, splits, rms);
+  GB_CUDA_OK(launch_next(norm_wide_kernel<T, VEC, PT, THREADS>, dim3(grid), dim3(THREADS), kSmem, st, A, G, Tn, F, eps, gw, gb, ws, splits, rms));
   return GHOST_OK;
 }
 template <typename T, bool VEC>
@@ -810,7 +816,7 @@ static int launch_ln_warp(dim3 grid, size_t smem, const T* A, const T* G, long l
     GB_CUDA_OK(cudaFuncSetAttribute(layernorm_persample_kernel<T, NCHUNK, FULL>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     attr_set[ds->device] = true;
   }
-  layernorm_persample_kernel<T, NCHUNK, FULL><<<grid, 256, smem, st>>>(A, G, Tn, F, eps, gw, gb, ws, splits, rms);
+  GB_CUDA_OK(launch_next(layernorm_persample_kernel<T, NCHUNK, FULL>, dim3(grid), dim3(256), smem, st, A, G, Tn, F, eps, gw, gb, ws, splits, rms));
   return GHOST_OK;
 }
 
@@ -849,7 +855,7 @@ static int launch_ln(const T* A, const T* G, int N, long long Tn, int F, float e
     const long long total = static_cast<long long>(N) * 2 * F;
     long long blocks = (total + 255) / 256;
     if (blocks > ds->sm_count * 8) blocks = ds->sm_count * 8;
-    layernorm_reduce_kernel<<<static_cast<int>(blocks), 256, 0, st>>>(ws, N, F, splits, gw, gb);
+    GB_CUDA_OK(launch_next(layernorm_reduce_kernel, dim3(static_cast<int>(blocks)), dim3(256), 0, st, ws, N, F, splits, gw, gb));
     count_launch();
     return post_launch("layernorm_reduce_kernel");
   }

@@ -108,6 +108,7 @@ tile_dot_f32_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_const
   }
   if (warp == 8 && lane == 0) { tma_prefetch_desc(&tm_v); tma_prefetch_desc(&tm_w); }
   __syncthreads();
+  stream_order();
 
   if (warp == 8) {
     // ---------------------------------------------------------------- TMA producer
@@ -311,6 +312,7 @@ tile_dot_mma_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_const
   }
   if (warp == 8 && lane == 0) { tma_prefetch_desc(&tm_v); tma_prefetch_desc(&tm_w); }
   __syncthreads();
+  stream_order();
 
   if (warp == 8) {
     // ---------------------------------------------------------------- TMA producer
@@ -503,6 +505,7 @@ tile_dot_mma_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_const
 template <typename OutT>
 __global__ void tile_sum_finalize_kernel(const float* __restrict__ sum, int n_tiles_n, OutT* __restrict__ out,
                                          int rows, int cols, float scale, int accumulate) {
+  stream_order();
   const long long n = static_cast<long long>(rows) * cols;
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n;
        i += static_cast<long long>(gridDim.x) * blockDim.x) {
@@ -531,7 +534,7 @@ static int launch_tile_dot_f32(const void* V, int v_samples, const void* W, int 
   if (ctas > p.stages) ctas = p.stages;
   p.stages_per_cta = (p.stages + ctas - 1) / ctas;
   ctas = (p.stages + p.stages_per_cta - 1) / p.stages_per_cta;
-  tile_dot_f32_kernel<VR><<<static_cast<int>(ctas), 288, Cfg::kSmemBytes, st>>>(tv, tw, p);
+  GB_CUDA_OK(launch_next(tile_dot_f32_kernel<VR>, dim3(static_cast<int>(ctas)), dim3(288), Cfg::kSmemBytes, st, tv, tw, p));
   count_launch();
   return post_launch("tile_dot_f32_kernel");
 }
@@ -559,7 +562,7 @@ static int launch_tile_dot_mma_t(const void* V, int v_samples, const void* W, in
   if (ctas > p.stages) ctas = p.stages;
   p.stages_per_cta = (p.stages + ctas - 1) / ctas;
   ctas = (p.stages + p.stages_per_cta - 1) / p.stages_per_cta;
-  tile_dot_mma_kernel<NVT, MT><<<static_cast<int>(ctas), 288, Cfg::kSmemBytes, st>>>(tv, tw, p);
+  GB_CUDA_OK(launch_next(tile_dot_mma_kernel<NVT, MT>, dim3(static_cast<int>(ctas)), dim3(288), Cfg::kSmemBytes, st, tv, tw, p));
   count_launch();
   return post_launch("tile_dot_mma_kernel");
 }
@@ -603,9 +606,9 @@ int launch_tile_sum_finalize(const float* sum, int n_tiles_n, void* out, int out
   long long blocks = (n + 255) / 256;
   if (blocks > ds->sm_count * 8) blocks = ds->sm_count * 8;
   if (out_is_f32)
-    tile_sum_finalize_kernel<float><<<static_cast<int>(blocks), 256, 0, st>>>(sum, n_tiles_n, static_cast<float*>(out), rows, cols, scale, accumulate);
+    GB_CUDA_OK(launch_next(tile_sum_finalize_kernel<float>, dim3(static_cast<int>(blocks)), dim3(256), 0, st, sum, n_tiles_n, static_cast<float*>(out), rows, cols, scale, accumulate));
   else
-    tile_sum_finalize_kernel<__nv_bfloat16><<<static_cast<int>(blocks), 256, 0, st>>>(sum, n_tiles_n, static_cast<__nv_bfloat16*>(out), rows, cols, scale, accumulate);
+    GB_CUDA_OK(launch_next(tile_sum_finalize_kernel<__nv_bfloat16>, dim3(static_cast<int>(blocks)), dim3(256), 0, st, sum, n_tiles_n, static_cast<__nv_bfloat16*>(out), rows, cols, scale, accumulate));
   count_launch();
   return post_launch("tile_sum_finalize_kernel");
 }

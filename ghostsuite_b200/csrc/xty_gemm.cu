@@ -142,9 +142,6 @@ xty_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant_
     *abort_flag = 0;
     fence_barrier_init();
   }
-  if (p.zero != nullptr)
-    for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < p.zero_n; i += gridDim.x * blockDim.x)
-      p.zero[i] = 0.f;
   if (warp == 5) {
     tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
@@ -157,6 +154,10 @@ xty_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant_
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  stream_order();
+  if (p.zero != nullptr)
+    for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < p.zero_n; i += gridDim.x * blockDim.x)
+      p.zero[i] = 0.f;
 
   auto decode = [&](long long u, int& tile, int& sample, int& kb0, int& kb1) {
     if (p.sample_major) {
@@ -396,6 +397,7 @@ xty_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant_
 template <typename OutT>
 __global__ void xty_finalize_kernel(const float* __restrict__ ws, long long ld_ws, OutT* __restrict__ out,
                                     int rows, int cols, float scale, int accumulate) {
+  stream_order();
   const long long n = static_cast<long long>(rows) * cols;
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n;
        i += static_cast<long long>(gridDim.x) * blockDim.x) {
@@ -423,7 +425,7 @@ static int launch_xty_t(const CUtensorMap& tx, const CUtensorMap& ty, const CUte
                                     XtyCfg<PARTS>::kSmemBytes));
     attr_set[ds->device] = true;
   }
-  xty_gemm_kernel<kColsum, PARTS><<<grid, kColsum ? 320 : 192, XtyCfg<PARTS>::kSmemBytes, st>>>(tx, ty, tout, p);
+  GB_CUDA_OK(launch_next(xty_gemm_kernel<kColsum, PARTS>, dim3(grid), dim3(kColsum ? 320 : 192), XtyCfg<PARTS>::kSmemBytes, st, tx, ty, tout, p));
   count_launch();
   return post_launch("xty_gemm_kernel");
 }
@@ -461,9 +463,9 @@ int finalize_xty(const float* ws, long long ld_ws, void* out, int out_is_f32, in
   const long long n = static_cast<long long>(rows) * cols;
   const int grid = static_cast<int>(n / 256 + 1 < 148 * 8 ? n / 256 + 1 : 148 * 8);
   if (out_is_f32)
-    xty_finalize_kernel<float><<<grid, 256, 0, st>>>(ws, ld_ws, static_cast<float*>(out), rows, cols, scale, accumulate);
+    GB_CUDA_OK(launch_next(xty_finalize_kernel<float>, dim3(grid), dim3(256), 0, st, ws, ld_ws, static_cast<float*>(out), rows, cols, scale, accumulate));
   else
-    xty_finalize_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(ws, ld_ws, static_cast<__nv_bfloat16*>(out), rows, cols, scale, accumulate);
+    GB_CUDA_OK(launch_next(xty_finalize_kernel<__nv_bfloat16>, dim3(grid), dim3(256), 0, st, ws, ld_ws, static_cast<__nv_bfloat16*>(out), rows, cols, scale, accumulate));
   count_launch();
   return post_launch("xty_finalize_kernel");
 }

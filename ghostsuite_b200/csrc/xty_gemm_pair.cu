@@ -162,9 +162,6 @@ xty_gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
     *abort_flag = 0;
     fence_barrier_init();
   }
-  if (p.zero != nullptr)
-    for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < p.zero_n; i += gridDim.x * blockDim.x)
-      p.zero[i] = 0.f;
   if (warp == 5) {
     tmem_alloc_pair(tmem_slot, 512);
     tmem_relinquish_pair();
@@ -179,6 +176,10 @@ xty_gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
   cluster_sync_all();          // both CTAs' barriers are initialised before anyone signals them
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  stream_order();
+  if (p.zero != nullptr)
+    for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < p.zero_n; i += gridDim.x * blockDim.x)
+      p.zero[i] = 0.f;
 
   if (warp == 4) {
     // ------------------------------------------------------------------ TMA producer (both CTAs)
@@ -460,7 +461,7 @@ static int launch_pair(const XtyOperands& o, long long samples, long long rows, 
   const long long units = static_cast<long long>(p.m_tiles) * p.n_tiles * p.samples;
   long long pairs = ds->sm_count / 2;
   if (pairs > units) pairs = units;
-  xty_gemm_pair_kernel<PARTS><<<static_cast<int>(2 * pairs), p.cs_of ? 320 : 192, Cfg::kSmemBytes, st>>>(tx, ty, tout ? *tout : tx, p);
+  GB_CUDA_OK(launch_next(xty_gemm_pair_kernel<PARTS>, dim3(static_cast<int>(2 * pairs)), dim3(p.cs_of ? 320 : 192), Cfg::kSmemBytes, st, tx, ty, tout ? *tout : tx, p));
   count_launch();
   return post_launch("xty_gemm_pair_kernel");
 }
