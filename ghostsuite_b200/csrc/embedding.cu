@@ -223,7 +223,7 @@ struct EmbBuckets {
   int *rank;                            // [n_tok] position inside the bucket, -1 for an id outside the table
   int *perm_b, *perm_v;
   int *totals;                          // [0] train tokens placed, [1] validation, [2] big rows, [3] items, [4] hot ids, [5] small rows,
-                                        // [6, 7] 64-bit count of gradient items handed out, [8] CTAs done with the join
+                                        // [6, 7] 64-bit count of gradient items handed out, [8] CTAs done with the join, [9] table rows looked over
   int4 *small;                          // (id, offset, tokens) of the rows with 1 to kEmbSmallBucket train tokens
   int *big;                             // ids with more than kEmbSmallBucket train tokens
   int4 *items;                          // join items: (first train position, train rows, first validation position
@@ -241,10 +241,10 @@ constexpr int kEmbChunk = 8;             // train rows of a join item
 constexpr int kEmbValChunk = 32;         // validation rows of a join item
 
 // Counting hands every token its place in the bucket, so filling needs no second round of atomics.
-// It also clears the sums that the join adds to two launches later, and zero-fills the gradient, most of
-// whose rows stay empty: the stores go out under the latency of the atomics.
+// It also clears the sums that the join adds to two launches later, and zero-fills a gradient of odd width.
 __global__ void __launch_bounds__(256) emb_count_kernel(const EmbBuckets q, double* __restrict__ M64, long long m_size,
                                                         uint4* __restrict__ zero, long long zero_size) {
+  stream_order();
   if (M64 != nullptr)
     for (long long i = blockIdx.x * 256ll + threadIdx.x; i < m_size; i += gridDim.x * 256ll) M64[i] = 0.;
   for (long long j = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; j < q.n_tok;
@@ -265,6 +265,7 @@ __global__ void __launch_bounds__(256) emb_count_kernel(const EmbBuckets q, doub
 // a scan over the whole table (22 us in one block for 50 k ids, 4.6 us now).  Also listed here: the
 // gradient's rows by size, join items, and ids that many validation tokens share (padding, separators).
 __global__ void __launch_bounds__(256) emb_alloc_kernel(const EmbBuckets q) {
+  stream_order();
   __shared__ int s_warp[3][8], s_base[3];
   const int id = blockIdx.x * 256 + threadIdx.x;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -337,6 +338,7 @@ __global__ void __launch_bounds__(256) emb_alloc_kernel(const EmbBuckets q) {
 }
 
 __global__ void __launch_bounds__(256) emb_fill_kernel(const EmbBuckets q) {
+  stream_order();
   for (long long j = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; j < q.n_tok;
        j += static_cast<long long>(gridDim.x) * blockDim.x) {
     const int r = q.rank[j];
@@ -353,6 +355,7 @@ __global__ void __launch_bounds__(256) emb_fill_kernel(const EmbBuckets q) {
 template <typename T>
 __global__ void __launch_bounds__(256)
 emb_hot_reduce_kernel(const EmbBuckets q, const T* __restrict__ Gv, long long Tn, int d, int n_val, float* __restrict__ R) {
+  stream_order();
   __shared__ int s_tok[1024];
   __shared__ __align__(16) float s_sum[256 * 8];
   __shared__ int s_n;
@@ -861,13 +864,35 @@ __device__ __forceinline__ void emb_big_rows(const EmbBuckets& q, const T* __res
 // What bounds it is issue slots and latency, not bandwidth, and the same holds for the join: launched beside
 // this grid's tail (a programmatic launch: it reads nothing written here), both together take 66 us
 // instead of 78.
+// Zeroes the gradient's rows without tokens, 32 ids a warp drawn from a counter.  It runs behind the sums, on the warps that
+// find no more of them: the longest row's sum leaves HBM idle for 30 us, and the counting kernel, which zeroed all
+// rows ahead of everything else, took 13 us for it on a table of 50304 x 768 bf16.
+template <typename T>
+__device__ void emb_zero_rows(const EmbBuckets& q, int d, T* __restrict__ out) {
+  const int lane = threadIdx.x & 31;
+  const int pieces = static_cast<int>(d * sizeof(T) / 16);
+  const uint4 z = make_uint4(0u, 0u, 0u, 0u);
+  while (true) {
+    int first = 0;
+    if (lane == 0) first = atomicAdd(q.totals + 9, 32);
+    first = __shfl_sync(0xffffffffu, first, 0);
+    if (first >= q.vocab) break;
+    const bool empty = first + lane < q.vocab && q.cnt_b[first + lane] == 0;
+    for (unsigned todo = __ballot_sync(0xffffffffu, empty); todo != 0; todo &= todo - 1) {
+      uint4* row = reinterpret_cast<uint4*>(out + static_cast<long long>(first + __ffs(todo) - 1) * d);
+      for (int i = lane; i < pieces; i += 32) row[i] = z;
+    }
+  }
+}
+
 template <typename T>
 __global__ void __launch_bounds__(kEmbGradThreads, 6)
 emb_grad_kernel(const EmbBuckets q, const T* __restrict__ G, int d, int slices, float pre_scale, float divisor,
-                int accumulate, T* __restrict__ out) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");      // the join may start beside this grid's tail
+                int accumulate, int zero_rows, T* __restrict__ out) {
+  stream_order();                        // from here on the join may start beside this grid's tail
   emb_big_rows<T>(q, G, d, slices, pre_scale, divisor, accumulate, out);
   emb_small_rows<T>(q, G, d, pre_scale, divisor, accumulate, out);
+  if (zero_rows) emb_zero_rows<T>(q, d, out);
 }
 
 static inline long long up256(long long x) { return (x + 255) / 256 * 256; }
@@ -906,22 +931,26 @@ static int emb_pass(const EmbBuckets& q, const T* Gb, const T* Gv, int n_train, 
                     float* M, long long pitch, double* M64, float* R, float pre_scale, float divisor, int accumulate, T* out, const DeviceState* ds, cudaStream_t st) {
   int blocks = static_cast<int>((q.n_tok + 255) / 256);
   if (blocks > ds->sm_count * 8) blocks = ds->sm_count * 8;
-  // the gradient is zero-filled by the counting kernel where 16-byte stores can (torch buffers always)
+  // Rows without tokens are zeroed behind the sums where 16-byte stores can, by the counting kernel where the table as a
+  // whole takes them (rows of odd widths), or by a memset.
   const long long out_bytes = static_cast<long long>(q.vocab) * d * static_cast<long long>(sizeof(T));
-  const bool fill = out != nullptr && !accumulate, quick = fill && out_bytes % 16 == 0 && (reinterpret_cast<uintptr_t>(out) & 15u) == 0;
-  if (fill && !quick) GB_CUDA_OK(cudaMemsetAsync(out, 0, out_bytes, st));
+  const bool fill = out != nullptr && !accumulate, aligned = (reinterpret_cast<uintptr_t>(out) & 15u) == 0;
+  const bool by_rows = fill && aligned && d * sizeof(T) % 16 == 0 && q.vocab < INT_MAX - (1 << 24);
+  const bool quick = fill && !by_rows && aligned && out_bytes % 16 == 0;
+  if (fill && !by_rows && !quick) GB_CUDA_OK(cudaMemsetAsync(out, 0, out_bytes, st));
+  const int tokens = blocks;
   if (quick) blocks = ds->sm_count * 8;
-  emb_count_kernel<<<blocks, 256, 0, st>>>(q, M64, static_cast<long long>(n_val) * n_train, reinterpret_cast<uint4*>(out),
-                                           quick ? out_bytes / 16 : 0);
-  emb_alloc_kernel<<<ceil_div(q.vocab, 256), 256, 0, st>>>(q);
-  emb_fill_kernel<<<blocks, 256, 0, st>>>(q);
+  GB_CUDA_OK(launch_next(emb_count_kernel, dim3(blocks), dim3(256), 0, st, q, M64, static_cast<long long>(n_val) * n_train,
+                         reinterpret_cast<uint4*>(out), quick ? out_bytes / 16 : 0ll));
+  GB_CUDA_OK(launch_next(emb_alloc_kernel, dim3(ceil_div(q.vocab, 256)), dim3(256), 0, st, q));
+  GB_CUDA_OK(launch_next(emb_fill_kernel, dim3(tokens), dim3(256), 0, st, q));
   count_launch(3);
   const bool vec = d % 8 == 0 && ((reinterpret_cast<uintptr_t>(Gb) | reinterpret_cast<uintptr_t>(Gv)) & 15u) == 0;
   if (M != nullptr) {
     if (static_cast<long long>(n_val) * Tn > q.hot_threshold) {
       int hb = kEmbHotCap * n_val;
       if (hb > ds->sm_count * 8) hb = ds->sm_count * 8;
-      emb_hot_reduce_kernel<T><<<hb, 256, 0, st>>>(q, Gv, Tn, d, n_val, R);
+      GB_CUDA_OK(launch_next(emb_hot_reduce_kernel<T>, dim3(hb), dim3(256), 0, st, q, Gv, Tn, d, n_val, R));
       count_launch();
     }
   }
@@ -930,9 +959,14 @@ static int emb_pass(const EmbBuckets& q, const T* Gb, const T* Gv, int n_train, 
     const long long rows = q.vocab < q.first_val ? q.vocab : q.first_val;      // at most one row per token
     const int slices = ceil_div(d, 256 / static_cast<int>(sizeof(T)));
     const long long most = rows * slices;
-    const int gb = static_cast<int>(most < ds->sm_count * 6 ? most : ds->sm_count * 6);
+    int gb = static_cast<int>(most < ds->sm_count * 6 ? most : ds->sm_count * 6);
+    if (by_rows) {                       // warps enough for the empty rows too
+      const int zb = ceil_div(q.vocab, kEmbGradThreads), all = ds->sm_count * 6;
+      if (gb < zb) gb = zb < all ? zb : all;
+    }
     constexpr int kBigRing = kBigSlots * kBigStage * 256;
-    emb_grad_kernel<T><<<gb, kEmbGradThreads, kBigRing, st>>>(q, Gb, d, slices, pre_scale, divisor, accumulate, out);
+    GB_CUDA_OK(launch_next(emb_grad_kernel<T>, dim3(gb), dim3(kEmbGradThreads), kBigRing, st, q, Gb, d, slices, pre_scale, divisor,
+                           accumulate, by_rows ? 1 : 0, out));
     count_launch();
   }
   if (M != nullptr) {
