@@ -27,7 +27,8 @@ static constexpr int kPassThreads = 256;
 // rows 10.8 us, 9.5 now; of 768: 6.7 and 5.0); no more than the list's longest vector needs, which leaves room for the CTAs of other kernels.
 static constexpr int kPassMost = 512;
 __host__ __device__ constexpr int pass_pitch(int sub) { return sub + 4; }      // rows 16 bytes apart modulo 128: no bank conflicts
-__host__ __device__ constexpr int pass_smem(int sub) { return 40 * pass_pitch(sub) * 4; }      // 32 train rows, then eight validation rows
+// 32 train rows, then nv validation rows; behind them the warps' partial sums
+__host__ __device__ constexpr int pass_smem(int sub, int nv) { return (32 + nv) * pass_pitch(sub) * 4 + 8 * nv * 32 * 4; }
 __host__ __device__ constexpr int pass_chunk(int F) { return ((F + kPassCluster - 1) / kPassCluster + 7) / 8 * 8; }
 
 static constexpr double kPassOneMatrix = 1 << 21;     // products of a single matrix that the clusters take
@@ -40,12 +41,14 @@ __device__ __forceinline__ const float* pass_val_row(const ghost_pass_job& j, in
                                static_cast<long long>(v % j.v_per_rank) * j.F;
 }
 
-// Columns [f, f + width) of the block's rows into shared memory, zero up to the next multiple of four
+// Columns [f, f + width) of the block's rows from row `first` on (0: train rows, 32: validation rows) into shared memory,
+// zero up to the next multiple of four
+template <int NV>
 __device__ __forceinline__ void pass_stage(const ghost_pass_job& j, bool vec, int b0, int v0, int f, int width, float* st,
-                                           int pitch) {
+                                           int pitch, int first) {
   const int quads = (width + 3) / 4;
-  for (int i = threadIdx.x; i < 40 * quads; i += kPassThreads) {
-    const int r = i / quads, q = (i - r * quads) * 4;
+  for (int i = threadIdx.x; i < (32 + NV - first) * quads; i += kPassThreads) {
+    const int row = i / quads, r = row + first, q = (i - row * quads) * 4;
     const float* src;
     if (r < 32) src = b0 + r < j.n_train ? j.X + static_cast<long long>(b0 + r) * j.F : nullptr;
     else src = v0 + r - 32 < j.n_val ? pass_val_row(j, v0 + r - 32) : nullptr;
@@ -131,13 +134,15 @@ template <typename F> __device__ __forceinline__ float pass_sum8(F&& v) {
   return ((v(0) + v(1)) + (v(2) + v(3))) + ((v(4) + v(5)) + (v(6) + v(7)));
 }
 
-template <int CAP>
+// NV: validation rows that go through a block together, 16 where a job has more than eight.  256 + 32 vectors of 1024 took
+// 21 us in four rounds that each brought the train rows again, 16 in two; with eight or fewer, 16 would stage rows of zeros.
+template <int CAP, int NV>
 __global__ void __cluster_dims__(kPassCluster, 1, 1) __launch_bounds__(kPassThreads)
 pass_reduce_kernel(const __grid_constant__ PassJobs<CAP> jobs) {
-  extern __shared__ __align__(16) float stage[];       // pass_smem(sub) bytes
+  extern __shared__ __align__(16) float stage[];       // pass_smem(sub, NV) bytes
   const int pitch = pass_pitch(jobs.sub);
   stream_order();
-  __shared__ float part[2][8][32];       // this CTA's share of F, read by rank 0 of the cluster
+  __shared__ float part[2][NV][32];      // this CTA's share of F, read by rank 0 of the cluster
   __shared__ float cols[8][32];
   const ghost_pass_job& j = jobs.job[blockIdx.z];
   const int n_blk = (j.n_train + 31) / 32, step = gridDim.y;       // one block each, unless a job has more than a grid
@@ -180,41 +185,46 @@ pass_reduce_kernel(const __grid_constant__ PassJobs<CAP> jobs) {
       const int b = blk * 32 + lane;
       const bool live = b < j.n_train;
       float col = 0.f;                     // rank 0: this thread's share of vec
-      for (int v0 = 0; v0 < j.n_val; v0 += 8, buf ^= 1) {
-        float4 acc[8];                     // a sum per quarter of the columns: short chains, as one warp per pair had
+      for (int v0 = 0; v0 < j.n_val; v0 += NV, buf ^= 1) {
+        float4 acc[NV];                    // a sum per quarter of the columns: short chains, as one warp per pair had
 #pragma unroll
-        for (int i = 0; i < 8; ++i) acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int i = 0; i < NV; ++i) acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
         for (int f = f0; f < f1; f += jobs.sub) {
           const int width = f1 - f < jobs.sub ? f1 - f : jobs.sub;
           __syncthreads();
-          pass_stage(j, vec, blk * 32, v0, f, width, stage, pitch);
+          // one round holds all columns: the train rows are there already
+          pass_stage<NV>(j, vec, blk * 32, v0, f, width, stage, pitch, v0 > 0 && chunk <= jobs.sub ? 32 : 0);
           __syncthreads();
           if (staged_sums && v0 == 0) pass_staged_sums(j, f, width, stage, pitch);
           for (int q = warp * 4; q < width; q += 32) {
             const float4 x = *reinterpret_cast<const float4*>(stage + lane * pitch + q);
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
+            for (int i = 0; i < NV; ++i) {
               const float4 y = *reinterpret_cast<const float4*>(stage + (32 + i) * pitch + q);
               acc[i].x = fmaf(x.x, y.x, acc[i].x); acc[i].y = fmaf(x.y, y.y, acc[i].y);
               acc[i].z = fmaf(x.z, y.z, acc[i].z); acc[i].w = fmaf(x.w, y.w, acc[i].w);
             }
           }
         }
-        __syncthreads();
-        float* red = stage;                // [warp][validation row][train lane]
+        float* red = stage + (32 + NV) * pitch;        // [warp][validation row][train lane]
 #pragma unroll
-        for (int i = 0; i < 8; ++i) red[(warp * 8 + i) * 32 + lane] = (acc[i].x + acc[i].y) + (acc[i].z + acc[i].w);
+        for (int i = 0; i < NV; ++i) red[(warp * NV + i) * 32 + lane] = (acc[i].x + acc[i].y) + (acc[i].z + acc[i].w);
         __syncthreads();
-        // thread (warp, lane) now owns pair (v0 + warp, b)
-        part[buf][warp][lane] = pass_sum8([&](int w) { return red[(w * 8 + warp) * 32 + lane]; });
+        // thread (warp, lane) now owns pairs (v0 + warp, b), (v0 + 8 + warp, b)
+#pragma unroll
+        for (int h = 0; h < NV; h += 8)
+          part[buf][h + warp][lane] = pass_sum8([&](int w) { return red[(w * NV + h + warp) * 32 + lane]; });
         // one cluster barrier per block: `part` alternates, and rank 0 reads block k's before it
         // arrives at block k + 1's barrier, which every CTA passes before writing that buffer again
         cluster.sync();
         if (rank == 0) {
-          const float m = j.dot_scale * pass_sum8([&](int r) { return *cluster.map_shared_rank(&part[buf][warp][lane], r); });
-          if (v0 + warp < j.n_val && live) {
-            j.M[static_cast<long long>(v0 + warp) * j.n_train + b] = m;
-            col += m;
+#pragma unroll
+          for (int h = 0; h < NV; h += 8) {
+            const float m = j.dot_scale * pass_sum8([&](int r) { return *cluster.map_shared_rank(&part[buf][h + warp][lane], r); });
+            if (v0 + h + warp < j.n_val && live) {
+              j.M[static_cast<long long>(v0 + h + warp) * j.n_train + b] = m;
+              col += m;
+            }
           }
         }
       }
@@ -322,11 +332,11 @@ __global__ void __launch_bounds__(256) rows_sum_kernel(const float* __restrict__
   }
 }
 
-template <int CAP>
+template <int CAP, int NV>
 static int launch_pass(const ghost_pass_job* jobs, int n, int blocks, const DeviceState* ds, cudaStream_t st) {
   static bool attr_set[64] = {};
   if (!attr_set[ds->device]) {
-    GB_CUDA_OK(cudaFuncSetAttribute(pass_reduce_kernel<CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, pass_smem(kPassMost)));
+    GB_CUDA_OK(cudaFuncSetAttribute(pass_reduce_kernel<CAP, NV>, cudaFuncAttributeMaxDynamicSharedMemorySize, pass_smem(kPassMost, NV)));
     attr_set[ds->device] = true;
   }
   PassJobs<CAP> batch;
@@ -337,7 +347,7 @@ static int launch_pass(const ghost_pass_job* jobs, int n, int blocks, const Devi
   const int sub = (pass_chunk(longest) + 31) / 32 * 32;
   // the row sums of longer lists reduce 8 x 4 x 128 partial sums in the same memory
   batch.sub = sub < 128 ? 128 : sub > kPassMost ? kPassMost : sub;
-  GB_CUDA_OK(launch_next(pass_reduce_kernel<CAP>, dim3(dim3(kPassCluster, blocks, n)), dim3(kPassThreads), pass_smem(batch.sub), st, batch));
+  GB_CUDA_OK(launch_next(pass_reduce_kernel<CAP, NV>, dim3(dim3(kPassCluster, blocks, n)), dim3(kPassThreads), pass_smem(batch.sub, NV), st, batch));
   count_launch();
   return post_launch("pass_reduce_kernel");
 }
@@ -418,9 +428,13 @@ extern "C" int ghost_pass_reduce(const ghost_pass_job* jobs, int n_jobs, void* s
     int most = 1;
     for (int i = 0; i < n; ++i) most = jobs[first + i].n_train > most ? jobs[first + i].n_train : most;
     const int blocks = ceil_div(most, 32) < 65535 ? ceil_div(most, 32) : 65535;
-    const int rc = n <= 4 ? launch_pass<4>(jobs + first, n, blocks, ds, st)
-                 : n <= 40 ? launch_pass<40>(jobs + first, n, blocks, ds, st)
-                           : launch_pass<kLarge>(jobs + first, n, blocks, ds, st);
+    bool many = false;
+    for (int i = 0; i < n; ++i) many |= jobs[first + i].M != nullptr && jobs[first + i].X != nullptr && jobs[first + i].n_val > 8;
+    const ghost_pass_job* list = jobs + first;
+    const int rc = n <= 4    ? many ? launch_pass<4, 16>(list, n, blocks, ds, st) : launch_pass<4, 8>(list, n, blocks, ds, st)
+                   : n <= 40 ? many ? launch_pass<40, 16>(list, n, blocks, ds, st) : launch_pass<40, 8>(list, n, blocks, ds, st)
+                   : many    ? launch_pass<kLarge, 16>(list, n, blocks, ds, st)
+                             : launch_pass<kLarge, 8>(list, n, blocks, ds, st);
     if (rc != GHOST_OK) return rc;
   }
   return GHOST_OK;

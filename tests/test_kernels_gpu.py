@@ -856,6 +856,26 @@ def test_small_reduce_batch_matches_single_launches():
             assert torch.equal(job["sum_out"], rec["sum"])
 
 
+# validation rows on both sides of a block's 8 and 16, train rows of one block and of two, vectors staged in one round and in more
+@pytest.mark.parametrize("n_t,n_v", [(32, 9), (5, 16), (40, 17), (33, 35)])
+@pytest.mark.parametrize("F", [37, 1024, 4100])
+def test_pass_reduce_of_many_validation_rows(n_t, n_v, F):
+    o = ops()
+    X = torch.randn(n_t + n_v, F, generator=torch.Generator().manual_seed(5)).cuda()
+    M, S = torch.full((n_v, n_t), 7.0, device="cuda"), torch.full((F,), 7.0, device="cuda")
+    few = torch.full((3, n_t), 7.0, device="cuda")
+    vec, = o.pass_reduce([{"X": X, "n_train": n_t, "n_val": n_v, "M": M, "sum_out": S, "dot_scale": 0.5},
+                          {"X": X, "n_train": n_t, "n_val": 3, "M": few, "dot_scale": 0.5}], [M])
+    after()
+    T, V = X[:n_t].double(), X[n_t:].double()
+    # chains of F / 256 products in each of 256 accumulators, then pairs: a rounding of 2^-24 per level
+    bound = (F / 256 + 10) * 2.0 ** -24 * 0.5 * (V.abs() @ T.abs().t())
+    assert ((M.double() - 0.5 * V @ T.t()).abs() <= bound).all()
+    assert torch.equal(few, M[:3])
+    assert ((vec.double() - M.double().sum(0)).abs() <= (n_v / 8 + 3) * 2.0 ** -24 * M.double().abs().sum(0)).all()
+    assert ((S.double() - T.sum(0)).abs() <= n_t * 2.0 ** -24 * T.abs().sum(0)).all()
+
+
 # one matrix on its own, beyond what the batched launch's blocks take: vector and scalar loads, remainders
 @pytest.mark.parametrize("n_t,n_v,F", [(300, 30, 772), (2000, 3, 1001), (70, 40, 4100), (5, 3, 150001), (600, 8, 512)])
 def test_small_gram_of_large_vectors(n_t, n_v, F):
