@@ -50,6 +50,7 @@ PROTOTYPES = {
     "ghost_cast_split_bf16": (_i, [_vp, _i, _ll, _ll, _i, _ll, _vp, _ll, _i, _i, _i, _i, _i, _i, _vp]),
     "ghost_split_operands": (_i, [_vp, _i, _i, _vp, _i, _i, _i, _ll, _ll, _i, _vp, _vp, _vp, _vp, _vp]),
     "ghost_conv_tokens_bf16": (_i, [_vp, _i, _ll] + [_i] * 11 + [_vp, _ll] + [_i] * 6 + [_vp]),
+    "ghost_conv_operands": (_i, [_vp, _i, _vp, _i, _ll] + [_i] * 16 + [_vp, _vp, _vp, _vp]),
     "ghost_row_sums": (_i, [_vp, _i, _ll, _ll, _vp, _vp]),
     "ghost_gram_dot_bf16": (_i, [_vp, _vp, _vp, _vp, _i, _i, _ll, _i, _i, _ll, _ll, _ll, _ll, _i, _f, _vp, _vp]),
     "ghost_gram_dot_parts": (_i, [_vp, _vp, _i, _i, _i, _ll, _i, _i, _ll, _ll, _i, _f, _vp, _vp]),

@@ -176,7 +176,7 @@ PyObject* py_arena_clear(PyObject*, PyObject* const*, Py_ssize_t) {
 // hi/lo layouts of an fp32 operand pair so that sum_k L[k] R[k] = hi*hi + lo*hi + hi*lo
 constexpr int kSplitLeft[3] = {0, 1, 0};
 constexpr int kPlain[3] = {0, 0, 0};
-enum { kSideBySide = 0, kStackRows = 1, kStackBatch = 2 };     // where the parts of a copy lie (kStackBatch: convolutions)
+enum { kSideBySide = 0 };      // where the parts of a copy lie
 
 // An operand [N, T, cols] of the layer math: a tensor with exactly these dimensions, or a convolution
 // operand [N, C, H, W] whose tokens are the output positions.
@@ -191,19 +191,12 @@ struct Operand {
   int f32() const { return is_f32(t); }
   // readable as it is by the tensor-core entry points
   bool ready() const { return conv == nullptr && tma_ready(t); }
-  // bf16 copy of samples [first, first + samples)
+  // bf16 copy of samples [first, first + samples) of a tensor
   void cast(long long first, long long samples, void* dst, long long ld_dst, long long cpad, int parts, const int (&kinds)[3],
             int stack, void* st) const {
-    const long long per = conv ? static_cast<long long>(conv->C) * conv->H * conv->W : T * cols;
-    const char* p = static_cast<const char*>(t.data_ptr()) + first * per * t.element_size();
-    const int cp = static_cast<int>(cpad);
-    if (conv)
-      check(ghost_conv_tokens_bf16(p, f32(), samples, conv->C, conv->H, conv->W, conv->kh, conv->kw, conv->sy, conv->sx,
-                                   conv->py, conv->px, conv->dy, conv->dx, dst, ld_dst, cp, parts, kinds[0], kinds[1],
-                                   kinds[2], stack, st));
-    else
-      check(ghost_cast_split_bf16(p, f32(), samples, T, static_cast<int>(cols), cols, dst, ld_dst, cp, parts, kinds[0],
-                                  kinds[1], kinds[2], stack, st));
+    const char* p = static_cast<const char*>(t.data_ptr()) + first * T * cols * t.element_size();
+    check(ghost_cast_split_bf16(p, f32(), samples, T, static_cast<int>(cols), cols, dst, ld_dst, static_cast<int>(cpad), parts, kinds[0],
+                                kinds[1], kinds[2], stack, st));
   }
 };
 
@@ -234,10 +227,11 @@ struct XtyOperands {
   const void* where(int i, char* base) const { return copy[i] ? static_cast<const void*>(base + off[i]) : x[i]->t.data_ptr(); }
   // Lays out what has to be copied, with the column sums of operand sums_of (1 or 2, both operands copied) on the way
   void prepare(char* base, void* st, int sums_of = 0, float* sums = nullptr) const {
-    if (x[0]->conv || x[1]->conv) {
-      const int kinds[3] = {0, 1, 0};
-      for (int i = 0; i < 2; ++i)
-        if (copy[i]) x[i]->cast(0, count, base + off[i], ld[i], ld[i], parts(), kinds, merged ? kStackBatch : kStackRows, st);
+    if (x[0]->conv) {                    // the out-grad, then the input under its window
+      const Conv &b = *x[0]->conv, &a = *x[1]->conv;
+      check(ghost_conv_operands(x[1]->t.data_ptr(), x[1]->f32(), x[0]->t.data_ptr(), x[0]->f32(), count, a.C, a.H, a.W, a.kh, a.kw,
+                                a.sy, a.sx, a.py, a.px, a.dy, a.dx, b.C, b.H, b.W, parts(), merged ? 1 : 0, base + off[1],
+                                base + off[0], sums_of == 1 ? sums : nullptr, st));
     } else if (copy[0] || copy[1]) {
       auto src = [&](int i) { return copy[i] ? x[i]->t.data_ptr() : nullptr; };
       auto dst = [&](int i) { return copy[i] ? base + off[i] : nullptr; };
@@ -327,16 +321,16 @@ PerSample persample_dot(const Launch& L, const Operand& X, const Operand& Y, lon
   const long long off_ws = ws.plan(ws_bytes);
   char* base = ws.commit(L, X.t);
   // Column sums: of bf16 operands the GEMM pass takes them along (colsum_of), of float32 ones their conversion does
-  // (split_sums_of) unless a sample has too few rows for a block of it.
-  const int sums_of = !ops.split ? colsum_of : T >= 16 && !X.conv ? split_sums_of : 0;
+  // (split_sums_of) unless a sample has too few rows for a block of it; of a convolution's, the copy does.
+  const int sums_of = X.conv ? split_sums_of : !ops.split ? colsum_of : T >= 16 ? split_sums_of : 0;
   if (sums_of) r.colsums = empty({N, ops.x[sums_of - 1]->cols}, X.t, at::kFloat);
   float* sums = sums_of ? r.colsums.data_ptr<float>() : nullptr;
-  if (ops.split) ops.prepare(base, L.st(), sums_of, sums);
+  if (ops.split || X.conv) ops.prepare(base, L.st(), sums_of, sums);
   else ops.prepare(base, L.st());
   check(ghost_persample_dot_parts(ops.where(0, base), ops.where(1, base), ops.parts(), static_cast<int>(n_train),
                                   static_cast<int>(n_val), T, m, n, ops.ld[0], ops.ld[1], dot_scale, r.M.data_ptr<float>(),
                                   want_grad ? r.grad.data_ptr() : nullptr, want_grad ? is_f32(r.grad) : 0, grad_scale, 0,
-                                  ops.split ? 0 : sums_of, ops.split ? nullptr : sums, base + off_ws, ws_bytes, L.st()));
+                                  ops.split || X.conv ? 0 : sums_of, ops.split || X.conv ? nullptr : sums, base + off_ws, ws_bytes, L.st()));
   return r;
 }
 
@@ -427,7 +421,7 @@ void dense_paths(const Launch& L, const Operand& A, const Operand& B, long long 
     const long long ws_bytes = grad.defined() ? ghost_wgrad_workspace_bytes(m, n) : 0, off_ws = ws.plan(ws_bytes);
     XtyOperands ops(ws, X, Y, N, true);
     char* base = ws.commit(L, A.t);
-    const bool take = bias && ops.split && A.T >= 16 && !A.conv;
+    const bool take = bias && (A.conv || (ops.split && A.T >= 16));
     if (take) sums = empty({N, B.cols}, A.t, at::kFloat);
     ops.prepare(base, L.st(), take ? b + 1 : 0, take ? sums.data_ptr<float>() : nullptr);
     launch_gram(L, ops, 1 - b, base, n_val, 0, 1.f, M);
@@ -504,12 +498,8 @@ PyObject* py_conv_hook(PyObject*, PyObject* const* a, Py_ssize_t n) {
     check_split(n_train, n_val, "conv_hook");
     const bool bias = integer(a[7]) != 0;
     Tensor M, grad, sums;
-    dense_paths(L, Operand(A, ca, T), Operand(B, cb, T), n_val, false, integer(a[4]) != 0, integer(a[5]), real(a[6]), false, false, M,
+    dense_paths(L, Operand(A, ca, T), Operand(B, cb, T), n_val, false, integer(a[4]) != 0, integer(a[5]), real(a[6]), bias, false, M,
                 grad, sums);
-    if (bias) {
-      sums = empty({N, p}, A, at::kFloat);
-      check(ghost_row_sums(B.data_ptr(), is_f32(B), N * p, T, sums.data_ptr<float>(), L.st()));
-    }
     Tensor Mb = bias ? empty({n_val, n_train}, A, at::kFloat) : Tensor();
     Tensor sb = optional_empty({p}, A, bias ? integer(a[8]) : -1);
     return Py_BuildValue("(NNNNN)", wrap(M), wrap_or_none(grad), wrap_or_none(sums), wrap_or_none(Mb), wrap_or_none(sb));

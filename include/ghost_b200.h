@@ -83,6 +83,12 @@ int ghost_conv_tokens_bf16(const void* src, int src_is_f32, long long samples, i
                            int kw, int sy, int sx, int py, int px, int dy, int dx, void* dst,
                            long long ld_dst, int cpad, int parts, int kind0, int kind1, int kind2,
                            int row_stack, void* stream);
+/* Both operands of a convolution in one launch, in one or two parts with rows padded to multiples of 64 as ghost_split_operands
+ * leaves them: A [samples, C, H, W] under its window, B [samples, p, Ho, Wo]; merged: parts stacked over the batch.
+ * b_sums [samples, p], if not NULL: the sums of B over the positions (fp32), the bias terms. */
+int ghost_conv_operands(const void* A, int a_is_f32, const void* B, int b_is_f32, long long samples, int C, int H,
+                        int W, int kh, int kw, int sy, int sx, int py, int px, int dy, int dx, int p, int Ho, int Wo,
+                        int parts, int merged, void* A_out, void* B_out, float* b_sums, void* stream);
 /* out[r] = sum_i x[r, i] of a dense [rows, len] matrix (fp32 sums): bias terms of a convolution. */
 int ghost_row_sums(const void* x, int is_f32, long long rows, long long len, float* out, void* stream);
 

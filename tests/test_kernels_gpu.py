@@ -426,6 +426,37 @@ def test_conv_hook(case, use_gram, dtype):
     assert O.rel_fro(sums, Bt.sum(1)) < 1e-5
 
 
+# a window whose padding alone needs 64-bit offsets; bias sums behind one block of positions and behind many
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("use_gram", [False, True])
+@pytest.mark.parametrize("case", [(2, 1, 3, 2, 2, 5, (1, 1), (20000, 20000), (20000, 20000), (1, 1)),
+                                  (2, 1, 2, 40, 40, 130, (3, 3), (1, 1), (1, 1), (1, 1))])
+def test_conv_operands_in_one_launch(case, use_gram, dtype):
+    test_conv_hook(case, use_gram, dtype)
+
+
+def test_conv_operands_beyond_one_grid():
+    """More blocks of features than a grid has rows: an operand a launch, the bytes of the single-operand entry."""
+    from ghostsuite_b200 import _lib
+    lib = _lib.load()
+    C, p, N = 65535 * 64, 70, 2
+    A, B = torch.randn(N, C, 1, 1).cuda(), torch.randn(N, p, 1, 1).cuda()
+    st = torch.cuda.current_stream().cuda_stream
+    got = [torch.zeros(N, 2, 1, w, dtype=torch.bfloat16, device="cuda") for w in (C, 128)]
+    sums = torch.zeros(N, p, device="cuda")
+    _lib.check(lib.ghost_conv_operands(A.data_ptr(), 1, B.data_ptr(), 1, N, C, 1, 1, 1, 1, 1, 1, 0, 0, 1, 1, p, 1, 1, 2, 0,
+                                       got[0].data_ptr(), got[1].data_ptr(), sums.data_ptr(), st))
+    for x, c, out in ((A, C, got[0]), (B, p, got[1])):
+        want = torch.zeros_like(out)
+        _lib.check(lib.ghost_conv_tokens_bf16(x.data_ptr(), 1, N, c, 1, 1, 1, 1, 1, 1, 0, 0, 1, 1, want.data_ptr(), out.shape[3],
+                                              out.shape[3], 2, 0, 1, 0, 1, st))
+        after()
+        assert torch.equal(out, want)
+        # hi + lo: 2^-9 of the value is left to lo, which is rounded to 2^-9 of itself
+        assert ((out.float().sum(1)[:, 0, :c] - x[:, :, 0, 0]).abs() <= 2.0 ** -17 * x[:, :, 0, 0].abs()).all()
+    assert torch.equal(sums, B[:, :, 0, 0])
+
+
 # edges of the one-launch kernel: T on both sides of its 8 x 4 token tile and of whole-sample groups,
 # one sample, widths off and on its 64 / 128 / 1024 column units, odd widths (no 16-byte loads)
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
