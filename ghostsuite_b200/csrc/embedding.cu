@@ -521,7 +521,7 @@ __device__ __forceinline__ float emb_plain_dot(const VT* v, const BT* b, int d, 
 // to be infinite, or lies beyond the parts' range) is made again from the rows as they are.  Lane
 // (g, c) holds entries (g, 2c), (g, 2c + 1), (g + 8, 2c), (g + 8, 2c + 1); `lv` is its two validation rows.
 template <typename VT, typename BT>
-__device__ __noinline__ float4 emb_redo(const VT* V, const BT* B, int2 lv, int my_b, unsigned todo, int d, float4 sums) {
+__device__ __noinline__ float4 emb_redo(const VT* V, const BT* B, int2 lv, int my_b, unsigned todo, int d, int dk, float4 sums) {
   float acc[4] = {sums.x, sums.y, sums.z, sums.w};
   const int lane = threadIdx.x & 31;
   for (unsigned who_mask = __ballot_sync(0xffffffffu, todo != 0); who_mask != 0; who_mask &= who_mask - 1) {
@@ -532,7 +532,7 @@ __device__ __noinline__ float4 emb_redo(const VT* V, const BT* B, int2 lv, int m
     for (int e = 0; e < 4; ++e) {
       const int b = __shfl_sync(0xffffffffu, my_b, 2 * (who & 3) + (e & 1));
       if (!(what >> e & 1)) continue;
-      const float s = emb_plain_dot<VT, BT>(V + static_cast<long long>(e < 2 ? r0 : r1) * d, B + static_cast<long long>(b) * d, d, lane);
+      const float s = emb_plain_dot<VT, BT>(V + static_cast<long long>(e < 2 ? r0 : r1) * d, B + static_cast<long long>(b) * d, dk, lane);
       if (lane == who) acc[e] = s;
     }
   }
@@ -546,7 +546,13 @@ __device__ __noinline__ float4 emb_redo(const VT* V, const BT* B, int2 lv, int m
 // fall apart into many) and the next item's entry in flight.  Forms before it, for text ids (40 x 1024 tokens
 // of 768 bf16 features): a chain walk per train token, 150 us; validation rows in registers and
 // products on the CUDA cores, 80 us at eight warps per SM.
-template <typename T, bool VEC>
+// An item's rows arrive over several rounds of loads in a row, 0.7 us each, so a batch with fewer items than warps leaves the
+// kernel waiting for the longest: 16 + 4 x 512 text tokens of 2048 float32 features, 32 rounds an item, took 229 us with the
+// hook, 168 now (9 + 3 x 333 of 701 67 and 50).  There (CUT) items fall into pieces of a range of features where that shortens
+// the rounds that a warp goes through, a piece's indices and sums counted as kEmbJoinAround of them.  Batches
+// of more train tokens than four a warp have items enough (at 32 x 1024 the arithmetic alone cost 1.2 us of 99).
+constexpr int kEmbJoinAround = 2;
+template <typename T, bool VEC, bool CUT>
 __global__ void __launch_bounds__(256, 2)
 emb_join_kernel(const EmbBuckets q, const T* __restrict__ Gb, const T* __restrict__ Gv, int n_train, int n_val, int Tn, int d,
                 const float* __restrict__ R, float scale, double* __restrict__ M64, float* __restrict__ M, long long pitch,
@@ -566,14 +572,27 @@ emb_join_kernel(const EmbBuckets q, const T* __restrict__ Gb, const T* __restric
   };
   const bool single = n_val == 1 && n_train == 1;
   const int n_items = q.totals[3], stride = gridDim.x * 8;
-  int it = blockIdx.x * 8 + (threadIdx.x >> 5);
-  int4 item = it < n_items ? q.items[it] : make_int4(0, 0, 0, 0);
-  for (; it < n_items; it += stride) {
+  int pieces = 1, width = d;
+  if (CUT && n_items < 2 * stride && d > 128) {                // every lane weighs one number of pieces (see kEmbJoinAround)
+    constexpr int kStep = sizeof(T) == 2 ? 128 : 64;           // features of a round of loads
+    const unsigned tried = ((d + lane) / (lane + 1) + 127) / 128 * 128;
+    const unsigned rounds = (n_items * ((d + tried - 1) / tried) + stride - 1) / stride;
+    const unsigned cost = rounds * (kEmbJoinAround + (tried + kStep - 1) / kStep);
+    const unsigned least = __reduce_min_sync(0xffffffffu, cost);
+    width = __shfl_sync(0xffffffffu, tried, __ffs(__ballot_sync(0xffffffffu, cost == least)) - 1);
+    pieces = (d + width - 1) / width;
+  }
+  const int n_units = n_items * pieces;
+  auto item_of = [&](int u) { return CUT ? u / pieces : u; };
+  int unit = blockIdx.x * 8 + (threadIdx.x >> 5);
+  int4 item = unit < n_units ? q.items[item_of(unit)] : make_int4(0, 0, 0, 0);
+  for (; unit < n_units; unit += stride) {
     const int nb = item.y, at_v = item.z;
     const bool hot = item.w < 0;
     const int cv = hot ? n_val : item.w;
     const int my_b = lane < nb ? q.perm_b[item.x + lane] : 0;
-    if (it + stride < n_items) item = q.items[it + stride];
+    const int k0 = CUT ? unit % pieces * width : 0, dk = CUT && width < d - k0 ? width : d - k0;
+    if (unit + stride < n_units) item = q.items[item_of(unit + stride)];
     const int jb = __shfl_sync(0xffffffffu, my_b, g);
     const bool b_ok = g < nb;
     const int col = my_b / Tn;             // lanes 0..7: train sample of row `lane`
@@ -584,24 +603,25 @@ emb_join_kernel(const EmbBuckets q, const T* __restrict__ Gb, const T* __restric
       float acc[4] = {0.f, 0.f, 0.f, 0.f};
       int s0 = r0, s1 = r1, j0 = 0, j1 = 0;
       if (hot) {
-        const float* base = R + static_cast<long long>(at_v) * n_val * d;
+        const float* base = R + static_cast<long long>(at_v) * n_val * d + k0;
         emb_mma_rows<float, T, VEC>(base + static_cast<long long>(ok0 ? r0 : 0) * d, base + static_cast<long long>(ok1 ? r1 : 0) * d,
-                                    Gb + static_cast<long long>(jb) * d, ok0, ok1, b_ok, d, c, acc);
+                                    Gb + static_cast<long long>(jb) * d + k0, ok0, ok1, b_ok, dk, c, acc);
       } else {
         j0 = ok0 ? q.perm_v[at_v + r0] : 0;
         j1 = ok1 ? q.perm_v[at_v + r1] : 0;
         s0 = j0 / Tn;
         s1 = j1 / Tn;
-        emb_mma_rows<T, T, VEC>(Gv + static_cast<long long>(j0) * d, Gv + static_cast<long long>(j1) * d,
-                                Gb + static_cast<long long>(jb) * d, ok0, ok1, b_ok, d, c, acc);
+        emb_mma_rows<T, T, VEC>(Gv + static_cast<long long>(j0) * d + k0, Gv + static_cast<long long>(j1) * d + k0,
+                                Gb + static_cast<long long>(jb) * d + k0, ok0, ok1, b_ok, dk, c, acc);
       }
       const bool c0 = 2 * c < nb, c1 = 2 * c + 1 < nb;      // an absent row times an infinite one is no zero
       const unsigned redo = (ok0 && c0 && !isfinite(acc[0]) ? 1u : 0u) | (ok0 && c1 && !isfinite(acc[1]) ? 2u : 0u) |
                             (ok1 && c0 && !isfinite(acc[2]) ? 4u : 0u) | (ok1 && c1 && !isfinite(acc[3]) ? 8u : 0u);
       if (__any_sync(0xffffffffu, redo != 0)) {
         const float4 was = make_float4(acc[0], acc[1], acc[2], acc[3]);
-        const float4 is = hot ? emb_redo<float, T>(R + static_cast<long long>(at_v) * n_val * d, Gb, make_int2(s0, s1), my_b, redo, d, was)
-                              : emb_redo<T, T>(Gv, Gb, make_int2(j0, j1), my_b, redo, d, was);
+        const float4 is = hot ? emb_redo<float, T>(R + static_cast<long long>(at_v) * n_val * d + k0, Gb + k0, make_int2(s0, s1), my_b,
+                                                   redo, d, dk, was)
+                              : emb_redo<T, T>(Gv + k0, Gb + k0, make_int2(j0, j1), my_b, redo, d, dk, was);
         acc[0] = is.x; acc[1] = is.y; acc[2] = is.z; acc[3] = is.w;
       }
       if (single) {                        // every entry belongs to the one pair
@@ -976,6 +996,9 @@ static int emb_pass(const EmbBuckets& q, const T* Gb, const T* Gv, int n_train, 
     const int Ti = static_cast<int>(Tn);
     const long long most = (q.max_items + 7) / 8;
     const int jb = static_cast<int>(most < ds->sm_count * 2 ? most : ds->sm_count * 2);
+    const bool cut = q.first_val <= 4ll * 8 * jb;
+    const auto join = cut ? vec ? emb_join_kernel<T, true, true> : emb_join_kernel<T, false, true>
+                          : vec ? emb_join_kernel<T, true, false> : emb_join_kernel<T, false, false>;
     cudaLaunchAttribute beside = {};
     beside.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     beside.val.programmaticStreamSerializationAllowed = 1;
@@ -986,7 +1009,7 @@ static int emb_pass(const EmbBuckets& q, const T* Gb, const T* Gv, int n_train, 
     cfg.stream = st;
     cfg.attrs = &beside;
     cfg.numAttrs = out != nullptr ? 1 : 0;
-    GB_CUDA_OK(cudaLaunchKernelEx(&cfg, vec ? emb_join_kernel<T, true> : emb_join_kernel<T, false>, q, Gb, Gv, n_train, n_val, Ti,
+    GB_CUDA_OK(cudaLaunchKernelEx(&cfg, join, q, Gb, Gv, n_train, n_val, Ti,
                                   d, static_cast<const float*>(R), scale, M64, M, pitch, local));
     count_launch();
     if (!local) {

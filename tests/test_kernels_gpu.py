@@ -557,6 +557,26 @@ def test_embedding(case, dtype):
     assert torch.equal(grad.cpu().float(), ref.float())
 
 
+# the join's items cut into ranges of features: widths on and off the 128 features of a cut and of the 16-byte loads, one
+# cut or many, an infinite entry in one of them, hot ids
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("d", [128, 136, 701, 2056, 4224])
+@pytest.mark.parametrize("n_t,n_v,T,vocab", [(3, 2, 20, 7), (2, 2, 200, 3)])
+def test_embedding_dot_of_few_items(n_t, n_v, T, vocab, d, dtype):
+    g = torch.Generator().manual_seed(12)
+    ids = torch.randint(0, vocab, (n_t + n_v, T), generator=g)
+    G = (torch.randn(n_t + n_v, T, d, generator=g) / d ** 0.5).to(dtype)
+    M = ops().embedding_dot(ids.cuda(), G.cuda(), n_v, vocab)
+    after()
+    assert O.rel_fro(M, O.embedding_dot_exact(ids, G, n_v)) < (1e-5 if dtype == torch.float32 else 1e-4)
+    G[0, 0], G[0, 0, d - 1] = 0, float("inf")              # sample 0's row of one id: an infinity in the last range
+    G[n_t:, :, d - 1] = 1
+    ids[n_t:, 0] = ids[0, 0]
+    M = ops().embedding_dot(ids.cuda(), G.cuda(), n_v, vocab)
+    after()
+    assert (M[:, 0] == float("inf")).all() and torch.isfinite(M[:, 1:]).all()
+
+
 def test_embedding_position_ids_and_golden(golden):
     # position-embedding pattern: every sample has ids 0..T-1 (all buckets hold n_train tokens)
     n_t, n_v, T, d = 40, 2, 16, 24
