@@ -68,9 +68,9 @@ def _token_count(A: torch.Tensor) -> int:
 
 def _fp32_path_seconds(n_t: int, n_v: int, T: int, rows: int, cols: int):
     """``(per-sample path, Gram path)``: measured cost of a float32 layer of short samples with a weight of
-    ``rows x cols``, train gradient included.  At these sizes the fixed launches, the padding of the tiles and the second conversion of
-    both operands (the Gram path lays them out once for the Grams and once for the gradient) decide;
-    the rates alone chose the Gram path for 24 + 5 samples of 197 x (768 -> 1000), 176 us a hook against 112.
+    ``rows x cols``, train gradient included.  At these sizes the fixed launches, the padding of the tiles and the conversion of
+    the operands decide; the rates alone chose the Gram path for 24 + 5 samples of 197 x (768 -> 1000), 176 us a hook
+    against 112 when the costs were taken (the Gram path laid its operands out twice then), and against 83 now.
 
     Only for ``T <= 256`` and ``2 T <= d + p``: the tensor cores' float32 accumulation leaves a relative error
     of about 1e-8 per contracted token in the per-sample products and 5e-9 per feature in the Grams (70

@@ -564,7 +564,7 @@ def gradproj_embedding(ids: torch.Tensor, G: torch.Tensor, P_o_prepared: torch.T
     if _timing is None:
         return _native().gradproj_embedding(ids, G, P_o_prepared, P_i_t, k_o, k_i, scale, out)
     rows, d = ids.numel(), _cols(G)
-    with _Timed("gradproj_embedding_kernel", "hbm", 2.0 * rows * (d * k_o + k_o * k_i),
+    with _Timed("gradproj_kernel", "hbm", 2.0 * rows * (d * k_o + k_o * k_i),
                 float(rows) * (d * G.element_size() + 8 + 4 * k_i) + 4.0 * ids.shape[0] * k_o * k_i):
         return _native().gradproj_embedding(ids, G, P_o_prepared, P_i_t, k_o, k_i, scale, out)
 
