@@ -62,6 +62,10 @@ inline cudaError_t launch_next(void (*kernel)(P...), dim3 grid, dim3 block, size
 // The other half of launch_next, in every kernel that is launched so, before its first access to global memory and in every
 // block: waits until all work ahead in the stream has ended and can be read, then lets the next kernel come up.  (In
 // that order: a kernel that ends has waited, so its end stands for everything before it.)
+//
+// Such a kernel exists while the one ahead still writes, so what it reads is not read-only for as long as it lives: no
+// __ldg and no const __restrict__ pointers, whose loads may be served from a line that is older than the wait, or be moved
+// ahead of it.  Ordinary loads stay behind the wait.
 __device__ __forceinline__ void stream_order() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

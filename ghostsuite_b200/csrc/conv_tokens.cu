@@ -108,7 +108,7 @@ __device__ __forceinline__ void conv_tile(const ConvTokens& q, unsigned t0, int 
   }
 }
 
-template <typename E> __device__ __forceinline__ void row_sum(const E* __restrict__ x, long long r, long long len, float* __restrict__ out) {
+template <typename E> __device__ __forceinline__ void row_sum(const E* x, long long r, long long len, float* __restrict__ out) {
   float s = 0.f;
 #pragma unroll 4
   for (long long i = threadIdx.x & 31; i < len; i += 32) s += ct_f32<E>(x[r * len + i]);
@@ -142,7 +142,7 @@ __global__ void __launch_bounds__(256) conv_tokens_kernel(const __grid_constant_
 // out[r] = sum of row r of a dense [rows, len] matrix: per-sample, per-channel sums of an NCHW out-grad.
 // One warp per row; the rows are contiguous, so the loads are.
 template <typename E>
-__global__ void __launch_bounds__(256) row_sums_kernel(const E* __restrict__ x, long long rows, long long len, float* __restrict__ out) {
+__global__ void __launch_bounds__(256) row_sums_kernel(const E* x, long long rows, long long len, float* __restrict__ out) {
   stream_order();
   const long long r = blockIdx.x * 8ll + (threadIdx.x >> 5);
   if (r < rows) row_sum(x, r, len, out);

@@ -33,9 +33,9 @@ __device__ __forceinline__ float4 sd_load4(const E* p, int left) {
   if constexpr (VEC) {
     if (left <= 0) return make_float4(0.f, 0.f, 0.f, 0.f);
     if constexpr (sizeof(E) == 4) {
-      return __ldg(reinterpret_cast<const float4*>(p));
+      return *reinterpret_cast<const float4*>(p);
     } else {
-      const uint2 w = __ldg(reinterpret_cast<const uint2*>(p));
+      const uint2 w = *reinterpret_cast<const uint2*>(p);
       return make_float4(__uint_as_float(w.x << 16), __uint_as_float(w.x & 0xffff0000u), __uint_as_float(w.y << 16),
                          __uint_as_float(w.y & 0xffff0000u));
     }

@@ -134,7 +134,7 @@ emb_chain_dot_kernel(const long long* __restrict__ ids, const T* __restrict__ G,
 
 // Shared pieces of the two segment-sum kernels.  A thread owns 8 consecutive features.
 template <typename T>
-__device__ __forceinline__ void emb_load_row(const T* __restrict__ G, int j, int d, int f, bool vec, float (&x)[8]) {
+__device__ __forceinline__ void emb_load_row(const T* G, int j, int d, int f, bool vec, float (&x)[8]) {
   const T* row = G + static_cast<long long>(j) * d + f;
   if (vec) {
     if (f < d) {
@@ -354,7 +354,7 @@ __global__ void __launch_bounds__(256) emb_fill_kernel(const EmbBuckets q) {
 // features of every groups-th token, four rows in flight, and the groups meet in shared memory.
 template <typename T>
 __global__ void __launch_bounds__(256)
-emb_hot_reduce_kernel(const EmbBuckets q, const T* __restrict__ Gv, long long Tn, int d, int n_val, float* __restrict__ R) {
+emb_hot_reduce_kernel(const EmbBuckets q, const T* Gv, long long Tn, int d, int n_val, float* __restrict__ R) {
   stream_order();
   __shared__ int s_tok[1024];
   __shared__ __align__(16) float s_sum[256 * 8];
@@ -551,6 +551,8 @@ __device__ __noinline__ float4 emb_redo(const VT* V, const BT* B, int2 lv, int m
 // hook, 168 now (9 + 3 x 333 of 701 67 and 50).  There (CUT) items fall into pieces of a range of features where that shortens
 // the rounds that a warp goes through, a piece's indices and sums counted as kEmbJoinAround of them.  Batches
 // of more train tokens than four a warp have items enough (at 32 x 1024 the arithmetic alone cost 1.2 us of 99).
+// What it reads (rows, buckets, hot sums) was written before the gradient kernel ahead of it passed its own wait, and so before
+// a block of the join came up: read-only for the join's whole life, unlike in the kernels that wait at their start.
 constexpr int kEmbJoinAround = 2;
 template <typename T, bool VEC, bool CUT>
 __global__ void __launch_bounds__(256, 2)
@@ -677,7 +679,7 @@ __global__ void __launch_bounds__(256) emb_round_kernel(const double* __restrict
 constexpr int kEmbGrab = 4;
 
 template <typename T>
-__device__ __forceinline__ void emb_small_rows(const EmbBuckets& q, const T* __restrict__ G, int d, float pre_scale,
+__device__ __forceinline__ void emb_small_rows(const EmbBuckets& q, const T* G, int d, float pre_scale,
                                                float divisor, int accumulate, T* __restrict__ out) {
   const int lane = threadIdx.x & 31;
   const bool vec = (d % 8 == 0) && ((reinterpret_cast<uintptr_t>(G) & 15u) == 0) &&
@@ -762,7 +764,7 @@ constexpr int kBigList = 2048;           // list entries held at a time
 constexpr int kBigStage = 32, kBigSlots = 3;
 
 template <typename T>
-__device__ __forceinline__ void emb_big_rows(const EmbBuckets& q, const T* __restrict__ G, int d, int slices, float pre_scale,
+__device__ __forceinline__ void emb_big_rows(const EmbBuckets& q, const T* G, int d, int slices, float pre_scale,
                                              float divisor, int accumulate, T* __restrict__ out) {
   constexpr int kFeat = 256 / static_cast<int>(sizeof(T));
   constexpr int kPer = 16 / static_cast<int>(sizeof(T));       // features of a 16-byte piece
@@ -907,7 +909,7 @@ __device__ void emb_zero_rows(const EmbBuckets& q, int d, T* __restrict__ out) {
 
 template <typename T>
 __global__ void __launch_bounds__(kEmbGradThreads, 6)
-emb_grad_kernel(const EmbBuckets q, const T* __restrict__ G, int d, int slices, float pre_scale, float divisor,
+emb_grad_kernel(const EmbBuckets q, const T* G, int d, int slices, float pre_scale, float divisor,
                 int accumulate, int zero_rows, T* __restrict__ out) {
   stream_order();                        // from here on the join may start beside this grid's tail
   emb_big_rows<T>(q, G, d, slices, pre_scale, divisor, accumulate, out);

@@ -109,12 +109,12 @@ template <> struct GpRows<kSrcF32> {
     for (int i = 0; i < 8; ++i, p += 2 * ld) {
       const bool in = r0 + 2 * i < rows;
       if (vec) {                           // widths are multiples of four here
-        v[i] = in && cols > 0 ? __ldg(reinterpret_cast<const float4*>(p)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        v[i] = in && cols > 0 ? *reinterpret_cast<const float4*>(p) : make_float4(0.f, 0.f, 0.f, 0.f);
       } else {
-        v[i].x = in && cols > 0 ? __ldg(p) : 0.f;
-        v[i].y = in && cols > 1 ? __ldg(p + 1) : 0.f;
-        v[i].z = in && cols > 2 ? __ldg(p + 2) : 0.f;
-        v[i].w = in && cols > 3 ? __ldg(p + 3) : 0.f;
+        v[i].x = in && cols > 0 ? *p : 0.f;
+        v[i].y = in && cols > 1 ? p[1] : 0.f;
+        v[i].z = in && cols > 2 ? p[2] : 0.f;
+        v[i].w = in && cols > 3 ? p[3] : 0.f;
       }
     }
   }
@@ -144,14 +144,14 @@ template <> struct GpRows<kSrcBf16> {
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         const bool in = r0 + 2 * i < rows && c < left;         // widths are multiples of four here
-        const uint2 w = in ? __ldg(reinterpret_cast<const uint2*>(p + (r0 + 2 * i) * ld + c)) : make_uint2(0u, 0u);
+        const uint2 w = in ? *reinterpret_cast<const uint2*>(p + (r0 + 2 * i) * ld + c) : make_uint2(0u, 0u);
         v[2 * i] = w.x; v[2 * i + 1] = w.y;
       }
     } else {
 #pragma unroll
       for (int i = 0; i < 32; ++i) {
         const int r = i >> 1, c = (i & 1) * 32 + lane;
-        v[i] = r < rows && c < left ? __ldg(p + r * ld + c) : 0u;
+        v[i] = r < rows && c < left ? p[r * ld + c] : 0u;
       }
     }
   }
@@ -416,12 +416,12 @@ gradproj_kernel(const __grid_constant__ CUtensorMap tm_g, const __grid_constant_
         mine[q] = make_float4(0.f, 0.f, 0.f, 0.f);
         if (id < 0 || 4 * q >= p.k_c) continue;
         if (p.rows_vec) {
-          mine[q] = __ldg(reinterpret_cast<const float4*>(src + 4 * q));
+          mine[q] = *reinterpret_cast<const float4*>(src + 4 * q);
         } else {
-          mine[q].x = __ldg(src + 4 * q);
-          if (4 * q + 1 < p.k_c) mine[q].y = __ldg(src + 4 * q + 1);
-          if (4 * q + 2 < p.k_c) mine[q].z = __ldg(src + 4 * q + 2);
-          if (4 * q + 3 < p.k_c) mine[q].w = __ldg(src + 4 * q + 3);
+          mine[q].x = src[4 * q];
+          if (4 * q + 1 < p.k_c) mine[q].y = src[4 * q + 1];
+          if (4 * q + 2 < p.k_c) mine[q].z = src[4 * q + 2];
+          if (4 * q + 3 < p.k_c) mine[q].w = src[4 * q + 3];
         }
       }
     };

@@ -59,8 +59,10 @@ __device__ __forceinline__ void pass_stage(const ghost_pass_job& j, bool vec, in
       asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))),
                    "l"(src + f + q) : "memory");
     } else {
+      float x[4];
 #pragma unroll
-      for (int e = 0; e < 4; ++e) dst[e] = q + e < width ? __ldg(src + f + q + e) : 0.f;
+      for (int e = 0; e < 4; ++e) x[e] = q + e < width ? src[f + q + e] : 0.f;
+      *reinterpret_cast<float4*>(dst) = make_float4(x[0], x[1], x[2], x[3]);
     }
   }
   asm volatile("cp.async.wait_all;" ::: "memory");
@@ -83,14 +85,14 @@ __device__ __forceinline__ void pass_row_sums(const ghost_pass_job& j, int f0, i
         const int c = c0 + g * 128 * n_blk + lane * 4;
         if constexpr (VEC) {
           if (c < f1) {
-            const float4 x = __ldg(reinterpret_cast<const float4*>(row + c));
+            const float4 x = *reinterpret_cast<const float4*>(row + c);
             acc[g].x += x.x; acc[g].y += x.y; acc[g].z += x.z; acc[g].w += x.w;
           }
         } else {
-          if (c < f1) acc[g].x += __ldg(row + c);
-          if (c + 1 < f1) acc[g].y += __ldg(row + c + 1);
-          if (c + 2 < f1) acc[g].z += __ldg(row + c + 2);
-          if (c + 3 < f1) acc[g].w += __ldg(row + c + 3);
+          if (c < f1) acc[g].x += row[c];
+          if (c + 1 < f1) acc[g].y += row[c + 1];
+          if (c + 2 < f1) acc[g].z += row[c + 2];
+          if (c + 3 < f1) acc[g].w += row[c + 3];
         }
       }
     }
@@ -249,7 +251,7 @@ pass_reduce_kernel(const __grid_constant__ PassJobs<CAP> jobs) {
 // are too few to fill the GPU once a pair is long or the validation rows are many (a cluster goes through
 // them eight at a time).  256 x 256 pairs of 768: 93 us in the clusters, 31 here; 256 x 32 of 50257: 473 and 141;
 // 16384 x 1 of 1024: 49 and 19.  Smaller ones, and every matrix of a batch, stay with the clusters, which fetch a row once.
-__global__ void __launch_bounds__(256) small_gram_kernel(const float* __restrict__ X, int n_train, unsigned pairs, int F,
+__global__ void __launch_bounds__(256) small_gram_kernel(const float* X, int n_train, unsigned pairs, int F,
                                                          float scale, float* __restrict__ M) {
   stream_order();
   const unsigned pair = blockIdx.x * 8u + (threadIdx.x >> 5);
@@ -261,7 +263,7 @@ __global__ void __launch_bounds__(256) small_gram_kernel(const float* __restrict
   float even[4] = {0.f, 0.f, 0.f, 0.f}, odd[4] = {0.f, 0.f, 0.f, 0.f};      // short chains: 256 sums a pair
   if ((F & 3) == 0 && (reinterpret_cast<uintptr_t>(X) & 15) == 0) {
     auto add = [&](int f, float (&sum)[4]) {
-      const float4 x = __ldg(reinterpret_cast<const float4*>(xv) + f), y = __ldg(reinterpret_cast<const float4*>(xb) + f);
+      const float4 x = reinterpret_cast<const float4*>(xv)[f], y = reinterpret_cast<const float4*>(xb)[f];
       sum[0] = fmaf(x.x, y.x, sum[0]); sum[1] = fmaf(x.y, y.y, sum[1]);
       sum[2] = fmaf(x.z, y.z, sum[2]); sum[3] = fmaf(x.w, y.w, sum[3]);
     };
@@ -276,8 +278,8 @@ __global__ void __launch_bounds__(256) small_gram_kernel(const float* __restrict
 #pragma unroll
       for (int u = 0; u < 16; ++u) {
         const bool in = f0 + u * 32 < F;
-        x[u] = in ? __ldg(xv + f0 + u * 32) : 0.f;
-        y[u] = in ? __ldg(xb + f0 + u * 32) : 0.f;
+        x[u] = in ? xv[f0 + u * 32] : 0.f;
+        y[u] = in ? xb[f0 + u * 32] : 0.f;
       }
 #pragma unroll
       for (int u = 0; u < 16; ++u) {
@@ -297,7 +299,7 @@ __global__ void __launch_bounds__(256) small_gram_kernel(const float* __restrict
 // blocks that a job's pairs ask for.  4 rows of 1000003: 245 us in the
 // batched kernel, 17 here; 256 of 50257: 68 and 16; 16384 of 1024: 626 and 123.
 template <int COLS>
-__global__ void __launch_bounds__(256) rows_sum_kernel(const float* __restrict__ X, int n_rows, int F, float scale,
+__global__ void __launch_bounds__(256) rows_sum_kernel(const float* X, int n_rows, int F, float scale,
                                                        void* __restrict__ out, int out_is_f32, int accumulate) {
   stream_order();
   constexpr int PER = COLS / 32;
@@ -312,7 +314,7 @@ __global__ void __launch_bounds__(256) rows_sum_kernel(const float* __restrict__
     const float* row = X + static_cast<long long>(n) * F + c0;
 #pragma unroll
     for (int g = 0; g < PER; ++g)
-      if (c0 + g * 32 + lane < F) acc[g] += __ldg(row + g * 32 + lane);
+      if (c0 + g * 32 + lane < F) acc[g] += row[g * 32 + lane];
   }
 #pragma unroll
   for (int g = 0; g < PER; ++g) red[warp][g * 32 + lane] = acc[g];
@@ -374,7 +376,7 @@ matrix_sum_kernel(const __grid_constant__ MatrixList list, int n, int n_val, int
     float s = 0.f;
     if (live) {
 #pragma unroll 8
-      for (int p = grp; p < n; p += 4) s += __ldg(list.m[p] + at);
+      for (int p = grp; p < n; p += 4) s += list.m[p][at];
     }
     red[grp][row][lane] = s;
     __syncthreads();

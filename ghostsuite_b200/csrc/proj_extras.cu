@@ -82,15 +82,15 @@ template <typename PT, bool VEC> struct SimOct {
       if (VEC) {
         const bool in = ok && k < d;       // D % 8 == 0
         const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
-        *reinterpret_cast<float4*>(&v[0]) = in ? __ldg(reinterpret_cast<const float4*>(row + k)) : z;
-        *reinterpret_cast<float4*>(&v[4]) = in ? __ldg(reinterpret_cast<const float4*>(row + k + 4)) : z;
+        *reinterpret_cast<float4*>(&v[0]) = in ? *reinterpret_cast<const float4*>(row + k) : z;
+        *reinterpret_cast<float4*>(&v[4]) = in ? *reinterpret_cast<const float4*>(row + k + 4) : z;
       } else {
 #pragma unroll
-        for (int e = 0; e < 8; ++e) v[e] = ok && k + e < d ? __ldg(row + k + e) : 0.f;
+        for (int e = 0; e < 8; ++e) v[e] = ok && k + e < d ? row[k + e] : 0.f;
       }
     } else {
       if (VEC) {
-        raw = ok && k < d ? __ldg(reinterpret_cast<const uint4*>(row + k)) : make_uint4(0u, 0u, 0u, 0u);
+        raw = ok && k < d ? *reinterpret_cast<const uint4*>(row + k) : make_uint4(0u, 0u, 0u, 0u);
       } else {
         __nv_bfloat16 x[8];
 #pragma unroll

@@ -216,7 +216,7 @@ __global__ void __launch_bounds__(256, 4) split_pair_kernel(const SplitParams p)
 // per-sample column sums: out[n, c] += sum_{t in split} G[n, t, c]
 // ------------------------------------------------------------------------------------------
 template <typename T>
-__global__ void colsum_kernel(const T* __restrict__ G, long long Tn, int cols, long long ld,
+__global__ void colsum_kernel(const T* G, long long Tn, int cols, long long ld,
                               float* __restrict__ out, int t_splits) {
   // block: 32 column vectors (256 columns) x 8 row lanes
   __shared__ float red[8][256 + 8];
@@ -316,7 +316,7 @@ constexpr int kLnSlots = 3;
 
 template <typename T, int NCHUNK, bool FULL>
 __global__ void __launch_bounds__(256, NCHUNK <= 3 ? 2 : 1)
-layernorm_persample_kernel(const T* __restrict__ A, const T* __restrict__ G, long long Tn, int F,
+layernorm_persample_kernel(const T* A, const T* G, long long Tn, int F,
                            float eps, float* __restrict__ gw, float* __restrict__ gb,
                            float* __restrict__ part, int t_splits, int rms) {
   stream_order();
@@ -437,7 +437,7 @@ layernorm_persample_kernel(const T* __restrict__ A, const T* __restrict__ G, lon
 }
 
 // second stage: sum the per-split partials in a fixed order (deterministic)
-__global__ void layernorm_reduce_kernel(const float* __restrict__ part, int N, int F, int t_splits,
+__global__ void layernorm_reduce_kernel(const float* part, int N, int F, int t_splits,
                                         float* __restrict__ gw, float* __restrict__ gb) {
   stream_order();
   const long long total = static_cast<long long>(N) * 2 * F;
@@ -461,7 +461,7 @@ __global__ void layernorm_reduce_kernel(const float* __restrict__ part, int N, i
 // 380 -> 97, F = 731 173 -> 60; RMS norm, 12 x 1024 rows of F = 8192: 1179 -> 138.
 template <typename T, bool VEC, int PT, int THREADS>
 __global__ void __launch_bounds__(THREADS, THREADS == 256 ? 2 : 1)
-norm_wide_kernel(const T* __restrict__ A, const T* __restrict__ G, long long Tn, int F, float eps, float* __restrict__ gw,
+norm_wide_kernel(const T* A, const T* G, long long Tn, int F, float eps, float* __restrict__ gw,
                  float* __restrict__ gb, float* __restrict__ part, int t_splits, int rms) {
   constexpr int R = 32 / PT, W = THREADS / 32;
   // Rows added up in registers before they join the totals: one chain over all rows of a split had 1.7 times the

@@ -503,7 +503,7 @@ tile_dot_mma_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_const
 
 // out[r, c] (= or +=) scale * sum[tile(r, c)][r % 128][c % 256], cast to the parameter dtype
 template <typename OutT>
-__global__ void tile_sum_finalize_kernel(const float* __restrict__ sum, int n_tiles_n, OutT* __restrict__ out,
+__global__ void tile_sum_finalize_kernel(const float* sum, int n_tiles_n, OutT* __restrict__ out,
                                          int rows, int cols, float scale, int accumulate) {
   stream_order();
   const long long n = static_cast<long long>(rows) * cols;

@@ -43,7 +43,7 @@ __device__ __forceinline__ void xty_colsum_finish(const float (&a)[8], int cbase
 // the next multiple of eight columns) into out[cbase ..].  ct = 0..127 is the thread's index among
 // the column-sum warps; red is 8 * 128 floats of shared memory; up to sixteen 16-byte loads are in flight
 // per thread.
-__device__ __forceinline__ void xty_colsum_128(const __nv_bfloat16* __restrict__ src, XtyRows rows, bool alone, long long ld,
+__device__ __forceinline__ void xty_colsum_128(const __nv_bfloat16* src, XtyRows rows, bool alone, long long ld,
                                                int cbase, int total_cols, float* red, float* __restrict__ out, int ct, int bar_id) {
   const int cv = ct & 15, rl = ct >> 4;     // 16 column vectors x 8 row lanes
   const int c0 = cbase + cv * 8;
@@ -67,19 +67,19 @@ __device__ __forceinline__ void xty_colsum_128(const __nv_bfloat16* __restrict__
     for (; t + 120 < T; t += 128) {
       uint4 w[16];
 #pragma unroll
-      for (int q = 0; q < 16; ++q) w[q] = __ldg(reinterpret_cast<const uint4*>(base + (t + 8 * q) * ld));
+      for (int q = 0; q < 16; ++q) w[q] = *reinterpret_cast<const uint4*>(base + (t + 8 * q) * ld);
 #pragma unroll
       for (int q = 0; q < 16; q += 4) add4(w[q], w[q + 1], w[q + 2], w[q + 3]);
     }
     for (; t + 24 < T; t += 32) {
-      const uint4 w0 = __ldg(reinterpret_cast<const uint4*>(base + t * ld));
-      const uint4 w1 = __ldg(reinterpret_cast<const uint4*>(base + (t + 8) * ld));
-      const uint4 w2 = __ldg(reinterpret_cast<const uint4*>(base + (t + 16) * ld));
-      const uint4 w3 = __ldg(reinterpret_cast<const uint4*>(base + (t + 24) * ld));
+      const uint4 w0 = *reinterpret_cast<const uint4*>(base + t * ld);
+      const uint4 w1 = *reinterpret_cast<const uint4*>(base + (t + 8) * ld);
+      const uint4 w2 = *reinterpret_cast<const uint4*>(base + (t + 16) * ld);
+      const uint4 w3 = *reinterpret_cast<const uint4*>(base + (t + 24) * ld);
       add4(w0, w1, w2, w3);
     }
     for (; t < T; t += 8) {
-      const uint4 w = __ldg(reinterpret_cast<const uint4*>(base + t * ld));
+      const uint4 w = *reinterpret_cast<const uint4*>(base + t * ld);
       const uint32_t x[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
       for (int e = 0; e < 4; ++e) { a[2 * e] += lo(x[e]); a[2 * e + 1] += hi(x[e]); }

@@ -395,7 +395,7 @@ xty_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant_
 
 // finalize: out = (accumulate ? out : 0) + scale * ws, cast to the parameter dtype
 template <typename OutT>
-__global__ void xty_finalize_kernel(const float* __restrict__ ws, long long ld_ws, OutT* __restrict__ out,
+__global__ void xty_finalize_kernel(const float* ws, long long ld_ws, OutT* __restrict__ out,
                                     int rows, int cols, float scale, int accumulate) {
   stream_order();
   const long long n = static_cast<long long>(rows) * cols;

@@ -1,0 +1,50 @@
+"""CPU checks of rules that the CUDA sources keep and that no compiler checks."""
+import glob
+import os
+import re
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "ghostsuite_b200", "csrc")
+
+
+def _sources():
+    """``{file name: text}`` without comments."""
+    out = {}
+    for path in sorted(glob.glob(os.path.join(CSRC, "*.cu")) + glob.glob(os.path.join(CSRC, "*.cuh"))):
+        text = open(path).read()
+        out[os.path.basename(path)] = re.sub(r"//[^\n]*", "", re.sub(r"/\*.*?\*/", "", text, flags=re.S))
+    return out
+
+
+def _body(text, start):
+    """``text`` from the first brace at or after ``start`` to the one that closes it."""
+    i = text.index("{", start)
+    depth = 0
+    for j in range(i, len(text)):
+        depth += {"{": 1, "}": -1}.get(text[j], 0)
+        if depth == 0:
+            return text[i:j + 1]
+    raise AssertionError("unbalanced braces")
+
+
+def _kernels(text):
+    """``(name, parameters, body)`` of every ``__global__`` function that is defined in ``text``."""
+    for m in re.finditer(r"__global__\b", text):
+        head = re.compile(r"\b(\w+_kernel)\s*\(([^{;]*)\)\s*\{").search(text, m.end())
+        yield head.group(1), head.group(2), _body(text, head.end() - 1)
+
+
+def test_kernels_that_start_early_read_with_ordinary_loads():
+    """A kernel launched with programmatic stream order lives while the one ahead of it still writes, so its
+    loads must not go through the read-only path (``ld.global.nc``: memory that nobody writes while the
+    kernel lives)."""
+    early = 0
+    for name, text in _sources().items():
+        for kernel, params, body in _kernels(text):
+            if "stream_order()" in body:
+                early += 1
+                assert not re.search(r"const\s+\w+\s*\*\s*__restrict__", params), f"{name}: {kernel}"
+        if name == "embedding.cu":       # the rows of the join, which come up behind everything that it reads
+            for m in re.finditer(r"struct EmbOct<\w+>", text):
+                text = text.replace(_body(text, m.end()), "{" + " " * (len(_body(text, m.end())) - 2) + "}")
+        assert "__ldg(" not in text and "ld.global.nc" not in text, name
+    assert early >= 20

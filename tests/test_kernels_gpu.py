@@ -1194,3 +1194,39 @@ def test_gradproj_embedding_unit_counts_and_widths(case, dtype):
     after()
     ref = torch.einsum("bto,bti->boi", G.double() @ P_o.double().t(), P_i.double().t()[ids])
     assert O.rel_fro(out, ref.flatten(1)) < (2 * 2.0 ** -15 if split else 2 * 2.0 ** -8)
+
+
+@pytest.mark.parametrize("n_t,n_v,T,F", [(32, 8, 64, 768), (5, 2, 9, 701), (48, 12, 3, 4096)])
+def test_kernels_that_start_early_see_what_the_kernel_ahead_wrote(n_t, n_v, T, F):
+    """A chain of deterministic reductions, again and again in the same buffers with other values: launched
+    as usual, each kernel up while the one ahead still writes, and captured, where the order is plain.  The
+    same additions in the same order: the same bits."""
+    from ghostsuite_b200 import _lib
+    A, G = torch.empty(n_t + n_v, T, F, device="cuda"), torch.empty(n_t + n_v, T, F, device="cuda")
+
+    def chain():
+        gw, gb = ops().layernorm_persample(A, G, 1e-5)
+        M, Mb = ops().small_gram(gw, n_v), ops().small_gram(gb, n_v)
+        s = ops().rows_sum(gw, n_t, 1.0, torch.float32)
+        return gw, gb, M, Mb, s, ops().matrix_sum([M, Mb])[:(n_v + 1) * n_t]      # the word behind them is the error word
+
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    A.normal_(generator=gen)
+    G.normal_(generator=gen)
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        chain()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        plain = chain()
+    for _ in range(50):
+        A.normal_(generator=gen)
+        G.normal_(generator=gen)
+        early = chain()
+        graph.replay()
+        for x, y in zip(early, plain):
+            assert torch.equal(x, y)
+        del early, x
+    torch.cuda.synchronize()
+    _lib.poll_kernel_error()
