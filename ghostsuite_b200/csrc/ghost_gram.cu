@@ -17,6 +17,7 @@
 // Pipeline: kStages shared-memory stages (train tile 128xBK + val tile BNxBK bf16 in 64-element atoms, 128B swizzle),
 // full/empty mbarriers per stage, acc_full/acc_empty mbarriers per accumulator buffer.
 #include "common.cuh"
+#include "gram_operands.cuh"
 #include "sm100_ptx.cuh"
 
 namespace gb {
@@ -278,19 +279,10 @@ ghost_gram_kernel(const __grid_constant__ CUtensorMap tm_at, const __grid_consta
   }
 }
 
-// Operands of the two Grams: rows of train and validation tokens
-struct GramOperands {
-  const void *a_t, *a_v, *g_t, *g_v;
-  long long ld_at, ld_av, ld_gt, ld_gv;
-  int ka, kg;
-  int parts;
-  long long part_rows;     // parts == 2: rows of a part in memory
-};
 static int gram_map(CUtensorMap* t, const GramOperands& o, const void* base, long long rows, int k, long long ld, int box_rows) {
   return o.parts == 2 ? make_tmap_bf16_part_rows(t, base, o.part_rows, rows, ld, box_rows)
                       : make_tmap_bf16_2d(t, base, rows, k, ld, box_rows);
 }
-// Maps of the four operands: train rows in boxes of box_t, validation rows of box_v
 int gram_maps(CUtensorMap (&t)[4], const GramOperands& o, long long rows_t, long long rows_v, int box_t, int box_v) {
   int rc;
   if ((rc = gram_map(&t[0], o, o.a_t, rows_t, o.ka, o.ld_at, box_t)) != GHOST_OK) return rc;
@@ -332,9 +324,6 @@ static int launch_gram(const GramOperands& o, int n_train, int n_val, long long 
   count_launch();
   return post_launch("ghost_gram_kernel");
 }
-
-int launch_gram_pair(const GramOperands& o, int n_train, int n_val, long long T, int round_mode, float scale, float* M,
-                     const DeviceState* ds, cudaStream_t stream);
 
 // 0: single-CTA kernels only; 1: CTA-pair kernel for problems with at least 512 train tokens and 256
 // to 8192 validation tokens (where it measured faster: 1474 against 1339 TFLOP/s with 32768 x 4096

@@ -12,6 +12,7 @@
 // acc_empty lives in the leader and counts the eight epilogue warps of the pair.  All mbarrier
 // waits are bounded; the cluster barrier before teardown is reached by every thread.
 #include "common.cuh"
+#include "gram_operands.cuh"
 #include "sm100_ptx.cuh"
 
 namespace gb {
@@ -262,15 +263,6 @@ ghost_gram_pair_kernel(const __grid_constant__ CUtensorMap tm_at, const __grid_c
     tmem_dealloc_pair(tmem_base, 512);
   }
 }
-
-struct GramOperands {      // as in ghost_gram.cu
-  const void *a_t, *a_v, *g_t, *g_v;
-  long long ld_at, ld_av, ld_gt, ld_gv;
-  int ka, kg;
-  int parts;
-  long long part_rows;
-};
-int gram_maps(CUtensorMap (&t)[4], const GramOperands& o, long long rows_t, long long rows_v, int box_t, int box_v);
 
 template <int PARTS>
 static int launch_gram_pair_t(const CUtensorMap (&t)[4], const GramPairParams& p, const DeviceState* ds, cudaStream_t stream) {

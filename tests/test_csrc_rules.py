@@ -48,3 +48,19 @@ def test_kernels_that_start_early_read_with_ordinary_loads():
                 text = text.replace(_body(text, m.end()), "{" + " " * (len(_body(text, m.end())) - 2) + "}")
         assert "__ldg(" not in text and "ld.global.nc" not in text, name
     assert early >= 20
+
+
+def test_a_type_is_defined_once():
+    """The translation units pass structures to each other by reference: a second definition of one that is
+    changed later would still link."""
+    where = {}
+    for name, text in _sources().items():
+        for m in re.finditer(r"\b(?:struct|class|union)\s+(\w+(?:<[^<>{};]*>)?)\s*(?::[^{;]*)?\{", text):
+            where.setdefault(m.group(1), []).append(name)
+    assert len(where) > 20
+    assert {k: v for k, v in where.items() if len(v) > 1} == {}
+
+
+def test_every_header_makes_the_library_stale():
+    from ghostsuite_b200 import build
+    assert {n for n in _sources() if n.endswith(".cuh")} <= set(build.HEADERS)
