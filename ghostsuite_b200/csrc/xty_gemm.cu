@@ -67,7 +67,9 @@ struct XtyCfg {
   static constexpr int kStages = 4;
   static constexpr int kColsumBytes = PARTS == 1 ? 8 * 128 * 4 : 0;      // reduction scratch of the column-sum warps
   static constexpr int kBoxBytes = PARTS * 4 * 32 * 32 * 4;  // store_grad_block32 (a box per epilogue warp), store_tile_f32
-  static constexpr int kSmemBytes = kStages * kStageBytes + 1024 + 256 + kColsumBytes + kBoxBytes;
+  // stages, boxes, barriers, scratch, from a 1024-byte boundary on, which the dynamic shared memory need not start at
+  static constexpr int kBarOffset = kStages * kStageBytes + kBoxBytes, kRedOffset = kBarOffset + 256;
+  static constexpr int kSmemBytes = 1024 + kRedOffset + kColsumBytes;
 };
 
 // one 256-bit store (the address must be 32-byte aligned)
@@ -107,7 +109,7 @@ xty_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant_
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* store_box = smem + kStages * Cfg::kStageBytes;      // 1024-byte aligned
-  uint64_t* bars = reinterpret_cast<uint64_t*>(store_box + Cfg::kBoxBytes);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::kBarOffset);
   uint64_t* full_bar = bars;
   uint64_t* empty_bar = bars + kStages;
   uint64_t* acc_full = bars + 2 * kStages;     // [2]
@@ -272,7 +274,7 @@ xty_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant_
   } else if (kColsum && warp >= 6) {
     // ---------------------------------------------------------------- column sums (warps 6-9)
     // see xty_colsum.cuh
-    float* red = reinterpret_cast<float*>(smem + kStages * Cfg::kStageBytes + Cfg::kBoxBytes + 1024 + 256);
+    float* red = reinterpret_cast<float*>(smem + Cfg::kRedOffset);
     const int ct = static_cast<int>(threadIdx.x) - 192;
     const bool of_y = p.cs.of == 2;
     const int total_cols = of_y ? p.n_cols : p.m_cols;

@@ -81,7 +81,9 @@ struct XtyPairCfg {
   static constexpr int kStoreBoxBytes = 128 * 32 * 2 * PARTS;
   static constexpr int kStoreBytes = 2 * kStoreBoxBytes;
   static constexpr int kColsumBytes = PARTS == 1 ? 8 * 128 * 4 : 0;      // cross-row-lane reduction of the column-sum warps
-  static constexpr int kSmemBytes = kStages * kStageBytes + kStoreBytes + 1024 + 256 + kColsumBytes;
+  // stages, boxes, barriers, scratch, from a 1024-byte boundary on, which the dynamic shared memory need not start at
+  static constexpr int kBarOffset = kStages * kStageBytes + kStoreBytes, kRedOffset = kBarOffset + 256;
+  static constexpr int kSmemBytes = 1024 + kRedOffset + kColsumBytes;
 };
 
 __device__ __forceinline__ void st_global_v8_pair(void* addr, const uint32_t* v) {
@@ -114,7 +116,7 @@ xty_gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* store_box = smem + kStages * Cfg::kStageBytes;      // 1024-byte aligned
-  uint64_t* bars = reinterpret_cast<uint64_t*>(store_box + Cfg::kStoreBytes);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::kBarOffset);
   uint64_t* full_bar = bars;                 // used in the leader only
   uint64_t* empty_bar = bars + kStages;      // both CTAs
   uint64_t* acc_full = bars + 2 * kStages;   // [2], both CTAs
@@ -263,7 +265,7 @@ xty_gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
     // ------------------------------------------------------------------ column sums (warps 6-9, both CTAs)
     // Present only in launches that ask for them (320 threads): CTA r takes the 128 columns of a 256-column block
     // that it also loads for the tensor core.
-    float* red = reinterpret_cast<float*>(smem + kStages * Cfg::kStageBytes + Cfg::kStoreBytes + 1024 + 256);
+    float* red = reinterpret_cast<float*>(smem + Cfg::kRedOffset);
     const int ct = static_cast<int>(threadIdx.x) - 192;
     for (long long u = pair; u < units; u += num_pairs) {
       int sample, tm, tn;

@@ -64,3 +64,14 @@ def test_a_type_is_defined_once():
 def test_every_header_makes_the_library_stale():
     from ghostsuite_b200 import build
     assert {n for n in _sources() if n.endswith(".cuh")} <= set(build.HEADERS)
+
+
+def test_alignment_slack_of_the_shared_memory_is_not_used():
+    """Dynamic shared memory is asked for with 1024 bytes to spare, by which its start is rounded up: no piece
+    may be placed as if the start were aligned already."""
+    placed = 0
+    for name, text in _sources().items():
+        for m in re.finditer(r"\bsmem \+ [^;,]*", text):
+            placed += 1
+            assert "1024" not in m.group(0), f"{name}: {m.group(0)}"
+    assert placed > 20
