@@ -18,12 +18,15 @@ namespace gb {
 void set_error(const char* fmt, ...);
 int fail(int code, const char* fmt, ...);
 
+// The status goes to the caller and not also to whoever asks the runtime for its last error next
 #define GB_CUDA_OK(expr)                                                                   \
   do {                                                                                     \
     cudaError_t _e = (expr);                                                               \
-    if (_e != cudaSuccess)                                                                 \
+    if (_e != cudaSuccess) {                                                               \
+      (void)cudaGetLastError();                                                            \
       return ::gb::fail(GHOST_ERR_CUDA, "%s failed: %s (%s:%d)", #expr,                    \
                         cudaGetErrorString(_e), __FILE__, __LINE__);                       \
+    }                                                                                      \
   } while (0)
 
 #define GB_REQUIRE(cond, ...)                                                              \
@@ -42,7 +45,11 @@ int post_launch(const char* what);  // cudaGetLastError -> status
 // against 79).
 inline int early_start(cudaLaunchAttribute* attr, cudaStream_t st) {
   cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(st, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone) return 0;
+  if (cudaStreamIsCapturing(st, &capturing) != cudaSuccess) {
+    (void)cudaGetLastError();            // the launch itself says what is wrong, if anything is
+    return 0;
+  }
+  if (capturing != cudaStreamCaptureStatusNone) return 0;
   attr->id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr->val.programmaticStreamSerializationAllowed = 1;
   return 1;

@@ -88,3 +88,36 @@ def test_binding_of_another_torch_is_stale(tmp_path, monkeypatch):
     other.write_bytes(other.read_bytes().replace(b"built for torch " + torch.__version__.encode(), b"built for torch 0"))
     monkeypatch.setattr(build, "BINDING", str(other))
     assert build._binding_stale() and not _lib.binding_built_for(torch.__version__, str(other))
+
+
+_FAKE_RUNTIME = r"""
+#include "common.cuh"
+namespace gb { int fail(int code, const char*, ...) { return code; } }
+static cudaError_t last = cudaSuccess, query = cudaSuccess;      // the runtime's last error; what the query answers
+extern "C" {
+cudaError_t cudaStreamIsCapturing(cudaStream_t, cudaStreamCaptureStatus* s) { *s = cudaStreamCaptureStatusNone; return last = query; }
+cudaError_t cudaGetLastError(void) { cudaError_t e = last; last = cudaSuccess; return e; }
+const char* cudaGetErrorString(cudaError_t) { return ""; }
+}
+static int refused_launch() { GB_CUDA_OK(last = cudaErrorInvalidConfiguration); return GHOST_OK; }
+int main() {
+  cudaLaunchAttribute a;
+  if (gb::early_start(&a, nullptr) != 1 || last != cudaSuccess) return 1;
+  query = cudaErrorStreamCaptureImplicit;
+  if (gb::early_start(&a, nullptr) != 0 || last != cudaSuccess) return 2;
+  if (refused_launch() != GHOST_ERR_CUDA || last != cudaSuccess) return 3;
+  return 0;
+}
+"""
+
+
+def test_failed_runtime_calls_leave_no_error_for_the_next_caller(tmp_path):
+    """A status that is returned, or dropped, is taken out of the runtime's last error too: the next launch check
+    of any library would report it again.  The runtime is a fake here."""
+    import subprocess
+    from ghostsuite_b200 import build
+    cuda = os.path.dirname(os.path.dirname(build._nvcc()))
+    src, exe = tmp_path / "fake.cpp", tmp_path / "fake"
+    src.write_text(_FAKE_RUNTIME)
+    subprocess.run(["g++", "-std=c++17", f"-I{cuda}/include", f"-I{build.CSRC}", str(src), "-o", str(exe)], check=True)
+    assert subprocess.run([str(exe)]).returncode == 0
