@@ -429,15 +429,16 @@ static int dispatch_similarity(const SimParams& p, bool vec, const DeviceState* 
   constexpr double kSplitCost = sizeof(PT) == 4 ? 3.5 : 0.5, kProducts = sizeof(PT) == 4 ? 48. : 16.;
   struct Shape { int mt, nt, wm, wn; };
   static constexpr Shape shapes[] = {{1, 1, 1, 1}, {1, 2, 1, 1}, {1, 4, 1, 2}, {2, 4, 1, 1}, {2, 4, 1, 2}, {2, 2, 2, 1}, {2, 4, 2, 2}};
-  int best = 0;
+  int best = -1;
   double least = 0.;
   for (int i = 0; i < 7; ++i) {
     const Shape& s = shapes[i];
     const double bi = ceil_div(p.n1, 16 * s.mt * s.wm), bj = ceil_div(p.n2, 8 * s.nt * s.wn);
+    if (bi > 65535 || bj > 65535) continue;                  // no grid of such blocks
     const double arrive = (bj * p.n1 + bi * p.n2) * 32. * sizeof(PT) / 24.;
     const double work = bi * bj * s.wm * s.wn * (kSplitCost * (16 * s.mt + 8 * s.nt) + kProducts * s.mt * s.nt) * 1.3 / 4.;
     const double cost = arrive > work ? arrive : work;
-    if (i == 0 || cost < least) { least = cost; best = i; }
+    if (best < 0 || cost < least) { least = cost; best = i; }
   }
   switch (best) {
     case 0: return launch_similarity<PT, 1, 1, 1, 1>(p, vec, ds, st);

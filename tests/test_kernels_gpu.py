@@ -1230,3 +1230,17 @@ def test_kernels_that_start_early_see_what_the_kernel_ahead_wrote(n_t, n_v, T, F
         del early, x
     torch.cuda.synchronize()
     _lib.poll_kernel_error()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("n1,n2", [(32 * 65535 + 1, 17), (32 * 65535 + 1, 33), (17, 32 * 65535 + 1)])
+def test_similarity_of_more_rows_than_a_grid_has_small_blocks(n1, n2, dtype):
+    """The block shape that costs least has no grid for these rows: the next one takes them."""
+    d = 8
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    P1 = torch.randn((n1, d), generator=gen, device="cuda").to(dtype)
+    P2 = torch.randn((n2, d), generator=gen, device="cuda").to(dtype)
+    got = ops().projection_similarity(P1, P2)
+    after()
+    # eight products of 16-bit parts and eight additions in float32
+    assert O.rel_fro(got.cpu(), (P1.double() @ P2.double().t()).cpu()) < 3e-5
