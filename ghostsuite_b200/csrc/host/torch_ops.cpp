@@ -609,14 +609,12 @@ PyObject* py_gradproj_dense(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const Tensor &G0 = cuda_tensor(a[0]), &A0 = cuda_tensor(a[1]), &P_r = cuda_tensor(a[2]), &P_c = cuda_tensor(a[3]);
     const Tensor& out = cuda_tensor(a[7]);
     Launch L(G0);
-    Tensor G = as3d(G0), A = as3d(A0);
+    const Tensor G = as3d(G0), A = as3d(A0);
     const long long B = G.size(0), T = G.size(1), k_r = integer(a[4]), k_c = integer(a[5]);
     if (A.size(0) != B || A.size(1) != T)
       throw GhostError(kNotCuda, "Batch size mismatch between activations and output gradients");
     check_projection_out(out, B, k_r * k_c, "gradproj");
     const bool split = is_f32(G) || is_f32(A);
-    if (split && !is_f32(G)) G = G.to(at::kFloat);
-    if (split && !is_f32(A)) A = A.to(at::kFloat);
     const long long n_r = G.size(2), n_c = A.size(2), cp_r = pad8(n_r), cp_c = pad8(n_c);
     if (P_r.size(1) != (split ? 3 : 1) * cp_r || P_c.size(1) != (split ? 3 : 1) * cp_c)
       invalid("projection matrices were prepared for a different dtype/feature size");
@@ -625,7 +623,8 @@ PyObject* py_gradproj_dense(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const bool copies = !split && (!tma_ready(G) || !tma_ready(A)) && B * T * (n_r + n_c) > (1 << 20);
     if (k_r <= 64 && k_c <= 64 && !copies) {
       // the prepared split lays a float32 matrix out as (hi, hi, lo): the residual part starts at 2 * cp
-      check(ghost_gradproj_dense(G.data_ptr(), A.data_ptr(), split ? 1 : 0, static_cast<int>(B), T, static_cast<int>(n_r),
+      const int f32 = !split ? 0 : !is_f32(A) ? 2 : !is_f32(G) ? 3 : 1;
+      check(ghost_gradproj_dense(G.data_ptr(), A.data_ptr(), f32, static_cast<int>(B), T, static_cast<int>(n_r),
                                  static_cast<int>(n_c), n_r, n_c, P_r.data_ptr(), P_c.data_ptr(), static_cast<int>(k_r),
                                  static_cast<int>(k_c), P_r.size(1), P_c.size(1), split ? static_cast<int>(2 * cp_r) : 0,
                                  split ? static_cast<int>(2 * cp_c) : 0, real(a[6]), out.data_ptr<float>(), out.stride(0), L.st()));
@@ -637,12 +636,13 @@ PyObject* py_gradproj_dense(PyObject*, PyObject* const* a, Py_ssize_t n) {
       const void* at[2];
       for (int i = 0; i < 2; ++i) {
         len[i] = (split ? 3 : 1) * cp[i];
-        if (!tma_ready(*x[i])) off[i] = ws.plan(B * T * len[i] * 2);
+        if (split || !tma_ready(*x[i])) off[i] = ws.plan(B * T * len[i] * 2);
       }
       char* base = ws.commit(L, G);
       for (int i = 0; i < 2; ++i) {
-        at[i] = tma_ready(*x[i]) ? x[i]->data_ptr() : base + off[i];
-        if (!tma_ready(*x[i])) Operand(*x[i]).cast(0, B, base + off[i], len[i], cp[i], split ? 3 : 1, kSplitLeft, kSideBySide, L.st());
+        const bool copy = split || !tma_ready(*x[i]);
+        at[i] = copy ? base + off[i] : x[i]->data_ptr();
+        if (copy) Operand(*x[i]).cast(0, B, base + off[i], len[i], cp[i], split ? 3 : 1, kSplitLeft, kSideBySide, L.st());
       }
       check(ghost_gradproj_dense_bf16(at[0], at[1], static_cast<int>(B), T, static_cast<int>(len[0]), static_cast<int>(len[1]), len[0],
                                       len[1], P_r.data_ptr(), P_c.data_ptr(), static_cast<int>(k_r), static_cast<int>(k_c),

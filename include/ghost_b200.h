@@ -348,7 +348,8 @@ int ghost_gradproj_dense_bf16(const void* G, const void* A, int B, long long T, 
                               long long ldg, long long lda, const void* P_r, const void* P_c, int k_r,
                               int k_c, long long ldpr, long long ldpc, float scale, float* out,
                               long long out_stride, void* stream);
-/* The same for operands of any alignment and pitch, bf16 or (is_f32) fp32, without copies of them.  P_r and P_c: bf16
+/* The same for operands of any alignment and pitch, bf16 (is_f32 = 0), fp32 (1), or fp32 G with bf16 A (2) and the
+ * other way round (3), without copies of them.  P_r and P_c: bf16
  * rows of whole pitches, for fp32 operands bf16(P) in columns [0, n) and the residual P - bf16(P) in columns
  * [lo, lo + n), finite values elsewhere (ghost_cast_split_bf16 with parts side by side leaves hi, hi, lo: lo = 2 cpad);
  * for bf16 operands zero beyond column n.  Ranks up to 64. */

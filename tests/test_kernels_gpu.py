@@ -1244,3 +1244,26 @@ def test_similarity_of_more_rows_than_a_grid_has_small_blocks(n1, n2, dtype):
     after()
     # eight products of 16-bit parts and eight additions in float32
     assert O.rel_fro(got.cpu(), (P1.double() @ P2.double().t()).cpu()) < 3e-5
+
+
+@pytest.mark.parametrize("f32", ["G", "A"])
+@pytest.mark.parametrize("case", [(2, 1, 7, 5, 1, 1), (4, 130, 72, 200, 32, 32), (2, 129, 333, 1001, 16, 17), (1, 300, 512, 2944, 44, 44),
+                                  (3, 40, 130, 71, 70, 9)])
+def test_gradproj_dense_of_mixed_operands(case, f32):
+    """One operand float32, the other bf16, on vector boundaries and off them, shared units and whole ones, ranks beyond the
+    loaders': the bf16 operand counts as the values it holds, and no copy of it in float32 is made."""
+    B, T, n_i, n_o, k_i, k_o = case
+    A, G = make(B, T, n_i, n_o, torch.float32, seed=29)
+    G, A = (G, A.bfloat16()) if f32 == "G" else (G.bfloat16(), A)
+    g = torch.Generator().manual_seed(30)
+    P_i, P_o = torch.randn(k_i, n_i, generator=g) / k_i ** 0.5, torch.randn(k_o, n_o, generator=g) / k_o ** 0.5
+    o = ops()
+    Pr, Pc = o.prepare_projection(P_o.cuda(), True), o.prepare_projection(P_i.cuda(), True)
+    out, Gd, Ad = torch.empty((B, k_o * k_i), device="cuda"), G.cuda(), A.cuda()
+    o.gradproj_dense(Gd, Ad, Pr, Pc, k_o, k_i, 1.0, out)
+    after()
+    ref = O.gradproj_dense(A.double(), G.double(), P_i, P_o, compute_dtype=torch.float64) / B
+    assert O.rel_fro(out.reshape(B, k_o, k_i), ref) < 1e-4
+    made = torch.cuda.memory_stats()["allocation.all.allocated"]
+    o.gradproj_dense(Gd, Ad, Pr, Pc, k_o, k_i, 1.0, out)
+    assert torch.cuda.memory_stats()["allocation.all.allocated"] == made      # workspaces are kept from the first call
