@@ -50,19 +50,20 @@ struct CastParams {
   int parts;
   int kind[3];
   int row_stack;            // 0: parts side by side; 1: parts stacked along rows within a sample
+  unsigned blocks;          // of the launch
 };
+struct CastPair { CastParams job[2]; };
 
 // Bound by HBM once the index arithmetic is in 32 bits (I: unsigned wherever the element groups and rows fit)
 // and hi and lo parts are made once an element: 64-bit divisions were most of its instructions (both
 // operands of 29 samples of 197 x (768, 1000) float32: 18.8 us before, 14.4 now).
 template <typename T, typename I>
-__global__ void cast_split_kernel(const CastParams p) {
-  stream_order();
+__device__ __forceinline__ void cast_rows(const CastParams& p, unsigned block) {
   const I cvec = static_cast<I>(p.cpad / 8);
   const I total = static_cast<I>(p.samples * p.T) * cvec;
   const bool stacked = p.row_stack && p.parts > 1;
   const long long stride = stacked ? p.T * p.ld_dst : p.cpad;
-  for (I i = blockIdx.x * static_cast<I>(blockDim.x) + threadIdx.x; i < total; i += gridDim.x * static_cast<I>(blockDim.x)) {
+  for (I i = block * static_cast<I>(blockDim.x) + threadIdx.x; i < total; i += p.blocks * static_cast<I>(blockDim.x)) {
     const I row = i / cvec;
     const int c0 = static_cast<int>(i - row * cvec) * 8;
     float x[8];
@@ -93,9 +94,23 @@ __global__ void cast_split_kernel(const CastParams p) {
     }
   }
 }
+template <typename T, typename I>
+__global__ void cast_split_kernel(const CastParams p) {
+  stream_order();
+  cast_rows<T, I>(p, blockIdx.x);
+}
+// bf16 rows of two operands, padded, in one launch.  A warp takes 256 neighbouring columns: the panels of split_pair_kernel
+// below, two rows of 128 to a warp, touch more lines a load where rows lie off 16-byte boundaries (15 x 1220 tokens
+// of 64 -> 13119, a hook: 506 us with them, 445 so; 171 x 1984 of 64 -> 133 125 and 105).
+template <typename I>
+__global__ void cast_pair_kernel(const CastPair p) {
+  stream_order();
+  const bool second = blockIdx.x >= p.job[0].blocks;
+  cast_rows<__nv_bfloat16, I>(p.job[second ? 1 : 0], blockIdx.x - (second ? p.job[0].blocks : 0u));
+}
 
 // Both operands of a token-contracted GEMM in one launch: rows zero-padded to ld (a multiple of 64) columns, as the
-// values alone (PARTS = 1) or as values and residuals, [samples, 2, T, ld] or [2, samples * T, ld].  A block takes a panel of 128 columns of
+// values alone (PARTS = 1; bf16 rows whose sums are not asked for go through cast_pair_kernel) or as values and residuals, [samples, 2, T, ld] or [2, samples * T, ld].  A block takes a panel of 128 columns of
 // some rows, a thread eight columns of every 16th row, two rows in flight.  Where the column sums of an operand are
 // wanted the rows are one sample's (or a chunk of it, added with atomics), and they cost no second pass over it.
 // Bound by HBM and, on small layers, by the round trip of one round of loads: 8 x 2048 rows of (1024, 2048) float32 at
@@ -651,6 +666,15 @@ layernorm_persample_generic_kernel(const T* __restrict__ A, const T* __restrict_
 
 using namespace gb;
 
+static unsigned cast_blocks(long long octets, const DeviceState* ds) {
+  const long long blocks = (octets + 255) / 256, most = ds->sm_count * 16;
+  return static_cast<unsigned>(blocks < most ? blocks : most);
+}
+// element groups and rows fit 32 bits, a grid stride further too
+static bool cast_narrow(const CastParams& p) {
+  return p.samples * p.T * (p.cpad / 8) < (1ll << 31) && p.samples * p.T < (1ll << 31);
+}
+
 extern "C" int ghost_cast_split_bf16(const void* src, int src_is_f32, long long samples, long long T,
                                      int cols, long long ld_src, void* dst, long long ld_dst, int cpad,
                                      int parts, int kind0, int kind1, int kind2, int row_stack,
@@ -664,24 +688,11 @@ extern "C" int ghost_cast_split_bf16(const void* src, int src_is_f32, long long 
   GB_REQUIRE(ld_dst % 8 == 0 && ld_dst >= (row_stack ? cpad : parts * cpad), "ghost_cast_split_bf16: bad destination pitch");
   GB_REQUIRE((reinterpret_cast<uintptr_t>(dst) & 15u) == 0,
              "ghost_cast_split_bf16: destination must be 16-byte aligned");
-  CastParams p;
-  p.src = src;
-  p.dst = static_cast<__nv_bfloat16*>(dst);
-  p.samples = samples;
-  p.T = T;
-  p.cols = cols;
-  p.cpad = cpad;
-  p.ld_src = ld_src;
-  p.ld_dst = ld_dst;
-  p.parts = parts;
-  p.kind[0] = kind0; p.kind[1] = kind1; p.kind[2] = kind2;
-  p.row_stack = row_stack;
-  const long long total = samples * T * (cpad / 8);
-  long long blocks = (total + 255) / 256;
-  if (blocks > ds->sm_count * 16) blocks = ds->sm_count * 16;
+  const CastParams p = {src, static_cast<__nv_bfloat16*>(dst), samples, T, cols, cpad, ld_src, ld_dst, parts, {kind0, kind1, kind2},
+                        row_stack, cast_blocks(samples * T * (cpad / 8), ds)};
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const int grid = static_cast<int>(blocks);
-  if (total < (1ll << 31) && samples * T < (1ll << 31)) {      // a grid stride further still fits 32 bits
+  const unsigned grid = p.blocks;
+  if (cast_narrow(p)) {
     if (src_is_f32) GB_CUDA_OK(launch_next(cast_split_kernel<float, unsigned>, dim3(grid), dim3(256), 0, st, p));
     else GB_CUDA_OK(launch_next(cast_split_kernel<__nv_bfloat16, unsigned>, dim3(grid), dim3(256), 0, st, p));
   } else {
@@ -713,6 +724,22 @@ extern "C" int ghost_split_operands(const void* X, int x_is_f32, int x_cols, con
   GB_REQUIRE(((reinterpret_cast<uintptr_t>(X_out) | reinterpret_cast<uintptr_t>(Y_out)) & 15u) == 0,
              "ghost_split_operands: destinations must be 16-byte aligned");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (parts == 1 && !x_sums && !y_sums && !(X && x_is_f32) && !(Y && y_is_f32)) {
+    CastPair pair = {};
+    auto copy = [&](CastParams& q, const void* src, int cols, void* dst) {
+      if (!src) return;
+      const int cpad = (cols + 63) / 64 * 64;
+      q = CastParams{src, static_cast<__nv_bfloat16*>(dst), samples, T, cols, cpad, cols, cpad, 1, {0, 0, 0}, 1,
+                     cast_blocks(samples * T * (cpad / 8), ds)};
+    };
+    copy(pair.job[0], X, x_cols, X_out);
+    copy(pair.job[1], Y, y_cols, Y_out);
+    const dim3 grid(pair.job[0].blocks + pair.job[1].blocks);
+    if (cast_narrow(pair.job[0]) && cast_narrow(pair.job[1])) GB_CUDA_OK(launch_next(cast_pair_kernel<unsigned>, grid, dim3(256), 0, st, pair));
+    else GB_CUDA_OK(launch_next(cast_pair_kernel<long long>, grid, dim3(256), 0, st, pair));
+    count_launch();
+    return post_launch("cast_pair_kernel");
+  }
   SplitParams p = {};
   p.T = T;
   p.part_rows = merged ? samples * T : T;
