@@ -27,53 +27,87 @@ struct SimParams {
   int* err;
 };
 
-// The end of a block, from its warps' partial sums part[WK][BM * BN] in shared memory.  The CTAs of a cluster (grid.x) add their
-// blocks up through distributed shared memory before one of them touches the scores: with an addition per CTA and score
-// the 1.2 million atomics of a 64 x 64 block over 296 CTAs were a quarter of a 20 us call.  A contraction that one cluster
-// covers is stored without a zeroed result.
-template <int WK, int BM, int BN, int THREADS>
+// The end of a block, from its warps' partial sums part[WK][BM * BN] in shared memory: added to zeroed scores, or stored where no
+// other CTA has a share.  kCluster: the CTAs of a cluster (grid.x) cover the contraction and add their blocks up through distributed
+// shared memory first.  A form of its own: with the cluster's code in the other one its main loops came out slower as well (37 x 43
+// unaligned rows of 927511 float32: 142 us, 132 without).
+//
+// A thread takes four neighbouring scores of a row where rows of S start on 16-byte boundaries, else one, so that a warp's additions
+// cover neighbouring scores either way (four there as well: 4 x 59 rows of 522904 float32 38 us, 31 one by one).
+template <int WK, int BM, int BN, int THREADS, bool kCluster>
 __device__ __forceinline__ void sim_finish(float* part, const SimParams& p) {
-  static_assert(BM * BN % 4 == 0 && BN % 4 == 0, "four scores a thread");
+  static_assert(BN % 4 == 0, "four scores a thread");
   __syncthreads();
-  for (int e = threadIdx.x; e < BM * BN; e += THREADS) {
-    float v = 0.f;
+  const int rows = p.n1 - static_cast<int>(blockIdx.y) * BM, cols = p.n2 - static_cast<int>(blockIdx.z) * BN;      // of this block
+  auto at = [&](int e) {
+    return p.S + static_cast<long long>(static_cast<int>(blockIdx.y) * BM + e / BN) * p.ld_s + static_cast<int>(blockIdx.z) * BN + e % BN;
+  };
+  auto out4 = [&](int e, float4 v) {
+    v.x *= p.scale; v.y *= p.scale; v.z *= p.scale; v.w *= p.scale;
+    if (p.direct) *reinterpret_cast<float4*>(at(e)) = v;
+    else asm volatile("red.global.v4.f32.add [%0], {%1, %2, %3, %4};" ::"l"(at(e)), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
+  };
+  auto out1 = [&](int e, float v) {
+    if (p.direct) *at(e) = p.scale * v;
+    else atomicAdd(at(e), p.scale * v);
+  };
+  auto inside = [&](int e) { return e / BN < rows && e % BN < cols; };
+  if constexpr (kCluster) {
+    for (int e = threadIdx.x; e < BM * BN; e += THREADS) {
+      float v = 0.f;
 #pragma unroll
-    for (int w = 0; w < WK; ++w) v += part[w * (BM * BN) + e];
-    part[e] = v;
-  }
-  cg::cluster_group cluster = cg::this_cluster();
-  const int ranks = static_cast<int>(cluster.num_blocks()), rank = static_cast<int>(cluster.block_rank());
-  cluster.sync();
-  // four neighbouring scores of a row a thread, dealt to the CTAs of the cluster
-  for (int q = rank * THREADS + static_cast<int>(threadIdx.x); q < BM * BN / 4; q += ranks * THREADS) {
-    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 4
-    for (int r = 0; r < ranks; ++r) {
-      const float4 x = *reinterpret_cast<const float4*>(cluster.map_shared_rank(&part[4 * q], r));
-      v.x += x.x; v.y += x.y; v.z += x.z; v.w += x.w;
+      for (int w = 0; w < WK; ++w) v += part[w * (BM * BN) + e];
+      part[e] = v;
     }
-    const int i = static_cast<int>(blockIdx.y) * BM + 4 * q / BN, j = static_cast<int>(blockIdx.z) * BN + 4 * q % BN;
-    if (i >= p.n1) continue;
-    float* dst = p.S + static_cast<long long>(i) * p.ld_s + j;
-    const float out[4] = {p.scale * v.x, p.scale * v.y, p.scale * v.z, p.scale * v.w};
-    if (p.vec_s && j + 4 <= p.n2) {
-      if (p.direct) *reinterpret_cast<float4*>(dst) = make_float4(out[0], out[1], out[2], out[3]);
-      else
-        asm volatile("red.global.v4.f32.add [%0], {%1, %2, %3, %4};" ::"l"(dst), "f"(out[0]), "f"(out[1]), "f"(out[2]), "f"(out[3])
-                     : "memory");
+    cg::cluster_group cluster = cg::this_cluster();
+    const int ranks = static_cast<int>(cluster.num_blocks()), rank = static_cast<int>(cluster.block_rank());
+    cluster.sync();
+    if (p.vec_s) {
+      for (int e = 4 * (rank * THREADS + static_cast<int>(threadIdx.x)); e < BM * BN; e += 4 * ranks * THREADS) {
+        if (!inside(e)) continue;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+        for (int r = 0; r < ranks; ++r) {
+          const float4 x = *reinterpret_cast<const float4*>(cluster.map_shared_rank(&part[e], r));
+          v.x += x.x; v.y += x.y; v.z += x.z; v.w += x.w;
+        }
+        out4(e, v);
+      }
     } else {
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        if (j + e >= p.n2) continue;
-        if (p.direct) dst[e] = out[e];
-        else atomicAdd(dst + e, out[e]);
+      for (int e = rank * THREADS + static_cast<int>(threadIdx.x); e < BM * BN; e += ranks * THREADS) {
+        if (!inside(e)) continue;
+        float v = 0.f;
+#pragma unroll 4
+        for (int r = 0; r < ranks; ++r) v += *cluster.map_shared_rank(&part[e], r);
+        out1(e, v);
       }
     }
+    cluster.sync();          // no CTA leaves while another reads its block
+  } else if (p.vec_s) {
+    for (int e = 4 * static_cast<int>(threadIdx.x); e < BM * BN; e += 4 * THREADS) {
+      if (!inside(e)) continue;
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int w = 0; w < WK; ++w) {
+        const float4 x = *reinterpret_cast<const float4*>(&part[w * (BM * BN) + e]);
+        v.x += x.x; v.y += x.y; v.z += x.z; v.w += x.w;
+      }
+      out4(e, v);
+    }
+  } else {
+    for (int e = threadIdx.x; e < BM * BN; e += THREADS) {
+      if (!inside(e)) continue;
+      float v = 0.f;
+#pragma unroll
+      for (int w = 0; w < WK; ++w) v += part[w * (BM * BN) + e];
+      out1(e, v);
+    }
   }
-  cluster.sync();            // no CTA leaves while another reads its block
 }
 
-// Eight consecutive contraction elements of one row: hi parts, and lo parts for float rows
+// Eight consecutive contraction elements of one row: hi parts, and lo parts for float rows.  Elements one by one (not VEC) go
+// through the read-only path, which leaves their order to the compiler (97 x 127 rows of 814571 float32: 870 us with ordinary loads, 718
+// so): that form is not launched early, and nobody writes its rows while it lives.
 template <typename PT, bool VEC> struct SimOct {
   float v[sizeof(PT) == 4 ? 8 : 1];
   uint4 raw;
@@ -86,7 +120,7 @@ template <typename PT, bool VEC> struct SimOct {
         *reinterpret_cast<float4*>(&v[4]) = in ? *reinterpret_cast<const float4*>(row + k + 4) : z;
       } else {
 #pragma unroll
-        for (int e = 0; e < 8; ++e) v[e] = ok && k + e < d ? row[k + e] : 0.f;
+        for (int e = 0; e < 8; ++e) v[e] = ok && k + e < d ? __ldg(row + k + e) : 0.f;
       }
     } else {
       if (VEC) {
@@ -117,13 +151,13 @@ template <typename PT, bool VEC> struct SimOct {
 // tile the CTA's block and WK of them split its range, so operand rows are fetched once per block of up
 // to 64 x 64 scores (again from L2 / L1 for the next block and the neighbouring warps) instead of once
 // per 16 x 16.  All loads of a 32-element step go out together.
-template <typename PT, int MT, int NT, int WM, int WN, bool VEC>
+template <typename PT, int MT, int NT, int WM, int WN, bool VEC, bool kCluster>
 __global__ void __launch_bounds__(256, 2) proj_similarity_kernel(const SimParams p) {
   constexpr int WK = 8 / (WM * WN);
   constexpr int BM = 16 * MT * WM, BN = 8 * NT * WN;
   constexpr bool kSplit = sizeof(PT) == 4;
   __shared__ __align__(16) float part[WK * BM * BN];
-  stream_order();
+  if constexpr (VEC) stream_order();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, c = lane & 3;
   const int wk = warp / (WM * WN), wm = warp % (WM * WN) / WN, wn = warp % WN;
@@ -192,7 +226,7 @@ __global__ void __launch_bounds__(256, 2) proj_similarity_kernel(const SimParams
 #pragma unroll
       for (int e = 0; e < 4; ++e)
         part[wk * (BM * BN) + (wm * 16 * MT + 16 * m + g + 8 * (e >> 1)) * BN + wn * 8 * NT + 8 * n + 2 * c + (e & 1)] = acc[m][n][e];
-  sim_finish<WK, BM, BN, 256>(part, p);
+  sim_finish<WK, BM, BN, 256, kCluster>(part, p);
 }
 
 // A stage holds PANELS panels of 128 bytes of columns of all rows of a block, each an [BM][128 bytes] and a [BN][128 bytes]
@@ -233,8 +267,7 @@ __device__ __forceinline__ void sim_parts(const uint8_t* row, int r, int c, int 
 }
 
 // The same for rows that TMA can read, once there are many bytes of them: eight warps work on stages that a ninth keeps coming,
-// 200 KB of them on their way per SM, where the kernel above has what its registers hold in flight.  64 x 64 rows of 98304 float32:
-// 24.2 us with fragments from global memory and an atomic per CTA and score, 18.8 here; of 2^20 bf16 75 and 59.
+// 200 KB of them on their way per SM, where the kernel above has what its registers hold in flight (times of both: dispatch_similarity).
 template <typename PT, int MT, int NT, int WM, int WN>
 __global__ void __launch_bounds__(288, 1)
 proj_similarity_tma_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b, const SimParams p) {
@@ -345,39 +378,76 @@ proj_similarity_tma_kernel(const __grid_constant__ CUtensorMap tm_a, const __gri
         for (int e = 0; e < 4; ++e)
           part[wk * (BM * BN) + (wm * 16 * MT + 16 * m + g + 8 * (e >> 1)) * BN + wn * 8 * NT + 8 * n + 2 * c + (e & 1)] = acc[m][n][e];
   }
-  sim_finish<WK, BM, BN, Cfg::kThreads>(part, p);
+  sim_finish<WK, BM, BN, Cfg::kThreads, false>(part, p);
 }
 
-// Grid and cluster of a call: `most` is the largest number of splits worth making of the contraction
-struct SimGrid { long long splits; int ranks; };
-static SimGrid sim_grid(SimParams& p, int bi, int bj, long long slots, long long most, long long units) {
-  long long splits = slots / (static_cast<long long>(bi) * bj);
-  if (splits > most) splits = most;
-  if (splits < 1) splits = 1;
-  // Up to eight splits are one cluster.  Beyond that two to a cluster: GPCs have 18 or 20 SMs, which larger ones do not fill,
-  // and the clusters left over take a second round (64 x 64 x 2^20 float32, clusters of four: 222 us, 132 in pairs).
-  int ranks = 1;
-  if (splits <= 8) { while (ranks < splits) ranks *= 2; }
-  else ranks = 2;
-  splits = splits <= 8 ? ranks : splits / ranks * ranks;
-  p.per_cta = (units + splits - 1) / splits;
-  p.direct = splits == ranks;
-  p.vec_s = p.ld_s % 4 == 0 && (reinterpret_cast<uintptr_t>(p.S) & 15u) == 0;
-  return {splits, ranks};
+// Warps and blocks of a form of the kernels (their template arguments)
+struct SimShape {
+  int mt, nt, wm, wn;
+  int bm() const { return 16 * mt * wm; }
+  int bn() const { return 8 * nt * wn; }
+  int wk() const { return 8 / (wm * wn); }
+};
+
+// How a call is spread: `splits` CTAs for each of the bi x bj blocks, in clusters of `ranks`
+struct SimGrid {
+  SimShape shape;
+  long long bi, bj, splits, per_cta;     // per_cta: steps (ring: stages) of the contraction
+  int ranks;
+  bool direct;                           // one cluster covers the contraction: no zeroed result, no additions to it
+  double cost;
+};
+
+// In a cluster up to eight splits are all of them and their sums the scores (5 x 6 rows of 688 float32 6.2 us with a zeroed result,
+// 4.3 without); else each adds to the scores by itself.  More than eight in clusters of two halve those additions, but
+// their barriers cost every small call 2 us (9 x 3 rows of 215550 bf16: 10.3 us, 8.3 without), and larger clusters leave SMs idle.
+static SimGrid sim_grid(const SimParams& p, const SimShape& s, long long slots, long long units, long long least, bool cluster) {
+  SimGrid g = {s, (p.n1 + s.bm() - 1ll) / s.bm(), (p.n2 + s.bn() - 1ll) / s.bn()};
+  const long long blocks = g.bi * g.bj, most = (units + least - 1) / least;
+  g.splits = slots / blocks < most ? slots / blocks : most;
+  if (g.splits < 1) g.splits = 1;
+  g.ranks = 1;
+  if (cluster) {
+    while (g.ranks < g.splits && g.ranks < 8) g.ranks *= 2;
+    g.splits = g.ranks;
+  }
+  g.direct = g.splits == g.ranks;
+  g.per_cta = (units + g.splits - 1) / g.splits;
+  return g;
+}
+
+// What tells the shapes apart, in arbitrary units: rounds of a warp one after the other, each the latency of its loads; what the
+// warps of an SM issue in a round (products of a warp's 16 x 8 blocks, loads, eight for one where rows are off vector boundaries); the
+// rows that arrive, once per block that needs them; additions to a zeroed result.  In the ring the rows arrive beside the
+// work on them.  The constants are fits to all seven shapes at 330 sizes (rows 1 to 128, 256 to 2^20 elements, both types, aligned
+// and not): the shape with the least sum is within 2 % of the best one in the mean.
+static double sim_cost(const SimParams& p, const SimGrid& g, int esize, bool vec, bool ring, int sms) {
+  const SimShape& s = g.shape;
+  const double products = (esize == 4 ? 48. : 16.) * s.mt * s.nt;
+  const double arrive = (static_cast<double>(g.bj) * p.n1 + static_cast<double>(g.bi) * p.n2) * p.D * esize * 1e-6;
+  const double ctas = static_cast<double>(g.bi) * g.bj * g.splits;
+  if (ring) {
+    const double stages = g.per_cta * (ctas > sms ? ctas / sms : 1.), stage = (s.bm() + s.bn()) * 128. * s.wk();
+    const double work = stages * (0.66 + 1.0e-3 * products * (esize == 4 ? 1 : 2) + 2.1e-6 * stage);
+    return work > 0.22 * arrive ? work : 0.22 * arrive;
+  }
+  const double rounds = static_cast<double>((g.per_cta + s.wk() - 1) / s.wk()) * (ctas > 2. * sms ? ctas / (2. * sms) : 1.);
+  const double loads = (16. * s.mt + 8. * s.nt) * (vec ? 4.2e-4 * esize / 16. : 1.0e-2);
+  return (g.direct ? 0. : 0.91) + rounds * (0.26 + (ctas > sms ? 2. : 1.) * (8.7e-4 * products + loads)) + 8.3e-3 * arrive;
 }
 
 template <typename K, typename... A>
-static int sim_launch(K kernel, const SimParams& p, SimGrid g, int bi, int bj, int threads, size_t smem, cudaStream_t st, const A&... args) {
+static int sim_launch(K kernel, bool early, const SimParams& p, const SimGrid& g, int threads, size_t smem, cudaStream_t st, const A&... args) {
   if (!p.direct)
     GB_CUDA_OK(cudaMemset2DAsync(p.S, static_cast<size_t>(p.ld_s) * 4, 0, static_cast<size_t>(p.n2) * 4, static_cast<size_t>(p.n1), st));
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[2];
-  cfg.gridDim = dim3(static_cast<unsigned>(g.splits), static_cast<unsigned>(bi), static_cast<unsigned>(bj));
+  cfg.gridDim = dim3(static_cast<unsigned>(g.splits), static_cast<unsigned>(g.bi), static_cast<unsigned>(g.bj));
   cfg.blockDim = dim3(threads, 1, 1);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cfg.attrs = attr;
-  cfg.numAttrs = early_start(attr, st);
+  cfg.numAttrs = early ? early_start(attr, st) : 0;
   if (g.ranks > 1) {
     cudaLaunchAttribute& cluster = attr[cfg.numAttrs++];
     cluster.id = cudaLaunchAttributeClusterDimension;
@@ -391,13 +461,12 @@ static int sim_launch(K kernel, const SimParams& p, SimGrid g, int bi, int bj, i
 }
 
 template <typename PT, int MT, int NT, int WM, int WN>
-static int launch_similarity(SimParams p, bool vec, const DeviceState* ds, cudaStream_t st) {
+static int launch_similarity(SimParams p, const SimGrid& g, bool vec, bool ring, const DeviceState* ds, cudaStream_t st) {
   using Cfg = SimCfg<PT, MT, NT, WM, WN>;
-  const int bi = ceil_div(p.n1, Cfg::BM), bj = ceil_div(p.n2, Cfg::BN);
-  GB_REQUIRE(bi <= 65535 && bj <= 65535, "ghost_projection_similarity: too many rows");
-  // Below 16 MB a call is launch, ramp and reduction, and the fragments' kernel is ahead (97 x 8 rows of 9104 bf16: 9.5 us in the
-  // ring, 6 there); TMA also wants box coordinates that are ints.
-  if (vec && (static_cast<double>(p.n1) + p.n2) * p.D * sizeof(PT) >= 16e6 && p.D < (1ll << 31) - 4096) {
+  p.per_cta = g.per_cta;
+  p.direct = g.direct;
+  p.vec_s = p.n2 % 4 == 0 && p.ld_s % 4 == 0 && (reinterpret_cast<uintptr_t>(p.S) & 15u) == 0;
+  if (ring) {
     CUtensorMap ta, tb;
     int rc;
     if ((rc = make_tmap_rows(&ta, p.P1, sizeof(PT), p.n1, p.D, p.ld1, Cfg::BM)) != GHOST_OK) return rc;
@@ -408,46 +477,49 @@ static int launch_similarity(SimParams p, bool vec, const DeviceState* ds, cudaS
                                       Cfg::kSmemBytes));
       attr_set[ds->device] = true;
     }
-    // one CTA per SM, two stages each at least
-    const long long stages = (p.D + Cfg::PANELS * Cfg::kPanelCols - 1) / (Cfg::PANELS * Cfg::kPanelCols);
-    const SimGrid g = sim_grid(p, bi, bj, ds->sm_count, (stages + 1) / 2, stages);
-    return sim_launch(proj_similarity_tma_kernel<PT, MT, NT, WM, WN>, p, g, bi, bj, Cfg::kThreads, Cfg::kSmemBytes, st, ta, tb, p);
+    return sim_launch(proj_similarity_tma_kernel<PT, MT, NT, WM, WN>, true, p, g, Cfg::kThreads, Cfg::kSmemBytes, st, ta, tb, p);
   }
-  // one wave of two CTAs per SM, but at least eight steps for each of a CTA's WK warps of a block
-  const long long steps = (p.D + 31) / 32, least = 8 * Cfg::WK;
-  const SimGrid g = sim_grid(p, bi, bj, 2ll * ds->sm_count, (steps + least - 1) / least, steps);
-  if (vec) return sim_launch(proj_similarity_kernel<PT, MT, NT, WM, WN, true>, p, g, bi, bj, 256, 0, st, p);
-  return sim_launch(proj_similarity_kernel<PT, MT, NT, WM, WN, false>, p, g, bi, bj, 256, 0, st, p);
+  if (g.ranks > 1) {
+    if (vec) return sim_launch(proj_similarity_kernel<PT, MT, NT, WM, WN, true, true>, true, p, g, 256, 0, st, p);
+    return sim_launch(proj_similarity_kernel<PT, MT, NT, WM, WN, false, true>, false, p, g, 256, 0, st, p);
+  }
+  if (vec) return sim_launch(proj_similarity_kernel<PT, MT, NT, WM, WN, true, false>, true, p, g, 256, 0, st, p);
+  return sim_launch(proj_similarity_kernel<PT, MT, NT, WM, WN, false, false>, false, p, g, 256, 0, st, p);
 }
 
-// Block shape with the least time per 32-element step over all blocks, in cycles of an SM: what the rows take to arrive
-// (24 bytes a cycle) or the instructions of its warps (three per row and lane to split float32, six or two products
-// per 16 x 8 scores), whichever is more.  One 64 x 64 block for everything beyond 16 rows padded 18 x 74 rows to 64 x 128
-// (710864 floats: 177 us).
+// The ring takes aligned rows once there are 16 MB of them, of bf16 128, and more than 16 on either side (TMA also wants box
+// coordinates that are ints).  Below that a call is launch, ramp and reduction, and with few rows on one side its stages are mostly
+// rows that are not there and its eight warps the bound, where sixteen work on fragments.  In the ring and as fragments, us: float32
+// 32 x 32 rows of 98304 12.5 and 20.5, 128 x 128 48 and 74, 64 x 64 of 2^20 133 and 195, 1 x 98 of 895136 117 and 84; bf16 76 x 59
+// of 418048 47 and 43, 64 x 64 of 2^20 57 and 77.
 template <typename PT>
 static int dispatch_similarity(const SimParams& p, bool vec, const DeviceState* ds, cudaStream_t st) {
-  constexpr double kSplitCost = sizeof(PT) == 4 ? 3.5 : 0.5, kProducts = sizeof(PT) == 4 ? 48. : 16.;
-  struct Shape { int mt, nt, wm, wn; };
-  static constexpr Shape shapes[] = {{1, 1, 1, 1}, {1, 2, 1, 1}, {1, 4, 1, 2}, {2, 4, 1, 1}, {2, 4, 1, 2}, {2, 2, 2, 1}, {2, 4, 2, 2}};
+  static constexpr SimShape shapes[] = {{1, 1, 1, 1}, {1, 2, 1, 1}, {1, 4, 1, 2}, {2, 4, 1, 1}, {2, 4, 1, 2}, {2, 2, 2, 1}, {2, 4, 2, 2}};
+  const bool ring = vec && p.n1 > 16 && p.n2 > 16 && (static_cast<double>(p.n1) + p.n2) * p.D * sizeof(PT) >= (sizeof(PT) == 4 ? 16e6 : 128e6) && p.D < (1ll << 31) - 4096;
   int best = -1;
-  double least = 0.;
-  for (int i = 0; i < 7; ++i) {
-    const Shape& s = shapes[i];
-    const double bi = ceil_div(p.n1, 16 * s.mt * s.wm), bj = ceil_div(p.n2, 8 * s.nt * s.wn);
-    if (bi > 65535 || bj > 65535) continue;                  // no grid of such blocks
-    const double arrive = (bj * p.n1 + bi * p.n2) * 32. * sizeof(PT) / 24.;
-    const double work = bi * bj * s.wm * s.wn * (kSplitCost * (16 * s.mt + 8 * s.nt) + kProducts * s.mt * s.nt) * 1.3 / 4.;
-    const double cost = arrive > work ? arrive : work;
-    if (best < 0 || cost < least) { least = cost; best = i; }
+  SimGrid grid = {};
+  for (int i = 0; i < 14; ++i) {
+    const SimShape& s = shapes[i / 2];
+    const bool cluster = i % 2 == 0;
+    if (ring && cluster) continue;
+    constexpr int kPanelCols = 128 / static_cast<int>(sizeof(PT));
+    // one CTA per SM of two stages at least, or two CTAs of four steps for each of their warps of a block
+    const long long panels = (p.D + kPanelCols - 1) / kPanelCols;
+    SimGrid g = ring ? sim_grid(p, s, ds->sm_count, (panels + s.wk() - 1) / s.wk(), 2, false)
+                     : sim_grid(p, s, 2ll * ds->sm_count, (p.D + 31) / 32, 4 * s.wk(), cluster);
+    if (g.bi > 65535 || g.bj > 65535) continue;              // no grid of such blocks
+    g.cost = sim_cost(p, g, sizeof(PT), vec, ring, ds->sm_count);
+    if (best < 0 || g.cost < grid.cost) { grid = g; best = i / 2; }
   }
   switch (best) {
-    case 0: return launch_similarity<PT, 1, 1, 1, 1>(p, vec, ds, st);
-    case 1: return launch_similarity<PT, 1, 2, 1, 1>(p, vec, ds, st);
-    case 2: return launch_similarity<PT, 1, 4, 1, 2>(p, vec, ds, st);
-    case 3: return launch_similarity<PT, 2, 4, 1, 1>(p, vec, ds, st);
-    case 4: return launch_similarity<PT, 2, 4, 1, 2>(p, vec, ds, st);
-    case 5: return launch_similarity<PT, 2, 2, 2, 1>(p, vec, ds, st);
-    default: return launch_similarity<PT, 2, 4, 2, 2>(p, vec, ds, st);
+    case 0: return launch_similarity<PT, 1, 1, 1, 1>(p, grid, vec, ring, ds, st);
+    case 1: return launch_similarity<PT, 1, 2, 1, 1>(p, grid, vec, ring, ds, st);
+    case 2: return launch_similarity<PT, 1, 4, 1, 2>(p, grid, vec, ring, ds, st);
+    case 3: return launch_similarity<PT, 2, 4, 1, 1>(p, grid, vec, ring, ds, st);
+    case 4: return launch_similarity<PT, 2, 4, 1, 2>(p, grid, vec, ring, ds, st);
+    case 5: return launch_similarity<PT, 2, 2, 2, 1>(p, grid, vec, ring, ds, st);
+    case 6: return launch_similarity<PT, 2, 4, 2, 2>(p, grid, vec, ring, ds, st);
+    default: return fail(GHOST_ERR_INVALID, "ghost_projection_similarity: too many rows");
   }
 }
 

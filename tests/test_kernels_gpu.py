@@ -1267,3 +1267,25 @@ def test_gradproj_dense_of_mixed_operands(case, f32):
     made = torch.cuda.memory_stats()["allocation.all.allocated"]
     o.gradproj_dense(Gd, Ad, Pr, Pc, k_o, k_i, 1.0, out)
     assert torch.cuda.memory_stats()["allocation.all.allocated"] == made      # workspaces are kept from the first call
+
+
+# both sides of what sends rows through the ring (16 MB of float32, 128 of bf16, more than 16 rows on either side); one CTA to a block
+# of scores; eight splits and nine
+@pytest.mark.parametrize("n1,n2,D,dtype", [
+    (16, 17, 131072, torch.float32), (17, 17, 131072, torch.float32), (17, 17, 131073, torch.float32), (1100, 1090, 2048, torch.float32),
+    (64, 66, 491520 + 8, torch.bfloat16), (64, 66, 500000 + 8, torch.bfloat16), (5, 7, 8 * 1024, torch.float32), (5, 7, 9 * 1024, torch.bfloat16)])
+def test_projection_similarity_routes(n1, n2, D, dtype):
+    """Also into rows of a wider matrix: nothing beside the scores is written."""
+    from ghostsuite_b200 import _lib
+    lib, stream = _lib.load(), torch.cuda.current_stream().cuda_stream
+    g = torch.Generator(device="cuda").manual_seed(25)
+    a, b = (torch.randn(n, D, generator=g, device="cuda").to(dtype) for n in (n1, n2))
+    ref = a.double() @ b.double().t()
+    bound = 2.0 ** -15 * a.double().norm(dim=1)[:, None] * b.double().norm(dim=1)[None]
+    for pitch in (n2, (n2 + 7) // 4 * 4):
+        S = torch.full((n1, pitch), 7.0, device="cuda")
+        _lib.check(lib.ghost_projection_similarity(a.data_ptr(), b.data_ptr(), 1 if dtype == torch.float32 else 0, n1, n2, D, D, D,
+                                                   1.0, S.data_ptr(), pitch, stream))
+        after()
+        assert ((S[:, :n2].double() - ref).abs() <= bound).all()
+        assert (S[:, n2:] == 7.0).all()
