@@ -880,26 +880,23 @@ __device__ __forceinline__ void emb_big_rows(const EmbBuckets& q, const T* G, in
   }
 }
 
-// One launch for both: every CTA takes its share of the long rows, whose chains are the longest, and goes on
-// with the short ones.  Apart, a launch of each (text ids, 40 x 1024 tokens of 768 bf16 features) took 46 and
-// 35 us, mostly with a few warps left per SM; 39 us together, 30 of them the longest rows' chains.
-// What bounds it is issue slots and latency, not bandwidth, and the same holds for the join: launched beside
-// this grid's tail (a programmatic launch: it reads nothing written here), both together take 66 us
-// instead of 78.
-// Zeroes the gradient's rows without tokens, 32 ids a warp drawn from a counter.  It runs behind the sums, on the warps that
-// find no more of them: the longest row's sum leaves HBM idle for 30 us, and the counting kernel, which zeroed all
-// rows ahead of everything else, took 13 us for it on a table of 50304 x 768 bf16.
+// Zeroes the gradient's rows without tokens, `each` (up to 32) ids a warp drawn from a counter.  It runs behind the sums, on the warps
+// that find no more of them: the longest row's sum leaves HBM idle for 30 us, and the counting kernel, which zeroed all
+// rows ahead of everything else, took 13 us for it on a table of 50304 x 768 bf16.  A draw is at most kEmbZeroBytes of rows: 32 wide
+// rows of a small table leave most warps without a draw (3 + 7 x 22 text tokens, table of 18455 x 1664 bf16: a hook of 55 us, 39 with
+// four; 9 + 4 x 112 positions, 4096 x 1280 float32: 73 and 40).
+constexpr int kEmbZeroBytes = 24 * 1024;
 template <typename T>
-__device__ void emb_zero_rows(const EmbBuckets& q, int d, T* __restrict__ out) {
+__device__ void emb_zero_rows(const EmbBuckets& q, int d, int each, T* __restrict__ out) {
   const int lane = threadIdx.x & 31;
   const int pieces = static_cast<int>(d * sizeof(T) / 16);
   const uint4 z = make_uint4(0u, 0u, 0u, 0u);
   while (true) {
     int first = 0;
-    if (lane == 0) first = atomicAdd(q.totals + 9, 32);
+    if (lane == 0) first = atomicAdd(q.totals + 9, each);
     first = __shfl_sync(0xffffffffu, first, 0);
     if (first >= q.vocab) break;
-    const bool empty = first + lane < q.vocab && q.cnt_b[first + lane] == 0;
+    const bool empty = lane < each && first + lane < q.vocab && q.cnt_b[first + lane] == 0;
     for (unsigned todo = __ballot_sync(0xffffffffu, empty); todo != 0; todo &= todo - 1) {
       uint4* row = reinterpret_cast<uint4*>(out + static_cast<long long>(first + __ffs(todo) - 1) * d);
       for (int i = lane; i < pieces; i += 32) row[i] = z;
@@ -907,14 +904,20 @@ __device__ void emb_zero_rows(const EmbBuckets& q, int d, T* __restrict__ out) {
   }
 }
 
+// One launch for both: every CTA takes its share of the long rows, whose chains are the longest, and goes on
+// with the short ones.  Apart, a launch of each (text ids, 40 x 1024 tokens of 768 bf16 features) took 46 and
+// 35 us, mostly with a few warps left per SM; 39 us together, 30 of them the longest rows' chains.
+// What bounds it is issue slots and latency, not bandwidth, and the same holds for the join: launched beside
+// this grid's tail (a programmatic launch: it reads nothing written here), both together take 66 us
+// instead of 78.
 template <typename T>
 __global__ void __launch_bounds__(kEmbGradThreads, 6)
 emb_grad_kernel(const EmbBuckets q, const T* G, int d, int slices, float pre_scale, float divisor,
-                int accumulate, int zero_rows, T* __restrict__ out) {
+                int accumulate, int zero_each, T* __restrict__ out) {
   stream_order();                        // from here on the join may start beside this grid's tail
   emb_big_rows<T>(q, G, d, slices, pre_scale, divisor, accumulate, out);
   emb_small_rows<T>(q, G, d, pre_scale, divisor, accumulate, out);
-  if (zero_rows) emb_zero_rows<T>(q, d, out);
+  if (zero_each) emb_zero_rows<T>(q, d, zero_each, out);
 }
 
 static inline long long up256(long long x) { return (x + 255) / 256 * 256; }
@@ -986,9 +989,11 @@ static int emb_pass(const EmbBuckets& q, const T* Gb, const T* Gv, int n_train, 
       const int zb = ceil_div(q.vocab, kEmbGradThreads), all = ds->sm_count * 6;
       if (gb < zb) gb = zb < all ? zb : all;
     }
+    int zero_each = 32;
+    while (zero_each > 4 && zero_each * d * sizeof(T) > kEmbZeroBytes) zero_each /= 2;
     constexpr int kBigRing = kBigSlots * kBigStage * 256;
     GB_CUDA_OK(launch_next(emb_grad_kernel<T>, dim3(gb), dim3(kEmbGradThreads), kBigRing, st, q, Gb, d, slices, pre_scale, divisor,
-                           accumulate, by_rows ? 1 : 0, out));
+                           accumulate, by_rows ? zero_each : 0, out));
     count_launch();
   }
   if (M != nullptr) {

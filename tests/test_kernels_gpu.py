@@ -1289,3 +1289,27 @@ def test_projection_similarity_routes(n1, n2, D, dtype):
         after()
         assert ((S[:, :n2].double() - ref).abs() <= bound).all()
         assert (S[:, n2:] == 7.0).all()
+
+
+# rows of which 32, 16, 8, four and more than a whole draw's bytes are drawn at once; tables of a part of a draw, one and many
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("d", [8, 384, 392, 1544, 6152])
+@pytest.mark.parametrize("vocab", [3, 33, 1025])
+def test_embedding_rows_without_tokens_are_zero(vocab, d, dtype):
+    """Beside rows that have some: their gradient is the tokens' sum, all others are zero whatever the buffer held."""
+    n_t, n_v, T = 3, 1, 5
+    g = torch.Generator(device="cuda").manual_seed(8)
+    ids = torch.randint(0, vocab, (n_t + n_v, T), generator=g, device="cuda")
+    G = torch.randn((n_t + n_v, T, d), generator=g, device="cuda").to(dtype)
+    ref = torch.zeros((vocab, d), dtype=torch.float64, device="cuda")
+    ref.index_add_(0, ids[:n_t].flatten(), G[:n_t].flatten(0, 1).double())
+    for _ in range(2):
+        held = torch.full((vocab, d), float("nan"), device="cuda", dtype=dtype)      # the buffer that the result may get
+        del held
+        grad = ops().embedding_wgrad(ids[:n_t], G[:n_t], n_t, vocab, 1.0, 1.0)
+        after()
+        # up to 15 tokens a row: the sum is float32, rounded once
+        assert ((grad.double() - ref).abs() <= (2.0 ** -7 if dtype == torch.bfloat16 else 2.0 ** -20) * (1 + ref.abs())).all()
+        empty = torch.ones(vocab, dtype=torch.bool, device="cuda")
+        empty[ids[:n_t].flatten()] = False
+        assert (grad[empty] == 0).all()
