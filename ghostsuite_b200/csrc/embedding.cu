@@ -550,7 +550,10 @@ __device__ __noinline__ float4 emb_redo(const VT* V, const BT* B, int2 lv, int m
 // kernel waiting for the longest: 16 + 4 x 512 text tokens of 2048 float32 features, 32 rounds an item, took 229 us with the
 // hook, 168 now (9 + 3 x 333 of 701 67 and 50).  There (CUT) items fall into pieces of a range of features where that shortens
 // the rounds that a warp goes through, a piece's indices and sums counted as kEmbJoinAround of them.  Batches
-// of more train tokens than four a warp have items enough (at 32 x 1024 the arithmetic alone cost 1.2 us of 99).
+// of more train tokens than four a warp have items enough (at 32 x 1024 the arithmetic alone cost 1.2 us of 99).  With one or two
+// validation samples the entries of an item fall on so few scores that their additions wait for each other, and more
+// pieces are more additions; bf16 rows that arrive in whole vectors are back before that (5 + 1 x 515 tokens of 768: 66 us in
+// pieces, 49 whole; 4 + 2 x 512: 62 and 49; but 36 + 1 x 253 of 1472 float32 45 and 66).
 // What it reads (rows, buckets, hot sums) was written before the gradient kernel ahead of it passed its own wait, and so before
 // a block of the join came up: read-only for the join's whole life, unlike in the kernels that wait at their start.
 constexpr int kEmbJoinAround = 2;
@@ -1003,7 +1006,7 @@ static int emb_pass(const EmbBuckets& q, const T* Gb, const T* Gv, int n_train, 
     const int Ti = static_cast<int>(Tn);
     const long long most = (q.max_items + 7) / 8;
     const int jb = static_cast<int>(most < ds->sm_count * 2 ? most : ds->sm_count * 2);
-    const bool cut = q.first_val <= 4ll * 8 * jb;
+    const bool cut = q.first_val <= 4ll * 8 * jb && !(n_val <= 2 && sizeof(T) == 2 && vec);
     const auto join = cut ? vec ? emb_join_kernel<T, true, true> : emb_join_kernel<T, false, true>
                           : vec ? emb_join_kernel<T, true, false> : emb_join_kernel<T, false, false>;
     cudaLaunchAttribute beside = {};
