@@ -1313,3 +1313,110 @@ def test_embedding_rows_without_tokens_are_zero(vocab, d, dtype):
         empty = torch.ones(vocab, dtype=torch.bool, device="cuda")
         empty[ids[:n_t].flatten()] = False
         assert (grad[empty] == 0).all()
+
+
+def _rows(samples, T, cols, ld, seed):
+    """bf16 rows of `cols` columns in rows of `ld`, NaN between them: whoever reads past a row shows it."""
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    x = torch.full((samples, T, ld), float("nan"), device="cuda", dtype=torch.bfloat16)
+    x[..., :cols] = torch.randn((samples, T, cols), generator=g, device="cuda").bfloat16()
+    return x
+
+
+@pytest.mark.parametrize("mode", [0, 1, 2])
+@pytest.mark.parametrize("n_t,n_v,T,ka,kg", [(3, 2, 5, 24, 17), (5, 1, 130, 64, 40), (3, 2, 257, 200, 136)])
+def test_gram_entry_point_on_four_buffers(n_t, n_v, T, ka, kg, mode):
+    """ghost_gram_dot_bf16 as a C caller has it: train and validation rows in buffers of their own, every one with
+    its own pitch, either rounding, each kernel."""
+    from ghostsuite_b200 import _lib
+    lib, stream = _lib.load(), torch.cuda.current_stream().cuda_stream
+    up = lambda n: (n + 7) // 8 * 8
+    ld = (up(ka), up(ka) + 8, up(kg) + 16, up(kg))
+    at, av = _rows(n_t, T, ka, ld[0], 1), _rows(n_v, T, ka, ld[1], 2)
+    gt, gv = _rows(n_t, T, kg, ld[2], 3), _rows(n_v, T, kg, ld[3], 4)
+    a = torch.einsum("btk,vsk->vbst", at[..., :ka].double(), av[..., :ka].double())
+    g = torch.einsum("btk,vsk->vbst", gt[..., :kg].double(), gv[..., :kg].double())
+    try:
+        _lib.check(lib.ghost_set_gram_pair_mode(mode))
+        for rounding in (0, 1):
+            M = torch.full((n_v, n_t), float("nan"), device="cuda")
+            _lib.check(lib.ghost_gram_dot_bf16(at.data_ptr(), av.data_ptr(), gt.data_ptr(), gv.data_ptr(), n_t, n_v, T, ka, kg,
+                                               *ld, rounding, 0.5, M.data_ptr(), stream))
+            after()
+            # products of bf16 values are exact, sums float32; rounded entries carry three roundings of 2^-9
+            assert O.rel_fro(M, 0.5 * (a * g).sum((2, 3))) < (1e-4 if rounding == 0 else 2e-2)
+    finally:
+        _lib.check(lib.ghost_set_gram_pair_mode(1))
+
+
+@pytest.mark.parametrize("mode", [0, 2])
+@pytest.mark.parametrize("rows,m,n", [(7, 24, 17), (300, 256, 320), (5000, 72, 130), (9000, 256, 64)])
+def test_wgrad_entry_point_on_strided_rows(rows, m, n, mode):
+    """ghost_wgrad_bf16 on rows inside wider ones, written and accumulated, in either type, in one split and several."""
+    from ghostsuite_b200 import _lib
+    lib, stream = _lib.load(), torch.cuda.current_stream().cuda_stream
+    ldx, ldy = (m + 7) // 8 * 8 + 8, (n + 7) // 8 * 8 + 24
+    X, Y = _rows(1, rows, m, ldx, 5), _rows(1, rows, n, ldy, 6)
+    ref = 0.25 * X[0, :, :m].double().t() @ Y[0, :, :n].double()
+    size = int(lib.ghost_wgrad_workspace_bytes(m, n))
+    ws = torch.empty(size, dtype=torch.uint8, device="cuda")
+    try:
+        _lib.check(lib.ghost_set_wgrad_pair_mode(mode))
+        for dtype in (torch.float32, torch.bfloat16):
+            for accumulate in (0, 1):
+                out = torch.full((m, n), 2.0 if accumulate else float("nan"), device="cuda", dtype=dtype)
+                _lib.check(lib.ghost_wgrad_bf16(X.data_ptr(), Y.data_ptr(), rows, m, n, ldx, ldy, 0.25, accumulate, out.data_ptr(),
+                                                1 if dtype == torch.float32 else 0, ws.data_ptr(), size, stream))
+                after()
+                assert O.rel_fro(out, ref + 2.0 * accumulate) < (1e-4 if dtype == torch.float32 else 1e-2)
+    finally:
+        _lib.check(lib.ghost_set_wgrad_pair_mode(1))
+
+
+@pytest.mark.parametrize("mode", [0, 2])
+@pytest.mark.parametrize("n_t,n_v,T,m,n", [(3, 2, 5, 24, 17), (5, 9, 70, 256, 320), (33, 1, 9, 72, 130)])
+def test_persample_entry_point_on_strided_rows(n_t, n_v, T, m, n, mode):
+    """ghost_persample_dot_bf16 on rows inside wider ones: bf16 tiles with the column sums of either operand, and
+    float32 tiles of the three stacked parts that ghost_cast_split_bf16 makes of float32 rows."""
+    from ghostsuite_b200 import _lib
+    lib, stream = _lib.load(), torch.cuda.current_stream().cuda_stream
+    N = n_t + n_v
+    ldx, ldy = (m + 7) // 8 * 8 + 8, (n + 7) // 8 * 8 + 16
+
+    def call(X, Y, tokens, ldx, ldy, f32, colsum_of, sums):
+        size = int(lib.ghost_persample_workspace_bytes(n_t, n_v, m, n, f32))
+        ws = torch.empty(size, dtype=torch.uint8, device="cuda")
+        M, grad = torch.full((n_v, n_t), float("nan"), device="cuda"), torch.full((m, n), float("nan"), device="cuda")
+        _lib.check(lib.ghost_persample_dot_bf16(X.data_ptr(), Y.data_ptr(), n_t, n_v, tokens, m, n, ldx, ldy, 2.0, M.data_ptr(), f32,
+                                                grad.data_ptr(), 1, 0.5, 0, colsum_of, sums.data_ptr() if colsum_of else None,
+                                                ws.data_ptr(), size, stream))
+        after()
+        return M, grad
+
+    def reference(x, y):
+        w = torch.einsum("btm,btn->bmn", x.double(), y.double())
+        return 2.0 * torch.einsum("vmn,bmn->vb", w[n_t:], w[:n_t]), 0.5 * w[:n_t].sum(0)
+
+    try:
+        _lib.check(lib.ghost_set_persample_pair_mode(mode))
+        X, Y = _rows(N, T, m, ldx, 7), _rows(N, T, n, ldy, 8)
+        M_ref, grad_ref = reference(X[..., :m], Y[..., :n])
+        for colsum_of in (0, 1, 2):
+            sums = torch.full((N, n if colsum_of == 2 else m), float("nan"), device="cuda")
+            M, grad = call(X, Y, T, ldx, ldy, 0, colsum_of, sums)
+            assert O.rel_fro(M, M_ref) < 2e-2 and O.rel_fro(grad, grad_ref) < 2e-2     # tiles in bf16
+            if colsum_of:
+                assert O.rel_fro(sums, (X[..., :m] if colsum_of == 1 else Y[..., :n]).double().sum(1)) < 1e-5
+        g = torch.Generator(device="cuda").manual_seed(9)
+        x, y = torch.randn((N, T, m), generator=g, device="cuda"), torch.randn((N, T, n), generator=g, device="cuda")
+        stacked = []
+        for src, ld, kinds in ((x, ldx, (0, 1, 0)), (y, ldy, (0, 0, 1))):
+            cols = src.shape[-1]
+            dst = torch.full((N, 3 * T, ld), float("nan"), device="cuda", dtype=torch.bfloat16)
+            _lib.check(lib.ghost_cast_split_bf16(src.data_ptr(), 1, N, T, cols, cols, dst.data_ptr(), ld, (cols + 7) // 8 * 8, 3, *kinds, 1, stream))
+            stacked.append(dst)
+        M_ref, grad_ref = reference(x, y)
+        M, grad = call(*stacked, 3 * T, ldx, ldy, 1, 0, None)
+        assert O.rel_fro(M, M_ref) < 1e-4 and O.rel_fro(grad, grad_ref) < 1e-4
+    finally:
+        _lib.check(lib.ghost_set_persample_pair_mode(1))
