@@ -128,9 +128,6 @@ int make_tmap_bf16_parts(CUtensorMap* out, const void* base, uint64_t samples, u
 int make_tmap_bf16_gathered_tiles(CUtensorMap* out, const void* base, uint64_t ranks, uint64_t tiles,
                                   uint64_t per_rank, uint32_t box_rows, uint32_t box_blocks);
 
-// Plain (unswizzled) 2-D map of a row-major matrix of 2- or 4-byte elements; box = [box_rows, box_cols].
-int make_tmap_plain_2d(CUtensorMap* out, const void* base, int elem_bytes, uint64_t rows, uint64_t cols,
-                       uint64_t ld, uint32_t box_rows, uint32_t box_cols);
 // 2-D map of a dense row-major bf16 matrix for tiled STORES of [box_rows, 32 columns] boxes (64-byte
 // rows) from shared memory written with the 64-byte swizzle: 16-byte chunk c of row r sits at
 // r * 64 + ((c ^ ((r >> 1) & 3)) * 16).

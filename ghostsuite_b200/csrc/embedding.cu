@@ -910,9 +910,8 @@ __device__ void emb_zero_rows(const EmbBuckets& q, int d, int each, T* __restric
 // One launch for both: every CTA takes its share of the long rows, whose chains are the longest, and goes on
 // with the short ones.  Apart, a launch of each (text ids, 40 x 1024 tokens of 768 bf16 features) took 46 and
 // 35 us, mostly with a few warps left per SM; 39 us together, 30 of them the longest rows' chains.
-// What bounds it is issue slots and latency, not bandwidth, and the same holds for the join: launched beside
-// this grid's tail (a programmatic launch: it reads nothing written here), both together take 66 us
-// instead of 78.
+// What bounds it is issue slots and latency, not bandwidth, and the same holds for the join, which is launched beside
+// this grid's tail (a programmatic launch: it reads nothing written here); one after the other they took a fifth longer.
 template <typename T>
 __global__ void __launch_bounds__(kEmbGradThreads, 6)
 emb_grad_kernel(const EmbBuckets q, const T* G, int d, int slices, float pre_scale, float divisor,

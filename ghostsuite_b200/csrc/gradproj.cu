@@ -623,7 +623,7 @@ static int launch_gradproj_t(const CUtensorMap& tg, const CUtensorMap& tpr, cons
   return post_launch("gradproj_kernel");
 }
 
-// CTAs that share a unit: as many as keep the GPU's SMs busy with one unit per cluster.  A GPC has 16 to 20 SMs, so about
+// CTAs that share a unit: as many as keep the GPU's SMs busy with one unit per cluster.  A GPC has 18 or 20 SMs, so about
 // 16 clusters of eight and 34 of four are resident at once.  The cluster's two barriers and the exchange cost about
 // 2 us; a stage is 0.5 us of a unit's chain, and the contraction of 128 tokens, which the CTAs share too, 3 us at
 // 64 x 64 and 1 us at 32 x 32 (32 x 64 tokens of 256 + 256 columns, four stages, k = 32: 10.3 us alone, 11.3 in pairs;

@@ -175,7 +175,6 @@ PyObject* py_arena_clear(PyObject*, PyObject* const*, Py_ssize_t) {
 
 // hi/lo layouts of an fp32 operand pair so that sum_k L[k] R[k] = hi*hi + lo*hi + hi*lo
 constexpr int kSplitLeft[3] = {0, 1, 0};
-constexpr int kPlain[3] = {0, 0, 0};
 enum { kSideBySide = 0 };      // where the parts of a copy lie
 
 // An operand [N, T, cols] of the layer math: a tensor with exactly these dimensions, or a convolution

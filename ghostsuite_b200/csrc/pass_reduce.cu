@@ -249,8 +249,8 @@ pass_reduce_kernel(const __grid_constant__ PassJobs<CAP> jobs) {
 
 // M[v, b] = scale * <X[n_train + v], X[b]> with a warp per pair: for one matrix on its own, whose blocks above
 // are too few to fill the GPU once a pair is long or the validation rows are many (a cluster goes through
-// them eight at a time).  256 x 256 pairs of 768: 93 us in the clusters, 31 here; 256 x 32 of 50257: 473 and 141;
-// 16384 x 1 of 1024: 49 and 19.  Smaller ones, and every matrix of a batch, stay with the clusters, which fetch a row once.
+// them sixteen at a time).  256 x 256 pairs of 768: 47 us in the clusters, 19 here; 256 x 32 of 50257: 308 and 139;
+// 16384 x 1 of 1024: 64 and 11; 256 x 128 of 256 19 and 9.  Smaller ones (64 x 64 of 512: 11.6 in the clusters), and every matrix of a batch, stay with the clusters, which fetch a row once.
 __global__ void __launch_bounds__(256) small_gram_kernel(const float* X, int n_train, unsigned pairs, int F,
                                                          float scale, float* __restrict__ M) {
   stream_order();

@@ -114,8 +114,8 @@ __global__ void cast_pair_kernel(const CastPair p) {
 // some rows, a thread eight columns of every 16th row, two rows in flight.  Where the column sums of an operand are
 // wanted the rows are one sample's (or a chunk of it, added with atomics), and they cost no second pass over it.
 // Bound by HBM and, on small layers, by the round trip of one round of loads: 8 x 2048 rows of (1024, 2048) float32 at
-// 5.5 TB/s, 29 x 197 of (768, 1000) 22.5 us from cold caches (two launches of cast_split_kernel with three parts
-// 17.4, and 8.5 for the sums in a pass of their own).
+// 5.5 TB/s, 29 x 197 of (768, 1000) with their sums 17 us from cold caches, 14 with the operands in L2 (two launches of
+// cast_split_kernel with three parts 17.4, and 8.5 for the sums in a pass of their own).
 static constexpr int kSplitCols = 128, kSplitLanes = 16;       // columns and row lanes of a block
 struct SplitJob {
   const void* src;
@@ -326,7 +326,7 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
 //
 // Bound by issue slots before HBM: 388 instructions a row of 768 bf16 features kept the schedulers 60 % busy at
 // 4.35 TB/s.  So features go in pairs (f32x2), and a width that fills the lanes (FULL: F = 256 NCHUNK) has no tests:
-// 40 x 1024 rows went from 30.1 to 24.2 us (5.2 TB/s).
+// 40 x 1024 rows went from 30.1 to 24.2 us (5.2 TB/s) with a part of them in L2; from cold caches they take 30.4.
 constexpr int kLnSlots = 3;
 
 template <typename T, int NCHUNK, bool FULL>

@@ -70,7 +70,10 @@ def _fp32_path_seconds(n_t: int, n_v: int, T: int, rows: int, cols: int):
     """``(per-sample path, Gram path)``: measured cost of a float32 layer of short samples with a weight of
     ``rows x cols``, train gradient included.  At these sizes the fixed launches, the padding of the tiles and the conversion of
     the operands decide; the rates alone chose the Gram path for 24 + 5 samples of 197 x (768 -> 1000), 176 us a hook
-    against 112 when the costs were taken (the Gram path laid its operands out twice then), and against 83 now.
+    against 112 when the costs were taken.  Both paths are faster since, the Gram path, which lays its operands out once now, by
+    more: 83 us against 100 there, where the model has 109 and 229.  So it still chooses well where the paths differ by
+    their tiles, and keeps the per-sample path too long for many short samples (60 + 7 x 100 x (1024 -> 1024): 179 us
+    against 114; 16 + 16 x 30 x (512 -> 2048): 98 against 70).
 
     Only for ``T <= 256`` and ``2 T <= d + p``: the tensor cores' float32 accumulation leaves a relative error
     of about 1e-8 per contracted token in the per-sample products and 5e-9 per feature in the Grams (70

@@ -570,8 +570,8 @@ def gradproj_embedding(ids: torch.Tensor, G: torch.Tensor, P_o_prepared: torch.T
 
 
 #: largest block (rows of either operand) the similarity kernel is used for.  Beyond it a library GEMM
-#: takes bf16 operands faster (192 x 192 scores over 98304 elements: 28 us against 69) and float32 ones
-#: more accurately (1.1e-6 off the 64-bit result against 4.4e-6; 486 us against 146)
+#: takes bf16 operands faster (192 x 192 scores over 98304 elements: 28 us against 51) and float32 ones
+#: more accurately (rows of both signs: 1.2e-6 off the 64-bit result against 4.4e-6; 494 us against 97)
 SIMILARITY_KERNEL_MAX_ROWS = 128
 
 
