@@ -159,14 +159,15 @@ int make_tmap_f32_store_2d(CUtensorMap* out, const void* base, uint64_t rows, ui
   return make_tmap_store_2d(out, base, 4, rows, cols, box_rows);
 }
 
-int make_tmap_f32_tiles(CUtensorMap* out, const void* base, uint64_t tiles, uint64_t samples, uint32_t box_rows) {
+int make_tmap_f32_tiles(CUtensorMap* out, const void* base, uint64_t tiles, uint64_t samples, uint64_t first, uint32_t box_rows) {
   EncodeTiledFn fn = encode_fn();
   if (!fn) return fail(GHOST_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
   if ((reinterpret_cast<uintptr_t>(base) & 15u) != 0)
     return fail(GHOST_ERR_INVALID, "TMA operand base %p is not 16-byte aligned", base);
-  if (tiles == 0 || samples == 0 || box_rows == 0 || box_rows > 256) return fail(GHOST_ERR_INVALID, "bad fp32 tile map");
+  if (tiles == 0 || first == 0 || first > samples || box_rows == 0 || box_rows > 256)
+    return fail(GHOST_ERR_INVALID, "bad fp32 tile map");
   const uint64_t tile_bytes = 32768ull * 4;
-  cuuint64_t dims[4] = {32, samples, 1024, tiles};
+  cuuint64_t dims[4] = {32, first, 1024, tiles};
   cuuint64_t strides[3] = {tile_bytes, 128, samples * tile_bytes};
   cuuint32_t box[4] = {32, box_rows, 8, 1};
   cuuint32_t estr[4] = {1, 1, 1, 1};

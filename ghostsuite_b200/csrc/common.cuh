@@ -138,10 +138,10 @@ int make_tmap_f32_store_2d(CUtensorMap* out, const void* base, uint64_t rows, ui
 // 2-D map of a row-major matrix of 2- or 4-byte elements for boxes of 128 bytes of columns and `box_rows` rows with the
 // 128-byte swizzle.  Coordinates: (column, row).
 int make_tmap_rows(CUtensorMap* out, const void* base, int elem_bytes, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows);
-// Per-sample fp32 tiles [tiles][samples][32768], seen as [tiles, 1024 panels, samples, 32]: a box holds
-// eight panels (256 elements) of `box_rows` samples, each panel a swizzled [box_rows][32] block.
-// Coordinates: (0, sample, panel, tile).
-int make_tmap_f32_tiles(CUtensorMap* out, const void* base, uint64_t tiles, uint64_t samples, uint32_t box_rows);
+// Per-sample fp32 tiles [tiles][samples][32768], of whose samples the `first` ones count (those behind read as zero), seen as
+// [tiles, 1024 panels, first, 32]: a box holds eight panels (256 elements) of `box_rows` samples, each panel a
+// swizzled [box_rows][32] block.  Coordinates: (0, sample, panel, tile).
+int make_tmap_f32_tiles(CUtensorMap* out, const void* base, uint64_t tiles, uint64_t samples, uint64_t first, uint32_t box_rows);
 
 inline int ceil_div(long long a, long long b) { return static_cast<int>((a + b - 1) / b); }
 

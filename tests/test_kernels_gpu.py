@@ -257,6 +257,31 @@ def test_padded_and_split_operands(case, dtype):
         _lib.check(lib.ghost_set_wgrad_pair_mode(1))
 
 
+# sample counts around the streaming pass's blocks: 4, 8, 16, 32 validation and 8, 16, 32 train rows a stage; a budget of
+# 1 MiB makes groups of single samples, whose sums go through the workspace
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("case", [(1, 1, 3, 5, 7), (8, 4, 3, 70, 130), (9, 5, 2, 300, 129), (16, 8, 3, 257, 33), (17, 9, 2, 513, 20),
+                                  (32, 16, 2, 256, 128), (33, 17, 2, 130, 140), (70, 33, 1, 40, 300), (40, 3, 4, 700, 260)])
+def test_streaming_pass_blocks(case, dtype):
+    """Whole numbers whose products and sums float32 holds, and whose tiles bf16 does: equal in any order of addition."""
+    from ghostsuite_b200 import _lib
+    lib = _lib.load()
+    n_t, n_v, T, d, p = case
+    g = torch.Generator().manual_seed(n_t)
+    A, G = (torch.randint(-2, 3, (n_t + n_v, T, c), generator=g).to(dtype) for c in (d, p))
+    S = torch.einsum("ntp,ntd->npd", G.double(), A.double())
+    ref, gref = torch.einsum("vpd,bpd->vb", S[n_t:], S[:n_t]), S[:n_t].sum(0)
+    assert S.abs().max() <= 256 and S[n_t:].flatten(1).norm(dim=1).max() * S[:n_t].flatten(1).norm(dim=1).max() < 2 ** 24
+    try:
+        for budget in (12 << 30, 1 << 20):
+            _lib.check(lib.ghost_set_persample_budget_bytes(budget))
+            M, grad = ops().persample_dot(G.cuda(), A.cuda(), n_v, want_grad=True, grad_scale=0.5, grad_dtype=torch.float32)[:2]
+            after()
+            assert torch.equal(M.cpu().double(), ref) and torch.equal(grad.cpu().double(), 0.5 * gref)
+    finally:
+        _lib.check(lib.ghost_set_persample_budget_bytes(12 << 30))
+
+
 @pytest.mark.parametrize("sizes", [(37, 11, 70, 136, 264), (70, 35, 12, 72, 264)])
 def test_persample_dot_in_groups(sizes):
     """A small workspace budget forces the train samples through in several groups (and several
