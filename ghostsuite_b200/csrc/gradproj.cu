@@ -23,10 +23,14 @@
 // float32, k = 32: 189 -> 97 us; token table of 1024 float32 features, 16 x 2048 tokens: 107 -> 56 with mma.sync before).
 //
 // Few (sample, 128-token) units: a unit is one CTA's chain over all columns of G and A, whatever the number of
-// tokens in it, so a small batch leaves the GPU idle for the length of that chain.  There (kCluster) a cluster of
+// tokens in it, so a small batch leaves the GPU idle for the length of that chain.  There (kSome, kWhole) a cluster of
 // up to eight CTAs shares a unit: each projects its part of the columns, the partial [128, k] blocks are added through
 // distributed shared memory in rank order, and every CTA contracts its share of the tokens (10 tokens of 4407 + 452
 // float32, k = 44: 77 -> 22 us; 6 x 54 tokens of 2944 + 6528 bf16, k = 13: 47 -> 15).
+//
+// Where one CTA or one cluster has all tokens of a sample (up to 128 of them, or gradproj_group) the result is stored, without
+// zeroing it before and adding to it: calls of up to 128 tokens are 1.04 to 1.18 times as fast (12 x 1 token
+// of 128 + 2112 bf16, k = 44: 18.1 -> 15.6 us with the host's part, 14 x 12 of 1088 + 256 float32 17.8 -> 15.3).
 //
 // CTA layout: warps 0-3 epilogue, warp 4 TMA producer, warp 5 MMA issuer, warps 6-13 loaders where kSrc asks for them.
 #include "common.cuh"
@@ -52,6 +56,9 @@ struct GpParams {
   int half_g, half_a;      // kSrcMixed: which operand is bf16
   float scale;
   float* out;              // sample b at out + b * out_stride, [k_r, k_c] row-major
+  int accumulate;          // added to what is there, which the caller has zeroed or wants
+  int direct;              // one CTA or one cluster has all of a sample's units: stored, neither zeroed before nor added to
+  int group;               // > 1, with kNone: CTAs of the cluster that has a sample's units
   long long out_stride;
   int out_ld;              // pitch of an output row (k_c, or more inside a wider block)
   // embedding form: token ids [B, T] and the rows that stand for A P_c^T, [vocab, >= k_c] fp32
@@ -62,9 +69,10 @@ struct GpParams {
   int* err;
 };
 
+enum { kNone = 0, kSome = 1, kWhole = 2 };      // a cluster for each unit: no; with others of the sample; which is the sample
 enum { kSrcTma = 0, kSrcF32 = 1, kSrcBf16 = 2, kSrcMixed = 3 };      // how the rows of G and A reach shared memory
 
-template <int KMAX, int kSrc, bool kCluster>   // KMAX: largest padded rank this instantiation handles (32, 64 or 128)
+template <int KMAX, int kSrc, int kCluster>   // KMAX: largest padded rank this instantiation handles (32, 64 or 128)
 struct GpCfg {
   static constexpr int BM = 128, BK = 64;                  // BK: one 128-byte swizzle atom of bf16
   static constexpr int PARTS = kSrc == kSrcF32 || kSrc == kSrcMixed ? 2 : 1;    // bf16 parts of an element
@@ -78,7 +86,7 @@ struct GpCfg {
   // The pipeline is bound by how many bytes are in flight per SM, so the fp32 staging of the
   // projected blocks is kept to half a tile (64 tokens at a time; a cluster's partial blocks are
   // staged whole) and the rest goes to stages: it fills the 227 KB of shared memory.
-  static constexpr int kStageRows = kCluster ? 128 : 64;
+  static constexpr int kStageRows = kCluster != kNone ? 128 : 64;
   static constexpr int kProjBytes = 2 * kStageRows * KMAX * 4;
   static constexpr int kRoom = (232448 - 1280 - kProjBytes) / kStageBytes;
   static constexpr int kStages = kRoom < 8 ? kRoom : 8;
@@ -218,7 +226,13 @@ __device__ __forceinline__ float4 gp_ld_cluster(uint32_t addr) {
   return v;
 }
 
-template <int KMAX, int kSrc, bool kEmb, bool kCluster>
+__device__ __forceinline__ float gp_ld_cluster1(uint32_t addr) {
+  float v;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+  return v;
+}
+
+template <int KMAX, int kSrc, bool kEmb, int kCluster>
 __global__ void __launch_bounds__(kSrc == kSrcTma ? 192 : 448, 1)
 gradproj_kernel(const __grid_constant__ CUtensorMap tm_g, const __grid_constant__ CUtensorMap tm_pr,
                 const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_pc,
@@ -246,13 +260,19 @@ gradproj_kernel(const __grid_constant__ CUtensorMap tm_g, const __grid_constant_
   long long u0, u1;
   int kb0 = 0, kb1 = kb_total;
   uint32_t rank = 0, ranks = 1;
-  if constexpr (kCluster) {
+  if constexpr (kCluster != kNone) {
     rank = cluster_ctarank();
     asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(ranks));
     u0 = blockIdx.x / ranks;
     u1 = u0 + 1;
     kb0 = static_cast<int>(rank * kb_total / ranks);
     kb1 = static_cast<int>((rank + 1) * kb_total / ranks);
+  } else if (p.group > 1) {
+    rank = cluster_ctarank();
+    ranks = p.group;
+    const long long first = static_cast<long long>(blockIdx.x / ranks) * p.chunks_per_sample;
+    u0 = first + static_cast<long long>(rank) * p.chunks_per_sample / ranks;
+    u1 = first + static_cast<long long>(rank + 1) * p.chunks_per_sample / ranks;
   } else {
     const long long bx = blockIdx.x;
     u0 = bx * p.units_per_cta + (bx < p.units_extra ? bx : p.units_extra);
@@ -434,6 +454,32 @@ gradproj_kernel(const __grid_constant__ CUtensorMap tm_g, const __grid_constant_
         }
       }
     };
+    // This CTA, or the cluster, has all of sample b: its block goes through shared memory -- a cluster's through that of the
+    // stages, which nothing is on its way to any more -- and each CTA adds up and stores its share, in rank order.
+    auto store = [&](int b) {
+      float* block = ranks > 1 ? reinterpret_cast<float*>(smem) : s_r;            // [KMAX][KMAX]
+#pragma unroll
+      for (int i = 0; i < RT; ++i)
+#pragma unroll
+        for (int j = 0; j < CT; j += 4) {
+          *reinterpret_cast<float4*>(&block[(ty * RT + i) * KMAX + tx * CT + j]) = make_float4(o[i][j], o[i][j + 1], o[i][j + 2], o[i][j + 3]);
+          o[i][j] = o[i][j + 1] = o[i][j + 2] = o[i][j + 3] = 0.f;
+        }
+      if (ranks > 1) cluster_sync_all();
+      else asm volatile("bar.sync 1, 128;" ::: "memory");
+      float* dst = p.out + static_cast<long long>(b) * p.out_stride;
+#pragma unroll 1
+      for (int e = static_cast<int>(rank) * 128 + tid; e < p.k_r * KMAX; e += static_cast<int>(ranks) * 128) {
+        if (e % KMAX >= p.k_c) continue;
+        float sum = block[e];
+        if (ranks > 1) {
+          sum = 0.f;
+          for (uint32_t k = 0; k < ranks; ++k) sum += gp_ld_cluster1(map_to_cta(smem_u32(block + e), k));
+        }
+        dst[static_cast<long long>(e / KMAX) * p.out_ld + e % KMAX] = sum * p.scale;
+      }
+      if (ranks == 1) asm volatile("bar.sync 1, 128;" ::: "memory");
+    };
     // TMEM -> shared (fp32): row `tid` of one projected block
     auto stage_block = [&](uint32_t taddr, int kpad, float* dst) {
 #pragma unroll 1
@@ -497,7 +543,7 @@ gradproj_kernel(const __grid_constant__ CUtensorMap tm_g, const __grid_constant_
       }
     };
 
-    if constexpr (kCluster) {
+    if constexpr (kCluster != kNone) {
       // One unit.  Row `tid` of this CTA's partial blocks is staged; rows [first, first + share) of all CTAs' blocks are
       // then added up here, in place: nobody else reads them from this CTA.
       const int share = BM / static_cast<int>(ranks), first = static_cast<int>(rank) * share;
@@ -542,13 +588,21 @@ gradproj_kernel(const __grid_constant__ CUtensorMap tm_g, const __grid_constant_
         if (!kEmb) add_up(s_c, p.kc_pad, false);
         asm volatile("bar.sync 1, 128;" ::: "memory");
         contract(first, first + share);
-        flush(b);
+        if constexpr (kCluster == kSome) flush(b);
       }
+      __syncwarp();
+      if constexpr (kCluster == kWhole) store(b);
     }
     bool alive = true;
-    for (long long u = u0; u < u1 && !kCluster; ++u) {
+    for (long long u = u0; u < u1 && kCluster == kNone; ++u) {
       const int b = static_cast<int>(u / p.chunks_per_sample);
-      if (b != cur_b) { if (cur_b >= 0) flush(cur_b); cur_b = b; }
+      if (b != cur_b) {
+        if (cur_b >= 0) {
+          if (p.direct) store(cur_b);
+          else flush(cur_b);
+        }
+        cur_b = b;
+      }
       if constexpr (kEmb) gather(b, u % p.chunks_per_sample * BM + tid);
       if (!named_bar_and(2, 128, mbar_wait(&acc_full[acc], acc_phase, abort_flag, p.err, 124))) { alive = false; break; }
       tc_fence_after_sync();
@@ -575,12 +629,20 @@ gradproj_kernel(const __grid_constant__ CUtensorMap tm_g, const __grid_constant_
       }
       if (++acc == 2) { acc = 0; acc_phase ^= 1; }
     }
-    if (alive && cur_b >= 0) flush(cur_b);
+    if (kCluster == kNone && p.group > 1) cur_b = static_cast<int>(blockIdx.x / ranks);      // a CTA without units takes part too
+    if (kCluster == kNone && (p.group > 1 || (alive && cur_b >= 0))) {
+      __syncwarp();
+      if (p.direct) store(cur_b);
+      else flush(cur_b);
+    }
   }
 
-  if constexpr (kCluster) {
+  if (kCluster != kNone || p.group > 1) {
     __syncwarp();
-    if (warp >= 4) cluster_sync_all();     // the epilogue's barrier before the partial blocks are added up
+    if (warp >= 4) {
+      if constexpr (kCluster != kNone) cluster_sync_all();        // the epilogue's barrier before the partial blocks are added up
+      if (kCluster != kSome) cluster_sync_all();                  // and the one before the results are
+    }
     cluster_sync_all();                    // no CTA leaves while another reads its blocks
   }
   tc_fence_before_sync();
@@ -588,7 +650,7 @@ gradproj_kernel(const __grid_constant__ CUtensorMap tm_g, const __grid_constant_
   if (warp == 5) { tc_fence_after_sync(); tmem_dealloc(tmem_base, 512); }
 }
 
-template <int KMAX, int kSrc, bool kEmb, bool kCluster>
+template <int KMAX, int kSrc, bool kEmb, int kCluster>
 static int launch_gradproj_t(const CUtensorMap& tg, const CUtensorMap& tpr, const CUtensorMap& ta, const CUtensorMap& tpc,
                              GpParams& p, int ranks, const DeviceState* ds, cudaStream_t st) {
   using Cfg = GpCfg<KMAX, kSrc, kCluster>;
@@ -605,13 +667,13 @@ static int launch_gradproj_t(const CUtensorMap& tg, const CUtensorMap& tpr, cons
   cfg.blockDim = dim3(Cfg::kThreads, 1, 1);
   cfg.dynamicSmemBytes = Cfg::kSmemBytes;
   cfg.stream = st;
-  if (kCluster) {
+  if (kCluster != kNone || p.group > 1) {
     cudaLaunchAttribute& cluster = attr[cfg.numAttrs++];
     cluster.id = cudaLaunchAttributeClusterDimension;
     cluster.val.clusterDim.x = ranks;
     cluster.val.clusterDim.y = 1;
     cluster.val.clusterDim.z = 1;
-    cfg.gridDim = dim3(static_cast<unsigned>(p.units * ranks), 1, 1);
+    cfg.gridDim = dim3(static_cast<unsigned>((kCluster != kNone ? p.units : p.B) * ranks), 1, 1);
   } else {
     const int grid = static_cast<int>(p.units < ds->sm_count ? p.units : ds->sm_count);
     p.units_per_cta = static_cast<int>(p.units / grid);
@@ -633,6 +695,19 @@ static int gradproj_ranks(long long units, int stages, int kmax) {
   return units <= 16 ? 8 : units <= 34 ? 4 : units <= 74 ? 2 : 1;
 }
 
+// CTAs of a cluster that takes all units of a sample and stores its result, or 1: units dealt over the GPU, results added to zeros.
+// A cluster wherever its CTAs get no more units than those would: it saves the zeroing, a launch of 2 us on the
+// host and on the GPU, and the additions (4 x 796 tokens of 192 bf16, embedding form: 15.9 -> 14.5 us; 32 x 512 of 1024 + 4096, k = 32:
+// 36.6 -> 34.9).  At most as many clusters as are resident at once: sixteen of eight were not (16 x 2048 of 1024, embedding
+// form: 20 against 36 us).
+static int gradproj_group(int B, int chunks, int sm_count) {
+  if (chunks == 1) return 1;
+  const long long units = static_cast<long long>(B) * chunks, most = (units + sm_count - 1) / sm_count;
+  for (int c = 8; c > 1; c /= 2)
+    if (B <= (c == 8 ? 8 : c == 4 ? 32 : 72) && (chunks + c - 1) / c <= most) return c;
+  return 1;
+}
+
 // Operands of one projection as the entry points get them.
 struct GpOperands {
   const void *G, *A;               // A null: the embedding form
@@ -645,6 +720,15 @@ struct GpOperands {
 
 template <int KMAX, int kSrc, bool kEmb>
 static int launch_gradproj_src(const GpOperands& o, GpParams& p, const DeviceState* ds, cudaStream_t st) {
+  constexpr int kCols = GpCfg<KMAX, kSrc, kNone>::ATOMS * 64;
+  const int stages = ceil_div(p.n_r, kCols) + (kEmb ? 0 : ceil_div(p.n_c, kCols));
+  const int ranks = gradproj_ranks(p.units, stages, KMAX);
+  p.group = ranks > 1 || p.accumulate ? 1 : gradproj_group(p.B, p.chunks_per_sample, ds->sm_count);
+  // a sample's tokens are one CTA's or one cluster's: the results are stored, else added to zeros (written before the host
+  // is busy with the tensor maps)
+  p.direct = !p.accumulate && (p.chunks_per_sample == 1 || p.group > 1);
+  if (!p.accumulate && !p.direct)
+    GB_CUDA_OK(cudaMemset2DAsync(p.out, p.out_stride * sizeof(float), 0, static_cast<size_t>(p.k_r) * p.k_c * sizeof(float), p.B, st));
   CUtensorMap tg = {}, tpr, ta = {}, tpc = {};
   int rc;
   // the projection matrices as one-sample 3-D operands, so that one TMA instruction form serves all four
@@ -654,11 +738,10 @@ static int launch_gradproj_src(const GpOperands& o, GpParams& p, const DeviceSta
     if ((rc = make_tmap_bf16_3d(&tg, o.G, p.B, p.T, p.n_r, o.ldg, 128)) != GHOST_OK) return rc;
     if (!kEmb && (rc = make_tmap_bf16_3d(&ta, o.A, p.B, p.T, p.n_c, o.lda, 128)) != GHOST_OK) return rc;
   }
-  constexpr int kCols = GpCfg<KMAX, kSrc, false>::ATOMS * 64;
-  const int stages = ceil_div(p.n_r, kCols) + (kEmb ? 0 : ceil_div(p.n_c, kCols));
-  const int ranks = gradproj_ranks(p.units, stages, KMAX);
-  if (ranks > 1) return launch_gradproj_t<KMAX, kSrc, kEmb, true>(tg, tpr, ta, tpc, p, ranks, ds, st);
-  return launch_gradproj_t<KMAX, kSrc, kEmb, false>(tg, tpr, ta, tpc, p, 1, ds, st);
+  // (as one form with the test inside, those that add came out up to 4 % slower)
+  if (ranks > 1 && p.direct) return launch_gradproj_t<KMAX, kSrc, kEmb, kWhole>(tg, tpr, ta, tpc, p, ranks, ds, st);
+  if (ranks > 1) return launch_gradproj_t<KMAX, kSrc, kEmb, kSome>(tg, tpr, ta, tpc, p, ranks, ds, st);
+  return launch_gradproj_t<KMAX, kSrc, kEmb, kNone>(tg, tpr, ta, tpc, p, p.group, ds, st);
 }
 
 template <int kSrc, bool kEmb>
@@ -716,7 +799,6 @@ static int gradproj_dense(const GpOperands& o, GpParams& p, long long out_stride
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   p.out_stride = out_stride;
   p.out_ld = p.k_c;
-  GB_CUDA_OK(cudaMemset2DAsync(p.out, out_stride * sizeof(float), 0, static_cast<size_t>(p.k_r) * p.k_c * sizeof(float), p.B, st));
   return launch_gradproj<false>(o, p, ds, st);
 }
 
@@ -775,10 +857,8 @@ extern "C" int ghost_gradproj_embedding(const long long* ids, const void* G, int
   GB_REQUIRE(!g_is_f32 || (p_lo_offset % 8 == 0 && p_lo_offset >= p_cols && p_lo_offset + p_cols <= ldp_o),
              "ghost_gradproj_embedding: float out-grads need the residual part of P_o inside its rows");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (!accumulate)
-    GB_CUDA_OK(cudaMemset2DAsync(out, static_cast<size_t>(out_stride) * 4, 0, static_cast<size_t>(k_o) * k_i * 4,
-                                 static_cast<size_t>(B), st));
   GpParams p = {};
+  p.accumulate = accumulate ? 1 : 0;
   p.B = B; p.T = T; p.n_r = d; p.k_r = k_o; p.k_c = k_i; p.scale = scale;
   p.out = out; p.out_stride = out_stride; p.out_ld = out_ld;
   p.lo_r = p_lo_offset;

@@ -1186,7 +1186,10 @@ def test_norm_wide_rows(dtype, rms, N, T, F):
 @pytest.mark.parametrize("case", [(1, 1, 7, 5, 1, 1), (1, 10, 4407, 452, 44, 44), (2, 129, 333, 1000, 16, 17), (16, 127, 130, 70, 33, 9),
                                   (17, 128, 512, 300, 64, 64), (35, 100, 260, 516, 5, 60), (3, 300, 2050, 3072, 32, 48),
                                   (75, 64, 200, 136, 20, 20), (160, 33, 97, 104, 9, 4), (5, 140, 640, 259, 100, 128),
-                                  (80, 200, 321, 192, 128, 65)])
+                                  (80, 200, 321, 192, 128, 65),
+                                  # samples of several units in a cluster of eight, four, two, and too many for one
+                                  (8, 1000, 64, 130, 7, 11), (3, 129, 72, 70, 64, 64), (32, 300, 100, 64, 17, 128), (33, 300, 64, 64, 5, 6),
+                                  (72, 257, 66, 128, 20, 12), (7, 1025, 128, 64, 100, 128)])
 def test_gradproj_dense_unit_counts_and_widths(case, dtype):
     B, T, n_r, n_c, k_r, k_c = case
     g = torch.Generator().manual_seed(17)
