@@ -17,6 +17,7 @@
 
 #include "common.cuh"
 #include "mma_sync.cuh"
+#include "sm100_ptx.cuh"
 
 namespace gb {
 
@@ -239,16 +240,11 @@ constexpr int kEmbHotCap = 256;
 constexpr int kEmbTotals = 12;
 constexpr int kEmbChunk = 8;             // train rows of a join item
 constexpr int kEmbValChunk = 32;         // validation rows of a join item
+constexpr int kEmbBucketTokens = 8192;   // largest batch of emb_bucket_kernel
 
 // Counting hands every token its place in the bucket, so filling needs no second round of atomics.
-// It also clears the sums that the join adds to two launches later, and zero-fills a gradient of odd width.
-__global__ void __launch_bounds__(256) emb_count_kernel(const EmbBuckets q, double* __restrict__ M64, long long m_size,
-                                                        uint4* __restrict__ zero, long long zero_size) {
-  stream_order();
-  if (M64 != nullptr)
-    for (long long i = blockIdx.x * 256ll + threadIdx.x; i < m_size; i += gridDim.x * 256ll) M64[i] = 0.;
-  for (long long j = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; j < q.n_tok;
-       j += static_cast<long long>(gridDim.x) * blockDim.x) {
+__device__ __forceinline__ void emb_count_tokens(const EmbBuckets& q, long long first, long long step) {
+  for (long long j = first; j < q.n_tok; j += step) {
     const long long id = j < q.first_val ? q.ids_b[j] : q.ids_v[j - q.first_val];
     if (id >= 0 && id < q.vocab) {
       q.rank[j] = atomicAdd((j < q.first_val ? q.cnt_b : q.cnt_v) + id, 1);
@@ -257,6 +253,14 @@ __global__ void __launch_bounds__(256) emb_count_kernel(const EmbBuckets q, doub
       atomicExch(q.err, kErrBadIndex);
     }
   }
+}
+// It also clears the sums that the join adds to two launches later, and zero-fills a gradient of odd width.
+__global__ void __launch_bounds__(256) emb_count_kernel(const EmbBuckets q, double* __restrict__ M64, long long m_size,
+                                                        uint4* __restrict__ zero, long long zero_size) {
+  stream_order();
+  if (M64 != nullptr)
+    for (long long i = blockIdx.x * 256ll + threadIdx.x; i < m_size; i += gridDim.x * 256ll) M64[i] = 0.;
+  emb_count_tokens(q, blockIdx.x * 256ll + threadIdx.x, gridDim.x * 256ll);
   const uint4 z = make_uint4(0u, 0u, 0u, 0u);
   for (long long i = blockIdx.x * 256ll + threadIdx.x; i < zero_size; i += gridDim.x * 256ll) zero[i] = z;
 }
@@ -264,12 +268,11 @@ __global__ void __launch_bounds__(256) emb_count_kernel(const EmbBuckets q, doub
 // Buckets may lie in any order, so a block of ids takes its space with one atomic instead of waiting for
 // a scan over the whole table (22 us in one block for 50 k ids, 4.6 us now).  Also listed here: the
 // gradient's rows by size, join items, and ids that many validation tokens share (padding, separators).
-__global__ void __launch_bounds__(256) emb_alloc_kernel(const EmbBuckets q) {
-  stream_order();
-  __shared__ int s_warp[3][8], s_base[3];
-  const int id = blockIdx.x * 256 + threadIdx.x;
+// Every thread of the block has an id of its own, or none (in).
+template <int WARPS>
+__device__ __forceinline__ void emb_alloc_ids(const EmbBuckets& q, int id, bool in) {
+  __shared__ int s_warp[3][WARPS], s_base[3];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const bool in = id < q.vocab;
   const int tokens = in ? q.cnt_b[id] : 0;
   const int n[3] = {tokens, in && q.cnt_v ? q.cnt_v[id] : 0, q.want_rows && tokens > 0 && tokens <= kEmbSmallBucket ? 1 : 0};
   int before[3];
@@ -288,7 +291,7 @@ __global__ void __launch_bounds__(256) emb_alloc_kernel(const EmbBuckets q) {
   if (threadIdx.x < 3) {
     int sum = 0;
 #pragma unroll
-    for (int w = 0; w < 8; ++w) { const int c = s_warp[threadIdx.x][w]; s_warp[threadIdx.x][w] = sum; sum += c; }
+    for (int w = 0; w < WARPS; ++w) { const int c = s_warp[threadIdx.x][w]; s_warp[threadIdx.x][w] = sum; sum += c; }
     s_base[threadIdx.x] = sum ? atomicAdd(q.totals + (threadIdx.x == 2 ? 5 : threadIdx.x), sum) : 0;
   }
   __syncthreads();
@@ -337,15 +340,60 @@ __global__ void __launch_bounds__(256) emb_alloc_kernel(const EmbBuckets q) {
   }
 }
 
-__global__ void __launch_bounds__(256) emb_fill_kernel(const EmbBuckets q) {
+__global__ void __launch_bounds__(256) emb_alloc_kernel(const EmbBuckets q) {
   stream_order();
-  for (long long j = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; j < q.n_tok;
-       j += static_cast<long long>(gridDim.x) * blockDim.x) {
+  const int id = blockIdx.x * 256 + threadIdx.x;
+  emb_alloc_ids<8>(q, id, id < q.vocab);
+}
+
+__device__ __forceinline__ void emb_fill_buckets(const EmbBuckets& q, long long first, long long step) {
+  for (long long j = first; j < q.n_tok; j += step) {
     const int r = q.rank[j];
     if (r < 0) continue;
     if (j < q.first_val) q.perm_b[q.off_b[q.ids_b[j]] + r] = static_cast<int>(j);
     else q.perm_v[q.off_v[q.ids_v[j - q.first_val]] + r] = static_cast<int>(j - q.first_val);
   }
+}
+__global__ void __launch_bounds__(256) emb_fill_kernel(const EmbBuckets q) {
+  stream_order();
+  emb_fill_buckets(q, blockIdx.x * 256ll + threadIdx.x, gridDim.x * 256ll);
+}
+
+// All of it for a small batch in one launch, zeroing included: one cluster with a thread for each token, whose barriers part the
+// steps.  Instead of the whole table it looks at the ids that occur: the first token of an id (the first validation token of
+// one without train tokens) allocates it, and of the validation counts only those of ids that occur are cleared (the train
+// counts all: the gradient's empty rows are found by them).  The GPU takes about as long as for the three kernels and the memset, whose
+// launches bounded the host: hooks of up to 5000 tokens 39 - 41 -> 30 us where the host bounds them (8 + 2 x 41 tokens of 320 bf16,
+// vocabulary 36761), 8 + 2 x 512 of 768, 50304: 53.6 -> 51.1.  A thread for two tokens, 16384 of them: 53.9 -> 62.
+constexpr int kEmbBucketCtas = 8, kEmbBucketThreads = kEmbBucketTokens / kEmbBucketCtas;
+__global__ void __cluster_dims__(kEmbBucketCtas, 1, 1) __launch_bounds__(kEmbBucketThreads)
+emb_bucket_kernel(const EmbBuckets q, double* __restrict__ M64, long long m_size) {
+  stream_order();
+  const int j = blockIdx.x * kEmbBucketThreads + threadIdx.x, n_b = static_cast<int>(q.first_val);
+  const bool train = j < n_b;
+  int id = -1;
+  if (j < q.n_tok) {
+    const long long x = train ? q.ids_b[j] : q.ids_v[j - n_b];
+    if (x >= 0 && x < q.vocab) {
+      id = static_cast<int>(x);
+      if (q.cnt_v != nullptr) q.cnt_v[id] = 0;
+    } else {
+      atomicExch(q.err, kErrBadIndex);
+    }
+  }
+  const int zero = kEmbTotals + q.vocab;               // totals and train counts lie behind each other
+  for (int i = j; i < zero / 4; i += kEmbBucketTokens) reinterpret_cast<uint4*>(q.totals)[i] = make_uint4(0u, 0u, 0u, 0u);
+  if (j < (zero & 3)) q.totals[(zero & ~3) + j] = 0;
+  if (M64 != nullptr)
+    for (long long i = j; i < m_size; i += kEmbBucketTokens) M64[i] = 0.;
+  cluster_sync_all();
+  const int rank = id >= 0 ? atomicAdd((train ? q.cnt_b : q.cnt_v) + id, 1) : -1;
+  cluster_sync_all();
+  emb_alloc_ids<kEmbBucketThreads / 32>(q, id, rank == 0 && (train || q.cnt_b[id] == 0));
+  cluster_sync_all();
+  if (id < 0) return;
+  if (train) q.perm_b[q.off_b[id] + rank] = j;
+  else q.perm_v[q.off_v[id] + rank] = j - n_b;
 }
 
 // ---------------------------------------------------------------- dot product: join by id
@@ -967,11 +1015,17 @@ static int emb_pass(const EmbBuckets& q, const T* Gb, const T* Gv, int n_train, 
   if (fill && !by_rows && !quick) GB_CUDA_OK(cudaMemsetAsync(out, 0, out_bytes, st));
   const int tokens = blocks;
   if (quick) blocks = ds->sm_count * 8;
-  GB_CUDA_OK(launch_next(emb_count_kernel, dim3(blocks), dim3(256), 0, st, q, M64, static_cast<long long>(n_val) * n_train,
-                         reinterpret_cast<uint4*>(out), quick ? out_bytes / 16 : 0ll));
-  GB_CUDA_OK(launch_next(emb_alloc_kernel, dim3(ceil_div(q.vocab, 256)), dim3(256), 0, st, q));
-  GB_CUDA_OK(launch_next(emb_fill_kernel, dim3(tokens), dim3(256), 0, st, q));
-  count_launch(3);
+  if (q.n_tok <= kEmbBucketTokens && !quick) {
+    GB_CUDA_OK(launch_next(emb_bucket_kernel, dim3(kEmbBucketCtas), dim3(kEmbBucketThreads), 0, st, q, M64, static_cast<long long>(n_val) * n_train));
+    count_launch();
+  } else {
+    GB_CUDA_OK(cudaMemsetAsync(q.totals, 0, 4 * (kEmbTotals + static_cast<long long>(q.vocab) * (M != nullptr ? 2 : 1)), st));
+    GB_CUDA_OK(launch_next(emb_count_kernel, dim3(blocks), dim3(256), 0, st, q, M64, static_cast<long long>(n_val) * n_train,
+                           reinterpret_cast<uint4*>(out), quick ? out_bytes / 16 : 0ll));
+    GB_CUDA_OK(launch_next(emb_alloc_kernel, dim3(ceil_div(q.vocab, 256)), dim3(256), 0, st, q));
+    GB_CUDA_OK(launch_next(emb_fill_kernel, dim3(tokens), dim3(256), 0, st, q));
+    count_launch(3);
+  }
   const bool vec = d % 8 == 0 && ((reinterpret_cast<uintptr_t>(Gb) | reinterpret_cast<uintptr_t>(Gv)) & 15u) == 0;
   if (M != nullptr) {
     if (static_cast<long long>(n_val) * Tn > q.hot_threshold) {
@@ -1047,8 +1101,7 @@ static int emb_pass_group(const long long* ids, const void* G, int is_f32, int n
   q.first_val = tb;
   q.n_tok = tb + tv;
   q.vocab = vocab;
-  const long long zero_bytes = 4ll * (2 * static_cast<long long>(vocab) + kEmbTotals);
-  q.totals = static_cast<int*>(take(zero_bytes));
+  q.totals = static_cast<int*>(take(4ll * (2 * static_cast<long long>(vocab) + kEmbTotals)));
   q.cnt_b = q.totals + kEmbTotals;
   q.cnt_v = M ? q.cnt_b + vocab : nullptr;
   q.off_b = static_cast<int*>(take(4ll * vocab));
@@ -1069,7 +1122,6 @@ static int emb_pass_group(const long long* ids, const void* G, int is_f32, int n
   q.max_parts = kEmbMaxParts;
   q.want_rows = out != nullptr;
   q.err = ds->err_word;
-  GB_CUDA_OK(cudaMemsetAsync(q.totals, 0, M ? zero_bytes : 4ll * (vocab + kEmbTotals), st));
   float* Mg = M ? M + b0 : nullptr;
   if (is_f32) {
     const float* g = static_cast<const float*>(G);

@@ -1159,6 +1159,38 @@ def test_embedding_hook_small_rows_exact(dtype, n_t, n_v, d):
     assert torch.equal(grad.cpu(), (per[:n_t].sum(0).to(dtype) / n_t).to(dtype))
 
 
+# tokens around what one cluster buckets (8192) and around a warp; the table larger and smaller than them, ids of one side
+# only, ids that most tokens share, ids outside of the table
+@pytest.mark.parametrize("n_t,n_v,T,vocab", [(1, 1, 1, 1), (3, 2, 13, 5), (7, 1, 1024, 300), (6, 2, 1024, 50000), (3, 1, 2048, 7),
+                                             (2731, 1, 3, 900), (4, 4, 1023, 20001), (1, 5, 700, 64)])
+def test_embedding_buckets_of_one_cluster(n_t, n_v, T, vocab):
+    from ghostsuite_b200 import _lib
+    gen = torch.Generator().manual_seed(T)
+    ids = torch.randint(0, vocab, (n_t + n_v, T), generator=gen)
+    common = torch.rand(ids.shape, generator=gen)
+    ids[common < 0.3] = 0
+    ids[:n_t][common[:n_t] > 0.95] = vocab // 2          # mostly train tokens
+    G = torch.randint(-3, 4, (n_t + n_v, T, 8), generator=gen).float()
+    bad = ids.clone()
+    bad[common > 0.999] = vocab + 3
+    for tokens in (ids, bad):
+        keep = tokens < vocab
+        M, grad = ops().embedding_hook(tokens.cuda(), G.cuda(), n_v, vocab, 1.0)
+        torch.cuda.synchronize()
+        if bool(keep.all()):
+            _lib.poll_kernel_error()
+        else:
+            with pytest.raises(IndexError):
+                _lib.poll_kernel_error()
+        # whole numbers: exact in any order
+        x, k = (G * keep.unsqueeze(-1)).double(), tokens.clamp(max=vocab - 1)
+        val = torch.zeros(n_v, vocab, 8, dtype=torch.float64).scatter_add_(1, k[n_t:].unsqueeze(-1).expand(-1, -1, 8), x[n_t:])
+        ref = torch.stack([(val[:, k[b]] * x[b]).sum((1, 2)) for b in range(n_t)], dim=1)
+        gref = torch.zeros(vocab, 8, dtype=torch.float64).index_add_(0, k[:n_t].flatten(), x[:n_t].flatten(0, 1))
+        assert torch.equal(M.cpu().double(), ref)
+        assert torch.equal(grad.cpu(), (gref.float() / n_t))
+
+
 # widths around the lines of the block-per-rows kernel (1024, 2048, 4096, 8192, multiples of eight or not), row
 # counts that leave a group of rows unfinished, one row, several splits
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
