@@ -185,7 +185,7 @@ def _prepare_sample_grad_or_dotprod(layer: nn.Module, grad_output: Tuple[torch.T
     # undo it in their epilogue
     own["_ghost_backprop_scale"] = float(backprops.shape[0]) if loss_reduction == "mean" else 1.0
     # the per-parameter [n_train] vectors are reduced in one batched op when the backward pass ends
-    if _layers._PENDING_DOTS is None and _layers.begin_deferred_dots():
+    if _layers.begin_deferred_dots():
         try:
             torch.autograd.Variable._execution_engine.queue_callback(_layers.finalize_pending_dots)
         except Exception:
@@ -232,8 +232,8 @@ def _apply_train_grad(layer: nn.Module, val_batch_size: int, loss_reduction: str
         if type(layer) in _layers._SELF_APPLYING or isinstance(layer, nn.LayerNorm):
             train_grad_fn(layer, layer.activations, layer.backprops, val_batch_size)
         else:
-            weight = _layers._param(layer, "weight")
-            if weight is not None and _layers._wanted(weight, weight.requires_grad):
+            weight = getattr(layer, "weight", None)
+            if weight is not None and getattr(weight, "initially_requires_grad", weight.requires_grad):
                 grad_weight = train_grad_fn(layer, layer.activations, layer.backprops, val_batch_size)
                 if grad_weight is None:
                     raise ValueError(
@@ -241,8 +241,8 @@ def _apply_train_grad(layer: nn.Module, val_batch_size: int, loss_reduction: str
                         "Ensure the compute_layer_train_grad function is implemented correctly.")
                 if grad_weight is not _layers.DEFERRED:      # else: handed over by the launch that makes it
                     _create_or_accumulate_train_grad(weight, grad_weight)
-            bias = _layers._param(layer, "bias")
-            if bias is not None and _layers._wanted(bias, bias.requires_grad):
+            bias = getattr(layer, "bias", None)
+            if bias is not None and getattr(bias, "initially_requires_grad", bias.requires_grad):
                 _train_grad_bias_from_layer(layer, val_batch_size, loss_reduction)
     finally:
         own = layer.__dict__
@@ -265,9 +265,8 @@ def _train_grad_bias_from_layer(layer: nn.Module, val_batch_size: int, loss_redu
     scale = float(getattr(layer, "_ghost_backprop_scale", 1.0))
     if loss_reduction == "mean":
         scale /= n_train
-    bias = _layers._param(layer, "bias")
-    out_dtype = bias.dtype if bias.dtype in (torch.float32, torch.bfloat16) else torch.float32
-    _layers._train_grad_from_vectors(bias, colsums, n_train, scale, out_dtype, layer.__dict__.get("_ghost_bias_grad"))
+    out_dtype = layer.bias.dtype if layer.bias.dtype in (torch.float32, torch.bfloat16) else torch.float32
+    _layers._train_grad_from_vectors(layer.bias, colsums, n_train, scale, out_dtype, layer.__dict__.get("_ghost_bias_grad"))
 
 
 def _compute_train_grad_bias(B: torch.Tensor, val_batch_size: int, loss_reduction: str = "mean") -> torch.Tensor:
