@@ -59,6 +59,7 @@ PROTOTYPES = {
     "ghost_set_wgrad_pair_mode": (_i, [_i]),
     "ghost_wgrad_workspace_bytes": (_ll, [_i, _i]),
     "ghost_wgrad_bf16": (_i, [_vp, _vp, _ll, _i, _i, _ll, _ll, _f, _i, _vp, _i, _vp, _ll, _vp]),
+    "ghost_gram_pass": (_i, [_vp, _vp, _i, _i, _i, _ll, _i, _i, _ll, _ll, _i, _vp, _f, _vp, _i, _vp, _ll, _vp]),
     "ghost_wgrad_parts": (_i, [_vp, _vp, _i, _ll, _ll, _i, _i, _ll, _ll, _f, _i, _vp, _i, _vp, _ll, _vp]),
     "ghost_persample_workspace_bytes": (_ll, [_i, _i, _i, _i, _i]),
     "ghost_set_persample_budget_bytes": (_i, [_ll]),

@@ -331,7 +331,7 @@ static int launch_gram(const GramOperands& o, int n_train, int n_val, long long 
 static int g_gram_pair_mode = 1;
 bool xty_pair_usable(const DeviceState* ds);     // a cluster of two ~198 KB CTAs fits on the device
 
-static int gram_dot(const GramOperands& o, int n_train, int n_val, long long T, int round_mode, float scale, float* M_out, void* stream) {
+int gram_dot(const GramOperands& o, int n_train, int n_val, long long T, int round_mode, float scale, float* M_out, bool cleared, void* stream) {
   const DeviceState* ds = device_state();
   if (!ds) return GHOST_ERR_DEVICE;
   GB_REQUIRE(o.a_t && o.a_v && o.g_t && o.g_v && M_out, "ghost_gram_dot_bf16: null pointer");
@@ -342,7 +342,7 @@ static int gram_dot(const GramOperands& o, int n_train, int n_val, long long T, 
              static_cast<long long>(n_val) * T < (1ll << 31) - 256,
              "ghost_gram_dot_bf16: more than 2^31 tokens");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  GB_CUDA_OK(cudaMemsetAsync(M_out, 0, sizeof(float) * static_cast<size_t>(n_val) * n_train, st));
+  if (!cleared) GB_CUDA_OK(cudaMemsetAsync(M_out, 0, sizeof(float) * static_cast<size_t>(n_val) * n_train, st));
   const long long rows_t = static_cast<long long>(n_train) * T, rows_v = static_cast<long long>(n_val) * T;
   // Rounds of tiles over the GPU times the cycles of a K step of a tile (128 for 256 x 256 on a pair and 128 x 256 on one
   // SM, 64 for 128 x 128, a tenth more for its operand traffic): 2048 x 1024 tokens are 32 tiles of 256 x 256 on 74
@@ -374,7 +374,7 @@ extern "C" int ghost_gram_dot_bf16(const void* a_train, const void* a_val, const
                                    long long ld_gv, int round_mode, float scale, float* M_out,
                                    void* stream) {
   const gb::GramOperands o = {a_train, a_val, g_train, g_val, ld_at, ld_av, ld_gt, ld_gv, ka, kg, 1, 0};
-  return gb::gram_dot(o, n_train, n_val, T, round_mode, scale, M_out, stream);
+  return gb::gram_dot(o, n_train, n_val, T, round_mode, scale, M_out, false, stream);
 }
 
 extern "C" int ghost_gram_dot_parts(const void* A, const void* G, int parts, int n_train, int n_val, long long T, int d, int p,
@@ -384,9 +384,5 @@ extern "C" int ghost_gram_dot_parts(const void* A, const void* G, int parts, int
   GB_REQUIRE(parts == 1 || parts == 2, "ghost_gram_dot_parts: one or two parts");
   GB_REQUIRE(n_train > 0, "No training samples to compute dot product, check batch sizes.");
   GB_REQUIRE(n_val > 0 && T > 0 && d > 0 && p > 0 && ld_a >= d && ld_g >= p, "ghost_gram_dot_parts: bad dimensions");
-  const long long rows_t = static_cast<long long>(n_train) * T;
-  const char *a = static_cast<const char*>(A), *g = static_cast<const char*>(G);
-  const GramOperands o = {a, a + rows_t * ld_a * 2, g, g + rows_t * ld_g * 2, ld_a, ld_a, ld_g, ld_g, d, p, parts,
-                          rows_t + static_cast<long long>(n_val) * T};
-  return gram_dot(o, n_train, n_val, T, round_mode, scale, M_out, stream);
+  return gram_dot(gram_operands(A, G, parts, n_train, n_val, T, d, p, ld_a, ld_g), n_train, n_val, T, round_mode, scale, M_out, false, stream);
 }

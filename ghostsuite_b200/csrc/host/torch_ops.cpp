@@ -411,7 +411,7 @@ void dense_paths(const Launch& L, const Operand& A, const Operand& B, long long 
   const Operand &X = in_by_out ? A : B, &Y = in_by_out ? B : A;
   if (gram) {
     // one copy of what has to be copied serves the Grams and the gradient, and gives the bias its sums
-    const long long N = A.N, rows = (N - n_val) * A.T;
+    const long long N = A.N;
     const int m = static_cast<int>(X.cols), n = static_cast<int>(Y.cols), b = in_by_out ? 1 : 0;
     check_split(N - n_val, n_val, "gram_dot");
     M = empty({n_val, N - n_val}, A.t, at::kFloat);
@@ -423,10 +423,10 @@ void dense_paths(const Launch& L, const Operand& A, const Operand& B, long long 
     const bool take = bias && (A.conv || (ops.split && A.T >= 16));
     if (take) sums = empty({N, B.cols}, A.t, at::kFloat);
     ops.prepare(base, L.st(), take ? b + 1 : 0, take ? sums.data_ptr<float>() : nullptr);
-    launch_gram(L, ops, 1 - b, base, n_val, 0, 1.f, M);
-    if (grad.defined())
-      check(ghost_wgrad_parts(ops.where(0, base), ops.where(1, base), ops.parts(), N * A.T, rows, m, n, ops.ld[0], ops.ld[1], scale, 0,
-                              grad.data_ptr(), is_f32(grad), base + off_ws, ws_bytes, L.st()));
+    const int a = 1 - b;
+    check(ghost_gram_pass(ops.where(a, base), ops.where(b, base), ops.parts(), static_cast<int>(N - n_val), static_cast<int>(n_val), A.T,
+                          static_cast<int>(A.cols), static_cast<int>(B.cols), ops.ld[a], ops.ld[b], in_by_out ? 1 : 0, M.data_ptr<float>(), scale,
+                          grad.defined() ? grad.data_ptr() : nullptr, grad.defined() ? is_f32(grad) : 0, base + off_ws, ws_bytes, L.st()));
   } else {
     PerSample r = persample_dot(L, X, Y, n_val, 1.f, gdt >= 0, scale, gdt == 0 ? at::kBFloat16 : at::kFloat,
                                 !fuse ? 0 : in_by_out ? 2 : 1, !bias ? 0 : in_by_out ? 2 : 1);

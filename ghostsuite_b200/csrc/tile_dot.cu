@@ -42,7 +42,8 @@ struct TileDotParams {
   float* M;                   // [n_val, n_train]
   float* sum;                 // [tiles * 32768] fp32 or null
   int sum_init;               // 1: this group overwrites sum, 0: it accumulates
-  // direct output of the train gradient (single-group case): out[r, c] (= or +=) out_scale * sum
+  // direct output of the train gradient (single-group case): out[r, c] (= or +=) out_scale * sum.  With `sum` too (bf16 tiles) the
+  // blocks of train rows before the last one add up there, and the last one rounds to `out` once
   void* out;                  // [m_cols, n_cols] row-major in the parameter dtype, or null
   int out_is_f32, out_accumulate;
   int m_cols, n_cols, n_tiles_n;
@@ -499,13 +500,19 @@ tile_dot_mma_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_const
         if (++stage == kStages) { stage = 0; phase ^= 1; }
         if (do_sum && g < CW) {
           const int e0 = warp * (CW * 8) + g * 8 + q * 2;    // element inside the stage
-          if (p.out != nullptr) {
+          float2* at = reinterpret_cast<float2*>(p.sum + s * kMmaCols + e0);
+          if (p.sum != nullptr && !(p.sum_init && j0 == 0)) {
+            const float2 old = *at;
+            t0 += old.x;
+            t1 += old.y;
+          }
+          if (p.out != nullptr && (p.sum == nullptr || j0 + TR >= p.n_grp)) {
             // one stage is kMmaCols / 256 row segments (256 columns each) of one 128 x 256 tile
             const int r = tm * 128 + in_tile * (kMmaCols / 256) + (e0 >> 8);
             const int c = tn * 256 + (e0 & 255);
             if (r < p.m_cols && c < p.n_cols) {
               const long long o = static_cast<long long>(r) * p.n_cols + c;
-              const bool rmw = p.out_accumulate || j0 > 0;
+              const bool rmw = p.out_accumulate || (p.sum == nullptr && j0 > 0);
               const bool pair = (c + 1 < p.n_cols) && ((p.n_cols & 1) == 0);     // o is even then
               t0 *= p.out_scale; t1 *= p.out_scale;
               if (p.out_is_f32) {
@@ -533,10 +540,7 @@ tile_dot_mma_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_const
               }
             }
           } else {
-            float2* dst = reinterpret_cast<float2*>(p.sum + s * kMmaCols + e0);
-            float2 v = make_float2(t0, t1);
-            if (!(p.sum_init && j0 == 0)) { const float2 old = *dst; v.x += old.x; v.y += old.y; }
-            *dst = v;
+            *at = make_float2(t0, t1);
           }
         }
         if (++in_tile == kStagesPerTile) {

@@ -22,6 +22,7 @@
 #include "common.cuh"
 #include "sm100_ptx.cuh"
 #include "xty_colsum.cuh"
+#include "gram_operands.cuh"
 #include "xty_operands.cuh"
 #include "xty_store.cuh"
 
@@ -414,7 +415,7 @@ __global__ void xty_finalize_kernel(const float* ws, long long ld_ws, OutT* __re
 int launch_xty_pair_tiles(const XtyOperands& o, long long n_samples_total, long long T, int samples, int sample0, void* vgrad,
                           int v_is_f32, const XtyColsum& cs, float* zero, long long zero_n, const DeviceState* ds, cudaStream_t st);
 int launch_xty_pair_wgrad(const XtyOperands& o, long long n_rows, int splits, float* acc_ws, long long ld_acc, void* out,
-                          int out_is_f32, float scale, int accumulate, const DeviceState* ds, cudaStream_t st);
+                          int out_is_f32, float scale, int accumulate, float* zero, long long zero_n, const DeviceState* ds, cudaStream_t st);
 bool xty_pair_usable(const DeviceState* ds);
 static int g_wgrad_pair_mode = 1;      // same meaning as below
 static int g_persample_pair_mode = 1;  // 0 off, 1 where no half of a pair would idle, 2 wherever applicable
@@ -505,9 +506,9 @@ extern "C" long long ghost_wgrad_workspace_bytes(int m_cols, int n_cols) {
   return static_cast<long long>(m_cols) * round_up(n_cols, 4) * 4;
 }
 
-// D[m_cols, n_cols] = scale * sum_{rows < n_rows} X[row, :]^T Y[row, :]
+// D[m_cols, n_cols] = scale * sum_{rows < n_rows} X[row, :]^T Y[row, :]; `zero` is cleared for the kernel that follows, or null
 static int wgrad(const XtyOperands& o, long long n_rows, float scale, int accumulate, void* out, int out_is_f32, void* ws,
-                 long long ws_bytes, void* stream) {
+                 long long ws_bytes, float* zero, long long zero_n, void* stream) {
   const DeviceState* ds = device_state();
   if (!ds) return GHOST_ERR_DEVICE;
   const int m_cols = o.cols[0], n_cols = o.cols[1];
@@ -534,6 +535,8 @@ static int wgrad(const XtyOperands& o, long long n_rows, float scale, int accumu
   p.out_scale = scale;
   p.out_accumulate = accumulate;
   p.out_vec = n_cols % 8 == 0 && (reinterpret_cast<uintptr_t>(out) & 15u) == 0;
+  p.zero = zero;
+  p.zero_n = zero_n;
   p.err = ds->err_word;
   int rc;
   const bool pair = pair_kernel_fits(g_wgrad_pair_mode, o, ds);
@@ -545,7 +548,7 @@ static int wgrad(const XtyOperands& o, long long n_rows, float scale, int accumu
   if (splits > 1) GB_CUDA_OK(cudaMemsetAsync(ws, 0, static_cast<size_t>(m_cols) * p.ld_acc * 4, st));
   else p.mode = kEpiDirect;
   if (pair) {
-    rc = launch_xty_pair_wgrad(o, n_rows, splits, p.acc_ws, p.ld_acc, out, out_is_f32, scale, accumulate, ds, st);
+    rc = launch_xty_pair_wgrad(o, n_rows, splits, p.acc_ws, p.ld_acc, out, out_is_f32, scale, accumulate, zero, zero_n, ds, st);
   } else {
     p.kb_per_split = ceil_div(kb, splits);
     p.k_splits = ceil_div(kb, p.kb_per_split);
@@ -558,7 +561,7 @@ static int wgrad(const XtyOperands& o, long long n_rows, float scale, int accumu
 extern "C" int ghost_wgrad_bf16(const void* X, const void* Y, long long n_rows, int m_cols, int n_cols,
                                 long long ldx, long long ldy, float scale, int accumulate, void* out,
                                 int out_is_f32, void* ws, long long ws_bytes, void* stream) {
-  return wgrad(XtyOperands{{X, Y}, {m_cols, n_cols}, {ldx, ldy}, 1, 0, false}, n_rows, scale, accumulate, out, out_is_f32, ws, ws_bytes, stream);
+  return wgrad(XtyOperands{{X, Y}, {m_cols, n_cols}, {ldx, ldy}, 1, 0, false}, n_rows, scale, accumulate, out, out_is_f32, ws, ws_bytes, nullptr, 0, stream);
 }
 
 extern "C" int ghost_wgrad_parts(const void* X, const void* Y, int parts, long long part_rows, long long n_rows, int m_cols, int n_cols, long long ldx,
@@ -567,7 +570,29 @@ extern "C" int ghost_wgrad_parts(const void* X, const void* Y, int parts, long l
   const int rc = check_parts(X, Y, parts, m_cols, n_cols, ldx, ldy);
   if (rc != GHOST_OK) return rc;
   GB_REQUIRE(part_rows >= n_rows, "ghost_wgrad_parts: more rows than a part has");
-  return wgrad(XtyOperands{{X, Y}, {m_cols, n_cols}, {ldx, ldy}, parts, part_rows, true}, n_rows, scale, accumulate, out, out_is_f32, ws, ws_bytes, stream);
+  return wgrad(XtyOperands{{X, Y}, {m_cols, n_cols}, {ldx, ldy}, parts, part_rows, true}, n_rows, scale, accumulate, out, out_is_f32, ws, ws_bytes, nullptr, 0,
+               stream);
+}
+
+// The train gradient first: its GEMM clears the matrix that the Grams add to, whose memset before them cost a launch (2 us on
+// the host, 1.5 and a gap on the GPU).
+extern "C" int ghost_gram_pass(const void* A, const void* G, int parts, int n_train, int n_val, long long T, int d, int p, long long ld_a,
+                               long long ld_g, int in_by_out, float* M_out, float grad_scale, void* grad_out, int grad_is_f32, void* ws,
+                               long long ws_bytes, void* stream) {
+  GB_REQUIRE(A && G && M_out, "ghost_gram_pass: null pointer");
+  GB_REQUIRE(n_train > 0, "No training samples to compute dot product, check batch sizes.");
+  GB_REQUIRE(n_val > 0 && T > 0 && d > 0 && p > 0, "ghost_gram_pass: empty dimension");
+  int rc = check_parts(A, G, parts, d, p, ld_a, ld_g);
+  if (rc != GHOST_OK) return rc;
+  if (grad_out) {
+    const long long rows = static_cast<long long>(n_train + n_val) * T;
+    const XtyOperands o = in_by_out ? XtyOperands{{A, G}, {d, p}, {ld_a, ld_g}, parts, rows, true}
+                                    : XtyOperands{{G, A}, {p, d}, {ld_g, ld_a}, parts, rows, true};
+    rc = wgrad(o, static_cast<long long>(n_train) * T, grad_scale, 0, grad_out, grad_is_f32, ws, ws_bytes, M_out,
+               static_cast<long long>(n_val) * n_train, stream);
+    if (rc != GHOST_OK) return rc;
+  }
+  return gram_dot(gram_operands(A, G, parts, n_train, n_val, T, d, p, ld_a, ld_g), n_train, n_val, T, 0, 1.f, M_out, grad_out != nullptr, stream);
 }
 
 namespace gb {
@@ -671,15 +696,14 @@ static int persample_dot(const XtyOperands& o, int n_train, int n_val, long long
     p.sample0 = 0;
     p.vgrad = vws;
     if ((rc = tile_pass(p)) != GHOST_OK) return rc;
-    // With a single group the streaming kernel can write the train gradient itself (scaled, in the
-    // parameter dtype): no fp32 sum buffer, no finalize pass.  A bf16 output is only written
-    // directly when one 32-sample block covers the batch, so it is rounded once.
-    const bool direct = grad_out && (grad_is_f32 || n_train <= 32);
+    // With a single group the streaming kernel writes the train gradient itself (scaled, in the
+    // parameter dtype): no finalize pass.  A bf16 output of more than one block of 32 train samples is summed up in the
+    // fp32 buffer first and rounded once, by the last block (of fp32 tiles by a finalize pass: that kernel has no registers left).
+    // 233 + 17 x 2033 of 42 x 64 bf16: the pass after it took 2.3 us and its launch as much on the host, 95.9 -> 92.4 a hook.
+    const bool blocks = grad_out && !grad_is_f32 && n_train > 32, direct = grad_out && !(blocks && v_is_f32);
     if ((rc = launch_tile_dot(vws, static_cast<int>(N), n_train, vws, static_cast<int>(N), v_is_f32, tiles,
-                              n_val, n_train, 0, n_train, dot_scale, M_out,
-                              (grad_out && !direct) ? sum : nullptr, 1, direct ? grad_out : nullptr,
-                              grad_is_f32, grad_accumulate, m_cols, n_cols, p.n_tiles, grad_scale, ds,
-                              st)) != GHOST_OK)
+                              n_val, n_train, 0, n_train, dot_scale, M_out, blocks ? sum : nullptr, 1, direct ? grad_out : nullptr,
+                              grad_is_f32, grad_accumulate, m_cols, n_cols, p.n_tiles, grad_scale, ds, st)) != GHOST_OK)
       return rc;
     if (direct || !grad_out) return GHOST_OK;
   } else {

@@ -516,7 +516,7 @@ int launch_xty_pair_tiles(const XtyOperands& o, long long n_samples_total, long 
 // Train-gradient pass over n_rows token rows (one sample), operands in the blocked layout: one split stores
 // scale * X^T Y to `out`, more of them add into acc_ws[m_cols, ld_acc] (fp32, zeroed by the caller).
 int launch_xty_pair_wgrad(const XtyOperands& o, long long n_rows, int splits, float* acc_ws, long long ld_acc, void* out,
-                          int out_is_f32, float scale, int accumulate, const DeviceState* ds, cudaStream_t st) {
+                          int out_is_f32, float scale, int accumulate, float* zero, long long zero_n, const DeviceState* ds, cudaStream_t st) {
   XtyPairParams p = pair_params(o, ds);
   p.T = n_rows;
   p.accumulate = splits == 1 ? 2 : 1;
@@ -527,6 +527,8 @@ int launch_xty_pair_wgrad(const XtyOperands& o, long long n_rows, int splits, fl
   p.out_scale = scale;
   p.acc_ws = acc_ws;
   p.ld_acc = ld_acc;
+  p.zero = zero;
+  p.zero_n = zero_n;
   const int kb = ceil_div(n_rows, o.parts == 2 ? XtyPairCfg<2>::BK : XtyPairCfg<1>::BK);
   p.kb_per_split = ceil_div(kb, splits);
   p.samples = ceil_div(kb, p.kb_per_split);

@@ -136,6 +136,12 @@ int ghost_wgrad_parts(const void* X, const void* Y, int parts, long long part_ro
                       long long ldy, float scale, int accumulate, void* out, int out_is_f32, void* ws, long long ws_bytes,
                       void* stream);
 
+/* ghost_gram_dot_parts (scale 1, no rounding) and, if grad_out != NULL, ghost_wgrad_parts over the train rows in one call, whose GEMM
+ * clears M_out for the Grams.  A: activations, G: out-grad, merged; the gradient is [p, d], with in_by_out [d, p]. */
+int ghost_gram_pass(const void* A, const void* G, int parts, int n_train, int n_val, long long T, int d, int p, long long ld_a,
+                    long long ld_g, int in_by_out, float* M_out, float grad_scale, void* grad_out, int grad_is_f32, void* ws,
+                    long long ws_bytes, void* stream);
+
 /* ---- Linear / Conv1D weight dot product, per-sample-gradient path ---------------------------- */
 /* X, Y: [n_train + n_val, T, cols] bf16.  M[v,b] = dot_scale * <X_v^T Y_v, X_b^T Y_b>.  Per-sample
  * weight-gradient tiles are formed in TMEM by a tcgen05 GEMM over each sample's tokens and written

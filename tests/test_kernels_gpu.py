@@ -278,6 +278,9 @@ def test_streaming_pass_blocks(case, dtype):
             M, grad = ops().persample_dot(G.cuda(), A.cuda(), n_v, want_grad=True, grad_scale=0.5, grad_dtype=torch.float32)[:2]
             after()
             assert torch.equal(M.cpu().double(), ref) and torch.equal(grad.cpu().double(), 0.5 * gref)
+            half = ops().persample_dot(G.cuda(), A.cuda(), n_v, want_grad=True, grad_scale=0.5, grad_dtype=torch.bfloat16)[1]
+            after()
+            assert torch.equal(half.cpu(), (0.5 * gref).bfloat16())          # summed in float32, rounded once
     finally:
         _lib.check(lib.ghost_set_persample_budget_bytes(12 << 30))
 
