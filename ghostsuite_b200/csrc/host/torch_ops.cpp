@@ -601,18 +601,19 @@ void check_projection_out(const Tensor& out, long long B, long long k, const cha
     invalid(std::string(who) + " output must be a float32 [B, >= k_r*k_c] row-major view");
 }
 
-// (G, A, P_r, P_c, k_r, k_c, scale, out)
+// (G, A, P_r, P_c, k_r, k_c, scale, out or None: a new [B, k_r, k_c])
 PyObject* py_gradproj_dense(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return guarded([&]() -> PyObject* {
     need(n, 8, "gradproj_dense");
     const Tensor &G0 = cuda_tensor(a[0]), &A0 = cuda_tensor(a[1]), &P_r = cuda_tensor(a[2]), &P_c = cuda_tensor(a[3]);
-    const Tensor& out = cuda_tensor(a[7]);
     Launch L(G0);
     const Tensor G = as3d(G0), A = as3d(A0);
     const long long B = G.size(0), T = G.size(1), k_r = integer(a[4]), k_c = integer(a[5]);
     if (A.size(0) != B || A.size(1) != T)
       throw GhostError(kNotCuda, "Batch size mismatch between activations and output gradients");
-    check_projection_out(out, B, k_r * k_c, "gradproj");
+    const bool have = present(a[7]);
+    const Tensor out = have ? cuda_tensor(a[7]) : empty({B, k_r, k_c}, G, at::kFloat);
+    if (have) check_projection_out(out, B, k_r * k_c, "gradproj");
     const bool split = is_f32(G) || is_f32(A);
     const long long n_r = G.size(2), n_c = A.size(2), cp_r = pad8(n_r), cp_c = pad8(n_c);
     if (P_r.size(1) != (split ? 3 : 1) * cp_r || P_c.size(1) != (split ? 3 : 1) * cp_c)
@@ -647,6 +648,7 @@ PyObject* py_gradproj_dense(PyObject*, PyObject* const* a, Py_ssize_t n) {
                                       len[1], P_r.data_ptr(), P_c.data_ptr(), static_cast<int>(k_r), static_cast<int>(k_c),
                                       P_r.size(1), P_c.size(1), real(a[6]), out.data_ptr<float>(), out.stride(0), L.st()));
     }
+    if (!have) return wrap(out);
     Py_INCREF(a[7]);
     return a[7];
   });

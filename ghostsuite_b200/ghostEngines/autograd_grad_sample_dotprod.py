@@ -22,6 +22,8 @@ import torch.nn as nn
 from .. import _lib, ops
 from . import supported_layers_grad_samplers_dotprod as _layers
 from .supported_layers_grad_samplers_dotprod import (
+    _param,
+    _wanted,
     _supported_layers_dotprod,
     _create_or_accumulate_train_grad,
 )
@@ -185,7 +187,7 @@ def _prepare_sample_grad_or_dotprod(layer: nn.Module, grad_output: Tuple[torch.T
     # undo it in their epilogue
     own["_ghost_backprop_scale"] = float(backprops.shape[0]) if loss_reduction == "mean" else 1.0
     # the per-parameter [n_train] vectors are reduced in one batched op when the backward pass ends
-    if _layers.begin_deferred_dots():
+    if _layers._PENDING_DOTS is None and _layers.begin_deferred_dots():
         try:
             torch.autograd.Variable._execution_engine.queue_callback(_layers.finalize_pending_dots)
         except Exception:
@@ -222,18 +224,19 @@ _PASS_ATTRIBUTES = ("activations", "backprops", "_ghost_backprop_scale", "_ghost
 
 def _apply_train_grad(layer: nn.Module, val_batch_size: int, loss_reduction: str = "mean"):
     """Backward hook, part 2: averaged train gradients into ``param.train_grad`` (reference :140-196)."""
-    _, train_grad_fn = _supported_layers_dotprod.get(type(layer), (None, None))
-    val_batch_size = layer.__dict__.get("_ghost_val_batch", val_batch_size)
+    own, kind = layer.__dict__, type(layer)
+    _, train_grad_fn = _supported_layers_dotprod.get(kind, (None, None))
+    val_batch_size = own.get("_ghost_val_batch", val_batch_size)
     if not train_grad_fn:
         raise ValueError(
             f"Layer {layer.__class__.__name__} is not supported for training gradient computation. "
             "Ensure it is included in the _supported_layers_dotprod dictionary.")
     try:
-        if type(layer) in _layers._SELF_APPLYING or isinstance(layer, nn.LayerNorm):
+        if kind in _layers._SELF_APPLYING or isinstance(layer, nn.LayerNorm):
             train_grad_fn(layer, layer.activations, layer.backprops, val_batch_size)
         else:
-            weight = getattr(layer, "weight", None)
-            if weight is not None and getattr(weight, "initially_requires_grad", weight.requires_grad):
+            weight, bias = _param(layer, "weight"), _param(layer, "bias")
+            if weight is not None and _wanted(weight, weight.requires_grad):
                 grad_weight = train_grad_fn(layer, layer.activations, layer.backprops, val_batch_size)
                 if grad_weight is None:
                     raise ValueError(
@@ -241,11 +244,9 @@ def _apply_train_grad(layer: nn.Module, val_batch_size: int, loss_reduction: str
                         "Ensure the compute_layer_train_grad function is implemented correctly.")
                 if grad_weight is not _layers.DEFERRED:      # else: handed over by the launch that makes it
                     _create_or_accumulate_train_grad(weight, grad_weight)
-            bias = getattr(layer, "bias", None)
-            if bias is not None and getattr(bias, "initially_requires_grad", bias.requires_grad):
+            if bias is not None and _wanted(bias, bias.requires_grad):
                 _train_grad_bias_from_layer(layer, val_batch_size, loss_reduction)
     finally:
-        own = layer.__dict__
         for attr in _PASS_ATTRIBUTES:
             own.pop(attr, None)
 
@@ -257,7 +258,8 @@ def _train_grad_bias_from_layer(layer: nn.Module, val_batch_size: int, loss_redu
     n_train = B.size(0) - val_batch_size
     if n_train <= 0:
         raise ValueError("No training samples to compute gradients, check batch sizes.")
-    colsums = layer.__dict__.get("_ghost_colsums")
+    own = layer.__dict__
+    colsums = own.get("_ghost_colsums")
     if colsums is None:
         if isinstance(layer, nn.Conv2d):      # features are dim 1 there: [N, p, H, W] -> [N, H*W, p]
             B = B.reshape(B.size(0), B.size(1), -1).transpose(1, 2).contiguous()
@@ -265,8 +267,9 @@ def _train_grad_bias_from_layer(layer: nn.Module, val_batch_size: int, loss_redu
     scale = float(getattr(layer, "_ghost_backprop_scale", 1.0))
     if loss_reduction == "mean":
         scale /= n_train
-    out_dtype = layer.bias.dtype if layer.bias.dtype in (torch.float32, torch.bfloat16) else torch.float32
-    _layers._train_grad_from_vectors(layer.bias, colsums, n_train, scale, out_dtype, layer.__dict__.get("_ghost_bias_grad"))
+    bias = _param(layer, "bias")
+    out_dtype = torch.bfloat16 if bias.dtype is torch.bfloat16 else torch.float32
+    _layers._train_grad_from_vectors(bias, colsums, n_train, scale, out_dtype, own.get("_ghost_bias_grad"))
 
 
 def _compute_train_grad_bias(B: torch.Tensor, val_batch_size: int, loss_reduction: str = "mean") -> torch.Tensor:

@@ -21,6 +21,8 @@ from ..autograd_grad_sample_dotprod import register_hook_pair
 
 def _flatten_tokens(x: torch.Tensor) -> torch.Tensor:
     """``[B, D] -> [B, 1, D]``; ``[B, ..., D] -> [B, T, D]``."""
+    if x.dim() == 3:
+        return x
     if x.dim() <= 2:
         return x.unsqueeze(1)
     return x.reshape(x.shape[0], -1, x.shape[-1])
@@ -70,16 +72,20 @@ class GradProjHooks:
         if A_raw is None:
             raise RuntimeError(f"Missing cached activations for GradProjection in {self.layer_name}")
         B_out = grad_output[0]
+        # instance attributes are written to the dictionary: nn.Module.__setattr__ searches the parameter,
+        # buffer and module tables for each of these names first
+        own = module.__dict__
         if B_out is None:
-            module._ghost_grad_proj = None
-            delattr(module, "_ghost_A_raw")
+            own["_ghost_grad_proj"] = None
+            own.pop("_ghost_A_raw", None)
             return
-        B_out = B_out.detach()
+        if B_out.requires_grad:
+            B_out = B_out.detach()
         if self.layer_type == "Embedding":
             self._compute_embedding_proj(module, A_raw, B_out)
         else:
             self._compute_dense_proj(module, A_raw, B_out)
-        delattr(module, "_ghost_A_raw")
+        own.pop("_ghost_A_raw", None)
 
     def _compute_dense_proj(self, module: nn.Module, A_raw: torch.Tensor, B_out: torch.Tensor) -> None:
         """``module._ghost_grad_proj[b] = batch_size * (P_o grad W_b P_i^T)`` as ``[B, k_o, k_i]`` float32
@@ -88,23 +94,24 @@ class GradProjHooks:
         is_conv1d = module.__class__.__name__ == "Conv1D"
         A = _flatten_tokens(A_raw)
         B = _flatten_tokens(B_out)
-        if A.dtype != B.dtype:
+        if A.dtype is not B.dtype:
             common = torch.promote_types(A.dtype, B.dtype)
             A, B = A.to(common), B.to(common)
-        batch = A.shape[0]
-        if B.shape[0] != batch or B.shape[1] != A.shape[1]:
+        batch = A.size(0)
+        if B.size(0) != batch or B.size(1) != A.size(1):
             raise RuntimeError(f"Batch size mismatch between activations and gradients in {self.layer_name}")
-        split = A.dtype == torch.float32
+        split = A.dtype is torch.float32
         P_i, P_o = self._prepared(split)
-        k_i, k_o = self.P_i.shape[0], self.P_o.shape[0]
+        k_i, k_o = self.P_i.size(0), self.P_o.size(0)
         if is_conv1d:
             P_r, P_c, k_r, k_c = P_i, P_o, k_i, k_o
         else:
             P_r, P_c, k_r, k_c = P_o, P_i, k_o, k_i
-        out = self._out_fn(batch) if self._out_fn is not None else \
-            torch.empty((batch, k_r * k_c), dtype=torch.float32, device=A.device)
-        ops.gradproj_dense(B, A, P_r, P_c, k_r, k_c, float(batch), out)
-        module._ghost_grad_proj = out.view(batch, k_r, k_c)
+        if self._out_fn is None:
+            proj = ops.gradproj_dense(B, A, P_r, P_c, k_r, k_c, float(batch))
+        else:
+            proj = ops.gradproj_dense(B, A, P_r, P_c, k_r, k_c, float(batch), self._out_fn(batch)).view(batch, k_r, k_c)
+        module.__dict__["_ghost_grad_proj"] = proj
 
     def _compute_embedding_proj(self, module: nn.Module, indices: torch.Tensor,
                                 grad_output: torch.Tensor) -> None:
@@ -112,19 +119,18 @@ class GradProjHooks:
         ``[B, k_o, k_i]`` float32 (reference :167-222, a Python loop over every token there): one
         kernel that streams the out-grad rows once and gathers the rows of ``P_i^T`` by token id."""
         batch = indices.shape[0]
-        ids = indices.reshape(batch, -1)
-        g = grad_output.reshape(batch, ids.shape[1], grad_output.shape[-1])
+        ids = indices if indices.dim() == 2 else indices.reshape(batch, -1)
+        g = grad_output if grad_output.dim() == 3 and grad_output.shape[:2] == ids.shape else \
+            grad_output.reshape(batch, ids.shape[1], grad_output.shape[-1])
         if g.dtype not in (torch.float32, torch.bfloat16):
             g = g.float()
-        split = g.dtype == torch.float32
+        split = g.dtype is torch.float32
         _, P_o = self._prepared(split)
         if self._P_i_t is None:
             self._P_i_t = ops.prepare_embedding_projection(self.P_i.to(g.device))
-        k_i, k_o = self.P_i.shape[0], self.P_o.shape[0]
-        out = self._out_fn(batch) if self._out_fn is not None else \
-            torch.empty((batch, k_o * k_i), dtype=torch.float32, device=g.device)
-        ops.gradproj_embedding(ids, g, P_o, self._P_i_t, k_o, k_i, 1.0, out)
-        module._ghost_grad_proj = out.view(batch, k_o, k_i)
+        k_i, k_o = self.P_i.size(0), self.P_o.size(0)
+        out = ops.gradproj_embedding(ids, g, P_o, self._P_i_t, k_o, k_i, 1.0, None if self._out_fn is None else self._out_fn(batch))
+        module.__dict__["_ghost_grad_proj"] = out.view(batch, k_o, k_i)
 
     def attach(self, module: nn.Module) -> None:
         self._handles = register_hook_pair(module, self.forward_hook_store_inputs, self.backward_hook_compute_proj,

@@ -130,6 +130,19 @@ def _should_use_ghost_computation(layer: nn.Module, A: torch.Tensor, B: torch.Te
     layer.use_ghost_computation = layer._ghost_rule_choice = bool(gram <= per)
 
 
+def _param(layer: nn.Module, name: str):
+    """``getattr(layer, name, None)`` for a parameter.  nn.Module finds its parameters after the search for an
+    attribute has failed, 0.4 us each time; a layer's hook asks for weight and bias a dozen times."""
+    params = layer.__dict__["_parameters"]
+    return params[name] if name in params else getattr(layer, name, None)
+
+
+def _wanted(param: torch.Tensor, otherwise: bool) -> bool:
+    """``param.initially_requires_grad``, which the engines set, or ``otherwise``.  (From the dictionary:
+    on a parameter without the attribute a search that fails costs half a microsecond.)"""
+    return bool(param.__dict__.get("initially_requires_grad", otherwise))
+
+
 #: optional observer ``fn(param)`` called every time a layer has added its contribution to
 #: ``param.train_grad`` (the data-parallel layer uses it to start all-reducing finished gradients
 #: while the backward pass is still running)
@@ -142,10 +155,11 @@ def _create_or_accumulate_train_grad(param: torch.Tensor, grad: torch.Tensor) ->
         f"Gradient shape ({grad.shape}) does not match parameter shape ({param.shape})"
     if grad.requires_grad:
         grad = grad.detach()
-    if hasattr(param, "train_grad"):
-        param.train_grad.add_(grad)
+    own = param.__dict__
+    if "train_grad" in own:
+        own["train_grad"].add_(grad)
     else:
-        param.train_grad = grad
+        own["train_grad"] = grad
     if TRAIN_GRAD_OBSERVER is not None:
         TRAIN_GRAD_OBSERVER(param)
 
@@ -181,8 +195,9 @@ def _small_job_for(X: torch.Tensor, n_train: int, n_val: int, want: str):
     with _PENDING_LOCK:
         if _PENDING_SMALL is None:
             return None
-        for job in reversed(_PENDING_SMALL[-4:]):
-            if job["X"] is X and job["n_train"] == n_train and job.get(want) is None:
+        for back in range(1, min(4, len(_PENDING_SMALL)) + 1):
+            job = _PENDING_SMALL[-back]
+            if job["X"] is X and want not in job and job["n_train"] == n_train:
                 return job
         job = {"X": X, "n_train": n_train, "n_val": n_val}
         _PENDING_SMALL.append(job)
@@ -226,35 +241,38 @@ def finalize_pending_dots() -> None:
     with _PENDING_LOCK:
         pending, _PENDING_DOTS = _PENDING_DOTS, None
         small, _PENDING_SMALL = _PENDING_SMALL, None
+    if not pending and not small:
+        return
     if small:
         _exchange_pending_val_rows(small)        # validation rows of a batch split over ranks
-    last = {id(param): (param, M) for param, M in pending or ()}
+    last = {id(item[0]): item for item in pending or ()}
     on_device = [item for item in last.values() if item[1].is_cuda]
     if small or on_device:
         vectors = ops.pass_reduce(small or [], [M for _, M in on_device])
         for (param, M), vector in zip(on_device, vectors):
-            if getattr(param, "grad_dot_prod_matrix", None) is M:
-                param.grad_dot_prod = vector
+            own = param.__dict__
+            if own.get("grad_dot_prod_matrix") is M:
+                own["grad_dot_prod"] = vector
         for job in small or ():
             param = job.get("param")
             if param is not None:
                 grad = job["sum_out"]
                 _create_or_accumulate_train_grad(param, grad if grad.shape == param.shape else grad.view_as(param))
-    for param, M in last.values():
-        if not M.is_cuda and getattr(param, "grad_dot_prod_matrix", None) is M:
-            param.grad_dot_prod = M.sum(dim=0)
+    if len(on_device) != len(last):
+        for param, M in last.values():
+            if not M.is_cuda and getattr(param, "grad_dot_prod_matrix", None) is M:
+                param.grad_dot_prod = M.sum(dim=0)
 
 
 def _set_dot(param: torch.Tensor, M: torch.Tensor) -> None:
-    param.grad_dot_prod_matrix = M
+    own = param.__dict__
+    own["grad_dot_prod_matrix"] = M
     with _PENDING_LOCK:
         deferred = _PENDING_DOTS is not None
         if deferred:
             _PENDING_DOTS.append((param, M))
-    if deferred:
-        param.grad_dot_prod = M          # placeholder until the backward pass ends
-    else:
-        param.grad_dot_prod = M.sum(dim=0)
+    # inside a backward pass a placeholder until it ends
+    own["grad_dot_prod"] = M if deferred else M.sum(dim=0)
 
 
 def _check_batch(A, B, val_batch_size: int) -> int:
@@ -350,7 +368,7 @@ def _exchange_pending_val_rows(jobs) -> None:
     """One all-gather for the validation rows of every job that waits for them: each rank sends its
     jobs' rows packed one after the other; job ``j`` then reads row ``r * per_rank + i`` at
     ``gathered[r, offset_j + i * F]`` (``ops.small_reduce_batch``)."""
-    waiting = [j for j in jobs if j.get("val_exchange") is not None and j.get("M") is not None]
+    waiting = [j for j in jobs if "val_exchange" in j and j["val_exchange"] is not None and j.get("M") is not None]
     if not waiting:
         return
     ex = waiting[0]["val_exchange"]
@@ -429,9 +447,12 @@ def dot_product_with_exchange(layer: nn.Module, A: torch.Tensor, B: torch.Tensor
 def _dense_dot_product(layer: nn.Module, A: torch.Tensor, B: torch.Tensor, val_batch_size: int,
                        weight_is_in_by_out: bool) -> None:
     n_train = _check_batch(A, B, val_batch_size)
-    A = A.detach()
-    B = B.detach()
-    _should_use_ghost_computation(layer, A, B, val_batch_size=val_batch_size)
+    if A.requires_grad:
+        A = A.detach()
+    if B.requires_grad:
+        B = B.detach()
+    if not hasattr(layer, "use_ghost_computation"):
+        _should_use_ghost_computation(layer, A, B, val_batch_size=val_batch_size)
     if val_batch_size > 0 and "_ghost_backprop_scale" in layer.__dict__:
         _dense_hook(layer, A, B, val_batch_size, n_train, weight_is_in_by_out)
         return
@@ -465,17 +486,15 @@ def _dense_hook(layer: nn.Module, A: torch.Tensor, B: torch.Tensor, n_val: int, 
     """``_dense_dot_product`` inside a backward hook: the train gradients are asked for right after the
     dot products, so one native call computes both and allocates what the end of the pass fills."""
     own = layer.__dict__
-    weight = layer.weight
-    bias = getattr(layer, "bias", None)
-    scale = own["_ghost_backprop_scale"] / n_train
+    weight, bias = _param(layer, "weight"), _param(layer, "bias")
     bias_dtype = None
-    if bias is not None and getattr(bias, "initially_requires_grad", bias.requires_grad):
+    if bias is not None and _wanted(bias, bias.requires_grad):
         bias_dtype = torch.bfloat16 if bias.dtype is torch.bfloat16 else torch.float32
+    use_gram = own.get("use_ghost_computation")
     M, grad, colsums, bias_M, bias_grad = ops.dense_hook(
-        A, B, n_val, weight_is_in_by_out, layer.use_ghost_computation,
-        _grad_dtype(weight, A) if getattr(weight, "initially_requires_grad", True) else None, scale,
-        bias is not None, bias_dtype,
-        PATH_RULE == "cost" and own.get("_ghost_rule_choice") is own.get("use_ghost_computation"), FUSE_BIAS_COLSUMS)
+        A, B, n_val, weight_is_in_by_out, layer.use_ghost_computation if use_gram is None else use_gram,
+        _grad_dtype(weight, A) if _wanted(weight, True) else None, own["_ghost_backprop_scale"] / n_train,
+        bias is not None, bias_dtype, PATH_RULE == "cost" and own.get("_ghost_rule_choice") is use_gram, FUSE_BIAS_COLSUMS)
     if grad is not None:
         own["_ghost_cached_train_grad"] = (A.data_ptr(), B.data_ptr(), A.size(0), grad)
     _set_dot(weight, M)
@@ -534,14 +553,14 @@ def _compute_embedding_dot_product(layer: nn.Embedding, A: torch.Tensor, B: torc
                                    val_batch_size: int):
     """nn.Embedding: id-equality-masked Gram of the out-grad rows (reference :181-211)."""
     _check_batch(A, B, val_batch_size)
-    own = layer.__dict__
+    own, weight = layer.__dict__, _param(layer, "weight")
     if "_ghost_backprop_scale" in own and val_batch_size > 0 and A.numel() < 2 ** 31 - 1 \
-            and getattr(layer.weight, "initially_requires_grad", layer.weight.requires_grad):
+            and _wanted(weight, weight.requires_grad):
         # inside a backward hook: the train gradient is asked for next and needs the same buckets (whose
         # token indices are 32-bit for the whole batch; on their own either half may have as many)
-        M, grad = ops.embedding_hook(A, B, val_batch_size, layer.weight.shape[0], own["_ghost_backprop_scale"])
+        M, grad = ops.embedding_hook(A, B, val_batch_size, weight.shape[0], own["_ghost_backprop_scale"])
         own["_ghost_cached_train_grad"] = (A.data_ptr(), B.data_ptr(), A.size(0), grad)
-        _set_dot(layer.weight, M)
+        _set_dot(weight, M)
         return
     M = ops.embedding_dot(A.detach(), B.detach(), val_batch_size, layer.weight.shape[0])
     _set_dot(layer.weight, M)
@@ -558,9 +577,8 @@ def _compute_embedding_train_grad(layer: nn.Embedding, A: torch.Tensor, B: torch
         grad = cached[3]
     else:
         grad = ops.embedding_wgrad(A, B, n_train, layer.weight.shape[0], _backprop_scale(layer), float(n_train))
-    if grad.dtype != layer.weight.dtype:
-        grad = grad.to(layer.weight.dtype)
-    return grad
+    dtype = _param(layer, "weight").dtype
+    return grad if grad.dtype is dtype else grad.to(dtype)
 
 
 # --------------------------------------------------------------------------------------------
@@ -583,7 +601,7 @@ def _norm_hook(layer: nn.Module, A: torch.Tensor, B: torch.Tensor, n_val: int, e
     right after: one native call for the vectors and every output.  False when the layer is called
     on its own, or has parameters of a type the batched launch does not write."""
     own = layer.__dict__
-    weight, bias = layer.weight, getattr(layer, "bias", None)
+    weight, bias = _param(layer, "weight"), _param(layer, "bias")
     if "_ghost_backprop_scale" not in own or "_ghost_ln_cache" in own or n_val <= 0 or not A.is_cuda \
             or weight.dtype not in _GRAD_TYPES or not (bias is None or bias.dtype in _GRAD_TYPES):
         return False
@@ -623,9 +641,10 @@ def _compute_layernorm_train_grad(layer: nn.LayerNorm, A: torch.Tensor, B: torch
     layer.__dict__.pop("_ghost_ln_cache", None)
     scale = _backprop_scale(layer) / n_train
     sw, sb = layer.__dict__.pop("_ghost_norm_grads", (None, None))
-    _train_grad_from_vectors(layer.weight, gw, n_train, scale, layer.weight.dtype, sw)
-    if layer.bias is not None:
-        _train_grad_from_vectors(layer.bias, gb, n_train, scale, layer.bias.dtype, sb)
+    weight, bias = _param(layer, "weight"), _param(layer, "bias")
+    _train_grad_from_vectors(weight, gw, n_train, scale, weight.dtype, sw)
+    if bias is not None:
+        _train_grad_from_vectors(bias, gb, n_train, scale, bias.dtype, sb)
     return None
 
 
@@ -715,10 +734,11 @@ def _conv_hook(layer: nn.Conv2d, A: torch.Tensor, B: torch.Tensor, n_val: int) -
     mode other than zeros or padding given by name, other data types)."""
     own = layer.__dict__
     if "_ghost_backprop_scale" not in own or n_val <= 0 or layer.groups != 1 or layer.padding_mode != "zeros" \
-            or isinstance(layer.padding, str) or A.dtype not in _GRAD_TYPES or B.dtype is not A.dtype or A.dim() != 4 \
-            or A.size(0) > 65535 or layer.weight[0].numel() > 1 << 21:      # limits of the kernel's grid
+            or isinstance(layer.padding, str) or A.dtype not in _GRAD_TYPES or B.dtype is not A.dtype or A.dim() != 4:
         return False
-    weight, bias = layer.weight, layer.bias
+    weight, bias = _param(layer, "weight"), _param(layer, "bias")
+    if A.size(0) > 65535 or weight.numel() // max(1, weight.size(0)) > 1 << 21:      # limits of the kernel's grid
+        return False
     n_train = A.size(0) - n_val
     if not hasattr(layer, "use_ghost_computation"):
         N, p = B.shape[0], B.shape[1]
@@ -726,11 +746,11 @@ def _conv_hook(layer: nn.Conv2d, A: torch.Tensor, B: torch.Tensor, n_val: int) -
         _should_use_ghost_computation(layer, A.new_empty(()).expand(N, d, T), B.new_empty(()).expand(N, p, T), conv=True,
                                       val_batch_size=n_val)
     bias_dtype = None
-    if bias is not None and getattr(bias, "initially_requires_grad", bias.requires_grad):
+    if bias is not None and _wanted(bias, bias.requires_grad):
         bias_dtype = torch.bfloat16 if bias.dtype is torch.bfloat16 else torch.float32
     M, grad, sums, bias_M, bias_grad = ops.conv_hook(
         A, B, n_val, (*layer.kernel_size, *layer.stride, *layer.padding, *layer.dilation), layer.use_ghost_computation,
-        _grad_dtype(weight, A) if getattr(weight, "initially_requires_grad", True) else None,
+        _grad_dtype(weight, A) if _wanted(weight, True) else None,
         own["_ghost_backprop_scale"] / n_train, bias is not None, bias_dtype)
     if grad is not None:
         own["_ghost_cached_train_grad"] = (A.data_ptr(), B.data_ptr(), A.size(0), grad)
@@ -774,7 +794,7 @@ def _compute_conv2d_train_grad(layer: nn.Conv2d, A: torch.Tensor, B: torch.Tenso
         grad = ops.wgrad(B_tok[:n_train], A_tok[:n_train], _backprop_scale(layer) / n_train,
                          _grad_dtype(layer.weight, A))
     layer.__dict__.pop("_ghost_conv_tokens", None)
-    return grad.view_as(layer.weight)
+    return grad.view_as(_param(layer, "weight"))
 
 
 _supported_layers_dotprod = {

@@ -534,9 +534,9 @@ def prepare_projection(P: torch.Tensor, split: bool) -> torch.Tensor:
 
 
 def gradproj_dense(G: torch.Tensor, A: torch.Tensor, P_r: torch.Tensor, P_c: torch.Tensor,
-                   k_r: int, k_c: int, scale: float, out: torch.Tensor) -> torch.Tensor:
+                   k_r: int, k_c: int, scale: float, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """``out[b] = scale * (G_b P_r^T)^T (A_b P_c^T)`` written into ``out`` (``[B, >= k_r*k_c]`` fp32,
-    possibly a column slice of a wider row-major buffer).  ``P_r``/``P_c`` come from
+    possibly a column slice of a wider row-major buffer), or into a new ``[B, k_r, k_c]`` tensor.  ``P_r``/``P_c`` come from
     :func:`prepare_projection` (split layout iff the activations are fp32)."""
     if _timing is None:
         return _native().gradproj_dense(G, A, P_r, P_c, k_r, k_c, scale, out)
