@@ -54,17 +54,29 @@ inline int early_start(cudaLaunchAttribute* attr, cudaStream_t st) {
   attr->val.programmaticStreamSerializationAllowed = 1;
   return 1;
 }
+// With blocks in clusters of a shape other than (1, 1, 1) that divides the grid.
 template <typename... P, typename... A>
-inline cudaError_t launch_next(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
-  cudaLaunchAttribute attr;
+inline cudaError_t launch_next_cluster(dim3 cluster, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+  cudaLaunchAttribute attr[2];
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
-  cfg.attrs = &attr;
-  cfg.numAttrs = early_start(&attr, st);
+  cfg.attrs = attr;
+  cfg.numAttrs = early_start(attr, st);
+  if (cluster.x * cluster.y * cluster.z > 1) {
+    cudaLaunchAttribute& c = attr[cfg.numAttrs++];
+    c.id = cudaLaunchAttributeClusterDimension;
+    c.val.clusterDim.x = cluster.x;
+    c.val.clusterDim.y = cluster.y;
+    c.val.clusterDim.z = cluster.z;
+  }
   return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+}
+template <typename... P, typename... A>
+inline cudaError_t launch_next(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+  return launch_next_cluster(dim3(1, 1, 1), kernel, grid, block, smem, st, std::forward<A>(args)...);
 }
 // The other half of launch_next, in every kernel that is launched so, before its first access to global memory and in every
 // block: waits until all work ahead in the stream has ended and can be read, then lets the next kernel come up.  (In

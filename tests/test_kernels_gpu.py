@@ -218,7 +218,9 @@ def test_persample_dot_column_sums(case, which):
 # tiles of 128; every operand needs a copy, so the padded and the two-part layouts are what runs
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("case", [(3, 2, 1, 63, 65), (2, 1, 16, 127, 129), (3, 1, 17, 257, 63), (2, 2, 33, 130, 70),
-                                  (2, 1, 63, 65, 257), (2, 1, 129, 300, 140), (33, 3, 5, 71, 199), (2, 1, 260, 190, 510)])
+                                  (2, 1, 63, 65, 257), (2, 1, 129, 300, 140), (33, 3, 5, 71, 199), (2, 1, 260, 190, 510),
+                                  # chunks of 64 rows that add up their sums as a cluster of two to eight, and more of them
+                                  (1, 1, 65, 70, 130), (2, 1, 300, 129, 66), (1, 2, 512, 64, 300), (1, 1, 513, 33, 72)])
 def test_padded_and_split_operands(case, dtype):
     """Padded bf16 copies and two-part float32 operands: matrix, train gradient, column sums, and the
     gradient GEMM with results that no 16-byte store fits, through both tile kernels."""
@@ -513,7 +515,8 @@ def test_dense_small(case, dtype, in_by_out):
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
-@pytest.mark.parametrize("shape", [(8, 6, 24), (12, 1, 10), (5, 300, 520), (3, 1024, 768)])
+@pytest.mark.parametrize("shape", [(8, 6, 24), (12, 1, 10), (5, 300, 520), (3, 1024, 768),
+                                   (3, 65, 300), (4, 129, 24), (3, 2000, 40), (40, 449, 513)])
 def test_colsum_and_bias(shape, dtype):
     N, T, p = shape
     g = torch.Generator().manual_seed(4)
