@@ -33,6 +33,8 @@
 // of 128 + 2112 bf16, k = 44: 18.1 -> 15.6 us with the host's part, 14 x 12 of 1088 + 256 float32 17.8 -> 15.3).
 //
 // CTA layout: warps 0-3 epilogue, warp 4 TMA producer, warp 5 MMA issuer, warps 6-13 loaders where kSrc asks for them.
+#include <atomic>
+
 #include "common.cuh"
 #include "sm100_ptx.cuh"
 
@@ -546,7 +548,8 @@ gradproj_kernel(const __grid_constant__ CUtensorMap tm_g, const __grid_constant_
     if constexpr (kCluster != kNone) {
       // One unit.  Row `tid` of this CTA's partial blocks is staged; rows [first, first + share) of all CTAs' blocks are
       // then added up here, in place: nobody else reads them from this CTA.
-      const int share = BM / static_cast<int>(ranks), first = static_cast<int>(rank) * share;
+      const int most = (BM + static_cast<int>(ranks) - 1) / static_cast<int>(ranks), first = static_cast<int>(rank) * most;
+      const int share = first + most < BM ? most : BM - first;
       const int b = static_cast<int>(u0 / p.chunks_per_sample);
       const long long t_first = u0 % p.chunks_per_sample * BM;
       const bool owned = tid >= first && tid < first + share;
@@ -685,26 +688,65 @@ static int launch_gradproj_t(const CUtensorMap& tg, const CUtensorMap& tpr, cons
   return post_launch("gradproj_kernel");
 }
 
-// CTAs that share a unit: as many as keep the GPU's SMs busy with one unit per cluster.  A GPC has 18 or 20 SMs, so about
-// 16 clusters of eight and 34 of four are resident at once.  The cluster's two barriers and the exchange cost about
+// Clusters of `ranks` CTAs of this kernel that are resident at once, as the driver counts them: a cluster stays inside a GPC,
+// whose SMs differ from device to device.  (A 148-SM device: 16 of eight by its GPCs of 18 and 20, but sixteen of them, 24 of six or
+// 48 of three took two rounds: 17.5 us against 32.1 for 48 x 100 tokens of 640 + 640, k = 40.)
+template <int KMAX, int kSrc, bool kEmb, int kCluster>
+static int gradproj_resident(int ranks, const DeviceState* ds) {
+  using Cfg = GpCfg<KMAX, kSrc, kCluster>;
+  static std::atomic<int> known[64][9];      // count + 1; several threads may find the same
+  std::atomic<int>& slot = known[ds->device][ranks];
+  int n = slot.load(std::memory_order_relaxed);
+  if (n == 0) {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = ranks;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.gridDim = dim3(ranks, 1, 1);
+    cfg.blockDim = dim3(Cfg::kThreads, 1, 1);
+    cfg.dynamicSmemBytes = Cfg::kSmemBytes;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    int count = 0;
+    if (cudaFuncSetAttribute(gradproj_kernel<KMAX, kSrc, kEmb, kCluster>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&count, gradproj_kernel<KMAX, kSrc, kEmb, kCluster>, &cfg) != cudaSuccess) {
+      (void)cudaGetLastError();
+      count = 0;
+    }
+    n = count + 1;
+    slot.store(n, std::memory_order_relaxed);
+  }
+  return n - 1;
+}
+
+// CTAs that share a unit: as many as are resident with one unit per cluster.  The cluster's two barriers and the exchange cost about
 // 2 us; a stage is 0.5 us of a unit's chain, and the contraction of 128 tokens, which the CTAs share too, 3 us at
 // 64 x 64 and 1 us at 32 x 32 (32 x 64 tokens of 256 + 256 columns, four stages, k = 32: 10.3 us alone, 11.3 in pairs;
-// 12 x 1 token of 128 + 2112, k = 44: 23.6 and 13.1 in eights).
-static int gradproj_ranks(long long units, int stages, int kmax) {
-  if (stages < 8 && kmax <= 32) return 1;
-  return units <= 16 ? 8 : units <= 34 ? 4 : units <= 74 ? 2 : 1;
+// 12 x 1 token of 128 + 2112, k = 44: 23.6 and 13.1 in eights).  Three or six, whose shares are
+// uneven, only from so many stages on (17 x 60 of 640 + 640, ten stages: 13.9 us in fours, 14.8 in sixes): 9 x 464 of 9792 + 4160
+// float32 154 us in pairs, 109 in threes, 20 x 100 of the same bf16 21.0 in fours, 16.9 in sixes.  Fives lost (24 units of 32
+// stages: 26.3 against 24.7 in fours).
+template <int KMAX, int kSrc, bool kEmb>
+static int gradproj_ranks(long long units, int stages, const DeviceState* ds) {
+  if ((stages < 8 && KMAX <= 32) || 2 * units > ds->sm_count) return 1;
+  for (const int r : {8, 6, 4, 3, 2}) {
+    if ((r == 6 && stages < 18) || (r == 3 && stages < 8)) continue;
+    if (r * units <= ds->sm_count && units <= gradproj_resident<KMAX, kSrc, kEmb, kSome>(r, ds)) return r;
+  }
+  return 1;
 }
 
 // CTAs of a cluster that takes all units of a sample and stores its result, or 1: units dealt over the GPU, results added to zeros.
 // A cluster wherever its CTAs get no more units than those would: it saves the zeroing, a launch of 2 us on the
 // host and on the GPU, and the additions (4 x 796 tokens of 192 bf16, embedding form: 15.9 -> 14.5 us; 32 x 512 of 1024 + 4096, k = 32:
-// 36.6 -> 34.9).  At most as many clusters as are resident at once: sixteen of eight were not (16 x 2048 of 1024, embedding
-// form: 20 against 36 us).
-static int gradproj_group(int B, int chunks, int sm_count) {
+// 36.6 -> 34.9), as long as all of them are resident (16 x 2048 of 1024, embedding form, in eights: 20 against 36 us).
+template <int KMAX, int kSrc, bool kEmb>
+static int gradproj_group(int B, int chunks, const DeviceState* ds) {
   if (chunks == 1) return 1;
-  const long long units = static_cast<long long>(B) * chunks, most = (units + sm_count - 1) / sm_count;
+  const long long units = static_cast<long long>(B) * chunks, most = (units + ds->sm_count - 1) / ds->sm_count;
   for (int c = 8; c > 1; c /= 2)
-    if (B <= (c == 8 ? 8 : c == 4 ? 32 : 72) && (chunks + c - 1) / c <= most) return c;
+    if (c * B <= ds->sm_count && (chunks + c - 1) / c <= most && B <= gradproj_resident<KMAX, kSrc, kEmb, kNone>(c, ds)) return c;
   return 1;
 }
 
@@ -722,8 +764,8 @@ template <int KMAX, int kSrc, bool kEmb>
 static int launch_gradproj_src(const GpOperands& o, GpParams& p, const DeviceState* ds, cudaStream_t st) {
   constexpr int kCols = GpCfg<KMAX, kSrc, kNone>::ATOMS * 64;
   const int stages = ceil_div(p.n_r, kCols) + (kEmb ? 0 : ceil_div(p.n_c, kCols));
-  const int ranks = gradproj_ranks(p.units, stages, KMAX);
-  p.group = ranks > 1 || p.accumulate ? 1 : gradproj_group(p.B, p.chunks_per_sample, ds->sm_count);
+  const int ranks = gradproj_ranks<KMAX, kSrc, kEmb>(p.units, stages, ds);
+  p.group = ranks > 1 || p.accumulate ? 1 : gradproj_group<KMAX, kSrc, kEmb>(p.B, p.chunks_per_sample, ds);
   // a sample's tokens are one CTA's or one cluster's: the results are stored, else added to zeros (written before the host
   // is busy with the tensor maps)
   p.direct = !p.accumulate && (p.chunks_per_sample == 1 || p.group > 1);
