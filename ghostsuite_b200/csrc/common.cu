@@ -31,6 +31,31 @@ int post_launch(const char* what) {
   return GHOST_OK;
 }
 
+__global__ void clear_kernel(float4* dst, long long quads, float* tail, int words) {
+  stream_order();
+  for (long long i = blockIdx.x * 256ll + threadIdx.x; i < quads; i += gridDim.x * 256ll) dst[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (blockIdx.x == 0 && static_cast<int>(threadIdx.x) < words) tail[threadIdx.x] = 0.f;
+}
+int clear_ahead(void* dst, size_t bytes, cudaStream_t st) {
+  cudaLaunchAttribute attr[1];
+  if (bytes == 0) return GHOST_OK;
+  if ((reinterpret_cast<uintptr_t>(dst) & 15u) != 0 || bytes % 4 != 0 || bytes > kClearMost || early_start(attr, st) == 0) {
+    GB_CUDA_OK(cudaMemsetAsync(dst, 0, bytes, st));
+    return GHOST_OK;
+  }
+  const long long quads = static_cast<long long>(bytes / 16);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(quads < 1024 ? 1 : quads < 1024 * 1184 ? (quads + 1023) / 1024 : 1184));
+  cfg.blockDim = dim3(256);
+  cfg.stream = st;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  GB_CUDA_OK(cudaLaunchKernelEx(&cfg, clear_kernel, static_cast<float4*>(dst), quads, static_cast<float*>(dst) + 4 * quads,
+                                static_cast<int>(bytes % 16 / 4)));
+  count_launch();
+  return post_launch("clear_kernel");
+}
+
 // The error word kernels write to.  One copy per device that loads the library.
 __device__ int g_kernel_error_word;
 

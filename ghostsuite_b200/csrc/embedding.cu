@@ -1019,7 +1019,7 @@ static int emb_pass(const EmbBuckets& q, const T* Gb, const T* Gv, int n_train, 
     GB_CUDA_OK(launch_next(emb_bucket_kernel, dim3(kEmbBucketCtas), dim3(kEmbBucketThreads), 0, st, q, M64, static_cast<long long>(n_val) * n_train));
     count_launch();
   } else {
-    GB_CUDA_OK(cudaMemsetAsync(q.totals, 0, 4 * (kEmbTotals + static_cast<long long>(q.vocab) * (M != nullptr ? 2 : 1)), st));
+    if (int rc = clear_ahead(q.totals, 4 * (kEmbTotals + static_cast<size_t>(q.vocab) * (M != nullptr ? 2 : 1)), st)) return rc;
     GB_CUDA_OK(launch_next(emb_count_kernel, dim3(blocks), dim3(256), 0, st, q, M64, static_cast<long long>(n_val) * n_train,
                            reinterpret_cast<uint4*>(out), quick ? out_bytes / 16 : 0ll));
     GB_CUDA_OK(launch_next(emb_alloc_kernel, dim3(ceil_div(q.vocab, 256)), dim3(256), 0, st, q));

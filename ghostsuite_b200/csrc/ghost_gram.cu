@@ -342,7 +342,8 @@ int gram_dot(const GramOperands& o, int n_train, int n_val, long long T, int rou
              static_cast<long long>(n_val) * T < (1ll << 31) - 256,
              "ghost_gram_dot_bf16: more than 2^31 tokens");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (!cleared) GB_CUDA_OK(cudaMemsetAsync(M_out, 0, sizeof(float) * static_cast<size_t>(n_val) * n_train, st));
+  if (!cleared)
+    if (int rc = clear_ahead(M_out, sizeof(float) * static_cast<size_t>(n_val) * n_train, st)) return rc;
   const long long rows_t = static_cast<long long>(n_train) * T, rows_v = static_cast<long long>(n_val) * T;
   // Rounds of tiles over the GPU times the cycles of a K step of a tile (128 for 256 x 256 on a pair and 128 x 256 on one
   // SM, 64 for 128 x 128, a tenth more for its operand traffic): 2048 x 1024 tokens are 32 tiles of 256 x 256 on 74

@@ -738,15 +738,17 @@ static int gradproj_ranks(long long units, int stages, const DeviceState* ds) {
 }
 
 // CTAs of a cluster that takes all units of a sample and stores its result, or 1: units dealt over the GPU, results added to zeros.
-// A cluster wherever its CTAs get no more units than those would: it saves the zeroing, a launch of 2 us on the
-// host and on the GPU, and the additions (4 x 796 tokens of 192 bf16, embedding form: 15.9 -> 14.5 us; 32 x 512 of 1024 + 4096, k = 32:
-// 36.6 -> 34.9), as long as all of them are resident (16 x 2048 of 1024, embedding form, in eights: 20 against 36 us).
+// A cluster saves the launch that zeroes and the additions (embedding form of bf16: 4 x 796 tokens of 192 11.6 -> 9.1 us, 32 x 256
+// of 768 11.6 -> 10.4; 12 x 900 of 256 + 512 11.0 -> 10.7) where each of its CTAs has a unit at most, all clusters are resident
+// (16 x 2048 of 1024, embedding form, in eights: 20 against 36 us) and a quarter of the SMs stays free: with the GPU full of
+// units the clusters come up later than CTAs do (64 x 256 of 768 + 768: 14.2 without, 14.7 with them; 32 x 512 of 1024 + 4096 34.3
+// and 34.7; 64 x 300 of 512, embedding form, 14.8 and 15.2).  The largest that fits: its CTAs share the storing (16 x 250 of
+// 320 + 320, k = 32, two units a sample: 10.8 in eights, 11.2 in pairs).
 template <int KMAX, int kSrc, bool kEmb>
 static int gradproj_group(int B, int chunks, const DeviceState* ds) {
-  if (chunks == 1) return 1;
-  const long long units = static_cast<long long>(B) * chunks, most = (units + ds->sm_count - 1) / ds->sm_count;
-  for (int c = 8; c > 1; c /= 2)
-    if (c * B <= ds->sm_count && (chunks + c - 1) / c <= most && B <= gradproj_resident<KMAX, kSrc, kEmb, kNone>(c, ds)) return c;
+  if (chunks == 1 || 4ll * B * chunks > 3ll * ds->sm_count) return 1;
+  for (int c = 8; c > 1 && c >= chunks; c /= 2)
+    if (c * B <= ds->sm_count && B <= gradproj_resident<KMAX, kSrc, kEmb, kNone>(c, ds)) return c;
   return 1;
 }
 
@@ -769,10 +771,13 @@ static int launch_gradproj_src(const GpOperands& o, GpParams& p, const DeviceSta
   // a sample's tokens are one CTA's or one cluster's: the results are stored, else added to zeros (written before the host
   // is busy with the tensor maps)
   p.direct = !p.accumulate && (p.chunks_per_sample == 1 || p.group > 1);
-  if (!p.accumulate && !p.direct)
-    GB_CUDA_OK(cudaMemset2DAsync(p.out, p.out_stride * sizeof(float), 0, static_cast<size_t>(p.k_r) * p.k_c * sizeof(float), p.B, st));
-  CUtensorMap tg = {}, tpr, ta = {}, tpc = {};
   int rc;
+  const size_t row = static_cast<size_t>(p.k_r) * p.k_c * sizeof(float);
+  if (!p.accumulate && !p.direct) {
+    if (p.out_stride * sizeof(float) != row) GB_CUDA_OK(cudaMemset2DAsync(p.out, p.out_stride * sizeof(float), 0, row, p.B, st));
+    else if ((rc = clear_ahead(p.out, row * p.B, st)) != GHOST_OK) return rc;
+  }
+  CUtensorMap tg = {}, tpr, ta = {}, tpc = {};
   // the projection matrices as one-sample 3-D operands, so that one TMA instruction form serves all four
   if ((rc = make_tmap_bf16_3d(&tpr, o.P_r, 1, p.k_r, o.pr_cols, o.ldpr, p.kr_pad)) != GHOST_OK) return rc;
   if (!kEmb && (rc = make_tmap_bf16_3d(&tpc, o.P_c, 1, p.k_c, o.pc_cols, o.ldpc, p.kc_pad)) != GHOST_OK) return rc;

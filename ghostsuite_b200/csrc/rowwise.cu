@@ -808,9 +808,9 @@ extern "C" int ghost_split_operands(const void* X, int x_is_f32, int x_cols, con
   fill(p.job[0], X, x_is_f32, x_cols, X_out, x_sums);
   fill(p.job[1], Y, y_is_f32, y_cols, Y_out, y_sums);
   // The chunks of a sample add their sums up as a cluster, of up to eight; sums of both operands, or of more chunks, are added
-  // to zeros, whose memset is a launch: 2 us where the host bounds the hook (10 x 512 of (256, 256) float32 46.3 -> 43.1, 34 x 127
-  // of (126, 640) 44.2 -> 42.8).  Large operands keep it: clusters walk down a panel where blocks on their own read along
-  // the rows (29 x 197 of (768, 1000), 41 MB: 79.2 against 80.6).
+  // to zeros, which take a launch: 3 us or more where the host bounds the hook (10 x 512 of (256, 256) float32 44.9 -> 41.2, 34 x 127
+  // of (126, 640) 44.7 -> 40.9).  Large operands keep it: clusters walk down a panel where blocks on their own read along
+  // the rows (29 x 197 of (768, 1000), 41 MB: 77.6 against 80.3; 30 x 200 of (500, 700), 29 MB: 47.6 against 50.0).
   const int summed = p.job[0].sums ? 0 : 1;
   const bool both = p.job[0].sums && p.job[1].sums;
   double read = 0.;
@@ -820,7 +820,7 @@ extern "C" int ghost_split_operands(const void* X, int x_is_f32, int x_cols, con
     j.ranks = j.sums ? ranks : 1;
     j.blocks = (j.used + ranks - 1) / ranks * ranks;
     if (j.sums && j.chunks > 1 && ranks == 1)
-      GB_CUDA_OK(cudaMemsetAsync(j.sums, 0, sizeof(float) * static_cast<size_t>(samples) * j.cols, st));
+      if (int rc = clear_ahead(j.sums, sizeof(float) * static_cast<size_t>(samples) * j.cols, st)) return rc;
   }
   const long long blocks = p.job[0].blocks + p.job[1].blocks;
   GB_REQUIRE(blocks < (1ll << 31), "ghost_split_operands: too many rows");
@@ -838,13 +838,14 @@ extern "C" int ghost_colsum(const void* G, int is_f32, int N, long long T, int c
   GB_REQUIRE(N > 0 && T > 0 && cols > 0 && N <= 65535, "ghost_colsum: bad dimensions");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int cblocks = ceil_div(cols, 256);
-  // Up to eight splits are a cluster that adds up their sums (6 x 512 rows of 768 bf16, the hook: 45.4 -> 43.1 us, the host's); more, of
-  // longer samples, add to zeros, and so do large operands (6 x 512 of 3072: 52.1 against 52.6).
+  // Up to eight splits are a cluster that adds up their sums (6 x 512 rows of 768 bf16, the hook: 45.1 -> 41.3 us, the host's); more, of
+  // longer samples, add to zeros, and so do large operands (6 x 512 of 3072: 50.4 against 51.5).
   const bool small = static_cast<double>(N) * T * cols * (is_f32 ? 4 : 2) <= kClusterBytes;
   int splits = pick_splits(T, static_cast<long long>(cblocks) * N, ds->sm_count, 64);
   if (small && splits > 8 && T <= 8 * 128) splits = 8;
   const int ranks = small && splits <= 8 ? splits : 1;
-  if (splits > ranks) GB_CUDA_OK(cudaMemsetAsync(out, 0, sizeof(float) * static_cast<size_t>(N) * cols, st));
+  if (splits > ranks)
+    if (int rc = clear_ahead(out, sizeof(float) * static_cast<size_t>(N) * cols, st)) return rc;
   const dim3 grid(cblocks, splits, N), cluster(1, ranks, 1);
   if (is_f32) GB_CUDA_OK(launch_next_cluster(cluster, colsum_kernel<float>, grid, dim3(256), 0, st, static_cast<const float*>(G), T, cols, ld, out, splits, ranks > 1 ? 1 : 0));
   else GB_CUDA_OK(launch_next_cluster(cluster, colsum_kernel<__nv_bfloat16>, grid, dim3(256), 0, st, static_cast<const __nv_bfloat16*>(G), T, cols, ld, out, splits, ranks > 1 ? 1 : 0));

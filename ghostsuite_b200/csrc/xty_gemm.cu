@@ -545,8 +545,8 @@ static int wgrad(const XtyOperands& o, long long n_rows, float scale, int accumu
   const int splits = pair ? pick_k_splits(static_cast<long long>(ceil_div(m_cols, 256)) * p.n_tiles, ds->sm_count / 2, kb_pair, 32,
                                           elems, out_is_f32 != 0)
                           : pick_k_splits(tiles, ds->sm_count, kb, 64, elems, out_is_f32 != 0);
-  if (splits > 1) GB_CUDA_OK(cudaMemsetAsync(ws, 0, static_cast<size_t>(m_cols) * p.ld_acc * 4, st));
-  else p.mode = kEpiDirect;
+  if (splits == 1) p.mode = kEpiDirect;
+  else if ((rc = clear_ahead(ws, static_cast<size_t>(m_cols) * p.ld_acc * 4, st)) != GHOST_OK) return rc;
   if (pair) {
     rc = launch_xty_pair_wgrad(o, n_rows, splits, p.acc_ws, p.ld_acc, out, out_is_f32, scale, accumulate, zero, zero_n, ds, st);
   } else {
@@ -820,7 +820,7 @@ extern "C" int ghost_tile_dot_bf16(const void* V, int v_ranks, int v_per_rank, c
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int n_tiles_n = ceil_div(n_cols, XtyCfg<1>::BN);
   const long long tiles = static_cast<long long>(ceil_div(m_cols, XtyCfg<1>::BM)) * n_tiles_n;
-  GB_CUDA_OK(cudaMemsetAsync(M_out, 0, sizeof(float) * static_cast<size_t>(n_val) * n_train, st));
+  if (int rc = clear_ahead(M_out, sizeof(float) * static_cast<size_t>(n_val) * n_train, st)) return rc;
   return launch_tile_dot(V, n_val, 0, W, n_train, 0, tiles, n_val, n_train, 0, n_train, dot_scale, M_out, nullptr, 1,
                          grad_out, grad_is_f32, grad_accumulate, m_cols, n_cols, n_tiles_n, grad_scale, ds, st,
                          v_per_rank);

@@ -27,8 +27,7 @@ struct XtyColsum {
 // Zeroes the sums of a launch's samples where several of its units add to each
 inline int xty_colsum_clear(const XtyColsum& cs, int parts, int sample0, int samples, int cols, cudaStream_t st) {
   if (cs.of == 0 || parts == 1) return GHOST_OK;
-  GB_CUDA_OK(cudaMemsetAsync(cs.out + static_cast<long long>(sample0) * cols, 0, sizeof(float) * static_cast<size_t>(samples) * cols, st));
-  return GHOST_OK;
+  return clear_ahead(cs.out + static_cast<long long>(sample0) * cols, sizeof(float) * static_cast<size_t>(samples) * cols, st);
 }
 
 // Map of operand i for boxes of `rows_box` tokens and `blocks` 64-column blocks (both parts of a split operand)

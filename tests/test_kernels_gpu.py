@@ -1359,6 +1359,36 @@ def test_projection_similarity_routes(n1, n2, D, dtype):
         assert (S[:, n2:] == 7.0).all()
 
 
+# one to three words past the last sixteen bytes and none, results off sixteen bytes, both sides of 8 MB of operands
+@pytest.mark.parametrize("offset", [0, 1, 4])
+@pytest.mark.parametrize("n1,n2,D", [(3, 7, 250000), (5, 18, 90001), (9, 11, 100008), (16, 32, 20000), (31, 45, 300008)])
+def test_projection_similarity_over_old_values(n1, n2, D, offset):
+    """Scores that several blocks add up: what was there does not count, and nothing beside them is written."""
+    from ghostsuite_b200 import _lib
+    lib, stream = _lib.load(), torch.cuda.current_stream().cuda_stream
+    g = torch.Generator(device="cuda").manual_seed(31)
+    a, b = (torch.randn(n, D, generator=g, device="cuda") for n in (n1, n2))
+    buf = torch.full((n1 * n2 + 16,), float("nan"), device="cuda")
+    S = buf[offset:offset + n1 * n2]
+    for _ in range(2):
+        _lib.check(lib.ghost_projection_similarity(a.data_ptr(), b.data_ptr(), 1, n1, n2, D, D, D, 1.0, S.data_ptr(), n2, stream))
+    after()
+    bound = 2.0 ** -15 * a.double().norm(dim=1)[:, None] * b.double().norm(dim=1)[None]
+    assert ((S.view(n1, n2).double() - a.double() @ b.double().t()).abs() <= bound).all()
+    assert int(buf.isnan().sum()) == 16
+
+
+# 8, 17, 21 and 34 MB of split sums: one round of the blocks that clear them, several, and a memset
+@pytest.mark.parametrize("m,n", [(1024, 2048), (2048, 2048), (2048, 2560), (2048, 4160)])
+def test_wgrad_split_sums_over_old_values(m, n):
+    g = torch.Generator(device="cuda").manual_seed(32)
+    X, Y = (torch.randn(1, 6000, c, generator=g, device="cuda").bfloat16() for c in (m, n))
+    for scale in (1.0, 0.25):
+        out = ops().wgrad(X, Y, scale, torch.float32)
+        after()
+        assert O.rel_fro(out, scale * (X[0].double().t() @ Y[0].double())) < 1e-5      # exact products, float32 sums
+
+
 # rows of which 32, 16, 8, four and more than a whole draw's bytes are drawn at once; tables of a part of a draw, one and many
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("d", [8, 384, 392, 1544, 6152])
