@@ -240,7 +240,6 @@ constexpr int kEmbHotCap = 256;
 constexpr int kEmbTotals = 12;
 constexpr int kEmbChunk = 8;             // train rows of a join item
 constexpr int kEmbValChunk = 32;         // validation rows of a join item
-constexpr int kEmbBucketTokens = 8192;   // largest batch of emb_bucket_kernel
 
 // Counting hands every token its place in the bucket, so filling needs no second round of atomics.
 __device__ __forceinline__ void emb_count_tokens(const EmbBuckets& q, long long first, long long step) {
@@ -362,14 +361,14 @@ __global__ void __launch_bounds__(256) emb_fill_kernel(const EmbBuckets q) {
 // All of it for a small batch in one launch, zeroing included: one cluster with a thread for each token, whose barriers part the
 // steps.  Instead of the whole table it looks at the ids that occur: the first token of an id (the first validation token of
 // one without train tokens) allocates it, and of the validation counts only those of ids that occur are cleared (the train
-// counts all: the gradient's empty rows are found by them).  The GPU takes about as long as for the three kernels and the memset, whose
-// launches bounded the host: hooks of up to 5000 tokens 39 - 41 -> 30 us where the host bounds them (8 + 2 x 41 tokens of 320 bf16,
-// vocabulary 36761), 8 + 2 x 512 of 768, 50304: 53.6 -> 51.1.  A thread for two tokens, 16384 of them: 53.9 -> 62.
-constexpr int kEmbBucketCtas = 8, kEmbBucketThreads = kEmbBucketTokens / kEmbBucketCtas;
-__global__ void __cluster_dims__(kEmbBucketCtas, 1, 1) __launch_bounds__(kEmbBucketThreads)
+// counts all: the gradient's empty rows are found by them).  TOKENS is the largest batch, 4096 or 8192 (emb_one_cluster).
+constexpr int kEmbBucketCtas = 8;
+template <int TOKENS>
+__global__ void __cluster_dims__(kEmbBucketCtas, 1, 1) __launch_bounds__(TOKENS / kEmbBucketCtas)
 emb_bucket_kernel(const EmbBuckets q, double* __restrict__ M64, long long m_size) {
+  constexpr int kThreads = TOKENS / kEmbBucketCtas;
   stream_order();
-  const int j = blockIdx.x * kEmbBucketThreads + threadIdx.x, n_b = static_cast<int>(q.first_val);
+  const int j = blockIdx.x * kThreads + threadIdx.x, n_b = static_cast<int>(q.first_val);
   const bool train = j < n_b;
   int id = -1;
   if (j < q.n_tok) {
@@ -382,18 +381,29 @@ emb_bucket_kernel(const EmbBuckets q, double* __restrict__ M64, long long m_size
     }
   }
   const int zero = kEmbTotals + q.vocab;               // totals and train counts lie behind each other
-  for (int i = j; i < zero / 4; i += kEmbBucketTokens) reinterpret_cast<uint4*>(q.totals)[i] = make_uint4(0u, 0u, 0u, 0u);
+  for (int i = j; i < zero / 4; i += TOKENS) reinterpret_cast<uint4*>(q.totals)[i] = make_uint4(0u, 0u, 0u, 0u);
   if (j < (zero & 3)) q.totals[(zero & ~3) + j] = 0;
   if (M64 != nullptr)
-    for (long long i = j; i < m_size; i += kEmbBucketTokens) M64[i] = 0.;
+    for (long long i = j; i < m_size; i += TOKENS) M64[i] = 0.;
   cluster_sync_all();
   const int rank = id >= 0 ? atomicAdd((train ? q.cnt_b : q.cnt_v) + id, 1) : -1;
   cluster_sync_all();
-  emb_alloc_ids<kEmbBucketThreads / 32>(q, id, rank == 0 && (train || q.cnt_b[id] == 0));
+  emb_alloc_ids<kThreads / 32>(q, id, rank == 0 && (train || q.cnt_b[id] == 0));
   cluster_sync_all();
   if (id < 0) return;
   if (train) q.perm_b[q.off_b[id] + rank] = j;
   else q.perm_v[q.off_v[id] + rank] = j - n_b;
+}
+
+// Tokens of the cluster's kernel that a batch takes, 0: the three kernels behind a cleared table of counts.  Their launches bound
+// the host, and up to 4096 tokens the cluster is as fast on the GPU (three kernels and the cluster, hooks of bf16, us: 8 + 2 x 41 tokens of
+// 320, vocabulary 36761, 38.9 and 31.3; 12 + 4 x 250 of 768, 50304, text ids 51.2 and 46.7, uniform 39.1 and 34.7; 8 + 2 x 200 the same,
+// text ids, 41.2 and 42.2).  Up to 8192, with twice the threads, it is the slower one on the GPU, so that is for tables whose
+// gradient is written in less time than the host takes (12 + 4 x 330 of 256, 50304: 39.2 and 31.1; 2 + 1 x 2000 of 1024, 8000: 39.1 and 32.9;
+// 8 + 2 x 512 of 768, 50304, 50.7 and 52.4).  A thread for two tokens, 16384 of them: 53.9 and 62.
+static int emb_one_cluster(long long tokens, double table_bytes) {
+  if (tokens <= 4096) return 4096;
+  return tokens <= 8192 && table_bytes <= 32e6 ? 8192 : 0;
 }
 
 // ---------------------------------------------------------------- dot product: join by id
@@ -1015,8 +1025,10 @@ static int emb_pass(const EmbBuckets& q, const T* Gb, const T* Gv, int n_train, 
   if (fill && !by_rows && !quick) GB_CUDA_OK(cudaMemsetAsync(out, 0, out_bytes, st));
   const int tokens = blocks;
   if (quick) blocks = ds->sm_count * 8;
-  if (q.n_tok <= kEmbBucketTokens && !quick) {
-    GB_CUDA_OK(launch_next(emb_bucket_kernel, dim3(kEmbBucketCtas), dim3(kEmbBucketThreads), 0, st, q, M64, static_cast<long long>(n_val) * n_train));
+  const int one = quick ? 0 : emb_one_cluster(q.n_tok, static_cast<double>(out_bytes));
+  if (one > 0) {
+    GB_CUDA_OK(launch_next(one == 4096 ? emb_bucket_kernel<4096> : emb_bucket_kernel<8192>, dim3(kEmbBucketCtas), dim3(one / kEmbBucketCtas), 0, st,
+                           q, M64, static_cast<long long>(n_val) * n_train));
     count_launch();
   } else {
     if (int rc = clear_ahead(q.totals, 4 * (kEmbTotals + static_cast<size_t>(q.vocab) * (M != nullptr ? 2 : 1)), st)) return rc;

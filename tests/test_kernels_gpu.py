@@ -1165,10 +1165,10 @@ def test_embedding_hook_small_rows_exact(dtype, n_t, n_v, d):
     assert torch.equal(grad.cpu(), (per[:n_t].sum(0).to(dtype) / n_t).to(dtype))
 
 
-# tokens around what one cluster buckets (8192) and around a warp; the table larger and smaller than them, ids of one side
+# tokens around what one cluster buckets (4096, 8192) and around a warp; the table larger and smaller than them, ids of one side
 # only, ids that most tokens share, ids outside of the table
 @pytest.mark.parametrize("n_t,n_v,T,vocab", [(1, 1, 1, 1), (3, 2, 13, 5), (7, 1, 1024, 300), (6, 2, 1024, 50000), (3, 1, 2048, 7),
-                                             (2731, 1, 3, 900), (4, 4, 1023, 20001), (1, 5, 700, 64)])
+                                             (2731, 1, 3, 900), (4, 4, 1023, 20001), (1, 5, 700, 64), (3, 1, 1024, 9000), (16, 1, 241, 77)])
 def test_embedding_buckets_of_one_cluster(n_t, n_v, T, vocab):
     from ghostsuite_b200 import _lib
     gen = torch.Generator().manual_seed(T)
