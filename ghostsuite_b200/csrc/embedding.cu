@@ -380,9 +380,10 @@ emb_bucket_kernel(const EmbBuckets q, double* __restrict__ M64, long long m_size
       atomicExch(q.err, kErrBadIndex);
     }
   }
-  const int zero = kEmbTotals + q.vocab;               // totals and train counts lie behind each other
-  for (int i = j; i < zero / 4; i += TOKENS) reinterpret_cast<uint4*>(q.totals)[i] = make_uint4(0u, 0u, 0u, 0u);
-  if (j < (zero & 3)) q.totals[(zero & ~3) + j] = 0;
+  // totals and train counts lie behind each other; with a table of nearly 2^31 rows they are more words than an int counts
+  const long long zero = kEmbTotals + static_cast<long long>(q.vocab);
+  for (long long i = j; i < zero / 4; i += TOKENS) reinterpret_cast<uint4*>(q.totals)[i] = make_uint4(0u, 0u, 0u, 0u);
+  if (j < (zero & 3)) q.totals[(zero & ~3ll) + j] = 0;
   if (M64 != nullptr)
     for (long long i = j; i < m_size; i += TOKENS) M64[i] = 0.;
   cluster_sync_all();

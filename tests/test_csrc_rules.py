@@ -82,3 +82,11 @@ def test_alignment_slack_of_the_shared_memory_is_not_used():
             placed += 1
             assert "1024" not in m.group(0), f"{name}: {m.group(0)}"
     assert placed > 20
+
+
+def test_words_of_an_embedding_table_are_counted_in_64_bits():
+    """A table may have up to 2^31 - 1 rows; its counts and the totals before them are more words than that."""
+    sums = [line for line in _sources()["embedding.cu"].splitlines() if "vocab" in line and re.search(r"kEmbTotals \+|\+ kEmbTotals", line)]
+    assert len(sums) >= 4
+    for line in sums:
+        assert re.search(r"static_cast<(long long|size_t)>\(\w*\.?vocab\)", line), line

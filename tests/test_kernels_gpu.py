@@ -1197,6 +1197,29 @@ def test_embedding_buckets_of_one_cluster(n_t, n_v, T, vocab):
         assert torch.equal(grad.cpu(), (gref.float() / n_t))
 
 
+@pytest.mark.parametrize("n_t,n_v,T", [(3, 2, 40), (5, 1, 1024)])
+def test_embedding_dot_of_the_largest_table(n_t, n_v, T):
+    """2^31 - 1 rows: the counts and the totals before them are more words than an int counts, and all of them are
+    cleared, whatever the workspace (34 GB) held."""
+    from ghostsuite_b200 import _lib
+    lib, vocab, d = _lib.load(), 2 ** 31 - 1, 8
+    g = torch.Generator().manual_seed(T)
+    ids = torch.randint(0, 60, (n_t + n_v, T), generator=g)
+    ids[ids >= 30] += vocab - 60
+    G = torch.randint(-3, 4, (n_t + n_v, T, d), generator=g).float()
+    same = (ids[n_t:, None, :, None] == ids[None, :n_t, None, :]).double()
+    ref = torch.einsum("vbst,vsd,btd->vb", same, G[n_t:].double(), G[:n_t].double())
+    size = int(lib.ghost_embedding_pass_workspace_bytes(n_t, n_v, T, vocab, d))
+    ws = torch.full((size,), 0x5b, dtype=torch.uint8, device="cuda")
+    M, ids_d, G_d = torch.full((n_v, n_t), float("nan"), device="cuda"), ids.cuda(), G.cuda()
+    _lib.check(lib.ghost_embedding_dot(ids_d.data_ptr(), G_d.data_ptr(), 1, n_t, n_v, T, d, vocab, 1.0, M.data_ptr(), ws.data_ptr(), size,
+                                       torch.cuda.current_stream().cuda_stream))
+    after()
+    del ws
+    torch.cuda.empty_cache()
+    assert torch.equal(M.cpu().double(), ref)          # whole numbers: exact in any order
+
+
 # widths around the lines of the block-per-rows kernel (1024, 2048, 4096, 8192, multiples of eight or not), row
 # counts that leave a group of rows unfinished, one row, several splits
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
