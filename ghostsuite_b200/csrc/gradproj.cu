@@ -468,7 +468,7 @@ gradproj_kernel(const __grid_constant__ CUtensorMap tm_g, const __grid_constant_
           o[i][j] = o[i][j + 1] = o[i][j + 2] = o[i][j + 3] = 0.f;
         }
       if (ranks > 1) cluster_sync_all();
-      else asm volatile("bar.sync 1, 128;" ::: "memory");
+      else named_bar_sync(1, 128);
       float* dst = p.out + static_cast<long long>(b) * p.out_stride;
 #pragma unroll 1
       for (int e = static_cast<int>(rank) * 128 + tid; e < p.k_r * KMAX; e += static_cast<int>(ranks) * 128) {
@@ -480,7 +480,7 @@ gradproj_kernel(const __grid_constant__ CUtensorMap tm_g, const __grid_constant_
         }
         dst[static_cast<long long>(e / KMAX) * p.out_ld + e % KMAX] = sum * p.scale;
       }
-      if (ranks == 1) asm volatile("bar.sync 1, 128;" ::: "memory");
+      if (ranks == 1) named_bar_sync(1, 128);
     };
     // TMEM -> shared (fp32): row `tid` of one projected block
     auto stage_block = [&](uint32_t taddr, int kpad, float* dst) {
@@ -589,7 +589,7 @@ gradproj_kernel(const __grid_constant__ CUtensorMap tm_g, const __grid_constant_
         };
         add_up(s_r, p.kr_pad, true);
         if (!kEmb) add_up(s_c, p.kc_pad, false);
-        asm volatile("bar.sync 1, 128;" ::: "memory");
+        named_bar_sync(1, 128);
         contract(first, first + share);
         if constexpr (kCluster == kSome) flush(b);
       }
@@ -626,9 +626,9 @@ gradproj_kernel(const __grid_constant__ CUtensorMap tm_g, const __grid_constant_
           __syncwarp();
           if (lane == 0) mbar_arrive(&acc_empty[acc]);     // four arrivals per tile, one per warp
         }
-        asm volatile("bar.sync 1, 128;" ::: "memory");     // the four epilogue warps only
+        named_bar_sync(1, 128);     // the four epilogue warps only
         contract(0, Cfg::kStageRows);
-        asm volatile("bar.sync 1, 128;" ::: "memory");
+        named_bar_sync(1, 128);
       }
       if (++acc == 2) { acc = 0; acc_phase ^= 1; }
     }

@@ -115,9 +115,13 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity,
   const bool ok = mbar_wait(bar, parity, abort_flag, err, code);
   return __all_sync(0xffffffffu, ok);
 }
+// Barriers for whole warps (bar and barrier.cluster.*.aligned): all lanes of a warp have to enter them together, also behind
+// a loop or a condition that parted them, so each brings the warp together first.
+//
 // Named barrier over `nthreads` threads that also ANDs a predicate across them.
 __device__ __forceinline__ bool named_bar_and(int id, int nthreads, bool pred) {
   uint32_t r;
+  __syncwarp();
   asm volatile(
       "{\n"
       " .reg .pred P, Q;\n"
@@ -189,6 +193,7 @@ template <int N> __device__ __forceinline__ void bulk_wait_group() {
   asm volatile("cp.async.bulk.wait_group %0;" ::"n"(N) : "memory");
 }
 __device__ __forceinline__ void named_bar_sync(int id, int nthreads) {
+  __syncwarp();
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }
 __device__ __forceinline__ void st_shared_v4(void* p, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
@@ -271,6 +276,7 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 __device__ __forceinline__ void cluster_sync_all() {
+  __syncwarp();
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }

@@ -290,7 +290,7 @@ tile_dot_f32_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_const
           }
         }
       }
-      asm volatile("bar.sync 2, 256;" ::: "memory");
+      named_bar_sync(2, 256);
       for (int idx = threadIdx.x; idx < TR * VR; idx += 256) {
         const int b = idx % TR, v = idx / TR;
         const float* from = s_red + v / WR * (8 / WP) * (TR * WR) + v % WR * TR + b;
@@ -300,7 +300,7 @@ tile_dot_f32_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_const
         if (v0 + v < p.n_val && j0 + b < p.n_grp && t != 0.f)
           atomicAdd(&p.M[static_cast<long long>(v0 + v) * p.n_train + p.b0 + j0 + b], t * p.scale);
       }
-      asm volatile("bar.sync 2, 256;" ::: "memory");
+      named_bar_sync(2, 256);
     }
   }
 }
@@ -565,7 +565,7 @@ tile_dot_mma_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_const
                 *slot = turn ? *slot + acc[mt][nt][e] : acc[mt][nt][e];
               }
         }
-        asm volatile("bar.sync 2, %0;" ::"n"(kWarps * 32) : "memory");
+        named_bar_sync(2, kWarps * 32);
       }
       for (int idx = threadIdx.x; idx < TR * VR; idx += kWarps * 32) {
         float t = 0.f;
@@ -575,7 +575,7 @@ tile_dot_mma_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_const
         if (v < p.n_val && b < p.n_grp && t != 0.f)
           atomicAdd(&p.M[static_cast<long long>(v) * p.n_train + p.b0 + b], t * p.scale);
       }
-      asm volatile("bar.sync 2, %0;" ::"n"(kWarps * 32) : "memory");
+      named_bar_sync(2, kWarps * 32);
     }
   }
 }

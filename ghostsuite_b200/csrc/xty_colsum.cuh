@@ -28,7 +28,7 @@ __device__ __forceinline__ void xty_colsum_finish(const float (&a)[8], int cbase
   const int cv = ct & 15, rl = ct >> 4;
 #pragma unroll
   for (int j = 0; j < 8; ++j) red[rl * 128 + cv * 8 + j] = a[j];
-  asm volatile("bar.sync %0, 128;" ::"r"(bar_id) : "memory");
+  named_bar_sync(bar_id, 128);
   float sum = 0.f;
 #pragma unroll
   for (int r = 0; r < 8; ++r) sum += red[r * 128 + ct];
@@ -36,7 +36,7 @@ __device__ __forceinline__ void xty_colsum_finish(const float (&a)[8], int cbase
     if (alone) out[cbase + ct] = sum;
     else if (sum != 0.f) atomicAdd(out + cbase + ct, sum);
   }
-  asm volatile("bar.sync %0, 128;" ::"r"(bar_id) : "memory");
+  named_bar_sync(bar_id, 128);
 }
 
 // Sums rows of columns [cbase, cbase + 128) of `src` (row pitch ld, 16-byte aligned, rows readable up to

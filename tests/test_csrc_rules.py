@@ -90,3 +90,16 @@ def test_words_of_an_embedding_table_are_counted_in_64_bits():
     assert len(sums) >= 4
     for line in sums:
         assert re.search(r"static_cast<(long long|size_t)>\(\w*\.?vocab\)", line), line
+
+
+def test_barriers_of_whole_warps_bring_the_warp_together():
+    """``bar`` and ``barrier.cluster.*.aligned`` must be entered by all lanes of a warp at once: they stand in functions that
+    see to it, and nowhere else."""
+    sources = _sources()
+    for name in ("named_bar_and", "named_bar_sync", "cluster_sync_all"):
+        text = sources["sm100_ptx.cuh"]
+        body = _body(text, re.search(r"\b%s\([^)]*\) \{" % name, text).start())
+        assert "__syncwarp();" in body[:body.index("asm")], name
+        sources["sm100_ptx.cuh"] = text.replace(body, "{}")
+    for name, text in sources.items():
+        assert not re.search(r"\bbar\.(sync|red|arrive)|\bbarrier\.cluster", text), name
