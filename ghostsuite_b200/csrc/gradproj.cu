@@ -438,7 +438,6 @@ gradproj_kernel(const __grid_constant__ CUtensorMap tm_g, const __grid_constant_
     for (int i = 0; i < RT; ++i)
 #pragma unroll
       for (int j = 0; j < CT; ++j) o[i][j] = 0.f;
-    int cur_b = -1;
     int acc = 0; uint32_t acc_phase = 0;
     const uint32_t lane_base = static_cast<uint32_t>(warp * 32) << 16;
 
@@ -567,7 +566,6 @@ gradproj_kernel(const __grid_constant__ CUtensorMap tm_g, const __grid_constant_
             for (int q = 0; q < kRowQuads; ++q) *reinterpret_cast<float4*>(&s_c[gp_staged_index<KMAX>(tid, 4 * q)]) = mine[q];
         }
       }
-      __syncwarp();
       cluster_sync_all();
       if (alive) {
         // ranks [0, last_r] hold columns of G, [first_c, ranks) columns of A
@@ -593,55 +591,57 @@ gradproj_kernel(const __grid_constant__ CUtensorMap tm_g, const __grid_constant_
         contract(first, first + share);
         if constexpr (kCluster == kSome) flush(b);
       }
-      __syncwarp();
       if constexpr (kCluster == kWhole) store(b);
     }
-    bool alive = true;
-    for (long long u = u0; u < u1 && kCluster == kNone; ++u) {
-      const int b = static_cast<int>(u / p.chunks_per_sample);
-      if (b != cur_b) {
-        if (cur_b >= 0) {
-          if (p.direct) store(cur_b);
-          else flush(cur_b);
-        }
-        cur_b = b;
-      }
-      if constexpr (kEmb) gather(b, u % p.chunks_per_sample * BM + tid);
-      if (!named_bar_and(2, 128, mbar_wait(&acc_full[acc], acc_phase, abort_flag, p.err, 124))) { alive = false; break; }
-      tc_fence_after_sync();
-      const uint32_t t_r = tmem_base + lane_base + acc * 256;
-      // two halves of 64 tokens: warps 0-1 own TMEM lanes 0-63, warps 2-3 lanes 64-127
+    // (one place that stores or adds and no wide counters: with two places the embedding form of float32 and unaligned rows spilled
+    // more registers, 237 us for 16 x 2048 tokens of 4000 float32, k = 64, and 200 as it is; 65 and 59 for 701)
+    if constexpr (kCluster == kNone) {
+      bool alive = true;
+      int b = static_cast<int>(u0 / p.chunks_per_sample);
+      int chunk = static_cast<int>(u0 % p.chunks_per_sample);
+      // a cluster's CTA without a unit takes part in the storing too
 #pragma unroll 1
-      for (int half = 0; half < 2; ++half) {
-        if ((warp >> 1) == half) {
-          stage_block(t_r, p.kr_pad, s_r);
-          if constexpr (kEmb) {
+      for (long long left = u1 - u0; left > 0 || p.group > 1; --left) {
+        if (left > 0) {
+          if constexpr (kEmb) gather(b, static_cast<long long>(chunk) * BM + tid);
+          if (!named_bar_and(2, 128, mbar_wait(&acc_full[acc], acc_phase, abort_flag, p.err, 124))) { alive = false; break; }
+          tc_fence_after_sync();
+          const uint32_t t_r = tmem_base + lane_base + acc * 256;
+          // two halves of 64 tokens: warps 0-1 own TMEM lanes 0-63, warps 2-3 lanes 64-127
+#pragma unroll 1
+          for (int half = 0; half < 2; ++half) {
+            if ((warp >> 1) == half) {
+              stage_block(t_r, p.kr_pad, s_r);
+              if constexpr (kEmb) {
 #pragma unroll
-            for (int q = 0; q < kRowQuads; ++q)
-              *reinterpret_cast<float4*>(&s_c[gp_staged_index<KMAX>(tid & 63, 4 * q)]) = mine[q];
-          } else {
-            stage_block(t_r + 128, p.kc_pad, s_c);
+                for (int q = 0; q < kRowQuads; ++q)
+                  *reinterpret_cast<float4*>(&s_c[gp_staged_index<KMAX>(tid & 63, 4 * q)]) = mine[q];
+              } else {
+                stage_block(t_r + 128, p.kc_pad, s_c);
+              }
+              tc_fence_before_sync();
+              __syncwarp();
+              if (lane == 0) mbar_arrive(&acc_empty[acc]);     // four arrivals per tile, one per warp
+            }
+            named_bar_sync(1, 128);                            // the four epilogue warps only
+            contract(0, Cfg::kStageRows);
+            named_bar_sync(1, 128);
           }
-          tc_fence_before_sync();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&acc_empty[acc]);     // four arrivals per tile, one per warp
+          if (++acc == 2) { acc = 0; acc_phase ^= 1; }
         }
-        named_bar_sync(1, 128);     // the four epilogue warps only
-        contract(0, Cfg::kStageRows);
-        named_bar_sync(1, 128);
+        if (++chunk == p.chunks_per_sample || left <= 1) {     // done with the sample, or with this CTA's part of it
+          if (p.direct) store(b);
+          else flush(b);
+          if (p.group > 1) break;
+          chunk = 0;
+          ++b;
+        }
       }
-      if (++acc == 2) { acc = 0; acc_phase ^= 1; }
-    }
-    if (kCluster == kNone && p.group > 1) cur_b = static_cast<int>(blockIdx.x / ranks);      // a CTA without units takes part too
-    if (kCluster == kNone && (p.group > 1 || (alive && cur_b >= 0))) {
-      __syncwarp();
-      if (p.direct) store(cur_b);
-      else flush(cur_b);
+      if (!alive && p.group > 1) cluster_sync_all();           // the one that the others wait at in store()
     }
   }
 
   if (kCluster != kNone || p.group > 1) {
-    __syncwarp();
     if (warp >= 4) {
       if constexpr (kCluster != kNone) cluster_sync_all();        // the epilogue's barrier before the partial blocks are added up
       if (kCluster != kSome) cluster_sync_all();                  // and the one before the results are
