@@ -712,7 +712,7 @@ static int gradproj_resident(int ranks, const DeviceState* ds) {
     if (cudaFuncSetAttribute(gradproj_kernel<KMAX, kSrc, kEmb, kCluster>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes) != cudaSuccess ||
         cudaOccupancyMaxActiveClusters(&count, gradproj_kernel<KMAX, kSrc, kEmb, kCluster>, &cfg) != cudaSuccess) {
       (void)cudaGetLastError();
-      count = 0;
+      return 0;                              // no cluster for this call; the next one asks again
     }
     n = count + 1;
     slot.store(n, std::memory_order_relaxed);

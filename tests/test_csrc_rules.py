@@ -103,3 +103,12 @@ def test_barriers_of_whole_warps_bring_the_warp_together():
         sources["sm100_ptx.cuh"] = text.replace(body, "{}")
     for name, text in sources.items():
         assert not re.search(r"\bbar\.(sync|red|arrive)|\bbarrier\.cluster", text), name
+
+
+def test_a_count_that_the_driver_refused_is_not_kept():
+    """How many clusters are resident is asked once per kernel and device, unless the question failed."""
+    text = _sources()["gradproj.cu"]
+    body = _body(text, text.index("gradproj_resident(int ranks"))
+    refused = _body(body, body.index("cudaOccupancyMaxActiveClusters"))
+    assert "return 0;" in refused and "store" not in refused
+    assert body.index(refused) < body.index("slot.store(")
