@@ -396,15 +396,26 @@ emb_bucket_kernel(const EmbBuckets q, double* __restrict__ M64, long long m_size
   else q.perm_v[q.off_v[id] + rank] = j - n_b;
 }
 
-// Tokens of the cluster's kernel that a batch takes, 0: the three kernels behind a cleared table of counts.  Their launches bound
-// the host, and up to 4096 tokens the cluster is as fast on the GPU (three kernels and the cluster, hooks of bf16, us: 8 + 2 x 41 tokens of
-// 320, vocabulary 36761, 38.9 and 31.3; 12 + 4 x 250 of 768, 50304, text ids 51.2 and 46.7, uniform 39.1 and 34.7; 8 + 2 x 200 the same,
-// text ids, 41.2 and 42.2).  Up to 8192, with twice the threads, it is the slower one on the GPU, so that is for tables whose
-// gradient is written in less time than the host takes (12 + 4 x 330 of 256, 50304: 39.2 and 31.1; 2 + 1 x 2000 of 1024, 8000: 39.1 and 32.9;
-// 8 + 2 x 512 of 768, 50304, 50.7 and 52.4).  A thread for two tokens, 16384 of them: 53.9 and 62.
-static int emb_one_cluster(long long tokens, double table_bytes) {
-  if (tokens <= 4096) return 4096;
-  return tokens <= 8192 && table_bytes <= 32e6 ? 8192 : 0;
+// Tokens of the cluster's kernel that a batch takes, 0: the three kernels behind a cleared table of counts.  The cluster saves
+// launches, which bound the host, and looks at no ids that do not occur; it pays by clearing the counts and the sums of the
+// matrix from eight SMs, 0.45 TB/s, where the others have the counts cleared at full rate and the sums by a block for
+// every 256 tokens.  Bytes of counts and of sums (0: no matrix wanted); three kernels and the cluster, bf16, us:
+// * up to 4096 tokens.  Hooks: 8 + 2 x 41 tokens of 320, vocabulary 36761, 38.9 and 31.3; 12 + 4 x 250 of 768, 50304, text ids 51.2
+//   and 46.7.  Matrix alone: 34 x 100 of 64, a million ids 24.7 and 24.5, two million 31.3 and 32.8; 2000 + 250 samples of one
+//   token, 4 MB of sums, 28.4 and 26.6, 3900 + 130 25.7 and 26.4, 2048 + 2048 64 and 94.  Gradient alone, which saves one launch less
+//   and reads the whole table anyway: 34 x 100 of 64, 200000 ids 28.8 and 27.8, 300000 32.3 and 34.0, a million 71.6 and 76.1;
+// * up to 8192, with twice the threads: hooks of tables whose gradient is written in less time than the host takes (12 + 4 x 330
+//   of 256, 50304: 39.2 and 31.1; 8 + 2 x 512 of 768, the same, 50.7 and 52.4; 16 x 400 of 8, 100000 ids 40.9 and 34.1, 262000 41.1
+//   and 41.6).  A result on its own leaves the host time enough (16 x 400 of 8, 100000 ids: matrix 18.7 and 20.4, gradient 24.7
+//   and 27.9).
+// A thread for two tokens, 16384 of them: 53.9 and 62.
+static int emb_one_cluster(long long tokens, double table_bytes, long long counts, long long sums, bool grad) {
+  constexpr long long little = 3 << 18;
+  if (tokens <= 4096) {
+    if (sums == 0) return counts <= little ? 4096 : 0;
+    return counts <= 4 << 20 && (tokens <= 2048 || sums <= 2 << 20) ? 4096 : 0;
+  }
+  return tokens <= 8192 && grad && sums > 0 && table_bytes <= 32e6 && counts + sums <= little ? 8192 : 0;
 }
 
 // ---------------------------------------------------------------- dot product: join by id
@@ -1026,7 +1037,8 @@ static int emb_pass(const EmbBuckets& q, const T* Gb, const T* Gv, int n_train, 
   if (fill && !by_rows && !quick) GB_CUDA_OK(cudaMemsetAsync(out, 0, out_bytes, st));
   const int tokens = blocks;
   if (quick) blocks = ds->sm_count * 8;
-  const int one = quick ? 0 : emb_one_cluster(q.n_tok, static_cast<double>(out_bytes));
+  const int one = quick ? 0 : emb_one_cluster(q.n_tok, static_cast<double>(out_bytes), 4 * (kEmbTotals + static_cast<long long>(q.vocab)),
+                                              M64 != nullptr ? 8ll * n_val * n_train : 0, out != nullptr);
   if (one > 0) {
     GB_CUDA_OK(launch_next(one == 4096 ? emb_bucket_kernel<4096> : emb_bucket_kernel<8192>, dim3(kEmbBucketCtas), dim3(one / kEmbBucketCtas), 0, st,
                            q, M64, static_cast<long long>(n_val) * n_train));

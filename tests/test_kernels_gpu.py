@@ -1197,6 +1197,41 @@ def test_embedding_buckets_of_one_cluster(n_t, n_v, T, vocab):
         assert torch.equal(grad.cpu(), (gref.float() / n_t))
 
 
+# both sides of what one cluster clears: 4 MB of counts (0.75 without a matrix), 2 MB of sums above 2048 tokens; twice the tokens
+# for both results only
+@pytest.mark.parametrize("n_t,n_v,T,vocab,matrix,grad,one", [
+    (9, 2, 2, 1048564, True, False, True), (9, 2, 2, 1048565, True, False, False),
+    (9, 2, 2, 196596, False, True, True), (9, 2, 2, 196597, False, True, False), (9, 2, 2, 196597, True, True, True),
+    (1024, 1024, 1, 70, True, False, True), (2000, 131, 1, 70, True, True, True), (2000, 132, 1, 70, True, True, False),
+    (2000, 2000, 1, 70, True, False, False), (2500, 9, 2, 70, True, True, True), (1250, 1250, 2, 70, True, False, False),
+    (2500, 9, 2, 70, False, True, False)])
+def test_embedding_buckets_by_what_has_to_be_cleared(n_t, n_v, T, vocab, matrix, grad, one):
+    from ghostsuite_b200 import _lib
+    gen = torch.Generator().manual_seed(n_t)
+    ids = torch.randint(0, min(vocab, 70), (n_t + n_v, T), generator=gen)
+    ids[ids >= 35] += vocab - 70
+    G = torch.randint(-3, 4, (n_t + n_v, T, 8), generator=gen).float()
+    ids_d, G_d = ids.cuda(), G.cuda()
+    before, M, out = _lib.launch_count(), None, None
+    if matrix and grad:
+        M, out = ops().embedding_hook(ids_d, G_d, n_v, vocab, 1.0)
+    elif matrix:
+        M = ops().embedding_dot(ids_d, G_d, n_v, vocab)
+    else:
+        out = ops().embedding_wgrad(ids_d[:n_t], G_d[:n_t], n_t, vocab, 1.0, n_t)
+    # buckets; join, rounding of a matrix that shared memory does not hold; gradient
+    assert _lib.launch_count() - before == (1 if one else 4) + (1 + (n_t * n_v > 4096) if matrix else 0) + grad
+    after()
+    small = torch.where(ids >= 35, ids - (vocab - 70), ids)
+    hot = torch.nn.functional.one_hot(small, 70).double()
+    rows = torch.einsum("nti,ntd->nid", hot, G.double())               # whole numbers: exact in any order
+    if matrix:
+        assert torch.equal(M.cpu().double(), rows[n_t:].flatten(1) @ rows[:n_t].flatten(1).t())
+    if grad:
+        ref = torch.zeros(vocab, 8).index_add_(0, ids[:n_t].flatten(), G[:n_t].flatten(0, 1)) / n_t
+        assert torch.equal(out.cpu(), ref)
+
+
 @pytest.mark.parametrize("n_t,n_v,T", [(3, 2, 40), (5, 1, 1024)])
 def test_embedding_dot_of_the_largest_table(n_t, n_v, T):
     """2^31 - 1 rows: the counts and the totals before them are more words than an int counts, and all of them are
