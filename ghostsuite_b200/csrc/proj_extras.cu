@@ -516,9 +516,12 @@ static int dispatch_similarity(const SimParams& p, bool vec, const DeviceState* 
     g.cost = sim_cost(p, g, sizeof(PT), vec, ring, ds->sm_count);
     if (best < 0 || g.cost < grid.cost) { grid = g; best = i / 2; }
   }
-  // smaller operands are read in less time than the host takes for two kernels (64 x 8 rows of 50000 bf16: 6.9 us with a
-  // memset, 7.8 without; 3 x 57 of 200000 9.1 and 7.8)
-  grid.clear_ahead = bytes >= 8e6;
+  // A kernel's zeros hide behind the call ahead and cost the host a launch, which a call that comes alone waits for.  Back to back with
+  // a memset and with the kernel, and the same alone, us: float32 23 x 17 rows of 300000 16.4 and 13.0, 24.0 and 25.4; 32 x 32 of 98304 10.3
+  // and 7.5, 18.4 and 19.8; 64 x 64 16.5 and 15.2, 27.2 and 31; 40 x 40 of 50000 12.4 and 10.0, 22.0 and 22.2; bf16 3 x 57 of
+  // 200000 8.7 and 7.3, 17.4 and 18.5.  Below 16 MB it gives no more than it costs: float32 16 x 16 of 98304 8.2 and 7.4, 15.6 and
+  // 16.5; 64 x 8 of 50000 8.2 and 7.4, 16.0 and 17.1; bf16 7 x 28 of 153620 10.3 and 10.3, 19.4 and 20.9.
+  grid.clear_ahead = bytes >= 16e6;
   switch (best) {
     case 0: return launch_similarity<PT, 1, 1, 1, 1>(p, grid, vec, ring, ds, st);
     case 1: return launch_similarity<PT, 1, 2, 1, 1>(p, grid, vec, ring, ds, st);

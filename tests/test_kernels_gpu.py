@@ -1417,9 +1417,10 @@ def test_projection_similarity_routes(n1, n2, D, dtype):
         assert (S[:, n2:] == 7.0).all()
 
 
-# one to three words past the last sixteen bytes and none, results off sixteen bytes, both sides of 8 MB of operands
+# one to three words past the last sixteen bytes and none, results off sixteen bytes, both sides of 16 MB of operands
 @pytest.mark.parametrize("offset", [0, 1, 4])
-@pytest.mark.parametrize("n1,n2,D", [(3, 7, 250000), (5, 18, 90001), (9, 11, 100008), (16, 32, 20000), (31, 45, 300008)])
+@pytest.mark.parametrize("n1,n2,D", [(3, 7, 250000), (5, 18, 90001), (9, 11, 100008), (16, 32, 20000), (31, 45, 300008),
+                                     (5, 18, 173913), (5, 18, 173914), (31, 45, 52628), (31, 45, 52632), (9, 11, 200008)])
 def test_projection_similarity_over_old_values(n1, n2, D, offset):
     """Scores that several blocks add up: what was there does not count, and nothing beside them is written."""
     from ghostsuite_b200 import _lib
