@@ -1437,15 +1437,95 @@ def test_projection_similarity_over_old_values(n1, n2, D, offset):
     assert int(buf.isnan().sum()) == 16
 
 
-# 8, 17, 21 and 34 MB of split sums: one round of the blocks that clear them, several, and a memset
-@pytest.mark.parametrize("m,n", [(1024, 2048), (2048, 2048), (2048, 2560), (2048, 4160)])
-def test_wgrad_split_sums_over_old_values(m, n):
+# 8, 19, 24 and 40 MB of split sums: blocks that clear 1024 vectors each, more than the largest grid does in one round (two of
+# them), and a memset above 32 MB.  The sums are merged by a launch of their own, so it shows that there are several
+@pytest.mark.parametrize("mode", [0, 2])
+@pytest.mark.parametrize("rows,m,n", [(6000, 1024, 2048), (16384, 2048, 2432), (16384, 2048, 3072), (32768, 2560, 4096)])
+def test_wgrad_split_sums_over_old_values(rows, m, n, mode):
+    """Whole numbers whose sums float32 holds: equal whatever the splits, unless old sums count."""
+    from ghostsuite_b200 import _lib
+    lib = _lib.load()
     g = torch.Generator(device="cuda").manual_seed(32)
-    X, Y = (torch.randn(1, 6000, c, generator=g, device="cuda").bfloat16() for c in (m, n))
-    for scale in (1.0, 0.25):
-        out = ops().wgrad(X, Y, scale, torch.float32)
-        after()
-        assert O.rel_fro(out, scale * (X[0].double().t() @ Y[0].double())) < 1e-5      # exact products, float32 sums
+    X, Y = (torch.randint(-2, 3, (1, rows, c), generator=g, device="cuda").bfloat16() for c in (m, n))
+    ref = X[0].float().t() @ Y[0].float()
+    try:
+        _lib.check(lib.ghost_set_wgrad_pair_mode(mode))
+        for scale in (1.0, 0.25):            # the second one over the sums of the first
+            before = _lib.launch_count()
+            out = ops().wgrad(X, Y, scale, torch.float32)
+            assert _lib.launch_count() - before == (3 if m * n * 4 <= 32 << 20 else 2)
+            after()
+            assert torch.equal(out, scale * ref)
+    finally:
+        _lib.check(lib.ghost_set_wgrad_pair_mode(1))
+
+
+# just below 32 MB, 32 MB, more (a memset); a word, two and three behind the last sixteen bytes; results off sixteen bytes
+@pytest.mark.parametrize("n_t,n_v,offset", [(4095, 2048, 0), (4096, 2048, 0), (4097, 2048, 0), (4096, 2048, 4), (4096, 2048, 1),
+                                            (3, 1, 0), (2, 1, 0), (1, 1, 0), (5, 1, 0), (13, 315, 0), (1024, 4, 0), (1025, 4, 0)])
+def test_gram_matrix_over_old_values(n_t, n_v, offset):
+    """All of the matrix that the Grams add to is cleared, and nothing beside it is written."""
+    from ghostsuite_b200 import _lib
+    lib, stream = _lib.load(), torch.cuda.current_stream().cuda_stream
+    g = torch.Generator(device="cuda").manual_seed(n_t)
+    a, b, u, v = (torch.randint(-2, 3, (n, 8), generator=g, device="cuda").bfloat16() for n in (n_t, n_v, n_t, n_v))
+    buf = torch.full((n_v * n_t + 16,), float("nan"), device="cuda")
+    M = buf[offset:offset + n_v * n_t]
+    _lib.check(lib.ghost_gram_dot_bf16(a.data_ptr(), b.data_ptr(), u.data_ptr(), v.data_ptr(), n_t, n_v, 1, 8, 8, 8, 8, 8, 8, 0, 1.0,
+                                       M.data_ptr(), stream))
+    after()
+    assert torch.equal(M.view(n_v, n_t), (b.float() @ a.float().t()) * (v.float() @ u.float().t()))      # whole numbers
+    assert int(buf.isnan().sum()) == 16
+
+
+# one block of tokens and several; a gradient in one split and in several (5000 and 9000 rows), by one CTA or a pair; a matrix of more
+# entries than the GEMM's grid has threads (150 x 300 and 400 x 400)
+@pytest.mark.parametrize("parts", [1, 2])
+@pytest.mark.parametrize("n_t,n_v,T,d,p", [(3, 2, 5, 64, 128), (5, 1, 130, 192, 64), (4, 2, 1250, 256, 128), (9, 1, 1000, 128, 256),
+                                           (300, 150, 2, 64, 64), (400, 400, 1, 128, 256)])
+def test_gram_pass_entry_point(n_t, n_v, T, d, p, parts):
+    """ghost_gram_pass over matrices of old values: Grams with the gradient, whose GEMM clears them, and without; either order of
+    the gradient, each kernel; nothing beside the results is written."""
+    from ghostsuite_b200 import _lib
+    lib, stream = _lib.load(), torch.cuda.current_stream().cuda_stream
+    g = torch.Generator(device="cuda").manual_seed(n_t)
+    N = n_t + n_v
+    # whole numbers: exact in any order, and in one bf16 part; the second part (a residual) is then zero
+    A, G = (torch.randint(-1, 2, (N * T, c), generator=g, device="cuda").bfloat16() for c in (d, p))
+    At, Av, Gt, Gv = A[:n_t * T].float(), A[n_t * T:].float(), G[:n_t * T].float(), G[n_t * T:].float()
+    ref = ((Av @ At.t()) * (Gv @ Gt.t())).view(n_v, T, n_t, T).double().sum((1, 3))
+    assert ref.abs().max() < 2 ** 24
+    if parts == 2:
+        A, G = (torch.cat([x, torch.zeros_like(x)]) for x in (A, G))
+    size = int(lib.ghost_wgrad_workspace_bytes(max(d, p), max(d, p)))
+    ws = torch.full((size,), 0xff, dtype=torch.uint8, device="cuda")
+    try:
+        for mode in (0, 2):
+            _lib.check(lib.ghost_set_wgrad_pair_mode(mode))
+            for in_by_out in (0, 1):
+                for with_grad, dtype in ((True, torch.float32), (True, torch.bfloat16), (False, torch.float32)):
+                    buf = torch.full((n_v * n_t + 16,), float("nan"), device="cuda")
+                    M = buf[8:8 + n_v * n_t]
+                    shape = (d, p) if in_by_out else (p, d)
+                    grad = torch.full(shape, float("nan"), device="cuda", dtype=dtype)
+                    _lib.check(lib.ghost_gram_pass(A.data_ptr(), G.data_ptr(), parts, n_t, n_v, T, d, p, d, p, in_by_out, M.data_ptr(), 0.5,
+                                                   grad.data_ptr() if with_grad else None, int(dtype == torch.float32), ws.data_ptr(), size, stream))
+                    after()
+                    assert torch.equal(M.view(n_v, n_t).double(), ref)
+                    assert int(buf.isnan().sum()) == 16
+                    want = 0.5 * (At.t() @ Gt if in_by_out else Gt.t() @ At)
+                    if with_grad:
+                        assert torch.equal(grad, want.to(dtype))
+                    else:
+                        assert bool(grad.isnan().all())
+    finally:
+        _lib.check(lib.ghost_set_wgrad_pair_mode(1))
+    bad = (None, G.data_ptr(), parts, n_t, n_v, T, d, p, d, p, 0, M.data_ptr(), 0.5, None, 1, ws.data_ptr(), size, stream)
+    for at, value in ((0, None), (2, 3), (3, 0), (4, 0), (5, 0), (6, 0), (8, d - 8), (11, None)):
+        args = list(bad)
+        args[0] = A.data_ptr()
+        args[at] = value
+        assert lib.ghost_gram_pass(*args) != 0
 
 
 # rows of which 32, 16, 8, four and more than a whole draw's bytes are drawn at once; tables of a part of a draw, one and many
