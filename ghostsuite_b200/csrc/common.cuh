@@ -80,11 +80,10 @@ inline cudaError_t launch_next(void (*kernel)(P...), dim3 grid, dim3 block, size
 }
 // Zeros for the kernel behind it in the stream, that adds to them: a kernel in the same programmatic order.  A memset waits for
 // the kernel ahead to end, and the kernel behind it for the memset, 1.5 to 3 us at either edge; this one is there by then and lets the
-// next come up while it writes.  Calls back to back with a memset and with it, us: similarity of 64 x 64 rows of 98304 float32 16.5 and
-// 15.2, of 32 x 32 10.3 and 7.9; GradProj of 4 x 649 tokens of 640 + 8448 20.0 and 17.0, of 8 x 4096 of 4096 + 14336 209 and 205;
-// embedding hook of 16 x 1024 tokens 54.0 and 52.1; hook of 29 x 197 rows of (768, 1000) float32 80.0 and 77.6.  On the host it is a
-// launch instead of a memset, 0.9 us more.  Words off sixteen bytes, large buffers, which a memset's bandwidth
-// counts for, and captures, whose edges are plain ones, keep the memset.
+// next come up while it writes.  With a memset and with it, us: GradProj of 4 x 649 tokens of 640 + 8448 20.0 and 17.0; embedding
+// hook of 16 x 1024 tokens of 768 54.3 and 52.2.  Alone it hides behind nothing, and on the host it is a launch instead of a memset, 0.9 us
+// more: a user whose chain is one kernel weighs that (dispatch_similarity).  Words off sixteen bytes, large buffers, which a memset's
+// bandwidth counts for, and captures, whose edges are plain ones, keep the memset.
 static constexpr size_t kClearMost = 32u << 20;
 int clear_ahead(void* dst, size_t bytes, cudaStream_t st);
 // The other half of launch_next, in every kernel that is launched so, before its first access to global memory and in every

@@ -689,8 +689,8 @@ static int launch_gradproj_t(const CUtensorMap& tg, const CUtensorMap& tpr, cons
 }
 
 // Clusters of `ranks` CTAs of this kernel that are resident at once, as the driver counts them: a cluster stays inside a GPC,
-// whose SMs differ from device to device.  (A 148-SM device: 16 of eight by its GPCs of 18 and 20, but sixteen of them, 24 of six or
-// 48 of three took two rounds: 17.5 us against 32.1 for 48 x 100 tokens of 640 + 640, k = 40.)
+// whose SMs differ from device to device.  (On a 148-SM device 15 of eight, 22 of six, 33 of four, 45 of three; one more of them and
+// the call takes two rounds: 17.5 us against 32.1 for 48 x 100 tokens of 640 + 640, k = 40, in threes.)
 template <int KMAX, int kSrc, bool kEmb, int kCluster>
 static int gradproj_resident(int ranks, const DeviceState* ds) {
   using Cfg = GpCfg<KMAX, kSrc, kCluster>;
@@ -720,13 +720,13 @@ static int gradproj_resident(int ranks, const DeviceState* ds) {
   return n - 1;
 }
 
-// CTAs that share a unit: as many as are resident with one unit per cluster.  The cluster's two barriers and the exchange cost about
-// 2 us; a stage is 0.5 us of a unit's chain, and the contraction of 128 tokens, which the CTAs share too, 3 us at
-// 64 x 64 and 1 us at 32 x 32 (32 x 64 tokens of 256 + 256 columns, four stages, k = 32: 10.3 us alone, 11.3 in pairs;
-// 12 x 1 token of 128 + 2112, k = 44: 23.6 and 13.1 in eights).  Three or six, whose shares are
-// uneven, only from so many stages on (17 x 60 of 640 + 640, ten stages: 13.9 us in fours, 14.8 in sixes): 9 x 464 of 9792 + 4160
-// float32 154 us in pairs, 109 in threes, 20 x 100 of the same bf16 21.0 in fours, 16.9 in sixes.  Fives lost (24 units of 32
-// stages: 26.3 against 24.7 in fours).
+// CTAs that share a unit: as many as are resident with one unit per cluster.
+// * Short chains of small ranks stay alone: the cluster's barriers and the exchange cost about 2 us, a stage is 0.5 us of a unit's
+//   chain, the contraction, which the CTAs share too, 1 us at 32 x 32 and 3 at 64 x 64 (32 x 64 tokens of 256 + 256 columns, four
+//   stages, k = 32: 10.3 us alone, 11.3 in pairs; 12 x 1 token of 128 + 2112, k = 44: 23.6 alone, 13.1 in eights).
+// * Three or six share unevenly, which pays from so many stages on (17 x 60 of 640 + 640, ten stages: 13.9 us in fours, 14.8 in sixes;
+//   20 x 100 of 9792 + 4160 bf16 21.0 and 16.9; 9 x 464 of the same float32 154 in pairs, 109 in threes).
+// * Fives lost (24 units of 32 stages: 26.3 us, 24.7 in fours).
 template <int KMAX, int kSrc, bool kEmb>
 static int gradproj_ranks(long long units, int stages, const DeviceState* ds) {
   if ((stages < 8 && KMAX <= 32) || 2 * units > ds->sm_count) return 1;
@@ -738,12 +738,12 @@ static int gradproj_ranks(long long units, int stages, const DeviceState* ds) {
 }
 
 // CTAs of a cluster that takes all units of a sample and stores its result, or 1: units dealt over the GPU, results added to zeros.
-// A cluster saves the launch that zeroes and the additions (embedding form of bf16: 4 x 796 tokens of 192 11.6 -> 9.1 us, 32 x 256
-// of 768 11.6 -> 10.4; 12 x 900 of 256 + 512 11.0 -> 10.7) where each of its CTAs has a unit at most, all clusters are resident
-// (16 x 2048 of 1024, embedding form, in eights: 20 against 36 us) and a quarter of the SMs stays free: with the GPU full of
-// units the clusters come up later than CTAs do (64 x 256 of 768 + 768: 14.2 without, 14.7 with them; 32 x 512 of 1024 + 4096 34.3
-// and 34.7; 64 x 300 of 512, embedding form, 14.8 and 15.2).  The largest that fits: its CTAs share the storing (16 x 250 of
-// 320 + 320, k = 32, two units a sample: 10.8 in eights, 11.2 in pairs).
+// A cluster saves the launch that zeroes and the additions (embedding form of bf16: 4 x 796 tokens of 192 11.6 -> 9.1 us; 12 x 900 of
+// 256 + 512 11.0 -> 10.7).  It is taken where
+// * each of its CTAs has a unit at most and all clusters are resident (16 x 2048 of 1024, embedding form, in eights: 36 us against 20);
+// * a quarter of the SMs stays free: with the GPU full of units clusters come up later than CTAs do (64 x 256 of 768 + 768: 14.7
+//   against 14.2; 64 x 300 of 512, embedding form, 15.2 and 14.8).
+// The largest that fits: its CTAs share the storing (16 x 250 of 320 + 320, two units a sample: 10.8 in eights, 11.2 in pairs).
 template <int KMAX, int kSrc, bool kEmb>
 static int gradproj_group(int B, int chunks, const DeviceState* ds) {
   if (chunks == 1 || 4ll * B * chunks > 3ll * ds->sm_count) return 1;

@@ -124,7 +124,7 @@ __global__ void cast_pair_kernel(const CastPair p) {
 // Both operands of a token-contracted GEMM in one launch: rows zero-padded to ld (a multiple of 64) columns, as the
 // values alone (PARTS = 1; bf16 rows whose sums are not asked for go through cast_pair_kernel) or as values and residuals, [samples, 2, T, ld] or [2, samples * T, ld].  A block takes a panel of 128 columns of
 // some rows, a thread eight columns of every 16th row, two rows in flight.  Where the column sums of an operand are
-// wanted the rows are one sample's (or a chunk of it, added with atomics), and they cost no second pass over it.
+// wanted the rows are one sample's, or a chunk of it whose sums meet in a cluster or are added to zeros, and they cost no second pass.
 // Bound by HBM and, on small layers, by the round trip of one round of loads: 8 x 2048 rows of (1024, 2048) float32 at
 // 5.5 TB/s, 29 x 197 of (768, 1000) with their sums 17 us from cold caches, 14 with the operands in L2 (two launches of
 // cast_split_kernel with three parts 17.4, and 8.5 for the sums in a pass of their own).
@@ -259,7 +259,7 @@ __global__ void __launch_bounds__(256, 4) split_pair_kernel(const SplitParams p)
 }
 
 // ------------------------------------------------------------------------------------------
-// per-sample column sums: out[n, c] += sum_{t in split} G[n, t, c]
+// per-sample column sums: out[n, c] = sum_t G[n, t, c], of one split or of several that are a cluster; others add theirs to zeros
 // ------------------------------------------------------------------------------------------
 template <typename T>
 __global__ void colsum_kernel(const T* G, long long Tn, int cols, long long ld,

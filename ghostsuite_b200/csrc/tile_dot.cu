@@ -8,12 +8,12 @@
 //     sum[k]   (+)= sum_b W[b][k]                        (the train gradient, reference :168)
 //
 // HBM-bound by design, so it is built as a copy pipeline: one producer thread feeds a ring of
-// shared-memory stages with TMA (one box of validation rows and one of 16 or 32 train rows per stage,
-// 256 float32 or 512 bf16 elements wide); the compute warps consume them.  Each CTA owns a contiguous range of stages:
+// shared-memory stages with TMA (one box of validation rows and one of train rows per stage: float32 8, 16 or 32
+// train rows, 256 elements wide, bf16 16 or 32 of 512); the compute warps consume them.  Each CTA owns a contiguous range of stages:
 // the train-gradient sum is a plain read-modify-write (deterministic, no atomics); the dot
 // products are reduced inside the CTA and added to M once per CTA and block.
 //
-// bf16 tiles (tile_dot_mma_kernel): the stage is loaded as four 128-byte-swizzled 64-element
+// bf16 tiles (tile_dot_mma_kernel): the stage is loaded as eight 128-byte-swizzled 64-element
 // panels per operand, and both contractions run on the tensor cores through mma.sync
 // (m16n8k16, fp32 accumulate) fed by ldmatrix: the dot products as W[16 train x 16 k] x
 // V[16 k x 8 val], the train-gradient sum as mask[16 x 16 train] x W[16 train x 8 k] (a
@@ -634,7 +634,7 @@ static int launch_tile_dot_mma_t(const void* V, int v_samples, const void* W, in
   using Cfg = TdMmaCfg<NVT, MT>;
   CUtensorMap tv, tw;
   int rc;
-  // [tiles][samples][32768] seen as [tiles][512 panels][samples][64]: one box = 4 panels of the stage
+  // [tiles][samples][32768] seen as [tiles][512 panels][samples][64]: one box = the stage's 8 panels
   if (p.v_per_rank > 0)
     rc = make_tmap_bf16_gathered_tiles(&tv, V, v_samples / p.v_per_rank, tiles, p.v_per_rank, Cfg::kValRows, Cfg::kPanels);
   else

@@ -1286,7 +1286,8 @@ def test_norm_wide_rows(dtype, rms, N, T, F):
                                   # samples of several units in a cluster of eight, four, two, and too many for one
                                   (8, 1000, 64, 130, 7, 11), (3, 129, 72, 70, 64, 64), (32, 300, 100, 64, 17, 128), (33, 300, 64, 64, 5, 6),
                                   (72, 257, 66, 128, 20, 12), (7, 1025, 128, 64, 100, 128),
-                                  # units shared by seven to three CTAs, whose tokens do not divide evenly
+                                  # units shared by six CTAs (of 20 only with float32's longer chains, else four), four (24 units) and
+                                  # three (38), whose tokens do not divide evenly
                                   (18, 128, 900, 1000, 40, 33), (20, 90, 2000, 64, 16, 16), (2, 1500, 1300, 700, 64, 64), (38, 128, 640, 520, 9, 64)])
 def test_gradproj_dense_unit_counts_and_widths(case, dtype):
     B, T, n_r, n_c, k_r, k_c = case
