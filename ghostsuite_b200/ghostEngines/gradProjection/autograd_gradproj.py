@@ -21,7 +21,7 @@ from ..autograd_grad_sample_dotprod import register_hook_pair
 
 def _flatten_tokens(x: torch.Tensor) -> torch.Tensor:
     """``[B, D] -> [B, 1, D]``; ``[B, ..., D] -> [B, T, D]``."""
-    if x.dim() == 3:
+    if x.dim() == 3 and x.size(0):       # the reshape refuses an empty batch
         return x
     if x.dim() <= 2:
         return x.unsqueeze(1)
@@ -119,7 +119,7 @@ class GradProjHooks:
         ``[B, k_o, k_i]`` float32 (reference :167-222, a Python loop over every token there): one
         kernel that streams the out-grad rows once and gathers the rows of ``P_i^T`` by token id."""
         batch = indices.shape[0]
-        ids = indices if indices.dim() == 2 else indices.reshape(batch, -1)
+        ids = indices if indices.dim() == 2 and batch else indices.reshape(batch, -1)      # (refuses an empty one)
         g = grad_output if grad_output.dim() == 3 and grad_output.shape[:2] == ids.shape else \
             grad_output.reshape(batch, ids.shape[1], grad_output.shape[-1])
         if g.dtype not in (torch.float32, torch.bfloat16):

@@ -229,3 +229,15 @@ def test_embedding_batch_beyond_one_set_of_buckets(monkeypatch):
         L._compute_embedding_dot_product(layer, A, B, 1)
         L._compute_embedding_train_grad(layer, A, B, 1)
         assert calls == want
+
+
+@pytest.mark.parametrize("kind", ["linear", "embedding"])
+def test_gradproj_hooks_refuse_an_empty_batch(kind):
+    """With the error of the reshape that it does not fit, whatever else is missing (here the GPU)."""
+    from ghostsuite_b200.ghostEngines.gradProjection.autograd_gradproj import create_projection_hooks
+    layer = torch.nn.Linear(6, 4, bias=False) if kind == "linear" else torch.nn.Embedding(6, 4)
+    hooks = create_projection_hooks(layer, "layer", torch.randn(2, 6), torch.randn(3, 4))
+    inp = torch.zeros(0, 5, 6) if kind == "linear" else torch.zeros(0, 5, dtype=torch.long)
+    hooks.forward_hook_store_inputs(layer, (inp,), None)
+    with pytest.raises(RuntimeError, match="reshape"):
+        hooks.backward_hook_compute_proj(layer, None, (torch.zeros(0, 5, 4),))
