@@ -569,9 +569,9 @@ def gradproj_embedding(ids: torch.Tensor, G: torch.Tensor, P_o_prepared: torch.T
         return _native().gradproj_embedding(ids, G, P_o_prepared, P_i_t, k_o, k_i, scale, out)
 
 
-#: largest block (rows of either operand) the similarity kernel is used for.  Beyond it a library GEMM
-#: takes bf16 operands faster (192 x 192 scores over 98304 elements: 28 us against 51) and float32 ones
-#: more accurately (rows of both signs: 1.2e-6 off the 64-bit result against 4.4e-6; 494 us against 97)
+#: largest block (rows of either operand) the similarity kernel is used for whatever the rows' type.  Beyond it a
+#: library GEMM takes float32 rows more accurately (192 x 192 scores over 98304 elements of both signs: 1.2e-6 off the
+#: 64-bit result against 4.4e-6; 494 us against 97); bfloat16 rows: projection_utils._bf16_sets_for_kernel
 SIMILARITY_KERNEL_MAX_ROWS = 128
 
 

@@ -241,3 +241,21 @@ def test_gradproj_hooks_refuse_an_empty_batch(kind):
     hooks.forward_hook_store_inputs(layer, (inp,), None)
     with pytest.raises(RuntimeError, match="reshape"):
         hooks.backward_hook_compute_proj(layer, None, (torch.zeros(0, 5, 4),))
+
+
+def test_large_similarity_sets_that_the_kernel_takes():
+    from ghostsuite_b200.ghostEngines.gradProjection import projection_utils as U
+    rows = lambda n, d: torch.zeros(n, d, dtype=torch.bfloat16)
+    takes = U._bf16_sets_for_kernel
+    assert takes(rows(1, 8), rows(65536, 8)) and takes(rows(129, 31), rows(512, 31))
+    assert takes(rows(600, 24)[:, 8:16], rows(3, 8)) and not takes(rows(600, 24)[:, 4:12], rows(3, 8))
+    assert not takes(rows(1, 8), rows(65537, 8)) and not takes(rows(513, 31), rows(1, 31))
+    assert not takes(rows(0, 8), rows(200, 8)) and not takes(rows(200, 0), rows(200, 0))
+    assert not takes(rows(200, 8), rows(200, 8).float()) and not takes(rows(200, 8).double(), rows(200, 8).double())
+    assert not takes(rows(1, 8).expand(200, 8), rows(2, 8)) and not takes(rows(8, 200).t(), rows(2, 8))
+    assert not takes(rows(200, 8).requires_grad_(), rows(2, 8))
+    with torch.autograd.forward_ad.dual_level():
+        assert not takes(rows(200, 8), rows(2, 8))
+    seen = []
+    torch.func.vmap(lambda x: seen.append(takes(x, rows(2, 8))) or x.sum())(torch.zeros(3, 200, 8, dtype=torch.bfloat16))
+    assert seen == [False]

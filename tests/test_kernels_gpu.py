@@ -884,6 +884,35 @@ def test_projection_similarity_block_shapes(case, dtype):
     assert (err <= 2.0 ** -15 * a.double().norm(dim=1)[:, None] * b.double().norm(dim=1)[None]).all()
 
 
+# more rows than ops.SIMILARITY_KERNEL_MAX_ROWS: bf16 sets go to the kernel, also as columns of wider rows; gradients, overlapping
+# rows and mixed types stay where they were
+@pytest.mark.parametrize("n1, n2, D", [(1, 129, 1), (129, 3, 257), (512, 200, 64), (700, 513, 200), (513, 2, 31)])
+def test_projection_similarity_of_large_bf16_sets(n1, n2, D):
+    from ghostsuite_b200.ghostEngines.gradProjection import projection_utils as U
+    g = torch.Generator(device="cuda").manual_seed(25)
+    a, b = (torch.randn(n, D, generator=g, device="cuda").bfloat16() for n in (n1, n2))
+    wide = torch.full((n1, D + 3), 1e30, device="cuda").bfloat16()
+    wide[:, 2:2 + D] = a
+    ref = a.double() @ b.double().t()
+    # exact products; the sums of 2 D / 32 partial sums are off by 2^-24 each at most, those inside a step by one truncation per product
+    bound = (D + 32) * 2.0 ** -23 * a.double().abs() @ b.double().abs().t()
+    before = ops().launch_count()
+    for rows in (a, wide[:, 2:2 + D]):
+        S = U.projection_similarity(rows, b)
+        after()
+        assert S.dtype == torch.float32 and ((S.double() - ref).abs() <= bound).all()
+    aligned = D % 8 == 0
+    assert ops().launch_count() > before if aligned or max(n1, n2) <= 512 else ops().launch_count() == before
+    bits = a.clone()
+    bits[0, 0] = float("inf")
+    assert torch.equal(torch.isfinite(U.projection_similarity(bits, b)), torch.isfinite(bits.double() @ b.double().t()))
+    count = ops().launch_count()
+    assert U.projection_similarity(a.clone().requires_grad_(), b).grad_fn is not None
+    assert U.projection_similarity(a[:1].expand(max(n1, 200), D), b).shape == (max(n1, 200), n2)
+    assert U.projection_similarity(a, b.float()).dtype == torch.float32
+    assert ops().launch_count() == count
+
+
 # one stage, one cluster and many of them; rows that TMA reads and rows that it cannot (odd lengths, odd pitches), each at
 # the ends of a panel of 32 floats / 64 bf16 elements; scores with and without whole 16-byte pieces per row
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
