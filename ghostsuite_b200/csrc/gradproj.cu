@@ -17,10 +17,12 @@
 // The embedding form (kEmb) has token ids in place of A: the rows of P_c^T are gathered by id straight into
 // the staged block, out[b] = scale * sum_t (P_r g_t)(P_c[:, id_t])^T, and only G is streamed.
 //
-// float32 rows, and bf16 rows that TMA cannot read, come through the registers of eight more warps (kSrc), which write
-// the swizzled bf16 blocks -- of float32 data value and residual, three products -- so that such operands too are
-// read once: copies in parts beforehand moved 16 bytes for every element of four (8 x 4096 tokens of 1024 + 1024
-// float32, k = 32: 189 -> 97 us; token table of 1024 float32 features, 16 x 2048 tokens: 107 -> 56 with mma.sync before).
+// float32 rows, and bf16 rows that TMA cannot read, come through shared memory as they are (kSrc): eight more warps keep
+// 16-byte copies of them on their way and write what has arrived as the swizzled bf16 blocks -- of float32 data value and residual,
+// three products -- so that such operands too are read once, and several stages ahead (16 x 2048 tokens of 1024 + 1024 float32,
+// k = 32: 99 us with eight warps that loaded into registers, two stages each, 63 so; 4 x 4096 of 2048 + 2049, k = 64: 109 and 94;
+// 32 x 3000 of 1001 + 2003 bf16, k = 64, which were copied with padded rows before: 369 and 217; token table of 4000 float32 features,
+// 16 x 2048 tokens, k = 64: 198 and 164).  Bound by the latency and the shared-memory traffic of the conversion.
 //
 // Few (sample, 128-token) units: a unit is one CTA's chain over all columns of G and A, whatever the number of
 // tokens in it, so a small batch leaves the GPU idle for the length of that chain.  There (kSome, kWhole) a cluster of
@@ -32,8 +34,10 @@
 // zeroing it before and adding to it: calls of up to 128 tokens are 1.04 to 1.18 times as fast (12 x 1 token
 // of 128 + 2112 bf16, k = 44: 18.1 -> 15.6 us with the host's part, 14 x 12 of 1088 + 256 float32 17.8 -> 15.3).
 //
-// CTA layout: warps 0-3 epilogue, warp 4 TMA producer, warp 5 MMA issuer, warps 6-13 loaders where kSrc asks for them.
+// CTA layout: warps 0-3 epilogue, warp 4 TMA producer, warp 5 MMA issuer, from warp 6 on 8 or 16 loaders where kSrc asks for them; all of
+// them add up a cluster's blocks.
 #include <atomic>
+#include <type_traits>
 
 #include "common.cuh"
 #include "sm100_ptx.cuh"
@@ -74,28 +78,46 @@ struct GpParams {
 enum { kNone = 0, kSome = 1, kWhole = 2 };      // a cluster for each unit: no; with others of the sample; which is the sample
 enum { kSrcTma = 0, kSrcF32 = 1, kSrcBf16 = 2, kSrcMixed = 3 };      // how the rows of G and A reach shared memory
 
-template <int KMAX, int kSrc, int kCluster>   // KMAX: largest padded rank this instantiation handles (32, 64 or 128)
+template <int KMAX, int kSrc, bool kEmb, int kCluster>   // KMAX: largest padded rank this instantiation handles (32, 64 or 128)
 struct GpCfg {
   static constexpr int BM = 128, BK = 64;                  // BK: one 128-byte swizzle atom of bf16
+  static constexpr bool kLoaders = kSrc != kSrcTma;
   static constexpr int PARTS = kSrc == kSrcF32 || kSrc == kSrcMixed ? 2 : 1;    // bf16 parts of an element
   // Columns per pipeline stage = ATOMS * 64.  The single threads that drive the pipeline pay a few
   // hundred cycles per stage for the barrier round trip, so a stage carries two atoms when the
   // shared memory allows it.
-  static constexpr int ATOMS = (KMAX == 128 || kSrc != kSrcTma) ? 1 : 2;
+  static constexpr int ATOMS = (KMAX == 128 || kLoaders) ? 1 : 2;
   static constexpr int kActAtomBytes = BM * BK * 2;
   static constexpr int kProjAtomBytes = KMAX * BK * 2;
-  static constexpr int kStageBytes = ATOMS * PARTS * (kActAtomBytes + kProjAtomBytes);
+  static constexpr int kActBytes = ATOMS * PARTS * kActAtomBytes, kProjStageBytes = ATOMS * PARTS * kProjAtomBytes;
+  // Activation and projection blocks of a stage lie side by side and arrive together, or, behind loaders, in rings of their
+  // own: converted blocks wait for nothing but the tensor core, so two stages of them do, while projection blocks take
+  // their time through L2 and the memory goes to rows on their way.
+  static constexpr int kStageBytes = kActBytes + (kLoaders ? 0 : kProjStageBytes);
   // The pipeline is bound by how many bytes are in flight per SM, so the fp32 staging of the
   // projected blocks is kept to half a tile (64 tokens at a time; a cluster's partial blocks are
-  // staged whole) and the rest goes to stages: it fills the 227 KB of shared memory.
+  // staged whole, behind loaders where the stages were) and the rest goes to stages: it fills the 227 KB of shared memory.
   static constexpr int kStageRows = kCluster != kNone ? 128 : 64;
-  static constexpr int kProjBytes = 2 * kStageRows * KMAX * 4;
-  static constexpr int kRoom = (232448 - 1280 - kProjBytes) / kStageBytes;
-  static constexpr int kStages = kRoom < 8 ? kRoom : 8;
-  static constexpr int kSmemBytes = kStages * kStageBytes + kProjBytes + 1024 + 256;
-  static constexpr int kThreads = kSrc == kSrcTma ? 192 : 448;
+  static constexpr int kProjBytes = kLoaders && kCluster != kNone ? 0 : 2 * kStageRows * KMAX * 4;
+  static constexpr int kFree = 232448 - 1280 - kProjBytes;
+  static constexpr int kStages = kLoaders ? (PARTS == 2 ? (KMAX == 32 ? 3 : 2) : 5) : kFree / kStageBytes < 8 ? kFree / kStageBytes : 8;
+  static constexpr int kProjStages = kLoaders ? 3 : kStages;
+  static constexpr int kRings = kStages * kStageBytes + (kLoaders ? kProjStages * kProjStageBytes : 0);
+  // Sixteen loader warps, eight to a stage, where the epilogue leaves them registers (embedding form, k = 32, with its gathered
+  // rows in them: 10.9 us with eight, 13.5 with sixteen and spills) and the memory two slots each.  A warp's time for a stage is the
+  // latency of its instructions, so two groups take turns: 16 x 2048 tokens of 1024 + 1024 float32 77 us with eight, 64 with sixteen.
+  static constexpr int kLoaderWarps = !kLoaders ? 0 : (kEmb && (KMAX == 64 || kCluster == kNone)) || (KMAX == 64 && PARTS == 2 && kCluster == kNone) ? 8 : 16;
+  // Rows on their way: a slot is 128 bytes of columns of a loader warp's 16 rows, from the 16-byte boundary before them
+  static constexpr int kSlotPitch = 128 + 16, kSlotBytes = 16 * kSlotPitch;
+  static constexpr int kSlotsBytes = kLoaderWarps * kSlotBytes;      // a slot of every warp
+  static constexpr int kSlots = !kLoaders ? 0 : (kFree - kRings) / kSlotsBytes < 8 ? (kFree - kRings) / kSlotsBytes : 8;
+  static constexpr int kSmemBytes = kRings + kSlots * kSlotsBytes + kProjBytes + 1024 + 256;
+  static constexpr int kThreads = 192 + 32 * kLoaderWarps;
   static constexpr int RT = KMAX / 16;   // output rows per thread (16 thread rows)
   static constexpr int CT = KMAX / 8;    // output cols per thread (8 thread cols)
+  static_assert(!kLoaders || kSlots >= 2, "rows on their way");
+  static_assert(!kLoaders || kLoaderWarps / 8 <= kStages, "a stage for each group of loader warps");
+  static_assert(!kLoaders || kCluster == kNone || KMAX * KMAX * 4 + 2 * kStageRows * KMAX * 4 <= kRings, "a cluster's blocks lie in the rings");
 };
 
 // Staged fp32 rows are stored with their float4 chunks XOR-permuted by the row index, so that the
@@ -105,122 +127,179 @@ __device__ __forceinline__ int gp_staged_index(int row, int elem) {
   return row * KMAX + ((((elem >> 2) ^ row) & (KMAX / 4 - 1)) << 2) + (elem & 3);
 }
 
-// A loader warp's share of a stage, 16 rows of 64 columns, held in registers between its load and its store; nothing looks
-// at a loaded value before the store.  float32: lane l has columns 4 (l % 16) .. + 3 of rows l / 16 + 2 i, a vector where
-// rows are on its boundaries.  bf16 rows the same way, but element by element where they are not: there a lane has
-// columns l and l + 32 of all rows, so that a load of the warp covers neighbouring elements.
-template <int kSrc> struct GpRows;
-template <> struct GpRows<kSrcF32> {
-  float4 v[8];
-  // base + at: the warp's first row, column of the stage's first column; `left` columns and `rows` rows from there on
-  __device__ __forceinline__ void load(const void* base, long long at, long long ld, int left, long long rows, bool vec, int lane) {
-    const int r0 = lane >> 4, c = (lane & 15) * 4, cols = left - c;
-    const float* p = static_cast<const float*>(base) + at + r0 * ld + c;
+// Rows of a unit that a loader warp brings: one of every eight, so that short units too are shared by all warps.  Row i lies 8 i rows
+// below one of two rows, by the parity of i, which are four rows apart: what is written of two neighbours then lies in different
+// banks.  Eight rows are a multiple of 16 bytes whatever their pitch, so that all of one parity begin as far behind a 16-byte boundary.
+__device__ __forceinline__ int gp_loader_row(int warp, int i) { return 8 * i + ((warp + 4 * (i & 1)) & 7); }
+
+// `bytes` from `src` (a multiple of 16) on, and zeros up to 16
+__device__ __forceinline__ void gp_copy16(uint32_t dst, uintptr_t src, int bytes) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+
+__device__ __forceinline__ void gp_copy16(uint32_t dst, uintptr_t src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+
+// One operand's part of a unit: the unit's rows, and of them the columns of the stages of this CTA that a group of loader warps
+// fills, every kGroups-th, in slices of 128 bytes
+struct GpSegment {
+  uintptr_t at;            // first row, first column
+  long long pitch;         // bytes from row to row
+  long long bytes;         // of a row from there on
+  int jump;                // bytes from a stage's last slice to the next one's first
+  int rows, slices;        // (the second half of a last float32 stage may hold nothing)
+  bool half, vec;          // bf16; float32 rows on 16-byte boundaries with widths that are multiples of four
+};
+
+// A lane's 16-byte pieces of a segment's slices: of rows row + 32 j the piece lane % 8, and of row `lane` the ninth, where rows begin behind
+// a boundary.  A piece may begin before the row does, but not before the 16 bytes that hold the row's first element, and no byte
+// behind the row's last one is read.
+template <int kSlotPitch> struct GpAsk {
+  uintptr_t c, c8;
+  long long step;
+  int jump, odd;           // 1 where a stage is two slices
+  bool all;                // every row is there
+  int n, end, end8, left;  // pieces of the first kind; bytes of the slice's rows from a piece's start on, were all of them whole; slices
+  long long bytes;
+  __device__ __forceinline__ void open(const GpSegment& x, int warp, int lane) {
+    const int i = lane >> 3, row = gp_loader_row(warp, i), q = 16 * (lane & 7), row8 = gp_loader_row(warp, lane & 15);
+    const uintptr_t a = x.at + row * x.pitch, a8 = x.at + row8 * x.pitch;
+    c = (a & ~uintptr_t(15)) + q;
+    c8 = (a8 & ~uintptr_t(15)) + 128;
+    step = 32 * x.pitch;
+    n = (x.rows - row + 31) >> 5;
+    all = x.rows == 128;
+    end = static_cast<int>(a & 15) - q;
+    end8 = !x.vec && lane < 16 && row8 < x.rows ? static_cast<int>(a8 & 15) - 128 : -128;
+    left = x.slices;
+    bytes = x.bytes;
+    jump = x.jump;
+    odd = x.half ? 0 : 1;
+  }
+  __device__ __forceinline__ void request(uint32_t slot, int lane) {
+    const int now = bytes >= 128 ? 128 : bytes > 0 ? static_cast<int>(bytes) : -16;       // nothing: no piece
+    const int b8 = now + end8;
+    const uint32_t dst = slot + (lane >> 3) * kSlotPitch + 16 * (lane & 7);
+    if (all && bytes >= 128) {             // also of a row that begins behind a boundary the first eight pieces are whole
 #pragma unroll
-    for (int i = 0; i < 8; ++i, p += 2 * ld) {
-      const bool in = r0 + 2 * i < rows;
-      if (vec) {                           // widths are multiples of four here
-        v[i] = in && cols > 0 ? *reinterpret_cast<const float4*>(p) : make_float4(0.f, 0.f, 0.f, 0.f);
-      } else {
-        v[i].x = in && cols > 0 ? *p : 0.f;
-        v[i].y = in && cols > 1 ? p[1] : 0.f;
-        v[i].z = in && cols > 2 ? p[2] : 0.f;
-        v[i].w = in && cols > 3 ? p[3] : 0.f;
+      for (int j = 0; j < 4; ++j) gp_copy16(dst + j * 4 * kSlotPitch, c + j * step);
+    } else {
+      const int b = now + end < 16 ? now + end : 16;
+      if (b > 0) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          if (j < n) gp_copy16(dst + j * 4 * kSlotPitch, c + j * step, b);
       }
     }
-  }
-  // into the stage's two [128 rows][64 columns] swizzled blocks; first: the warp's first row in them
-  __device__ __forceinline__ void store(uint8_t* block, int lo_bytes, int first, int lane) const {
-    const int c = (lane & 15) * 4;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int row = first + (lane >> 4) + 2 * i;
-      uint8_t* dst = block + row * 128 + (((c >> 3) ^ (row & 7)) << 4) + (c & 4) * 2;
-      const __nv_bfloat162 h0 = __floats2bfloat162_rn(v[i].x, v[i].y), h1 = __floats2bfloat162_rn(v[i].z, v[i].w);
-      const __nv_bfloat162 l0 = __floats2bfloat162_rn(v[i].x - __bfloat162float(h0.x), v[i].y - __bfloat162float(h0.y));
-      const __nv_bfloat162 l1 = __floats2bfloat162_rn(v[i].z - __bfloat162float(h1.x), v[i].w - __bfloat162float(h1.y));
-      *reinterpret_cast<uint2*>(dst) = make_uint2(*reinterpret_cast<const uint32_t*>(&h0), *reinterpret_cast<const uint32_t*>(&h1));
-      *reinterpret_cast<uint2*>(dst + lo_bytes) = make_uint2(*reinterpret_cast<const uint32_t*>(&l0), *reinterpret_cast<const uint32_t*>(&l1));
-    }
+    if (b8 > 0) gp_copy16(slot + lane * kSlotPitch + 128, c8, b8);
+    const int go = (left & odd) == odd ? jump : 128;     // of two slices the second one has an odd number to go
+    c += go;
+    c8 += go;
+    bytes -= go;
+    --left;
   }
 };
-// A float32 operand beside a bf16 one, whose elements stay as they are, without a residual.  A form of its own: with
-// the type looked at in GpRows<kSrcF32> 10 x 3780 float32 tokens of 782 + 1024 took 149 us instead of 135.
-template <> struct GpRows<kSrcMixed> : GpRows<kSrcF32> {
-  int form;                // 0 float32; bf16: 1 vectors (bits of two elements each in x and y), 2 elements (one each in x to w)
-  __device__ __forceinline__ void load(const void* base, long long at, long long ld, int left, long long rows, bool vec, bool half, int lane) {
-    form = !half ? 0 : vec ? 1 : 2;
-    if (!half) {
-      GpRows<kSrcF32>::load(base, at, ld, left, rows, vec, lane);
-      return;
-    }
-    const int r0 = lane >> 4, c = (lane & 15) * 4, cols = left - c;
-    const unsigned short* p = static_cast<const unsigned short*>(base) + at + r0 * ld + c;
+
+// Writes an arrived slice into the stage's swizzled [128 rows][64 columns] block, from its column `column` on, and of float32
+// rows the residuals into the block `lo` bytes behind it.  `left` bytes of a row are there; columns that are not become
+// zeros.  Rows that are not there keep what the block held: nobody reads what the tensor core makes of them.  off: how far behind a 16-byte boundary the lane's rows begin (all of one parity, gp_loader_row).
+//
+// bf16 rows go by sixteen bytes, shifted in registers; unaligned float32 ones by single elements, whose shifts would cost more than the
+// loads they save (32 x 1000 tokens of 777 + 1025: 75.8 us so, 83.6 with shifts; bf16 32 x 3000 of 1001 + 2003: 223.5 by elements, 217).
+template <int PARTS, int kSlotPitch, bool kHalf, bool kVec>
+__device__ __forceinline__ void gp_convert(uint8_t* block, int lo, int column, const uint8_t* slot, int off, int rows,
+                                           long long left, int warp, int lane) {
+  // store(j) for all of a lane's rows, or for those that are there
+  auto each = [&](auto count, int n, auto&& store) {
+    constexpr int kCount = decltype(count)::value;
+    if (rows == 128) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i, p += 2 * ld) {
-      const bool in = r0 + 2 * i < rows;
-      if (vec) {                           // widths are multiples of four here
-        const uint2 w = in && cols > 0 ? *reinterpret_cast<const uint2*>(p) : make_uint2(0u, 0u);
-        v[i].x = __uint_as_float(w.x);
-        v[i].y = __uint_as_float(w.y);
-      } else {
-        v[i].x = __uint_as_float(in && cols > 0 ? p[0] : 0u);
-        v[i].y = __uint_as_float(in && cols > 1 ? p[1] : 0u);
-        v[i].z = __uint_as_float(in && cols > 2 ? p[2] : 0u);
-        v[i].w = __uint_as_float(in && cols > 3 ? p[3] : 0u);
-      }
-    }
-  }
-  __device__ __forceinline__ void store(uint8_t* block, int lo_bytes, int first, int lane) const {
-    if (form == 0) {
-      GpRows<kSrcF32>::store(block, lo_bytes, first, lane);
-      return;
-    }
-    const int c = (lane & 15) * 4;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int row = first + (lane >> 4) + 2 * i;
-      uint8_t* dst = block + row * 128 + (((c >> 3) ^ (row & 7)) << 4) + (c & 4) * 2;
-      uint2 w = make_uint2(__float_as_uint(v[i].x), __float_as_uint(v[i].y));
-      if (form == 2) w = make_uint2(w.x | w.y << 16, __float_as_uint(v[i].z) | __float_as_uint(v[i].w) << 16);
-      *reinterpret_cast<uint2*>(dst) = w;
-      *reinterpret_cast<uint2*>(dst + lo_bytes) = make_uint2(0u, 0u);
-    }
-  }
-};
-template <> struct GpRows<kSrcBf16> {
-  uint32_t v[32];
-  bool vec;
-  __device__ __forceinline__ void load(const void* base, long long at, long long ld, int left, long long rows, bool by_vector, int lane) {
-    const unsigned short* p = static_cast<const unsigned short*>(base) + at;
-    vec = by_vector;
-    if (vec) {
-      const int r0 = lane >> 4, c = (lane & 15) * 4;
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const bool in = r0 + 2 * i < rows && c < left;         // widths are multiples of four here
-        const uint2 w = in ? *reinterpret_cast<const uint2*>(p + (r0 + 2 * i) * ld + c) : make_uint2(0u, 0u);
-        v[2 * i] = w.x; v[2 * i + 1] = w.y;
-      }
+      for (int j = 0; j < kCount; ++j) store(j);
     } else {
 #pragma unroll
-      for (int i = 0; i < 32; ++i) {
-        const int r = i >> 1, c = (i & 1) * 32 + lane;
-        v[i] = r < rows && c < left ? p[r * ld + c] : 0u;
-      }
+      for (int j = 0; j < kCount; ++j)
+        if (j < n) store(j);
     }
-  }
-  __device__ __forceinline__ void store(uint8_t* block, int, int first, int lane) const {
+  };
+  if constexpr (kHalf) {                   // sixteen bytes a lane, four rows at a time, from the two aligned pieces that hold them
+    const int i0 = lane >> 3, q = lane & 7, r = gp_loader_row(warp, i0);
+    uint4 v[4], w[4];
 #pragma unroll
-    for (int i = 0; i < 32; ++i) {
-      if (vec && i >= 8) break;
-      const int row = vec ? first + (lane >> 4) + 2 * i : first + (i >> 1), c = vec ? (lane & 15) * 4 : (i & 1) * 32 + lane;
-      uint8_t* dst = block + row * 128 + (((c >> 3) ^ (row & 7)) << 4) + (c & 7) * 2;
-      if (vec) *reinterpret_cast<uint2*>(dst) = make_uint2(v[(2 * i) & 31], v[(2 * i + 1) & 31]);
-      else *reinterpret_cast<unsigned short*>(dst) = static_cast<unsigned short>(v[i]);
+    for (int j = 0; j < 4; ++j) v[j] = *reinterpret_cast<const uint4*>(slot + (i0 + 4 * j) * kSlotPitch + 16 * q);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) w[j] = *reinterpret_cast<const uint4*>(slot + (i0 + 4 * j) * kSlotPitch + 16 * q + 16);
+    const bool one = off & 4, two = off & 8;
+    const uint32_t pick = off & 2 ? 0x5432 : 0x3210;
+    uint32_t keep[4] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu};
+    if (left < 128) {
+      const int here = static_cast<int>(left) - 16 * q;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) keep[k] = here >= 4 * k + 4 ? 0xffffffffu : here == 4 * k + 2 ? 0xffffu : 0u;
+    }
+    uint8_t* d = block + r * 128 + ((q ^ (r & 7)) << 4);
+    each(std::integral_constant<int, 4>(), (rows - r + 31) >> 5, [&](int j) {
+      uint32_t x[8] = {v[j].x, v[j].y, v[j].z, v[j].w, w[j].x, w[j].y, w[j].z, w[j].w};
+#pragma unroll
+      for (int k = 0; k < 7; ++k) x[k] = one ? x[k + 1] : x[k];
+#pragma unroll
+      for (int k = 0; k < 5; ++k) x[k] = two ? x[k + 2] : x[k];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) x[k] = __byte_perm(x[k], x[k + 1], pick) & keep[k];
+      *reinterpret_cast<uint4*>(d + j * 4096) = make_uint4(x[0], x[1], x[2], x[3]);
+      if (PARTS == 2) *reinterpret_cast<uint4*>(d + j * 4096 + lo) = make_uint4(0u, 0u, 0u, 0u);
+    });
+  } else if constexpr (PARTS == 2) {
+    auto split = [](float x0, float x1, uint32_t& h, uint32_t& l) {
+      const __nv_bfloat162 hh = __floats2bfloat162_rn(x0, x1);
+      const __nv_bfloat162 ll = __floats2bfloat162_rn(x0 - __bfloat162float(hh.x), x1 - __bfloat162float(hh.y));
+      h = *reinterpret_cast<const uint32_t*>(&hh);
+      l = *reinterpret_cast<const uint32_t*>(&ll);
+    };
+    if constexpr (kVec) {                  // four neighbouring elements a lane, four rows at a time
+      const int i0 = lane >> 3, r = gp_loader_row(warp, i0), c = column + 4 * (lane & 7);
+      float4 f[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) f[j] = *reinterpret_cast<const float4*>(slot + (i0 + 4 * j) * kSlotPitch + 16 * (lane & 7));
+      if (left < 128 && 16 * (lane & 7) >= left) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) f[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+      uint8_t* d = block + r * 128 + (((c >> 3) ^ (r & 7)) << 4) + (c & 4) * 2;
+      each(std::integral_constant<int, 4>(), (rows - r + 31) >> 5, [&](int j) {
+        uint2 h, l;
+        split(f[j].x, f[j].y, h.x, l.x);
+        split(f[j].z, f[j].w, h.y, l.y);
+        *reinterpret_cast<uint2*>(d + j * 4096) = h;
+        *reinterpret_cast<uint2*>(d + j * 4096 + lo) = l;
+      });
+    } else {                               // two, two rows at a time
+      const int i0 = lane >> 4, r = gp_loader_row(warp, i0), e = 2 * (lane & 15), c = column + e;
+      const float* w = reinterpret_cast<const float*>(slot + i0 * kSlotPitch + off) + e;
+      float f[16];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        f[2 * j] = w[j * (2 * kSlotPitch / 4)];
+        f[2 * j + 1] = w[j * (2 * kSlotPitch / 4) + 1];
+      }
+      if (left < 128) {
+        const int cols = static_cast<int>(left) / 4 - e;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          if (cols <= 0) f[2 * j] = 0.f;
+          if (cols <= 1) f[2 * j + 1] = 0.f;
+        }
+      }
+      uint8_t* d = block + r * 128 + (((c >> 3) ^ (r & 7)) << 4) + (c & 7) * 2;
+      each(std::integral_constant<int, 8>(), (rows - r + 15) >> 4, [&](int j) {
+        uint32_t h, l;
+        split(f[2 * j], f[2 * j + 1], h, l);
+        *reinterpret_cast<uint32_t*>(d + j * 2048) = h;
+        *reinterpret_cast<uint32_t*>(d + j * 2048 + lo) = l;
+      });
     }
   }
-};
+}
 
 __device__ __forceinline__ float4 gp_ld_cluster(uint32_t addr) {
   float4 v;
@@ -228,29 +307,121 @@ __device__ __forceinline__ float4 gp_ld_cluster(uint32_t addr) {
   return v;
 }
 
-__device__ __forceinline__ float gp_ld_cluster1(uint32_t addr) {
-  float v;
-  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
-  return v;
+// Element-wise sum, in rank order, of four floats that lie at `at` in the shared memory of those CTAs of the cluster that have a bit
+// in `mask`.  BATCH loads go out together, all eight where registers are free: one after the other they took most of a small call (5 x 4 tokens of 368 + 448 float32, k = 42,
+// cycles: partial blocks 5850, results 3850 of 24000).
+template <int BATCH>
+__device__ __forceinline__ float4 gp_cluster_sum(const float* at, uint32_t mask) {
+  float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+  for (int r0 = 0; r0 < 8; r0 += BATCH) {
+    float4 v[BATCH];
+#pragma unroll
+    for (int r = 0; r < BATCH; ++r)
+      if (mask >> (r0 + r) & 1) v[r] = gp_ld_cluster(map_to_cta(smem_u32(at), r0 + r));
+#pragma unroll
+    for (int r = 0; r < BATCH; ++r)
+      if (mask >> (r0 + r) & 1) { sum.x += v[r].x; sum.y += v[r].y; sum.z += v[r].z; sum.w += v[r].w; }
+  }
+  return sum;
+}
+
+// o[r, c] += sum over staged rows [t0, t1) of s_r[t][r] * s_c[t][c], for the RT x CT block of thread (ty, tx)
+template <int KMAX>
+__device__ __forceinline__ void gp_contract(const float* s_r, const float* s_c, int t0, int t1, int ty, int tx, float (&o)[KMAX / 16][KMAX / 8]) {
+  constexpr int RT = KMAX / 16, CT = KMAX / 8;
+#pragma unroll 4
+  for (int t = t0; t < t1; ++t) {
+    float rr[RT], cc[CT];
+    if constexpr (RT >= 4) {
+#pragma unroll
+      for (int i = 0; i < RT; i += 4)
+        *reinterpret_cast<float4*>(&rr[i]) = *reinterpret_cast<const float4*>(&s_r[gp_staged_index<KMAX>(t, ty * RT + i)]);
+    } else {
+      *reinterpret_cast<float2*>(&rr[0]) = *reinterpret_cast<const float2*>(&s_r[gp_staged_index<KMAX>(t, ty * RT)]);
+    }
+#pragma unroll
+    for (int j = 0; j < CT; j += 4)
+      *reinterpret_cast<float4*>(&cc[j]) = *reinterpret_cast<const float4*>(&s_c[gp_staged_index<KMAX>(t, tx * CT + j)]);
+#pragma unroll
+    for (int i = 0; i < RT; ++i)
+#pragma unroll
+      for (int j = 0; j < CT; ++j) o[i][j] = fmaf(rr[i], cc[j], o[i][j]);
+  }
+}
+
+// The block of thread (ty, tx) in shared memory, [KMAX][KMAX], and zeros in its place
+template <int KMAX>
+__device__ __forceinline__ void gp_put_block(float* block, int ty, int tx, float (&o)[KMAX / 16][KMAX / 8]) {
+  constexpr int RT = KMAX / 16, CT = KMAX / 8;
+#pragma unroll
+  for (int i = 0; i < RT; ++i)
+#pragma unroll
+    for (int j = 0; j < CT; j += 4) {
+      *reinterpret_cast<float4*>(&block[(ty * RT + i) * KMAX + tx * CT + j]) = make_float4(o[i][j], o[i][j + 1], o[i][j + 2], o[i][j + 3]);
+      o[i][j] = o[i][j + 1] = o[i][j + 2] = o[i][j + 3] = 0.f;
+    }
+}
+
+// Adds the block of thread (ty, tx) to a sample's result, and zeros in its place
+template <int KMAX>
+__device__ __forceinline__ void gp_add_block(const GpParams& p, int b, int ty, int tx, float (&o)[KMAX / 16][KMAX / 8]) {
+  constexpr int RT = KMAX / 16, CT = KMAX / 8;
+  float* dst = p.out + static_cast<long long>(b) * p.out_stride;
+#pragma unroll
+  for (int i = 0; i < RT; ++i) {
+    const int r = ty * RT + i;
+#pragma unroll
+    for (int j = 0; j < CT; ++j) {
+      const int c = tx * CT + j;
+      if (r < p.k_r && c < p.k_c && o[i][j] != 0.f)
+        atomicAdd(dst + static_cast<long long>(r) * p.out_ld + c, o[i][j] * p.scale);
+      o[i][j] = 0.f;
+    }
+  }
+}
+
+// A sample's result from the blocks of `ranks` CTAs (rank order), of which this one stores its share with `threads` threads
+template <int KMAX, int BATCH>
+__device__ __forceinline__ void gp_store_block(const GpParams& p, int b, const float* block, uint32_t rank, uint32_t ranks, int tid, int threads) {
+  float* dst = p.out + static_cast<long long>(b) * p.out_stride;
+  const uint32_t mask = (1u << ranks) - 1;
+#pragma unroll 1
+  for (int e = 4 * (static_cast<int>(rank) * threads + tid); e < p.k_r * KMAX; e += 4 * static_cast<int>(ranks) * threads) {
+    const int c = e % KMAX;
+    if (c >= p.k_c) continue;
+    const float4 v = ranks > 1 ? gp_cluster_sum<BATCH>(block + e, mask) : *reinterpret_cast<const float4*>(block + e);
+    float* to = dst + static_cast<long long>(e / KMAX) * p.out_ld + c;
+    to[0] = v.x * p.scale;
+    if (c + 1 < p.k_c) to[1] = v.y * p.scale;
+    if (c + 2 < p.k_c) to[2] = v.z * p.scale;
+    if (c + 3 < p.k_c) to[3] = v.w * p.scale;
+  }
 }
 
 template <int KMAX, int kSrc, bool kEmb, int kCluster>
-__global__ void __launch_bounds__(kSrc == kSrcTma ? 192 : 448, 1)
+__global__ void __launch_bounds__((GpCfg<KMAX, kSrc, kEmb, kCluster>::kThreads), 1)
 gradproj_kernel(const __grid_constant__ CUtensorMap tm_g, const __grid_constant__ CUtensorMap tm_pr,
                 const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_pc,
                 const GpParams p) {
-  using Cfg = GpCfg<KMAX, kSrc, kCluster>;
+  using Cfg = GpCfg<KMAX, kSrc, kEmb, kCluster>;
   constexpr int BM = Cfg::BM, BK = Cfg::BK, kStages = Cfg::kStages, RT = Cfg::RT, CT = Cfg::CT;
-  constexpr int ATOMS = Cfg::ATOMS, PARTS = Cfg::PARTS;
+  constexpr int ATOMS = Cfg::ATOMS, PARTS = Cfg::PARTS, kProjStages = Cfg::kProjStages;
+  constexpr bool kLoaders = Cfg::kLoaders;
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  float* s_r = reinterpret_cast<float*>(smem + kStages * Cfg::kStageBytes);   // [kStageRows][KMAX]
+  uint8_t* slots = smem + Cfg::kRings;                                         // [loader warps][kSlots]
+  // Behind a cluster's loaders the staged blocks lie in the rings, whose last stage has been consumed by then, after the block that
+  // store() puts at their start
+  float* s_r = reinterpret_cast<float*>(kLoaders && kCluster != kNone ? smem + KMAX * KMAX * 4 : slots + Cfg::kSlots * Cfg::kSlotsBytes);   // [kStageRows][KMAX]
   float* s_c = s_r + Cfg::kStageRows * KMAX;                                  // [kStageRows][KMAX]
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kStages * Cfg::kStageBytes + Cfg::kProjBytes);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(slots + Cfg::kSlots * Cfg::kSlotsBytes + Cfg::kProjBytes);
   uint64_t* full_bar = bars;
   uint64_t* empty_bar = bars + kStages;
-  uint64_t* acc_full = bars + 2 * kStages;    // [2]
+  uint64_t* proj_full = kLoaders ? bars + 2 * kStages : full_bar;             // the projection blocks' own ring
+  uint64_t* proj_empty = kLoaders ? proj_full + kProjStages : empty_bar;
+  uint64_t* acc_full = bars + 2 * kStages + (kLoaders ? 2 * kProjStages : 0);  // [2]
   uint64_t* acc_empty = acc_full + 2;         // [2]
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
@@ -281,9 +452,26 @@ gradproj_kernel(const __grid_constant__ CUtensorMap tm_g, const __grid_constant_
     u1 = u0 + p.units_per_cta + (bx < p.units_extra ? 1 : 0);
     if (u1 > p.units) u1 = p.units;
   }
+  // sample and 128-token chunk of the first unit; a division of 64 bits is the time of a pipeline stage
+  const int chunks = p.chunks_per_sample;
+  const int b0 = u0 >> 32 ? static_cast<int>(u0 / chunks) : static_cast<int>(static_cast<uint32_t>(u0) / static_cast<uint32_t>(chunks));
+  const int chunk0 = static_cast<int>(u0 - static_cast<long long>(b0) * chunks);
+  auto rows_of = [&](int chunk) -> int {     // tokens in a unit
+    const long long left = p.T - static_cast<long long>(chunk) * BM;
+    return left < BM ? static_cast<int>(left) : BM;
+  };
+  // a cluster's CTA adds up and contracts tokens [first, first + share) of its unit
+  int first = 0, share = 0;
+  if constexpr (kCluster != kNone) {
+    const int rows = rows_of(chunk0), most = (rows + static_cast<int>(ranks) - 1) / static_cast<int>(ranks);
+    first = min(static_cast<int>(rank) * most, rows);
+    share = min(most, rows - first);
+  }
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < kStages; ++s) { mbar_init(&full_bar[s], kSrc == kSrcTma ? 1 : 9); mbar_init(&empty_bar[s], 1); }
+    for (int s = 0; s < kStages; ++s) { mbar_init(&full_bar[s], kLoaders ? 8 : 1); mbar_init(&empty_bar[s], 1); }
+    if (kLoaders)
+      for (int s = 0; s < kProjStages; ++s) { mbar_init(&proj_full[s], 1); mbar_init(&proj_empty[s], 1); }
     for (int a = 0; a < 2; ++a) { mbar_init(&acc_full[a], 1); mbar_init(&acc_empty[a], 4); }
     *abort_flag = 0;
     fence_barrier_init();
@@ -307,20 +495,21 @@ gradproj_kernel(const __grid_constant__ CUtensorMap tm_g, const __grid_constant_
     constexpr int kActBoxes = kSrc == kSrcTma ? ATOMS : 0, kProjBoxes = ATOMS * PARTS;
     const bool is_p = lane >= kActBoxes;
     const int box = is_p ? lane - kActBoxes : lane;
-    const uint32_t dst_off = is_p ? ATOMS * PARTS * Cfg::kActAtomBytes + box * Cfg::kProjAtomBytes
-                                  : box * Cfg::kActAtomBytes;
+    uint8_t* const dst = kLoaders ? smem + kStages * Cfg::kStageBytes + box * Cfg::kProjAtomBytes
+                                  : smem + (is_p ? Cfg::kActBytes + box * Cfg::kProjAtomBytes : box * Cfg::kActAtomBytes);
+    constexpr int kPitch = kLoaders ? Cfg::kProjStageBytes : Cfg::kStageBytes;
     int stage = 0; uint32_t phase = 0; bool ok = true;
+    int b = b0, chunk = chunk0;
     for (long long u = u0; u < u1 && ok; ++u) {
-      const int b = static_cast<int>(u / p.chunks_per_sample);
-      const int row0 = static_cast<int>(u % p.chunks_per_sample) * BM;
+      const int row0 = chunk * BM;
       for (int kb = kb0; kb < kb1; ++kb) {
         int w = 1;
-        if (lane == 0) w = mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag, p.err, 421) ? 1 : 0;
+        if (lane == 0) w = mbar_wait(&proj_empty[stage], phase ^ 1, abort_flag, p.err, 421) ? 1 : 0;
         w = __shfl_sync(0xffffffffu, w, 0);
         if (!w) { ok = false; break; }
         const bool first = kb < kb_r;
         const int kpad = first ? p.kr_pad : p.kc_pad;
-        if (lane == 0) mbar_arrive_expect_tx(&full_bar[stage], (kActBoxes * BM + kProjBoxes * kpad) * BK * 2);
+        if (lane == 0) mbar_arrive_expect_tx(&proj_full[stage], (kActBoxes * BM + kProjBoxes * kpad) * BK * 2);
         __syncwarp();
         if (lane < kActBoxes + kProjBoxes) {
           // an atom past the last column starts out of range and is zero-filled; what a residual box reads beyond
@@ -329,105 +518,142 @@ gradproj_kernel(const __grid_constant__ CUtensorMap tm_g, const __grid_constant_
           if (PARTS == 2) col += box == 0 ? 0 : (first ? p.lo_r : p.lo_c);
           else col += box * BK;
           const CUtensorMap* m = first ? (is_p ? &tm_pr : &tm_g) : (is_p ? &tm_pc : &tm_a);
-          tma_load_3d(smem + stage * Cfg::kStageBytes + dst_off, m, &full_bar[stage], col,
-                      is_p ? 0 : row0, is_p ? 0 : b);
+          tma_load_3d(dst + stage * kPitch, m, &proj_full[stage], col, is_p ? 0 : row0, is_p ? 0 : b);
         }
-        if (++stage == kStages) { stage = 0; phase ^= 1; }
+        if (++stage == kProjStages) { stage = 0; phase ^= 1; }
       }
+      if (++chunk == chunks) { chunk = 0; ++b; }
     }
-  } else if (kSrc != kSrcTma && warp >= 6) {
-    // Loader warps: 16 rows of a unit each.  The loads of the next stage are in flight while a stage is converted
-    // and stored: two register sets.
-    if constexpr (kSrc != kSrcTma) {
-      const int lw = warp - 6;
-      GpRows<kSrc> set[2];
-      long long row = 0, rows_left = 0;                  // of the unit being fetched: this warp's first row, rows from there on
-      auto fetch = [&](int kb, GpRows<kSrc>& q) {
-        const bool first = kb < kb_r;
-        const int col = (first ? kb : kb - kb_r) * BK;
-        const long long ld = first ? p.ldg : p.lda;
-        const void* src = first ? p.g : p.a;
-        const int left = (first ? p.n_r : p.n_c) - col;
-        const bool vec = first ? p.vec_g : p.vec_a;
-        if constexpr (kSrc == kSrcMixed) q.load(src, row * ld + col, ld, left, rows_left, vec, first ? p.half_g : p.half_a, lane);
-        else q.load(src, row * ld + col, ld, left, rows_left, vec, lane);
+  } else if (kLoaders && warp >= 6) {
+    // Loader warps: 16 rows of a stage each, requested kSlots - 1 slices ahead of the one that is converted
+    if constexpr (kLoaders) {
+      constexpr int kSlots = Cfg::kSlots, kGroups = Cfg::kLoaderWarps / 8;
+      const int lw = (warp - 6) & 7, group = (warp - 6) >> 3;
+      uint8_t* mine = slots + (warp - 6) * kSlots * Cfg::kSlotBytes;
+      struct Place { long long left; int before, b, chunk; bool second; };     // units to come, stages behind, where
+      const Place start = {u1 - u0, 0, b0, chunk0, false};
+      auto advance = [&](Place& at) {
+        at.second = !at.second;
+        if (at.second) return;
+        --at.left;
+        at.before ^= kb1 - kb0;                          // their parity
+        if (++at.chunk == chunks) { at.chunk = 0; ++at.b; }
       };
-      int stage = 0; uint32_t phase = 0;
-      auto put = [&](const GpRows<kSrc>& q) -> bool {
-        int w = 1;
-        if (lane == 0) w = mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag, p.err, 621) ? 1 : 0;
-        w = __shfl_sync(0xffffffffu, w, 0);
-        __syncwarp();
-        if (!w) return false;
-        q.store(smem + stage * Cfg::kStageBytes, Cfg::kActAtomBytes, lw * 16, lane);
-        fence_proxy_async_smem();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&full_bar[stage]);
-        if (++stage == kStages) { stage = 0; phase ^= 1; }
+      auto segment = [&](const Place& at, GpSegment& x) -> bool {
+        const bool second = at.second;
+        int k0 = second && kb0 < kb_r ? kb_r : kb0;
+        const int k1 = !second && kb1 > kb_r ? kb_r : kb1;
+        if (kGroups == 2) k0 += (at.before + k0 - kb0 + group) & 1;      // the group's first stage
+        if (k0 >= k1) return false;
+        const long long t0 = static_cast<long long>(at.chunk) * BM;
+        x.half = kSrc == kSrcBf16 || (kSrc == kSrcMixed && (second ? p.half_a : p.half_g));
+        x.vec = !x.half && (second ? p.vec_a : p.vec_g);
+        const int size = x.half ? 2 : 4;
+        const long long from = static_cast<long long>(second ? k0 - kb_r : k0) * BK * size;
+        x.pitch = (second ? p.lda : p.ldg) * size;
+        x.at = reinterpret_cast<uintptr_t>(second ? p.a : p.g) + (at.b * p.T + t0) * x.pitch + from;
+        x.bytes = static_cast<long long>(second ? p.n_c : p.n_r) * size - from;
+        x.rows = rows_of(at.chunk);
+        x.slices = (k1 - k0 + kGroups - 1) / kGroups * (x.half ? 1 : 2);
+        x.jump = 128 + (kGroups - 1) * (x.half ? 128 : 256);
         return true;
       };
-      const long long n = (u1 - u0) * (kb1 - kb0);       // this CTA's stages
-      long long fu = u0;
-      int fk = kb0;
-      auto advance = [&](GpRows<kSrc>& q) {
-        if (fu >= u1) return;
-        if (fk == kb0) {
-          const long long b = fu / p.chunks_per_sample, t0 = (fu - b * p.chunks_per_sample) * BM + lw * 16;
-          row = b * p.T + t0;
-          rows_left = p.T - t0;
+      int stage = group; uint32_t phase = 0;
+      int to = 0, from = 0;                              // slots
+      GpAsk<Cfg::kSlotPitch> ask;
+      ask.left = 0;
+      Place asked = start;                               // unit and operand to be requested next
+      auto request = [&]() {
+        while (ask.left == 0 && asked.left > 0) {
+          GpSegment x;
+          if (segment(asked, x)) ask.open(x, lw, lane);
+          advance(asked);
         }
-        fetch(fk, q);
-        if (++fk == kb1) { fk = kb0; ++fu; }
+        if (ask.left > 0) ask.request(smem_u32(mine + to * Cfg::kSlotBytes), lane);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        if (++to == kSlots) to = 0;
       };
-      if (n > 0) advance(set[0]);
-      for (long long i = 0; i < n; i += 2) {
-        advance(set[1]);
-        if (!put(set[0])) break;
-        if (i + 1 >= n) break;
-        advance(set[0]);
-        if (!put(set[1])) break;
+      for (int i = 0; i < kSlots - 1; ++i) request();
+      auto convert = [&](const GpSegment& x, auto half, auto vec) -> bool {
+        constexpr bool kHalf = decltype(half)::value, kVec = decltype(vec)::value;
+        constexpr int kPerStage = kHalf ? 1 : 2;
+        const int off = static_cast<int>((x.at + gp_loader_row(lw, kHalf ? lane >> 3 : lane >> 4) * x.pitch) & 15);
+        long long bytes = x.bytes;
+        for (int n = x.slices; n > 0; n -= kPerStage) {
+          uint8_t* block = smem + stage * Cfg::kStageBytes;
+#pragma unroll
+          for (int part = 0; part < kPerStage; ++part) {
+            request();
+            asm volatile("cp.async.wait_group %0;" ::"n"(kSlots - 1) : "memory");
+            if (part == 0 && !mbar_wait_warp(&empty_bar[stage], phase ^ 1, abort_flag, p.err, 621)) return false;
+            __syncwarp();                                // all lanes' pieces have arrived
+            gp_convert<PARTS, Cfg::kSlotPitch, kHalf, kVec>(block, Cfg::kActAtomBytes, part * 32, mine + from * Cfg::kSlotBytes, off, x.rows, bytes, lw, lane);
+            bytes -= part == kPerStage - 1 ? x.jump : 128;
+            if (++from == kSlots) from = 0;
+            if (part == kPerStage - 1) fence_proxy_async_smem();
+            __syncwarp();                                // all lanes are done with the slot, and with the stage
+          }
+          if (lane == 0) mbar_arrive(&full_bar[stage]);
+          stage += kGroups;
+          if (stage >= kStages) { stage -= kStages; phase ^= 1; }
+        }
+        return true;
+      };
+      bool ok = true;
+      for (Place at = start; ok && at.left > 0; advance(at)) {
+        GpSegment x;
+        if (!segment(at, x)) continue;
+        if constexpr (PARTS == 1) ok = convert(x, std::true_type(), std::false_type());
+        else if (kSrc == kSrcMixed && x.half) ok = convert(x, std::true_type(), std::false_type());
+        else if (x.vec) ok = convert(x, std::false_type(), std::true_type());
+        else ok = convert(x, std::false_type(), std::false_type());
       }
+      asm volatile("cp.async.wait_all;" ::: "memory");
     }
   } else if (warp == 5) {
-    if (lane == 0) {
-      const uint32_t idesc_r = make_idesc_bf16(BM, p.kr_pad, 0, 0);
-      const uint32_t idesc_c = make_idesc_bf16(BM, p.kc_pad, 0, 0);
-      int stage = 0; uint32_t phase = 0; int acc = 0; uint32_t acc_phase = 0; bool ok = true;
-      for (long long u = u0; u < u1 && ok; ++u) {
-        if (!mbar_wait(&acc_empty[acc], acc_phase ^ 1, abort_flag, p.err, 522)) { ok = false; break; }
+    // The whole warp follows the loop, so that what the elected lane's instructions take is the same for all lanes and
+    // lies in uniform registers: a product takes 60 cycles to issue, 100 from inside a branch of one lane (8 x 4096 tokens of
+    // 4096 + 1024 bf16, k = 64: 70.6 -> 68.3 us).
+    const uint32_t idesc_r = make_idesc_bf16(BM, p.kr_pad, 0, 0);
+    const uint32_t idesc_c = make_idesc_bf16(BM, p.kc_pad, 0, 0);
+    const uint64_t a0 = make_smem_desc_sw128(smem_u32(smem), 16, 1024);
+    const uint64_t b0 = make_smem_desc_sw128(smem_u32(smem + (kLoaders ? kStages * Cfg::kStageBytes : Cfg::kActBytes)), 16, 1024);
+    int stage = 0; uint32_t phase = 0; int acc = 0; uint32_t acc_phase = 0; bool ok = true;
+    int ps = 0; uint32_t p_phase = 0;                    // of the projection blocks, where they have a ring of their own
+    for (long long u = u0; u < u1 && ok; ++u) {
+      if (!mbar_wait_warp(&acc_empty[acc], acc_phase ^ 1, abort_flag, p.err, 522)) { ok = false; break; }
+      tc_fence_after_sync();
+      const uint32_t d_r = tmem_base + acc * 256;
+      for (int kb = kb0; kb < kb1; ++kb) {
+        if (kLoaders && !mbar_wait_warp(&proj_full[ps], p_phase, abort_flag, p.err, 524)) { ok = false; break; }
+        if (!mbar_wait_warp(&full_bar[stage], phase, abort_flag, p.err, 523)) { ok = false; break; }
         tc_fence_after_sync();
-        const uint32_t d_r = tmem_base + acc * 256;
-        const uint32_t d_c = d_r + 128;
-        for (int kb = kb0; kb < kb1; ++kb) {
-          if (!mbar_wait(&full_bar[stage], phase, abort_flag, p.err, 523)) { ok = false; break; }
-          tc_fence_after_sync();
-          const uint32_t sa = smem_u32(smem + stage * Cfg::kStageBytes);
-          const bool first = kb < kb_r;
-          const bool fresh = (kb == kb0) || (kb == kb_r);
-          const uint32_t d = first ? d_r : d_c;
-          const uint32_t idesc = first ? idesc_r : idesc_c;
+        const bool first = kb < kb_r;
+        const uint32_t d = first ? d_r : d_r + 128, idesc = first ? idesc_r : idesc_c;
+        const uint32_t more = kb == kb0 || kb == kb_r ? 0u : 1u;
+        const uint64_t adesc = a0 + stage * (Cfg::kStageBytes / 16);
+        const uint64_t bdesc = b0 + (kLoaders ? ps * (Cfg::kProjStageBytes / 16) : stage * (Cfg::kStageBytes / 16));
+        if (elect_one()) {
 #pragma unroll
-          for (int at = 0; at < ATOMS; ++at) {
-            const uint64_t adesc = make_smem_desc_sw128(sa + at * Cfg::kActAtomBytes, 16, 1024);
-            const uint64_t bdesc = make_smem_desc_sw128(sa + ATOMS * PARTS * Cfg::kActAtomBytes + at * Cfg::kProjAtomBytes, 16, 1024);
-#pragma unroll
-            for (int k = 0; k < BK / 16; ++k) {
-              const uint32_t add = (fresh && at == 0 && k == 0) ? 0u : 1u;
-              if constexpr (PARTS == 2) {      // residual parts lie behind the values
-                umma_bf16(d, adesc + 2 * k + Cfg::kActAtomBytes / 16, bdesc + 2 * k, idesc, add);
-                umma_bf16(d, adesc + 2 * k, bdesc + 2 * k + Cfg::kProjAtomBytes / 16, idesc, 1u);
-                umma_bf16(d, adesc + 2 * k, bdesc + 2 * k, idesc, 1u);
-              } else {
-                umma_bf16(d, adesc + 2 * k, bdesc + 2 * k, idesc, add);
-              }
+          for (int k = 0; k < ATOMS * BK / 16; ++k) {
+            const uint64_t ak = adesc + (k / 4) * (Cfg::kActAtomBytes / 16) + 2 * (k % 4), bk = bdesc + (k / 4) * (Cfg::kProjAtomBytes / 16) + 2 * (k % 4);
+            if constexpr (PARTS == 2) {      // residual parts lie behind the values
+              umma_bf16(d, ak + Cfg::kActAtomBytes / 16, bk, idesc, k == 0 ? more : 1u);
+              umma_bf16(d, ak, bk + Cfg::kProjAtomBytes / 16, idesc, 1u);
+              umma_bf16(d, ak, bk, idesc, 1u);
+            } else {
+              umma_bf16(d, ak, bk, idesc, k == 0 ? more : 1u);
             }
           }
           umma_commit(&empty_bar[stage]);
-          if (++stage == kStages) { stage = 0; phase ^= 1; }
+          if (kLoaders) umma_commit(&proj_empty[ps]);
+          if (kb == kb1 - 1) umma_commit(&acc_full[acc]);
         }
-        if (ok) umma_commit(&acc_full[acc]);
-        if (++acc == 2) { acc = 0; acc_phase ^= 1; }
+        __syncwarp();
+        if (++stage == kStages) { stage = 0; phase ^= 1; }
+        if (kLoaders && ++ps == kProjStages) { ps = 0; p_phase ^= 1; }
       }
+      if (++acc == 2) { acc = 0; acc_phase ^= 1; }
     }
   } else {
     // ------------------------------------------------------------ epilogue: warps 0-3
@@ -441,44 +667,14 @@ gradproj_kernel(const __grid_constant__ CUtensorMap tm_g, const __grid_constant_
     int acc = 0; uint32_t acc_phase = 0;
     const uint32_t lane_base = static_cast<uint32_t>(warp * 32) << 16;
 
-    auto flush = [&](int b) {
-      float* dst = p.out + static_cast<long long>(b) * p.out_stride;
-#pragma unroll
-      for (int i = 0; i < RT; ++i) {
-        const int r = ty * RT + i;
-#pragma unroll
-        for (int j = 0; j < CT; ++j) {
-          const int c = tx * CT + j;
-          if (r < p.k_r && c < p.k_c && o[i][j] != 0.f)
-            atomicAdd(dst + static_cast<long long>(r) * p.out_ld + c, o[i][j] * p.scale);
-          o[i][j] = 0.f;
-        }
-      }
-    };
     // This CTA, or the cluster, has all of sample b: its block goes through shared memory -- a cluster's through that of the
-    // stages, which nothing is on its way to any more -- and each CTA adds up and stores its share, in rank order.
+    // stages, which nothing is on its way to any more -- and each CTA adds up and stores its share.
     auto store = [&](int b) {
       float* block = ranks > 1 ? reinterpret_cast<float*>(smem) : s_r;            // [KMAX][KMAX]
-#pragma unroll
-      for (int i = 0; i < RT; ++i)
-#pragma unroll
-        for (int j = 0; j < CT; j += 4) {
-          *reinterpret_cast<float4*>(&block[(ty * RT + i) * KMAX + tx * CT + j]) = make_float4(o[i][j], o[i][j + 1], o[i][j + 2], o[i][j + 3]);
-          o[i][j] = o[i][j + 1] = o[i][j + 2] = o[i][j + 3] = 0.f;
-        }
+      gp_put_block<KMAX>(block, ty, tx, o);
       if (ranks > 1) cluster_sync_all();
       else named_bar_sync(1, 128);
-      float* dst = p.out + static_cast<long long>(b) * p.out_stride;
-#pragma unroll 1
-      for (int e = static_cast<int>(rank) * 128 + tid; e < p.k_r * KMAX; e += static_cast<int>(ranks) * 128) {
-        if (e % KMAX >= p.k_c) continue;
-        float sum = block[e];
-        if (ranks > 1) {
-          sum = 0.f;
-          for (uint32_t k = 0; k < ranks; ++k) sum += gp_ld_cluster1(map_to_cta(smem_u32(block + e), k));
-        }
-        dst[static_cast<long long>(e / KMAX) * p.out_ld + e % KMAX] = sum * p.scale;
-      }
+      gp_store_block<KMAX, 2>(p, b, block, rank, ranks, tid, 128);
       if (ranks == 1) named_bar_sync(1, 128);
     };
     // TMEM -> shared (fp32): row `tid` of one projected block
@@ -522,37 +718,11 @@ gradproj_kernel(const __grid_constant__ CUtensorMap tm_g, const __grid_constant_
       }
     };
 
-    // out[r, c] += sum over staged rows [t0, t1) of s_r[t][r] * s_c[t][c]
-    auto contract = [&](int t0, int t1) {
-#pragma unroll 4
-      for (int t = t0; t < t1; ++t) {
-        float rr[RT], cc[CT];
-        if constexpr (RT >= 4) {
-#pragma unroll
-          for (int i = 0; i < RT; i += 4)
-            *reinterpret_cast<float4*>(&rr[i]) = *reinterpret_cast<const float4*>(&s_r[gp_staged_index<KMAX>(t, ty * RT + i)]);
-        } else {
-          *reinterpret_cast<float2*>(&rr[0]) = *reinterpret_cast<const float2*>(&s_r[gp_staged_index<KMAX>(t, ty * RT)]);
-        }
-#pragma unroll
-        for (int j = 0; j < CT; j += 4)
-          *reinterpret_cast<float4*>(&cc[j]) = *reinterpret_cast<const float4*>(&s_c[gp_staged_index<KMAX>(t, tx * CT + j)]);
-#pragma unroll
-        for (int i = 0; i < RT; ++i)
-#pragma unroll
-          for (int j = 0; j < CT; ++j) o[i][j] = fmaf(rr[i], cc[j], o[i][j]);
-      }
-    };
-
     if constexpr (kCluster != kNone) {
-      // One unit.  Row `tid` of this CTA's partial blocks is staged; rows [first, first + share) of all CTAs' blocks are
-      // then added up here, in place: nobody else reads them from this CTA.
-      const int most = (BM + static_cast<int>(ranks) - 1) / static_cast<int>(ranks), first = static_cast<int>(rank) * most;
-      const int share = first + most < BM ? most : BM - first;
-      const int b = static_cast<int>(u0 / p.chunks_per_sample);
-      const long long t_first = u0 % p.chunks_per_sample * BM;
+      // One unit: row `tid` of this CTA's partial blocks is staged
+      const long long t_first = static_cast<long long>(chunk0) * BM;
       const bool owned = tid >= first && tid < first + share;
-      if constexpr (kEmb) { if (owned) gather(b, t_first + tid); }
+      if constexpr (kEmb) { if (owned) gather(b0, t_first + tid); }
       bool alive = true;
       if (kb1 > kb0) alive = named_bar_and(2, 128, mbar_wait(&acc_full[0], 0, abort_flag, p.err, 124));
       if (alive) {
@@ -566,39 +736,12 @@ gradproj_kernel(const __grid_constant__ CUtensorMap tm_g, const __grid_constant_
             for (int q = 0; q < kRowQuads; ++q) *reinterpret_cast<float4*>(&s_c[gp_staged_index<KMAX>(tid, 4 * q)]) = mine[q];
         }
       }
-      cluster_sync_all();
-      if (alive) {
-        // ranks [0, last_r] hold columns of G, [first_c, ranks) columns of A
-        auto begin = [&](int r) { return static_cast<int>(static_cast<unsigned>(r) * kb_total / ranks); };
-        auto add_up = [&](float* block, int kpad, bool of_r) {
-          const int quads = kpad / 4;
-          for (int i = tid; i < share * quads; i += 128) {
-            float* at = &block[gp_staged_index<KMAX>(first + i / quads, i % quads * 4)];
-            float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 4
-            for (int r = 0; r < static_cast<int>(ranks); ++r) {
-              const int s0 = begin(r), s1 = begin(r + 1);
-              if (s0 == s1 || (of_r ? s0 >= kb_r : s1 <= kb_r)) continue;
-              const float4 v = gp_ld_cluster(map_to_cta(smem_u32(at), r));
-              sum.x += v.x; sum.y += v.y; sum.z += v.z; sum.w += v.w;
-            }
-            *reinterpret_cast<float4*>(at) = sum;
-          }
-        };
-        add_up(s_r, p.kr_pad, true);
-        if (!kEmb) add_up(s_c, p.kc_pad, false);
-        named_bar_sync(1, 128);
-        contract(first, first + share);
-        if constexpr (kCluster == kSome) flush(b);
-      }
-      if constexpr (kCluster == kWhole) store(b);
     }
     // (one place that stores or adds and no wide counters: with two places the embedding form of float32 and unaligned rows spilled
     // more registers, 237 us for 16 x 2048 tokens of 4000 float32, k = 64, and 200 as it is; 65 and 59 for 701)
     if constexpr (kCluster == kNone) {
       bool alive = true;
-      int b = static_cast<int>(u0 / p.chunks_per_sample);
-      int chunk = static_cast<int>(u0 % p.chunks_per_sample);
+      int b = b0, chunk = chunk0;
       // a cluster's CTA without a unit takes part in the storing too
 #pragma unroll 1
       for (long long left = u1 - u0; left > 0 || p.group > 1; --left) {
@@ -624,14 +767,15 @@ gradproj_kernel(const __grid_constant__ CUtensorMap tm_g, const __grid_constant_
               if (lane == 0) mbar_arrive(&acc_empty[acc]);     // four arrivals per tile, one per warp
             }
             named_bar_sync(1, 128);                            // the four epilogue warps only
-            contract(0, Cfg::kStageRows);
+            const int here = rows_of(chunk) - half * Cfg::kStageRows;
+            gp_contract<KMAX>(s_r, s_c, 0, here < Cfg::kStageRows ? here : Cfg::kStageRows, ty, tx, o);
             named_bar_sync(1, 128);
           }
           if (++acc == 2) { acc = 0; acc_phase ^= 1; }
         }
-        if (++chunk == p.chunks_per_sample || left <= 1) {     // done with the sample, or with this CTA's part of it
+        if (++chunk == chunks || left <= 1) {     // done with the sample, or with this CTA's part of it
           if (p.direct) store(b);
-          else flush(b);
+          else gp_add_block<KMAX>(p, b, ty, tx, o);
           if (p.group > 1) break;
           chunk = 0;
           ++b;
@@ -641,12 +785,40 @@ gradproj_kernel(const __grid_constant__ CUtensorMap tm_g, const __grid_constant_
     }
   }
 
-  if (kCluster != kNone || p.group > 1) {
-    if (warp >= 4) {
-      if constexpr (kCluster != kNone) cluster_sync_all();        // the epilogue's barrier before the partial blocks are added up
-      if (kCluster != kSome) cluster_sync_all();                  // and the one before the results are
+  if constexpr (kCluster != kNone) {
+    // All warps: rows [first, first + share) of all CTAs' blocks are added up here, in place, as nobody else reads them from this CTA.
+    // Ranks with columns of G have a bit in `of_r`, those with columns of A in `of_c`.
+    const int s0 = static_cast<int>(static_cast<unsigned>(lane) * kb_total / ranks), s1 = static_cast<int>(static_cast<unsigned>(lane + 1) * kb_total / ranks);
+    const bool some = lane < static_cast<int>(ranks) && s0 < s1;
+    const uint32_t of_r = __ballot_sync(0xffffffffu, some && s0 < kb_r), of_c = __ballot_sync(0xffffffffu, some && s1 > kb_r);
+    cluster_sync_all();
+    const int quads_r = share * (p.kr_pad / 4), quads = quads_r + (kEmb ? 0 : share * (p.kc_pad / 4));
+    for (int i = threadIdx.x; i < quads; i += Cfg::kThreads) {
+      const bool r = i < quads_r;
+      const int e = r ? i : i - quads_r, per = (r ? p.kr_pad : p.kc_pad) / 4;
+      float* at = (r ? s_r : s_c) + gp_staged_index<KMAX>(first + e / per, e % per * 4);
+      *reinterpret_cast<float4*>(at) = gp_cluster_sum<8>(at, r ? of_r : of_c);
+    }
+    __syncthreads();
+    const int ty = threadIdx.x >> 3, tx = threadIdx.x & 7;         // of the first 128 threads
+    if (warp < 4) {
+      float o[RT][CT];
+#pragma unroll
+      for (int i = 0; i < RT; ++i)
+#pragma unroll
+        for (int j = 0; j < CT; ++j) o[i][j] = 0.f;
+      if (!*abort_flag) gp_contract<KMAX>(s_r, s_c, first, first + share, ty, tx, o);
+      if (kCluster == kSome) gp_add_block<KMAX>(p, b0, ty, tx, o);
+      else gp_put_block<KMAX>(reinterpret_cast<float*>(smem), ty, tx, o);
+    }
+    if constexpr (kCluster == kWhole) {
+      cluster_sync_all();
+      gp_store_block<KMAX, 8>(p, b0, reinterpret_cast<const float*>(smem), rank, ranks, threadIdx.x, Cfg::kThreads);
     }
     cluster_sync_all();                    // no CTA leaves while another reads its blocks
+  } else if (p.group > 1) {
+    if (warp >= 4) cluster_sync_all();     // the epilogue's before the results are added up
+    cluster_sync_all();
   }
   tc_fence_before_sync();
   __syncthreads();
@@ -656,7 +828,7 @@ gradproj_kernel(const __grid_constant__ CUtensorMap tm_g, const __grid_constant_
 template <int KMAX, int kSrc, bool kEmb, int kCluster>
 static int launch_gradproj_t(const CUtensorMap& tg, const CUtensorMap& tpr, const CUtensorMap& ta, const CUtensorMap& tpc,
                              GpParams& p, int ranks, const DeviceState* ds, cudaStream_t st) {
-  using Cfg = GpCfg<KMAX, kSrc, kCluster>;
+  using Cfg = GpCfg<KMAX, kSrc, kEmb, kCluster>;
   static bool attr_set[64] = {};
   if (!attr_set[ds->device]) {
     GB_CUDA_OK(cudaFuncSetAttribute(gradproj_kernel<KMAX, kSrc, kEmb, kCluster>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -693,7 +865,7 @@ static int launch_gradproj_t(const CUtensorMap& tg, const CUtensorMap& tpr, cons
 // the call takes two rounds: 17.5 us against 32.1 for 48 x 100 tokens of 640 + 640, k = 40, in threes.)
 template <int KMAX, int kSrc, bool kEmb, int kCluster>
 static int gradproj_resident(int ranks, const DeviceState* ds) {
-  using Cfg = GpCfg<KMAX, kSrc, kCluster>;
+  using Cfg = GpCfg<KMAX, kSrc, kEmb, kCluster>;
   static std::atomic<int> known[64][9];      // count + 1; several threads may find the same
   std::atomic<int>& slot = known[ds->device][ranks];
   int n = slot.load(std::memory_order_relaxed);
@@ -721,15 +893,18 @@ static int gradproj_resident(int ranks, const DeviceState* ds) {
 }
 
 // CTAs that share a unit: as many as are resident with one unit per cluster.
-// * Short chains of small ranks stay alone: the cluster's barriers and the exchange cost about 2 us, a stage is 0.5 us of a unit's
-//   chain, the contraction, which the CTAs share too, 1 us at 32 x 32 and 3 at 64 x 64 (32 x 64 tokens of 256 + 256 columns, four
-//   stages, k = 32: 10.3 us alone, 11.3 in pairs; 12 x 1 token of 128 + 2112, k = 44: 23.6 alone, 13.1 in eights).
+// * Short chains of small ranks stay alone: the cluster's barriers and the exchange cost about 1.5 us, a stage 0.3 to 0.6 us of a unit's
+//   chain, the contraction, which the CTAs share too, 1 us at 32 x 32 and 3 at 64 x 64.  (Four to seven stages, k <= 32, alone and in
+//   clusters: 56 x 2 tokens of 321 float32, embedding form, 11.8 and 9.4 us; 2 x 165 of 107 + 166 float32 13.9 and 11.1; 14 x 80 of
+//   134 + 192 bf16 10.1 and 8.8.  Fewer: 23 x 117 of 256 + 64 bf16 12.2 and 12.8.)  Rows that TMA reads in several units a sample, whose
+//   results are then added and not stored, from eight stages on: 2 x 281 of 384 + 128 bf16 9.1 alone, 11.1 in clusters.
 // * Three or six share unevenly, which pays from so many stages on (17 x 60 of 640 + 640, ten stages: 13.9 us in fours, 14.8 in sixes;
 //   20 x 100 of 9792 + 4160 bf16 21.0 and 16.9; 9 x 464 of the same float32 154 in pairs, 109 in threes).
 // * Fives lost (24 units of 32 stages: 26.3 us, 24.7 in fours).
 template <int KMAX, int kSrc, bool kEmb>
-static int gradproj_ranks(long long units, int stages, const DeviceState* ds) {
-  if ((stages < 8 && KMAX <= 32) || 2 * units > ds->sm_count) return 1;
+static int gradproj_ranks(long long units, int chunks, int stages, const DeviceState* ds) {
+  const int least = kSrc == kSrcTma && chunks > 1 ? 8 : 4;
+  if ((stages < least && KMAX <= 32) || 2 * units > ds->sm_count) return 1;
   for (const int r : {8, 6, 4, 3, 2}) {
     if ((r == 6 && stages < 18) || (r == 3 && stages < 8)) continue;
     if (r * units <= ds->sm_count && units <= gradproj_resident<KMAX, kSrc, kEmb, kSome>(r, ds)) return r;
@@ -764,9 +939,9 @@ struct GpOperands {
 
 template <int KMAX, int kSrc, bool kEmb>
 static int launch_gradproj_src(const GpOperands& o, GpParams& p, const DeviceState* ds, cudaStream_t st) {
-  constexpr int kCols = GpCfg<KMAX, kSrc, kNone>::ATOMS * 64;
+  constexpr int kCols = GpCfg<KMAX, kSrc, kEmb, kNone>::ATOMS * 64;
   const int stages = ceil_div(p.n_r, kCols) + (kEmb ? 0 : ceil_div(p.n_c, kCols));
-  const int ranks = gradproj_ranks<KMAX, kSrc, kEmb>(p.units, stages, ds);
+  const int ranks = gradproj_ranks<KMAX, kSrc, kEmb>(p.units, p.chunks_per_sample, stages, ds);
   p.group = ranks > 1 || p.accumulate ? 1 : gradproj_group<KMAX, kSrc, kEmb>(p.B, p.chunks_per_sample, ds);
   // a sample's tokens are one CTA's or one cluster's: the results are stored, else added to zeros (written before the host
   // is busy with the tensor maps)

@@ -1425,6 +1425,40 @@ def test_gradproj_dense_of_mixed_operands(case, f32):
     assert torch.cuda.memory_stats()["allocation.all.allocated"] == made      # workspaces are kept from the first call
 
 
+# Rows that begin anywhere, between values that nothing may take in: every distance of the first row from a 16-byte boundary, pitches of
+# all residues, tokens around the eights that loader warps share and the tile, columns around a slice of 128 bytes and a stage of 64;
+# stages of both groups of warps, and fewer than groups
+@pytest.mark.parametrize("kinds", [("bf16", "bf16"), ("f32", "f32"), ("f32", "bf16"), ("bf16", "f32")])
+@pytest.mark.parametrize("case", [(1, 1, 1, 3, 9, 5), (2, 7, 31, 33, 9, 33), (1, 130, 63, 65, 32, 17), (3, 128, 64, 127, 4, 4), (2, 9, 96, 97, 64, 40),
+                                  (160, 16, 66, 161, 8, 8), (150, 255, 35, 129, 40, 64), (1, 15, 1021, 700, 33, 64), (20, 33, 515, 258, 12, 12)])
+def test_gradproj_rows_that_begin_anywhere(case, kinds):
+    B, T, n_r, n_c, k_r, k_c = case
+    types = {"bf16": torch.bfloat16, "f32": torch.float32}
+    g = torch.Generator(device="cuda").manual_seed(31)
+    P_r, P_c = (torch.randn(k, n, generator=g, device="cuda") / k ** 0.5 for k, n in ((k_r, n_r), (k_c, n_c)))
+    split = "f32" in kinds
+    P = [ops().prepare_projection(x, split) for x in (P_r, P_c)]
+    bound = 2 * 2.0 ** -15 if split else 2 * 2.0 ** -8         # as in the test of unit counts and widths
+    for offset in range(8):
+        x = []
+        for kind, n in zip(kinds, (n_r, n_c)):
+            buf = torch.full((B * T * n + 16,), float("nan"), device="cuda").to(types[kind])
+            view = buf[offset:offset + B * T * n].view(B, T, n)
+            view.copy_(torch.randn(B, T, n, generator=g, device="cuda"))
+            x.append(view)
+        out = ops().gradproj_dense(x[0], x[1], P[0], P[1], k_r, k_c, 1.0, torch.full((B, k_r * k_c), 7.0, device="cuda"))
+        after()
+        ref = torch.einsum("btr,btc->brc", x[0].double() @ P_r.double().t(), x[1].double() @ P_c.double().t())
+        assert O.rel_fro(out.cpu(), ref.flatten(1).cpu()) < bound
+        if kinds[0] == kinds[1]:
+            ids = torch.randint(0, 50, (B, T), generator=g, device="cuda")
+            rows = torch.randn(k_c, 50, generator=g, device="cuda")
+            out = ops().gradproj_embedding(ids, x[0], P[0], ops().prepare_embedding_projection(rows), k_r, k_c)
+            after()
+            ref = torch.einsum("btr,btc->brc", x[0].double() @ P_r.double().t(), rows.double().t()[ids])
+            assert O.rel_fro(out.reshape(B, -1).cpu(), ref.flatten(1).cpu()) < bound
+
+
 # both sides of what sends rows through the ring (16 MB of float32, 128 of bf16, more than 16 rows on either side); one CTA to a block
 # of scores; eight splits and nine
 @pytest.mark.parametrize("n1,n2,D,dtype", [
