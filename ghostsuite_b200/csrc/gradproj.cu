@@ -308,7 +308,8 @@ __device__ __forceinline__ float4 gp_ld_cluster(uint32_t addr) {
 }
 
 // Element-wise sum, in rank order, of four floats that lie at `at` in the shared memory of those CTAs of the cluster that have a bit
-// in `mask`.  BATCH loads go out together, all eight where registers are free: one after the other they took most of a small call (5 x 4 tokens of 368 + 448 float32, k = 42,
+// in `mask`.  BATCH loads go out together, all eight where registers are free (in the loop over units one, as two cost it registers: 32 x 2000
+// tokens of 128 float32, embedding form, k = 64: 63.5 -> 66.3 us): one after the other they took most of a small call (5 x 4 tokens of 368 + 448 float32, k = 42,
 // cycles: partial blocks 5850, results 3850 of 24000).
 template <int BATCH>
 __device__ __forceinline__ float4 gp_cluster_sum(const float* at, uint32_t mask) {
@@ -621,7 +622,9 @@ gradproj_kernel(const __grid_constant__ CUtensorMap tm_g, const __grid_constant_
     int stage = 0; uint32_t phase = 0; int acc = 0; uint32_t acc_phase = 0; bool ok = true;
     int ps = 0; uint32_t p_phase = 0;                    // of the projection blocks, where they have a ring of their own
     for (long long u = u0; u < u1 && ok; ++u) {
-      if (!mbar_wait_warp(&acc_empty[acc], acc_phase ^ 1, abort_flag, p.err, 522)) { ok = false; break; }
+      int w = 1;                             // one lane polls: the epilogue is on the same schedulers
+      if (lane == 0) w = mbar_wait(&acc_empty[acc], acc_phase ^ 1, abort_flag, p.err, 522) ? 1 : 0;
+      if (!__shfl_sync(0xffffffffu, w, 0)) { ok = false; break; }
       tc_fence_after_sync();
       const uint32_t d_r = tmem_base + acc * 256;
       for (int kb = kb0; kb < kb1; ++kb) {
@@ -674,7 +677,7 @@ gradproj_kernel(const __grid_constant__ CUtensorMap tm_g, const __grid_constant_
       gp_put_block<KMAX>(block, ty, tx, o);
       if (ranks > 1) cluster_sync_all();
       else named_bar_sync(1, 128);
-      gp_store_block<KMAX, 2>(p, b, block, rank, ranks, tid, 128);
+      gp_store_block<KMAX, 1>(p, b, block, rank, ranks, tid, 128);
       if (ranks == 1) named_bar_sync(1, 128);
     };
     // TMEM -> shared (fp32): row `tid` of one projected block
@@ -767,8 +770,12 @@ gradproj_kernel(const __grid_constant__ CUtensorMap tm_g, const __grid_constant_
               if (lane == 0) mbar_arrive(&acc_empty[acc]);     // four arrivals per tile, one per warp
             }
             named_bar_sync(1, 128);                            // the four epilogue warps only
-            const int here = rows_of(chunk) - half * Cfg::kStageRows;
-            gp_contract<KMAX>(s_r, s_c, 0, here < Cfg::kStageRows ? here : Cfg::kStageRows, ty, tx, o);
+            if constexpr (kLoaders) {          // of rows that are not there the block has none
+              const int here = rows_of(chunk) - half * Cfg::kStageRows;
+              gp_contract<KMAX>(s_r, s_c, 0, here < Cfg::kStageRows ? here : Cfg::kStageRows, ty, tx, o);
+            } else {                           // TMA has written zeros
+              gp_contract<KMAX>(s_r, s_c, 0, Cfg::kStageRows, ty, tx, o);
+            }
             named_bar_sync(1, 128);
           }
           if (++acc == 2) { acc = 0; acc_phase ^= 1; }
