@@ -19,9 +19,10 @@
 #include <algorithm>
 #include <map>
 #include <mutex>
-#include <set>
 #include <stdexcept>
 #include <string>
+#include <unordered_map>
+#include <unordered_set>
 #include <utility>
 #include <vector>
 
@@ -61,6 +62,8 @@ template <typename F> PyObject* guarded(F&& f) {
     PyErr_SetString(type ? type : PyExc_RuntimeError, e.what_without_backtrace());
     Py_XDECREF(type);
     Py_XDECREF(mod);
+  } catch (python_error& e) {
+    if (!PyErr_Occurred()) PyErr_SetString(PyExc_RuntimeError, e.what());
   } catch (const std::exception& e) {
     PyErr_SetString(PyExc_RuntimeError, e.what());
   }
@@ -730,6 +733,7 @@ PyObject* py_projection_similarity(PyObject*, PyObject* const* a, Py_ssize_t n) 
 
 // ---- end of a backward pass ---------------------------------------------------------------------------------
 PyObject *k_X, *k_M, *k_sum_out, *k_n_train, *k_n_val, *k_dot_scale, *k_sum_scale, *k_Xv;
+PyObject *k_param, *k_matrix, *k_vector, *k_train_grad, *k_add, *k_parameters, *k_modules, *k_named_modules;
 
 PyObject* item(PyObject* dict, PyObject* key) { return PyDict_GetItemWithError(dict, key); }   // borrowed
 
@@ -778,79 +782,150 @@ ghost_pass_job read_job(PyObject* d, int* device) {
   return j;
 }
 
-// (jobs: list of dicts, matrices: list of [n_val, n_train] tensors) -> list of [n_train] tensors, one per
-// matrix: the jobs' reductions and every listed matrix's sum over the validation samples, one launch
-// per device.  A matrix that a job fills gets its sum from that job.
+// The jobs' reductions and every matrix's sum over the validation samples, one launch per device; the sums, one vector per
+// matrix.  A matrix that a job fills gets its sum from that job.
+std::vector<Tensor> reduce_pass(PyObject* jobs, const std::vector<PyObject*>& mats) {
+  struct OnDevice { int device; Tensor any; std::vector<ghost_pass_job> jobs; };      // a tensor of it, for its stream
+  std::vector<OnDevice> devices;
+  auto on = [&](int device, const Tensor& t) -> size_t {
+    for (size_t i = 0; i < devices.size(); ++i)
+      if (devices[i].device == device) return i;
+    devices.push_back({device, t, {}});
+    devices.back().jobs.reserve(mats.size() + static_cast<size_t>(PyList_GET_SIZE(jobs)));
+    return devices.size() - 1;
+  };
+  struct Filled { size_t device, job; const Tensor* vec; };
+  std::unordered_map<const float*, Filled> filled;
+  for (Py_ssize_t i = 0; i < PyList_GET_SIZE(jobs); ++i) {
+    PyObject* d = PyList_GET_ITEM(jobs, i);
+    int dev = 0;
+    ghost_pass_job j = read_job(d, &dev);
+    if (j.M == nullptr && j.sum_out == nullptr) invalid("small_reduce_batch: a job has no output");
+    const size_t at = on(dev, cuda_tensor(item(d, k_X)));
+    if (j.M) filled[j.M] = {at, devices[at].jobs.size(), nullptr};
+    devices[at].jobs.push_back(j);
+  }
+  std::vector<Tensor> out(mats.size());
+  // one buffer per run of equal column counts keeps the vectors' allocations to one or two
+  for (size_t i = 0; i < mats.size();) {
+    const Tensor first = cuda_tensor(mats[i]);
+    size_t e = i;
+    while (e < mats.size()) {
+      const Tensor& t = cuda_tensor(mats[e]);
+      if (t.scalar_type() != at::kFloat || t.dim() != 2 || !t.is_contiguous())
+        invalid("pass_reduce: matrices are contiguous float32 [n_val, n_train]");
+      if (t.size(1) != first.size(1) || t.get_device() != first.get_device()) break;
+      ++e;
+    }
+    Tensor vecs = empty({static_cast<long long>(e - i), first.size(1)}, first, at::kFloat);
+    for (size_t k = i; k < e; ++k) {
+      const Tensor& t = cuda_tensor(mats[k]);
+      auto it = filled.find(t.data_ptr<float>());
+      if (it != filled.end() && it->second.vec != nullptr) {
+        out[k] = *it->second.vec;           // listed again: a job of its own would read the matrix while the first one writes it
+        continue;
+      }
+      out[k] = vecs.select(0, static_cast<long long>(k - i));
+      float* vp = out[k].data_ptr<float>();
+      if (it != filled.end()) {
+        devices[it->second.device].jobs[it->second.job].vec = vp;
+        it->second.vec = &out[k];
+      } else {
+        ghost_pass_job j = {};
+        j.M = t.data_ptr<float>();
+        j.vec = vp;
+        j.n_val = static_cast<int>(t.size(0));
+        j.n_train = static_cast<int>(t.size(1));
+        devices[on(t.get_device(), t)].jobs.push_back(j);
+      }
+    }
+    i = e;
+  }
+  for (OnDevice& d : devices) {
+    Launch L(d.any);
+    check(ghost_pass_reduce(d.jobs.data(), static_cast<int>(d.jobs.size()), L.st()));
+  }
+  return out;
+}
+
+// (jobs: list of dicts, matrices: list of [n_val, n_train] tensors) -> list of [n_train] tensors, one per matrix
 PyObject* py_pass_reduce(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return guarded([&]() -> PyObject* {
     need(n, 2, "pass_reduce");
     if (!PyList_Check(a[0]) || !PyList_Check(a[1])) invalid("pass_reduce takes two lists");
-    std::map<int, std::vector<ghost_pass_job>> per_device;
-    std::map<int, Tensor> any;               // a tensor of each device, for its stream
-    struct Filled { int device; size_t job; PyObject* vec; };
-    std::map<const float*, Filled> filled;
-    for (Py_ssize_t i = 0; i < PyList_GET_SIZE(a[0]); ++i) {
-      PyObject* d = PyList_GET_ITEM(a[0], i);
-      int dev = 0;
-      ghost_pass_job j = read_job(d, &dev);
-      if (j.M == nullptr && j.sum_out == nullptr) invalid("small_reduce_batch: a job has no output");
-      if (j.M) filled[j.M] = {dev, per_device[dev].size(), nullptr};
-      per_device[dev].push_back(j);
-      any.emplace(dev, cuda_tensor(item(d, k_X)));
-    }
-    const Py_ssize_t n_mats = PyList_GET_SIZE(a[1]);
-    PyObject* out = PyList_New(n_mats);
+    std::vector<PyObject*> mats(static_cast<size_t>(PyList_GET_SIZE(a[1])));
+    for (size_t i = 0; i < mats.size(); ++i) mats[i] = PyList_GET_ITEM(a[1], static_cast<Py_ssize_t>(i));
+    const std::vector<Tensor> vecs = reduce_pass(a[0], mats);
+    PyObject* out = PyList_New(static_cast<Py_ssize_t>(vecs.size()));
     if (!out) throw std::bad_alloc();
-    try {
-      // one buffer per run of equal column counts keeps the vectors' allocations to one or two
-      for (Py_ssize_t i = 0; i < n_mats;) {
-        const Tensor first = cuda_tensor(PyList_GET_ITEM(a[1], i));
-        Py_ssize_t e = i;
-        while (e < n_mats) {
-          const Tensor& t = cuda_tensor(PyList_GET_ITEM(a[1], e));
-          if (t.scalar_type() != at::kFloat || t.dim() != 2 || !t.is_contiguous())
-            invalid("pass_reduce: matrices are contiguous float32 [n_val, n_train]");
-          if (t.size(1) != first.size(1) || t.get_device() != first.get_device()) break;
-          ++e;
-        }
-        Tensor vecs = empty({e - i, first.size(1)}, first, at::kFloat);
-        for (Py_ssize_t k = i; k < e; ++k) {
-          const Tensor& t = cuda_tensor(PyList_GET_ITEM(a[1], k));
-          auto it = filled.find(t.data_ptr<float>());
-          if (it != filled.end() && it->second.vec != nullptr) {
-            // listed again: a job of its own would read the matrix while the first one writes it
-            Py_INCREF(it->second.vec);
-            PyList_SET_ITEM(out, k, it->second.vec);
-            continue;
-          }
-          Tensor v = vecs.select(0, k - i);
-          float* vp = v.data_ptr<float>();
-          PyObject* wrapped = wrap(v);
-          PyList_SET_ITEM(out, k, wrapped);
-          if (it != filled.end()) {
-            per_device[it->second.device][it->second.job].vec = vp;
-            it->second.vec = wrapped;
-          } else {
-            ghost_pass_job j = {};
-            j.M = t.data_ptr<float>();
-            j.vec = vp;
-            j.n_val = static_cast<int>(t.size(0));
-            j.n_train = static_cast<int>(t.size(1));
-            per_device[t.get_device()].push_back(j);
-            any.emplace(t.get_device(), t);
-          }
-        }
-        i = e;
-      }
-      for (auto& [dev, jobs] : per_device) {
-        Launch L(any.at(dev));
-        check(ghost_pass_reduce(jobs.data(), static_cast<int>(jobs.size()), L.st()));
-      }
-    } catch (...) {
-      Py_DECREF(out);
-      throw;
-    }
+    for (size_t i = 0; i < vecs.size(); ++i) PyList_SET_ITEM(out, static_cast<Py_ssize_t>(i), wrap(vecs[i]));
     return out;
+  });
+}
+
+// A new reference that is given up at the end of the scope; null: a Python error is set.
+struct Owned {
+  PyObject* o;
+  explicit Owned(PyObject* p) : o(p) {
+    if (!o) throw python_error();
+  }
+  Owned(const Owned&) = delete;
+  Owned& operator=(const Owned&) = delete;
+  ~Owned() { Py_DECREF(o); }
+};
+// The instance dictionary of a parameter (a tensor of any class)
+PyObject* instance_dict(PyObject* o) { return PyObject_GenericGetDict(o, nullptr); }
+void set_item(PyObject* dict, PyObject* key, PyObject* value) {
+  if (PyDict_SetItem(dict, key, value) != 0) throw python_error();
+}
+
+// (jobs: list of dicts, dots: list of (parameter, matrix), observer or None) -> whether it was done: all matrices are on GPUs.
+// The hooks' lists at the end of a backward pass: pass_reduce, the vectors as <parameter>.grad_dot_prod, and the jobs'
+// train gradients as <parameter>.train_grad or added to it.  A parameter that is listed again keeps its last matrix, as it does
+// when every hook overwrites the attribute.
+PyObject* py_finish_pass(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    need(n, 3, "finish_pass");
+    if (!PyList_Check(a[0]) || !PyList_Check(a[1])) invalid("finish_pass takes two lists");
+    std::vector<PyObject*> params, mats;
+    std::unordered_map<PyObject*, size_t> where;
+    for (Py_ssize_t i = 0; i < PyList_GET_SIZE(a[1]); ++i) {
+      PyObject* e = PyList_GET_ITEM(a[1], i);
+      if (!PyTuple_Check(e) || PyTuple_GET_SIZE(e) != 2) invalid("finish_pass: pairs of a parameter and its matrix");
+      PyObject *param = PyTuple_GET_ITEM(e, 0), *m = PyTuple_GET_ITEM(e, 1);
+      if (!tensor(m).is_cuda()) Py_RETURN_FALSE;
+      const auto [it, is_new] = where.emplace(param, params.size());
+      if (is_new) {
+        params.push_back(param);
+        mats.push_back(m);
+      } else {
+        mats[it->second] = m;
+      }
+    }
+    const std::vector<Tensor> vecs = reduce_pass(a[0], mats);
+    for (size_t i = 0; i < vecs.size(); ++i) {
+      Owned own(instance_dict(params[i]));
+      if (item(own.o, k_matrix) != mats[i]) continue;
+      Owned v(wrap(vecs[i]));
+      set_item(own.o, k_vector, v.o);
+    }
+    for (Py_ssize_t i = 0; i < PyList_GET_SIZE(a[0]); ++i) {
+      PyObject *job = PyList_GET_ITEM(a[0], i), *param = item(job, k_param), *grad = item(job, k_sum_out);
+      if (!present(param) || !present(grad)) continue;
+      const Tensor &g = tensor(grad), &p = tensor(param);
+      Owned mine(g.sizes() == p.sizes() ? Py_NewRef(grad) : wrap(g.view(p.sizes())));
+      Owned own(instance_dict(param));
+      PyObject* sum = item(own.o, k_train_grad);
+      if (sum == nullptr) {
+        set_item(own.o, k_train_grad, mine.o);
+      } else {
+        const Owned added(PyObject_CallMethodOneArg(sum, k_add, mine.o));
+      }
+      if (present(a[2])) {
+        const Owned told(PyObject_CallOneArg(a[2], param));
+      }
+    }
+    Py_RETURN_TRUE;
   });
 }
 
@@ -885,46 +960,45 @@ PyObject* py_matrix_sum(PyObject*, PyObject* const* a, Py_ssize_t n) {
 // modules in a way of its own, and the caller asks torch.
 struct Walk {
   PyObject* named_modules;
-  std::set<PyObject*> seen;              // modules and parameters
-  std::set<PyTypeObject*> plain;         // module types with torch's own listing
+  std::unordered_set<PyObject*> seen;                // modules and parameters
+  std::unordered_set<PyTypeObject*> plain;           // module types with torch's own listing
 };
 bool walk_parameters(PyObject* module, const std::string& prefix, Walk& walk, PyObject* out) {
-  std::set<PyObject*>& seen = walk.seen;
-  if (!seen.insert(module).second) return true;
+  if (!walk.seen.insert(module).second) return true;
   if (walk.plain.find(Py_TYPE(module)) == walk.plain.end()) {
-    PyObject* listing = PyObject_GetAttrString(reinterpret_cast<PyObject*>(Py_TYPE(module)), "named_modules");
+    PyObject* listing = PyObject_GetAttr(reinterpret_cast<PyObject*>(Py_TYPE(module)), k_named_modules);
     if (!listing) PyErr_Clear();
     const bool own = listing != walk.named_modules;
     Py_XDECREF(listing);
     if (own) return false;
     walk.plain.insert(Py_TYPE(module));
   }
-  PyObject* dict = PyObject_GetAttrString(module, "__dict__");
+  PyObject* dict = PyObject_GenericGetDict(module, nullptr);
   if (!dict) { PyErr_Clear(); return false; }
+  Owned hold(dict);
   PyObject *key, *value;
   Py_ssize_t pos = 0;
-  PyObject* params = PyDict_Check(dict) ? PyDict_GetItemString(dict, "_parameters") : nullptr;
-  PyObject* modules = PyDict_Check(dict) ? PyDict_GetItemString(dict, "_modules") : nullptr;
-  bool ok = params && PyDict_Check(params) && modules && PyDict_Check(modules) && !PyDict_GetItemString(dict, "named_modules");
-  if (ok) {
-    while (PyDict_Next(params, &pos, &key, &value)) {
-      if (value == Py_None || !seen.insert(value).second) continue;
-      const char* name = PyUnicode_AsUTF8(key);
-      PyObject* entry = Py_BuildValue("(sO)", (prefix + (name ? name : "")).c_str(), value);
-      if (!entry || PyList_Append(out, entry) != 0) { Py_XDECREF(entry); Py_DECREF(dict); throw std::bad_alloc(); }
-      Py_DECREF(entry);
-    }
+  PyObject *params = item(dict, k_parameters), *modules = item(dict, k_modules);
+  if (!params || !PyDict_Check(params) || !modules || !PyDict_Check(modules) || item(dict, k_named_modules)) return false;
+  while (PyDict_Next(params, &pos, &key, &value)) {
+    if (value == Py_None || !walk.seen.insert(value).second) continue;
+    Py_ssize_t size = 0;
+    const char* name = PyUnicode_AsUTF8AndSize(key, &size);
+    if (!name) throw python_error();
+    const std::string full = prefix + std::string(name, static_cast<size_t>(size));
+    Owned text(PyUnicode_FromStringAndSize(full.data(), static_cast<Py_ssize_t>(full.size())));
+    Owned entry(PyTuple_Pack(2, text.o, value));
+    if (PyList_Append(out, entry.o) != 0) throw python_error();
   }
-  if (ok) {
-    pos = 0;
-    while (ok && PyDict_Next(modules, &pos, &key, &value)) {
-      if (value == Py_None) continue;
-      const char* name = PyUnicode_AsUTF8(key);
-      ok = walk_parameters(value, prefix + (name ? name : "") + ".", walk, out);
-    }
+  pos = 0;
+  while (PyDict_Next(modules, &pos, &key, &value)) {
+    if (value == Py_None) continue;
+    Py_ssize_t size = 0;
+    const char* name = PyUnicode_AsUTF8AndSize(key, &size);
+    if (!name) throw python_error();
+    if (!walk_parameters(value, prefix + std::string(name, static_cast<size_t>(size)) + ".", walk, out)) return false;
   }
-  Py_DECREF(dict);
-  return ok;
+  return true;
 }
 
 PyObject* py_named_parameters(PyObject*, PyObject* const* a, Py_ssize_t n) {
@@ -1021,7 +1095,8 @@ PyMethodDef kMethods[] = {
     GB_METHOD(norm_persample),    GB_METHOD(embedding_dot),
     GB_METHOD(embedding_wgrad),   GB_METHOD(gradproj_dense),
     GB_METHOD(gradproj_embedding), GB_METHOD(projection_similarity),
-    GB_METHOD(pass_reduce),       GB_METHOD(matrix_sum),
+    GB_METHOD(pass_reduce),       GB_METHOD(finish_pass),
+    GB_METHOD(matrix_sum),
     GB_METHOD(dense_hook),        GB_METHOD(conv_hook),
     GB_METHOD(norm_hook),
     GB_METHOD(embedding_hook),    GB_METHOD(named_parameters),
@@ -1039,7 +1114,11 @@ extern "C" __attribute__((visibility("default"), used)) const char ghost_torch_b
 PyMODINIT_FUNC PyInit__ghost_torch() {
   struct { PyObject** at; const char* name; } keys[] = {{&k_X, "X"}, {&k_M, "M"}, {&k_sum_out, "sum_out"}, {&k_n_train, "n_train"},
                                                         {&k_n_val, "n_val"}, {&k_dot_scale, "dot_scale"},
-                                                        {&k_sum_scale, "sum_scale"}, {&k_Xv, "Xv"}};
+                                                        {&k_sum_scale, "sum_scale"}, {&k_Xv, "Xv"}, {&k_param, "param"},
+                                                        {&k_matrix, "grad_dot_prod_matrix"}, {&k_vector, "grad_dot_prod"},
+                                                        {&k_train_grad, "train_grad"}, {&k_add, "add_"},
+                                                        {&k_parameters, "_parameters"}, {&k_modules, "_modules"},
+                                                        {&k_named_modules, "named_modules"}};
   for (auto& k : keys) *k.at = PyUnicode_InternFromString(k.name);
   return PyModule_Create(&kModule);
 }

@@ -219,7 +219,7 @@ def _prepare_sample_grad_or_dotprod(layer: nn.Module, grad_output: Tuple[torch.T
 
 
 _PASS_ATTRIBUTES = ("activations", "backprops", "_ghost_backprop_scale", "_ghost_val_batch", "_ghost_colsums",
-                    "_ghost_bias_grad", "_ghost_norm_grads", "_ghost_cached_train_grad", "_ghost_ln_cache", "_ghost_conv_tokens")
+                    "_ghost_bias_grad", "_ghost_jobs", "_ghost_norm_grads", "_ghost_cached_train_grad", "_ghost_ln_cache", "_ghost_conv_tokens")
 
 
 def _apply_train_grad(layer: nn.Module, val_batch_size: int, loss_reduction: str = "mean"):
@@ -268,6 +268,8 @@ def _train_grad_bias_from_layer(layer: nn.Module, val_batch_size: int, loss_redu
     if loss_reduction == "mean":
         scale /= n_train
     bias = _param(layer, "bias")
+    if _layers._sum_into_job(own, bias, colsums, n_train, scale, own.get("_ghost_bias_grad")):
+        return
     out_dtype = torch.bfloat16 if bias.dtype is torch.bfloat16 else torch.float32
     _layers._train_grad_from_vectors(bias, colsums, n_train, scale, out_dtype, own.get("_ghost_bias_grad"))
 

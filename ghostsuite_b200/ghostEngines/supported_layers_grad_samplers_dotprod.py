@@ -245,6 +245,8 @@ def finalize_pending_dots() -> None:
         return
     if small:
         _exchange_pending_val_rows(small)        # validation rows of a batch split over ranks
+    if ops.finish_pass(small or [], pending or [], TRAIN_GRAD_OBSERVER):
+        return
     last = {id(item[0]): item for item in pending or ()}
     on_device = [item for item in last.values() if item[1].is_cuda]
     if small or on_device:
@@ -273,6 +275,43 @@ def _set_dot(param: torch.Tensor, M: torch.Tensor) -> None:
             _PENDING_DOTS.append((param, M))
     # inside a backward pass a placeholder until it ends
     own["grad_dot_prod"] = M if deferred else M.sum(dim=0)
+
+
+def _record_hook(own: dict, n_train: int, n_val: int, entries) -> None:
+    """What a layer's backward hook leaves for the end of the pass, in one visit to the lists: for every
+    ``(parameter, M, X)`` the dot products of the parameter, whose matrix exists (``X`` None) or is the Gram of
+    the layer's per-sample vectors ``X``.  The jobs on vectors are kept in ``_ghost_jobs`` with the list
+    they stand in, for the train gradients that are asked for next (:func:`_sum_into_job`)."""
+    jobs = {}
+    with _PENDING_LOCK:
+        dots, small = _PENDING_DOTS, _PENDING_SMALL
+        if dots is not None:
+            for param, M, X in entries:
+                if X is not None:
+                    jobs[id(param)] = job = {"X": X, "n_train": n_train, "n_val": n_val, "M": M, "dot_scale": 1.0}
+                    small.append(job)
+                dots.append((param, M))
+    if dots is None:                 # no backward pass in flight
+        for param, M, X in entries:
+            _set_dot(param, M if X is None else _gram_of_vectors(X, n_val, M))
+        return
+    for param, M, _ in entries:
+        has = param.__dict__
+        has["grad_dot_prod_matrix"] = M
+        has["grad_dot_prod"] = M         # a placeholder until the pass ends
+    if jobs:
+        own["_ghost_jobs"] = (small, jobs)
+
+
+def _sum_into_job(own: dict, param: torch.Tensor, X: torch.Tensor, n_train: int, scale: float, out) -> bool:
+    """Let the job that :func:`_record_hook` has put up for ``param`` add up its train rows into ``out`` too.
+    False when there is none, or none that is still to run."""
+    small, jobs = own.get("_ghost_jobs", (None, None))
+    job = None if out is None or small is None or small is not _PENDING_SMALL else jobs.get(id(param))
+    if job is None or job["X"] is not X or job["n_train"] != n_train or "sum_out" in job:
+        return False
+    job["sum_out"], job["sum_scale"], job["param"] = out, scale, param
+    return True
 
 
 def _check_batch(A, B, val_batch_size: int) -> int:
@@ -368,7 +407,10 @@ def _exchange_pending_val_rows(jobs) -> None:
     """One all-gather for the validation rows of every job that waits for them: each rank sends its
     jobs' rows packed one after the other; job ``j`` then reads row ``r * per_rank + i`` at
     ``gathered[r, offset_j + i * F]`` (``ops.small_reduce_batch``)."""
-    waiting = [j for j in jobs if "val_exchange" in j and j["val_exchange"] is not None and j.get("M") is not None]
+    waiting = [j for j in jobs if "val_exchange" in j]
+    if not waiting:
+        return
+    waiting = [j for j in waiting if j["val_exchange"] is not None and j.get("M") is not None]
     if not waiting:
         return
     ex = waiting[0]["val_exchange"]
@@ -497,9 +539,10 @@ def _dense_hook(layer: nn.Module, A: torch.Tensor, B: torch.Tensor, n_val: int, 
         bias is not None, bias_dtype, PATH_RULE == "cost" and own.get("_ghost_rule_choice") is use_gram, FUSE_BIAS_COLSUMS)
     if grad is not None:
         own["_ghost_cached_train_grad"] = (A.data_ptr(), B.data_ptr(), A.size(0), grad)
-    _set_dot(weight, M)
-    if bias is not None:
-        _set_dot(bias, _gram_of_vectors(colsums, n_val, bias_M))
+    if bias is None:
+        _record_hook(own, n_train, n_val, ((weight, M, None),))
+    else:
+        _record_hook(own, n_train, n_val, ((weight, M, None), (bias, bias_M, colsums)))
         own["_ghost_colsums"] = colsums
         own["_ghost_bias_grad"] = bias_grad
 
@@ -612,9 +655,8 @@ def _norm_hook(layer: nn.Module, A: torch.Tensor, B: torch.Tensor, n_val: int, e
     key = (A.data_ptr(), B.data_ptr(), A.size(0))
     own["_ghost_ln_cache"] = (key, gw) if rms else (key, gw, gb)
     own["_ghost_norm_grads"] = (sw, sb)
-    _set_dot(weight, _gram_of_vectors(gw, n_val, Mw))
-    if bias is not None:
-        _set_dot(bias, _gram_of_vectors(gb, n_val, Mb))
+    entries = ((weight, Mw, gw),) if bias is None else ((weight, Mw, gw), (bias, Mb, gb))
+    _record_hook(own, key[2] - n_val, n_val, entries)
     return True
 
 
@@ -639,11 +681,13 @@ def _compute_layernorm_train_grad(layer: nn.LayerNorm, A: torch.Tensor, B: torch
         raise ValueError("No training samples to compute gradients, check batch sizes.")
     gw, gb = _layernorm_vectors(layer, A, B)
     layer.__dict__.pop("_ghost_ln_cache", None)
+    own = layer.__dict__
     scale = _backprop_scale(layer) / n_train
-    sw, sb = layer.__dict__.pop("_ghost_norm_grads", (None, None))
+    sw, sb = own.pop("_ghost_norm_grads", (None, None))
     weight, bias = _param(layer, "weight"), _param(layer, "bias")
-    _train_grad_from_vectors(weight, gw, n_train, scale, weight.dtype, sw)
-    if bias is not None:
+    if not _sum_into_job(own, weight, gw, n_train, scale, sw):
+        _train_grad_from_vectors(weight, gw, n_train, scale, weight.dtype, sw)
+    if bias is not None and not _sum_into_job(own, bias, gb, n_train, scale, sb):
         _train_grad_from_vectors(bias, gb, n_train, scale, bias.dtype, sb)
     return None
 
@@ -691,7 +735,8 @@ def _compute_rmsnorm_train_grad(layer: nn.Module, A: torch.Tensor, B: torch.Tens
     layer.__dict__.pop("_ghost_ln_cache", None)
     scale = _backprop_scale(layer) / n_train
     sw, _ = layer.__dict__.pop("_ghost_norm_grads", (None, None))
-    _train_grad_from_vectors(layer.weight, gw, n_train, scale, layer.weight.dtype, sw)
+    if not _sum_into_job(layer.__dict__, layer.weight, gw, n_train, scale, sw):
+        _train_grad_from_vectors(layer.weight, gw, n_train, scale, layer.weight.dtype, sw)
     return None
 
 
@@ -754,9 +799,10 @@ def _conv_hook(layer: nn.Conv2d, A: torch.Tensor, B: torch.Tensor, n_val: int) -
         own["_ghost_backprop_scale"] / n_train, bias is not None, bias_dtype)
     if grad is not None:
         own["_ghost_cached_train_grad"] = (A.data_ptr(), B.data_ptr(), A.size(0), grad)
-    _set_dot(weight, M)
-    if bias is not None:
-        _set_dot(bias, _gram_of_vectors(sums, n_val, bias_M))
+    if bias is None:
+        _record_hook(own, n_train, n_val, ((weight, M, None),))
+    else:
+        _record_hook(own, n_train, n_val, ((weight, M, None), (bias, bias_M, sums)))
         own["_ghost_colsums"] = sums
         own["_ghost_bias_grad"] = bias_grad
     return True

@@ -315,6 +315,8 @@ def _finish_exchange_job(job: dict) -> None:
 
 def finish_exchange_jobs() -> None:
     """Launch the streaming pass of every layer that still waits for its all-gather."""
+    if not _exchange_jobs:
+        return
     for key in list(_exchange_jobs):
         for job in _exchange_jobs.pop(key):
             _finish_exchange_job(job)
@@ -448,6 +450,17 @@ def pass_reduce(jobs: list, matrices: list) -> list:
         return _native().pass_reduce(jobs, matrices)
     with _Timed("pass_reduce_kernel", "hbm", 0.0, 4.0 * sum(j["X"].numel() for j in jobs)):
         return _native().pass_reduce(jobs, matrices)
+
+
+def finish_pass(jobs: list, dots: list, observer) -> bool:
+    """:func:`pass_reduce` for the lists that the hooks fill, and what follows it, in one native call: every
+    ``(parameter, matrix)`` of ``dots`` -- a parameter's last one counts -- gets its vector as
+    ``parameter.grad_dot_prod``, if ``grad_dot_prod_matrix`` still is that matrix, and the train gradient of every
+    job with a ``param`` becomes ``param.train_grad`` or is added to it, whereupon ``observer(param)`` is called.
+    False, with nothing done, when a matrix is not on a GPU or the library calls are timed one by one."""
+    if _timing is not None or (dots and not dots[0][1].is_cuda) or not _lib.binding_present():
+        return False
+    return _native().finish_pass(jobs, dots, observer)
 
 
 def matrix_sum(matrices: list) -> torch.Tensor:
