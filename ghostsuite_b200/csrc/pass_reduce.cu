@@ -5,6 +5,7 @@
 #include <string.h>
 
 #include <cooperative_groups.h>
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -24,8 +25,10 @@ static constexpr int kPassCluster = 8;
 static constexpr int kPassThreads = 256;
 // Columns staged at a time: a CTA's whole share up to kPassMost, so that one round of loads serves it and the sums of
 // the train rows come out of the same copy (32 + 8 vectors of 3072: two rounds and a second pass over the
-// rows 10.8 us, 9.5 now; of 768: 6.7 and 5.0); no more than the list's longest vector needs, which leaves room for the CTAs of other kernels.
-static constexpr int kPassMost = 512;
+// rows 10.8 us, 9.5 now; of 768: 6.7 and 5.0); no more than the list's longest vector needs, which leaves room for the CTAs of other kernels, and half of
+// kPassMost where the launch has more CTAs than three quarters of the SMs, which would wait for their memory then (32 + 8 vectors
+// of 8192, one job 22.2 us in halves and 18.0 whole; 24 jobs 25.6 and 49).
+static constexpr int kPassMost = 1024;
 __host__ __device__ constexpr int pass_pitch(int sub) { return sub + 4; }      // rows 16 bytes apart modulo 128: no bank conflicts
 // 32 train rows, then nv validation rows; behind them the warps' partial sums
 __host__ __device__ constexpr int pass_smem(int sub, int nv) { return (32 + nv) * pass_pitch(sub) * 4 + 8 * nv * 32 * 4; }
@@ -41,21 +44,17 @@ __device__ __forceinline__ const float* pass_val_row(const ghost_pass_job& j, in
                                static_cast<long long>(v % j.v_per_rank) * j.F;
 }
 
-// Columns [f, f + width) of the block's rows from row `first` on (0: train rows, 32: validation rows) into shared memory,
-// zero up to the next multiple of four
-template <int NV>
-__device__ __forceinline__ void pass_stage(const ghost_pass_job& j, bool vec, int b0, int v0, int f, int width, float* st,
-                                           int pitch, int first) {
+// Columns [f, f + width) of `train` train rows from b0 on and `val` validation rows from v0 on into shared memory, from rows 0 and 32 on,
+// zero up to the next multiple of four.  Rows that are not there stay what they were: what their lanes make of them is not
+// read.  (3 + 1 vectors of 8192: 18.1 us with 36 rows of zeros and two rounds of 512 columns, 12.7 so; 48 jobs of 8 + 2 41 and 28.8.)
+__device__ __forceinline__ void pass_stage(const ghost_pass_job& j, bool vec, int b0, int train, int v0, int val, int f, int width, float* st,
+                                           int pitch) {
   const int quads = (width + 3) / 4;
-  for (int i = threadIdx.x; i < (32 + NV - first) * quads; i += kPassThreads) {
-    const int row = i / quads, r = row + first, q = (i - row * quads) * 4;
-    const float* src;
-    if (r < 32) src = b0 + r < j.n_train ? j.X + static_cast<long long>(b0 + r) * j.F : nullptr;
-    else src = v0 + r - 32 < j.n_val ? pass_val_row(j, v0 + r - 32) : nullptr;
+  for (int i = threadIdx.x; i < (train + val) * quads; i += kPassThreads) {
+    const int row = i / quads, r = row < train ? row : row - train + 32, q = (i - row * quads) * 4;
+    const float* src = row < train ? j.X + static_cast<long long>(b0 + row) * j.F : pass_val_row(j, v0 + row - train);
     float* dst = st + r * pitch + q;
-    if (src == nullptr) {
-      *reinterpret_cast<float4*>(dst) = make_float4(0.f, 0.f, 0.f, 0.f);
-    } else if (vec) {                    // F is a multiple of four then, and so is every width
+    if (vec) {                    // F is a multiple of four then, and so is every width
       asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))),
                    "l"(src + f + q) : "memory");
     } else {
@@ -115,6 +114,7 @@ __device__ __forceinline__ void pass_row_sums(const ghost_pass_job& j, int f0, i
 }
 
 // The same sums, bit for bit, from the staged columns of a block that holds all train rows
+template <bool ALL>      // the block is full: no tests (32 + 8 vectors of 4096: 16.2 us with them, 13.8 without)
 __device__ __forceinline__ void pass_staged_sums(const ghost_pass_job& j, int f, int width, const float* st, int pitch) {
   for (int c = threadIdx.x; c < width; c += kPassThreads) {
     float s = 0.f;
@@ -122,7 +122,7 @@ __device__ __forceinline__ void pass_staged_sums(const ghost_pass_job& j, int f,
     for (int w = 0; w < 8; ++w) {
       float a = 0.f;
 #pragma unroll
-      for (int n = 0; n < 32; n += 8) a += st[(n + w) * pitch + c];
+      for (int n = 0; n < 32; n += 8) a += ALL || n + w < j.n_train ? st[(n + w) * pitch + c] : 0.f;
       s += a;
     }
     s *= j.sum_scale;
@@ -186,27 +186,37 @@ pass_reduce_kernel(const __grid_constant__ PassJobs<CAP> jobs) {
     for (int blk = blockIdx.y; blk < n_blk; blk += step) {
       const int b = blk * 32 + lane;
       const bool live = b < j.n_train;
+      const int train = j.n_train - blk * 32 < 32 ? j.n_train - blk * 32 : 32;
       float col = 0.f;                     // rank 0: this thread's share of vec
       for (int v0 = 0; v0 < j.n_val; v0 += NV, buf ^= 1) {
         float4 acc[NV];                    // a sum per quarter of the columns: short chains, as one warp per pair had
 #pragma unroll
         for (int i = 0; i < NV; ++i) acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        const int val = j.n_val - v0 < NV ? j.n_val - v0 : NV;
         for (int f = f0; f < f1; f += jobs.sub) {
           const int width = f1 - f < jobs.sub ? f1 - f : jobs.sub;
           __syncthreads();
           // one round holds all columns: the train rows are there already
-          pass_stage<NV>(j, vec, blk * 32, v0, f, width, stage, pitch, v0 > 0 && chunk <= jobs.sub ? 32 : 0);
+          pass_stage(j, vec, blk * 32, v0 > 0 && chunk <= jobs.sub ? 0 : train, v0, val, f, width, stage, pitch);
           __syncthreads();
-          if (staged_sums && v0 == 0) pass_staged_sums(j, f, width, stage, pitch);
-          for (int q = warp * 4; q < width; q += 32) {
-            const float4 x = *reinterpret_cast<const float4*>(stage + lane * pitch + q);
-#pragma unroll
-            for (int i = 0; i < NV; ++i) {
-              const float4 y = *reinterpret_cast<const float4*>(stage + (32 + i) * pitch + q);
-              acc[i].x = fmaf(x.x, y.x, acc[i].x); acc[i].y = fmaf(x.y, y.y, acc[i].y);
-              acc[i].z = fmaf(x.z, y.z, acc[i].z); acc[i].w = fmaf(x.w, y.w, acc[i].w);
-            }
+          if (staged_sums && v0 == 0) {
+            if (train == 32) pass_staged_sums<true>(j, f, width, stage, pitch);
+            else pass_staged_sums<false>(j, f, width, stage, pitch);
           }
+          auto products = [&](auto all) {      // all: NV rows, no tests (24 jobs of 32 + 8 vectors of 4096: 19.4 us with them, 15.9 without)
+            for (int q = warp * 4; q < width; q += 32) {
+              const float4 x = *reinterpret_cast<const float4*>(stage + lane * pitch + q);
+#pragma unroll
+              for (int i = 0; i < NV; ++i) {
+                if (!decltype(all)::value && i >= val) break;
+                const float4 y = *reinterpret_cast<const float4*>(stage + (32 + i) * pitch + q);
+                acc[i].x = fmaf(x.x, y.x, acc[i].x); acc[i].y = fmaf(x.y, y.y, acc[i].y);
+                acc[i].z = fmaf(x.z, y.z, acc[i].z); acc[i].w = fmaf(x.w, y.w, acc[i].w);
+              }
+            }
+          };
+          if (val == NV) products(std::true_type());
+          else products(std::false_type());
         }
         float* red = stage + (32 + NV) * pitch;        // [warp][validation row][train lane]
 #pragma unroll
@@ -348,7 +358,8 @@ static int launch_pass(const ghost_pass_job* jobs, int n, int blocks, const Devi
     if (jobs[i].X != nullptr && jobs[i].F > longest) longest = jobs[i].F;
   const int sub = (pass_chunk(longest) + 31) / 32 * 32;
   // the row sums of longer lists reduce 8 x 4 x 128 partial sums in the same memory
-  batch.sub = sub < 128 ? 128 : sub > kPassMost ? kPassMost : sub;
+  const int most = static_cast<long long>(blocks) * n * kPassCluster * 4 <= ds->sm_count * 3ll ? kPassMost : kPassMost / 2;
+  batch.sub = sub < 128 ? 128 : sub > most ? most : sub;
   GB_CUDA_OK(launch_next(pass_reduce_kernel<CAP, NV>, dim3(dim3(kPassCluster, blocks, n)), dim3(kPassThreads), pass_smem(batch.sub, NV), st, batch));
   count_launch();
   return post_launch("pass_reduce_kernel");

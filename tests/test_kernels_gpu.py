@@ -987,6 +987,25 @@ def test_pass_reduce_of_many_validation_rows(n_t, n_v, F):
     assert ((S.double() - T.sum(0)).abs() <= n_t * 2.0 ** -24 * T.abs().sum(0)).all()
 
 
+# fewer rows than a block has lanes, behind a launch that left NaN in the shared memory of every SM; a share of columns in one round and two
+@pytest.mark.parametrize("n_t,n_v", [(1, 1), (3, 1), (31, 7), (33, 9)])
+@pytest.mark.parametrize("F", [30, 8192, 8201])
+def test_pass_reduce_reads_only_rows_that_exist(n_t, n_v, F):
+    o = ops()
+    X = torch.randn(n_t + n_v, F, generator=torch.Generator().manual_seed(6)).cuda()
+    bad = torch.full((48, 8200), float("nan"), device="cuda")
+    spoilt = [{"X": bad, "n_train": 32, "n_val": 16, "M": torch.empty(16, 32, device="cuda")} for _ in range(24)]
+    o.pass_reduce(spoilt, [j["M"] for j in spoilt[:1]])
+    M, S = torch.full((n_v, n_t), 7.0, device="cuda"), torch.full((F,), 7.0, device="cuda")
+    vec, = o.pass_reduce([{"X": X, "n_train": n_t, "n_val": n_v, "M": M, "sum_out": S}], [M])
+    after()
+    T, V = X[:n_t].double(), X[n_t:].double()
+    bound = (F / 256 + 10) * 2.0 ** -24 * (V.abs() @ T.abs().t())        # as above
+    assert ((M.double() - V @ T.t()).abs() <= bound).all()
+    assert ((vec.double() - M.double().sum(0)).abs() <= (n_v / 8 + 3) * 2.0 ** -24 * M.double().abs().sum(0)).all()
+    assert ((S.double() - T.sum(0)).abs() <= n_t * 2.0 ** -24 * T.abs().sum(0)).all()
+
+
 # one matrix on its own, beyond what the batched launch's blocks take: vector and scalar loads, remainders
 @pytest.mark.parametrize("n_t,n_v,F", [(300, 30, 772), (2000, 3, 1001), (70, 40, 4100), (5, 3, 150001), (600, 8, 512)])
 def test_small_gram_of_large_vectors(n_t, n_v, F):
