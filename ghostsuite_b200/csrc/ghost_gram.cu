@@ -16,6 +16,8 @@
 //   warp  5    TMEM allocator + MMA issuer (one elected lane)
 // Pipeline: kStages shared-memory stages (train tile 128xBK + val tile BNxBK bf16 in 64-element atoms, 128B swizzle),
 // full/empty mbarriers per stage, acc_full/acc_empty mbarriers per accumulator buffer.
+#include <atomic>
+
 #include "common.cuh"
 #include "gram_operands.cuh"
 #include "sm100_ptx.cuh"
@@ -29,6 +31,7 @@ struct GramParams {
   int n_train, n_val;
   int ka, kg;         // contraction lengths (elements) of the activation / out-grad operands
   int m_tiles, n_tiles;
+  int ranks;          // CTAs that share a tile
   int round_mode;     // 0: fp32 product of fp32 Grams; 1: round Grams and product to bf16
   float scale;
   float* M;           // [n_val, n_train]
@@ -51,13 +54,91 @@ struct GramCfg {
   static constexpr int kSmemBytes = kStages * kStageBytes + 1024 /*align*/ + 256 /*barriers*/;
 };
 
-template <int BN, int PARTS>
-__global__ void __launch_bounds__(192, 1)
+// Adds the sums of a warp's 32 rows, `b` their train samples (-1: none), for validation sample v: once if all rows are of one sample.
+struct GramRows {
+  int b, b_first;
+  bool uniform;
+  __device__ __forceinline__ GramRows(const GramParams& p, long long row) {
+    b = row < p.rows_t ? static_cast<int>(row / p.T) : -1;
+    // rows are ascending, so the warp covers one train sample iff its first and last rows agree
+    b_first = __shfl_sync(0xffffffffu, b, 0);
+    uniform = b_first == __shfl_sync(0xffffffffu, b, 31) && b_first >= 0;
+  }
+  __device__ __forceinline__ void flush(const GramParams& p, float val, int v) const {
+    if (v >= p.n_val) return;
+    val *= p.scale;
+    if (uniform) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) val += __shfl_xor_sync(0xffffffffu, val, o);
+      if ((threadIdx.x & 31) == 0) atomicAdd(&p.M[static_cast<long long>(v) * p.n_train + b_first], val);
+    } else if (b >= 0) {
+      atomicAdd(&p.M[static_cast<long long>(v) * p.n_train + b], val);
+    }
+  }
+};
+
+__device__ __forceinline__ float gram_product(const GramParams& p, float x, float y) {
+  return p.round_mode == 0 ? x * y : bf16_round(bf16_round(x) * bf16_round(y));
+}
+
+// Four columns of an accumulator, summed in rank order over the CTAs of `mask`; the loads of all eight go out together
+__device__ __forceinline__ float4 gram_cluster_sum(const uint8_t* at, uint32_t mask) {
+  float4 v[8], sum = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+  for (int r = 0; r < 8; ++r)
+    if (mask >> r & 1) v[r] = ld_cluster_v4(map_to_cta(smem_u32(at), r));
+#pragma unroll
+  for (int r = 0; r < 8; ++r)
+    if (mask >> r & 1) { sum.x += v[r].x; sum.y += v[r].y; sum.z += v[r].z; sum.w += v[r].w; }
+  return sum;
+}
+
+// The columns of share `part` of `parts` of a tile whose partial accumulators lie in the cluster's shared memory ([column / 4][row][4] floats,
+// the activations' accumulator before the gradients'); a row a thread,
+// at which `smem` points.
+template <int BM, int BN>
+__device__ __forceinline__ void gram_split(const GramParams& p, const uint8_t* smem, uint32_t has_a, uint32_t has_g, int part, int parts,
+                                           long long row, long long n0) {
+  const GramRows rows(p, row);
+  const int quads = static_cast<int>((p.rows_v - n0 < BN ? p.rows_v - n0 : BN) + 3) / 4;
+  const int q0 = quads * part / parts, q1 = quads * (part + 1) / parts;
+  if (q0 == q1) return;
+  int v = static_cast<int>((n0 + 4 * q0) / p.T);
+  long long boundary = static_cast<long long>(v + 1) * p.T - n0;       // tile-relative column
+  float sum = 0.f;
+  for (int q = q0; q < q1; ++q) {
+    const float4 a = gram_cluster_sum(smem + q * BM * 16, has_a);
+    const float4 g = gram_cluster_sum(smem + (BN / 4 + q) * BM * 16, has_g);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      if (4 * q + e == boundary) {
+        rows.flush(p, sum, v++);
+        sum = 0.f;
+        boundary += p.T;
+      }
+      sum += gram_product(p, e == 0 ? a.x : e == 1 ? a.y : e == 2 ? a.z : a.w, e == 0 ? g.x : e == 1 ? g.y : e == 2 ? g.z : g.w);
+    }
+  }
+  rows.flush(p, sum, v);
+}
+
+// In a cluster the partial accumulators are laid out, fetched and multiplied by sixteen warps: with four, whose loads from
+// the other CTAs' shared memory wait on one another, it took 2 us longer.
+constexpr int gram_threads(bool split) { return split ? 512 : 192; }
+
+// SPLIT: a cluster shares a tile.  Its CTAs take equal runs of the K steps of both operands, lay their partial accumulators out in
+// the shared memory that the stages leave free, and each sums, multiplies and reduces its share of the columns over
+// the cluster (gram_split).  A tile alone is bound by what one SM has in flight, 0.53 us a step of 128 K elements whatever
+// the rest of the GPU does (0.61 a step of 64 in two parts): 4 + 2 x 64 tokens of 768 -> 20000 are two tiles, 97.3 us on two CTAs and
+// 27.6 on sixteen; float32 216 and 52.  The sums of the partial accumulators are rounded, where the tensor core's truncate.
+template <int BN, int PARTS, bool SPLIT>
+__global__ void __launch_bounds__(gram_threads(SPLIT), 1)
 ghost_gram_kernel(const __grid_constant__ CUtensorMap tm_at, const __grid_constant__ CUtensorMap tm_av,
                   const __grid_constant__ CUtensorMap tm_gt, const __grid_constant__ CUtensorMap tm_gv,
                   const GramParams p) {
   using Cfg = GramCfg<BN, PARTS>;
   static_assert(PARTS == 1 || BN == 128, "two parts of wider tiles leave two stages");
+  static_assert(!SPLIT || 2 * 128 * BN * 4 <= Cfg::kStages * Cfg::kStageBytes, "partial accumulators lie in the stages");
   constexpr int BM = Cfg::BM, BK = Cfg::BK, kStages = Cfg::kStages, kAccBufs = Cfg::kAccBufs;
 
   extern __shared__ uint8_t smem_raw[];
@@ -87,6 +168,11 @@ ghost_gram_kernel(const __grid_constant__ CUtensorMap tm_at, const __grid_consta
   };
   const int kb_a = (p.ka + BK - 1) / BK;
   const int kb_total = kb_a + (p.kg + BK - 1) / BK;
+  const int ranks = SPLIT ? p.ranks : 1;                   // CTAs of a tile
+  const int rank = SPLIT ? static_cast<int>(cluster_ctarank()) : 0;
+  auto k_first = [&](int r) { return SPLIT ? static_cast<int>(static_cast<long long>(kb_total) * r / ranks) : r * kb_total; };
+  const int kb0 = k_first(rank), kb1 = k_first(rank + 1);
+  const int tile0 = SPLIT ? blockIdx.x / ranks : blockIdx.x, tile_step = SPLIT ? num_tiles : gridDim.x;    // a cluster has one tile
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
@@ -122,12 +208,12 @@ ghost_gram_kernel(const __grid_constant__ CUtensorMap tm_at, const __grid_consta
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
-      for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
+      for (int tile = tile0; tile < num_tiles && ok; tile += tile_step) {
         int tm, tn;
         tile_coords(tile, tm, tn);
         const int m0 = tm * BM;
         const int n0 = tn * BN;
-        for (int kb = 0; kb < kb_total; ++kb) {
+        for (int kb = kb0; kb < kb1; ++kb) {
           if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag, p.err, 401)) { ok = false; break; }
           uint8_t* st = smem + stage * Cfg::kStageBytes;
           mbar_arrive_expect_tx(&full_bar[stage], Cfg::kStageBytes);
@@ -159,16 +245,16 @@ ghost_gram_kernel(const __grid_constant__ CUtensorMap tm_at, const __grid_consta
       int acc = 0;
       uint32_t acc_phase = 0;
       bool ok = true;
-      for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
+      for (int tile = tile0; tile < num_tiles && ok; tile += tile_step) {
         if (!mbar_wait(&acc_empty[acc], acc_phase ^ 1, abort_flag, p.err, 502)) { ok = false; break; }
         tc_fence_after_sync();
         const uint32_t d_a = tmem_base + acc * (2 * BN);
         const uint32_t d_g = d_a + BN;
-        for (int kb = 0; kb < kb_total; ++kb) {
+        for (int kb = kb0; kb < kb1; ++kb) {
           if (!mbar_wait(&full_bar[stage], phase, abort_flag, p.err, 503)) { ok = false; break; }
           tc_fence_after_sync();
           const uint32_t sa = smem_u32(smem + stage * Cfg::kStageBytes);
-          const bool first = (kb == 0) || (kb == kb_a);
+          const bool first = (kb == kb0) || (kb == kb_a);
           const uint32_t dst = (kb < kb_a) ? d_a : d_g;
 #pragma unroll
           for (int a = 0; a < BK / Cfg::kAtomK; ++a) {
@@ -193,6 +279,8 @@ ghost_gram_kernel(const __grid_constant__ CUtensorMap tm_at, const __grid_consta
         if (++acc == kAccBufs) { acc = 0; acc_phase ^= 1; }
       }
     }
+  } else if constexpr (SPLIT) {
+    if (warp < 4) mbar_wait_warp(&acc_full[0], 0, abort_flag, p.err, 104);
   } else {
     // ------------------------------------------------------------------ epilogue (warps 0-3)
     int acc = 0;
@@ -207,30 +295,13 @@ ghost_gram_kernel(const __grid_constant__ CUtensorMap tm_at, const __grid_consta
       tc_fence_after_sync();
 
       const long long row = m0 + threadIdx.x;
-      const bool row_ok = row < p.rows_t;
-      const int b = row_ok ? static_cast<int>(row / p.T) : -1;
-      // rows are ascending, so the warp covers one train sample iff its first and last rows agree
-      const int b_first = __shfl_sync(0xffffffffu, b, 0);
-      const int b_last = __shfl_sync(0xffffffffu, b, 31);
-      const bool warp_uniform = (b_first == b_last) && (b_first >= 0);
+      const GramRows rows(p, row);
 
       int cur_v = static_cast<int>(n0 / p.T);
       long long boundary = static_cast<long long>(cur_v + 1) * p.T - n0;   // tile-relative column
       float sum = 0.f;
       const uint32_t t_a = tmem_base + lane_base + acc * (2 * BN);
       const uint32_t t_g = t_a + BN;
-
-      auto flush = [&](float val, int v) {
-        if (v >= p.n_val) return;
-        val *= p.scale;
-        if (warp_uniform) {
-#pragma unroll
-          for (int o = 16; o > 0; o >>= 1) val += __shfl_xor_sync(0xffffffffu, val, o);
-          if (lane == 0) atomicAdd(&p.M[static_cast<long long>(v) * p.n_train + b_first], val);
-        } else if (row_ok) {
-          atomicAdd(&p.M[static_cast<long long>(v) * p.n_train + b], val);
-        }
-      };
 
 #pragma unroll 1
       for (int c0 = 0; c0 < BN; c0 += 32) {
@@ -251,13 +322,12 @@ ghost_gram_kernel(const __grid_constant__ CUtensorMap tm_at, const __grid_consta
 #pragma unroll
           for (int j = 0; j < 32; ++j) {
             if (c0 + j == boundary) {
-              flush(sum, cur_v);
+              rows.flush(p, sum, cur_v);
               sum = 0.f;
               ++cur_v;
               boundary += p.T;
             }
-            const float x = __uint_as_float(ra[j]), y = __uint_as_float(rg[j]);
-            sum += (p.round_mode == 0) ? x * y : bf16_round(bf16_round(x) * bf16_round(y));
+            sum += gram_product(p, __uint_as_float(ra[j]), __uint_as_float(rg[j]));
           }
         }
       }
@@ -265,9 +335,40 @@ ghost_gram_kernel(const __grid_constant__ CUtensorMap tm_at, const __grid_consta
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive(&acc_empty[acc]);
-      flush(sum, cur_v);
+      rows.flush(p, sum, cur_v);
       if (++acc == kAccBufs) { acc = 0; acc_phase ^= 1; }
     }
+  }
+
+  if constexpr (SPLIT) {
+    __syncthreads();                                       // the accumulators are complete, the stages free
+    tc_fence_after_sync();
+    int tm, tn;
+    tile_coords(tile0, tm, tn);
+    const int row = threadIdx.x & 127, grp = threadIdx.x >> 7;         // a lane of tensor memory is read by warps of its quarter
+    const long long m0 = static_cast<long long>(tm) * BM, n0 = static_cast<long long>(tn) * BN;
+    if (*abort_flag == 0) {
+      const uint32_t t_acc = tmem_base + (static_cast<uint32_t>(row & 96) << 16);
+#pragma unroll 1
+      for (int c0 = grp * 32; c0 < 2 * BN; c0 += 128) {    // the activations' accumulator, then the gradients'
+        if ((c0 < BN ? kb0 >= kb_a : kb1 <= kb_a) || (c0 & (BN - 1)) >= p.rows_v - n0) continue;
+        uint32_t r[32];
+        tmem_ld32(t_acc + c0, r);
+        tmem_ld_wait();
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+          st_shared_v4(smem + ((c0 / 4 + q) * BM + row) * 16, r[4 * q], r[4 * q + 1], r[4 * q + 2], r[4 * q + 3]);
+      }
+    }
+    tc_fence_before_sync();
+    cluster_sync_all();
+    uint32_t has_a = 0, has_g = 0;                         // CTAs with a partial of either accumulator
+    for (int r = 0; r < ranks; ++r) {
+      has_a |= static_cast<uint32_t>(k_first(r) < kb_a) << r;
+      has_g |= static_cast<uint32_t>(k_first(r + 1) > kb_a) << r;
+    }
+    gram_split<BM, BN>(p, smem + row * 16, has_a, has_g, rank * 4 + grp, ranks * 4, m0 + row, n0);
+    cluster_sync_all();                                    // no CTA leaves while another still reads its shared memory
   }
 
   // ------------------------------------------------------------------ teardown
@@ -291,6 +392,62 @@ int gram_maps(CUtensorMap (&t)[4], const GramOperands& o, long long rows_t, long
   return gram_map(&t[3], o, o.g_v, rows_v, o.kg, o.ld_gv, box_v);
 }
 
+template <int BN, int PARTS, bool SPLIT>
+static int gram_smem_attr(const DeviceState* ds) {
+  static bool attr_set[64] = {};
+  if (!attr_set[ds->device]) {
+    GB_CUDA_OK(cudaFuncSetAttribute(ghost_gram_kernel<BN, PARTS, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    GramCfg<BN, PARTS>::kSmemBytes));
+    attr_set[ds->device] = true;
+  }
+  return GHOST_OK;
+}
+
+// Clusters of `ranks` CTAs that the device holds at a time (the driver's count, asked once per device and size), or 0
+template <int PARTS>
+static int gram_resident(int ranks, const DeviceState* ds) {
+  static std::atomic<int> known[64][9];      // count + 1; several threads may find the same
+  std::atomic<int>& slot = known[ds->device][ranks];
+  int n = slot.load(std::memory_order_relaxed);
+  if (n == 0) {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = ranks;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.gridDim = dim3(ranks, 1, 1);
+    cfg.blockDim = dim3(gram_threads(true), 1, 1);
+    cfg.dynamicSmemBytes = GramCfg<128, PARTS>::kSmemBytes;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    int count = 0;
+    if (gram_smem_attr<128, PARTS, true>(ds) != GHOST_OK ||
+        cudaOccupancyMaxActiveClusters(&count, ghost_gram_kernel<128, PARTS, true>, &cfg) != cudaSuccess) {
+      (void)cudaGetLastError();
+      return 0;                              // no cluster for this call; the next one asks again
+    }
+    n = count + 1;
+    slot.store(n, std::memory_order_relaxed);
+  }
+  return n - 1;
+}
+
+// CTAs that share a tile: as many as make its chain of K steps shortest while all clusters are resident, against what the
+// cluster costs, 4 us, in steps, rounded up for those that share the L2 (us alone and split, bf16 and float32: 8 + 2 x 128 of 512 + 512 13.3 and 15.4,
+// 23.5 and 23.3; 1024 + 1024 17.4 and 17.5, 33.8 and 25.6; 768 + 3072 23.5 and 19.8, 54 and 33; 40 + 4 x 64, 40 tiles,
+// of 768 + 3072 26.5 and 21.9, 65 and 46, of 4096 + 4096 44 and 31, 122 and 77).
+static constexpr double kGramSplitCost = 10.;
+template <int PARTS>
+static int gram_ranks(long long tiles, int k_steps, const DeviceState* ds) {
+  int best = 1;
+  double cost = k_steps;
+  for (int r = 2; r <= 8 && r <= k_steps; ++r) {
+    const double c = (k_steps + r - 1) / r + kGramSplitCost;
+    if (c < cost && tiles * r <= ds->sm_count && tiles <= gram_resident<PARTS>(r, ds)) { best = r; cost = c; }
+  }
+  return best;
+}
+
 template <int BN, int PARTS>
 static int launch_gram(const GramOperands& o, int n_train, int n_val, long long T, int round_mode, float scale, float* M,
                        const DeviceState* ds, cudaStream_t stream) {
@@ -310,17 +467,23 @@ static int launch_gram(const GramOperands& o, int n_train, int n_val, long long 
   p.M = M;
   p.err = ds->err_word;
   CUtensorMap t[4];
-  const int rc = gram_maps(t, o, p.rows_t, p.rows_v, Cfg::BM, BN);
+  int rc = gram_maps(t, o, p.rows_t, p.rows_v, Cfg::BM, BN);
   if (rc != GHOST_OK) return rc;
-  static bool attr_set[64] = {};
-  if (!attr_set[ds->device]) {
-    GB_CUDA_OK(cudaFuncSetAttribute(ghost_gram_kernel<BN, PARTS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    Cfg::kSmemBytes));
-    attr_set[ds->device] = true;
-  }
   const long long tiles = static_cast<long long>(p.m_tiles) * p.n_tiles;
+  p.ranks = 1;
+  if constexpr (BN == 128) {
+    p.ranks = gram_ranks<PARTS>(tiles, ceil_div(p.ka, Cfg::BK) + ceil_div(p.kg, Cfg::BK), ds);
+    if (p.ranks > 1) {
+      if ((rc = gram_smem_attr<BN, PARTS, true>(ds)) != GHOST_OK) return rc;
+      GB_CUDA_OK(launch_next_cluster(dim3(p.ranks), ghost_gram_kernel<BN, PARTS, true>, dim3(static_cast<int>(tiles) * p.ranks), dim3(gram_threads(true)),
+                                     Cfg::kSmemBytes, stream, t[0], t[1], t[2], t[3], p));
+      count_launch();
+      return post_launch("ghost_gram_kernel");
+    }
+  }
+  if ((rc = gram_smem_attr<BN, PARTS, false>(ds)) != GHOST_OK) return rc;
   const int grid = static_cast<int>(tiles < ds->sm_count ? tiles : ds->sm_count);
-  GB_CUDA_OK(launch_next(ghost_gram_kernel<BN, PARTS>, dim3(grid), dim3(192), Cfg::kSmemBytes, stream, t[0], t[1], t[2], t[3], p));
+  GB_CUDA_OK(launch_next(ghost_gram_kernel<BN, PARTS, false>, dim3(grid), dim3(gram_threads(false)), Cfg::kSmemBytes, stream, t[0], t[1], t[2], t[3], p));
   count_launch();
   return post_launch("ghost_gram_kernel");
 }

@@ -301,12 +301,6 @@ __device__ __forceinline__ void gp_convert(uint8_t* block, int lo, int column, c
   }
 }
 
-__device__ __forceinline__ float4 gp_ld_cluster(uint32_t addr) {
-  float4 v;
-  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
-  return v;
-}
-
 // Element-wise sum, in rank order, of four floats that lie at `at` in the shared memory of those CTAs of the cluster that have a bit
 // in `mask`.  BATCH loads go out together, all eight where registers are free (in the loop over units one, as two cost it registers: 32 x 2000
 // tokens of 128 float32, embedding form, k = 64: 63.5 -> 66.3 us): one after the other they took most of a small call (5 x 4 tokens of 368 + 448 float32, k = 42,
@@ -319,7 +313,7 @@ __device__ __forceinline__ float4 gp_cluster_sum(const float* at, uint32_t mask)
     float4 v[BATCH];
 #pragma unroll
     for (int r = 0; r < BATCH; ++r)
-      if (mask >> (r0 + r) & 1) v[r] = gp_ld_cluster(map_to_cta(smem_u32(at), r0 + r));
+      if (mask >> (r0 + r) & 1) v[r] = ld_cluster_v4(map_to_cta(smem_u32(at), r0 + r));
 #pragma unroll
     for (int r = 0; r < BATCH; ++r)
       if (mask >> (r0 + r) & 1) { sum.x += v[r].x; sum.y += v[r].y; sum.z += v[r].z; sum.w += v[r].w; }

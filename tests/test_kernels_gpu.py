@@ -75,6 +75,28 @@ def test_gram_hook_tile_shapes(in_by_out, case, dtype):
     assert O.rel_fro(sums, G.double().sum(1)) < 1e-6
 
 
+# calls of few tiles and long rows, whose tiles are shared by clusters: K steps of both operands that part inside a CTA's run, at its
+# edge and leave most CTAs one operand only; columns and rows that end inside a quarter, one token, more tiles than clusters of eight
+@pytest.mark.parametrize("dtype,mode", [(torch.bfloat16, 0), (torch.float32, 0), (torch.bfloat16, 1)])
+@pytest.mark.parametrize("case", [(2, 1, 1, 2048, 2048), (5, 3, 13, 4096, 40), (3, 2, 70, 24, 5003), (9, 5, 41, 1031, 1500), (33, 4, 64, 1536, 1536)])
+def test_gram_tiles_shared_by_clusters(case, dtype, mode):
+    n_t, n_v, T, d, p = case
+    A, G = make(n_t + n_v, T, d, p, dtype, seed=34)
+    M = ops().gram_dot(A.cuda(), G.cuda(), n_v, round_mode=mode)
+    after()
+    a, g = A.cuda().double(), G.cuda().double()
+    S = torch.einsum("ntp,ntd->npd", g, a).flatten(1)
+    # as in test_gram_hook_tile_shapes; a rounded Gram entry and product are within 2^-8 of themselves each, no longer relative to a pair
+    # that cancels but to the token pairs' products
+    tol = (2 * 2.0 ** -16 if dtype == torch.float32 else 0.) + max(d, p) * 2.0 ** -23
+    scale = a.flatten(1).norm(dim=1) * g.flatten(1).norm(dim=1)
+    bound = tol * scale[n_t:, None] * scale[None, :n_t]
+    if mode:
+        ga = torch.einsum("vsd,btd->vbst", a[n_t:], a[:n_t]) * torch.einsum("vsp,btp->vbst", g[n_t:], g[:n_t])
+        bound = bound + 3 * 2.0 ** -8 * ga.abs().sum((2, 3))
+    assert ((M.double() - S[n_t:] @ S[:n_t].t()).abs() <= bound).all()
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("case", [(5, 3, 130, 72, 40), (4, 2, 256, 128, 64), (9, 2, 300, 200, 136),
                                   (700, 300, 1, 64, 48), (3, 5, 513, 96, 256)])
