@@ -67,7 +67,7 @@ struct XtyCfg {
   static constexpr int kStageBytes = (BM + BN) * BK * 2 * PARTS;   // 48 KB
   static constexpr int kStages = 4;
   static constexpr int kColsumBytes = PARTS == 1 ? 8 * 128 * 4 : 0;      // reduction scratch of the column-sum warps
-  static constexpr int kBoxBytes = PARTS * 4 * 32 * 32 * 4;  // store_grad_block32 (a box per epilogue warp), store_tile_f32
+  static constexpr int kBoxBytes = PARTS * 4 * 32 * 32 * 4;  // store_grad_rows (a box per epilogue warp), store_tile_f32
   // stages, boxes, barriers, scratch, from a 1024-byte boundary on, which the dynamic shared memory need not start at
   static constexpr int kBarOffset = kStages * kStageBytes + kBoxBytes, kRedOffset = kBarOffset + 256;
   static constexpr int kSmemBytes = 1024 + kRedOffset + kColsumBytes;
@@ -79,27 +79,6 @@ __device__ __forceinline__ void st_global_v8(void* addr, const uint32_t* v) {
                "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
                : "memory");
 }
-__device__ __forceinline__ void red_add_f32(float* addr, float v) {
-  asm volatile("red.global.add.f32 [%0], %1;" ::"l"(addr), "f"(v) : "memory");
-}
-__device__ __forceinline__ void red_add_f32x4(float* addr, float a, float b, float c, float d) {
-  asm volatile("red.global.v4.f32.add [%0], {%1, %2, %3, %4};" ::"l"(addr), "f"(a), "f"(b), "f"(c), "f"(d)
-               : "memory");
-}
-// 32 consecutive accumulator columns of one output row -> fp32 workspace (16-byte aligned rows)
-__device__ __forceinline__ void red_add_row32(float* dst, const uint32_t (&r)[32], int ncol) {
-  if (ncol >= 32) {
-#pragma unroll
-    for (int j = 0; j < 32; j += 4)
-      red_add_f32x4(dst + j, __uint_as_float(r[j]), __uint_as_float(r[j + 1]), __uint_as_float(r[j + 2]),
-                    __uint_as_float(r[j + 3]));
-  } else {
-#pragma unroll
-    for (int j = 0; j < 32; ++j)
-      if (j < ncol) red_add_f32(dst + j, __uint_as_float(r[j]));
-  }
-}
-
 template <bool kColsum, int PARTS>
 __global__ void __launch_bounds__(kColsum ? 320 : 192, 1)
 xty_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_y,
@@ -310,36 +289,14 @@ xty_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant_
       if (PARTS == 2 && p.tma_store) ok = named_bar_and(2, 128, ok);
       if (!ok) break;
       tc_fence_after_sync();
-      const int m = m0 + threadIdx.x;
-      const bool m_ok = m < p.m_cols;
       const uint32_t t_acc = tmem_base + lane_base + acc * BN;
       const bool empty_k = (kb0 >= kb1);   // nothing was accumulated: the tile is all zero
 
       if (p.mode == kEpiAccumulate) {
-#pragma unroll 1
-        for (int c0 = 0; c0 < BN; c0 += 32) {
-          if (n0 + c0 >= p.n_cols) break;
-          uint32_t r[32];
-          tmem_ld32(t_acc + c0, r);
-          tmem_ld_wait();
-          if (m_ok && !empty_k)
-            red_add_row32(p.acc_ws + static_cast<long long>(m) * p.ld_acc + n0 + c0, r, p.n_cols - (n0 + c0));
-        }
+        if (!empty_k) add_grad_rows(p.acc_ws, p.ld_acc, p.m_cols, p.n_cols, t_acc, m0 + warp * 32, n0, store_box + warp * 4096);
       } else if (p.mode == kEpiDirect) {
-#pragma unroll 1
-        for (int c0 = 0; c0 < BN; c0 += 32) {
-          if (n0 + c0 >= p.n_cols) break;
-          uint32_t r[32];
-          tmem_ld32(t_acc + c0, r);
-          tmem_ld_wait();
-          if (!p.out_vec)
-            store_grad_block32(p.vgrad, p.v_is_f32, p.out_accumulate, p.out_scale,
-                               static_cast<long long>(m0 + warp * 32) * p.n_cols + n0 + c0, p.n_cols, r, p.m_cols - (m0 + warp * 32),
-                               p.n_cols - (n0 + c0), reinterpret_cast<float*>(store_box) + warp * 1024);
-          else if (m_ok)
-            store_grad_row32(p.vgrad, p.v_is_f32, p.out_accumulate, p.out_scale,
-                             static_cast<long long>(m) * p.n_cols + n0 + c0, r, p.n_cols - (n0 + c0), p.out_vec != 0);
-        }
+        const GradOut g = {p.vgrad, p.m_cols, p.n_cols, p.v_is_f32, p.out_accumulate, p.out_vec, p.out_scale};
+        store_grad_rows(g, t_acc, m0 + warp * 32, n0, store_box + warp * 4096);
       } else if (PARTS == 2 && p.tma_store) {
         store_tile_f32(&tm_out, store_box, t_acc, static_cast<int>((static_cast<long long>(tile) * p.samples + sample) * BM), boxes);
       } else {

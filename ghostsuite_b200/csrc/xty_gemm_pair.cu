@@ -91,21 +91,6 @@ __device__ __forceinline__ void st_global_v8_pair(void* addr, const uint32_t* v)
                "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
                : "memory");
 }
-// 32 consecutive accumulator columns of one output row -> fp32 workspace (16-byte aligned rows)
-__device__ __forceinline__ void red_add_row32_pair(float* dst, const uint32_t (&r)[32], int ncol) {
-  if (ncol >= 32) {
-#pragma unroll
-    for (int j = 0; j < 32; j += 4)
-      asm volatile("red.global.v4.f32.add [%0], {%1, %2, %3, %4};" ::"l"(dst + j), "f"(__uint_as_float(r[j])),
-                   "f"(__uint_as_float(r[j + 1])), "f"(__uint_as_float(r[j + 2])), "f"(__uint_as_float(r[j + 3]))
-                   : "memory");
-  } else {
-#pragma unroll
-    for (int j = 0; j < 32; ++j)
-      if (j < ncol) asm volatile("red.global.add.f32 [%0], %1;" ::"l"(dst + j), "f"(__uint_as_float(r[j])) : "memory");
-  }
-}
-
 template <int PARTS>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(320, 1)
 xty_gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_y,
@@ -294,31 +279,15 @@ xty_gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
       if (!ok) break;
       tc_fence_after_sync();
       const int tile128 = tm * 2 + static_cast<int>(rank);      // this CTA's 128-row tile
-      if (p.accumulate) {
+      if (p.accumulate == 2) {
+        const GradOut g = {p.out, p.m_cols, p.n_cols, p.out_is_f32, p.out_accumulate, p.out_vec, p.out_scale};
+        store_grad_rows(g, tmem_base + lane_base + acc * BN, tile128 * BM + warp * 32, tn * BN, store_box + warp * 4096);
+      } else if (p.accumulate) {
         int kb0, kb1;
         k_range(sample, kb0, kb1);
-        const int m = tile128 * BM + static_cast<int>(threadIdx.x);
-        const int n0 = tn * BN;
-        const uint32_t t_acc = tmem_base + lane_base + acc * BN;
-        const bool live = m < p.m_cols && kb0 < kb1;      // no row block: nothing was accumulated
-#pragma unroll 1
-        for (int c0 = 0; c0 < BN; c0 += 32) {
-          if (n0 + c0 >= p.n_cols) break;
-          uint32_t r[32];
-          tmem_ld32(t_acc + c0, r);
-          tmem_ld_wait();
-          if (p.accumulate == 2 && !p.out_vec) {
-            const int m_first = tile128 * BM + warp * 32;
-            if (kb0 < kb1)
-              store_grad_block32(p.out, p.out_is_f32, p.out_accumulate, p.out_scale,
-                                 static_cast<long long>(m_first) * p.n_cols + n0 + c0, p.n_cols, r, p.m_cols - m_first,
-                                 p.n_cols - (n0 + c0), reinterpret_cast<float*>(store_box) + warp * 1024);
-          } else if (live && p.accumulate == 2)
-            store_grad_row32(p.out, p.out_is_f32, p.out_accumulate, p.out_scale, static_cast<long long>(m) * p.n_cols + n0 + c0,
-                             r, p.n_cols - (n0 + c0), p.out_vec != 0);
-          else if (live)
-            red_add_row32_pair(p.acc_ws + static_cast<long long>(m) * p.ld_acc + n0 + c0, r, p.n_cols - (n0 + c0));
-        }
+        if (kb0 < kb1)                     // no row block: nothing was accumulated
+          add_grad_rows(p.acc_ws, p.ld_acc, p.m_cols, p.n_cols, tmem_base + lane_base + acc * BN, tile128 * BM + warp * 32, tn * BN,
+                        store_box + warp * 4096);
       } else if (PARTS == 2 && tile128 < p.m_tiles128 && p.tma_store) {
         store_tile_f32(&tm_out, store_box, tmem_base + lane_base + acc * BN, ((tile128 * p.n_tiles + tn) * p.samples + sample) * BM, boxes);
       } else if (PARTS == 1 && tile128 < p.m_tiles128 && p.tma_store) {

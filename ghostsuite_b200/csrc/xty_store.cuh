@@ -1,6 +1,6 @@
-// Direct store of a train gradient: 32 consecutive accumulator columns of one output row, scaled, cast to
-// the parameter dtype and written (or added) to the row-major result.  Used where no other CTA adds to
-// the same tile, so that neither the fp32 workspace nor the scaling pass over it is needed.
+// Direct store of a train gradient: an accumulator tile, scaled, cast to the parameter dtype and written (or added)
+// to the row-major result.  Used where no other CTA adds to the same tile, so that neither the fp32 workspace
+// nor the scaling pass over it is needed.
 #pragma once
 #include <cuda_bf16.h>
 #include <stdint.h>
@@ -9,66 +9,162 @@
 
 namespace gb {
 
-// `vec`: rows start on 16-byte boundaries, so whole groups of 32 columns go out as 16-byte stores (one row a lane;
-// store_grad_block32 is the form for the rest)
-__device__ __forceinline__ void store_grad_row32(void* out, int is_f32, int accumulate, float scale, long long at,
-                                                 const uint32_t (&r)[32], int ncol, bool vec) {
-  if (is_f32) {
-    float* o = static_cast<float*>(out) + at;
-    if (vec && ncol >= 32 && !accumulate) {
+// A matrix that a GEMM with one split writes itself
+struct GradOut {
+  void* out;               // [rows, cols], row-major
+  int rows, cols;
+  int is_f32, accumulate;
+  int vec;                 // rows start on 16-byte boundaries
+  float scale;
+};
+
+// Elements of the block at `base` that lie in rows [0, nrow), this lane's of columns [0, ncol): `value(row)` reads what was staged,
+// loads of eight rows go out together.
+template <typename T, typename V>
+__device__ __forceinline__ void store_grad_columns(T* base, long long ld, int nrow, int col, int ncol, V&& value) {
+  T* o = base + col;
+#pragma unroll 1
+  for (int r0 = 0; r0 < 32; r0 += 8) {
+    T v[8];
 #pragma unroll
-      for (int j = 0; j < 32; j += 4)
-        *reinterpret_cast<float4*>(o + j) = make_float4(__uint_as_float(r[j]) * scale, __uint_as_float(r[j + 1]) * scale,
-                                                        __uint_as_float(r[j + 2]) * scale, __uint_as_float(r[j + 3]) * scale);
-    } else {
+    for (int i = 0; i < 8; ++i) v[i] = value(r0 + i);
 #pragma unroll
-      for (int j = 0; j < 32; ++j)
-        if (j < ncol) o[j] = __uint_as_float(r[j]) * scale + (accumulate ? o[j] : 0.f);
+    for (int i = 0; i < 8; ++i, o += ld)
+      if (r0 + i < nrow && col < ncol) *o = v[i];
+  }
+}
+
+// A warp's 32 rows (from `m0` on) of a 256-column accumulator tile (from column `n0` of the result on): scaled, cast and written, or
+// added, to the result.  Blocks of 128 bytes a row (64 columns in bf16, 32 in float32) are turned in shared memory (`box`, 4 KB of the warp's
+// own, 16-byte chunk c of row r at r * 128 + ((c ^ (r & 7)) << 4)), so that a store of the warp covers whole lines of four rows, or one
+// row's neighbouring columns where rows begin anywhere.
+// These stores are what bounds a call of few token rows.  With a row a lane (16-byte stores to 32 rows, aligned rows) and a
+// loop that waited for each row's value before its store (others), 364 rows of 3392 x 1488
+// (bf16) took 20.5 us and 3389 x 1484 49.5; 16.4 and 20.5 so.
+__device__ __forceinline__ void store_grad_rows(const GradOut& g, uint32_t t_acc, int m0, int n0, uint8_t* box) {
+  const int lane = threadIdx.x & 31;
+  const int nrow = g.rows - m0 < 32 ? g.rows - m0 : 32;
+  if (nrow <= 0) return;
+  const long long ld = g.cols;
+  uint8_t* mine = box + lane * 128;
+  const int turn = lane & 7;
+  auto chunk = [&](int row, int c) { return box + row * 128 + ((c ^ (row & 7)) << 4); };
+  // whole chunks: eight lanes a row
+  auto store_chunks = [&](uint8_t* base, int ncol_bytes) {
+    const int c = lane & 7;
+    uint4 v[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = *reinterpret_cast<const uint4*>(chunk(4 * i + (lane >> 3), c));
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int row = 4 * i + (lane >> 3);
+      if (row < nrow && c * 16 < ncol_bytes) *reinterpret_cast<uint4*>(base + row * ld * (g.is_f32 ? 4 : 2) + c * 16) = v[i];
     }
-  } else {
-    __nv_bfloat16* o = static_cast<__nv_bfloat16*>(out) + at;
-    if (vec && ncol >= 32 && !accumulate) {
+  };
+  if (g.is_f32 || g.accumulate) {
+#pragma unroll 1
+    for (int c0 = 0; c0 < 256 && n0 + c0 < g.cols; c0 += 32) {
+      const int ncol = g.cols - n0 - c0 < 32 ? g.cols - n0 - c0 : 32;
+      uint32_t r[32];
+      tmem_ld32(t_acc + c0, r);
+      tmem_ld_wait();
+      __syncwarp();                        // the block before has been read
 #pragma unroll
-      for (int j = 0; j < 32; j += 8) {
-        uint32_t w[4];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const __nv_bfloat162 h = __floats2bfloat162_rn(__uint_as_float(r[j + 2 * e]) * scale, __uint_as_float(r[j + 2 * e + 1]) * scale);
-          w[e] = *reinterpret_cast<const uint32_t*>(&h);
-        }
-        *reinterpret_cast<uint4*>(o + j) = make_uint4(w[0], w[1], w[2], w[3]);
+      for (int c = 0; c < 8; ++c) {
+        float4 w;
+        w.x = __uint_as_float(r[4 * c]) * g.scale; w.y = __uint_as_float(r[4 * c + 1]) * g.scale;
+        w.z = __uint_as_float(r[4 * c + 2]) * g.scale; w.w = __uint_as_float(r[4 * c + 3]) * g.scale;
+        *reinterpret_cast<float4*>(mine + ((c ^ turn) << 4)) = w;
       }
+      __syncwarp();
+      const long long at = m0 * ld + n0 + c0;
+      auto staged = [&](int row) { return *reinterpret_cast<const float*>(chunk(row, lane >> 2) + (lane & 3) * 4); };
+      auto there = [&](int row) { return row < nrow && lane < ncol; };
+      if (g.is_f32) {
+        float* base = static_cast<float*>(g.out) + at;
+        if (g.accumulate)
+          store_grad_columns(base, ld, nrow, lane, ncol, [&](int row) { return there(row) ? staged(row) + base[row * ld + lane] : 0.f; });
+        else if (g.vec)
+          store_chunks(reinterpret_cast<uint8_t*>(base), ncol * 4);
+        else
+          store_grad_columns(base, ld, nrow, lane, ncol, staged);
+      } else {
+        __nv_bfloat16* base = static_cast<__nv_bfloat16*>(g.out) + at;
+        store_grad_columns(base, ld, nrow, lane, ncol, [&](int row) {
+          return __float2bfloat16_rn(there(row) ? staged(row) + __bfloat162float(base[row * ld + lane]) : 0.f);
+        });
+      }
+    }
+    return;
+  }
+#pragma unroll 1
+  for (int c0 = 0; c0 < 256 && n0 + c0 < g.cols; c0 += 64) {
+    const int ncol = g.cols - n0 - c0 < 64 ? g.cols - n0 - c0 : 64;
+    uint32_t r[2][32];
+    tmem_ld32(t_acc + c0, r[0]);
+    tmem_ld32(t_acc + c0 + 32, r[1]);
+    tmem_ld_wait();
+    __syncwarp();                          // the block before has been read
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      uint32_t w[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int j = 8 * (c & 3) + 2 * e;
+        const __nv_bfloat162 h = __floats2bfloat162_rn(__uint_as_float(r[c >> 2][j]) * g.scale, __uint_as_float(r[c >> 2][j + 1]) * g.scale);
+        w[e] = *reinterpret_cast<const uint32_t*>(&h);
+      }
+      st_shared_v4(mine + ((c ^ turn) << 4), w[0], w[1], w[2], w[3]);
+    }
+    __syncwarp();
+    __nv_bfloat16* base = static_cast<__nv_bfloat16*>(g.out) + m0 * ld + n0 + c0;
+    if (g.vec) {
+      store_chunks(reinterpret_cast<uint8_t*>(base), ncol * 2);
     } else {
 #pragma unroll
-      for (int j = 0; j < 32; ++j)
-        if (j < ncol) o[j] = __float2bfloat16_rn(__uint_as_float(r[j]) * scale + (accumulate ? __bfloat162float(o[j]) : 0.f));
+      for (int h = 0; h < 2; ++h)
+        store_grad_columns(base, ld, nrow, lane + 32 * h, ncol, [&](int row) {
+          return *reinterpret_cast<const __nv_bfloat16*>(chunk(row, 4 * h + (lane >> 3)) + (lane & 7) * 2);
+        });
     }
   }
 }
 
-// The 32 x 32 block of a warp (lane r holds row r) where single rows cannot go out as whole 16-byte pieces: turned in
-// shared memory (`box`: 32 x 32 floats of the warp's own, columns rotated by the row against bank conflicts),
-// a store of the warp then covers neighbouring columns of one row.  With a row per lane every store touched 32 rows:
-// 15 x 51 tokens of 141 -> 64 in bf16 took 18 us for half a microsecond of work.
-__device__ __forceinline__ void store_grad_block32(void* out, int is_f32, int accumulate, float scale, long long row0_at,
-                                                   long long ld, const uint32_t (&r)[32], int nrow, int ncol, float* box) {
-  const int lane = threadIdx.x & 31;
-  __syncwarp();
+// The same rows added to the fp32 workspace of a result that several CTAs share: whole lines of four rows a store, rows of `ld` (a
+// multiple of four), from a 16-byte boundary where the caller's workspace begins on one.  (A row a lane: 8192 rows of 256 x 256 bf16 23.6 us,
+// 768 x 768 float32 43.4; 19.5 and 37.9 so.)
+__device__ __forceinline__ void add_grad_rows(float* ws, long long ld, int rows, int cols, uint32_t t_acc, int m0, int n0, uint8_t* box) {
+  const int lane = threadIdx.x & 31, c = lane & 7;
+  const int nrow = rows - m0 < 32 ? rows - m0 : 32;
+  if (nrow <= 0) return;
+  const bool aligned = (reinterpret_cast<uintptr_t>(ws) & 15) == 0;
+#pragma unroll 1
+  for (int c0 = 0; c0 < 256 && n0 + c0 < cols; c0 += 32) {
+    uint32_t r[32];
+    tmem_ld32(t_acc + c0, r);
+    tmem_ld_wait();
+    __syncwarp();                          // the block before has been read
 #pragma unroll
-  for (int j = 0; j < 32; ++j) box[lane * 32 + ((j + lane) & 31)] = __uint_as_float(r[j]);
-  __syncwarp();
-  if (lane < ncol) {
-#pragma unroll 8
-    for (int row = 0; row < 32; ++row) {
-      if (row >= nrow) break;
-      const float v = box[row * 32 + ((lane + row) & 31)] * scale;
-      const long long at = row0_at + row * ld + lane;
-      if (is_f32) {
-        float* o = static_cast<float*>(out) + at;
-        *o = accumulate ? v + *o : v;
+    for (int q = 0; q < 8; ++q) st_shared_v4(box + lane * 128 + ((q ^ c) << 4), r[4 * q], r[4 * q + 1], r[4 * q + 2], r[4 * q + 3]);
+    __syncwarp();
+    float4 v[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int row = 4 * i + (lane >> 3);
+      v[i] = *reinterpret_cast<const float4*>(box + row * 128 + ((c ^ (row & 7)) << 4));
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int row = 4 * i + (lane >> 3);
+      if (row >= nrow || n0 + c0 + 4 * c >= cols) continue;
+      float* at = ws + (m0 + row) * ld + n0 + c0 + 4 * c;
+      if (aligned) {                       // zeros behind the last column, up to the row's end
+        asm volatile("red.global.v4.f32.add [%0], {%1, %2, %3, %4};" ::"l"(at), "f"(v[i].x), "f"(v[i].y), "f"(v[i].z), "f"(v[i].w)
+                     : "memory");
       } else {
-        __nv_bfloat16* o = static_cast<__nv_bfloat16*>(out) + at;
-        *o = __float2bfloat16_rn(accumulate ? v + __bfloat162float(*o) : v);
+        const float e[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) asm volatile("red.global.add.f32 [%0], %1;" ::"l"(at + j), "f"(e[j]) : "memory");
       }
     }
   }

@@ -1565,6 +1565,33 @@ def test_wgrad_split_sums_over_old_values(rows, m, n, mode):
         _lib.check(lib.ghost_set_wgrad_pair_mode(1))
 
 
+# results that the GEMM writes itself (few rows) and adds up in a workspace: blocks of 32 rows and 32 or 64 columns that end early,
+# rows that begin on 16 bytes and anywhere, an unaligned result, old values kept; whole numbers, so exact in every type
+@pytest.mark.parametrize("parts,out_dtype", [(1, torch.bfloat16), (1, torch.float32), (2, torch.float32), (2, torch.bfloat16)])
+@pytest.mark.parametrize("m,n", [(1, 1), (33, 65), (129, 257), (160, 328), (300, 63)])
+@pytest.mark.parametrize("rows", [40, 3000])
+def test_train_gradient_stores(rows, m, n, parts, out_dtype):
+    from ghostsuite_b200 import _lib
+    lib = _lib.load()
+    gen = torch.Generator().manual_seed(7)
+    X, Y = (torch.zeros(parts, rows, -(-c // 64) * 64, dtype=torch.bfloat16) for c in (m, n))
+    X[0, :, :m], Y[0, :, :n] = (torch.randint(-1, 2, (rows, c), generator=gen).bfloat16() for c in (m, n))
+    X, Y = X.cuda(), Y.cuda()
+    want = X[0, :, :m].double().t() @ Y[0, :, :n].double()
+    assert want.abs().max() < 254
+    ws = torch.empty(lib.ghost_wgrad_workspace_bytes(m, n), dtype=torch.uint8, device="cuda")
+    for first in (0, 1):                              # elements in front of the result
+        buf = torch.full((first + m * n + 64,), 2.0, dtype=out_dtype, device="cuda")
+        out = buf[first:first + m * n]
+        for accumulate in (0, 1):
+            _lib.check(lib.ghost_wgrad_parts(X.data_ptr(), Y.data_ptr(), parts, rows, rows, m, n, X.shape[2], Y.shape[2], 1.0 if not accumulate else -1.0,
+                                             accumulate, out.data_ptr(), int(out_dtype == torch.float32), ws.data_ptr(), ws.numel(),
+                                             torch.cuda.current_stream().cuda_stream))
+            after()
+            assert torch.equal(out.double().view(m, n), want if not accumulate else 0 * want)
+        assert (buf[:first] == 2).all() and (buf[first + m * n:] == 2).all()
+
+
 # just below 32 MB, 32 MB, more (a memset); a word, two and three behind the last sixteen bytes; results off sixteen bytes
 @pytest.mark.parametrize("n_t,n_v,offset", [(4095, 2048, 0), (4096, 2048, 0), (4097, 2048, 0), (4096, 2048, 4), (4096, 2048, 1),
                                             (3, 1, 0), (2, 1, 0), (1, 1, 0), (5, 1, 0), (13, 315, 0), (1024, 4, 0), (1025, 4, 0)])
