@@ -27,7 +27,7 @@ static constexpr int kPassThreads = 256;
 // the train rows come out of the same copy (32 + 8 vectors of 3072: two rounds and a second pass over the
 // rows 10.8 us, 9.5 now; of 768: 6.7 and 5.0); no more than the list's longest vector needs, which leaves room for the CTAs of other kernels, and half of
 // kPassMost where the launch has more CTAs than three quarters of the SMs, which would wait for their memory then (32 + 8 vectors
-// of 8192, one job 22.2 us in halves and 18.0 whole; 24 jobs 25.6 and 49).
+// of 8192, one job 22.2 us in halves and 18.4 whole; 24 jobs 25.7 and 49).
 static constexpr int kPassMost = 1024;
 __host__ __device__ constexpr int pass_pitch(int sub) { return sub + 4; }      // rows 16 bytes apart modulo 128: no bank conflicts
 // 32 train rows, then nv validation rows; behind them the warps' partial sums
@@ -46,7 +46,7 @@ __device__ __forceinline__ const float* pass_val_row(const ghost_pass_job& j, in
 
 // Columns [f, f + width) of `train` train rows from b0 on and `val` validation rows from v0 on into shared memory, from rows 0 and 32 on,
 // zero up to the next multiple of four.  Rows that are not there stay what they were: what their lanes make of them is not
-// read.  (3 + 1 vectors of 8192: 18.1 us with 36 rows of zeros and two rounds of 512 columns, 12.7 so; 48 jobs of 8 + 2 41 and 28.8.)
+// read.  (3 + 1 vectors of 8192: 18.1 us with 36 rows of zeros and two rounds of 512 columns, 10.2 so; 48 jobs of 8 + 2 41 and 27.)
 __device__ __forceinline__ void pass_stage(const ghost_pass_job& j, bool vec, int b0, int train, int v0, int val, int f, int width, float* st,
                                            int pitch) {
   const int quads = (width + 3) / 4;
@@ -114,17 +114,18 @@ __device__ __forceinline__ void pass_row_sums(const ghost_pass_job& j, int f0, i
 }
 
 // The same sums, bit for bit, from the staged columns of a block that holds all train rows
-template <bool ALL>      // the block is full: no tests (32 + 8 vectors of 4096: 16.2 us with them, 13.8 without)
-__device__ __forceinline__ void pass_staged_sums(const ghost_pass_job& j, int f, int width, const float* st, int pitch) {
+// (`train` of them, staged up to the next multiple of eight)
+__device__ __forceinline__ void pass_staged_sums(const ghost_pass_job& j, int train, int f, int width, const float* st, int pitch) {
   for (int c = threadIdx.x; c < width; c += kPassThreads) {
+    float a[8] = {};
+#pragma unroll
+    for (int n = 0; n < 32; n += 8)
+      if (n < train)
+#pragma unroll
+        for (int w = 0; w < 8; ++w) a[w] += st[(n + w) * pitch + c];
     float s = 0.f;
 #pragma unroll
-    for (int w = 0; w < 8; ++w) {
-      float a = 0.f;
-#pragma unroll
-      for (int n = 0; n < 32; n += 8) a += ALL || n + w < j.n_train ? st[(n + w) * pitch + c] : 0.f;
-      s += a;
-    }
+    for (int w = 0; w < 8; ++w) s += a[w];
     s *= j.sum_scale;
     if (j.sum_is_f32) static_cast<float*>(j.sum_out)[f + c] = s;
     else static_cast<__nv_bfloat16*>(j.sum_out)[f + c] = __float2bfloat16_rn(s);
@@ -196,27 +197,27 @@ pass_reduce_kernel(const __grid_constant__ PassJobs<CAP> jobs) {
         for (int f = f0; f < f1; f += jobs.sub) {
           const int width = f1 - f < jobs.sub ? f1 - f : jobs.sub;
           __syncthreads();
+          if (staged_sums && v0 == 0)        // for the sums below: zeros up to the next multiple of eight rows
+            for (int i = threadIdx.x; i < (-train & 7) * pitch; i += kPassThreads) stage[train * pitch + i] = 0.f;
           // one round holds all columns: the train rows are there already
           pass_stage(j, vec, blk * 32, v0 > 0 && chunk <= jobs.sub ? 0 : train, v0, val, f, width, stage, pitch);
           __syncthreads();
-          if (staged_sums && v0 == 0) {
-            if (train == 32) pass_staged_sums<true>(j, f, width, stage, pitch);
-            else pass_staged_sums<false>(j, f, width, stage, pitch);
-          }
-          auto products = [&](auto all) {      // all: NV rows, no tests (24 jobs of 32 + 8 vectors of 4096: 19.4 us with them, 15.9 without)
+          if (staged_sums && v0 == 0) pass_staged_sums(j, train, f, width, stage, pitch);
+          auto products = [&](auto some) {     // of the first rows; a test a row costs more than products that are not read (24 jobs of 32 + 8
+                                               // vectors of 4096 19.4 us with tests, 16.4 without)
             for (int q = warp * 4; q < width; q += 32) {
               const float4 x = *reinterpret_cast<const float4*>(stage + lane * pitch + q);
 #pragma unroll
-              for (int i = 0; i < NV; ++i) {
-                if (!decltype(all)::value && i >= val) break;
+              for (int i = 0; i < decltype(some)::value; ++i) {
                 const float4 y = *reinterpret_cast<const float4*>(stage + (32 + i) * pitch + q);
                 acc[i].x = fmaf(x.x, y.x, acc[i].x); acc[i].y = fmaf(x.y, y.y, acc[i].y);
                 acc[i].z = fmaf(x.z, y.z, acc[i].z); acc[i].w = fmaf(x.w, y.w, acc[i].w);
               }
             }
           };
-          if (val == NV) products(std::true_type());
-          else products(std::false_type());
+          if (val > NV / 2) products(std::integral_constant<int, NV>());
+          else if (val > NV / 4) products(std::integral_constant<int, NV / 2>());
+          else products(std::integral_constant<int, NV / 4>());
         }
         float* red = stage + (32 + NV) * pitch;        // [warp][validation row][train lane]
 #pragma unroll
