@@ -7,6 +7,7 @@
 // share out the three results; nothing is converted, zeroed or written twice.  Layer 1024 -> 1024,
 // 64 + 16 samples of one token, float32: 11 launches, 93 us of GPU time before, one of 7 us now.
 #include "common.cuh"
+#include "sm100_ptx.cuh"
 
 namespace gb {
 
@@ -19,9 +20,11 @@ struct SmallDense {
   int grad_f32;
   float grad_scale;
   float* colsums;                       // [N, p]; null: not wanted
-  // blocks [0, gram_blocks): pairs of sample groups; then wgrad_blocks tiles of 64 x 64; then column sums
+  // blocks [0, gram_blocks): pairs of sample groups, a cluster of `ranks` to each in the SPLIT form; then wgrad_blocks tiles of
+  // 64 x 64; then column sums
   int sv, sb, groups_b, gram_blocks;    // samples of a group (validation, train)
   int tiles_n, wgrad_blocks;
+  int ranks;
 };
 
 // Four consecutive elements as they are loaded, and as numbers.  Two steps, so that the loads of several rows are in flight
@@ -73,12 +76,14 @@ static constexpr int kSdV = 8, kSdB = 4;   // validation x train rows of a Gram 
 // The 8 x 4 products of one tile over columns of X [.., K]: eight warps take 128-column units in turn, a
 // lane four columns of all twelve rows, so every row is read with full lines and once.  A butterfly
 // that halves the number of values with the distance leaves entry `lane` of the tile in every lane.
-template <typename E, bool VEC>
-__device__ __forceinline__ float sd_gram(const E* X, int K, long long row_v, int rows_v, long long row_b, int rows_b, int warp, int lane) {
+// SPLIT: `warp` counts over the `warps` of all blocks that share the tile.
+template <typename E, bool VEC, bool SPLIT>
+__device__ __forceinline__ float sd_gram(const E* X, int K, long long row_v, int rows_v, long long row_b, int rows_b, int warp, int warps,
+                                         int lane) {
   float acc[kSdV * kSdB];
 #pragma unroll
   for (int e = 0; e < kSdV * kSdB; ++e) acc[e] = 0.f;
-  for (int k0 = warp * 128; k0 < K; k0 += 1024) {
+  for (int k0 = warp * 128; k0 < K; k0 += SPLIT ? warps * 128 : 1024) {
     const int k = k0 + lane * 4;
     SdQuad<E, VEC> v[kSdV], b[kSdB];
 #pragma unroll
@@ -108,7 +113,7 @@ __device__ __forceinline__ float sd_gram(const E* X, int K, long long row_v, int
   return acc[0];
 }
 
-template <typename E, bool VEC>
+template <typename E, bool VEC, bool SPLIT>
 __global__ void __launch_bounds__(256, 2) dense_small_kernel(const SmallDense q) {
   stream_order();
   __shared__ __align__(16) float sm[2 * 2 * 16 * 64];
@@ -119,21 +124,48 @@ __global__ void __launch_bounds__(256, 2) dense_small_kernel(const SmallDense q)
 
   if (blk < q.gram_blocks) {
     float* red = sm;                     // [operand][warp][32 entries]
+    float* part = sm + 512;              // SPLIT: [tile parity][operand][32]: this block's share of the entries
+    const int ranks = SPLIT ? q.ranks : 1, rank = SPLIT ? blk % ranks : 0;
+    if (SPLIT) blk /= ranks;
+    int parity = 0;
     const int v0 = blk / q.groups_b * q.sv, b0 = blk % q.groups_b * q.sb;
     const int nv = min(q.sv, q.n_val - v0), nb = min(q.sb, q.n_train - b0);
     const long long first_v = static_cast<long long>(q.n_train + v0) * q.T, first_b = static_cast<long long>(b0) * q.T;
     const int rows_v = nv * q.T, rows_b = nb * q.T;      // T == 1, or one sample per side, or a few short ones
     float total = 0.f;                   // warp 0: T == 1: entry `lane`; else thread's pair (see below)
     for (int i0 = 0; i0 < rows_v; i0 += kSdV)
-      for (int j0 = 0; j0 < rows_b; j0 += kSdB) {
+      for (int j0 = 0; j0 < rows_b; j0 += kSdB, parity ^= 64) {
         const int rv = min(kSdV, rows_v - i0), rb = min(kSdB, rows_b - j0);
-        red[warp * 32 + lane] = sd_gram<E, VEC>(A, q.d, first_v + i0, rv, first_b + j0, rb, warp, lane);
-        red[256 + warp * 32 + lane] = sd_gram<E, VEC>(B, q.p, first_v + i0, rv, first_b + j0, rb, warp, lane);
+        red[warp * 32 + lane] = sd_gram<E, VEC, SPLIT>(A, q.d, first_v + i0, rv, first_b + j0, rb, rank * 8 + warp, ranks * 8, lane);
+        red[256 + warp * 32 + lane] = sd_gram<E, VEC, SPLIT>(B, q.p, first_v + i0, rv, first_b + j0, rb, rank * 8 + warp, ranks * 8, lane);
         __syncthreads();
-        if (warp == 0) {
-          float sa = 0.f, sg = 0.f;
+        if (SPLIT) {                     // rank 0 reads tile k's parts before it arrives at tile k + 1's barrier
+          if (warp == 0) {
+            float sa = 0.f, sg = 0.f;
 #pragma unroll
-          for (int w = 0; w < 8; ++w) { sa += red[w * 32 + lane]; sg += red[256 + w * 32 + lane]; }
+            for (int w = 0; w < 8; ++w) { sa += red[w * 32 + lane]; sg += red[256 + w * 32 + lane]; }
+            part[parity + lane] = sa;
+            part[parity + 32 + lane] = sg;
+          }
+          cluster_sync_all();
+        }
+        if (warp == 0 && rank == 0) {
+          float sa = 0.f, sg = 0.f;
+          if (SPLIT) {
+            float a[8], g[8];
+#pragma unroll
+            for (int r = 0; r < 8; ++r)
+              if (r < ranks) {
+                a[r] = ld_cluster_f32(map_to_cta(smem_u32(part + parity + lane), r));
+                g[r] = ld_cluster_f32(map_to_cta(smem_u32(part + parity + 32 + lane), r));
+              }
+#pragma unroll
+            for (int r = 0; r < 8; ++r)
+              if (r < ranks) { sa += a[r]; sg += g[r]; }
+          } else {
+#pragma unroll
+            for (int w = 0; w < 8; ++w) { sa += red[w * 32 + lane]; sg += red[256 + w * 32 + lane]; }
+          }
           const int i = lane / kSdB, j = lane % kSdB;
           const float prod = i < rv && j < rb ? sa * sg : 0.f;
           if (q.T == 1) {
@@ -150,7 +182,8 @@ __global__ void __launch_bounds__(256, 2) dense_small_kernel(const SmallDense q)
         }
         __syncthreads();
       }
-    if (warp == 0) {
+    if (SPLIT) cluster_sync_all();       // no block leaves while rank 0 still reads its shared memory
+    if (warp == 0 && rank == 0) {
       const int i = q.T == 1 ? lane / kSdB : lane / nb, j = q.T == 1 ? lane % kSdB : lane % nb;
       if (i < nv && j < nb) q.M[static_cast<long long>(v0 + i) * q.n_train + b0 + j] = total;
     }
@@ -231,7 +264,7 @@ __global__ void __launch_bounds__(256, 2) dense_small_kernel(const SmallDense q)
 
   const int blocks_c = (q.p + 1023) / 1024;
   const int s = blk / blocks_c, c = blk % blocks_c * 1024 + threadIdx.x * 4;
-  if (c >= q.p) return;
+  if (c >= q.p || (SPLIT && (q.colsums == nullptr || s >= q.n_train + q.n_val))) return;      // blocks that fill up the last cluster
   float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
   const E* row = B + static_cast<long long>(s) * q.T * q.p + c;
 #pragma unroll 4
@@ -273,6 +306,28 @@ extern "C" int ghost_dense_small_fits(int is_f32, int n_train, int n_val, long l
          train_rows <= chain ? 1 : 0;
 }
 
+template <typename E, bool VEC>
+static cudaError_t launch_small(const SmallDense& q, unsigned grid, cudaStream_t st) {
+  if (q.ranks > 1) return launch_next_cluster(dim3(q.ranks), dense_small_kernel<E, VEC, true>, dim3(grid), dim3(256), 0, st, q);
+  return launch_next(dense_small_kernel<E, VEC, false>, dim3(grid), dim3(256), 0, st, q);
+}
+
+// Blocks that share a pair of groups of samples.  A step of 1024 columns takes a block 1.1 us, and the pairs are few where the rows are
+// long (4 + 12 samples of one token, float32 108 -> 27072: 36.9 us in two blocks, 14.5 in sixteen; 8 + 2 of 20000 -> 10 35.9 and 14.3;
+// 2 + 2 x 8 of 4096 -> 512 17.0 and 14.5).  A tile costs a cluster's barrier, 1.5 us, on top (8 + 2 x 16 of 2048 -> 1024, eight
+// tiles a pair: 38.9, 41 shared).  Where the gradient's blocks take longer than the chain nothing is gained, and
+// they come up slower in clusters (2 + 1 of 768 -> 50000 71 and 77; 16 + 4 of 4095 -> 4097 47 and 53).
+static int small_ranks(long long gram, long long tiles, long long wgrad, long long rows, int d, int p, const DeviceState* ds) {
+  const double others = static_cast<double>((wgrad + 2 * ds->sm_count - 1) / (2 * ds->sm_count)) * (2.0 + 0.045 * rows);
+  int best = 1;
+  double cost = 1.1 * (ceil_div(d, 1024) + ceil_div(p, 1024)) * tiles;
+  for (int r = 2; r <= 8 && gram * r <= 2ll * ds->sm_count && cost > others; r *= 2) {
+    const double c = (1.1 * (ceil_div(d, 1024 * r) + ceil_div(p, 1024 * r)) + 1.5) * tiles;
+    if (c < cost) { best = r; cost = c; }
+  }
+  return best;
+}
+
 extern "C" int ghost_dense_small(const void* A, const void* B, int is_f32, int n_train, int n_val, long long T, int d,
                                  int p, int in_by_out, float* M_out, void* grad_out, int grad_is_f32, float grad_scale,
                                  float* colsum_out, void* stream) {
@@ -299,18 +354,19 @@ extern "C" int ghost_dense_small(const void* A, const void* B, int is_f32, int n
   const long long wgrad = grad_out ? static_cast<long long>(ceil_div(m, 64)) * q.tiles_n : 0;
   const long long col = colsum_out ? static_cast<long long>(n_train + n_val) * ceil_div(p, 1024) : 0;
   GB_REQUIRE(gram + wgrad + col < (1ll << 31), "ghost_dense_small: too many blocks");
-  q.gram_blocks = static_cast<int>(gram);
+  q.ranks = small_ranks(gram, (T + kSdV - 1) / kSdV * ((T + kSdB - 1) / kSdB), wgrad, n_train * T, d, p, ds);
+  q.gram_blocks = static_cast<int>(gram * q.ranks);
   q.wgrad_blocks = static_cast<int>(wgrad);
   const uintptr_t align = is_f32 ? 15 : 7;
   const bool vec = d % 4 == 0 && p % 4 == 0 && (reinterpret_cast<uintptr_t>(A) & align) == 0 && (reinterpret_cast<uintptr_t>(B) & align) == 0;
-  const unsigned grid = static_cast<unsigned>(gram + wgrad + col);
+  const unsigned grid = static_cast<unsigned>((gram * q.ranks + wgrad + col + q.ranks - 1) / q.ranks * q.ranks);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (is_f32) {
-    if (vec) GB_CUDA_OK(launch_next(dense_small_kernel<float, true>, dim3(grid), dim3(256), 0, st, q));
-    else GB_CUDA_OK(launch_next(dense_small_kernel<float, false>, dim3(grid), dim3(256), 0, st, q));
+    if (vec) GB_CUDA_OK((launch_small<float, true>(q, grid, st)));
+    else GB_CUDA_OK((launch_small<float, false>(q, grid, st)));
   } else {
-    if (vec) GB_CUDA_OK(launch_next(dense_small_kernel<__nv_bfloat16, true>, dim3(grid), dim3(256), 0, st, q));
-    else GB_CUDA_OK(launch_next(dense_small_kernel<__nv_bfloat16, false>, dim3(grid), dim3(256), 0, st, q));
+    if (vec) GB_CUDA_OK((launch_small<__nv_bfloat16, true>(q, grid, st)));
+    else GB_CUDA_OK((launch_small<__nv_bfloat16, false>(q, grid, st)));
   }
   count_launch();
   return post_launch("dense_small_kernel");

@@ -36,11 +36,7 @@ template <> struct Vec8<float> {
 // One value of every CTA of the cluster, added up in rank order
 __device__ __forceinline__ float cluster_sum(const float* mine, int ranks) {
   float v = 0.f;
-  for (int r = 0; r < ranks; ++r) {
-    float x;
-    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(x) : "r"(map_to_cta(smem_u32(mine), r)) : "memory");
-    v += x;
-  }
+  for (int r = 0; r < ranks; ++r) v += ld_cluster_f32(map_to_cta(smem_u32(mine), r));
   return v;
 }
 

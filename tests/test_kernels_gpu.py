@@ -1565,6 +1565,33 @@ def test_wgrad_split_sums_over_old_values(rows, m, n, mode):
         _lib.check(lib.ghost_set_wgrad_pair_mode(1))
 
 
+# layers of few rows whose pairs of samples are shared by clusters (long rows): one tile a pair and several, rows that end inside a
+# warp's columns, unaligned rows, blocks behind the column sums that fill up a cluster, no gradient
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("n_t,n_v,T,d,p", [(4, 12, 1, 109, 9001), (9, 3, 1, 8192, 260), (2, 2, 8, 4096, 33), (3, 2, 16, 5001, 16), (5, 1, 5, 100, 7000)])
+def test_few_rows_shared_by_clusters(n_t, n_v, T, d, p, dtype):
+    from ghostsuite_b200 import _lib
+    lib = _lib.load()
+    A, G = (x.cuda() for x in make(n_t + n_v, T, d, p, dtype, seed=35))
+    f32 = int(dtype == torch.float32)
+    assert lib.ghost_dense_small_fits(f32, n_t, n_v, T, d, p)
+    a, g = A.double(), G.double()
+    grams = [torch.einsum("vsd,btd->vbst", x[n_t:], x[:n_t]) for x in (a, g, a.abs(), g.abs())]
+    # chains of 4 K / 1024 products in each lane, then 31 values of other lanes, warps and blocks; T^2 entries added up
+    eps = ((4 * (d // 1024 + p // 1024 + 2)) + 2 * 31 + T * T) * 2.0 ** -24
+    bound = eps * (grams[2] * grams[3]).sum((2, 3))
+    for want_grad in (True, False):
+        M = torch.full((n_v, n_t), 7.0, device="cuda")
+        grad, sums = torch.full((p, d), 7.0, dtype=dtype, device="cuda"), torch.full((n_t + n_v, p), 7.0, device="cuda")
+        _lib.check(lib.ghost_dense_small(A.data_ptr(), G.data_ptr(), f32, n_t, n_v, T, d, p, 0, M.data_ptr(), grad.data_ptr() if want_grad else None,
+                                         f32, 0.5, sums.data_ptr() if want_grad else None, torch.cuda.current_stream().cuda_stream))
+        after()
+        assert ((M.double() - (grams[0] * grams[1]).sum((2, 3))).abs() <= bound).all()
+        if want_grad:
+            assert O.rel_fro(grad, 0.5 * torch.einsum("ntp,ntd->pd", g[:n_t], a[:n_t])) < (2.0 ** -8 if not f32 else 1e-6)
+            assert O.rel_fro(sums, g.sum(1)) < 1e-6
+
+
 # results that the GEMM writes itself (few rows) and adds up in a workspace: blocks of 32 rows and 32 or 64 columns that end early,
 # rows that begin on 16 bytes and anywhere, an unaligned result, old values kept; whole numbers, so exact in every type
 @pytest.mark.parametrize("parts,out_dtype", [(1, torch.bfloat16), (1, torch.float32), (2, torch.float32), (2, torch.bfloat16)])
