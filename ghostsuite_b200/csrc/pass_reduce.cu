@@ -26,9 +26,13 @@ static constexpr int kPassThreads = 256;
 // Columns staged at a time: a CTA's whole share up to kPassMost, so that one round of loads serves it and the sums of
 // the train rows come out of the same copy (32 + 8 vectors of 3072: two rounds and a second pass over the
 // rows 10.8 us, 9.5 now; of 768: 6.7 and 5.0); no more than the list's longest vector needs, which leaves room for the CTAs of other kernels, and half of
-// kPassMost where the launch has more CTAs than three quarters of the SMs, which would wait for their memory then (32 + 8 vectors
-// of 8192, one job 22.2 us in halves and 18.4 whole; 24 jobs 25.7 and 49).
+// kPassMost with blocks of sixteen validation rows, and where the launch has more CTAs than three quarters of the SMs, which would wait
+// for their memory then (32 + 8 vectors of 8192, one job 22.2 us in halves and 18.4 whole; 24 jobs 25.7 and 49).
 static constexpr int kPassMost = 1024;
+// Shared memory that keeps a second CTA off the SM.  Two of 111 KB turn all of an SM's memory into shared memory, and the kernel that
+// comes up there next has no L1 for its loads: RMS hooks of 6 + 2 x 1024 x 5120 float32 in a row took 104 us, 85.7 in halves, 80.8
+// so.  (Rounds of more than 512 with sixteen validation rows, 160 KB and up, do the same alone: 6 + 10 x 512 x 8192 113 us in halves, 126.)
+static constexpr int kPassAlone = 118 * 1024;
 __host__ __device__ constexpr int pass_pitch(int sub) { return sub + 4; }      // rows 16 bytes apart modulo 128: no bank conflicts
 // 32 train rows, then nv validation rows; behind them the warps' partial sums
 __host__ __device__ constexpr int pass_smem(int sub, int nv) { return (32 + nv) * pass_pitch(sub) * 4 + 8 * nv * 32 * 4; }
@@ -359,9 +363,11 @@ static int launch_pass(const ghost_pass_job* jobs, int n, int blocks, const Devi
     if (jobs[i].X != nullptr && jobs[i].F > longest) longest = jobs[i].F;
   const int sub = (pass_chunk(longest) + 31) / 32 * 32;
   // the row sums of longer lists reduce 8 x 4 x 128 partial sums in the same memory
-  const int most = static_cast<long long>(blocks) * n * kPassCluster * 4 <= ds->sm_count * 3ll ? kPassMost : kPassMost / 2;
+  const int most = NV == 8 && static_cast<long long>(blocks) * n * kPassCluster * 4 <= ds->sm_count * 3ll ? kPassMost : kPassMost / 2;
   batch.sub = sub < 128 ? 128 : sub > most ? most : sub;
-  GB_CUDA_OK(launch_next(pass_reduce_kernel<CAP, NV>, dim3(dim3(kPassCluster, blocks, n)), dim3(kPassThreads), pass_smem(batch.sub, NV), st, batch));
+  int smem = pass_smem(batch.sub, NV);
+  if (batch.sub > kPassMost / 2 && smem < kPassAlone) smem = kPassAlone;
+  GB_CUDA_OK(launch_next(pass_reduce_kernel<CAP, NV>, dim3(dim3(kPassCluster, blocks, n)), dim3(kPassThreads), smem, st, batch));
   count_launch();
   return post_launch("pass_reduce_kernel");
 }
