@@ -500,9 +500,67 @@ __global__ void layernorm_reduce_kernel(const float* part, int N, int F, int t_s
   }
 }
 
+// A thread's PT features of a row as they are loaded: pieces of eight, or every THREADS-th.  They are converted in a second
+// step: behind its bounds check a conversion makes each load of a group of rows wait for the one before (RMS hooks
+// of 6 + 2 x 1024 rows in bf16, us: F = 4096 60 and 52, 8192 94.5 and 82.5, 4097 109 and 92).
+template <typename T, bool VEC, int PT> struct NormRaw {
+  using Bits = typename std::conditional<sizeof(T) == 2, unsigned short, float>::type;
+  static constexpr int kWords = static_cast<int>(sizeof(T)) / 2;       // 16-byte words of eight features
+  uint4 v[VEC ? PT / 8 * kWords : 1];
+  Bits e[VEC ? 1 : PT];
+  template <int THREADS> __device__ __forceinline__ void load(const T* row, int F) {
+    if constexpr (VEC) {
+#pragma unroll
+      for (int c = 0; c < PT / 8; ++c) {
+        const int f = (c * THREADS + static_cast<int>(threadIdx.x)) * 8;
+#pragma unroll
+        for (int w = 0; w < kWords; ++w) {
+          v[c * kWords + w] = make_uint4(0u, 0u, 0u, 0u);
+          if (f < F) v[c * kWords + w] = reinterpret_cast<const uint4*>(row + f)[w];
+        }
+      }
+    } else {
+#pragma unroll
+      for (int c = 0; c < PT; ++c) {
+        const int f = c * THREADS + static_cast<int>(threadIdx.x);
+        e[c] = 0;
+        if (f < F) e[c] = reinterpret_cast<const Bits*>(row)[f];
+      }
+    }
+  }
+  __device__ __forceinline__ void values(float (&x)[PT]) const {
+    if constexpr (VEC) {
+#pragma unroll
+      for (int c = 0; c < PT / 8; ++c) {
+        if constexpr (sizeof(T) == 2) {
+          const uint32_t w[4] = {v[c].x, v[c].y, v[c].z, v[c].w};
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            x[c * 8 + 2 * j] = __uint_as_float(w[j] << 16);
+            x[c * 8 + 2 * j + 1] = __uint_as_float(w[j] & 0xffff0000u);
+          }
+        } else {
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const uint4 w = v[2 * c + h];
+            x[c * 8 + 4 * h] = __uint_as_float(w.x); x[c * 8 + 4 * h + 1] = __uint_as_float(w.y);
+            x[c * 8 + 4 * h + 2] = __uint_as_float(w.z); x[c * 8 + 4 * h + 3] = __uint_as_float(w.w);
+          }
+        }
+      }
+    } else {
+#pragma unroll
+      for (int c = 0; c < PT; ++c) {
+        if constexpr (sizeof(T) == 2) x[c] = __uint_as_float(static_cast<uint32_t>(e[c]) << 16);
+        else x[c] = e[c];
+      }
+    }
+  }
+};
+
 // F beyond the warp-per-row kernel (above 1024, or no multiple of eight) up to 8192: a block owns the whole
 // width, a thread PT features of it (pieces of eight, or every THREADS-th feature when rows are not
-// 16-byte aligned), and R = 32 / PT rows go through the two reductions together, so their loads are in
+// 16-byte aligned), and R = 32 / PT rows (whole ones) go through the two reductions together, so their loads are in
 // flight at once and one barrier serves R rows.  The gradients of a thread's features stay in registers.
 // Bound by the latency of a group of rows (loads, two reductions) more than by HBM: 3 to 4 TB/s.  The
 // block-per-row kernel below reads every row three times in single elements and meets at four
@@ -527,25 +585,6 @@ norm_wide_kernel(const T* A, const T* G, long long Tn, int F, float eps, float* 
   const float invF = 1.f / static_cast<float>(F);
   auto feature = [&](int e) -> int {
     return VEC ? (e / 8) * THREADS * 8 + static_cast<int>(threadIdx.x) * 8 + e % 8 : e * THREADS + static_cast<int>(threadIdx.x);
-  };
-  auto load = [&](const T* row, float (&x)[PT]) {
-    if constexpr (VEC) {
-#pragma unroll
-      for (int c = 0; c < PT / 8; ++c) {
-        float v[8];
-        if (feature(c * 8) < F) {
-          Vec8<T>::load(row + feature(c * 8), v);
-        } else {
-#pragma unroll
-          for (int j = 0; j < 8; ++j) v[j] = 0.f;
-        }
-#pragma unroll
-        for (int j = 0; j < 8; ++j) x[c * 8 + j] = v[j];
-      }
-    } else {
-#pragma unroll
-      for (int e = 0; e < PT; ++e) x[e] = feature(e) < F ? to_f32<T>(row[feature(e)]) : 0.f;
-    }
   };
   int buf = 0;
   // sums of one value per row over the block; the buffers alternate, so one barrier is enough
@@ -582,13 +621,16 @@ norm_wide_kernel(const T* A, const T* G, long long Tn, int F, float eps, float* 
   };
   int chain = 0;
   for (long long t = t0; t < t1; t += R) {
-    float x[R][PT], g[R][PT], s[R];
+    NormRaw<T, VEC, PT> ra[R], rg[R];
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       const long long row = (static_cast<long long>(n) * Tn + (t + r < t1 ? t + r : t)) * F;
-      load(A + row, x[r]);
-      load(G + row, g[r]);
+      ra[r].template load<THREADS>(A + row, F);
+      rg[r].template load<THREADS>(G + row, F);
     }
+    float x[R][PT], g[R][PT], s[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) { ra[r].values(x[r]); rg[r].values(g[r]); }
     if (!rms) {                          // RMS norm: no centring
 #pragma unroll
       for (int r = 0; r < R; ++r) {
@@ -619,7 +661,7 @@ norm_wide_kernel(const T* A, const T* G, long long Tn, int F, float eps, float* 
         ab[e] += g[r][e];
       }
     }
-    if ((chain += R) == kChain) { to_total(); chain = 0; }
+    if ((chain += R) >= kChain) { to_total(); chain = 0; }
   }
   if (!first) {
     to_total();
@@ -875,7 +917,7 @@ static int launch_norm_wide_of(dim3 grid, const T* A, const T* G, long long Tn, 
                                int splits, const DeviceState* ds, cudaStream_t st, int rms) {
   constexpr int kSmem = 2 * PT * THREADS * 4;
   static bool attr_set[64] = {};
-  if (kSmem > 48 * 1024 && !attr_set[ds->device]) {
+  if (kSmem > 47 * 1024 && !attr_set[ds->device]) {
     GB_CUDA_OK(cudaFuncSetAttribute(norm_wide_kernel<T, VEC, PT, THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
     attr_set[ds->device] = true;
   }
@@ -887,7 +929,18 @@ static int launch_norm_wide(dim3 grid, const T* A, const T* G, long long Tn, int
                             int splits, const DeviceState* ds, cudaStream_t st, int rms) {
   if (!VEC && F <= 1024) return launch_norm_wide_of<T, false, 4, 256>(grid, A, G, Tn, F, eps, gw, gb, ws, splits, ds, st, rms);
   if (F <= 2048) return launch_norm_wide_of<T, VEC, 8, 256>(grid, A, G, Tn, F, eps, gw, gb, ws, splits, ds, st, rms);
+  // Rows that begin anywhere are loaded element by element, and a feature beyond F costs its instructions all the same (bf16 RMS
+  // hooks of 6 + 2 x 1024, with 16 features a thread and as many as the row needs, us: F = 2501 52.4 and 42.4,
+  // 3001 54.9 and 47.7, 4097 92 and 72, 5999 106 and 92; float32 4097 84 and 73)
+  if constexpr (!VEC) {
+    if (F <= 2560) return launch_norm_wide_of<T, false, 10, 256>(grid, A, G, Tn, F, eps, gw, gb, ws, splits, ds, st, rms);
+    if (F <= 3072) return launch_norm_wide_of<T, false, 12, 256>(grid, A, G, Tn, F, eps, gw, gb, ws, splits, ds, st, rms);
+  }
   if (F <= 4096) return launch_norm_wide_of<T, VEC, 16, 256>(grid, A, G, Tn, F, eps, gw, gb, ws, splits, ds, st, rms);
+  if constexpr (!VEC) {
+    if (F <= 5120) return launch_norm_wide_of<T, false, 10, 512>(grid, A, G, Tn, F, eps, gw, gb, ws, splits, ds, st, rms);
+    if (F <= 6144) return launch_norm_wide_of<T, false, 12, 512>(grid, A, G, Tn, F, eps, gw, gb, ws, splits, ds, st, rms);
+  }
   return launch_norm_wide_of<T, VEC, 16, 512>(grid, A, G, Tn, F, eps, gw, gb, ws, splits, ds, st, rms);
 }
 

@@ -1345,6 +1345,16 @@ def test_norm_wide_rows(dtype, rms, N, T, F):
     assert O.rel_fro(gb, g.sum(1)) < 2e-6
 
 
+# rows that begin anywhere, as many features a thread as the width needs (10, 12, 16 of 256 and of 512 threads), three or two rows at a
+# time: widths on both sides of each form, row counts that leave a group unfinished, chains that end inside one
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("rms", [False, True])
+@pytest.mark.parametrize("N,T,F", [(2, 1, 2049), (1, 37, 2559), (2, 100, 2561), (1, 5, 3071), (1, 34, 3073), (2, 70, 4097), (1, 101, 5119), (1, 4, 5121),
+                                   (2, 35, 6143), (1, 7, 6145)])
+def test_norm_rows_that_begin_anywhere(dtype, rms, N, T, F):
+    test_norm_wide_rows(dtype, rms, N, T, F)
+
+
 # (B, T, columns of G, of A, k_r, k_c): one unit of 128 tokens to more than the GPU has SMs, so that every cluster size
 # and none is met, with fewer stages of columns than CTAs among them; token counts around a unit; columns that no
 # 16-byte load fits; ranks on both sides of each instantiation's largest
