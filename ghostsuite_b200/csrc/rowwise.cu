@@ -567,7 +567,7 @@ template <typename T, bool VEC, int PT> struct NormRaw {
 // barriers per row; whole LayerNorm hook, 24 samples of 1024 rows of bf16: F = 4096 803 -> 138 us, F = 2048
 // 380 -> 97, F = 731 173 -> 60; RMS norm, 12 x 1024 rows of F = 8192: 1179 -> 138.
 template <typename T, bool VEC, int PT, int THREADS>
-__global__ void __launch_bounds__(THREADS, THREADS == 256 ? 2 : 1)
+__global__ void __launch_bounds__(THREADS, THREADS <= 256 ? 2 : 1)
 norm_wide_kernel(const T* A, const T* G, long long Tn, int F, float eps, float* __restrict__ gw,
                  float* __restrict__ gb, float* __restrict__ part, int t_splits, int rms) {
   constexpr int R = 32 / PT, W = THREADS / 32;
@@ -927,19 +927,27 @@ static int launch_norm_wide_of(dim3 grid, const T* A, const T* G, long long Tn, 
 template <typename T, bool VEC>
 static int launch_norm_wide(dim3 grid, const T* A, const T* G, long long Tn, int F, float eps, float* gw, float* gb, float* ws,
                             int splits, const DeviceState* ds, cudaStream_t st, int rms) {
-  if (!VEC && F <= 1024) return launch_norm_wide_of<T, false, 4, 256>(grid, A, G, Tn, F, eps, gw, gb, ws, splits, ds, st, rms);
-  if (F <= 2048) return launch_norm_wide_of<T, VEC, 8, 256>(grid, A, G, Tn, F, eps, gw, gb, ws, splits, ds, st, rms);
   // Rows that begin anywhere are loaded element by element, and a feature beyond F costs its instructions all the same (bf16 RMS
   // hooks of 6 + 2 x 1024, with 16 features a thread and as many as the row needs, us: F = 2501 52.4 and 42.4,
-  // 3001 54.9 and 47.7, 4097 92 and 72, 5999 106 and 92; float32 4097 84 and 73)
+  // 3001 54.9 and 47.7, 4097 92 and 72, 5999 106 and 92; float32 4097 84 and 73; 16 features of fewer threads: 4097 93, float32 75).
+  // Pieces of eight keep 16 features a thread and take the threads that the row needs, which leaves each more registers for
+  // loads in flight (LayerNorm hooks, 256 or 512 threads and as many as needed: bf16 2304 44.7 and 39.6, 4104 84.5 and 69.6,
+  // 6144 89.8 and 78, 7000 95.4 and 92.3; float32 5120 97.7 and 84.3; 224 threads for 3456: no difference).
   if constexpr (!VEC) {
+    if (F <= 1024) return launch_norm_wide_of<T, false, 4, 256>(grid, A, G, Tn, F, eps, gw, gb, ws, splits, ds, st, rms);
+    if (F <= 2048) return launch_norm_wide_of<T, false, 8, 256>(grid, A, G, Tn, F, eps, gw, gb, ws, splits, ds, st, rms);
     if (F <= 2560) return launch_norm_wide_of<T, false, 10, 256>(grid, A, G, Tn, F, eps, gw, gb, ws, splits, ds, st, rms);
     if (F <= 3072) return launch_norm_wide_of<T, false, 12, 256>(grid, A, G, Tn, F, eps, gw, gb, ws, splits, ds, st, rms);
-  }
-  if (F <= 4096) return launch_norm_wide_of<T, VEC, 16, 256>(grid, A, G, Tn, F, eps, gw, gb, ws, splits, ds, st, rms);
-  if constexpr (!VEC) {
+    if (F <= 4096) return launch_norm_wide_of<T, false, 16, 256>(grid, A, G, Tn, F, eps, gw, gb, ws, splits, ds, st, rms);
     if (F <= 5120) return launch_norm_wide_of<T, false, 10, 512>(grid, A, G, Tn, F, eps, gw, gb, ws, splits, ds, st, rms);
     if (F <= 6144) return launch_norm_wide_of<T, false, 12, 512>(grid, A, G, Tn, F, eps, gw, gb, ws, splits, ds, st, rms);
+  } else {
+    if (F <= 2048) return launch_norm_wide_of<T, true, 8, 256>(grid, A, G, Tn, F, eps, gw, gb, ws, splits, ds, st, rms);
+    if (F <= 3072) return launch_norm_wide_of<T, true, 16, 192>(grid, A, G, Tn, F, eps, gw, gb, ws, splits, ds, st, rms);
+    if (F <= 4096) return launch_norm_wide_of<T, true, 16, 256>(grid, A, G, Tn, F, eps, gw, gb, ws, splits, ds, st, rms);
+    if (F <= 5120) return launch_norm_wide_of<T, true, 16, 320>(grid, A, G, Tn, F, eps, gw, gb, ws, splits, ds, st, rms);
+    if (F <= 6144) return launch_norm_wide_of<T, true, 16, 384>(grid, A, G, Tn, F, eps, gw, gb, ws, splits, ds, st, rms);
+    if (F <= 7168) return launch_norm_wide_of<T, true, 16, 448>(grid, A, G, Tn, F, eps, gw, gb, ws, splits, ds, st, rms);
   }
   return launch_norm_wide_of<T, VEC, 16, 512>(grid, A, G, Tn, F, eps, gw, gb, ws, splits, ds, st, rms);
 }

@@ -1355,6 +1355,15 @@ def test_norm_rows_that_begin_anywhere(dtype, rms, N, T, F):
     test_norm_wide_rows(dtype, rms, N, T, F)
 
 
+# rows of 16-byte pieces, 16 features for as many threads as the width needs: the widest and narrowest row of each form
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("rms", [False, True])
+@pytest.mark.parametrize("N,T,F", [(2, 3, 2056), (1, 67, 3072), (2, 34, 3080), (1, 5, 4096), (2, 67, 4104), (1, 33, 5120), (1, 4, 5128), (2, 66, 6144),
+                                   (1, 7, 6152), (1, 40, 7168), (1, 3, 7176)])
+def test_norm_rows_of_pieces(dtype, rms, N, T, F):
+    test_norm_wide_rows(dtype, rms, N, T, F)
+
+
 # (B, T, columns of G, of A, k_r, k_c): one unit of 128 tokens to more than the GPU has SMs, so that every cluster size
 # and none is met, with fewer stages of columns than CTAs among them; token counts around a unit; columns that no
 # 16-byte load fits; ranks on both sides of each instantiation's largest
