@@ -621,16 +621,25 @@ norm_wide_kernel(const T* A, const T* G, long long Tn, int F, float eps, float* 
   };
   int chain = 0;
   for (long long t = t0; t < t1; t += R) {
-    NormRaw<T, VEC, PT> ra[R], rg[R];
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const long long row = (static_cast<long long>(n) * Tn + (t + r < t1 ? t + r : t)) * F;
-      ra[r].template load<THREADS>(A + row, F);
-      rg[r].template load<THREADS>(G + row, F);
-    }
     float x[R][PT], g[R][PT], s[R];
+    auto at = [&](int r) { return (static_cast<long long>(n) * Tn + (t + r < t1 ? t + r : t)) * F; };
+    if constexpr (!VEC && PT == 4) {     // eight rows of four features: converted at once, 1 % faster (40 + 8 x 1024 x 1001 bf16 83.3 and 84.5 us)
 #pragma unroll
-    for (int r = 0; r < R; ++r) { ra[r].values(x[r]); rg[r].values(g[r]); }
+      for (int r = 0; r < R; ++r)
+#pragma unroll
+        for (int o = 0; o < 2; ++o)
+#pragma unroll
+          for (int e = 0; e < PT; ++e) (o ? g : x)[r][e] = feature(e) < F ? to_f32<T>(((o ? G : A) + at(r))[feature(e)]) : 0.f;
+    } else {
+      NormRaw<T, VEC, PT> ra[R], rg[R];
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        ra[r].template load<THREADS>(A + at(r), F);
+        rg[r].template load<THREADS>(G + at(r), F);
+      }
+#pragma unroll
+      for (int r = 0; r < R; ++r) { ra[r].values(x[r]); rg[r].values(g[r]); }
+    }
     if (!rms) {                          // RMS norm: no centring
 #pragma unroll
       for (int r = 0; r < R; ++r) {
