@@ -18,7 +18,7 @@ LIB = os.path.join(HERE, "libghost_b200.so")
 SOURCES = ["common.cu", "ghost_gram.cu", "ghost_gram_pair.cu", "xty_gemm.cu", "xty_gemm_pair.cu", "tile_dot.cu", "rowwise.cu", "pass_reduce.cu", "dense_small.cu", "conv_tokens.cu", "embedding.cu", "gradproj.cu", "proj_extras.cu", "workload_loss.cu"]
 BINDING = os.path.join(HERE, "_ghost_torch.so")
 BINDING_SOURCE = os.path.join("host", "torch_ops.cpp")
-HEADERS = ["common.cuh", "gram_operands.cuh", "sm100_ptx.cuh", "mma_sync.cuh", "xty_colsum.cuh", "xty_operands.cuh", "xty_store.cuh", os.path.join("..", "..", "include", "ghost_b200.h")]
+HEADERS = ["common.cuh", "gram_operands.cuh", "sm100_ptx.cuh", "mma_sync.cuh", "xty_colsum.cuh", "xty_operands.cuh", "xty_store.cuh", "launch_rules.h", os.path.join("..", "..", "include", "ghost_b200.h")]
 
 
 def _nvcc() -> str:
@@ -47,7 +47,7 @@ def _torch():
 
 
 def _binding_stale() -> bool:
-    return _stale(BINDING, [BINDING_SOURCE, HEADERS[-1]]) or not binding_built_for(_torch()[1], BINDING)
+    return _stale(BINDING, [BINDING_SOURCE] + HEADERS[-2:]) or not binding_built_for(_torch()[1], BINDING)
 
 
 def _start_binding():

@@ -27,6 +27,7 @@
 #include <vector>
 
 #include "../../../include/ghost_b200.h"
+#include "../launch_rules.h"
 
 namespace {
 
@@ -604,19 +605,6 @@ void check_projection_out(const Tensor& out, long long B, long long k, const cha
     invalid(std::string(who) + " output must be a float32 [B, >= k_r*k_c] row-major view");
 }
 
-// Whether bf16 rows that TMA cannot read are copied, padded, instead of being brought through the kernel's loader warps.
-// A copy is a launch and two passes over them; what the loaders add is about half a microsecond per 64 columns of a CTA's
-// chain.  Loaders and copies, us: 26 x 471 tokens of 9408 + 795 109 and 62 (only the 795 columns are copied); 10 x 30 of
-// 6912 + 2579 19.2 and 12.1; 28 x 5 of 3957 + 9063 44.8 and 21.2; 14 x 1894 of 1007 + 1088 51.7 and 54; 32 x 3000 of 1001 + 2003 217 and 369.
-bool gradproj_copies(long long B, long long T, long long n_r, long long n_c, bool ready_r, bool ready_c) {
-  if (ready_r && ready_c) return false;
-  const long long units = B * ((T + 127) / 128), sms = std::max(1, ghost_sm_count());
-  const double stages = (n_r + 63) / 64 + (n_c + 63) / 64;
-  const double chain = 2 * units > sms ? stages * ((units + sms - 1) / sms) : stages / std::min(8ll, sms / units);
-  const double bytes = 2. * B * T * ((ready_r ? 0 : n_r) + (ready_c ? 0 : n_c));
-  return 0.45 * chain > 4.0 + 2. * bytes / 4.5e6;
-}
-
 // (G, A, P_r, P_c, k_r, k_c, scale, out or None: a new [B, k_r, k_c])
 PyObject* py_gradproj_dense(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return guarded([&]() -> PyObject* {
@@ -634,7 +622,7 @@ PyObject* py_gradproj_dense(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const long long n_r = G.size(2), n_c = A.size(2), cp_r = pad8(n_r), cp_c = pad8(n_c);
     if (P_r.size(1) != (split ? 3 : 1) * cp_r || P_c.size(1) != (split ? 3 : 1) * cp_c)
       invalid("projection matrices were prepared for a different dtype/feature size");
-    const bool copies = !split && gradproj_copies(B, T, n_r, n_c, tma_ready(G), tma_ready(A));
+    const bool copies = !split && gb::gradproj_copies(B, T, n_r, n_c, tma_ready(G), tma_ready(A), ghost_sm_count());
     if (k_r <= 64 && k_c <= 64 && !copies) {
       // the prepared split lays a float32 matrix out as (hi, hi, lo): the residual part starts at 2 * cp
       const int f32 = !split ? 0 : !is_f32(A) ? 2 : !is_f32(G) ? 3 : 1;

@@ -2,6 +2,7 @@
 import glob
 import os
 import re
+import subprocess
 
 CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "ghostsuite_b200", "csrc")
 
@@ -70,7 +71,8 @@ def test_a_type_is_defined_once():
 
 def test_every_header_makes_the_library_stale():
     from ghostsuite_b200 import build
-    assert {n for n in _sources() if n.endswith(".cuh")} <= set(build.HEADERS)
+    headers = {os.path.basename(p) for p in glob.glob(os.path.join(CSRC, "*.cuh")) + glob.glob(os.path.join(CSRC, "*.h"))}
+    assert headers <= set(build.HEADERS) and "launch_rules.h" in build.HEADERS[-2:]
 
 
 def test_alignment_slack_of_the_shared_memory_is_not_used():
@@ -112,3 +114,25 @@ def test_a_count_that_the_driver_refused_is_not_kept():
     refused = _body(body, body.index("cudaOccupancyMaxActiveClusters"))
     assert "return 0;" in refused and "store" not in refused
     assert body.index(refused) < body.index("slot.store(")
+
+
+def _answers(tmp_path, calls):
+    """What the rules of launch_rules.h answer to ``calls`` (C++ expressions), each as a number."""
+    src, exe = tmp_path / "rules.cpp", tmp_path / "rules"
+    body = "".join(f'  std::printf("%.17g\\n", static_cast<double>(gb::{c}));\n' for c in calls)
+    src.write_text('#include <cstdio>\n#include "launch_rules.h"\nint main() {\n' + body + "}\n")
+    subprocess.run(["g++", "-std=c++17", "-Wall", "-Werror", f"-I{CSRC}", str(src), "-o", str(exe)], check=True)
+    done = subprocess.run([str(exe)], capture_output=True, text=True)
+    assert done.returncode == 0, f"ended by signal {-done.returncode}"
+    return [float(x) for x in done.stdout.split()]
+
+
+def test_copies_of_projection_operands(tmp_path):
+    """An empty call is answered too (the kernel's own check refuses it), and so is one on a device that was refused."""
+    empty = [f"gradproj_copies({b}, {t}, 65, 40, false, {ready}, {sms})"
+             for b, t in ((0, 5), (3, 0), (0, 0)) for ready in ("false", "true") for sms in (148, 0, -3)]
+    assert set(_answers(tmp_path, empty)) == {0}
+    # calls that are named beside the rule, each on its faster side
+    measured = {"26, 471, 9408, 795, true, false": 1, "10, 30, 6912, 2579, true, false": 1, "28, 5, 3957, 9063, false, false": 1,
+                "32, 3000, 1001, 2003, false, false": 0, "4, 9, 64, 64, true, true": 0}
+    assert _answers(tmp_path, [f"gradproj_copies({c}, 148)" for c in measured]) == list(measured.values())

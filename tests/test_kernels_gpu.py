@@ -1485,6 +1485,14 @@ def test_gradproj_dense_of_mixed_operands(case, f32):
     assert torch.cuda.memory_stats()["allocation.all.allocated"] == made      # workspaces are kept from the first call
 
 
+@pytest.mark.parametrize("B,T", [(0, 5), (3, 0)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_gradproj_dense_refuses_an_empty_call(B, T, dtype):
+    P = [ops().prepare_projection(torch.ones(4, n, device="cuda"), dtype == torch.float32) for n in (65, 40)]
+    with pytest.raises(ValueError):
+        ops().gradproj_dense(torch.zeros(B, T, 65, dtype=dtype, device="cuda"), torch.zeros(B, T, 40, dtype=dtype, device="cuda"), P[0], P[1], 4, 4, 1.0)
+
+
 # Rows that begin anywhere, between values that nothing may take in: every distance of the first row from a 16-byte boundary, pitches of
 # all residues, tokens around the eights that loader warps share and the tile, columns around a slice of 128 bytes and a stage of 64;
 # stages of both groups of warps, and fewer than groups
