@@ -114,6 +114,21 @@ def compute_projection_metadata(layer_name: str, layer: nn.Module, k_i: int, k_o
     return meta
 
 
+def _find_followed_by_torch():
+    """A function that says whether torch follows the operations of this thread one by one (a trace, a function transform,
+    forward-mode derivatives).  torch answers that only under names of its own; None where it has one of them no more."""
+    try:
+        tracing, transform = torch._C._get_tracing_state, torch._C._functorch.peek_interpreter_stack
+        forward = torch.autograd.forward_ad
+        forward._current_level
+    except AttributeError:
+        return None
+    return lambda: tracing() is not None or transform() is not None or forward._current_level >= 0
+
+
+_followed_by_torch = _find_followed_by_torch()
+
+
 def _bf16_sets_for_kernel(a: torch.Tensor, b: torch.Tensor) -> bool:
     """Whether sets of more than ``ops.SIMILARITY_KERNEL_MAX_ROWS`` rows go through the streaming kernel too.
 
@@ -128,8 +143,7 @@ def _bf16_sets_for_kernel(a: torch.Tensor, b: torch.Tensor) -> bool:
         return False
     if type(a) is not torch.Tensor or type(b) is not torch.Tensor or a.requires_grad or b.requires_grad \
             or torch.is_autocast_enabled() or torch.are_deterministic_algorithms_enabled() \
-            or torch.compiler.is_compiling() or torch._C._get_tracing_state() is not None \
-            or torch._C._functorch.peek_interpreter_stack() is not None or torch.autograd.forward_ad._current_level >= 0:
+            or torch.compiler.is_compiling() or _followed_by_torch is None or _followed_by_torch():
         return False
     dim, rows = a.shape[1], max(a.shape[0], b.shape[0])
     if min(a.shape[0], b.shape[0], dim) == 0 or rows > 1 << 16 or a.stride(1) != 1 or b.stride(1) != 1 \

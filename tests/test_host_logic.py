@@ -259,3 +259,23 @@ def test_large_similarity_sets_that_the_kernel_takes():
     seen = []
     torch.func.vmap(lambda x: seen.append(takes(x, rows(2, 8))) or x.sum())(torch.zeros(3, 200, 8, dtype=torch.bfloat16))
     assert seen == [False]
+
+
+@pytest.mark.parametrize("owner,name", [("torch._C", "_get_tracing_state"), ("torch._C._functorch", "peek_interpreter_stack"),
+                                        ("torch.autograd.forward_ad", "_current_level")])
+def test_similarity_without_a_name_of_torch_that_has_no_promise(owner, name, monkeypatch):
+    import importlib.util
+    import torch.autograd.forward_ad
+    from ghostsuite_b200.ghostEngines.gradProjection import projection_utils as U
+    holder = torch
+    for part in owner.split(".")[1:]:
+        holder = getattr(holder, part)
+    spec = importlib.util.spec_from_file_location(U.__name__, U.__file__)
+    fresh = importlib.util.module_from_spec(spec)
+    with monkeypatch.context() as m:
+        m.delattr(holder, name)
+        spec.loader.exec_module(fresh)
+        a, b = torch.ones(130, 128).bfloat16(), torch.ones(3, 128).bfloat16()
+        assert not fresh._bf16_sets_for_kernel(a, b)
+        assert (fresh.projection_similarity(a, b) == 128).all()
+    assert U._bf16_sets_for_kernel(a, b)
