@@ -115,15 +115,15 @@ def compute_projection_metadata(layer_name: str, layer: nn.Module, k_i: int, k_o
 
 
 def _find_followed_by_torch():
-    """A function that says whether torch follows the operations of this thread one by one (a trace, a function transform,
-    forward-mode derivatives).  torch answers that only under names of its own; None where it has one of them no more."""
+    """A function that says whether torch follows the operations of this thread one by one (a trace, a dispatch mode, a
+    function transform, forward-mode derivatives).  torch answers that only under names of its own; None where it has one of them no more."""
     try:
         tracing, transform = torch._C._get_tracing_state, torch._C._functorch.peek_interpreter_stack
-        forward = torch.autograd.forward_ad
+        forward, modes = torch.autograd.forward_ad, torch._C._len_torch_dispatch_stack
         forward._current_level
     except AttributeError:
         return None
-    return lambda: tracing() is not None or transform() is not None or forward._current_level >= 0
+    return lambda: modes() > 0 or tracing() is not None or transform() is not None or forward._current_level >= 0
 
 
 _followed_by_torch = _find_followed_by_torch()

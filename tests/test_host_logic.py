@@ -261,8 +261,27 @@ def test_large_similarity_sets_that_the_kernel_takes():
     assert seen == [False]
 
 
+def test_similarity_of_large_sets_inside_a_dispatch_mode():
+    """A mode that follows torch's operations (a trace with real tensors, a counter) does not see the kernel."""
+    from torch.fx.experimental.proxy_tensor import make_fx
+    from torch.utils.flop_counter import FlopCounterMode
+    from ghostsuite_b200.ghostEngines.gradProjection import projection_utils as U
+    a, b, seen = torch.ones(130, 128).bfloat16(), torch.ones(3, 128).bfloat16(), []
+
+    def scores(x, y):
+        seen.append(U._bf16_sets_for_kernel(x, y))
+        return U.projection_similarity(x, y)
+
+    traced = make_fx(scores, tracing_mode="real")(a, b)
+    assert (traced(2 * a, b) == 256).all()
+    with FlopCounterMode(display=False) as count:
+        scores(a, b)
+    assert count.get_total_flops() == 2 * 130 * 3 * 128
+    assert seen == [False, False] and U._bf16_sets_for_kernel(a, b)
+
+
 @pytest.mark.parametrize("owner,name", [("torch._C", "_get_tracing_state"), ("torch._C._functorch", "peek_interpreter_stack"),
-                                        ("torch.autograd.forward_ad", "_current_level")])
+                                        ("torch._C", "_len_torch_dispatch_stack"), ("torch.autograd.forward_ad", "_current_level")])
 def test_similarity_without_a_name_of_torch_that_has_no_promise(owner, name, monkeypatch):
     import importlib.util
     import torch.autograd.forward_ad
