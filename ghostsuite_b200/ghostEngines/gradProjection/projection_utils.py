@@ -137,11 +137,11 @@ def _bf16_sets_for_kernel(a: torch.Tensor, b: torch.Tensor) -> bool:
     98304 341 and 1628; 4096 x 4096 of 4096 716 and 2499; its error against 64 bits is 6e-8 to 1.6e-7 where the GEMM has 5e-8 to
     6e-7).  Rows that do not start on 16-byte boundaries are read by element: 512 x 512 of 25871 311 and 512,
     1024 x 1024 of them 1259 and 1174, so there it ends at 512 rows.  float32 rows stay with the GEMM, which
-    takes them as they are; so does what the kernel does not know: gradients, transforms, autocast, shared or
-    overlapping rows."""
+    takes them as they are; so does what the kernel does not know: gradients, transforms, autocast, sparse
+    layouts, lazy negation, shared or overlapping rows."""
     if a.dtype is not torch.bfloat16 or b.dtype is not torch.bfloat16 or a.device != b.device:
         return False
-    if type(a) is not torch.Tensor or type(b) is not torch.Tensor or a.requires_grad or b.requires_grad \
+    if any(type(t) is not torch.Tensor or t.layout is not torch.strided or t.is_neg() for t in (a, b)) or a.requires_grad or b.requires_grad \
             or torch.is_autocast_enabled() or torch.are_deterministic_algorithms_enabled() \
             or torch.compiler.is_compiling() or _followed_by_torch is None or _followed_by_torch():
         return False

@@ -261,6 +261,14 @@ def test_large_similarity_sets_that_the_kernel_takes():
     assert seen == [False]
 
 
+def test_large_similarity_sets_that_are_not_plain_rows():
+    from ghostsuite_b200.ghostEngines.gradProjection import projection_utils as U
+    a, b = torch.ones(130, 128).bfloat16(), torch.ones(3, 128).bfloat16()
+    assert U._bf16_sets_for_kernel(a, b)
+    for other in (a.to_sparse(), a.to_sparse_csr(), torch._neg_view(a)):
+        assert not U._bf16_sets_for_kernel(other, b) and not U._bf16_sets_for_kernel(b, other)
+
+
 def test_similarity_of_large_sets_inside_a_dispatch_mode():
     """A mode that follows torch's operations (a trace with real tensors, a counter) does not see the kernel."""
     from torch.fx.experimental.proxy_tensor import make_fx
