@@ -247,17 +247,19 @@ def test_large_similarity_sets_that_the_kernel_takes():
     from ghostsuite_b200.ghostEngines.gradProjection import projection_utils as U
     rows = lambda n, d: torch.zeros(n, d, dtype=torch.bfloat16)
     takes = U._bf16_sets_for_kernel
-    assert takes(rows(1, 8), rows(65536, 8)) and takes(rows(129, 31), rows(512, 31))
-    assert takes(rows(600, 24)[:, 8:16], rows(3, 8)) and not takes(rows(600, 24)[:, 4:12], rows(3, 8))
-    assert not takes(rows(1, 8), rows(65537, 8)) and not takes(rows(513, 31), rows(1, 31))
-    assert not takes(rows(0, 8), rows(200, 8)) and not takes(rows(200, 0), rows(200, 0))
-    assert not takes(rows(200, 8), rows(200, 8).float()) and not takes(rows(200, 8).double(), rows(200, 8).double())
-    assert not takes(rows(1, 8).expand(200, 8), rows(2, 8)) and not takes(rows(8, 200).t(), rows(2, 8))
-    assert not takes(rows(200, 8).requires_grad_(), rows(2, 8))
+    assert takes(rows(2, 96), rows(65536, 96)) and takes(rows(129, 101), rows(512, 101))
+    assert takes(rows(600, 120)[:, 8:104], rows(3, 96)) and not takes(rows(600, 120)[:, 4:100], rows(3, 96))
+    assert not takes(rows(2, 96), rows(65537, 96)) and not takes(rows(513, 101), rows(2, 101))
+    assert not takes(rows(1, 96), rows(200, 96)) and not takes(rows(200, 4096), rows(1, 4096))         # less exact than the GEMM
+    assert not takes(rows(200, 95), rows(200, 95)) and not takes(rows(200, 8), rows(200, 8))
+    assert not takes(rows(0, 96), rows(200, 96)) and not takes(rows(200, 0), rows(200, 0))
+    assert not takes(rows(200, 96), rows(200, 96).float()) and not takes(rows(200, 96).double(), rows(200, 96).double())
+    assert not takes(rows(1, 96).expand(200, 96), rows(2, 96)) and not takes(rows(96, 200).t(), rows(2, 96))
+    assert not takes(rows(200, 96).requires_grad_(), rows(2, 96))
     with torch.autograd.forward_ad.dual_level():
-        assert not takes(rows(200, 8), rows(2, 8))
+        assert not takes(rows(200, 96), rows(2, 96))
     seen = []
-    torch.func.vmap(lambda x: seen.append(takes(x, rows(2, 8))) or x.sum())(torch.zeros(3, 200, 8, dtype=torch.bfloat16))
+    torch.func.vmap(lambda x: seen.append(takes(x, rows(2, 96))) or x.sum())(torch.zeros(3, 200, 96, dtype=torch.bfloat16))
     assert seen == [False]
 
 
