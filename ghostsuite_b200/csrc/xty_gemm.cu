@@ -25,6 +25,7 @@
 #include "gram_operands.cuh"
 #include "xty_operands.cuh"
 #include "xty_store.cuh"
+#include "launch_rules.h"
 
 namespace gb {
 
@@ -499,9 +500,9 @@ static int wgrad(const XtyOperands& o, long long n_rows, float scale, int accumu
   const bool pair = pair_kernel_fits(g_wgrad_pair_mode, o, ds);
   // in row blocks of the kernel; a block of two-part operands is half as many tokens and three products
   const int kb_pair = ceil_div(n_rows, o.parts == 2 ? 64 : 128);
-  const int splits = pair ? pick_k_splits(static_cast<long long>(ceil_div(m_cols, 256)) * p.n_tiles, ds->sm_count / 2, kb_pair, out_is_f32 ? 32 : 6,
-                                          elems, out_is_f32 != 0)
-                          : pick_k_splits(tiles, ds->sm_count, kb, out_is_f32 ? 64 : 12, elems, out_is_f32 != 0);
+  const int splits = pair ? pick_k_splits(static_cast<long long>(ceil_div(m_cols, 256)) * p.n_tiles, ds->sm_count / 2, kb_pair, 0.65,
+                                          out_is_f32 ? 32 : 6, elems, out_is_f32 != 0)
+                          : pick_k_splits(tiles, ds->sm_count, kb, o.parts == 2 ? 0.5 : 0.35, out_is_f32 ? 64 : 12, elems, out_is_f32 != 0);
   if (splits == 1) p.mode = kEpiDirect;
   else if ((rc = clear_ahead(ws, static_cast<size_t>(m_cols) * p.ld_acc * 4, st)) != GHOST_OK) return rc;
   if (pair) {

@@ -198,28 +198,4 @@ __device__ __forceinline__ void store_tile_f32(const CUtensorMap* tm, uint8_t* s
   }
 }
 
-// Split-K factor of a train-gradient pass with the shortest critical path, in units of one row block
-// of one tile (0.65 us on the CTA pairs, 0.35 on single CTAs, whose blocks hold half the rows, as long as a tile's loads are
-// bound by their latency): ceil(units / workers) rounds of (row blocks per split + a
-// fixed cost per unit for the accumulator hand-over and the epilogue: `add_cost` with red.add
-// into the workspace, a quarter of it with plain stores).  Splitting also pays for zeroing
-// the fp32 workspace and for the scaling pass: two launches (5 us) and ten bytes per weight element
-// at 5 TB/s; one split stores the result itself.  With the costs of the epilogue that stored a row a lane and half the time a
-// block, splits came too late (bf16, us, then and now: 4096 rows of 128 x 128 32.8 and 13.3, 768 x 768 29.9 and 22.2, 8192
-// rows of 3072 x 768 53 and 48, 1600 x 1200 59 and 48; 4096 of 1600 x 1200 34.8 and 35.9).
-// The tensor core's accumulator truncates, so the error grows with the rows one split covers.  A bf16
-// result does not show it; a float32 result does (4096 rows of 768 x 768, bf16 operands: 4.2e-6 off the
-// 64-bit result in one split, 4.5e-7 in ten), so there the merge is not counted against splitting, and a higher add_cost
-// stands for it, which keeps large results in one split.
-inline int pick_k_splits(long long tiles, int workers, int kb, int add_cost, double weight_elems, bool f32_result) {
-  int splits = 1;
-  double best = static_cast<double>((tiles + workers - 1) / workers) * (kb + (f32_result ? add_cost : add_cost / 4));
-  const double merge = f32_result ? 0. : (5.0 + weight_elems * 10.0 / 5e6) / 0.65;
-  for (int s = 2; s <= 64 && s <= kb; ++s) {
-    const double cost = static_cast<double>((tiles * s + workers - 1) / workers) * ((kb + s - 1) / s + add_cost) + merge;
-    if (cost < best) { best = cost; splits = s; }
-  }
-  return splits;
-}
-
 }  // namespace gb

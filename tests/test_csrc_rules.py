@@ -136,3 +136,15 @@ def test_copies_of_projection_operands(tmp_path):
     measured = {"26, 471, 9408, 795, true, false": 1, "10, 30, 6912, 2579, true, false": 1, "28, 5, 3957, 9063, false, false": 1,
                 "32, 3000, 1001, 2003, false, false": 0, "4, 9, 64, 64, true, true": 0}
     assert _answers(tmp_path, [f"gradproj_copies({c}, 148)" for c in measured]) == list(measured.values())
+
+
+def test_splits_of_a_train_gradient(tmp_path):
+    """(tiles, CTAs, row blocks, time of one, cost of an addition, elements, float32) of measured calls on 148 SMs: what a
+    merge costs counts in the time of a block of the kernel that is meant."""
+    single = {"65, 148, 47, 0.35, 12, 1600. * 1200, false": 1, "65, 148, 64, 0.35, 12, 1600. * 1200, false": 1,
+              "65, 148, 128, 0.35, 12, 1600. * 1200, false": 2, "45, 148, 32, 0.35, 12, 1152. * 1152, false": 1}
+    pairs = {"36, 74, 64, 0.65, 6, 3072. * 768, false": 2}
+    assert _answers(tmp_path, [f"pick_k_splits({c})" for c in {**single, **pairs}]) == [*single.values(), *pairs.values()]
+    # few tiles are shared, one block is not
+    few, one = _answers(tmp_path, ["pick_k_splits(1, 148, 64, 0.35, 12, 128. * 128, false)", "pick_k_splits(1, 148, 1, 0.35, 12, 128. * 128, false)"])
+    assert few > 4 and one == 1
