@@ -132,39 +132,65 @@ __device__ __forceinline__ void store_grad_rows(const GradOut& g, uint32_t t_acc
 
 // The same rows added to the fp32 workspace of a result that several CTAs share: whole lines of four rows a store, rows of `ld` (a
 // multiple of four), from a 16-byte boundary where the caller's workspace begins on one.  (A row a lane: 8192 rows of 256 x 256 bf16 23.6 us,
-// 768 x 768 float32 43.4; 19.5 and 37.9 so.)
+// 768 x 768 float32 43.4; 19.5 and 37.9 so.)  A result of up to 48 rows has one or two warps of a tile at work, and the way through shared
+// memory is longer than it saves: those go a row a lane (bf16 results, us, lines and a row a lane: 6000 token rows of 16 x 4096 14.5 and 13.4,
+// 33 x 4096 15.1 and 13.8, 40 x 4096 15.2 and 14.3, 16384 of 40 x 1024 13.2 and 13.5; of 64 x 1024 13.6 and 15.1, of 96 x 1024 14.1 and 16.8).
 __device__ __forceinline__ void add_grad_rows(float* ws, long long ld, int rows, int cols, uint32_t t_acc, int m0, int n0, uint8_t* box) {
   const int lane = threadIdx.x & 31, c = lane & 7;
   const int nrow = rows - m0 < 32 ? rows - m0 : 32;
   if (nrow <= 0) return;
   const bool aligned = (reinterpret_cast<uintptr_t>(ws) & 15) == 0;
+  // zeros behind the last column, up to the row's end
+  auto add4 = [](float* at, float x, float y, float z, float w) {
+    asm volatile("red.global.v4.f32.add [%0], {%1, %2, %3, %4};" ::"l"(at), "f"(x), "f"(y), "f"(z), "f"(w) : "memory");
+  };
+  if (rows <= 48 && aligned) {
+    float* at = ws + (m0 + lane) * ld + n0;
 #pragma unroll 1
-  for (int c0 = 0; c0 < 256 && n0 + c0 < cols; c0 += 32) {
-    uint32_t r[32];
-    tmem_ld32(t_acc + c0, r);
-    tmem_ld_wait();
-    __syncwarp();                          // the block before has been read
+    for (int c0 = 0; c0 < 256 && n0 + c0 < cols; c0 += 32) {
+      uint32_t r[32];
+      tmem_ld32(t_acc + c0, r);
+      tmem_ld_wait();
+      if (lane < nrow) {
 #pragma unroll
-    for (int q = 0; q < 8; ++q) st_shared_v4(box + lane * 128 + ((q ^ c) << 4), r[4 * q], r[4 * q + 1], r[4 * q + 2], r[4 * q + 3]);
-    __syncwarp();
-    float4 v[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int row = 4 * i + (lane >> 3);
-      v[i] = *reinterpret_cast<const float4*>(box + row * 128 + ((c ^ (row & 7)) << 4));
+        for (int q = 0; q < 8; ++q)
+          if (n0 + c0 + 4 * q < cols)
+            add4(at + c0 + 4 * q, __uint_as_float(r[4 * q]), __uint_as_float(r[4 * q + 1]), __uint_as_float(r[4 * q + 2]), __uint_as_float(r[4 * q + 3]));
+      }
     }
+    return;
+  }
+#pragma unroll 1
+  for (int c0 = 0; c0 < 256 && n0 + c0 < cols; c0 += 64) {
+    uint32_t r[2][32];
+    tmem_ld32(t_acc + c0, r[0]);
+    tmem_ld32(t_acc + c0 + 32, r[1]);
+    tmem_ld_wait();
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int row = 4 * i + (lane >> 3);
-      if (row >= nrow || n0 + c0 + 4 * c >= cols) continue;
-      float* at = ws + (m0 + row) * ld + n0 + c0 + 4 * c;
-      if (aligned) {                       // zeros behind the last column, up to the row's end
-        asm volatile("red.global.v4.f32.add [%0], {%1, %2, %3, %4};" ::"l"(at), "f"(v[i].x), "f"(v[i].y), "f"(v[i].z), "f"(v[i].w)
-                     : "memory");
-      } else {
-        const float e[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
+    for (int h = 0; h < 2; ++h) {
+      __syncwarp();                        // the block before has been read
 #pragma unroll
-        for (int j = 0; j < 4; ++j) asm volatile("red.global.add.f32 [%0], %1;" ::"l"(at + j), "f"(e[j]) : "memory");
+      for (int q = 0; q < 8; ++q)
+        st_shared_v4(box + lane * 128 + ((q ^ c) << 4), r[h][4 * q], r[h][4 * q + 1], r[h][4 * q + 2], r[h][4 * q + 3]);
+      __syncwarp();
+      float4 v[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int row = 4 * i + (lane >> 3);
+        v[i] = *reinterpret_cast<const float4*>(box + row * 128 + ((c ^ (row & 7)) << 4));
+      }
+      const int col = n0 + c0 + 32 * h + 4 * c;
+      float* at = ws + (m0 + (lane >> 3)) * ld + col;
+#pragma unroll
+      for (int i = 0; i < 8; ++i, at += 4 * ld) {
+        if (4 * i + (lane >> 3) >= nrow || col >= cols) continue;
+        if (aligned) {
+          add4(at, v[i].x, v[i].y, v[i].z, v[i].w);
+        } else {
+          const float e[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
+#pragma unroll
+          for (int j = 0; j < 4; ++j) asm volatile("red.global.add.f32 [%0], %1;" ::"l"(at + j), "f"(e[j]) : "memory");
+        }
       }
     }
   }

@@ -1638,7 +1638,7 @@ def test_few_rows_shared_by_clusters(n_t, n_v, T, d, p, dtype):
 # results that the GEMM writes itself (few rows) and adds up in a workspace: blocks of 32 rows and 32 or 64 columns that end early,
 # rows that begin on 16 bytes and anywhere, an unaligned result, old values kept; whole numbers, so exact in every type
 @pytest.mark.parametrize("parts,out_dtype", [(1, torch.bfloat16), (1, torch.float32), (2, torch.float32), (2, torch.bfloat16)])
-@pytest.mark.parametrize("m,n", [(1, 1), (33, 65), (129, 257), (160, 328), (300, 63)])
+@pytest.mark.parametrize("m,n", [(1, 1), (33, 65), (129, 257), (160, 328), (300, 63), (48, 318), (49, 545)])
 @pytest.mark.parametrize("rows", [40, 3000])
 def test_train_gradient_stores(rows, m, n, parts, out_dtype):
     from ghostsuite_b200 import _lib
