@@ -55,10 +55,10 @@ struct GramCfg {
 };
 
 // Adds the sums of a warp's 32 rows, `b` their train samples (-1: none), for validation sample v: once if all rows are of one sample.
-struct GramRows {
+struct GramRowsAlone {
   int b, b_first;
   bool uniform;
-  __device__ __forceinline__ GramRows(const GramParams& p, long long row) {
+  __device__ __forceinline__ GramRowsAlone(const GramParams& p, long long row) {
     b = row < p.rows_t ? static_cast<int>(row / p.T) : -1;
     // rows are ascending, so the warp covers one train sample iff its first and last rows agree
     b_first = __shfl_sync(0xffffffffu, b, 0);
@@ -74,6 +74,37 @@ struct GramRows {
     } else if (b >= 0) {
       atomicAdd(&p.M[static_cast<long long>(v) * p.n_train + b], val);
     }
+  }
+};
+
+// Adds the sums of a warp's 32 rows for validation sample v, one addition per train sample among them: lane l takes in lane l + o
+// while that is a row of the same sample (rows are ascending).  A share of the columns is a sixteenth or less of a tile, so a row a lane
+// adds as many times more often to the same few sums: with one addition per row, where a warp holds two samples, 12 + 6 x 83 bf16 tokens
+// of 1792 + 64 took 22.8 us in four CTAs a tile, 15.3 alone and 13.8 so; 6 + 4 x 111 of 1344 + 798 25.4, 17.5 and 17.3.
+struct GramRows {
+  int b;                   // this lane's train sample, -1: none
+  uint32_t same;           // bit i: lane + 2^i has it too
+  bool first;              // of the sample's lanes
+  __device__ __forceinline__ GramRows(const GramParams& p, long long row) {
+    const int lane = threadIdx.x & 31;
+    b = row < p.rows_t ? static_cast<int>(row / p.T) : -1;
+    same = 0;
+#pragma unroll
+    for (int i = 0; i < 5; ++i) {
+      const int other = __shfl_down_sync(0xffffffffu, b, 1 << i);
+      same |= static_cast<uint32_t>(lane + (1 << i) < 32 && other == b) << i;
+    }
+    const int before = __shfl_up_sync(0xffffffffu, b, 1);
+    first = b >= 0 && (lane == 0 || before != b);
+  }
+  __device__ __forceinline__ void flush(const GramParams& p, float val, int v) const {
+    if (v >= p.n_val) return;
+#pragma unroll
+    for (int i = 0; i < 5; ++i) {
+      const float other = __shfl_down_sync(0xffffffffu, val, 1 << i);
+      if (same >> i & 1) val += other;
+    }
+    if (first) atomicAdd(&p.M[static_cast<long long>(v) * p.n_train + b], val * p.scale);
   }
 };
 
@@ -295,7 +326,7 @@ ghost_gram_kernel(const __grid_constant__ CUtensorMap tm_at, const __grid_consta
       tc_fence_after_sync();
 
       const long long row = m0 + threadIdx.x;
-      const GramRows rows(p, row);
+      const GramRowsAlone rows(p, row);
 
       int cur_v = static_cast<int>(n0 / p.T);
       long long boundary = static_cast<long long>(cur_v + 1) * p.T - n0;   // tile-relative column

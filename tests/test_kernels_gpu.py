@@ -76,9 +76,11 @@ def test_gram_hook_tile_shapes(in_by_out, case, dtype):
 
 
 # calls of few tiles and long rows, whose tiles are shared by clusters: K steps of both operands that part inside a CTA's run, at its
-# edge and leave most CTAs one operand only; columns and rows that end inside a quarter, one token, more tiles than clusters of eight
+# edge and leave most CTAs one operand only; columns and rows that end inside a quarter, one token, more tiles than clusters of eight; a
+# sample a lane, several a warp, two and one, and warps without rows
 @pytest.mark.parametrize("dtype,mode", [(torch.bfloat16, 0), (torch.float32, 0), (torch.bfloat16, 1)])
-@pytest.mark.parametrize("case", [(2, 1, 1, 2048, 2048), (5, 3, 13, 4096, 40), (3, 2, 70, 24, 5003), (9, 5, 41, 1031, 1500), (33, 4, 64, 1536, 1536)])
+@pytest.mark.parametrize("case", [(2, 1, 1, 2048, 2048), (5, 3, 13, 4096, 40), (3, 2, 70, 24, 5003), (9, 5, 41, 1031, 1500), (33, 4, 64, 1536, 1536),
+                                  (70, 9, 1, 3000, 64), (43, 3, 3, 64, 2500), (8, 2, 32, 1600, 300), (7, 3, 31, 900, 1800), (5, 2, 129, 2048, 64)])
 def test_gram_tiles_shared_by_clusters(case, dtype, mode):
     n_t, n_v, T, d, p = case
     A, G = make(n_t + n_v, T, d, p, dtype, seed=34)
