@@ -103,10 +103,16 @@ struct GpCfg {
   static constexpr int kStages = kLoaders ? (PARTS == 2 ? (KMAX == 32 ? 3 : 2) : 5) : kFree / kStageBytes < 8 ? kFree / kStageBytes : 8;
   static constexpr int kProjStages = kLoaders ? 3 : kStages;
   static constexpr int kRings = kStages * kStageBytes + (kLoaders ? kProjStages * kProjStageBytes : 0);
-  // Sixteen loader warps, eight to a stage, where the epilogue leaves them registers (embedding form, k = 32, with its gathered
-  // rows in them: 10.9 us with eight, 13.5 with sixteen and spills) and the memory two slots each.  A warp's time for a stage is the
-  // latency of its instructions, so two groups take turns: 16 x 2048 tokens of 1024 + 1024 float32 77 us with eight, 64 with sixteen.
-  static constexpr int kLoaderWarps = !kLoaders ? 0 : (kEmb && (KMAX == 64 || kCluster == kNone)) || (KMAX == 64 && PARTS == 2 && kCluster == kNone) ? 8 : 16;
+  // Sixteen loader warps, eight to a stage, or eight.  A warp's time for a stage is the latency of its instructions, so two groups take
+  // turns (16 x 2048 tokens of 1024 + 1024 float32 77 us with eight, 64 with sixteen; 30 x 1000 of 77 + 1025, k = 64, 77.3 and 69.6), but
+  // more threads come up later and leave each fewer registers.  Eight where that is the more, us with eight and with sixteen:
+  // * embedding form, whose epilogue holds gathered rows (spills: k = 32 of units alone 10.9 and 13.5; bf16 in clusters, 2 x 142 tokens of 510
+  //   7.5 and 8.0, 12 x 546 of 482 11.2 and 11.7), except float32 rows in clusters at k = 32 (8 x 372 of 1042 14.9 and 14.1);
+  // * mixed operands at k = 64, units alone (14 x 1658 float32 tokens of 352 and bf16 of 128 38.6 and 39.2, the other way round 36.8 and 38.2).
+  // Forms that spill a little with sixteen are the faster ones all the same (k = 64, bf16, units alone: 27 x 1543 of 3521 + 2048 208 and 175).
+  static constexpr int kLoaderWarps = !kLoaders ? 0
+                                      : kEmb    ? (kSrc == kSrcF32 && KMAX == 32 && kCluster != kNone ? 16 : 8)
+                                                : (kSrc == kSrcMixed && KMAX == 64 && kCluster == kNone ? 8 : 16);
   // Rows on their way: a slot is 128 bytes of columns of a loader warp's 16 rows, from the 16-byte boundary before them
   static constexpr int kSlotPitch = 128 + 16, kSlotBytes = 16 * kSlotPitch;
   static constexpr int kSlotsBytes = kLoaderWarps * kSlotBytes;      // a slot of every warp
