@@ -996,3 +996,66 @@ def test_validation_gradient_exchange_matches_replicated_validation(world, overl
     finally:
         L.PATH_RULE = old_rule
         gops.EXCHANGE_DEPTH = old_depth
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("native", [True, False])
+def test_end_of_a_pass_in_one_native_call(native, monkeypatch):
+    """The lists of a backward pass, finished natively and by the Python form beside it: a parameter with two jobs (its train gradients
+    add up, its last matrix counts), one whose matrix was replaced meanwhile, one with a matrix alone, one with a shape
+    of its own; the observer hears of every train gradient, in the order of the hooks."""
+    from ghostsuite_b200 import ops
+    from ghostsuite_b200.ghostEngines import supported_layers_grad_samplers_dotprod as L
+    if not native:
+        monkeypatch.setattr(ops, "finish_pass", lambda *a: False)
+    g = torch.Generator(device="cuda").manual_seed(5)
+    n_t, n_v, F = 6, 2, 40
+    twice, replaced, alone, shaped = (torch.nn.Parameter(torch.zeros(s, device="cuda")) for s in ((F,), (F,), (3, 4), (5, 8)))
+    X = [torch.randn(n_t + n_v, F, generator=g, device="cuda") for _ in range(4)]
+    M = [torch.full((n_v, n_t), 7.0, device="cuda") for _ in range(4)]
+    given = torch.randn(n_v, n_t, generator=g, device="cuda")
+    sums = [torch.full((F,), 7.0, device="cuda") for _ in range(4)]
+    heard = []
+    monkeypatch.setattr(L, "TRAIN_GRAD_OBSERVER", lambda p: heard.append(p))
+    assert L.begin_deferred_dots()
+    first, second = {}, {}
+    L._record_hook(first, n_t, n_v, ((twice, M[0], X[0]), (replaced, M[1], X[1]), (alone, given, None)))
+    assert L._sum_into_job(first, twice, X[0], n_t, 0.5, sums[0]) and L._sum_into_job(first, replaced, X[1], n_t, 0.5, sums[1])
+    assert not L._sum_into_job(first, twice, X[0], n_t, 0.5, sums[3])          # its job has an output already
+    assert not L._sum_into_job(first, alone, given, n_t, 0.5, sums[3])         # no job
+    L._record_hook(second, n_t, n_v, ((shaped, M[2], X[2]), (twice, M[3], X[3])))
+    assert L._sum_into_job(second, shaped, X[2], n_t, 0.25, sums[2]) and L._sum_into_job(second, twice, X[3], n_t, 2.0, sums[3])
+    other = torch.zeros(n_v, n_t, device="cuda")
+    replaced.grad_dot_prod_matrix = other
+    L.finalize_pending_dots()
+    assert not L._sum_into_job(first, replaced, X[1], n_t, 0.5, sums[1])       # the pass is over
+    torch.cuda.synchronize()
+    grams = [x[n_t:].double() @ x[:n_t].double().t() for x in X]
+    bound = F * 2.0 ** -23 * max(x.double().abs().max() for x in X) ** 2 * F
+    assert all(((m.double() - r).abs() <= bound).all() for m, r in zip(M, grams))
+    for p, m, vector in ((twice, M[3], M[3]), (alone, given, given), (shaped, M[2], M[2]), (replaced, other, M[1])):
+        assert p.grad_dot_prod_matrix is m
+        if p is not replaced:
+            assert p.grad_dot_prod.shape == (n_t,) and torch.allclose(p.grad_dot_prod, vector.sum(0), rtol=1e-5, atol=1e-5)
+    assert replaced.grad_dot_prod is M[1]                                      # the placeholder of the hook
+    rows = [x[:n_t].double().sum(0) for x in X]
+    for p, want in ((twice, 0.5 * rows[0] + 2.0 * rows[3]), (replaced, 0.5 * rows[1]), (shaped, 0.25 * rows[2].view(5, 8))):
+        assert p.train_grad.shape == p.shape and torch.allclose(p.train_grad.double(), want, rtol=1e-5, atol=1e-5)
+    assert not hasattr(alone, "train_grad") and [id(p) for p in heard] == [id(p) for p in (twice, replaced, shaped, twice)]
+
+
+@pytest.mark.gpu
+def test_end_of_a_pass_with_a_matrix_on_the_host():
+    """The native form does nothing and says so; the Python form takes both."""
+    from ghostsuite_b200 import ops
+    from ghostsuite_b200.ghostEngines import supported_layers_grad_samplers_dotprod as L
+    a, b = (torch.nn.Parameter(torch.zeros(3, device="cuda")) for _ in range(2))
+    mats = [torch.ones(2, 3, device="cuda"), torch.ones(2, 3)]
+    before = ops.launch_count()
+    assert ops.finish_pass([], [(a, mats[0]), (b, mats[1])], None) is False
+    assert ops.launch_count() == before and not hasattr(a, "grad_dot_prod") and not hasattr(b, "grad_dot_prod")
+    L.begin_deferred_dots()
+    for p, m in zip((a, b), mats):
+        L._set_dot(p, m)
+    L.finalize_pending_dots()
+    assert a.grad_dot_prod.tolist() == b.grad_dot_prod.tolist() == [2.0, 2.0, 2.0]
