@@ -55,6 +55,7 @@ PROTOTYPES = {
     "ghost_gram_dot_bf16": (_i, [_vp, _vp, _vp, _vp, _i, _i, _ll, _i, _i, _ll, _ll, _ll, _ll, _i, _f, _vp, _vp]),
     "ghost_gram_dot_parts": (_i, [_vp, _vp, _i, _i, _i, _ll, _i, _i, _ll, _ll, _i, _f, _vp, _vp]),
     "ghost_set_gram_pair_mode": (_i, [_i]),
+    "ghost_gram_cluster_size": (_i, [_i, _i, _i, _ll, _i, _i]),
     "ghost_set_persample_pair_mode": (_i, [_i]),
     "ghost_set_wgrad_pair_mode": (_i, [_i]),
     "ghost_wgrad_workspace_bytes": (_ll, [_i, _i]),
@@ -69,6 +70,7 @@ PROTOTYPES = {
     "ghost_persample_tiles_bf16": (_i, [_vp, _vp, _i, _ll, _i, _i, _ll, _ll, _i, _i, _i, _vp, _vp, _ll, _vp]),
     "ghost_tile_dot_bf16": (_i, [_vp, _i, _i, _vp, _i, _i, _i, _f, _vp, _vp, _i, _f, _i, _vp]),
     "ghost_dense_small_fits": (_i, [_i, _i, _i, _ll, _i, _i]),
+    "ghost_dense_small_cluster_size": (_i, [_i, _i, _ll, _i, _i, _i]),
     "ghost_dense_small": (_i, [_vp, _vp, _i, _i, _i, _ll, _i, _i, _i, _vp, _vp, _i, _f, _vp, _vp]),
     "ghost_colsum": (_i, [_vp, _i, _i, _ll, _i, _ll, _vp, _vp]),
     "ghost_layernorm_workspace_bytes": (_ll, [_i, _ll, _i]),

@@ -7,6 +7,7 @@
 // share out the three results; nothing is converted, zeroed or written twice.  Layer 1024 -> 1024,
 // 64 + 16 samples of one token, float32: 11 launches, 93 us of GPU time before, one of 7 us now.
 #include "common.cuh"
+#include "launch_rules.h"
 #include "sm100_ptx.cuh"
 
 namespace gb {
@@ -312,20 +313,25 @@ static cudaError_t launch_small(const SmallDense& q, unsigned grid, cudaStream_t
   return launch_next(dense_small_kernel<E, VEC, false>, dim3(grid), dim3(256), 0, st, q);
 }
 
-// Blocks that share a pair of groups of samples.  A step of 1024 columns takes a block 1.1 us, and the pairs are few where the rows are
-// long (4 + 12 samples of one token, float32 108 -> 27072: 36.9 us in two blocks, 14.5 in sixteen; 8 + 2 of 20000 -> 10 35.9 and 14.3;
-// 2 + 2 x 8 of 4096 -> 512 17.0 and 14.5).  A tile costs a cluster's barrier, 1.5 us, on top (8 + 2 x 16 of 2048 -> 1024, eight
-// tiles a pair: 38.9, 41 shared).  Where the gradient's blocks take longer than the chain nothing is gained, and
-// they come up slower in clusters (2 + 1 of 768 -> 50000 71 and 77; 16 + 4 of 4095 -> 4097 47 and 53).
-static int small_ranks(long long gram, long long tiles, long long wgrad, long long rows, int d, int p, const DeviceState* ds) {
-  const double others = static_cast<double>((wgrad + 2 * ds->sm_count - 1) / (2 * ds->sm_count)) * (2.0 + 0.045 * rows);
-  int best = 1;
-  double cost = 1.1 * (ceil_div(d, 1024) + ceil_div(p, 1024)) * tiles;
-  for (int r = 2; r <= 8 && gram * r <= 2ll * ds->sm_count && cost > others; r *= 2) {
-    const double c = (1.1 * (ceil_div(d, 1024 * r) + ceil_div(p, 1024 * r)) + 1.5) * tiles;
-    if (c < cost) { best = r; cost = c; }
-  }
-  return best;
+// Sample groups of a call, and what small_cluster() makes of it
+struct SmallGroups { int sv, sb, groups_b; long long gram, wgrad; int ranks; };
+static SmallGroups small_groups(int n_train, int n_val, long long T, int d, int p, bool want_grad, const DeviceState* ds) {
+  SmallGroups g;
+  // groups of whole samples: a tile's worth of one-token samples, fewer longer ones, at least one
+  g.sv = T >= kSdV ? 1 : static_cast<int>(kSdV / T);
+  g.sb = T >= kSdB ? 1 : static_cast<int>(kSdB / T);
+  g.groups_b = ceil_div(n_train, g.sb);
+  g.gram = static_cast<long long>(ceil_div(n_val, g.sv)) * g.groups_b;
+  g.wgrad = want_grad ? static_cast<long long>(ceil_div(d, 64)) * ceil_div(p, 64) : 0;
+  g.ranks = small_cluster(g.gram, (T + kSdV - 1) / kSdV * ((T + kSdB - 1) / kSdB), g.wgrad, n_train * T, d, p, ds->sm_count);
+  return g;
+}
+
+extern "C" int ghost_dense_small_cluster_size(int n_train, int n_val, long long T, int d, int p, int want_grad) {
+  const DeviceState* ds = device_state();
+  if (!ds) return GHOST_ERR_DEVICE;
+  GB_REQUIRE(n_train > 0 && n_val > 0 && T > 0 && d > 0 && p > 0, "ghost_dense_small_cluster_size: bad size");
+  return small_groups(n_train, n_val, T, d, p, want_grad != 0, ds).ranks;
 }
 
 extern "C" int ghost_dense_small(const void* A, const void* B, int is_f32, int n_train, int n_val, long long T, int d,
@@ -344,17 +350,12 @@ extern "C" int ghost_dense_small(const void* A, const void* B, int is_f32, int n
   q.M = M_out;
   q.grad = grad_out; q.grad_f32 = grad_is_f32; q.grad_scale = grad_scale;
   q.colsums = colsum_out;
-  // groups of whole samples: a tile's worth of one-token samples, fewer longer ones, at least one
-  q.sv = T >= kSdV ? 1 : static_cast<int>(kSdV / T);
-  q.sb = T >= kSdB ? 1 : static_cast<int>(kSdB / T);
-  q.groups_b = ceil_div(n_train, q.sb);
-  const long long gram = static_cast<long long>(ceil_div(n_val, q.sv)) * q.groups_b;
-  const int m = in_by_out ? d : p, n = in_by_out ? p : d;
-  q.tiles_n = ceil_div(n, 64);
-  const long long wgrad = grad_out ? static_cast<long long>(ceil_div(m, 64)) * q.tiles_n : 0;
+  const SmallGroups groups = small_groups(n_train, n_val, T, d, p, grad_out != nullptr, ds);
+  q.sv = groups.sv; q.sb = groups.sb; q.groups_b = groups.groups_b; q.ranks = groups.ranks;
+  q.tiles_n = ceil_div(in_by_out ? p : d, 64);
+  const long long gram = groups.gram, wgrad = groups.wgrad;
   const long long col = colsum_out ? static_cast<long long>(n_train + n_val) * ceil_div(p, 1024) : 0;
   GB_REQUIRE(gram + wgrad + col < (1ll << 31), "ghost_dense_small: too many blocks");
-  q.ranks = small_ranks(gram, (T + kSdV - 1) / kSdV * ((T + kSdB - 1) / kSdB), wgrad, n_train * T, d, p, ds);
   q.gram_blocks = static_cast<int>(gram * q.ranks);
   q.wgrad_blocks = static_cast<int>(wgrad);
   const uintptr_t align = is_f32 ? 15 : 7;

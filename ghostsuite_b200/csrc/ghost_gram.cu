@@ -20,6 +20,7 @@
 
 #include "common.cuh"
 #include "gram_operands.cuh"
+#include "launch_rules.h"
 #include "sm100_ptx.cuh"
 
 namespace gb {
@@ -459,20 +460,12 @@ static int gram_resident(int ranks, const DeviceState* ds) {
   return n - 1;
 }
 
-// CTAs that share a tile: as many as make its chain of K steps shortest while all clusters are resident, against what the
-// cluster costs, 4 us, in steps, rounded up for those that share the L2 (us alone and split, bf16 and float32: 8 + 2 x 128 of 512 + 512 13.3 and 15.4,
-// 23.5 and 23.3; 1024 + 1024 17.4 and 17.5, 33.8 and 25.6; 768 + 3072 23.5 and 19.8, 54 and 33; 40 + 4 x 64, 40 tiles,
-// of 768 + 3072 26.5 and 21.9, 65 and 46, of 4096 + 4096 44 and 31, 122 and 77).
-static constexpr double kGramSplitCost = 10.;
+// CTAs that share a tile of 128 x 128
 template <int PARTS>
-static int gram_ranks(long long tiles, int k_steps, const DeviceState* ds) {
-  int best = 1;
-  double cost = k_steps;
-  for (int r = 2; r <= 8 && r <= k_steps; ++r) {
-    const double c = (k_steps + r - 1) / r + kGramSplitCost;
-    if (c < cost && tiles * r <= ds->sm_count && tiles <= gram_resident<PARTS>(r, ds)) { best = r; cost = c; }
-  }
-  return best;
+static int gram_ranks(long long rows_t, long long rows_v, int ka, int kg, const DeviceState* ds) {
+  using Cfg = GramCfg<128, PARTS>;
+  const long long tiles = static_cast<long long>(ceil_div(rows_t, Cfg::BM)) * ceil_div(rows_v, 128);
+  return gram_cluster(tiles, ceil_div(ka, Cfg::BK) + ceil_div(kg, Cfg::BK), ds->sm_count, [&](int r) { return gram_resident<PARTS>(r, ds); });
 }
 
 template <int BN, int PARTS>
@@ -499,7 +492,7 @@ static int launch_gram(const GramOperands& o, int n_train, int n_val, long long 
   const long long tiles = static_cast<long long>(p.m_tiles) * p.n_tiles;
   p.ranks = 1;
   if constexpr (BN == 128) {
-    p.ranks = gram_ranks<PARTS>(tiles, ceil_div(p.ka, Cfg::BK) + ceil_div(p.kg, Cfg::BK), ds);
+    p.ranks = gram_ranks<PARTS>(p.rows_t, p.rows_v, p.ka, p.kg, ds);
     if (p.ranks > 1) {
       if ((rc = gram_smem_attr<BN, PARTS, true>(ds)) != GHOST_OK) return rc;
       GB_CUDA_OK(launch_next_cluster(dim3(p.ranks), ghost_gram_kernel<BN, PARTS, true>, dim3(static_cast<int>(tiles) * p.ranks), dim3(gram_threads(true)),
@@ -521,6 +514,20 @@ static int launch_gram(const GramOperands& o, int n_train, int n_val, long long 
 static int g_gram_pair_mode = 1;
 bool xty_pair_usable(const DeviceState* ds);     // a cluster of two ~198 KB CTAs fits on the device
 
+// Validation columns of a tile of one CTA, 128 or 256, or 0: tiles of 256 x 256 on CTA pairs.
+// Rounds of tiles over the GPU times the cycles of a K step of a tile (128 for 256 x 256 on a pair and 128 x 256 on one
+// SM, 64 for 128 x 128, a tenth more for its operand traffic): 2048 x 1024 tokens are 32 tiles of 256 x 256 on 74
+// pairs, and 128 of 128 x 128 on 148 SMs.
+static int gram_tile(int parts, long long rows_t, long long rows_v, const DeviceState* ds) {
+  auto tiles = [&](int bm, int bn) { return ((rows_t + bm - 1) / bm) * ((rows_v + bn - 1) / bn); };
+  auto rounds = [](long long n, long long workers) { return static_cast<double>((n + workers - 1) / workers); };
+  const double small_tiles = rounds(tiles(128, 128), ds->sm_count) * 70.;
+  const bool pair_wanted = g_gram_pair_mode == 2 || (g_gram_pair_mode == 1 && rows_v <= 8192 &&
+                                                     rounds(tiles(256, 256), ds->sm_count / 2) * 128. < small_tiles * 1.1);
+  if (pair_wanted && rows_v >= 256 && rows_t >= 512 && xty_pair_usable(ds)) return 0;
+  return parts == 2 || rows_v <= 128 || small_tiles * 1.1 < rounds(tiles(128, 256), ds->sm_count) * 128. ? 128 : 256;
+}
+
 int gram_dot(const GramOperands& o, int n_train, int n_val, long long T, int round_mode, float scale, float* M_out, bool cleared, void* stream) {
   const DeviceState* ds = device_state();
   if (!ds) return GHOST_ERR_DEVICE;
@@ -534,24 +541,24 @@ int gram_dot(const GramOperands& o, int n_train, int n_val, long long T, int rou
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (!cleared)
     if (int rc = clear_ahead(M_out, sizeof(float) * static_cast<size_t>(n_val) * n_train, st)) return rc;
-  const long long rows_t = static_cast<long long>(n_train) * T, rows_v = static_cast<long long>(n_val) * T;
-  // Rounds of tiles over the GPU times the cycles of a K step of a tile (128 for 256 x 256 on a pair and 128 x 256 on one
-  // SM, 64 for 128 x 128, a tenth more for its operand traffic): 2048 x 1024 tokens are 32 tiles of 256 x 256 on 74
-  // pairs, and 128 of 128 x 128 on 148 SMs.
-  auto tiles = [&](int bm, int bn) { return ((rows_t + bm - 1) / bm) * ((rows_v + bn - 1) / bn); };
-  auto rounds = [](long long n, long long workers) { return static_cast<double>((n + workers - 1) / workers); };
-  const double small_tiles = rounds(tiles(128, 128), ds->sm_count) * 70.;
-  const bool pair_wanted = g_gram_pair_mode == 2 || (g_gram_pair_mode == 1 && rows_v <= 8192 &&
-                                                     rounds(tiles(256, 256), ds->sm_count / 2) * 128. < small_tiles * 1.1);
-  if (pair_wanted && rows_v >= 256 && rows_t >= 512 && xty_pair_usable(ds))
-    return launch_gram_pair(o, n_train, n_val, T, round_mode, scale, M_out, ds, st);
+  const int bn = gram_tile(o.parts, static_cast<long long>(n_train) * T, static_cast<long long>(n_val) * T, ds);
+  if (bn == 0) return launch_gram_pair(o, n_train, n_val, T, round_mode, scale, M_out, ds, st);
   if (o.parts == 2) return launch_gram<128, 2>(o, n_train, n_val, T, round_mode, scale, M_out, ds, st);
-  if (rows_v <= 128 || small_tiles * 1.1 < rounds(tiles(128, 256), ds->sm_count) * 128.)
-    return launch_gram<128, 1>(o, n_train, n_val, T, round_mode, scale, M_out, ds, st);
+  if (bn == 128) return launch_gram<128, 1>(o, n_train, n_val, T, round_mode, scale, M_out, ds, st);
   return launch_gram<256, 1>(o, n_train, n_val, T, round_mode, scale, M_out, ds, st);
 }
 
 }  // namespace gb
+
+extern "C" int ghost_gram_cluster_size(int parts, int n_train, int n_val, long long T, int ka, int kg) {
+  using namespace gb;
+  const DeviceState* ds = device_state();
+  if (!ds) return GHOST_ERR_DEVICE;
+  GB_REQUIRE((parts == 1 || parts == 2) && n_train > 0 && n_val > 0 && T > 0 && ka > 0 && kg > 0, "ghost_gram_cluster_size: bad size");
+  const long long rows_t = static_cast<long long>(n_train) * T, rows_v = static_cast<long long>(n_val) * T;
+  if (gram_tile(parts, rows_t, rows_v, ds) != 128) return 1;
+  return parts == 2 ? gram_ranks<2>(rows_t, rows_v, ka, kg, ds) : gram_ranks<1>(rows_t, rows_v, ka, kg, ds);
+}
 
 extern "C" int ghost_set_gram_pair_mode(int mode) {
   if (mode < 0 || mode > 2) return GHOST_ERR_INVALID;

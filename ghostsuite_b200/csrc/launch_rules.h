@@ -41,4 +41,37 @@ inline int pick_k_splits(long long tiles, int workers, int kb, double block_us, 
   return splits;
 }
 
+// CTAs that share a tile of a Gram: as many as make its chain of K steps shortest while all clusters are resident, against what the
+// cluster costs, 4 us, in steps, rounded up for those that share the L2 (us alone and split, bf16 and float32: 8 + 2 x 128 of 512 + 512 13.3 and 15.4,
+// 23.5 and 23.3; 1024 + 1024 17.4 and 17.5, 33.8 and 25.6; 768 + 3072 23.5 and 19.8, 54 and 33; 40 + 4 x 64, 40 tiles,
+// of 768 + 3072 26.5 and 21.9, 65 and 46, of 4096 + 4096 44 and 31, 122 and 77).
+// `resident(r)`: clusters of r CTAs that the device holds at a time.
+template <typename Resident>
+int gram_cluster(long long tiles, int k_steps, int sms, Resident&& resident) {
+  constexpr double kSplitCost = 10.;
+  int best = 1;
+  double cost = k_steps;
+  for (int r = 2; r <= 8 && r <= k_steps; ++r) {
+    const double c = (k_steps + r - 1) / r + kSplitCost;
+    if (c < cost && tiles * r <= sms && tiles <= resident(r)) { best = r; cost = c; }
+  }
+  return best;
+}
+
+// Blocks that share a pair of groups of samples in the kernel of few-row layers.  A step of 1024 columns takes a block 1.1 us, and the
+// pairs are few where the rows are long (4 + 12 samples of one token, float32 108 -> 27072: 36.9 us in two blocks, 14.5 in sixteen; 8 + 2 of 20000 -> 10 35.9 and 14.3;
+// 2 + 2 x 8 of 4096 -> 512 17.0 and 14.5).  A tile costs a cluster's barrier, 1.5 us, on top (8 + 2 x 16 of 2048 -> 1024, eight
+// tiles a pair: 38.9, 41 shared).  Where the gradient's blocks take longer than the chain nothing is gained, and
+// they come up slower in clusters (2 + 1 of 768 -> 50000 71 and 77; 16 + 4 of 4095 -> 4097 47 and 53).
+inline int small_cluster(long long gram, long long tiles, long long wgrad, long long rows, long long d, long long p, int sms) {
+  const double others = static_cast<double>((wgrad + 2 * sms - 1) / (2 * sms)) * (2.0 + 0.045 * rows);
+  int best = 1;
+  double cost = 1.1 * ((d + 1023) / 1024 + (p + 1023) / 1024) * tiles;
+  for (int r = 2; r <= 8 && gram * r <= 2ll * sms && cost > others; r *= 2) {
+    const double c = (1.1 * ((d + 1024 * r - 1) / (1024 * r) + (p + 1024 * r - 1) / (1024 * r)) + 1.5) * tiles;
+    if (c < cost) { best = r; cost = c; }
+  }
+  return best;
+}
+
 }  // namespace gb

@@ -115,6 +115,8 @@ int ghost_gram_dot_parts(const void* A, const void* G, int parts, int n_train, i
  * validation tokens, unless smaller tiles fill the GPU better; 2 = the pair kernel from 512 x 256 tokens up.
  * Process-wide. */
 int ghost_set_gram_pair_mode(int mode);
+/* CTAs of a cluster that share a tile in such a call on the current device, 1: none do (operands of `parts` parts). */
+int ghost_gram_cluster_size(int parts, int n_train, int n_val, long long T, int ka, int kg);
 
 /* ---- train-gradient recovery ------------------------------------------------------------------- */
 /* out[m_cols, n_cols] (= or +=) scale * sum_{row < n_rows} X[row, :]^T Y[row, :].
@@ -213,6 +215,8 @@ int ghost_tile_dot_bf16(const void* V, int v_ranks, int v_per_rank, const void* 
  * both bf16, dense rows), products and sums in fp32.  For the sizes ghost_dense_small_fits accepts
  * (returns 1); others are GHOST_ERR_INVALID.  Replaces, for such layers, the lines of both paths. */
 int ghost_dense_small_fits(int is_f32, int n_train, int n_val, long long T, int d, int p);
+/* Blocks of a cluster that share a pair of groups of samples in such a call on the current device, 1: none do. */
+int ghost_dense_small_cluster_size(int n_train, int n_val, long long T, int d, int p, int want_grad);
 int ghost_dense_small(const void* A, const void* B, int is_f32, int n_train, int n_val, long long T, int d,
                       int p, int in_by_out, float* M_out, void* grad_out, int grad_is_f32,
                       float grad_scale, float* colsum_out, void* stream);

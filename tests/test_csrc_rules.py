@@ -148,3 +148,15 @@ def test_splits_of_a_train_gradient(tmp_path):
     # few tiles are shared, one block is not
     few, one = _answers(tmp_path, ["pick_k_splits(1, 148, 64, 0.35, 12, 128. * 128, false)", "pick_k_splits(1, 148, 1, 0.35, 12, 128. * 128, false)"])
     assert few > 4 and one == 1
+
+
+def test_clusters_of_gram_tiles_and_few_row_layers(tmp_path):
+    """Sizes on either side of the lines, on 148 SMs with as many clusters resident as fit: (tiles, K steps), and (pairs of groups, tiles a
+    pair, blocks of the gradient, train rows, columns of the operands)."""
+    gram = {"2, 163": 8, "8, 48": 8, "40, 30": 3, "32, 15": 4, "1, 11": 1, "75, 400": 1, "3, 1": 1}
+    answers = _answers(tmp_path, [f"gram_cluster({c}, 148, [](int r) {{ return 148 / r; }})" for c in gram])
+    assert answers == list(gram.values())
+    assert _answers(tmp_path, ["gram_cluster(2, 163, 148, [](int) { return 0; })"]) == [1]       # a refused question: no cluster
+    small = {"2, 1, 0, 4, 108, 27072": 8, "4, 1, 0, 8, 8192, 260": 8, "2, 8, 0, 128, 2048, 1024": 1, "1, 1, 9384, 2, 768, 50000": 1, "3, 1, 0, 4, 64, 64": 1,
+             "200, 1, 0, 200, 20000, 20000": 1}
+    assert _answers(tmp_path, [f"small_cluster({c}, 148)" for c in small]) == list(small.values())

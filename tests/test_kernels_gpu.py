@@ -84,6 +84,8 @@ def test_gram_hook_tile_shapes(in_by_out, case, dtype):
 def test_gram_tiles_shared_by_clusters(case, dtype, mode):
     n_t, n_v, T, d, p = case
     A, G = make(n_t + n_v, T, d, p, dtype, seed=34)
+    from ghostsuite_b200 import _lib
+    assert _lib.load().ghost_gram_cluster_size(2 if dtype == torch.float32 else 1, n_t, n_v, T, d, p) > 1
     M = ops().gram_dot(A.cuda(), G.cuda(), n_v, round_mode=mode)
     after()
     a, g = A.cuda().double(), G.cuda().double()
@@ -1626,6 +1628,7 @@ def test_few_rows_shared_by_clusters(n_t, n_v, T, d, p, dtype):
     eps = ((4 * (d // 1024 + p // 1024 + 2)) + 2 * 31 + T * T) * 2.0 ** -24
     bound = eps * (grams[2] * grams[3]).sum((2, 3))
     for want_grad in (True, False):
+        assert lib.ghost_dense_small_cluster_size(n_t, n_v, T, d, p, int(want_grad)) > 1
         M = torch.full((n_v, n_t), 7.0, device="cuda")
         grad, sums = torch.full((p, d), 7.0, dtype=dtype, device="cuda"), torch.full((n_t + n_v, p), 7.0, device="cuda")
         _lib.check(lib.ghost_dense_small(A.data_ptr(), G.data_ptr(), f32, n_t, n_v, T, d, p, 0, M.data_ptr(), grad.data_ptr() if want_grad else None,
