@@ -17,12 +17,15 @@
 // The embedding form (kEmb) has token ids in place of A: the rows of P_c^T are gathered by id straight into
 // the staged block, out[b] = scale * sum_t (P_r g_t)(P_c[:, id_t])^T, and only G is streamed.
 //
-// float32 rows, and bf16 rows that TMA cannot read, come through shared memory as they are (kSrc): eight more warps keep
+// float32 rows, and bf16 rows that TMA cannot read, come through shared memory as they are (kSrc): eight or sixteen more warps keep
 // 16-byte copies of them on their way and write what has arrived as the swizzled bf16 blocks -- of float32 data value and residual,
 // three products -- so that such operands too are read once, and several stages ahead (16 x 2048 tokens of 1024 + 1024 float32,
 // k = 32: 99 us with eight warps that loaded into registers, two stages each, 63 so; 4 x 4096 of 2048 + 2049, k = 64: 109 and 94;
 // 32 x 3000 of 1001 + 2003 bf16, k = 64, which were copied with padded rows before: 369 and 217; token table of 4000 float32 features,
-// 16 x 2048 tokens, k = 64: 198 and 164).  Bound by the latency and the shared-memory traffic of the conversion.
+// 16 x 2048 tokens, k = 64: 198 and 164).  Bound by the latency and the shared-memory traffic of the conversion.  (Those are times from
+// cold caches.  With both operands in L2 the way through shared memory is the longer one for rows of a few stages: 16 x 207 of 779 + 256
+// float32 13.6 and 14.5, 20 x 638 of 805 + 65, k = 64, 32 and 36, embedding form 7 x 923 of 76 9.8 and 10.7; from cold caches 19.5 and 19.5, 44
+// and 42, 16.4 and 16.4.)
 //
 // Few (sample, 128-token) units: a unit is one CTA's chain over all columns of G and A, whatever the number of
 // tokens in it, so a small batch leaves the GPU idle for the length of that chain.  There (kSome, kWhole) a cluster of
@@ -54,11 +57,11 @@ struct GpParams {
   long long units;         // B * chunks_per_sample
   int units_per_cta;       // base number of units per CTA
   int units_extra;         // the first `units_extra` CTAs take one more
-  // register loaders: the operands themselves, and where the residual part of P_r / P_c starts (kSrcF32)
+  // loader warps: the operands themselves, and where the residual part of P_r / P_c starts (kSrcF32, kSrcMixed)
   const void *g, *a;
   long long ldg, lda;
   int lo_r, lo_c;
-  int vec_g, vec_a;        // rows on 16-byte (float32) / 8-byte (bf16) boundaries
+  int vec_g, vec_a;        // float32: rows on 16-byte boundaries whose width is a multiple of four
   int half_g, half_a;      // kSrcMixed: which operand is bf16
   float scale;
   float* out;              // sample b at out + b * out_stride, [k_r, k_c] row-major
@@ -548,7 +551,7 @@ gradproj_kernel(const __grid_constant__ CUtensorMap tm_g, const __grid_constant_
         if (k0 >= k1) return false;
         const long long t0 = static_cast<long long>(at.chunk) * BM;
         x.half = kSrc == kSrcBf16 || (kSrc == kSrcMixed && (second ? p.half_a : p.half_g));
-        x.vec = !x.half && (second ? p.vec_a : p.vec_g);
+        x.vec = second ? p.vec_a : p.vec_g;
         const int size = x.half ? 2 : 4;
         const long long from = static_cast<long long>(second ? k0 - kb_r : k0) * BK * size;
         x.pitch = (second ? p.lda : p.ldg) * size;
@@ -981,7 +984,7 @@ static int launch_gradproj_k(const GpOperands& o, GpParams& p, const DeviceState
   return launch_gradproj_src<64, kSrc, kEmb>(o, p, ds, st);
 }
 
-// Chooses how the rows are read: bf16 through TMA where it can, else through registers
+// Chooses how the rows are read: bf16 through TMA where it can, else by loader warps
 template <bool kEmb>
 static int launch_gradproj(const GpOperands& o, GpParams& p, const DeviceState* ds, cudaStream_t st) {
   p.kr_pad = (p.k_r + 15) / 16 * 16;
@@ -998,8 +1001,8 @@ static int launch_gradproj(const GpOperands& o, GpParams& p, const DeviceState* 
   if (o.is_f32) {
     p.half_g = o.is_f32 == 3;
     p.half_a = o.is_f32 == 2;
-    p.vec_g = (p.half_g ? aligned(o.G, o.ldg, 8, 2) : aligned(o.G, o.ldg, 16, 4)) && p.n_r % 4 == 0;
-    p.vec_a = (p.half_a ? aligned(o.A, o.lda, 8, 2) : aligned(o.A, o.lda, 16, 4)) && p.n_c % 4 == 0;
+    p.vec_g = !p.half_g && aligned(o.G, o.ldg, 16, 4) && p.n_r % 4 == 0;
+    p.vec_a = !p.half_a && aligned(o.A, o.lda, 16, 4) && p.n_c % 4 == 0;
     if constexpr (!kEmb) {
       if (o.is_f32 != 1) return launch_gradproj_k<kSrcMixed, kEmb>(o, p, ds, st);
     }
@@ -1007,8 +1010,6 @@ static int launch_gradproj(const GpOperands& o, GpParams& p, const DeviceState* 
   }
   if (aligned(o.G, o.ldg, 16, 2) && (kEmb || aligned(o.A, o.lda, 16, 2)) && p.T < (1ll << 31) - 128)
     return launch_gradproj_k<kSrcTma, kEmb>(o, p, ds, st);
-  p.vec_g = aligned(o.G, o.ldg, 8, 2) && p.n_r % 4 == 0;
-  p.vec_a = aligned(o.A, o.lda, 8, 2) && p.n_c % 4 == 0;
   return launch_gradproj_k<kSrcBf16, kEmb>(o, p, ds, st);
 }
 

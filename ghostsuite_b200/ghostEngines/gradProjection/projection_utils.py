@@ -166,7 +166,9 @@ def projection_similarity(proj_a: torch.Tensor, proj_b: torch.Tensor) -> torch.T
     ``[B, total_proj_dim]`` buffers ``collect_batch`` returns) and larger sets of bfloat16 rows
     (:func:`_bf16_sets_for_kernel`) go through the library's streaming kernel; other larger sets are a
     plain dense GEMM and use cuBLAS through torch, in full fp32 so that scores do not depend on the
-    TF32 setting.  Host tensors are multiplied on the host."""
+    TF32 setting.  The kernel's scores may differ in their last bits from call to call, as the parts of a long row are
+    added in any order; with ``torch.use_deterministic_algorithms`` the larger sets are the GEMM's.  Host tensors are
+    multiplied on the host."""
     if proj_a.shape[-1] != proj_b.shape[-1]:
         raise ValueError("projection sets have different dimensions")
     if proj_a.is_cuda and proj_b.is_cuda and proj_a.dim() == 2 and proj_b.dim() == 2 and \

@@ -386,7 +386,8 @@ int ghost_gradproj_embedding(const long long* ids, const void* G, int g_is_f32, 
 /* S[n1, n2] (row pitch ld_s, fp32) <- scale * P1 P2^T for two blocks of projection rows
  * P1: [n1, D], P2: [n2, D] (both fp32 or both bf16, row pitches ld1, ld2).  Meant for batch-sized
  * blocks (tens of rows) against a very long D = total_proj_dim, where both operands are streamed
- * once; larger blocks are correct but re-read the operands once per 16 x 16 output block.
+ * once, and for larger sets of bf16 rows; those read the operands once per block of scores of up to 64 x 64 (through L2).
+ * Where a block's contraction is spread over more CTAs than a cluster has, they add to the scores in any order.
  * Replaces the proj1 @ proj2.t() of Examples/ghost_gradproj_lm.py:190-196 and
  * Examples/GradProj_LM/plot_error_with_dim.py:69-86 while the rows are still on the device. */
 int ghost_projection_similarity(const void* P1, const void* P2, int is_f32, int n1, int n2, long long D,
