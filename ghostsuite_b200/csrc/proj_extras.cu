@@ -534,6 +534,138 @@ static int dispatch_similarity(const SimParams& p, bool vec, const DeviceState* 
   }
 }
 
+// One bf16 row against many: exact products, float32 sums that are kept apart by lane and element and added up over lanes, warps and
+// CTAs in a fixed order.  The tensor core's sums truncate, and where there is one row to share out its chains are long: 1 x 200 rows of
+// 512 came out 5.8e-8 off the 64-bit scores (float32 GEMM of the library: 4.3e-8, here 4.3e-8), of 65536 1.3e-7 (6.7e-8, 4.6e-8).
+// A warp has four rows, so that the one row's elements are loaded once for four products, and eight loads of theirs are in flight.
+// Bound by streaming the rows (1 x 512 of 262144 5.8 TB/s); unaligned ones by their element loads.
+struct SimRow {
+  const __nv_bfloat16 *one, *many;       // [D], [n, D] with row pitch ld
+  int n, warps, ranks;     // warps of a CTA and CTAs of a cluster that share four rows
+  long long D, ld;
+  float scale;
+  float* S;                // score i at S + i * step
+  long long step;
+};
+
+// Sum of the first n of eight values, n a power of two, in pairs of pairs
+template <typename F> __device__ __forceinline__ float row_sum8(int n, F&& v) {
+  float x[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    x[i] = 0.f;
+    if (i < n) x[i] = v(i);
+  }
+  return ((x[0] + x[1]) + (x[2] + x[3])) + ((x[4] + x[5]) + (x[6] + x[7]));
+}
+
+template <bool VEC>
+__global__ void __launch_bounds__(256, 2) proj_row_kernel(const SimRow q) {
+  stream_order();
+  __shared__ float part[8][4];
+  __shared__ float total[4];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rank = static_cast<int>(blockIdx.x) % q.ranks;
+  const long long row0 = 4 * (static_cast<long long>(blockIdx.x / q.ranks) * (8 / q.warps) + warp / q.warps);
+  const int share = rank * q.warps + warp % q.warps, shares = q.ranks * q.warps;
+  float acc[4][8];
+#pragma unroll
+  for (int r = 0; r < 4; ++r)
+#pragma unroll
+    for (int e = 0; e < 8; ++e) acc[r][e] = 0.f;
+  if (row0 < q.n) {
+    const __nv_bfloat16* y[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) y[r] = q.many + (row0 + r < q.n ? row0 + r : q.n - 1) * q.ld;
+    if constexpr (VEC) {                 // D is a multiple of eight
+      const long long step = shares * 256ll;
+      for (long long k0 = (share * 32 + lane) * 8; k0 < q.D; k0 += 2 * step) {
+        uint4 a[2], b[2][4];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const long long k = k0 + i * step;
+          const bool in = k < q.D;
+          a[i] = make_uint4(0u, 0u, 0u, 0u);
+          if (in) a[i] = *reinterpret_cast<const uint4*>(q.one + k);
+#pragma unroll
+          for (int r = 0; r < 4; ++r) {
+            b[i][r] = make_uint4(0u, 0u, 0u, 0u);
+            if (in) b[i][r] = *reinterpret_cast<const uint4*>(y[r] + k);
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+          for (int r = 0; r < 4; ++r) {
+            const uint32_t u[4] = {a[i].x, a[i].y, a[i].z, a[i].w}, v[4] = {b[i][r].x, b[i][r].y, b[i][r].z, b[i][r].w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              acc[r][2 * e] = fmaf(__uint_as_float(u[e] << 16), __uint_as_float(v[e] << 16), acc[r][2 * e]);
+              acc[r][2 * e + 1] = fmaf(__uint_as_float(u[e] & 0xffff0000u), __uint_as_float(v[e] & 0xffff0000u), acc[r][2 * e + 1]);
+            }
+          }
+      }
+    } else {                             // rows that begin anywhere: element by element
+      auto bits = [](const __nv_bfloat16* at) { return static_cast<uint32_t>(*reinterpret_cast<const unsigned short*>(at)) << 16; };
+      const long long step = shares * 32ll;
+      for (long long k0 = share * 32 + lane; k0 < q.D; k0 += 8 * step) {
+        uint32_t a[8], b[8][4];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const long long k = k0 + i * step;
+          const bool in = k < q.D;
+          a[i] = 0u;
+          if (in) a[i] = bits(q.one + k);
+#pragma unroll
+          for (int r = 0; r < 4; ++r) {
+            b[i][r] = 0u;
+            if (in) b[i][r] = bits(y[r] + k);
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+          for (int r = 0; r < 4; ++r) acc[r][i] = fmaf(__uint_as_float(a[i]), __uint_as_float(b[i][r]), acc[r][i]);
+      }
+    }
+  }
+  float sum = 0.f;                       // lanes 0 to 3: of row0 + lane
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    float v = ((acc[r][0] + acc[r][1]) + (acc[r][2] + acc[r][3])) + ((acc[r][4] + acc[r][5]) + (acc[r][6] + acc[r][7]));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (lane == r) sum = v;
+  }
+  if (q.warps > 1) {
+    if (lane < 4) part[warp][lane] = sum;
+    __syncthreads();
+    if (lane < 4) sum = row_sum8(q.warps, [&](int w) { return part[warp / q.warps * q.warps + w][lane]; });
+  }
+  if (q.ranks > 1) {                     // the CTA's warps share the same rows
+    if (threadIdx.x < 4) total[lane] = sum;
+    cluster_sync_all();
+    if (rank == 0 && threadIdx.x < 4) sum = row_sum8(q.ranks, [&](int r) { return ld_cluster_f32(map_to_cta(smem_u32(&total[lane]), r)); });
+    cluster_sync_all();                  // no CTA leaves while another reads its sums
+  }
+  if (rank == 0 && warp % q.warps == 0 && lane < 4 && row0 + lane < q.n) q.S[(row0 + lane) * q.step] = sum * q.scale;
+}
+
+// Warps that share four rows, in CTAs of eight: as many as two CTAs an SM hold while a lane has a piece of eight elements.
+static int launch_row(SimRow q, bool vec, const DeviceState* ds, cudaStream_t st) {
+  const long long fours = (q.n + 3ll) / 4;
+  int shares = 1;
+  while (shares < 64 && 2 * shares * fours <= 16ll * ds->sm_count && 2ll * shares * 256 <= q.D) shares *= 2;
+  q.warps = shares < 8 ? shares : 8;
+  q.ranks = shares / q.warps;
+  const int per_cta = 8 / q.warps;
+  const unsigned grid = static_cast<unsigned>((fours + per_cta - 1) / per_cta) * q.ranks;
+  if (vec) GB_CUDA_OK(launch_next_cluster(dim3(q.ranks), proj_row_kernel<true>, dim3(grid), dim3(256), 0, st, q));
+  else GB_CUDA_OK(launch_next_cluster(dim3(q.ranks), proj_row_kernel<false>, dim3(grid), dim3(256), 0, st, q));
+  count_launch();
+  return post_launch("proj_row_kernel");
+}
+
 }  // namespace gb
 
 using namespace gb;
@@ -554,5 +686,17 @@ extern "C" int ghost_projection_similarity(const void* P1, const void* P2, int i
   p.err = ds->err_word;
   const bool vec = D % 8 == 0 && (ld1 * esize) % 16 == 0 && (ld2 * esize) % 16 == 0 &&
                    ((reinterpret_cast<uintptr_t>(P1) | reinterpret_cast<uintptr_t>(P2)) & 15u) == 0;
+  // Longer sets against one row, which callers would else send to a float32 product (us, this kernel and the ones below: 1 x 129 rows of 2048
+  // 2.4 and 3.6, 1 x 512 of 262144 45.9 and 59.6, 1 x 200 of 1711 4.3 and 6.3; 1 x 200 of 128 2.1 and 1.7, 1 x 65536 of it 12.3 and 6.8).
+  if (!is_f32 && (n1 == 1 || n2 == 1) && (n1 > 128 || n2 > 128) && D >= 96) {
+    SimRow q = {};
+    q.one = static_cast<const __nv_bfloat16*>(n1 == 1 ? P1 : P2);
+    q.many = static_cast<const __nv_bfloat16*>(n1 == 1 ? P2 : P1);
+    q.n = n1 == 1 ? n2 : n1;
+    q.ld = n1 == 1 ? ld2 : ld1;
+    q.step = n1 == 1 ? 1 : ld_s;
+    q.D = D; q.scale = scale; q.S = S;
+    return launch_row(q, vec, ds, st);
+  }
   return is_f32 ? dispatch_similarity<float>(p, vec, ds, st) : dispatch_similarity<__nv_bfloat16>(p, vec, ds, st);
 }

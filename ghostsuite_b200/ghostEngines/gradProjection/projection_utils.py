@@ -134,11 +134,9 @@ def _bf16_sets_for_kernel(a: torch.Tensor, b: torch.Tensor) -> bool:
 
     Products of bfloat16 values are exact in its float32 sums, so it needs no float32 copies of the rows, and
     no float32 GEMM either (3 x 200 rows of 98304: 7.3 us against 213; 128 x 512 of 4096 8.7 and 87; 512 x 512 of
-    98304 339 and 1627; 4096 x 4096 of 4096 715 and 2499).  It is taken where its error against 64 bits is no larger than the GEMM's
-    (0.3 to 1.0 times, 1.03 once, from two rows of 96 elements on), which leaves out
-    * one row against many, which the library reduces in a better order (1 x 200 of 512 5.9e-8 and 4.2e-8, of 65536 1.3e-7 and 7e-8);
-    * short rows: below 96 elements 1.0 to 1.3 times (2 x 200 of 64 5.1e-8 and 4.7e-8), and with many scores the kernel's stores are the slower
-      ones too (20000 x 20000 of 8: 793 us and 564).
+    98304 339 and 1627; 4096 x 4096 of 4096 715 and 2499; 1 x 512 of 65536 10.6 and 139).  It is taken where its error against 64 bits is no
+    larger than the GEMM's: from 96 elements on 0.3 to 1.04 times that, shorter rows 1.0 to 1.3 times (2 x 200 of 64 5.1e-8 and
+    4.7e-8); many scores of short rows are the GEMM's by time too (20000 x 20000 of 8: 564 us, in the kernel 793).
     Rows that do not start on 16-byte boundaries are read by element: 512 x 512 of 25871 311 us and 512,
     1024 x 1024 of them 1259 and 1174, so there it ends at 512 rows.  float32 rows stay with the GEMM, which
     takes them as they are; so does what the kernel does not know: gradients, transforms, autocast, sparse
@@ -150,7 +148,7 @@ def _bf16_sets_for_kernel(a: torch.Tensor, b: torch.Tensor) -> bool:
             or torch.compiler.is_compiling() or _followed_by_torch is None or _followed_by_torch():
         return False
     dim, rows = a.shape[1], max(a.shape[0], b.shape[0])
-    if min(a.shape[0], b.shape[0]) < 2 or dim < 96 or rows > 1 << 16 or a.stride(1) != 1 or b.stride(1) != 1 \
+    if min(a.shape[0], b.shape[0]) == 0 or dim < 96 or rows > 1 << 16 or a.stride(1) != 1 or b.stride(1) != 1 \
             or min(a.stride(0), b.stride(0)) < dim:
         return False
     aligned = dim % 8 == 0 and all(t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0 for t in (a, b))

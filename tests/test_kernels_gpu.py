@@ -927,8 +927,8 @@ def test_projection_similarity_of_large_bf16_sets(n1, n2, D):
         S = U.projection_similarity(rows, b)
         after()
         assert S.dtype == torch.float32 and ((S.double() - ref).abs() <= bound).all()
-    # one row, short rows and many unaligned ones stay with the GEMM
-    kernel = min(n1, n2) > 1 and D >= 96 and (D % 8 == 0 or max(n1, n2) <= 512)
+    # short rows and many unaligned ones stay with the GEMM
+    kernel = D >= 96 and (D % 8 == 0 or max(n1, n2) <= 512)
     assert ops().launch_count() > before if kernel else ops().launch_count() == before
     bits = a.clone()
     bits[0, 0] = float("inf")
@@ -953,6 +953,34 @@ def test_error_of_large_bf16_similarity_sets(n1, n2, D):
         errors.append([((x.double() - ref).norm() / ref.norm()).item() ** 2 for x in (U.projection_similarity(a, b), a.float() @ b.float().t())])
     after()
     assert sum(e[0] for e in errors) <= 1.1 ** 2 * sum(e[1] for e in errors)
+
+
+# one row against more than 128: rows that no four of a warp fill, one warp to 64 of them to a row, one round of loads and several, columns that end
+# inside one; rows on 16-byte boundaries and anywhere, between values that nothing may take in; scores as a row, a column, and a column of
+# wider rows
+@pytest.mark.parametrize("n, D", [(129, 96), (130, 97), (131, 264), (132, 511), (133, 4104), (200, 2049), (129, 131080), (130, 70001), (9475, 256), (9480, 101)])
+def test_similarity_of_one_bf16_row(n, D):
+    from ghostsuite_b200 import _lib
+    lib = _lib.load()
+    g = torch.Generator(device="cuda").manual_seed(27)
+    nan = torch.full((n * (D + 8) + 16,), float("nan"), device="cuda").bfloat16()
+    for offset in (0, 8) if D % 8 == 0 else (0, 3):
+        one = nan[:D + 16].clone()[offset:offset + D]
+        many = nan.clone()[offset:offset + n * (D + 8)].view(n, D + 8)[:, :D]
+        one.copy_(torch.randn(D, generator=g, device="cuda"))
+        many.copy_(torch.randn(n, D, generator=g, device="cuda"))
+        ref = 0.5 * (many.double() @ one.double())
+        # products are exact; a lane's chains are D / 256 sums, then a tree over elements, lanes, warps and CTAs
+        bound = (D / 256 + 16) * 2.0 ** -24 * 0.5 * (many.double().abs() @ one.double().abs())
+        one = one.view(1, D)
+        rows = [ops().projection_similarity(one, many, 0.5), ops().projection_similarity(many, one, 0.5).t()]
+        wide = torch.full((n, 3), 7.0, device="cuda")
+        _lib.check(lib.ghost_projection_similarity(many.data_ptr(), one.data_ptr(), 0, n, 1, D, D + 8, D, 0.5, wide.data_ptr(), 3, torch.cuda.current_stream().cuda_stream))
+        after()
+        for S in (*rows, wide[:, :1].t()):
+            assert ((S[0].double() - ref).abs() <= bound).all()
+        assert torch.equal(rows[0], rows[1]) and torch.equal(rows[0], wide[:, :1].t()) and (wide[:, 1:] == 7).all()
+        assert torch.equal(rows[0], ops().projection_similarity(one, many, 0.5))           # the same bits again
 
 
 # one stage, one cluster and many of them; rows that TMA reads and rows that it cannot (odd lengths, odd pitches), each at
