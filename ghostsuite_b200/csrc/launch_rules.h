@@ -7,7 +7,9 @@ namespace gb {
 // Whether bf16 rows of a GradProj call that TMA cannot read are copied, padded, instead of being brought through the kernel's loader
 // warps.  A copy is a launch and two passes over them; what the loaders add is about half a microsecond per 64 columns of a CTA's
 // chain.  Loaders and copies, us: 26 x 471 tokens of 9408 + 795 109 and 62 (only the 795 columns are copied); 10 x 30 of
-// 6912 + 2579 19.2 and 12.1; 28 x 5 of 3957 + 9063 44.8 and 21.2; 14 x 1894 of 1007 + 1088 51.7 and 54; 32 x 3000 of 1001 + 2003 217 and 369.
+// 6912 + 2579 19.2 and 12.1; 28 x 5 of 3957 + 9063 44.8 and 21.2; 32 x 3000 of 1001 + 2003 217 and 369; 14 x 1894 of 1007 + 1088, where the two
+// meet, 51.1 and 51.3.  A copy counts as 4 us, more than it takes on the GPU, for the launch on the host: hook of 44 x 211 of 384 + 79 13.3
+// and 15.5, its kernels 13.6 and 11.3.
 inline bool gradproj_copies(long long B, long long T, long long n_r, long long n_c, bool ready_r, bool ready_c, int sm_count) {
   if ((ready_r && ready_c) || B <= 0 || T <= 0) return false;      // nothing to copy; an empty call is the kernel's to refuse
   const long long units = B * ((T + 127) / 128), sms = std::max(1, sm_count);
