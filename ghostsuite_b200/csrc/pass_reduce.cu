@@ -209,6 +209,9 @@ pass_reduce_kernel(const __grid_constant__ PassJobs<CAP> jobs) {
           if (staged_sums && v0 == 0) pass_staged_sums(j, train, f, width, stage, pitch);
           auto products = [&](auto some) {     // of the first rows; a test a row costs more than products that are not read (24 jobs of 32 + 8
                                                // vectors of 4096 19.4 us with tests, 16.4 without)
+            // two steps of sixteen rows at a time would take 143 registers, which leaves an SM one block: 48 jobs of 53 + 17 vectors of 2560 77 us so, 42
+            // with 128; 24 of 11 + 13 x 640 9.4 and 6.0
+#pragma unroll (NV == 16 ? 1 : 2)
             for (int q = warp * 4; q < width; q += 32) {
               const float4 x = *reinterpret_cast<const float4*>(stage + lane * pitch + q);
 #pragma unroll
